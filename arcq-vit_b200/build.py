@@ -18,7 +18,7 @@ LIB_PATH = PKG_DIR / "libarcq_b200.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-    "--shared", "-Xcompiler", "-fPIC",
+    "--shared", "-Xcompiler", "-fPIC", "--split-compile=0",
 ]
 
 

@@ -2,6 +2,7 @@
 // The kernels live in the .cuh files included below; this is the only translation unit.
 #include <cuda_runtime.h>
 #include <mutex>
+#include <type_traits>
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -13,8 +14,8 @@
 #include "../../include/arcq_b200.h"
 #include "ptx.cuh"
 #include "act_quant.cuh"
-#include "act_quant_v2.cuh"
-#include "act_quant_v4.cuh"
+#include "group_quant.cuh"
+#include "act_quant_tile.cuh"
 #include "codes.cuh"
 #include "packed_gemm.cuh"
 #include "gemm_ws.cuh"
@@ -152,120 +153,6 @@ cudaError_t launch_act_quant(const void* x, long long groups, const float* th, c
   return cudaGetLastError();
 }
 
-// Second-design quantizer (one thread per group, staged loads): taken when the buffers are aligned for its
-// 16-byte accesses and the reconstruction, if asked for, has the input's element type.
-template <typename T, int BITS, int PRE = 0>
-cudaError_t launch_act_quant_v2(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed,
-                                float* mu, float* sg, float* cs, void* xhat, cudaStream_t st) {
-  const size_t smem = arcq::aq2_smem_bytes<T>();
-  const long long tiles = (groups + arcq::kAq2Threads - 1) / arcq::kAq2Threads;
-  const long long cap = static_cast<long long>(sm_count()) * 4;
-  const int grid = static_cast<int>(tiles < cap ? tiles : cap);
-  const T* xt = static_cast<const T*>(x);
-  cudaError_t e;
-  if (xhat == nullptr) {
-    auto k = arcq::act_quant_v2_kernel<T, BITS, T, false, PRE>;
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-    launch_pdl(k, grid, arcq::kAq2Threads, smem, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<T*>(nullptr));
-  } else if (packed == nullptr) {
-    auto k = arcq::act_quant_v2_kernel<T, BITS, T, true, PRE, false>;
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-    launch_pdl(k, grid, arcq::kAq2Threads, smem, st, xt, groups, th, cb, static_cast<uint8_t*>(nullptr), mu, sg, cs, static_cast<T*>(xhat));
-  } else {
-    auto k = arcq::act_quant_v2_kernel<T, BITS, T, true, PRE>;
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-    launch_pdl(k, grid, arcq::kAq2Threads, smem, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<T*>(xhat));
-  }
-  return cudaGetLastError();
-}
-
-// Two-lanes-per-group form of the staged quantizer (16-bit element types): same results, twice the warps.
-template <typename T, int BITS, int PRE = 0>
-cudaError_t launch_act_quant_v4(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed,
-                                float* mu, float* sg, float* cs, void* xhat, cudaStream_t st) {
-  const size_t smem = arcq::aq4_smem_bytes<T>();
-  const long long tiles = (groups + arcq::kAq4Groups - 1) / arcq::kAq4Groups;
-  const long long cap = static_cast<long long>(sm_count()) * 4;
-  const int grid = static_cast<int>(tiles < cap ? tiles : cap);
-  const T* xt = static_cast<const T*>(x);
-  T* xo = static_cast<T*>(xhat);
-  cudaError_t e;
-#define ARCQ_AQ4(WX, WP)                                                                                          \
-  do {                                                                                                           \
-    auto k = arcq::act_quant_v4_kernel<T, BITS, WX, PRE, WP>;                                                    \
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));            \
-    if (e != cudaSuccess) return e;                                                                              \
-    launch_pdl(k, grid, arcq::kAq4Threads, smem, st, xt, groups, th, cb, packed, mu, sg, cs, xo);                  \
-  } while (0)
-  if (xhat == nullptr) ARCQ_AQ4(false, true);
-  else if (packed == nullptr) ARCQ_AQ4(true, false);
-  else ARCQ_AQ4(true, true);
-#undef ARCQ_AQ4
-  return cudaGetLastError();
-}
-
-template <typename T> struct IsSixteenBit { static constexpr bool value = sizeof(T) == 2; };
-
-template <typename T, int BITS, int PRE>
-cudaError_t launch_staged(bool two_lane, const void* x, long long groups, const float* th, const float* cb,
-                          uint8_t* packed, float* mu, float* sg, float* cs, void* xhat, cudaStream_t st) {
-  if constexpr (IsSixteenBit<T>::value) {
-    if (two_lane) return launch_act_quant_v4<T, BITS, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, st);
-  }
-  return launch_act_quant_v2<T, BITS, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, st);
-}
-
-template <typename T, int PRE>
-cudaError_t dispatch_act_quant_bits(int bits, const void* x, int x_dtype, long long groups, const float* th,
-                                    const float* cb, uint8_t* packed, float* mu, float* sg, float* cs, void* xhat,
-                                    int xhat_dtype, cudaStream_t st) {
-  // The one-thread-per-group kernel needs enough groups to fill the machine (148 SMs x 4 blocks x 128
-  // threads); below that the 8-lanes-per-group kernel has 8 times the parallelism and lower latency.
-  const long long min_groups = opt(O_AQ2_MIN_GROUPS) > 0 ? opt(O_AQ2_MIN_GROUPS) : static_cast<long long>(sm_count()) * 4 * arcq::kAq2Threads / 2;
-  const bool enough = groups >= min_groups;
-  const bool v2 = enough && opt(O_ACT_QUANT_V1) == 0 && aligned(x, 16) &&
-                  (packed == nullptr || aligned(packed, 16)) &&
-                  (xhat == nullptr || (xhat_dtype == x_dtype && aligned(xhat, 16)));
-  if (v2) {
-    // The two-lanes-per-group form (16-bit inputs) measured faster only where the per-element arithmetic is
-    // long, i.e. with the fused GELU (42 vs 48 us on [12608,1536]); the plain quantizer stays one thread per
-    // group (9.3 vs 10.8 us on [12608,384]).  ARCQ_ACT_QUANT_V2 = 1 / 2 forces the one-lane / two-lane form.
-    const int force = opt(O_ACT_QUANT_V2);
-    const bool two_lane = force == 2 || (force == 0 && PRE == 1);
-    switch (bits) {
-      case 4: return launch_staged<T, 4, PRE>(two_lane, x, groups, th, cb, packed, mu, sg, cs, xhat, st);
-      case 3: return launch_staged<T, 3, PRE>(two_lane, x, groups, th, cb, packed, mu, sg, cs, xhat, st);
-      default: return launch_staged<T, 2, PRE>(two_lane, x, groups, th, cb, packed, mu, sg, cs, xhat, st);
-    }
-  }
-  switch (bits) {
-    case 4: return launch_act_quant<T, 4, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st);
-    case 3: return launch_act_quant<T, 3, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st);
-    default: return launch_act_quant<T, 2, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st);
-  }
-}
-
-// Tile width for the packed GEMM: the widest multiple of 16 (<= 256) that divides N, narrowed while
-// the grid would leave most of the SMs idle.
-int choose_bn(long long M, long long N) {
-  static const int cand[] = {256, 192, 128, 96, 64, 48, 32, 16};
-  const long long tiles_m = (M + arcq::kTileM - 1) / arcq::kTileM;
-  int widest = 0, narrowest = 0;
-  for (int c : cand) {
-    if (N % c != 0) continue;
-    if (widest == 0) widest = c;
-    if (tiles_m * (N / c) >= sm_count()) return c;  // widest tile that still fills the machine
-    if (c >= 32 || narrowest == 0) narrowest = c;
-  }
-  if (widest != 0) return narrowest;
-  const long long r = (N + 15) / 16 * 16;  // N not a multiple of 16: pad the last tile column
-  return static_cast<int>(r < 256 ? r : 256);
-}
-
-
 // ---- tensor maps (driver entry point fetched through the runtime, so libcuda is not linked) ----
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {   // resolved once; the initialisation is thread-safe
@@ -319,6 +206,107 @@ bool make_tensor_map_2d(CUtensorMap* tm, const void* base, CUtensorMapDataType d
   slot.used = true;
   return true;
 }
+
+// Tile form of the quantizer (a thread per group, tiles by TMA): taken when the buffers are aligned for 16-byte accesses and
+// the reconstruction, if asked for, has the input's element type or is the fp16 one of an fp32 input.
+template <typename T, int BITS, int PRE, typename XH, bool WX, bool WP>
+cudaError_t launch_act_quant_tile(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed,
+                                  float* mu, float* sg, float* cs, void* xhat, cudaStream_t st) {
+  auto k = arcq::act_quant_tile_kernel<T, BITS, XH, WX, PRE, WP>;
+  constexpr int smem = static_cast<int>(arcq::aqt_smem_bytes<T>());
+  static thread_local int done_dev = -1;      // shared-memory ceiling raised once per (host thread, device)
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (done_dev != dev) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    done_dev = dev;
+  }
+  // a group is one row of 64 16-bit values, or two rows of 32 fp32 values
+  auto map = [&](CUtensorMap* tm, const void* p, int bytes, CUtensorMapDataType dt) {
+    const int rows_per = bytes == 4 ? 2 : 1;
+    return make_tensor_map_2d(tm, p, dt, bytes, static_cast<uint64_t>(groups) * rows_per, 64 / rows_per, 64 / rows_per, 32 * rows_per,
+                              CU_TENSOR_MAP_SWIZZLE_128B);
+  };
+  auto type_of = [](auto v) {
+    using V = decltype(v);
+    return sizeof(V) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                          : std::is_same<V, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  };
+  CUtensorMap tm_x, tm_out;
+  if (!map(&tm_x, x, static_cast<int>(sizeof(T)), type_of(T{}))) return cudaErrorInvalidValue;
+  if (WX) {
+    if (!map(&tm_out, xhat, static_cast<int>(sizeof(XH)), type_of(XH{}))) return cudaErrorInvalidValue;
+  } else {
+    tm_out = tm_x;
+  }
+  const long long blocks = (groups + arcq::kAqtThreads - 1) / arcq::kAqtThreads;
+  const long long cap = static_cast<long long>(sm_count()) * (sizeof(T) == 2 ? 4 : 3);
+  launch_pdl(k, static_cast<unsigned>(blocks < cap ? blocks : cap), arcq::kAqtThreads, smem, st, tm_x, tm_out, groups, th, cb,
+             packed, mu, sg, cs, status_ptr());
+  return cudaGetLastError();
+}
+
+template <typename T, int BITS, int PRE, typename XH>
+cudaError_t launch_act_quant_tile_outputs(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed,
+                                          float* mu, float* sg, float* cs, void* xhat, cudaStream_t st) {
+  if (xhat == nullptr) return launch_act_quant_tile<T, BITS, PRE, XH, false, true>(x, groups, th, cb, packed, mu, sg, cs, xhat, st);
+  if (packed == nullptr) return launch_act_quant_tile<T, BITS, PRE, XH, true, false>(x, groups, th, cb, packed, mu, sg, cs, xhat, st);
+  return launch_act_quant_tile<T, BITS, PRE, XH, true, true>(x, groups, th, cb, packed, mu, sg, cs, xhat, st);
+}
+
+template <typename T, int BITS, int PRE>
+cudaError_t dispatch_act_quant_tile(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed, float* mu,
+                                    float* sg, float* cs, void* xhat, bool xhat_f16, cudaStream_t st) {
+  if constexpr (sizeof(T) == 4) {
+    if (xhat != nullptr && xhat_f16)
+      return launch_act_quant_tile_outputs<T, BITS, PRE, __half>(x, groups, th, cb, packed, mu, sg, cs, xhat, st);
+  }
+  return launch_act_quant_tile_outputs<T, BITS, PRE, T>(x, groups, th, cb, packed, mu, sg, cs, xhat, st);
+}
+
+template <typename T, int PRE>
+cudaError_t dispatch_act_quant_bits(int bits, const void* x, int x_dtype, long long groups, const float* th,
+                                    const float* cb, uint8_t* packed, float* mu, float* sg, float* cs, void* xhat,
+                                    int xhat_dtype, cudaStream_t st) {
+  // The one-thread-per-group kernel needs enough groups to fill the machine (148 SMs x 4 blocks x 128
+  // threads); below that the 8-lanes-per-group kernel has 8 times the parallelism and lower latency.
+  const long long min_groups = opt(O_AQ2_MIN_GROUPS) > 0 ? opt(O_AQ2_MIN_GROUPS) : static_cast<long long>(sm_count()) * 4 * arcq::kAqtThreads / 2;
+  const bool xhat_f16 = xhat != nullptr && xhat_dtype == ARCQ_DT_F16;
+  const bool tile = groups >= min_groups && groups < (1ll << 30) && opt(O_ACT_QUANT_V1) == 0 && aligned(x, 16) &&
+                    (packed == nullptr || aligned(packed, 16)) &&
+                    (xhat == nullptr || ((xhat_dtype == x_dtype || (x_dtype == ARCQ_DT_F32 && xhat_f16)) && aligned(xhat, 16)));
+  if (tile) {
+    switch (bits) {
+      case 4: return dispatch_act_quant_tile<T, 4, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st);
+      case 3: return dispatch_act_quant_tile<T, 3, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st);
+      default: return dispatch_act_quant_tile<T, 2, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st);
+    }
+  }
+  switch (bits) {
+    case 4: return launch_act_quant<T, 4, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st);
+    case 3: return launch_act_quant<T, 3, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st);
+    default: return launch_act_quant<T, 2, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st);
+  }
+}
+
+// Tile width for the packed GEMM: the widest multiple of 16 (<= 256) that divides N, narrowed while
+// the grid would leave most of the SMs idle.
+int choose_bn(long long M, long long N) {
+  static const int cand[] = {256, 192, 128, 96, 64, 48, 32, 16};
+  const long long tiles_m = (M + arcq::kTileM - 1) / arcq::kTileM;
+  int widest = 0, narrowest = 0;
+  for (int c : cand) {
+    if (N % c != 0) continue;
+    if (widest == 0) widest = c;
+    if (tiles_m * (N / c) >= sm_count()) return c;  // widest tile that still fills the machine
+    if (c >= 32 || narrowest == 0) narrowest = c;
+  }
+  if (widest != 0) return narrowest;
+  const long long r = (N + 15) / 16 * 16;  // N not a multiple of 16: pad the last tile column
+  return static_cast<int>(r < 256 ? r : 256);
+}
+
 
 struct WsConfig {
   int bn, ws, sa, nbb, stationary, grid;
@@ -1152,10 +1140,15 @@ int arcq_add_layernorm_act_quant(const void* x, const void* y, const float* gamm
   const unsigned grid = static_cast<unsigned>(tiles < cap ? tiles : cap);
   const size_t smem = arcq::lnq_smem_bytes();
   const __half *xh = static_cast<const __half*>(x), *yh = static_cast<const __half*>(y);
-  __half *so = static_cast<__half*>(sum_out), *ho = static_cast<__half*>(h_out), *xo = static_cast<__half*>(xhat);
+  __half *so = static_cast<__half*>(sum_out), *ho = static_cast<__half*>(h_out);
+  if (M * G >= (1ll << 30)) return fail(ARCQ_E_TOO_LARGE, "too many groups");
+  CUtensorMap tm_out;
+  if (!make_tensor_map_2d(&tm_out, xhat, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, static_cast<uint64_t>(M * G), 64, 64, 32,
+                          CU_TENSOR_MAP_SWIZZLE_128B))
+    return fail(ARCQ_E_CUDA, "cuTensorMapEncodeTiled failed for the reconstruction");
 #define ARCQ_LAUNCH_LNQ(LN, B, HASY)                                                                                   \
-  launch_pdl(arcq::add_layernorm_act_quant_kernel<LN, B, HASY>, grid, arcq::kLnqThreads, smem, st, xh, yh, gamma, beta, \
-             eps, static_cast<long long>(M), thresholds, codebook, so, ho, xo)
+  launch_pdl(arcq::add_layernorm_act_quant_kernel<LN, B, HASY>, grid, arcq::kLnqThreads, smem, st, tm_out, xh, yh, gamma, \
+             beta, eps, static_cast<long long>(M), thresholds, codebook, so, ho)
 #define ARCQ_LNQ_BITS(LN, HASY)                                                                                         \
   do {                                                                                                                  \
     if (bits == 4) ARCQ_LAUNCH_LNQ(LN, 4, HASY);                                                                         \

@@ -13,7 +13,7 @@
 // too small for a 128-row tensor-memory tile to pay (two thirds of a second tile would be padding), and the kernel is
 // bound by its latency chain, not by the tensor pipe.
 //
-// Quantizer epilogue: same arithmetic as the quantizer kernels (act_quant_v2.cuh), on the fp16-rounded outputs, so
+// Quantizer epilogue: same arithmetic as the quantizer kernels (group_quant.cuh), on the fp16-rounded outputs, so
 // the result is bit-identical to quantising the matrix the plain form of this kernel writes.  A row's 64 values
 // sit in four lanes (lane%4 = q holds columns 8n+2q, 8n+2q+1, n = 0..7): the reference's lane sums
 //   v[l] = ((x[l]+x[32+l]) + (x[8+l]+x[40+l])) + (x[16+l]+x[48+l])) + (x[24+l]+x[56+l])   for l = 2q, 2q+1
@@ -22,7 +22,7 @@
 #pragma once
 #include <cuda_fp16.h>
 #include "ptx.cuh"
-#include "act_quant_v2.cuh"
+#include "act_quant.cuh"
 
 namespace arcq {
 

@@ -9,102 +9,50 @@
 // replaces, so that the results are bit-identical to arcq_add_layernorm followed by arcq_act_quant:
 //   1. LayerNorm with the lane layout of add_layernorm_rows_kernel (LANES lanes per row, 16-byte accesses, the same
 //      device function), writing h into padded group rows of shared memory;
-//   2. the quantizer of act_quant_v2_kernel: one thread per 64-group reads its row, classifies with the exact
-//      division-free test and the first-guess grid (that file documents both), writes the reconstruction back over
-//      the row, and the block copies the rows out coalesced.
+//   2. the quantizer of group_quant.cuh: one thread per 64-group works on its row in place, and each warp sends its 32 rows
+//      out by TMA.
 // A tile is 128 consecutive groups (the quantizer's unit), whatever the row length: the LayerNorm phase computes
 // every row the tile touches (a row shared with the neighbouring tile is normalised by both; 1 row in 22 at
 // K = 384) and keeps the groups that are the tile's.  Rows are owned (s and h written) by the tile that holds
 // their first group.
 #pragma once
+#include <cuda.h>
 #include <cuda_fp16.h>
 #include "ptx.cuh"
 #include "act_quant.cuh"
-#include "act_quant_v2.cuh"
+#include "group_quant.cuh"
 #include "add_layernorm.cuh"
 
 namespace arcq {
 
 constexpr int kLnqThreads = 128;
-constexpr int kLnqPitch = 144;      // bytes between staged group rows (128 data bytes, conflict-free pitch)
 
 __host__ __device__ constexpr size_t lnq_smem_bytes() {
-  return kLnqThreads * kLnqPitch                // h, then reconstruction rows
-         + 16 * kLnqThreads * 4                 // per-thread limit columns
-         + 4 * 16 * 4 + kAq2Cells * 4 + 16;     // thresholds, half-gaps, codebook, grid positions, first guesses
+  return 1024 /* alignment */ + kLnqThreads * 128 /* h, then reconstruction: one group per row, 128-byte swizzle */ +
+         sizeof(GroupQuantTables);
 }
 
 template <int LANES, int BITS, bool HAS_Y>
 __global__ void __launch_bounds__(kLnqThreads, 4)
-    add_layernorm_act_quant_kernel(const __half* __restrict__ x, const __half* __restrict__ y,
-                                   const float* __restrict__ gamma, const float* __restrict__ beta, float eps,
-                                   long long M, const float* __restrict__ thresholds,
-                                   const float* __restrict__ codebook, __half* __restrict__ sum_out,
-                                   __half* __restrict__ h_out, __half* __restrict__ xhat) {
+    add_layernorm_act_quant_kernel(const __grid_constant__ CUtensorMap tm_out, const __half* __restrict__ x,
+                                   const __half* __restrict__ y, const float* __restrict__ gamma,
+                                   const float* __restrict__ beta, float eps, long long M,
+                                   const float* __restrict__ thresholds, const float* __restrict__ codebook,
+                                   __half* __restrict__ sum_out, __half* __restrict__ h_out) {
   pdl_launch_dependents();   // the next kernel of the stream may start its set-up
 
   constexpr int L = 1 << BITS;
   constexpr int K = LANES * 24, G = K / 64, kRowsPerWarp = 32 / LANES, kRowsPerPass = 4 * kRowsPerWarp;
   constexpr int kMaxRows = kLnqThreads / G + 2;                       // rows a tile of 128 groups can touch
   constexpr int kPasses = (kMaxRows + kRowsPerPass - 1) / kRowsPerPass;
-  constexpr int kTableStride = kLnqThreads;
-  extern __shared__ __align__(16) uint8_t lnq_smem[];
-  uint8_t* const s_rows = lnq_smem;                                                   // [128] group rows
-  float* const s_table = reinterpret_cast<float*>(s_rows + kLnqThreads * kLnqPitch);  // [16][128]
-  float* const s_th = s_table + 16 * kTableStride;                                    // [16]
-  float* const s_h = s_th + 16;
-  float* const s_cb = s_h + 16;
-  float* const s_pos = s_cb + 16;
-  int* const s_guess = reinterpret_cast<int*>(s_pos + 16);                            // [kAq2Cells]
+  extern __shared__ uint8_t lnq_smem_raw[];
+  uint8_t* const s_rows = lnq_smem_raw + ((1024u - (smem_u32(lnq_smem_raw) & 1023u)) & 1023u);
+  GroupQuantTables* const tables = reinterpret_cast<GroupQuantTables*>(s_rows + kLnqThreads * 128);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, l = lane % LANES, sub = lane / LANES;
-
-  // ---- per-block set-up (reads only this layer's constants, so it runs before the wait below)
-  int my_exact = 1;
-  if (tid < 16) {
-    float th = __int_as_float(0x7f800000), h = 0.0f;
-    if (tid < L - 1) {
-      th = thresholds[tid];
-      if (th == 0.0f) {
-        h = 0x1p-100f;
-      } else {
-        const int b = __float_as_int(th);
-        const float up = __int_as_float(th > 0.0f ? b + 1 : b - 1);
-        h = __fmul_rn(__fsub_rn(up, th), 0.5f);
-      }
-      my_exact = (th == 0.0f || fabsf(th) > 1.0e-15f) ? 1 : 0;
-    }
-    s_th[tid] = th;
-    s_h[tid] = h;
-    s_cb[tid] = tid < L ? codebook[tid] : 0.0f;
-  }
-  const bool exact_r = __syncthreads_and(my_exact) != 0;
-  float grid_scale = 0.0f, grid_off = 0.0f;
-  bool use_guess = false;
-  if (L >= 4) {
-    const float th_first = s_th[0], th_last = s_th[L - 2];
-    grid_scale = static_cast<float>(kAq2Cells - 2) / (th_last - th_first);
-    grid_off = 1.0f - th_first * grid_scale;
-    int gap_ok = 1;
-    if (tid < 16) {
-      const float pos = tid < L - 1 ? fmaf(s_th[tid], grid_scale, grid_off) : __int_as_float(0x7f800000);
-      s_pos[tid] = pos;
-      if (tid < L - 2) gap_ok = (fmaf(s_th[tid + 1], grid_scale, grid_off) - pos > 1.1f) ? 1 : 0;
-    }
-    use_guess = __syncthreads_and(gap_ok) != 0 && exact_r && isfinite(grid_scale);
-    for (int k = tid; k < kAq2Cells; k += kLnqThreads) {
-      const float lim = static_cast<float>(k) - 0.05f;
-      int c = (s_pos[7] < lim) ? 8 : 0;
-      c += (s_pos[c + 3] < lim) ? 4 : 0;
-      c += (s_pos[c + 1] < lim) ? 2 : 0;
-      c += (s_pos[c] < lim) ? 1 : 0;
-      s_guess[k] = c * (kLnqThreads * 4);
-    }
-  }
-  float* const my_table = s_table + tid;
-  const char* const col = reinterpret_cast<const char*>(my_table);
-  constexpr int kStep = kTableStride * 4;
-  static_assert(kStep == 512, "the code extraction below assumes a 512-byte table step");
-  uint8_t* const my_row = s_rows + tid * kLnqPitch;
+  if (tid == 0) tma_prefetch_desc(&tm_out);
+  // reads only this layer's constants, so it runs before the wait below
+  const GroupQuantParams gp = group_quant_tables<L>(tables, thresholds, codebook, tid, kLnqThreads,
+                                                    [](bool b) { return __syncthreads_and(b) != 0; });
 
   pdl_wait();                // x and y may be the previous kernels' outputs
 
@@ -133,9 +81,9 @@ __global__ void __launch_bounds__(kLnqThreads, 4)
 #pragma unroll
           for (int i = 0; i < 3; ++i) {
             const int ch = l + LANES * i;                          // 16-byte chunk of the row: group ch / 8, part ch % 8
-            const long long lg = lg0 + (ch >> 3);
+            const int lg = static_cast<int>(lg0) + (ch >> 3);
             if (lg >= 0 && lg < ngroups)
-              *reinterpret_cast<uint4*>(s_rows + lg * kLnqPitch + (ch & 7) * 16) = h[i];
+              *reinterpret_cast<uint4*>(s_rows + lg * 128 + (((ch ^ lg) & 7) << 4)) = h[i];
             if (owned && h_out != nullptr) reinterpret_cast<uint4*>(h_out + row * K)[ch] = h[i];
           }
         }
@@ -143,90 +91,19 @@ __global__ void __launch_bounds__(kLnqThreads, 4)
     }
     __syncthreads();
 
-    // ---- phase 2: the activation quantizer on h, one thread per group (same steps as act_quant_v2_kernel)
-    const bool valid = tid < ngroups;
-    float v[64];
-    if (valid) {
-      aq2_load_row<__half>(my_row, v);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 64; ++j) v[j] = 0.0f;
-    }
-    const float mean = __fdiv_rn(sum64_ref_order(v), 64.0f);
-    float var;
-    {
-      float q[64];
-#pragma unroll
-      for (int j = 0; j < 64; ++j) {
-        v[j] = __fsub_rn(v[j], mean);
-        q[j] = __fmul_rn(v[j], v[j]);
-      }
-      var = __fdiv_rn(sum64_ref_order(q), 64.0f);
-    }
-    const float scale = __fsqrt_rn(__fadd_rn(var, 1.0e-6f));
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float t = __int_as_float(0x7f800000);
-      if (i < L - 1) {
-        const float th = s_th[i];
-        const float hs = __fmul_rd(__fmul_rn(s_h[i], scale), th == 0.0f ? 0x1p-50f : 1.0f);
-        t = exact_r ? __fmaf_rd(th, scale, hs) : th;
-      }
-      if (i < L) my_table[i * kTableStride] = t;
-    }
-    const char* const cbp = reinterpret_cast<const char*>(s_cb);
-    if (use_guess) {
-      const float inv = grid_scale * __frcp_rn(scale);
-#pragma unroll
-      for (int j = 0; j < 64; ++j) {
-        const float r = v[j];
-        const unsigned cell = min(__float2uint_rz(fmaf(r, inv, grid_off)), static_cast<unsigned>(kAq2Cells - 1));
-        int off = s_guess[cell];
-        off += (r > *reinterpret_cast<const float*>(col + off)) ? kStep : 0;
-        v[j] = *reinterpret_cast<const float*>(cbp + (off >> 7));          // code = off / 512, four bytes per entry
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 64; ++j) {
-        const float key = exact_r ? v[j] : __fdiv_rn(v[j], scale);
-        int off = 0;
-        if (BITS >= 4) off += (key > *reinterpret_cast<const float*>(col + off + 7 * kStep)) ? 8 * kStep : 0;
-        if (BITS >= 3) off += (key > *reinterpret_cast<const float*>(col + off + 3 * kStep)) ? 4 * kStep : 0;
-        off += (key > *reinterpret_cast<const float*>(col + off + 1 * kStep)) ? 2 * kStep : 0;
-        off += (key > *reinterpret_cast<const float*>(col + off)) ? kStep : 0;
-        v[j] = *reinterpret_cast<const float*>(cbp + (off >> 7));
-      }
-    }
-    const float code_sum = sum64_ref_order(v);
-    if (valid) {
-      // reconstruction mean + scale*(cb[c] - code_sum/64) in the reference's three rounded steps
-      const float vm = __fmul_rn(code_sum, 1.0f / 64.0f);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        uint32_t o[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int e = 8 * c + 2 * j;
-          o[j] = aq2_pack2<__half>(__fadd_rn(mean, __fmul_rn(scale, __fsub_rn(v[e], vm))),
-                                   __fadd_rn(mean, __fmul_rn(scale, __fsub_rn(v[e + 1], vm))));
-        }
-        *reinterpret_cast<uint4*>(my_row + 16 * c) = make_uint4(o[0], o[1], o[2], o[3]);
-      }
-    }
-    __syncthreads();
-    // ---- coalesced copy-out of the reconstruction (groups are contiguous in memory)
-    {
-      const int nchunks = ngroups * 8;
-      uint8_t* xo = reinterpret_cast<uint8_t*>(xhat) + gi0 * 128;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int q = tid + kLnqThreads * i;
-        if (q < nchunks)
-          *reinterpret_cast<uint4*>(xo + q * 16) = *reinterpret_cast<const uint4*>(s_rows + (q >> 3) * kLnqPitch + (q & 7) * 16);
-      }
+    // ---- phase 2: the activation quantizer on h, one thread per group, in place; a warp sends its 32 rows out by TMA
+    // (rows of the last tile beyond the matrix hold stale values; the store clips them)
+    if (tid < ngroups) group_quantize_row<BITS, false>(smem_u32(s_rows) + tid * 128, lane & 7, tables, gp);
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_2d(&tm_out, s_rows + warp * 4096, 0, static_cast<int>(gi0) + warp * 32);
+      tma_store_commit();
+      tma_store_wait_read();
     }
     __syncthreads();   // the rows are free for the next tile
   }
+  if (lane == 0) tma_store_wait_all();
 }
 
 // ---------------------------------------------------------------------------------------------------------
