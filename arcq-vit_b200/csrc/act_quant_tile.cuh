@@ -1,10 +1,10 @@
-// Activation quantizer for large inputs: one thread per 64-value group (group_quant.cuh), a warp per 32 groups, each warp on
-// its own: it brings its tile in by TMA (32 rows of one group, 128-byte swizzle, so that a thread reads its row without bank
+// Activation quantizer for large inputs (group_quant.cuh): each warp works on its own tiles of 32 groups (16 with two lanes a
+// group).  It brings a tile in by TMA (a row per group, 128-byte swizzle, so that lanes read their rows without bank
 // conflicts), quantises it in place and sends the reconstruction out by TMA, with the next tile's load and the previous
 // tile's store in flight meanwhile.  No block-wide synchronisation after the table set-up.
 //
-// Bound by issue slots (15 to 16 instructions per value, 23 with the GELU), then by shared-memory reads (about four
-// wavefronts per 32 values); memory is half idle.
+// Bound by issue slots, then by shared-memory reads (about four wavefronts per 32 values); memory is half idle.
+// Reconstruction only: two lanes a group, 32 warps an SM.  With codes: one lane a group, which assembles the words.
 #pragma once
 #include <cuda.h>
 #include "ptx.cuh"
@@ -12,48 +12,38 @@
 
 namespace arcq {
 
-constexpr int kAqtWarps = 4, kAqtThreads = kAqtWarps * 32;
 constexpr int kStatusActQuantTimeout = 0x401;
 
-template <typename T> struct AqtTile {          // bytes of 32 group rows, and how many of them a warp cycles through
-  static constexpr int kBytes = 32 * 64 * static_cast<int>(sizeof(T)), kBufs = sizeof(T) == 2 ? 3 : 2;
+template <typename T, bool WRITE_PACKED> struct AqtShape {
+  static constexpr int kLpg = 1;
+  static constexpr int kWarps = 4, kThreads = kWarps * 32;
+  static constexpr int kGroups = 32 / kLpg;                                   // per warp and tile
+  static constexpr int kTile = kGroups * 64 * static_cast<int>(sizeof(T));    // bytes
+  static constexpr int kBufs = sizeof(T) == 2 ? 3 : 2;                        // tiles a warp cycles through
+  static constexpr int kTables = kWarps * kBufs * kTile;                      // a multiple of 1 KB
+  static constexpr int kBars = kTables + (static_cast<int>(sizeof(GroupQuantTables)) + 15) / 16 * 16;
+  static constexpr int kSmem = 1024 /* alignment */ + kBars + kWarps * kBufs * 8;
+  static constexpr int kBlocksPerSm = sizeof(T) == 4 ? 3 : 4;
 };
-template <typename T> __host__ __device__ constexpr size_t aqt_smem_bytes() {
-  return 1024 /* alignment */ + static_cast<size_t>(kAqtWarps) * AqtTile<T>::kBytes * AqtTile<T>::kBufs +
-         sizeof(GroupQuantTables) + 16 + kAqtWarps * AqtTile<T>::kBufs * 8;
-}
-
-template <typename T> __device__ __forceinline__ f32x2 sixteen_to_pair(uint32_t w);
-template <> __device__ __forceinline__ f32x2 sixteen_to_pair<__half>(uint32_t w) { return half2_to_pair(w); }
-template <> __device__ __forceinline__ f32x2 sixteen_to_pair<__nv_bfloat16>(uint32_t w) {
-  return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
-}
-template <typename T> __device__ __forceinline__ uint32_t pair_to_sixteen(f32x2 v);
-template <> __device__ __forceinline__ uint32_t pair_to_sixteen<__half>(f32x2 v) { return pair_to_half2(v); }
-template <> __device__ __forceinline__ uint32_t pair_to_sixteen<__nv_bfloat16>(f32x2 v) {
-  float a, b;
-  unpack2(v, a, b);
-  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
 
 // XH: element type of the reconstruction: T, or fp16 for an fp32 input.  PRE = 1: GELU first (fp16 input).
 template <typename T, int BITS, typename XH, bool WRITE_XHAT, int PRE, bool WRITE_PACKED>
-__global__ void __launch_bounds__(kAqtThreads, 4)
+__global__ void __launch_bounds__(AqtShape<T, WRITE_PACKED>::kThreads, AqtShape<T, WRITE_PACKED>::kBlocksPerSm)
     act_quant_tile_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_out,
                           long long total_groups, const float* __restrict__ thresholds, const float* __restrict__ codebook,
                           uint8_t* __restrict__ packed, float* __restrict__ mu_out, float* __restrict__ sigma_out,
                           float* __restrict__ codesum_out, int* status) {
   pdl_launch_dependents();   // the next kernel of the stream may start its set-up
-  constexpr int kTile = AqtTile<T>::kBytes, kBufs = AqtTile<T>::kBufs, L = 1 << BITS;
+  using S = AqtShape<T, WRITE_PACKED>;
+  constexpr int L = 1 << BITS, LPG = S::kLpg, PJ = 4 / LPG, kTile = S::kTile, kBufs = S::kBufs, kGroups = S::kGroups;
   static_assert(PRE == 0 || sizeof(T) == 2, "the GELU takes fp16");
   extern __shared__ uint8_t aqt_smem_raw[];
   uint8_t* const smem = aqt_smem_raw + ((1024u - (smem_u32(aqt_smem_raw) & 1023u)) & 1023u);
-  GroupQuantTables* const tables = reinterpret_cast<GroupQuantTables*>(smem + kAqtWarps * kBufs * kTile);
-  uint64_t* const bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(tables) + (sizeof(GroupQuantTables) + 15) / 16 * 16);
+  GroupQuantTables* const tables = reinterpret_cast<GroupQuantTables*>(smem + S::kTables);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int gl = lane / LPG, h = LPG == 2 ? lane & 1 : 0;            // group of the tile, lane of the group
   uint8_t* const bufs = smem + warp * kBufs * kTile;
-  uint64_t* const full = bars + warp * kBufs;
+  uint64_t* const full = reinterpret_cast<uint64_t*>(smem + S::kBars) + warp * kBufs;
   if (lane == 0) {
     for (int i = 0; i < kBufs; ++i) mbar_init(&full[i], 1);
     mbar_fence_init();
@@ -61,14 +51,15 @@ __global__ void __launch_bounds__(kAqtThreads, 4)
     if (WRITE_XHAT) tma_prefetch_desc(&tm_out);
   }
   // reads only the layer's constants, which no kernel of this library writes: done while the previous kernel still runs
-  const GroupQuantParams gp = group_quant_tables<L>(tables, thresholds, codebook, tid, kAqtThreads,
+  const GroupQuantParams gp = group_quant_tables<L>(tables, thresholds, codebook, tid, S::kThreads,
                                                     [](bool b) { return __syncthreads_and(b) != 0; });
-  const long long tiles = (total_groups + 31) >> 5;
-  const long long stride = static_cast<long long>(gridDim.x) * kAqtWarps;
-  long long tile = static_cast<long long>(blockIdx.x) * kAqtWarps + warp;
+  const long long tiles = (total_groups + kGroups - 1) / kGroups;
+  const long long stride = static_cast<long long>(gridDim.x) * S::kWarps;
+  long long tile = static_cast<long long>(blockIdx.x) * S::kWarps + warp;
+  constexpr int kRowsPerGroup = sizeof(T) == 2 ? 1 : 2;              // 128-byte rows
   auto load = [&](long long t, int b) {
     mbar_arrive_expect_tx(&full[b], kTile);
-    tma_load_2d(bufs + b * kTile, &tm_x, &full[b], 0, static_cast<int>(sizeof(T) == 2 ? t * 32 : t * 64));
+    tma_load_2d(bufs + b * kTile, &tm_x, &full[b], 0, static_cast<int>(t * (kGroups * kRowsPerGroup)));
   };
   pdl_wait();
   if (lane == 0 && tile < tiles) load(tile, 0);
@@ -84,35 +75,29 @@ __global__ void __launch_bounds__(kAqtThreads, 4)
       if (lane == 0) atomicExch(status, kStatusActQuantTimeout);
       break;
     }
-    const uint32_t row = smem_u32(bufs + buf * kTile);
-    f32x2 v[32];
+    const uint32_t base = smem_u32(bufs + buf * kTile);
+    const uint32_t row = base + gl * 128 + 8 * h, x7 = gl & 7;       // 16-bit rows: this lane's part
+    // fp32 rows: value chunk c (four values) of the group sits in row 2 gl + c / 8
+    auto chunk32 = [&](int c) { return base + (2 * gl + (c >> 3)) * 128 + (((c & 7) ^ ((2 * gl + (c >> 3)) & 7)) << 4); };
+    f32x2 v[32 / LPG];
     if constexpr (sizeof(T) == 2) {
-      const uint32_t r = row + lane * 128, x7 = lane & 7;
-      uint4 ch[8];
+      uint32_t w[32 / LPG];
+      row_load<LPG>(w, row, x7);
+      if (PRE == 1) gelu_words<LPG>(w, row, x7);
 #pragma unroll
-      for (int c = 0; c < 8; ++c) ch[c] = lds128(r + ((c ^ x7) << 4));
-      if (PRE == 1) gelu_row(ch, r, x7);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        v[4 * c] = sixteen_to_pair<T>(ch[c].x);
-        v[4 * c + 1] = sixteen_to_pair<T>(ch[c].y);
-        v[4 * c + 2] = sixteen_to_pair<T>(ch[c].z);
-        v[4 * c + 3] = sixteen_to_pair<T>(ch[c].w);
-      }
+      for (int i = 0; i < 32 / LPG; ++i) v[i] = sixteen_to_pair<T>(w[i]);
     } else {
-      // a group is two 128-byte rows of the tile
 #pragma unroll
-      for (int c = 0; c < 16; ++c) {
-        const uint32_t rr = 2 * lane + (c >> 3);
-        const uint4 u = lds128(row + rr * 128 + (((c & 7) ^ (rr & 7)) << 4));
+      for (int c = 0; c < 16 / LPG; ++c) {
+        const uint4 u = lds128(chunk32(LPG * c + h));
         v[2 * c] = pack2(__uint_as_float(u.x), __uint_as_float(u.y));
         v[2 * c + 1] = pack2(__uint_as_float(u.z), __uint_as_float(u.w));
       }
     }
     uint32_t words[8];
-    const GroupStats st = group_quantize<BITS, WRITE_PACKED>(v, tables, gp, words);
-    const long long gi = tile * 32 + lane;
-    if (gi < total_groups) {
+    const GroupStats st = group_quantize<BITS, WRITE_PACKED, LPG>(v, tables, gp, words);
+    const long long gi = tile * kGroups + gl;
+    if (gi < total_groups && h == 0) {
       if (WRITE_PACKED) {
         if (BITS == 4) {
           uint4* o = reinterpret_cast<uint4*>(packed + gi * 32);
@@ -148,28 +133,24 @@ __global__ void __launch_bounds__(kAqtThreads, 4)
     if (WRITE_XHAT) {
       const GroupRecon g = group_recon(st, gp);
       if constexpr (sizeof(XH) == 2) {
-        if (sizeof(T) == 4) __syncwarp();                    // the fp16 rows overlap other threads' fp32 rows
-        const uint32_t r = row + lane * 128, x7 = lane & 7;
+        if (sizeof(T) == 4) __syncwarp();                    // the fp16 rows overlap other lanes' fp32 rows
+        uint32_t w[32 / LPG];
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
-          sts128(r + ((c ^ x7) << 4), pair_to_sixteen<XH>(group_recon_pair(g, v[4 * c])),
-                 pair_to_sixteen<XH>(group_recon_pair(g, v[4 * c + 1])), pair_to_sixteen<XH>(group_recon_pair(g, v[4 * c + 2])),
-                 pair_to_sixteen<XH>(group_recon_pair(g, v[4 * c + 3])));
+        for (int i = 0; i < 32 / LPG; ++i) w[i] = pair_to_sixteen<XH>(group_recon_pair(g, v[i]));
+        row_store<LPG>(w, row, x7);
       } else {
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          const uint32_t rr = 2 * lane + (c >> 3);
+        for (int c = 0; c < 16 / LPG; ++c) {
           float f0, f1, f2, f3;
           unpack2(group_recon_pair(g, v[2 * c]), f0, f1);
           unpack2(group_recon_pair(g, v[2 * c + 1]), f2, f3);
-          sts128(row + rr * 128 + (((c & 7) ^ (rr & 7)) << 4), __float_as_uint(f0), __float_as_uint(f1), __float_as_uint(f2),
-                 __float_as_uint(f3));
+          sts128(chunk32(LPG * c + h), __float_as_uint(f0), __float_as_uint(f1), __float_as_uint(f2), __float_as_uint(f3));
         }
       }
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
-        tma_store_2d(&tm_out, bufs + buf * kTile, 0, static_cast<int>(sizeof(XH) == 2 ? tile * 32 : tile * 64));
+        tma_store_2d(&tm_out, bufs + buf * kTile, 0, static_cast<int>(tile * (kGroups * (sizeof(XH) == 2 ? 1 : 2))));
         tma_store_commit();
       }
     } else {

@@ -213,7 +213,8 @@ template <typename T, int BITS, int PRE, typename XH, bool WX, bool WP>
 cudaError_t launch_act_quant_tile(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed,
                                   float* mu, float* sg, float* cs, void* xhat, cudaStream_t st) {
   auto k = arcq::act_quant_tile_kernel<T, BITS, XH, WX, PRE, WP>;
-  constexpr int smem = static_cast<int>(arcq::aqt_smem_bytes<T>());
+  using Shape = arcq::AqtShape<T, WP>;
+  constexpr int smem = Shape::kSmem;
   static thread_local int done_dev = -1;      // shared-memory ceiling raised once per (host thread, device)
   int dev = 0;
   cudaGetDevice(&dev);
@@ -225,7 +226,8 @@ cudaError_t launch_act_quant_tile(const void* x, long long groups, const float* 
   // a group is one row of 64 16-bit values, or two rows of 32 fp32 values
   auto map = [&](CUtensorMap* tm, const void* p, int bytes, CUtensorMapDataType dt) {
     const int rows_per = bytes == 4 ? 2 : 1;
-    return make_tensor_map_2d(tm, p, dt, bytes, static_cast<uint64_t>(groups) * rows_per, 64 / rows_per, 64 / rows_per, 32 * rows_per,
+    return make_tensor_map_2d(tm, p, dt, bytes, static_cast<uint64_t>(groups) * rows_per, 64 / rows_per, 64 / rows_per,
+                              Shape::kGroups * rows_per,
                               CU_TENSOR_MAP_SWIZZLE_128B);
   };
   auto type_of = [](auto v) {
@@ -240,9 +242,10 @@ cudaError_t launch_act_quant_tile(const void* x, long long groups, const float* 
   } else {
     tm_out = tm_x;
   }
-  const long long blocks = (groups + arcq::kAqtThreads - 1) / arcq::kAqtThreads;
-  const long long cap = static_cast<long long>(sm_count()) * (sizeof(T) == 2 ? 4 : 3);
-  launch_pdl(k, static_cast<unsigned>(blocks < cap ? blocks : cap), arcq::kAqtThreads, smem, st, tm_x, tm_out, groups, th, cb,
+  constexpr int per_block = Shape::kWarps * Shape::kGroups;
+  const long long blocks = (groups + per_block - 1) / per_block;
+  const long long cap = static_cast<long long>(sm_count()) * Shape::kBlocksPerSm;
+  launch_pdl(k, static_cast<unsigned>(blocks < cap ? blocks : cap), Shape::kThreads, smem, st, tm_x, tm_out, groups, th, cb,
              packed, mu, sg, cs, status_ptr());
   return cudaGetLastError();
 }
@@ -271,7 +274,7 @@ cudaError_t dispatch_act_quant_bits(int bits, const void* x, int x_dtype, long l
                                     int xhat_dtype, cudaStream_t st) {
   // The one-thread-per-group kernel needs enough groups to fill the machine (148 SMs x 4 blocks x 128
   // threads); below that the 8-lanes-per-group kernel has 8 times the parallelism and lower latency.
-  const long long min_groups = opt(O_AQ2_MIN_GROUPS) > 0 ? opt(O_AQ2_MIN_GROUPS) : static_cast<long long>(sm_count()) * 4 * arcq::kAqtThreads / 2;
+  const long long min_groups = opt(O_AQ2_MIN_GROUPS) > 0 ? opt(O_AQ2_MIN_GROUPS) : static_cast<long long>(sm_count()) * 256;
   const bool xhat_f16 = xhat != nullptr && xhat_dtype == ARCQ_DT_F16;
   const bool tile = groups >= min_groups && groups < (1ll << 30) && opt(O_ACT_QUANT_V1) == 0 && aligned(x, 16) &&
                     (packed == nullptr || aligned(packed, 16)) &&

@@ -1,10 +1,13 @@
-// The ARCQ quantizer of one 64-value group, held by one thread: statistics, codes and reconstruction.  Shared by every
-// kernel that quantises activations a group per thread (act_quant_tile.cuh, ln_act_quant.cuh, attention.cuh,
-// gemm_pair_dense.cuh).
+// The ARCQ quantizer of one 64-value group, held by LPG = 1 or 2 lanes: statistics, codes and reconstruction.  Shared by
+// the kernels that quantise activations out of shared memory (act_quant_tile.cuh, ln_act_quant.cuh).
+//
+// Two lanes a group (lane h holds the reference's summation lanes l = 4h .. 4h+3, half of every 16-byte chunk) need 64
+// registers instead of 128 and half the straight-line code: 32 warps an SM instead of 16, and fewer instruction-cache
+// misses.  LASTLINE
 //
 // What bounds it is issue slots: nothing here waits for memory once the row is in shared memory.  So the arithmetic is
 // two values per instruction (add / mul / fma.f32x2; each half rounds like the scalar instruction, so the bits are those of
-// scalar code), and a code costs three table reads and one compare:
+// scalar code), and a code costs three table values and one compare:
 //
 //   * Bounded argument.  sum r^2 = 64 var, so |r| / s <= 8 for every element of a group: a grid over [-16, 16) needs no
 //     clamp.  One fma, rounded down, turns r into 1.5 * 2^21 + cell with two fraction bits below the cell, i.e. the low
@@ -68,12 +71,12 @@ __device__ __forceinline__ float min3_abs(float m, float a, float b) {
 
 // ---------------------------------------------------------------- per-layer tables in shared memory
 constexpr int kGqCells = 256;
-struct GroupQuantTables {            // 4 KB + 132 bytes
+struct GroupQuantTables {            // 4 KB + 132 bytes; placed on a 1 KB boundary, so that cell offset and base merge in one OR
   float cell_nth[kGqCells];          // minus the threshold that a value of the cell can be above or below
   float cell_lo[kGqCells];           // the level below that threshold ...
   float cell_hi[kGqCells];           // ... and above
-  float th[16], cb[16];              // +inf padded thresholds, levels
   uint32_t cell_code4[kGqCells];     // 4 * (code below the threshold), for kernels that also write codes
+  float th[16], cb[16];              // +inf padded thresholds, levels
   float nz;                          // -0
 };
 struct GroupQuantParams {            // the same in every thread of the block
@@ -116,7 +119,7 @@ __device__ __forceinline__ GroupQuantParams group_quant_tables(GroupQuantTables*
 #pragma unroll
     for (int i = 0; i < L - 1; ++i) c += (t->th[i] * p.cells_per_unit < lim) ? 1 : 0;
     if (k == kGqCells - 1) c = 0;                            // no quotient of a group gets here but NaN: code 0
-    t->cell_nth[k] = -t->th[c];                              // c == L - 1: -inf, nothing is above it
+    t->cell_nth[k] = -t->th[c];                               // c == L - 1: -inf, nothing is above it
     t->cell_lo[k] = t->cb[c];
     t->cell_hi[k] = t->cb[c + 1 < L ? c + 1 : L - 1];
     t->cell_code4[k] = 4u * static_cast<uint32_t>(c);
@@ -139,18 +142,29 @@ __device__ __forceinline__ int group_quant_exact_code(const GroupQuantTables* t,
 }
 
 // ---------------------------------------------------------------- the group
-// Values as pairs: v[4 * c + j] holds elements 8c + 2j and 8c + 2j + 1.  The reference adds (torch's CPU order)
+// The pairs of values of a lane: v[c * PJ + j], PJ = 4 / LPG, holds elements 8c + 4h + 2j and the next (h = 0 with one lane).
+// The reference adds (torch's CPU order)
 //   v[l] = ((x[l]+x[32+l]) + (x[8+l]+x[40+l])) + (x[16+l]+x[48+l])) + (x[24+l]+x[56+l]),  l = 0..7
 //   sum  = ((((((v0+v1)+v2)+v3)+v4)+v5)+v6)+v7
-__device__ __forceinline__ float sum64_pairs(const f32x2 (&v)[32]) {
-  float s = 0.0f;
+// The first line is local to a lane; with two lanes the chain crosses to the partner once and its end comes back.
+template <int LPG>
+__device__ __forceinline__ float sum64_pairs(const f32x2 (&v)[32 / LPG]) {
+  constexpr int PJ = 4 / LPG;
+  float p[8 / LPG];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const f32x2 a = add2(add2(add2(add2(v[j], v[16 + j]), add2(v[4 + j], v[20 + j])), add2(v[8 + j], v[24 + j])),
-                         add2(v[12 + j], v[28 + j]));
-    float e, o;
-    unpack2(a, e, o);
-    s = j == 0 ? __fadd_rn(e, o) : __fadd_rn(__fadd_rn(s, e), o);
+  for (int j = 0; j < PJ; ++j)
+    unpack2(add2(add2(add2(add2(v[j], v[4 * PJ + j]), add2(v[PJ + j], v[5 * PJ + j])), add2(v[2 * PJ + j], v[6 * PJ + j])),
+                 add2(v[3 * PJ + j], v[7 * PJ + j])),
+            p[2 * j], p[2 * j + 1]);
+  float s = p[0];
+#pragma unroll
+  for (int l = 1; l < 8 / LPG; ++l) s = __fadd_rn(s, p[l]);
+  if (LPG == 2) {
+    const int lane = threadIdx.x & 31;
+    float t = __shfl_sync(0xffffffffu, s, lane & ~1);              // the h = 0 lane's four
+#pragma unroll
+    for (int l = 0; l < 4; ++l) t = __fadd_rn(t, p[l]);            // meaningful in the h = 1 lane
+    s = __shfl_sync(0xffffffffu, t, lane | 1);
   }
   return s;
 }
@@ -159,81 +173,78 @@ struct GroupStats {
   float mean, scale, code_sum;
 };
 
-// In: v = the group's values.  Out: v = the levels of their codes, statistics; words[c] = the codes of elements
-// 8c .. 8c+7, one per nibble (CODES only).
-template <int BITS, bool CODES>
-__device__ __forceinline__ GroupStats group_quantize(f32x2 (&v)[32], const GroupQuantTables* t, const GroupQuantParams& p,
-                                                     uint32_t (&words)[8]) {
-  constexpr int L = 1 << BITS;
+// In: v = the lane's values.  Out: v = the levels of their codes, statistics; words[c] = the codes of elements
+// 8c .. 8c+7, one per nibble (CODES, one lane a group).
+template <int BITS, bool CODES, int LPG>
+__device__ __forceinline__ GroupStats group_quantize(f32x2 (&v)[32 / LPG], const GroupQuantTables* t,
+                                                     const GroupQuantParams& p, uint32_t (&words)[8]) {
+  static_assert(!CODES || LPG == 1, "codes are assembled by one lane");
+  constexpr int L = 1 << BITS, PJ = 4 / LPG, CH = 2 * PJ;          // pairs and values of a chunk
   GroupStats st;
-  st.mean = __fmul_rn(sum64_pairs(v), 0.015625f);           // / 64: exact
+  st.mean = __fmul_rn(sum64_pairs<LPG>(v), 0.015625f);           // / 64: exact
   {
     const f32x2 nm = pack2(-st.mean, -st.mean);
-    f32x2 q[32];
+    f32x2 q[32 / LPG];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
+    for (int i = 0; i < 32 / LPG; ++i) {
       v[i] = add2(v[i], nm);
       q[i] = mul2_rn(v[i], v[i], p.nz);
     }
-    st.scale = __fsqrt_rn(__fadd_rn(__fmul_rn(sum64_pairs(q), 0.015625f), 1.0e-6f));
+    st.scale = __fsqrt_rn(__fadd_rn(__fmul_rn(sum64_pairs<LPG>(q), 0.015625f), 1.0e-6f));
   }
   const float s = st.scale;
   const float a = __fdividef(p.cells_per_unit, s);           // an approximate quotient is enough for the cell
   const f32x2 a2 = pack2(a, a), s2 = pack2(s, s), magic = pack2(3145728.0f + 128.0f, 3145728.0f + 128.0f);
   const float tie = __fmul_rn(p.tie, s);
   const uint32_t tab = smem_u32(t);
-  constexpr uint32_t kLo = kGqCells * 4, kHi = 2 * kGqCells * 4, kCb = 3 * kGqCells * 4 + 64, kCode = 3 * kGqCells * 4 + 128;
+  constexpr uint32_t kLo = kGqCells * 4, kHi = 2 * kGqCells * 4, kCode = 3 * kGqCells * 4, kCb = 4 * kGqCells * 4 + 64;
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
-    float m = 1.0e38f, out[8];
+    float m = 1.0e38f, out[CH];
     uint32_t w = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < PJ; ++j) {
       float u0, u1, d0, d1;
-      unpack2(fma2_down(v[4 * c + j], a2, magic), u0, u1);
-      const uint32_t k0 = tab + (__float_as_uint(u0) & 0x3FCu), k1 = tab + (__float_as_uint(u1) & 0x3FCu);
-      unpack2(fma2(pack2(lds_f32(k0), lds_f32(k1)), s2, v[4 * c + j]), d0, d1);
+      unpack2(fma2_down(v[c * PJ + j], a2, magic), u0, u1);
+      const uint32_t o0 = (__float_as_uint(u0) & 0x3FCu) | tab, o1 = (__float_as_uint(u1) & 0x3FCu) | tab;
+      unpack2(fma2(pack2(lds_const_f32(o0), lds_const_f32(o1)), s2, v[c * PJ + j]), d0, d1);
       m = min3_abs(m, d0, d1);
       if (CODES) {
-        uint32_t o0 = lds32(k0 + kCode), o1 = lds32(k1 + kCode);
-        o0 += d0 > 0.0f ? 4u : 0u;
-        o1 += d1 > 0.0f ? 4u : 0u;
-        out[2 * j] = lds_f32(tab + kCb + o0);
-        out[2 * j + 1] = lds_f32(tab + kCb + o1);
-        w |= (o0 | (o1 << 4)) << (8 * j);                    // four times the codes; shifted down once per word below
-        if (j == 3) words[c] = (w >> 2) | ((o1 >> 4) << 30);
+        uint32_t c0 = lds_const_u32(o0 + kCode), c1 = lds_const_u32(o1 + kCode);
+        c0 += d0 > 0.0f ? 4u : 0u;
+        c1 += d1 > 0.0f ? 4u : 0u;
+        out[2 * j] = lds_const_f32(tab + kCb + c0);
+        out[2 * j + 1] = lds_const_f32(tab + kCb + c1);
+        w |= (c0 | (c1 << 4)) << (8 * j);                    // four times the codes; shifted down once per word below
+        if (j == PJ - 1) words[c] = (w >> 2) | ((c1 >> 4) << 30);
       } else {
-        const float l0 = lds_f32(k0 + kLo), h0 = lds_f32(k0 + kHi);
-        const float l1 = lds_f32(k1 + kLo), h1 = lds_f32(k1 + kHi);
+        const float l0 = lds_const_f32(o0 + kLo), h0 = lds_const_f32(o0 + kHi);
+        const float l1 = lds_const_f32(o1 + kLo), h1 = lds_const_f32(o1 + kHi);
         out[2 * j] = d0 > 0.0f ? h0 : l0;
         out[2 * j + 1] = d1 > 0.0f ? h1 : l1;
       }
     }
-    if (m <= tie) {
-      // rare: some value of the chunk is too close to a threshold for the sign of d alone
-      float r[8];
+    if (__builtin_expect(m <= tie, 0)) {
+      // rare: some value of the chunk is too close to a threshold for the sign of d alone (through local memory, so that the
+      // common path keeps its registers where they are)
+      float r[CH];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) unpack2(v[4 * c + j], r[2 * j], r[2 * j + 1]);
+      for (int j = 0; j < PJ; ++j) unpack2(v[c * PJ + j], r[2 * j], r[2 * j + 1]);
       uint32_t we = 0;
 #pragma unroll 1
-      for (int j = 0; j < 8; ++j) {
-        const int code = group_quant_exact_code<L>(t, r[0], s);
-        const float lv = t->cb[code];
-        we = (we >> 4) | (static_cast<uint32_t>(code) << 28);
-        // rotate: registers cannot be indexed by a loop counter
-#pragma unroll
-        for (int i = 0; i < 7; ++i) {
-          r[i] = r[i + 1];
-          out[i] = out[i + 1];
-        }
-        out[7] = lv;
+      for (int j = 0; j < CH; ++j) {
+        const int code = group_quant_exact_code<L>(t, r[j], s);
+        r[j] = t->cb[code];
+        we |= static_cast<uint32_t>(code) << (4 * j);
       }
+#pragma unroll
+      for (int j = 0; j < CH; ++j) out[j] = r[j];
       if (CODES) words[c] = we;
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) v[4 * c + j] = pack2(out[2 * j], out[2 * j + 1]);
+    for (int j = 0; j < PJ; ++j) v[c * PJ + j] = pack2(out[2 * j], out[2 * j + 1]);
   }
-  st.code_sum = sum64_pairs(v);
+  st.code_sum = sum64_pairs<LPG>(v);
   return st;
 }
 
@@ -249,26 +260,65 @@ __device__ __forceinline__ f32x2 group_recon_pair(const GroupRecon& g, f32x2 lev
   return add2(g.mean, mul2_rn(g.scale, add2(level, g.nvm), g.nz));
 }
 
-__device__ __forceinline__ f32x2 half2_to_pair(uint32_t h) {
-  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+// ---------------------------------------------------------------- 16-bit element types and rows in shared memory
+template <typename T> __device__ __forceinline__ f32x2 sixteen_to_pair(uint32_t w);
+template <> __device__ __forceinline__ f32x2 sixteen_to_pair<__half>(uint32_t w) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
   return pack2(f.x, f.y);
 }
-__device__ __forceinline__ uint32_t pair_to_half2(f32x2 v) {
+template <> __device__ __forceinline__ f32x2 sixteen_to_pair<__nv_bfloat16>(uint32_t w) {
+  return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+}
+template <typename T> __device__ __forceinline__ uint32_t pair_to_sixteen(f32x2 v);
+template <> __device__ __forceinline__ uint32_t pair_to_sixteen<__half>(f32x2 v) {
   float a, b;
   unpack2(v, a, b);
   const __half2 h = __floats2half2_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&h);
+}
+template <> __device__ __forceinline__ uint32_t pair_to_sixteen<__nv_bfloat16>(f32x2 v) {
+  float a, b;
+  unpack2(v, a, b);
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// The lane's part of a group's 128-byte row, 16-byte chunk c at ((c ^ x7) << 4): w[c * PJ + j] = the 32-bit word of pair j.
+// With two lanes `row` already includes 8 * h.
+template <int LPG>
+__device__ __forceinline__ void row_load(uint32_t (&w)[32 / LPG], uint32_t row, uint32_t x7) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const uint32_t a = row + ((static_cast<uint32_t>(c) ^ x7) << 4);
+    if constexpr (LPG == 1) {
+      const uint4 u = lds128(a);
+      w[4 * c] = u.x; w[4 * c + 1] = u.y; w[4 * c + 2] = u.z; w[4 * c + 3] = u.w;
+    } else {
+      const uint2 u = lds64(a);
+      w[2 * c] = u.x; w[2 * c + 1] = u.y;
+    }
+  }
+}
+template <int LPG>
+__device__ __forceinline__ void row_store(const uint32_t (&w)[32 / LPG], uint32_t row, uint32_t x7) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const uint32_t a = row + ((static_cast<uint32_t>(c) ^ x7) << 4);
+    if constexpr (LPG == 1) sts128(a, w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+    else sts64(a, w[2 * c], w[2 * c + 1]);
+  }
 }
 
 // ---------------------------------------------------------------- GELU of a group's fp16 values
 // g = x * (0.5 + x * R(x^2)) for |x| < 1.3125, with x * R(x^2) = erf(x / sqrt 2) / 2: R of degree 5 in x^2, fitted on
 // Chebyshev nodes (2e-8 relative before rounding).  Over every fp16 input of that range the fp16 result differs from the
 // correctly rounded one for 3 inputs of 31 742 (0.5 x (1 + erff(x / sqrt 2)) in fp32: 2).  Larger arguments keep the value of
-// x, are counted in a bit mask, and go through erff one by one in a loop over the group's row in shared memory: few
-// of them sit in a group, and the loop is one copy of erff in the code instead of 64.
-// `row`: the thread's own 128-byte row, 16-byte chunk c at ((c ^ x7) << 4), used for that exchange only.  The result is
-// rounded to fp16, the value a separate GELU kernel would store; ch[c] holds chunk c before and after.
-__device__ __forceinline__ void gelu_row(uint4 (&ch)[8], uint32_t row, uint32_t x7) {
+// x, are counted in a bit mask, and go through erff one by one in a loop over the lane's part of the row in shared memory:
+// few of them sit in a group, and the loop is one copy of erff in the code instead of 64.  The row is used for that
+// exchange only.  The result is rounded to fp16, the value a separate GELU kernel would store.
+template <int LPG>
+__device__ __forceinline__ void gelu_words(uint32_t (&w)[32 / LPG], uint32_t row, uint32_t x7) {
+  constexpr int PJ = 4 / LPG;
   const f32x2 c5 = pack2(-6.607886916754069e-06f, -6.607886916754069e-06f), c4 = pack2(0.00011030046152882278f, 0.00011030046152882278f);
   const f32x2 c3 = pack2(-0.0011828974820673466f, -0.0011828974820673466f), c2 = pack2(0.009971804916858673f, 0.009971804916858673f);
   const f32x2 c1 = pack2(-0.06649012118577957f, -0.06649012118577957f), c0 = pack2(0.3989422619342804f, 0.3989422619342804f);
@@ -276,71 +326,56 @@ __device__ __forceinline__ void gelu_row(uint4 (&ch)[8], uint32_t row, uint32_t 
   const __half2 lim = __floats2half2_rn(1.3125f, 1.3125f);
   uint32_t big[2] = {0u, 0u};
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    uint32_t* const w = reinterpret_cast<uint32_t*>(&ch[c]);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const __half2 xh = *reinterpret_cast<const __half2*>(&w[q]);
-      const uint32_t m = __hgeu2_mask(__habs2(xh), lim);                  // 0xffff per half (unordered: NaN counts as large)
-      const f32x2 x = half2_to_pair(w[q]);
-      const f32x2 s = mul2(x, x);
-      f32x2 r = fma2(c5, s, c4);
-      r = fma2(r, s, c3);
-      r = fma2(r, s, c2);
-      r = fma2(r, s, c1);
-      r = fma2(r, s, c0);
-      const uint32_t g = pair_to_half2(mul2(x, fma2(x, r, half)));
-      big[c >> 2] |= m & (0x00010001u << (4 * (c & 3) + q));
-      w[q] = (m & w[q]) | (~m & g);
-    }
+  for (int i = 0; i < 32 / LPG; ++i) {
+    const __half2 xh = *reinterpret_cast<const __half2*>(&w[i]);
+    const uint32_t m = __hgeu2_mask(__habs2(xh), lim);                  // 0xffff per half (unordered: NaN counts as large)
+    const f32x2 x = sixteen_to_pair<__half>(w[i]);
+    const f32x2 s = mul2(x, x);
+    f32x2 r = fma2(c5, s, c4);
+    r = fma2(r, s, c3);
+    r = fma2(r, s, c2);
+    r = fma2(r, s, c1);
+    r = fma2(r, s, c0);
+    const uint32_t g = pair_to_sixteen<__half>(mul2(x, fma2(x, r, half)));
+    big[i >> 4] |= m & (0x00010001u << (i & 15));
+    w[i] = (m & w[i]) | (~m & g);
   }
   if ((big[0] | big[1]) != 0u) {
-#pragma unroll
-    for (int c = 0; c < 8; ++c) sts128(row + ((static_cast<uint32_t>(c) ^ x7) << 4), ch[c].x, ch[c].y, ch[c].z, ch[c].w);
+    row_store<LPG>(w, row, x7);
 #pragma unroll 1
-    for (int hw = 0; hw < 2; ++hw) {
+    for (int hw = 0; hw < 2 / LPG; ++hw) {
       uint32_t b = hw ? big[1] : big[0];
 #pragma unroll 1
       while (b != 0u) {
-        const int i = __ffs(b) - 1;
+        const int k = __ffs(b) - 1;
         b &= b - 1u;
-        const uint32_t e = 32u * hw + 2u * (i & 15) + (i >> 4);           // element of the group
-        const uint32_t a = row + (((e >> 3) ^ x7) << 4) + 2u * (e & 7u);
+        const uint32_t i = 16u * hw + (k & 15);                          // the word, in chunk i / PJ
+        const uint32_t a = row + (((i / PJ) ^ x7) << 4) + 4u * (i % PJ) + 2u * (k >> 4);
         const float x = __half2float(__ushort_as_half(static_cast<unsigned short>(lds16(a))));
         const float g = x * 0.5f * (1.0f + erff(x * 0.70710678118654752440f));
         sts16(a, __half_as_ushort(__float2half_rn(g)));
       }
     }
-#pragma unroll
-    for (int c = 0; c < 8; ++c) ch[c] = lds128(row + ((static_cast<uint32_t>(c) ^ x7) << 4));
+    row_load<LPG>(w, row, x7);
   }
 }
 
-// The quantizer on the thread's fp16 row in shared memory, in place: values in, reconstruction out.
-template <int BITS, bool GELU>
+// The quantizer on a fp16 row in shared memory, in place: values in, reconstruction out.
+template <typename T, int BITS, bool GELU, int LPG>
 __device__ __forceinline__ void group_quantize_row(uint32_t row, uint32_t x7, const GroupQuantTables* t,
-                                                   const GroupQuantParams& p) {
-  f32x2 v[32];
-  {
-    uint4 ch[8];
+                                                   const GroupQuantParams& p, GroupStats* stats = nullptr) {
+  uint32_t w[32 / LPG], words[8];
+  f32x2 v[32 / LPG];
+  row_load<LPG>(w, row, x7);
+  if (GELU) gelu_words<LPG>(w, row, x7);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) ch[c] = lds128(row + ((static_cast<uint32_t>(c) ^ x7) << 4));
-    if (GELU) gelu_row(ch, row, x7);
+  for (int i = 0; i < 32 / LPG; ++i) v[i] = sixteen_to_pair<T>(w[i]);
+  const GroupStats st = group_quantize<BITS, false, LPG>(v, t, p, words);
+  const GroupRecon g = group_recon(st, p);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      v[4 * c] = half2_to_pair(ch[c].x);
-      v[4 * c + 1] = half2_to_pair(ch[c].y);
-      v[4 * c + 2] = half2_to_pair(ch[c].z);
-      v[4 * c + 3] = half2_to_pair(ch[c].w);
-    }
-  }
-  uint32_t words[8];
-  const GroupRecon g = group_recon(group_quantize<BITS, false>(v, t, p, words), p);
-#pragma unroll
-  for (int c = 0; c < 8; ++c)
-    sts128(row + ((static_cast<uint32_t>(c) ^ x7) << 4), pair_to_half2(group_recon_pair(g, v[4 * c])),
-           pair_to_half2(group_recon_pair(g, v[4 * c + 1])), pair_to_half2(group_recon_pair(g, v[4 * c + 2])),
-           pair_to_half2(group_recon_pair(g, v[4 * c + 3])));
+  for (int i = 0; i < 32 / LPG; ++i) w[i] = pair_to_sixteen<T>(group_recon_pair(g, v[i]));
+  row_store<LPG>(w, row, x7);
+  if (stats != nullptr) *stats = st;
 }
 
 }  // namespace arcq

@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kLnqThreads, 4)
 
     // ---- phase 2: the activation quantizer on h, one thread per group, in place; a warp sends its 32 rows out by TMA
     // (rows of the last tile beyond the matrix hold stale values; the store clips them)
-    if (tid < ngroups) group_quantize_row<BITS, false>(smem_u32(s_rows) + tid * 128, lane & 7, tables, gp);
+    if (tid < ngroups) group_quantize_row<__half, BITS, false, 1>(smem_u32(s_rows) + tid * 128, lane & 7, tables, gp);
     fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) {
