@@ -10,6 +10,7 @@ from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
 LIB_PATH = PKG_DIR / "libarcq_b200.so"
+HOST_PATH = PKG_DIR / "_arcq_host.so"
 
 DT_F32, DT_F16, DT_BF16 = 0, 1, 2
 
@@ -17,6 +18,7 @@ DT_F32, DT_F16, DT_BF16 = 0, 1, 2
 EXPORTS = (
     "arcq_version", "arcq_last_error_string", "arcq_device_status", "arcq_debug_trace", "arcq_debug_set_option", "arcq_debug_get_option", "arcq_debug_last_gemm_kernel", "arcq_debug_wait_timeout", "arcq_act_quant", "arcq_gelu_act_quant", "arcq_packed_gemm", "arcq_packed_weight_gemm", "arcq_dense_weight_gemm", "arcq_packed_linear_static_scratch", "arcq_add_layernorm", "arcq_add_layernorm_act_quant", "arcq_attention", "arcq_attention_act_quant", "arcq_patchify", "arcq_assemble_tokens",
     "arcq_unpack_codes", "arcq_pack_codes", "arcq_dequant", "arcq_unpack_weight_f16", "arcq_dense_weight_gemm_prefetch",
+    "arcq_act_quant_unpack", "arcq_add_layernorm_act_quant_unpack", "arcq_add_layernorm_strided",
 )
 
 _lib = None
@@ -66,6 +68,28 @@ def load() -> ctypes.CDLL:
         getattr(lib, name)  # AttributeError here means header and library disagree
     _lib = lib
     return lib
+
+
+_host = None
+
+
+def host():
+    """The native host path (``csrc/host_ext.cpp``), loaded once: a module whose functions take torch tensors and
+    return None for what they leave to the Python code."""
+    global _host
+    if _host is None:
+        import importlib.machinery
+        import importlib.util
+        import torch  # noqa: F401  its libraries have to be loaded first
+        load()
+        if not HOST_PATH.exists():
+            raise ArcqLibraryMissing(f"{HOST_PATH} is not built. Build it with `python {PKG_DIR / 'build.py'}`.")
+        loader = importlib.machinery.ExtensionFileLoader("_arcq_host", str(HOST_PATH))
+        spec = importlib.util.spec_from_file_location("_arcq_host", str(HOST_PATH), loader=loader)
+        mod = importlib.util.module_from_spec(spec)
+        loader.exec_module(mod)
+        _host = mod
+    return _host
 
 
 def last_error() -> str:

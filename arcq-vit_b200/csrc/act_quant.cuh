@@ -14,23 +14,10 @@
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 #include "ptx.cuh"
+#include "element_types.cuh"
+#include "codes.cuh"
 
 namespace arcq {
-
-template <typename T> __device__ __forceinline__ float load_f32(const T* p);
-template <> __device__ __forceinline__ float load_f32<float>(const float* p) { return __ldg(p); }
-template <> __device__ __forceinline__ float load_f32<__half>(const __half* p) {
-  return __half2float(__ldg(p));
-}
-template <> __device__ __forceinline__ float load_f32<__nv_bfloat16>(const __nv_bfloat16* p) {
-  return __bfloat162float(__ldg(p));
-}
-template <typename T> __device__ __forceinline__ void store_from_f32(T* p, float v);
-template <> __device__ __forceinline__ void store_from_f32<float>(float* p, float v) { *p = v; }
-template <> __device__ __forceinline__ void store_from_f32<__half>(__half* p, float v) { *p = __float2half_rn(v); }
-template <> __device__ __forceinline__ void store_from_f32<__nv_bfloat16>(__nv_bfloat16* p, float v) {
-  *p = __float2bfloat16_rn(v);
-}
 
 // Optional element-wise op applied to the input before it is quantised (fused from the preceding layer).
 // PRE = 1: exact GELU, 0.5*x*(1+erf(x/sqrt 2)) in fp32, then rounded to the input's element type -- the
@@ -115,8 +102,13 @@ __global__ void __launch_bounds__(256) act_quant_kernel(const T* __restrict__ x,
                                                         const float* __restrict__ codebook,
                                                         uint8_t* __restrict__ packed, float* __restrict__ mu_out,
                                                         float* __restrict__ sigma_out,
-                                                        float* __restrict__ codesum_out, XH* __restrict__ xhat) {
+                                                        float* __restrict__ codesum_out, XH* __restrict__ xhat,
+                                                        const __grid_constant__ UnpackJobs jobs) {
   pdl_launch_dependents();   // the next kernel of the stream may start its set-up
+  if (static_cast<int>(blockIdx.x) < jobs.blocks) {
+    unpack_jobs_block(jobs);
+    return;
+  }
 
   constexpr int L = 1 << BITS;
   __shared__ float s_th[16];
@@ -132,10 +124,10 @@ __global__ void __launch_bounds__(256) act_quant_kernel(const T* __restrict__ x,
   const int lane = threadIdx.x & 31;
   const int l = lane & 7;
   const int octet_base = lane & ~7;
-  const long long warps_total = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
+  const long long warps_total = static_cast<long long>(gridDim.x - jobs.blocks) * (blockDim.x >> 5);
   const long long tasks = (total_groups + 3) >> 2;
 
-  for (long long task = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); task < tasks;
+  for (long long task = static_cast<long long>(blockIdx.x - jobs.blocks) * (blockDim.x >> 5) + (threadIdx.x >> 5); task < tasks;
        task += warps_total) {
     const long long gi = task * 4 + (lane >> 3);
     const bool valid = gi < total_groups;

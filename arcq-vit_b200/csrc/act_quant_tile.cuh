@@ -9,6 +9,7 @@
 #include <cuda.h>
 #include "ptx.cuh"
 #include "group_quant.cuh"
+#include "codes.cuh"
 
 namespace arcq {
 
@@ -32,8 +33,12 @@ __global__ void __launch_bounds__(AqtShape<T, WRITE_PACKED>::kThreads, AqtShape<
     act_quant_tile_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_out,
                           long long total_groups, const float* __restrict__ thresholds, const float* __restrict__ codebook,
                           uint8_t* __restrict__ packed, float* __restrict__ mu_out, float* __restrict__ sigma_out,
-                          float* __restrict__ codesum_out, int* status) {
+                          float* __restrict__ codesum_out, int* status, const __grid_constant__ UnpackJobs jobs) {
   pdl_launch_dependents();   // the next kernel of the stream may start its set-up
+  if (static_cast<int>(blockIdx.x) < jobs.blocks) {
+    unpack_jobs_block(jobs);
+    return;
+  }
   using S = AqtShape<T, WRITE_PACKED>;
   constexpr int L = 1 << BITS, LPG = S::kLpg, PJ = 4 / LPG, kTile = S::kTile, kBufs = S::kBufs, kGroups = S::kGroups;
   static_assert(PRE == 0 || sizeof(T) == 2, "the GELU takes fp16");
@@ -54,8 +59,8 @@ __global__ void __launch_bounds__(AqtShape<T, WRITE_PACKED>::kThreads, AqtShape<
   const GroupQuantParams gp = group_quant_tables<L>(tables, thresholds, codebook, tid, S::kThreads,
                                                     [](bool b) { return __syncthreads_and(b) != 0; });
   const long long tiles = (total_groups + kGroups - 1) / kGroups;
-  const long long stride = static_cast<long long>(gridDim.x) * S::kWarps;
-  long long tile = static_cast<long long>(blockIdx.x) * S::kWarps + warp;
+  const long long stride = static_cast<long long>(gridDim.x - jobs.blocks) * S::kWarps;
+  long long tile = static_cast<long long>(blockIdx.x - jobs.blocks) * S::kWarps + warp;
   constexpr int kRowsPerGroup = sizeof(T) == 2 ? 1 : 2;              // 128-byte rows
   auto load = [&](long long t, int b) {
     mbar_arrive_expect_tx(&full[b], kTile);

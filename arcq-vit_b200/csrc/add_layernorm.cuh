@@ -1,4 +1,4 @@
-// Residual add + LayerNorm in one pass over fp16 rows (the glue between the packed linears of a block):
+// Residual add + LayerNorm in one pass over fp16 rows, ld values apart (the glue between the packed linears of a block):
 //   s = fp16(x + y)   (written out when y is given: the updated residual stream)
 //   h = fp16((s - mean(s)) * rsqrt(var(s) + eps) * gamma + beta)
 // One warp per row, 16-byte loads/stores, statistics in fp32 with a two-pass (mean, then centred sum of
@@ -14,7 +14,8 @@ constexpr int kLnMaxChunks = 8;  // 16-byte chunks per lane: rows up to 32 * 8 *
 __global__ void __launch_bounds__(256) add_layernorm_kernel(const __half* __restrict__ x, const __half* __restrict__ y,
                                                             const float* __restrict__ gamma,
                                                             const float* __restrict__ beta, float eps, long long M, int K,
-                                                            __half* __restrict__ sum_out, __half* __restrict__ h_out) {
+                                                            long long ld, __half* __restrict__ sum_out,
+                                                            __half* __restrict__ h_out) {
   pdl_launch_dependents();   // the next kernel of the stream may start its set-up
   pdl_wait();                // the input may be the previous kernel's output
 
@@ -22,8 +23,8 @@ __global__ void __launch_bounds__(256) add_layernorm_kernel(const __half* __rest
   const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
   const int chunks = K >> 3;
   for (long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); row < M; row += warps) {
-    const uint4* xr = reinterpret_cast<const uint4*>(x + row * K);
-    const uint4* yr = (y != nullptr) ? reinterpret_cast<const uint4*>(y + row * K) : nullptr;
+    const uint4* xr = reinterpret_cast<const uint4*>(x + row * ld);
+    const uint4* yr = (y != nullptr) ? reinterpret_cast<const uint4*>(y + row * ld) : nullptr;
     float v[kLnMaxChunks][8];
     float sum = 0.0f;
 #pragma unroll
@@ -214,7 +215,8 @@ __global__ void __launch_bounds__(256) add_layernorm_rows_kernel(const __half* _
                                                                  const __half* __restrict__ y,
                                                                  const float* __restrict__ gamma,
                                                                  const float* __restrict__ beta, float eps,
-                                                                 long long M, __half* __restrict__ sum_out,
+                                                                 long long M, long long ld,
+                                                                 __half* __restrict__ sum_out,
                                                                  __half* __restrict__ h_out) {
   pdl_launch_dependents();   // the next kernel of the stream may start its set-up
 
@@ -230,7 +232,8 @@ __global__ void __launch_bounds__(256) add_layernorm_rows_kernel(const __half* _
     const bool valid = row < M;
     const long long rs = valid ? row : M - 1;          // idle sub-warps shadow the last row, store nothing
     uint4 h[3];
-    layernorm_row<LANES>(x, y, rs, row, valid, l, gg, bb, eps, sum_out, h);
+    const long long skip = rs * (ld - K);              // input rows are ld values apart
+    layernorm_row<LANES>(x + skip, y != nullptr ? y + skip : nullptr, rs, row, valid, l, gg, bb, eps, sum_out, h);
     if (valid) {
 #pragma unroll
       for (int i = 0; i < 3; ++i) reinterpret_cast<uint4*>(h_out + row * K)[l + LANES * i] = h[i];

@@ -138,17 +138,18 @@ int grid_for(long long work_items, int per_block, int blocks_per_sm) {
 
 template <typename T, int BITS, int PRE = 0>
 cudaError_t launch_act_quant(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed,
-                             float* mu, float* sg, float* cs, void* xhat, int xhat_dtype, cudaStream_t st) {
-  const int grid = grid_for((groups + 3) / 4, 8, 8);
+                             float* mu, float* sg, float* cs, void* xhat, int xhat_dtype, cudaStream_t st,
+                             const arcq::UnpackJobs& jobs) {
+  const int grid = grid_for((groups + 3) / 4, 8, 8) + jobs.blocks;
   const T* xt = static_cast<const T*>(x);
   if (xhat == nullptr) {
-    launch_pdl(arcq::act_quant_kernel<T, BITS, float, false, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<float*>(nullptr));
+    launch_pdl(arcq::act_quant_kernel<T, BITS, float, false, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<float*>(nullptr), jobs);
   } else if (xhat_dtype == ARCQ_DT_F32) {
-    launch_pdl(arcq::act_quant_kernel<T, BITS, float, true, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<float*>(xhat));
+    launch_pdl(arcq::act_quant_kernel<T, BITS, float, true, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<float*>(xhat), jobs);
   } else if (xhat_dtype == ARCQ_DT_F16) {
-    launch_pdl(arcq::act_quant_kernel<T, BITS, __half, true, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<__half*>(xhat));
+    launch_pdl(arcq::act_quant_kernel<T, BITS, __half, true, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<__half*>(xhat), jobs);
   } else {
-    launch_pdl(arcq::act_quant_kernel<T, BITS, __nv_bfloat16, true, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<__nv_bfloat16*>(xhat));
+    launch_pdl(arcq::act_quant_kernel<T, BITS, __nv_bfloat16, true, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<__nv_bfloat16*>(xhat), jobs);
   }
   return cudaGetLastError();
 }
@@ -211,7 +212,8 @@ bool make_tensor_map_2d(CUtensorMap* tm, const void* base, CUtensorMapDataType d
 // the reconstruction, if asked for, has the input's element type or is the fp16 one of an fp32 input.
 template <typename T, int BITS, int PRE, typename XH, bool WX, bool WP>
 cudaError_t launch_act_quant_tile(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed,
-                                  float* mu, float* sg, float* cs, void* xhat, cudaStream_t st) {
+                                  float* mu, float* sg, float* cs, void* xhat, cudaStream_t st,
+                             const arcq::UnpackJobs& jobs) {
   auto k = arcq::act_quant_tile_kernel<T, BITS, XH, WX, PRE, WP>;
   using Shape = arcq::AqtShape<T, WP>;
   constexpr int smem = Shape::kSmem;
@@ -245,33 +247,36 @@ cudaError_t launch_act_quant_tile(const void* x, long long groups, const float* 
   constexpr int per_block = Shape::kWarps * Shape::kGroups;
   const long long blocks = (groups + per_block - 1) / per_block;
   const long long cap = static_cast<long long>(sm_count()) * Shape::kBlocksPerSm;
-  launch_pdl(k, static_cast<unsigned>(blocks < cap ? blocks : cap), Shape::kThreads, smem, st, tm_x, tm_out, groups, th, cb,
-             packed, mu, sg, cs, status_ptr());
+  launch_pdl(k, static_cast<unsigned>((blocks < cap ? blocks : cap) + jobs.blocks), Shape::kThreads, smem, st, tm_x, tm_out, groups, th, cb,
+             packed, mu, sg, cs, status_ptr(), jobs);
   return cudaGetLastError();
 }
 
 template <typename T, int BITS, int PRE, typename XH>
 cudaError_t launch_act_quant_tile_outputs(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed,
-                                          float* mu, float* sg, float* cs, void* xhat, cudaStream_t st) {
-  if (xhat == nullptr) return launch_act_quant_tile<T, BITS, PRE, XH, false, true>(x, groups, th, cb, packed, mu, sg, cs, xhat, st);
-  if (packed == nullptr) return launch_act_quant_tile<T, BITS, PRE, XH, true, false>(x, groups, th, cb, packed, mu, sg, cs, xhat, st);
-  return launch_act_quant_tile<T, BITS, PRE, XH, true, true>(x, groups, th, cb, packed, mu, sg, cs, xhat, st);
+                                          float* mu, float* sg, float* cs, void* xhat, cudaStream_t st,
+                             const arcq::UnpackJobs& jobs) {
+  if (xhat == nullptr) return launch_act_quant_tile<T, BITS, PRE, XH, false, true>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, jobs);
+  if (packed == nullptr) return launch_act_quant_tile<T, BITS, PRE, XH, true, false>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, jobs);
+  return launch_act_quant_tile<T, BITS, PRE, XH, true, true>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, jobs);
 }
 
 template <typename T, int BITS, int PRE>
 cudaError_t dispatch_act_quant_tile(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed, float* mu,
-                                    float* sg, float* cs, void* xhat, bool xhat_f16, cudaStream_t st) {
+                                    float* sg, float* cs, void* xhat, bool xhat_f16, cudaStream_t st,
+                             const arcq::UnpackJobs& jobs) {
   if constexpr (sizeof(T) == 4) {
     if (xhat != nullptr && xhat_f16)
-      return launch_act_quant_tile_outputs<T, BITS, PRE, __half>(x, groups, th, cb, packed, mu, sg, cs, xhat, st);
+      return launch_act_quant_tile_outputs<T, BITS, PRE, __half>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, jobs);
   }
-  return launch_act_quant_tile_outputs<T, BITS, PRE, T>(x, groups, th, cb, packed, mu, sg, cs, xhat, st);
+  return launch_act_quant_tile_outputs<T, BITS, PRE, T>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, jobs);
 }
 
 template <typename T, int PRE>
 cudaError_t dispatch_act_quant_bits(int bits, const void* x, int x_dtype, long long groups, const float* th,
                                     const float* cb, uint8_t* packed, float* mu, float* sg, float* cs, void* xhat,
-                                    int xhat_dtype, cudaStream_t st) {
+                                    int xhat_dtype, cudaStream_t st,
+                             const arcq::UnpackJobs& jobs) {
   // The one-thread-per-group kernel needs enough groups to fill the machine (148 SMs x 4 blocks x 128
   // threads); below that the 8-lanes-per-group kernel has 8 times the parallelism and lower latency.
   const long long min_groups = opt(O_AQ2_MIN_GROUPS) > 0 ? opt(O_AQ2_MIN_GROUPS) : static_cast<long long>(sm_count()) * 256;
@@ -281,15 +286,15 @@ cudaError_t dispatch_act_quant_bits(int bits, const void* x, int x_dtype, long l
                     (xhat == nullptr || ((xhat_dtype == x_dtype || (x_dtype == ARCQ_DT_F32 && xhat_f16)) && aligned(xhat, 16)));
   if (tile) {
     switch (bits) {
-      case 4: return dispatch_act_quant_tile<T, 4, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st);
-      case 3: return dispatch_act_quant_tile<T, 3, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st);
-      default: return dispatch_act_quant_tile<T, 2, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st);
+      case 4: return dispatch_act_quant_tile<T, 4, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st, jobs);
+      case 3: return dispatch_act_quant_tile<T, 3, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st, jobs);
+      default: return dispatch_act_quant_tile<T, 2, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st, jobs);
     }
   }
   switch (bits) {
-    case 4: return launch_act_quant<T, 4, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st);
-    case 3: return launch_act_quant<T, 3, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st);
-    default: return launch_act_quant<T, 2, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st);
+    case 4: return launch_act_quant<T, 4, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st, jobs);
+    case 3: return launch_act_quant<T, 3, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st, jobs);
+    default: return launch_act_quant<T, 2, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st, jobs);
   }
 }
 
@@ -703,9 +708,32 @@ int arcq_device_status(void) {
   return v;
 }
 
+// The unpack jobs of a call as kernel argument.  Blocks of 128 threads or more, each thread taking four 16-byte chunks a
+// round: enough blocks for one round, two per SM at most (they share the SMs with the kernel's own blocks).
+static int make_unpack_jobs(const arcq_unpack_job* jobs, int n, arcq::UnpackJobs* out) {
+  *out = arcq::UnpackJobs{};
+  if (n == 0) return ARCQ_OK;
+  if (jobs == nullptr || n < 0 || n > 2) return fail(ARCQ_E_BAD_ARG, "between 0 and 2 unpack jobs");
+  long long chunks = 0;
+  for (int i = 0; i < n; ++i) {
+    const arcq_unpack_job& j = jobs[i];
+    if (!j.packed || !j.mu || !j.sigma || !j.codesum || !j.codebook || !j.out) return fail(ARCQ_E_BAD_ARG, "null pointer in an unpack job");
+    if (j.bits < 2 || j.bits > 4) return fail(ARCQ_E_BAD_ARG, "bits must be 2, 3 or 4, got %d", j.bits);
+    if (j.rows <= 0 || j.K <= 0 || j.K % 64 != 0) return fail(ARCQ_E_BAD_SHAPE, "bad shape of a weight: rows=%lld K=%lld", (long long)j.rows, (long long)j.K);
+    if (!aligned(j.packed, 4) || !aligned(j.out, 16)) return fail(ARCQ_E_ALIGN, "packed codes must be 4-byte, out 16-byte aligned");
+    out->job[i] = arcq::UnpackWeightJob{j.packed, j.mu, j.sigma, j.codesum, j.codebook, static_cast<__half*>(j.out),
+                                        static_cast<long long>(j.rows), static_cast<int>(j.K), j.bits};
+    chunks += j.rows * (j.K / 8);
+  }
+  const long long want = (chunks + 511) / 512, cap = 2ll * sm_count();
+  out->blocks = static_cast<int>(want < cap ? want : cap);
+  return ARCQ_OK;
+}
+
 static int act_quant_impl(int pre, const void* x, int x_dtype, int64_t M, int64_t K, const float* thresholds,
                           const float* codebook, int bits, int group_size, uint8_t* packed_out, float* mu_out,
-                          float* sigma_out, float* codesum_out, void* xhat_out, int xhat_dtype, void* stream) {
+                          float* sigma_out, float* codesum_out, void* xhat_out, int xhat_dtype,
+                          const arcq_unpack_job* unpack, int n_unpack, void* stream) {
   if (x == nullptr || thresholds == nullptr || codebook == nullptr) return fail(ARCQ_E_BAD_ARG, "null input pointer");
   if (packed_out == nullptr && xhat_out == nullptr) return fail(ARCQ_E_BAD_ARG, "no output requested");
   if ((mu_out != nullptr) != (sigma_out != nullptr)) return fail(ARCQ_E_BAD_ARG, "mu_out and sigma_out go together");
@@ -721,22 +749,24 @@ static int act_quant_impl(int pre, const void* x, int x_dtype, int64_t M, int64_
   if (group_size != 64) return fail(ARCQ_E_UNSUPPORTED, "group_size %d: only 64 is built", group_size);
   if (packed_out != nullptr && !aligned(packed_out, 4)) return fail(ARCQ_E_ALIGN, "packed_out must be 4-byte aligned");
   if (M == 0) return ARCQ_OK;
+  arcq::UnpackJobs jobs;
+  if (const int rc = make_unpack_jobs(unpack, n_unpack, &jobs)) return rc;
   const long long groups = static_cast<long long>(M) * (K / 64);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t e;
   if (pre == 1) {
     if (x_dtype != ARCQ_DT_F16) return fail(ARCQ_E_UNSUPPORTED, "the fused GELU is built for fp16 input only");
     e = dispatch_act_quant_bits<__half, 1>(bits, x, x_dtype, groups, thresholds, codebook, packed_out, mu_out,
-                                           sigma_out, codesum_out, xhat_out, xhat_dtype, st);
+                                           sigma_out, codesum_out, xhat_out, xhat_dtype, st, jobs);
   } else if (x_dtype == ARCQ_DT_F32)
     e = dispatch_act_quant_bits<float, 0>(bits, x, x_dtype, groups, thresholds, codebook, packed_out, mu_out, sigma_out,
-                                          codesum_out, xhat_out, xhat_dtype, st);
+                                          codesum_out, xhat_out, xhat_dtype, st, jobs);
   else if (x_dtype == ARCQ_DT_F16)
     e = dispatch_act_quant_bits<__half, 0>(bits, x, x_dtype, groups, thresholds, codebook, packed_out, mu_out, sigma_out,
-                                           codesum_out, xhat_out, xhat_dtype, st);
+                                           codesum_out, xhat_out, xhat_dtype, st, jobs);
   else
     e = dispatch_act_quant_bits<__nv_bfloat16, 0>(bits, x, x_dtype, groups, thresholds, codebook, packed_out, mu_out,
-                                                  sigma_out, codesum_out, xhat_out, xhat_dtype, st);
+                                                  sigma_out, codesum_out, xhat_out, xhat_dtype, st, jobs);
   if (e != cudaSuccess) return cuda_fail(e, "act_quant launch");
   return ARCQ_OK;
 }
@@ -745,14 +775,21 @@ int arcq_act_quant(const void* x, int x_dtype, int64_t M, int64_t K, const float
                    int bits, int group_size, uint8_t* packed_out, float* mu_out, float* sigma_out, float* codesum_out,
                    void* xhat_out, int xhat_dtype, void* stream) {
   return act_quant_impl(0, x, x_dtype, M, K, thresholds, codebook, bits, group_size, packed_out, mu_out, sigma_out,
-                        codesum_out, xhat_out, xhat_dtype, stream);
+                        codesum_out, xhat_out, xhat_dtype, nullptr, 0, stream);
 }
 
 int arcq_gelu_act_quant(const void* x, int x_dtype, int64_t M, int64_t K, const float* thresholds,
                         const float* codebook, int bits, int group_size, uint8_t* packed_out, float* mu_out,
                         float* sigma_out, float* codesum_out, void* xhat_out, int xhat_dtype, void* stream) {
   return act_quant_impl(1, x, x_dtype, M, K, thresholds, codebook, bits, group_size, packed_out, mu_out, sigma_out,
-                        codesum_out, xhat_out, xhat_dtype, stream);
+                        codesum_out, xhat_out, xhat_dtype, nullptr, 0, stream);
+}
+
+int arcq_act_quant_unpack(int pre_gelu, const void* x, int x_dtype, int64_t M, int64_t K, const float* thresholds,
+                          const float* codebook, int bits, int group_size, void* xhat_out, int xhat_dtype,
+                          const arcq_unpack_job* unpack, int n_unpack, void* stream) {
+  return act_quant_impl(pre_gelu != 0, x, x_dtype, M, K, thresholds, codebook, bits, group_size, nullptr, nullptr, nullptr, nullptr,
+                        xhat_out, xhat_dtype, unpack, n_unpack, stream);
 }
 
 int arcq_packed_gemm(const uint8_t* packed_x, const float* mu_a, const float* sigma_a, const float* codesum_a,
@@ -1060,10 +1097,16 @@ int arcq_dense_weight_gemm_prefetch(const void* xhat, const void* w16, const flo
 
 int arcq_add_layernorm(const void* x, const void* y, const float* gamma, const float* beta, float eps, int64_t M,
                        int64_t K, void* sum_out, void* h_out, void* stream) {
+  return arcq_add_layernorm_strided(x, y, gamma, beta, eps, M, K, K, sum_out, h_out, stream);
+}
+
+int arcq_add_layernorm_strided(const void* x, const void* y, const float* gamma, const float* beta, float eps, int64_t M,
+                               int64_t K, int64_t ld, void* sum_out, void* h_out, void* stream) {
   if (x == nullptr || gamma == nullptr || beta == nullptr || h_out == nullptr)
     return fail(ARCQ_E_BAD_ARG, "null pointer argument");
   if (M < 0 || K <= 0) return fail(ARCQ_E_BAD_SHAPE, "bad shape M=%lld K=%lld", (long long)M, (long long)K);
   if (K % 8 != 0) return fail(ARCQ_E_BAD_SHAPE, "K=%lld must be a multiple of 8", (long long)K);
+  if (ld < K || ld % 8 != 0) return fail(ARCQ_E_BAD_SHAPE, "row stride %lld must be a multiple of 8, at least K", (long long)ld);
   if (K > 32 * 8 * arcq::kLnMaxChunks) return fail(ARCQ_E_TOO_LARGE, "rows longer than %d values are not built", 32 * 8 * arcq::kLnMaxChunks);
   if (!aligned(x, 16) || !aligned(h_out, 16) || (y != nullptr && !aligned(y, 16)) ||
       (sum_out != nullptr && !aligned(sum_out, 16)) || !aligned(gamma, 16) || !aligned(beta, 16))
@@ -1074,13 +1117,13 @@ int arcq_add_layernorm(const void* x, const void* y, const float* gamma, const f
   __half *so = static_cast<__half*>(sum_out), *ho = static_cast<__half*>(h_out);
   const bool plain = opt(O_LN_PLAIN) != 0;
   if (K == 384 && !plain) {          // 16 lanes per row, 2 rows per warp
-    launch_pdl(arcq::add_layernorm_rows_kernel<16>, grid_for(M, 16, 6), 256, 0, st, xh, yh, gamma, beta, eps, M, so, ho);
+    launch_pdl(arcq::add_layernorm_rows_kernel<16>, grid_for(M, 16, 6), 256, 0, st, xh, yh, gamma, beta, eps, M, ld, so, ho);
   } else if (K == 192 && !plain) {
-    launch_pdl(arcq::add_layernorm_rows_kernel<8>, grid_for(M, 32, 6), 256, 0, st, xh, yh, gamma, beta, eps, M, so, ho);
+    launch_pdl(arcq::add_layernorm_rows_kernel<8>, grid_for(M, 32, 6), 256, 0, st, xh, yh, gamma, beta, eps, M, ld, so, ho);
   } else if (K == 768 && !plain) {
-    launch_pdl(arcq::add_layernorm_rows_kernel<32>, grid_for(M, 8, 6), 256, 0, st, xh, yh, gamma, beta, eps, M, so, ho);
+    launch_pdl(arcq::add_layernorm_rows_kernel<32>, grid_for(M, 8, 6), 256, 0, st, xh, yh, gamma, beta, eps, M, ld, so, ho);
   } else {
-    launch_pdl(arcq::add_layernorm_kernel, grid_for(M, 8, 8), 256, 0, st, xh, yh, gamma, beta, eps, M, static_cast<int>(K), so, ho);
+    launch_pdl(arcq::add_layernorm_kernel, grid_for(M, 8, 8), 256, 0, st, xh, yh, gamma, beta, eps, M, static_cast<int>(K), ld, so, ho);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "add_layernorm launch");
@@ -1090,6 +1133,14 @@ int arcq_add_layernorm(const void* x, const void* y, const float* gamma, const f
 int arcq_add_layernorm_act_quant(const void* x, const void* y, const float* gamma, const float* beta, float eps,
                                  int64_t M, int64_t K, const float* thresholds, const float* codebook, int bits,
                                  int group_size, void* sum_out, void* h_out, void* xhat, void* stream) {
+  return arcq_add_layernorm_act_quant_unpack(x, y, gamma, beta, eps, M, K, thresholds, codebook, bits, group_size, sum_out, h_out,
+                                             xhat, nullptr, 0, stream);
+}
+
+int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const float* gamma, const float* beta, float eps,
+                                        int64_t M, int64_t K, const float* thresholds, const float* codebook, int bits,
+                                        int group_size, void* sum_out, void* h_out, void* xhat,
+                                        const arcq_unpack_job* unpack, int n_unpack, void* stream) {
   if (x == nullptr || gamma == nullptr || beta == nullptr || thresholds == nullptr || codebook == nullptr || xhat == nullptr)
     return fail(ARCQ_E_BAD_ARG, "null pointer argument");
   if (bits < 2 || bits > 4) return fail(ARCQ_E_BAD_ARG, "bits must be 2, 3 or 4, got %d", bits);
@@ -1103,23 +1154,25 @@ int arcq_add_layernorm_act_quant(const void* x, const void* y, const float* gamm
       (sum_out != nullptr && !aligned(sum_out, 16)) || (h_out != nullptr && !aligned(h_out, 16)))
     return fail(ARCQ_E_ALIGN, "all matrices must be 16-byte aligned");
   if (M == 0) return ARCQ_OK;
+  arcq::UnpackJobs jobs;
+  if (const int rc = make_unpack_jobs(unpack, n_unpack, &jobs)) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int G = static_cast<int>(K / 64);
   {
-    // Small inputs, where the tiled kernel's 128-group tiles would not give every SM a block: the twelve-warp
-    // form (48 groups per block, lower latency).  Both forms give the same bits.  (DeiT-T at batch 64, 37 824
-    // groups, measured 8 % slower through the small form than through the tiled one.)
-    const bool small = M * G < static_cast<long long>(sm_count()) * arcq::kLnqThreads && opt(O_LNQ_SMALL) != 0;
+    // Small inputs, where most SMs would get no 128-group tile: the twelve-warp form (48 groups per block, lower
+    // latency).  Both forms give the same bits.  The line is where they measured equal: 4 137 groups 3.4 against 5.9 us,
+    // 8 274 groups 6.5 against 5.6 us, 18 912 groups 9.8 against 6.0 us.
+    const bool small = M * G < static_cast<long long>(sm_count()) * 48 && opt(O_LNQ_SMALL) != 0;
     if (small) {
       const __half *xs = static_cast<const __half*>(x), *ys = static_cast<const __half*>(y);
       __half *so2 = static_cast<__half*>(sum_out), *ho2 = static_cast<__half*>(h_out), *xo2 = static_cast<__half*>(xhat);
       const int lanes = static_cast<int>(K / 24), rows_tile = 4 * (32 / lanes);
       const long long tiles2 = (M + rows_tile - 1) / rows_tile;
       const long long cap2 = static_cast<long long>(sm_count()) * 8;
-      const unsigned grid2 = static_cast<unsigned>(tiles2 < cap2 ? tiles2 : cap2);
+      const unsigned grid2 = static_cast<unsigned>((tiles2 < cap2 ? tiles2 : cap2) + jobs.blocks);
 #define ARCQ_LAUNCH_LNQ_ROWS(LN, B, HASY)                                                                            \
   launch_pdl(arcq::add_layernorm_act_quant_rows_kernel<LN, B, HASY>, grid2, arcq::kLnqRowsThreads, 0, st, xs, ys, gamma, beta, eps,     \
-             static_cast<long long>(M), thresholds, codebook, so2, ho2, xo2)
+             static_cast<long long>(M), thresholds, codebook, so2, ho2, xo2, jobs)
 #define ARCQ_LNQ_ROWS_BITS(LN, HASY)                                                                                  \
   do {                                                                                                                \
     if (bits == 4) ARCQ_LAUNCH_LNQ_ROWS(LN, 4, HASY);                                                                  \
@@ -1140,7 +1193,7 @@ int arcq_add_layernorm_act_quant(const void* x, const void* y, const float* gamm
   }
   const long long tiles = (M * G + arcq::kLnqThreads - 1) / arcq::kLnqThreads;
   const long long cap = static_cast<long long>(sm_count()) * 4;
-  const unsigned grid = static_cast<unsigned>(tiles < cap ? tiles : cap);
+  const unsigned grid = static_cast<unsigned>((tiles < cap ? tiles : cap) + jobs.blocks);
   const size_t smem = arcq::lnq_smem_bytes();
   const __half *xh = static_cast<const __half*>(x), *yh = static_cast<const __half*>(y);
   __half *so = static_cast<__half*>(sum_out), *ho = static_cast<__half*>(h_out);
@@ -1151,7 +1204,7 @@ int arcq_add_layernorm_act_quant(const void* x, const void* y, const float* gamm
     return fail(ARCQ_E_CUDA, "cuTensorMapEncodeTiled failed for the reconstruction");
 #define ARCQ_LAUNCH_LNQ(LN, B, HASY)                                                                                   \
   launch_pdl(arcq::add_layernorm_act_quant_kernel<LN, B, HASY>, grid, arcq::kLnqThreads, smem, st, tm_out, xh, yh, gamma, \
-             beta, eps, static_cast<long long>(M), thresholds, codebook, so, ho)
+             beta, eps, static_cast<long long>(M), thresholds, codebook, so, ho, jobs)
 #define ARCQ_LNQ_BITS(LN, HASY)                                                                                         \
   do {                                                                                                                  \
     if (bits == 4) ARCQ_LAUNCH_LNQ(LN, 4, HASY);                                                                         \

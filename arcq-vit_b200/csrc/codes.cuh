@@ -3,7 +3,7 @@
 #pragma once
 #include <cuda_fp16.h>
 #include "ptx.cuh"
-#include "act_quant.cuh"
+#include "element_types.cuh"
 
 namespace arcq {
 
@@ -160,6 +160,34 @@ __device__ __forceinline__ void unpack_weight_f16_chunks(const UnpackWeightJob& 
       }
       *reinterpret_cast<uint4*>(j.out + off[u]) = make_uint4(h[0], h[1], h[2], h[3]);
     }
+  }
+}
+
+// Weights that a kernel of the activation path unpacks on the side: its first `blocks` blocks take the jobs (chunks split over
+// their threads), the others do the kernel's own work.  The unpack then needs no launch and no second stream, and it runs
+// beside the quantizer, on SMs that a small input leaves idle.
+struct UnpackJobs {
+  UnpackWeightJob job[2];
+  int blocks;                // 0: none
+};
+__device__ __forceinline__ void unpack_jobs_block(const UnpackJobs& u) {
+  __shared__ __half s_ucb[2][16];
+  const int tid = threadIdx.x;
+  if (tid < 32) {
+    const UnpackWeightJob& j = u.job[tid >> 4];
+    const int i = tid & 15;
+    s_ucb[tid >> 4][i] = __float2half_rn(j.packed != nullptr && i < (1 << j.bits) ? __ldg(j.codebook + i) : 0.0f);
+  }
+  __syncthreads();
+  pdl_wait();                // the matrices written here may still be read by the kernel before this one
+  const long long first = static_cast<long long>(blockIdx.x) * blockDim.x + tid, stride = static_cast<long long>(u.blocks) * blockDim.x;
+#pragma unroll 1
+  for (int k = 0; k < 2; ++k) {
+    const UnpackWeightJob& j = u.job[k];
+    if (j.packed == nullptr) break;
+    if (j.bits == 4) unpack_weight_f16_chunks<4>(j, s_ucb[k], first, stride);
+    else if (j.bits == 3) unpack_weight_f16_chunks<3>(j, s_ucb[k], first, stride);
+    else unpack_weight_f16_chunks<2>(j, s_ucb[k], first, stride);
   }
 }
 

@@ -1,0 +1,444 @@
+// Host path of the package in native code: a CPython extension over libarcq_b200 that takes torch tensors.
+//
+// A packed linear is two short kernels; called from Python, argument checks, stream and allocator look-ups and ctypes
+// marshalling took 35 us a layer around 8 us of GPU work, and an eager ViT forward (about 250 calls) 5.5 ms around 0.7 ms.  Here
+// a layer is one call (about 6 us, launches included) and the forward of a packed ViT one call that launches every kernel.
+//
+// Every function returns None for what it does not take (other dtypes, devices, layouts, shapes); the Python code it
+// shortcuts then runs as before and raises what it always raised.  Module parameters are not copied or cached: a call
+// reads the tensors out of the modules' own dictionaries, so moved, replaced or re-typed parameters are seen.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <string>
+#include <vector>
+
+#include "../../include/arcq_b200.h"
+
+namespace {
+
+struct Fail {};   // a Python error is set
+
+void check(int rc, const char* what) {
+  if (rc != ARCQ_OK) {
+    PyErr_Format(PyExc_RuntimeError, "%s failed (%d): %s", what, rc, arcq_last_error_string());
+    throw Fail{};
+  }
+}
+
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+int dtype_code(at::ScalarType t) {
+  switch (t) {
+    case at::kFloat: return ARCQ_DT_F32;
+    case at::kHalf: return ARCQ_DT_F16;
+    case at::kBFloat16: return ARCQ_DT_BF16;
+    default: return -1;
+  }
+}
+
+at::Tensor empty_cuda(at::IntArrayRef sizes, at::ScalarType t, c10::Device dev) {
+  return at::detail::empty_cuda(sizes, t, dev, std::nullopt);
+}
+
+const at::Tensor* tensor_of(PyObject* o) { return o != nullptr && THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+PyObject* g_oom_error = nullptr;    // torch.OutOfMemoryError
+PyObject* g_key[16];
+enum Key { kPacked, kCenter, kScale, kCodeSum, kWCodebook, kACodebook, kAThresholds, kBiasTensor, kBias, kWeight, kKeys };
+const char* const kKeyNames[kKeys] = {"packed_weight_codes", "weight_center", "weight_scale", "weight_code_sum", "weight_codebook",
+                                      "activation_codebook", "activation_thresholds", "bias_tensor", "bias", "weight"};
+
+// A contiguous CUDA tensor of the given type out of a module's dictionary, or null.
+const at::Tensor* device_tensor(PyObject* dict, Key key, at::ScalarType t, const c10::Device& dev) {
+  const at::Tensor* v = tensor_of(PyDict_GetItem(dict, g_key[key]));
+  if (v == nullptr || v->scalar_type() != t || v->device() != dev || !v->is_contiguous()) return nullptr;
+  return v;
+}
+
+// The kernels' view of one packed linear.
+struct Linear {
+  int64_t N, K;
+  int bits;
+  const float *th, *acb, *bias;
+  arcq_unpack_job job;
+  int64_t weight_elems() const { return N * K; }
+};
+
+bool read_linear(PyObject* buffers, Key bias_key, const c10::Device& dev, Linear* l) {
+  if (!PyDict_Check(buffers)) return false;
+  const at::Tensor* codes = device_tensor(buffers, kPacked, at::kByte, dev);
+  const at::Tensor* f[6];
+  const Key keys[6] = {kCenter, kScale, kCodeSum, kWCodebook, kACodebook, kAThresholds};
+  for (int i = 0; i < 6; ++i)
+    if ((f[i] = device_tensor(buffers, keys[i], at::kFloat, dev)) == nullptr) return false;
+  if (codes == nullptr || codes->dim() != 2 || f[0]->dim() != 2) return false;
+  const int64_t levels = f[3]->numel();
+  l->bits = levels == 16 ? 4 : levels == 8 ? 3 : levels == 4 ? 2 : 0;
+  l->N = f[0]->size(0);
+  l->K = f[0]->size(1) * 64;
+  if (l->bits == 0 || l->N % 16 != 0 || l->N == 0 || l->K == 0 || codes->size(0) != l->N || codes->size(1) != l->K * l->bits / 8 ||
+      f[1]->numel() != f[0]->numel() || f[2]->numel() != f[0]->numel() || f[4]->numel() != levels || f[5]->numel() != levels - 1)
+    return false;
+  const at::Tensor* b = tensor_of(PyDict_GetItem(buffers, g_key[bias_key]));
+  l->bias = nullptr;
+  if (b != nullptr && b->numel() > 0) {
+    if (b->scalar_type() != at::kFloat || b->device() != dev || !b->is_contiguous() || b->numel() != l->N) return false;
+    l->bias = b->const_data_ptr<float>();
+  }
+  l->acb = f[4]->const_data_ptr<float>();
+  l->th = f[5]->const_data_ptr<float>();
+  l->job = arcq_unpack_job{codes->const_data_ptr<uint8_t>(), f[0]->const_data_ptr<float>(), f[1]->const_data_ptr<float>(),
+                           f[2]->const_data_ptr<float>(), f[3]->const_data_ptr<float>(), nullptr, l->N, l->K, l->bits};
+  return (reinterpret_cast<uintptr_t>(l->job.packed) & 3u) == 0;
+}
+
+// ---------------------------------------------------------------- one packed linear
+// linear(buffers, x, bias key 0 "bias_tensor" / 1 "bias", fp32 output, pre_gelu, pre_quantized) -> y or None
+PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  const at::Tensor* x = n == 6 ? tensor_of(args[1]) : nullptr;
+  if (x == nullptr || !x->is_cuda() || x->dim() < 1 || !x->is_contiguous()) Py_RETURN_NONE;
+  const bool float_chain = PyObject_IsTrue(args[3]), pre_gelu = PyObject_IsTrue(args[4]), ready = PyObject_IsTrue(args[5]);
+  const int xt = dtype_code(x->scalar_type());
+  if (xt < 0 || (!float_chain && xt != ARCQ_DT_F16) || ((pre_gelu || ready) && xt != ARCQ_DT_F16)) Py_RETURN_NONE;
+  Linear l;
+  if (!read_linear(args[0], PyObject_IsTrue(args[2]) ? kBias : kBiasTensor, x->device(), &l)) Py_RETURN_NONE;
+  const int64_t numel = x->numel();
+  if (x->size(-1) != l.K || numel == 0 || !aligned16(x->const_data_ptr())) Py_RETURN_NONE;
+  const int64_t M = numel / l.K;
+  const c10::cuda::CUDAGuard guard(x->device());
+  void* const st = c10::cuda::getCurrentCUDAStream().stream();
+  // the reconstructed activation and the unpacked weight, given back to the caching allocator on return
+  const at::Tensor scratch = empty_cuda({(ready ? 0 : numel) + l.weight_elems() + 8}, at::kHalf, x->device());
+  at::Half* const w16 = scratch.mutable_data_ptr<at::Half>();
+  const void* xhat = x->const_data_ptr();
+  l.job.out = w16;
+  if (ready) {
+    check(arcq_unpack_weight_f16(l.job.packed, l.job.mu, l.job.sigma, l.job.codesum, l.job.codebook, l.bits, 64, l.N, l.K, w16, st),
+          "arcq_unpack_weight_f16");
+  } else {
+    void* const xh = w16 + l.weight_elems();
+    check(arcq_act_quant_unpack(pre_gelu, xhat, xt, M, l.K, l.th, l.acb, l.bits, 64, xh, ARCQ_DT_F16, &l.job, 1, st), "arcq_act_quant");
+    xhat = xh;
+  }
+  c10::SmallVector<int64_t, 5> sizes(x->sizes().begin(), x->sizes().end());
+  sizes.back() = l.N;
+  at::Tensor y = empty_cuda(sizes, float_chain ? at::kFloat : at::kHalf, x->device());
+  check(arcq_dense_weight_gemm(xhat, w16, l.bias, M, l.N, l.K, y.mutable_data_ptr(), float_chain ? ARCQ_DT_F32 : ARCQ_DT_F16, st),
+        "arcq_dense_weight_gemm");
+  return THPVariable_Wrap(std::move(y));
+}
+
+// ---------------------------------------------------------------- operators
+// quantize_activation(x, thresholds, codebook, bits, want_code_sum, pre_gelu) -> (packed, center, scale, code_sum) or None
+PyObject* quantize_activation(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 6) Py_RETURN_NONE;
+  const at::Tensor *x = tensor_of(args[0]), *th = tensor_of(args[1]), *cb = tensor_of(args[2]);
+  if (x == nullptr || th == nullptr || cb == nullptr || !x->is_cuda() || x->dim() != 2 || !x->is_contiguous()) Py_RETURN_NONE;
+  const long bits = PyLong_AsLong(args[3]);
+  const int xt = dtype_code(x->scalar_type());
+  for (const at::Tensor* t : {th, cb})
+    if (t->scalar_type() != at::kFloat || t->device() != x->device() || !t->is_contiguous()) Py_RETURN_NONE;
+  const int64_t M = x->size(0), K = x->size(1);
+  if (xt < 0 || bits < 2 || bits > 4 || cb->numel() != (1 << bits) || th->numel() != (1 << bits) - 1 || M == 0 || K == 0 || K % 64 != 0)
+    Py_RETURN_NONE;
+  const bool want_cs = PyObject_IsTrue(args[4]), pre_gelu = PyObject_IsTrue(args[5]);
+  const c10::cuda::CUDAGuard guard(x->device());
+  at::Tensor packed = empty_cuda({M, K * bits / 8}, at::kByte, x->device());
+  at::Tensor mu = empty_cuda({M, K / 64}, at::kFloat, x->device()), sg = empty_cuda({M, K / 64}, at::kFloat, x->device());
+  at::Tensor cs = want_cs ? empty_cuda({M, K / 64}, at::kFloat, x->device()) : at::Tensor();
+  check((pre_gelu ? arcq_gelu_act_quant : arcq_act_quant)(
+            x->const_data_ptr(), xt, M, K, th->const_data_ptr<float>(), cb->const_data_ptr<float>(), static_cast<int>(bits), 64,
+            packed.mutable_data_ptr<uint8_t>(), mu.mutable_data_ptr<float>(), sg.mutable_data_ptr<float>(),
+            want_cs ? cs.mutable_data_ptr<float>() : nullptr, nullptr, 0, c10::cuda::getCurrentCUDAStream().stream()),
+        "arcq_act_quant");
+  PyObject* out = PyTuple_New(4);
+  PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(std::move(packed)));
+  PyTuple_SET_ITEM(out, 1, THPVariable_Wrap(std::move(mu)));
+  PyTuple_SET_ITEM(out, 2, THPVariable_Wrap(std::move(sg)));
+  if (want_cs) {
+    PyTuple_SET_ITEM(out, 3, THPVariable_Wrap(std::move(cs)));
+  } else {
+    Py_INCREF(Py_None);
+    PyTuple_SET_ITEM(out, 3, Py_None);
+  }
+  return out;
+}
+
+// dequant(packed, center, scale, code_sum, codebook, bits, fp32 output) -> [R, K] or None (group size 64)
+PyObject* dequant(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 7) Py_RETURN_NONE;
+  const at::Tensor* t[5];
+  for (int i = 0; i < 5; ++i) {
+    t[i] = tensor_of(args[i]);
+    if (t[i] == nullptr || !t[i]->is_cuda() || !t[i]->is_contiguous() || t[i]->scalar_type() != (i == 0 ? at::kByte : at::kFloat) ||
+        t[i]->device() != t[0]->device())
+      Py_RETURN_NONE;
+  }
+  const long bits = PyLong_AsLong(args[5]);
+  if (bits < 2 || bits > 4 || t[0]->dim() != 2 || t[1]->dim() != 2) Py_RETURN_NONE;
+  const int64_t R = t[1]->size(0), K = t[1]->size(1) * 64;
+  if (R == 0 || K == 0 || t[0]->size(0) != R || t[0]->size(1) != K * bits / 8 || t[2]->numel() != t[1]->numel() ||
+      t[3]->numel() != t[1]->numel() || t[4]->numel() != (1 << bits))
+    Py_RETURN_NONE;
+  const bool f32 = PyObject_IsTrue(args[6]);
+  const c10::cuda::CUDAGuard guard(t[0]->device());
+  at::Tensor out = empty_cuda({R, K}, f32 ? at::kFloat : at::kHalf, t[0]->device());
+  check(arcq_dequant(t[0]->const_data_ptr<uint8_t>(), t[1]->const_data_ptr<float>(), t[2]->const_data_ptr<float>(),
+                     t[3]->const_data_ptr<float>(), t[4]->const_data_ptr<float>(), static_cast<int>(bits), 64, R, K,
+                     out.mutable_data_ptr(), f32 ? ARCQ_DT_F32 : ARCQ_DT_F16, c10::cuda::getCurrentCUDAStream().stream()),
+        "arcq_dequant");
+  return THPVariable_Wrap(std::move(out));
+}
+
+// ---------------------------------------------------------------- the forward of a packed ViT
+// What a plan holds are references to the dictionaries of the model's modules; nothing of their content.
+struct Norm {
+  PyObject* params;             // _parameters of the LayerNorm
+  double eps;
+  at::Tensor gamma, beta;       // fp32 copies when the parameters are not fp32, remade when those change
+  const void* seen[2] = {nullptr, nullptr};
+  uint32_t version[2] = {0, 0};
+};
+struct VitBlock {
+  Norm norm1, norm2;
+  PyObject *qkv, *proj, *fc1, *fc2;   // _buffers
+};
+struct VitPlan {
+  int64_t dim, heads, patch;
+  PyObject *own, *patch_params, *head_params;      // _parameters of the model, of patch_embed.proj and of head
+  std::vector<VitBlock> blocks;
+  Norm norm;
+  std::vector<PyObject*> watch;       // (dict, key, expected value) triples: the modules the plan was made for
+  std::vector<PyObject*> empty;       // hook dictionaries that have to be empty
+  std::vector<PyObject*> refs;
+  ~VitPlan() {
+    for (PyObject* o : refs) Py_XDECREF(o);
+  }
+};
+
+uint32_t version_of(const at::Tensor& t) { return t.is_inference() ? 0u : static_cast<uint32_t>(t._version()); }
+
+bool read_norm(Norm* n, const c10::Device& dev, int64_t dim, const float** gamma, const float** beta) {
+  const at::Tensor* t[2] = {tensor_of(PyDict_GetItem(n->params, g_key[kWeight])), tensor_of(PyDict_GetItem(n->params, g_key[kBias]))};
+  for (int i = 0; i < 2; ++i) {
+    if (t[i] == nullptr || t[i]->device() != dev || t[i]->numel() != dim || dtype_code(t[i]->scalar_type()) < 0) return false;
+    at::Tensor& copy = i ? n->beta : n->gamma;
+    if (t[i]->scalar_type() == at::kFloat && t[i]->is_contiguous() && aligned16(t[i]->const_data_ptr())) {
+      *(i ? beta : gamma) = t[i]->const_data_ptr<float>();
+      continue;
+    }
+    const void* p = t[i]->const_data_ptr();
+    if (!copy.defined() || n->seen[i] != p || n->version[i] != version_of(*t[i]) || t[i]->is_inference() || copy.device() != dev) {
+      copy = t[i]->detach().to(at::kFloat).contiguous();
+      n->seen[i] = p;
+      n->version[i] = version_of(*t[i]);
+    }
+    *(i ? beta : gamma) = copy.const_data_ptr<float>();
+  }
+  return true;
+}
+
+void free_plan(PyObject* capsule) { delete static_cast<VitPlan*>(PyCapsule_GetPointer(capsule, "arcq_vit_plan")); }
+
+// vit_plan(dim, heads, patch, own params, patch params, head params, final norm (params, eps),
+//          blocks [(norm1 params, eps, norm2 params, eps, qkv, proj, fc1, fc2 buffers)], watch [dict, key, value, ...], empty [dict])
+PyObject* vit_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 11) {
+    PyErr_SetString(PyExc_TypeError, "vit_plan takes 11 arguments");
+    return nullptr;
+  }
+  auto* p = new VitPlan;
+  auto keep = [&](PyObject* o) {
+    Py_INCREF(o);
+    p->refs.push_back(o);
+    return o;
+  };
+  p->dim = PyLong_AsLongLong(a[0]);
+  p->heads = PyLong_AsLongLong(a[1]);
+  p->patch = PyLong_AsLongLong(a[2]);
+  p->own = keep(a[3]);
+  p->patch_params = keep(a[4]);
+  p->head_params = keep(a[5]);
+  p->norm.params = keep(a[6]);
+  p->norm.eps = PyFloat_AsDouble(a[7]);
+  for (Py_ssize_t i = 0; i < PyList_Size(a[8]); ++i) {
+    PyObject* t = PyList_GetItem(a[8], i);
+    VitBlock b;
+    b.norm1.params = keep(PyTuple_GetItem(t, 0));
+    b.norm1.eps = PyFloat_AsDouble(PyTuple_GetItem(t, 1));
+    b.norm2.params = keep(PyTuple_GetItem(t, 2));
+    b.norm2.eps = PyFloat_AsDouble(PyTuple_GetItem(t, 3));
+    b.qkv = keep(PyTuple_GetItem(t, 4));
+    b.proj = keep(PyTuple_GetItem(t, 5));
+    b.fc1 = keep(PyTuple_GetItem(t, 6));
+    b.fc2 = keep(PyTuple_GetItem(t, 7));
+    p->blocks.push_back(std::move(b));
+  }
+  for (Py_ssize_t i = 0; i < PyList_Size(a[9]); ++i) p->watch.push_back(keep(PyList_GetItem(a[9], i)));
+  for (Py_ssize_t i = 0; i < PyList_Size(a[10]); ++i) p->empty.push_back(keep(PyList_GetItem(a[10], i)));
+  if (PyErr_Occurred()) {
+    delete p;
+    return nullptr;
+  }
+  return PyCapsule_New(p, "arcq_vit_plan", free_plan);
+}
+
+// vit_forward(plan, images) -> logits; None: the model or the input is not one the plan covers
+PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 2) Py_RETURN_NONE;
+  auto* p = static_cast<VitPlan*>(PyCapsule_GetPointer(args[0], "arcq_vit_plan"));
+  if (p == nullptr) return nullptr;
+  const at::Tensor* img = tensor_of(args[1]);
+  if (img == nullptr || !img->is_cuda() || img->scalar_type() != at::kHalf || img->dim() != 4 || !img->is_contiguous() ||
+      img->numel() == 0 || !aligned16(img->const_data_ptr()))
+    Py_RETURN_NONE;
+  for (size_t i = 0; i < p->watch.size(); i += 3) {
+    PyObject* const got = PyDict_GetItem(p->watch[i], p->watch[i + 1]);
+    if (got != p->watch[i + 2] && !(got == nullptr && p->watch[i + 2] == Py_None)) Py_RETURN_NONE;   // None: no such module
+  }
+  for (PyObject* d : p->empty)
+    if (PyDict_Size(d) != 0) Py_RETURN_NONE;
+  const c10::Device dev = img->device();
+  const int64_t B = img->size(0), C = img->size(1), H = img->size(2), W = img->size(3), P = p->patch, D = p->dim;
+  if (H % P != 0 || W % P != 0) Py_RETURN_NONE;
+  const int64_t T = (H / P) * (W / P) + 1, M = B * T;
+
+  static PyObject* const k_cls = PyUnicode_InternFromString("cls_token");
+  static PyObject* const k_pos = PyUnicode_InternFromString("pos_embed");
+  const at::Tensor *cls = tensor_of(PyDict_GetItem(p->own, k_cls)), *pos = tensor_of(PyDict_GetItem(p->own, k_pos));
+  const at::Tensor* pw = device_tensor(p->patch_params, kWeight, at::kHalf, dev);
+  const at::Tensor* pb = device_tensor(p->patch_params, kBias, at::kHalf, dev);
+  const at::Tensor* hw = device_tensor(p->head_params, kWeight, at::kHalf, dev);
+  const at::Tensor* hb = device_tensor(p->head_params, kBias, at::kHalf, dev);
+  for (const at::Tensor* t : {cls, pos})
+    if (t == nullptr || t->scalar_type() != at::kHalf || t->device() != dev || !t->is_contiguous() || !aligned16(t->const_data_ptr()))
+      Py_RETURN_NONE;
+  if (pw == nullptr || pb == nullptr || hw == nullptr || hb == nullptr || cls->numel() != D || pos->numel() != T * D ||
+      pw->numel() != D * C * P * P)
+    Py_RETURN_NONE;
+  const size_t depth = p->blocks.size();
+  std::vector<Linear> lin(4 * depth);
+  std::vector<const float*> gb(4 * depth + 2);
+  int64_t scratch_elems[2] = {0, 0};                       // qkv + proj, fc1 + fc2
+  for (size_t i = 0; i < depth; ++i) {
+    VitBlock& b = p->blocks[i];
+    PyObject* const d[4] = {b.qkv, b.proj, b.fc1, b.fc2};
+    const int64_t shape[4][2] = {{3 * D, D}, {D, D}, {4 * D, D}, {D, 4 * D}};
+    for (int k = 0; k < 4; ++k) {
+      Linear& l = lin[4 * i + k];
+      if (!read_linear(d[k], kBiasTensor, dev, &l)) Py_RETURN_NONE;
+      // any hidden width, the rest as the block's structure fixes it
+      if (k < 2 ? (l.N != shape[k][0] || l.K != shape[k][1]) : k == 2 ? l.K != D : (l.N != D || l.K != lin[4 * i + 2].N)) Py_RETURN_NONE;
+    }
+    scratch_elems[0] = std::max(scratch_elems[0], lin[4 * i].weight_elems() + lin[4 * i + 1].weight_elems());
+    scratch_elems[1] = std::max(scratch_elems[1], lin[4 * i + 2].weight_elems() + lin[4 * i + 3].weight_elems());
+    if (!read_norm(&b.norm1, dev, D, &gb[4 * i], &gb[4 * i + 1]) || !read_norm(&b.norm2, dev, D, &gb[4 * i + 2], &gb[4 * i + 3]))
+      Py_RETURN_NONE;
+  }
+  if (!read_norm(&p->norm, dev, D, &gb[4 * depth], &gb[4 * depth + 1])) Py_RETURN_NONE;
+  int64_t hidden = 0;
+  for (size_t i = 0; i < depth; ++i) hidden = std::max(hidden, lin[4 * i + 2].N);
+
+  const c10::cuda::CUDAGuard guard(dev);
+  void* const st = c10::cuda::getCurrentCUDAStream().stream();
+  // one workspace: residual stream (two, written in turn), reconstruction, branch output, qkv / fc1 output, fc2 input, weights
+  const int64_t wide = std::max<int64_t>(3 * D, hidden);
+  const at::Tensor ws = empty_cuda({M * (4 * D + wide + hidden) + scratch_elems[0] + scratch_elems[1] + 64}, at::kHalf, dev);
+  at::Half* at_ptr = ws.mutable_data_ptr<at::Half>();
+  auto take = [&](int64_t elems) {
+    at::Half* r = at_ptr;
+    at_ptr += (elems + 7) / 8 * 8;
+    return r;
+  };
+  at::Half *x = take(M * D), *x_next = take(M * D), *xhat = take(M * D), *branch = take(M * D), *mid = take(M * wide), *xhat4 = take(M * hidden);
+  at::Half *w_attn = take(scratch_elems[0]), *w_mlp = take(scratch_elems[1]);
+  for (size_t i = 0; i < depth; ++i) {
+    lin[4 * i].job.out = w_attn;
+    lin[4 * i + 1].job.out = w_attn + lin[4 * i].weight_elems();
+    lin[4 * i + 2].job.out = w_mlp;
+    lin[4 * i + 3].job.out = w_mlp + lin[4 * i + 2].weight_elems();
+  }
+  auto norm_quant = [&](const at::Half* y, const float* gamma, const float* beta, double eps, const Linear& first, const Linear& second) {
+    const arcq_unpack_job jobs[2] = {first.job, second.job};
+    check(arcq_add_layernorm_act_quant_unpack(x, y, gamma, beta, static_cast<float>(eps), M, D, first.th, first.acb, first.bits, 64,
+                                              y != nullptr ? x_next : nullptr, nullptr, xhat, jobs, 2, st),
+          "arcq_add_layernorm_act_quant");
+    if (y != nullptr) std::swap(x, x_next);
+  };
+  auto gemm = [&](const at::Half* a, const Linear& l, at::Half* y) {
+    check(arcq_dense_weight_gemm(a, l.job.out, l.bias, M, l.N, l.K, y, ARCQ_DT_F16, st), "arcq_dense_weight_gemm");
+  };
+
+  {
+    const at::Tensor rows = empty_cuda({B * (T - 1), C * P * P}, at::kHalf, dev);
+    check(arcq_patchify(img->const_data_ptr(), B, C, H, W, static_cast<int>(P), rows.mutable_data_ptr(), st), "arcq_patchify");
+    const at::Tensor patches = at::linear(rows, pw->view({D, C * P * P}), *pb);
+    check(arcq_assemble_tokens(patches.const_data_ptr(), cls->const_data_ptr(), pos->const_data_ptr(), B, T - 1, D, x, st),
+          "arcq_assemble_tokens");
+  }
+  const at::Half* y = nullptr;
+  for (size_t i = 0; i < depth; ++i) {
+    const VitBlock& b = p->blocks[i];
+    const Linear *qkv = &lin[4 * i], *proj = qkv + 1, *fc1 = qkv + 2, *fc2 = qkv + 3;
+    norm_quant(y, gb[4 * i], gb[4 * i + 1], b.norm1.eps, *qkv, *proj);
+    gemm(xhat, *qkv, mid);
+    {
+      const at::Tensor t = at::from_blob(mid, {B, T, 3, p->heads, D / p->heads}, at::TensorOptions().dtype(at::kHalf).device(dev));
+      const at::Tensor r = t.permute({2, 0, 3, 1, 4});
+      const at::Tensor o = at::scaled_dot_product_attention(r[0], r[1], r[2]).transpose(1, 2).reshape({M, D});
+      check(arcq_act_quant(o.const_data_ptr(), ARCQ_DT_F16, M, D, proj->th, proj->acb, proj->bits, 64, nullptr, nullptr, nullptr, nullptr,
+                           xhat, ARCQ_DT_F16, st),
+            "arcq_act_quant");
+    }
+    gemm(xhat, *proj, branch);
+    norm_quant(branch, gb[4 * i + 2], gb[4 * i + 3], b.norm2.eps, *fc1, *fc2);
+    gemm(xhat, *fc1, mid);
+    check(arcq_gelu_act_quant(mid, ARCQ_DT_F16, M, fc2->K, fc2->th, fc2->acb, fc2->bits, 64, nullptr, nullptr, nullptr, nullptr, xhat4,
+                              ARCQ_DT_F16, st),
+          "arcq_gelu_act_quant");
+    gemm(xhat4, *fc2, branch);
+    y = branch;
+  }
+  // the head reads the class token of every image only
+  const at::Tensor h = empty_cuda({B, D}, at::kHalf, dev);
+  check(arcq_add_layernorm_strided(x, y, gb[4 * depth], gb[4 * depth + 1], static_cast<float>(p->norm.eps), B, D, T * D, nullptr,
+                                   h.mutable_data_ptr(), st),
+        "arcq_add_layernorm");
+  return THPVariable_Wrap(at::linear(h, *hw, *hb));
+}
+
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+  try {
+    return F(self, args, n);
+  } catch (const Fail&) {
+    return nullptr;
+  } catch (const c10::OutOfMemoryError& e) {
+    PyErr_SetString(g_oom_error, e.what_without_backtrace());
+    return nullptr;
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+}
+#define ARCQ_METHOD(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&guarded<f>)), METH_FASTCALL, nullptr}
+PyMethodDef g_methods[] = {ARCQ_METHOD(linear), ARCQ_METHOD(quantize_activation), ARCQ_METHOD(dequant), ARCQ_METHOD(vit_plan),
+                           ARCQ_METHOD(vit_forward), {nullptr, nullptr, 0, nullptr}};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_arcq_host", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__arcq_host() {
+  for (int i = 0; i < kKeys; ++i)
+    if ((g_key[i] = PyUnicode_InternFromString(kKeyNames[i])) == nullptr) return nullptr;
+  PyObject* const torch = PyImport_ImportModule("torch");
+  if (torch == nullptr || (g_oom_error = PyObject_GetAttrString(torch, "OutOfMemoryError")) == nullptr) return nullptr;
+  Py_DECREF(torch);
+  return PyModule_Create(&g_module);
+}

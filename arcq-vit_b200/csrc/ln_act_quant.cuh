@@ -21,6 +21,7 @@
 #include "ptx.cuh"
 #include "act_quant.cuh"
 #include "group_quant.cuh"
+#include "codes.cuh"
 #include "add_layernorm.cuh"
 
 namespace arcq {
@@ -38,8 +39,13 @@ __global__ void __launch_bounds__(kLnqThreads, 4)
                                    const __half* __restrict__ y, const float* __restrict__ gamma,
                                    const float* __restrict__ beta, float eps, long long M,
                                    const float* __restrict__ thresholds, const float* __restrict__ codebook,
-                                   __half* __restrict__ sum_out, __half* __restrict__ h_out) {
+                                   __half* __restrict__ sum_out, __half* __restrict__ h_out,
+                                   const __grid_constant__ UnpackJobs jobs) {
   pdl_launch_dependents();   // the next kernel of the stream may start its set-up
+  if (static_cast<int>(blockIdx.x) < jobs.blocks) {
+    unpack_jobs_block(jobs);
+    return;
+  }
 
   constexpr int L = 1 << BITS;
   constexpr int K = LANES * 24, G = K / 64, kRowsPerWarp = 32 / LANES, kRowsPerPass = 4 * kRowsPerWarp;
@@ -58,7 +64,7 @@ __global__ void __launch_bounds__(kLnqThreads, 4)
 
   const long long total_groups = M * G;
   const long long tiles = (total_groups + kLnqThreads - 1) / kLnqThreads;
-  for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+  for (long long tile = blockIdx.x - jobs.blocks; tile < tiles; tile += gridDim.x - jobs.blocks) {
     const long long gi0 = tile * kLnqThreads;
     const int ngroups = static_cast<int>(min(static_cast<long long>(kLnqThreads), total_groups - gi0));
     const long long r_first = gi0 / G;
@@ -129,8 +135,13 @@ __global__ void __launch_bounds__(kLnqRowsThreads) add_layernorm_act_quant_rows_
                                                                           const float* __restrict__ codebook,
                                                                           __half* __restrict__ sum_out,
                                                                           __half* __restrict__ h_out,
-                                                                          __half* __restrict__ xhat) {
+                                                                          __half* __restrict__ xhat,
+                                                                          const __grid_constant__ UnpackJobs jobs) {
   pdl_launch_dependents();
+  if (static_cast<int>(blockIdx.x) < jobs.blocks) {
+    unpack_jobs_block(jobs);
+    return;
+  }
   constexpr int L = 1 << BITS;
   constexpr int K = LANES * 24, G = K / 64, kRowsPerWarp = 32 / LANES, kRows = 4 * kRowsPerWarp;   // rows per tile
   constexpr int kSlots = kRows * G * 8;            // (group, lane-of-eight) pairs per tile: 384 for every width
@@ -149,7 +160,7 @@ __global__ void __launch_bounds__(kLnqRowsThreads) add_layernorm_act_quant_rows_
   pdl_wait();                // everything above is the layer's constants; x and y may be the previous kernel's output
 
   const int l8 = lane & 7, octet_base = lane & ~7;
-  for (long long row0 = static_cast<long long>(blockIdx.x) * kRows; row0 < M; row0 += static_cast<long long>(gridDim.x) * kRows) {
+  for (long long row0 = static_cast<long long>(blockIdx.x - jobs.blocks) * kRows; row0 < M; row0 += static_cast<long long>(gridDim.x - jobs.blocks) * kRows) {
     // ---- phase 1 (warps 0-3): one row per LANES lanes
     if (warp < 4) {
       const int local = warp * kRowsPerWarp + sub;

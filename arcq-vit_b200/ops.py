@@ -51,6 +51,10 @@ def quantize_activation(x: torch.Tensor, thresholds: torch.Tensor, codebook: tor
     Same contract as the reference's ``quantize_activation`` (arcq_activation_kernel.cu:188-237),
     except that fp16 / bf16 inputs are read as they are instead of being copied to fp32 first.
     """
+    if group_size == 64:
+        out = _cabi.host().quantize_activation(x, thresholds, codebook, bits, want_code_sum, pre_gelu)
+        if out is not None:
+            return out
     lib = _cabi.load()
     if x.dim() != 2:
         raise RuntimeError(f"x must be 2-D, got shape {tuple(x.shape)}")
@@ -383,6 +387,10 @@ def dequant(packed, center, scale, code_sum, codebook, bits: int, group_size: in
     """Packed codes + statistics -> [R, K] matrix; what the reference's ``unpack_weight_triton``
     (arcq_packed_triton.py:77-120) writes.  ``out``: write into this buffer (first R*K elements) instead
     of allocating, as the reference does with its ``_weight_buffer``."""
+    if out is None and group_size == 64 and out_dtype in (torch.float16, torch.float32):
+        made = _cabi.host().dequant(packed, center, scale, code_sum, codebook, bits, out_dtype == torch.float32)
+        if made is not None:
+            return made
     lib = _cabi.load()
     packed = _dev(packed, "packed", torch.uint8)
     center, scale, code_sum, codebook = (_dev(t, "stats", torch.float32) for t in (center, scale, code_sum, codebook))

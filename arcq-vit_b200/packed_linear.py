@@ -11,11 +11,10 @@ contract of the reference's packed layers:
   methods/fair_qat_framework/fair_qat/arcq_packed_on_the_fly.py:93-169.  Built from buffers;
   ``forward`` returns fp16 ("half chain").
 
-Both forwards are launches behind the C ABI: the activation quantizer (packed codes + per-group
-statistics, or the fp16 reconstruction) and a tcgen05 GEMM -- with the weight rebuilt inside the
-kernel, or unpacked by a third launch on a side stream while the previous layer runs (``staging.py``);
-the routes give the same bits.  There is no Triton, no cuBLAS and no CPU path; without the built
-library the forward raises.
+Both forwards are two launches behind one native call (``csrc/host_ext.cpp``): the activation quantizer, which unpacks the
+weight into an fp16 scratch matrix with blocks of its own, and a tcgen05 GEMM.  The other routes -- the weight rebuilt
+inside the GEMM, or unpacked on a side stream while the previous layer runs (``staging.py``) -- give the same bits.
+There is no Triton, no cuBLAS and no CPU path; without the built library the forward raises.
 
 Added on this side of the boundary (the reference never loads its own packed
 checkpoints back): ``ARCQPackedLinear.from_state_dict`` / ``from_buffers``.
@@ -30,7 +29,7 @@ from typing import Optional, Tuple
 import torch
 import torch.nn as nn
 
-from . import ops
+from . import _cabi, ops
 from .packing import pack_codes, unpack_codes_u8
 
 _FORMATS = ("packed", "u8", "dequant_gemm")
@@ -203,6 +202,9 @@ class ARCQPackedLinear(_KeepsFp32Metadata):
                                        self.group_size, self.in_features, self.out_features, out_dtype)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        y = _cabi.host().linear(self._buffers, x, True, True, False, False)
+        if y is not None:
+            return y
         shape = x.shape
         if shape[-1] != self.in_features:
             raise ValueError(f"expected last dim {self.in_features}, got {shape[-1]}")
@@ -267,8 +269,10 @@ class ARCQPackedLinearOnTheFly(_KeepsFp32Metadata):
     #             then read by TMA.  Needs a WeightStager on the model (attached by this package's converters).
     #   "packed": rebuilt from the codes inside the GEMM kernel, never in HBM.
     #   "dense":  unpacked on the layer's own stream right before the GEMM (no overlap, no stager needed).
-    #   "auto":   staged when the model has a stager and the GEMM has at least WeightStager.min_rows rows, else packed.
-    # The three forms produce the same bits: the unpack kernel writes exactly the fp16 values the packed-weight
+    #   "auto":   unpacked by blocks of the quantizer's own launch into a scratch matrix of the call (one native call a
+    #             layer).  Inputs that call does not take (other dtypes or devices, non-contiguous) go on as "staged" when
+    #             the model has a stager and the GEMM has at least WeightStager.min_rows rows, else as "packed".
+    # All forms produce the same bits: the unpack kernel writes exactly the fp16 values the packed-weight
     # kernels rebuild on chip.
     weight_form = os.environ.get("ARCQ_WEIGHT_FORM", "auto")
     _scratch: dict = {}
@@ -302,8 +306,7 @@ class ARCQPackedLinearOnTheFly(_KeepsFp32Metadata):
         """True if ``forward(x_hat, pre_quantized=True)`` is available: the layer runs the two-kernel route whose
         GEMM reads the reconstructed activation, so a caller may produce that activation itself
         (``ops.add_layernorm_quant`` with this layer's ``activation_thresholds`` / ``activation_codebook``)."""
-        return (self.group_size == 64 and self.in_features <= 1024
-                and ops.packed_weight_gemm_supported(self.in_features, self.out_features, self.bits, self.group_size))
+        return self.group_size == 64 and self.in_features <= 1024 and self.out_features % 16 == 0
 
     def forward(self, x: torch.Tensor, pre_gelu: bool = False, pre_quantized: bool = False) -> torch.Tensor:
         """``pre_gelu=True``: x is the pre-activation of the GELU in front of this layer; the result
@@ -312,15 +315,22 @@ class ARCQPackedLinearOnTheFly(_KeepsFp32Metadata):
         ``takes_reconstructed_input``); the quantizer is skipped."""
         if pre_quantized and (pre_gelu or not self.takes_reconstructed_input()):
             raise ValueError("pre_quantized input is not available for this layer / combination")
+        if self.weight_form == "auto":
+            y = _cabi.host().linear(self._buffers, x, False, False, pre_gelu, pre_quantized)
+            if y is not None:
+                return y
         shape = x.shape
         if shape[-1] != self.in_features:
             raise ValueError(f"expected last dim {self.in_features}, got {shape[-1]}")
         x2 = x.reshape(-1, self.in_features).to(device=self.packed_weight_codes.device, dtype=torch.float16).contiguous()
         bias = self.bias_tensor if self.bias_tensor.numel() else None
-        if ops.packed_weight_gemm_supported(self.in_features, self.out_features, self.bits, self.group_size):
+        if self.group_size == 64 and self.out_features % 16 == 0:
             # the reference's own data flow: fp16 activation quantised and reconstructed (its step 2),
             # then weight unpack + contraction + bias (its steps 3-5) in one persistent kernel
             route = self._weight_route(x2.shape[0])
+            if route == "packed" and not ops.packed_weight_gemm_supported(self.in_features, self.out_features, self.bits,
+                                                                          self.group_size):
+                route = "dense"         # e.g. 3-bit rows of 72 bytes: the packed-weight kernels want multiples of 16
             if route == "staged":
                 w16, ready, prefetch = self._stager.stage(self)     # also arranges the next layer's unpack
             x_hat = x2 if pre_quantized else ops.quantize_activation_dequant(
@@ -340,7 +350,7 @@ class ARCQPackedLinearOnTheFly(_KeepsFp32Metadata):
                                            self.weight_code_sum, self.weight_codebook, bias, self.bits,
                                            self.group_size, torch.float16)
         else:
-            # shapes the persistent kernel does not take (e.g. 3-bit rows of 72 bytes): packed codes both sides
+            # output widths the persistent kernels do not take: packed codes on both sides
             packed_x, mu, sg, cs = ops.quantize_activation(x2, self.activation_thresholds, self.activation_codebook,
                                                            self.bits, self.group_size, True, pre_gelu)
             y = ops.arcq_linear_forward(packed_x, mu, sg, cs, self.packed_weight_codes, self.weight_center,

@@ -13,15 +13,17 @@ floating point (ordinary PyTorch ops).
 from __future__ import annotations
 
 import os
+import weakref
 from typing import Callable, Dict, List, Tuple
 
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import _cabi
 from . import codebook as cbk
 from .packed_linear import ARCQPackedLinear, ARCQPackedLinearOnTheFly
-from .staging import attach_weight_stager
+from .staging import WeightStager, attach_weight_stager
 
 # name -> (embed dim, heads, depth); MLP hidden = 4 * dim; 224x224 input, patch 16, 1000 classes
 DEIT_CONFIGS: Dict[str, Tuple[int, int, int]] = {
@@ -33,8 +35,9 @@ DEIT_CONFIGS: Dict[str, Tuple[int, int, int]] = {
 
 class Attention(nn.Module):
     # "kernel": this package's attention kernel (heads of 64, at most 256 tokens, fp16 on a GPU), which also runs
-    # proj's activation quantizer when proj can take a reconstructed input; "sdpa": the library attention.
-    implementation = os.environ.get("ARCQ_ATTENTION", "sdpa")
+    # proj's activation quantizer when proj can take a reconstructed input; "sdpa": the library attention; "auto": the
+    # library attention, inside the model's one-call forward where that applies.
+    implementation = os.environ.get("ARCQ_ATTENTION", "auto")
 
     def __init__(self, dim: int, heads: int):
         super().__init__()
@@ -125,6 +128,9 @@ class VisionTransformer(nn.Module):
         self.head = nn.Linear(dim, num_classes)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        y = self._forward_native(x)
+        if y is not None:
+            return y
         x = self.patch_embed(x)
         if x.is_cuda and x.dtype == torch.float16 and x.shape[-1] % 8 == 0 and self.cls_token.dtype == torch.float16:
             from . import ops
@@ -136,6 +142,26 @@ class VisionTransformer(nn.Module):
         for blk in self.blocks:
             x = blk(x)
         return self.head(self.norm(x)[:, 0])
+
+    def _forward_native(self, x: torch.Tensor):
+        """The whole forward as one native call that launches every kernel (``csrc/host_ext.cpp``), or None where it does
+        not apply: anything but an unmodified packed model (hooks, replaced modules, tuning switches) on fp16 CUDA images
+        without gradients.  Same kernels in the same order as the code below."""
+        if (not x.is_cuda or torch.is_grad_enabled() or len(self.blocks) == 0 or self.fuse_norm_quant != "auto"
+                or type(self) is not VisionTransformer or ARCQPackedLinearOnTheFly.weight_form != "auto"
+                or WeightStager.mode != "stream" or Attention.implementation != "auto" or _has_global_hooks()):
+            return None
+        plan = _PLANS.get(self)
+        y = None if plan is None else _cabi.host().vit_forward(plan, x)
+        if y is None and isinstance(getattr(getattr(self.blocks[0], "attn", None), "qkv", None), ARCQPackedLinearOnTheFly):
+            # no plan yet, or the modules it was made for have changed
+            plan = _make_plan(self)
+            if plan is None:
+                _PLANS.pop(self, None)
+                return None
+            _PLANS[self] = plan
+            y = _cabi.host().vit_forward(plan, x)
+        return y
 
     def _forward_fused_glue(self, x: torch.Tensor) -> torch.Tensor:
         """Same computation as the loop over blocks, with every residual add merged into the LayerNorm
@@ -167,6 +193,55 @@ class VisionTransformer(nn.Module):
             else:
                 x, h = ops.add_layernorm(x, m, self.norm)
         return self.head(h[:, 0])
+
+
+_PLANS: "weakref.WeakKeyDictionary[VisionTransformer, object]" = weakref.WeakKeyDictionary()
+
+
+def _has_global_hooks() -> bool:
+    m = torch.nn.modules.module
+    return bool(m._global_forward_hooks or m._global_forward_pre_hooks)
+
+
+def _make_plan(model: VisionTransformer):
+    """References to the module dictionaries a native forward reads (parameters, buffers), the modules it was made for
+    (checked on every call) and the hook dictionaries that have to be empty; None for a model it cannot run."""
+    watch, empty, blocks = [], [], []
+
+    def child(parent: nn.Module, name: str, kind: type):
+        m = parent._modules.get(name)
+        if type(m) is not kind:
+            raise LookupError(name)
+        watch.extend((parent._modules, name, m))
+        empty.extend((m._forward_hooks, m._forward_pre_hooks))
+        return m
+
+    def linear(parent: nn.Module, name: str):
+        m = child(parent, name, ARCQPackedLinearOnTheFly)
+        if m.group_size != 64 or m.__dict__.get("weight_form", "auto") != "auto" or not m.supports_pre_gelu:
+            raise LookupError(name)
+        return m._buffers
+
+    try:
+        patch = child(child(model, "patch_embed", PatchEmbed), "proj", nn.Conv2d)
+        dim, heads = model.embed_dim, model.num_heads
+        if dim not in (192, 384, 768) or dim != 64 * heads or patch.kernel_size[0] != patch.kernel_size[1] or patch.kernel_size[0] % 8:
+            return None
+        stack = child(model, "blocks", nn.ModuleList)
+        for i in range(len(stack)):
+            blk = child(stack, str(i), Block)
+            attn, mlp = child(blk, "attn", Attention), child(blk, "mlp", Mlp)
+            n1, n2 = child(blk, "norm1", nn.LayerNorm), child(blk, "norm2", nn.LayerNorm)
+            if attn.num_heads != heads or "implementation" in attn.__dict__:
+                return None
+            blocks.append((n1._parameters, float(n1.eps), n2._parameters, float(n2.eps), linear(attn, "qkv"), linear(attn, "proj"),
+                           linear(mlp, "fc1"), linear(mlp, "fc2")))
+        norm, head = child(model, "norm", nn.LayerNorm), child(model, "head", nn.Linear)
+    except LookupError:
+        return None
+    watch.extend((stack._modules, str(len(stack)), None))          # no block was appended
+    return _cabi.host().vit_plan(dim, heads, int(patch.kernel_size[0]), model._parameters, patch._parameters, head._parameters,
+                                 norm._parameters, float(norm.eps), blocks, watch, empty)
 
 
 def create_vit(name: str, seed: int = 0, num_classes: int = 1000) -> VisionTransformer:
@@ -286,6 +361,7 @@ class GraphedModel:
     same way at batch 1, scripts/benchmark_arcq_on_the_fly.py:223-231)."""
 
     def __init__(self, model: nn.Module, example: torch.Tensor, warmup: int = 3):
+        self.model = model            # the graph reads its parameters and scratch memory: keep them
         self.static_in = example.clone()
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())

@@ -137,6 +137,32 @@ int arcq_gelu_act_quant(const void* x, int x_dtype, int64_t M, int64_t K,
                         void* xhat_out, int xhat_dtype, void* stream);
 
 /*
+ * A packed weight to be unpacked by blocks of the activation path's kernels (what arcq_unpack_weight_f16 writes):
+ * packed [rows, K*bits/8], statistics fp32 [rows, K/64], out fp16 [rows, K], 16-byte aligned; group size 64.
+ * The linear that consumes the quantizer's output needs its weight next: unpacked beside the quantizer it costs no
+ * launch of its own.  Up to two jobs a call; `out` must not be read by any kernel still running before the call.
+ */
+typedef struct arcq_unpack_job {
+  const uint8_t* packed;
+  const float* mu;
+  const float* sigma;
+  const float* codesum;
+  const float* codebook;
+  void* out;
+  int64_t rows, K;
+  int bits;
+} arcq_unpack_job;
+
+/*
+ * arcq_act_quant (pre_gelu = 0) or arcq_gelu_act_quant (1) with reconstruction output only, plus unpack jobs: steps 2
+ * and 3 of ARCQPackedLinearOnTheFly.forward (FQ/fair_qat/arcq_packed_on_the_fly.py:143-158: dequant_activation_triton,
+ * unpack_weight_triton) in one launch.
+ */
+int arcq_act_quant_unpack(int pre_gelu, const void* x, int x_dtype, int64_t M, int64_t K, const float* thresholds,
+                          const float* codebook, int bits, int group_size, void* xhat_out, int xhat_dtype,
+                          const arcq_unpack_job* unpack, int n_unpack, void* stream);
+
+/*
  * Packed linear:  y[m,n] = bias[n] + sum_k A^[m,k] * W^[n,k]  with both operands
  * reconstructed from packed codes, A^ = mu_a + sigma_a*(cbA[ca] - Sa/gs) and
  * likewise W^, contracted on the tensor cores in fp16 with fp32 accumulation.
@@ -214,6 +240,11 @@ int arcq_packed_linear_static_scratch(const void* xhat, const uint8_t* packed_w,
 int arcq_add_layernorm(const void* x, const void* y, const float* gamma, const float* beta, float eps,
                        int64_t M, int64_t K, void* sum_out, void* h_out, void* stream);
 
+/* The same with input rows `ld` values apart (ld >= K, a multiple of 8); sum_out and h_out stay contiguous.  The final
+ * norm of a ViT runs on the class token of every image: ld = tokens * K. */
+int arcq_add_layernorm_strided(const void* x, const void* y, const float* gamma, const float* beta, float eps, int64_t M,
+                               int64_t K, int64_t ld, void* sum_out, void* h_out, void* stream);
+
 /*
  * arcq_add_layernorm followed by the activation quantizer of the packed linear that consumes the LayerNorm
  * output (timm Block.forward: norm1 -> attn.qkv, norm2 -> mlp.fc1), in one kernel:
@@ -226,6 +257,12 @@ int arcq_add_layernorm(const void* x, const void* y, const float* gamma, const f
 int arcq_add_layernorm_act_quant(const void* x, const void* y, const float* gamma, const float* beta, float eps,
                                  int64_t M, int64_t K, const float* thresholds, const float* codebook, int bits,
                                  int group_size, void* sum_out, void* h_out, void* xhat, void* stream);
+
+/* The same with unpack jobs (see arcq_unpack_job) taken along by the launch. */
+int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const float* gamma, const float* beta, float eps,
+                                        int64_t M, int64_t K, const float* thresholds, const float* codebook, int bits,
+                                        int group_size, void* sum_out, void* h_out, void* xhat,
+                                        const arcq_unpack_job* unpack, int n_unpack, void* stream);
 
 /*
  * Multi-head self-attention on the output of the packed qkv linear, for short sequences (T <= 256) and heads of 64:
