@@ -19,6 +19,7 @@ EXPORTS = (
     "arcq_version", "arcq_last_error_string", "arcq_device_status", "arcq_debug_trace", "arcq_debug_set_option", "arcq_debug_get_option", "arcq_debug_last_gemm_kernel", "arcq_debug_wait_timeout", "arcq_act_quant", "arcq_gelu_act_quant", "arcq_packed_gemm", "arcq_packed_weight_gemm", "arcq_dense_weight_gemm", "arcq_packed_linear_static_scratch", "arcq_add_layernorm", "arcq_add_layernorm_act_quant", "arcq_attention", "arcq_attention_act_quant", "arcq_patchify", "arcq_assemble_tokens",
     "arcq_unpack_codes", "arcq_pack_codes", "arcq_dequant", "arcq_unpack_weight_f16", "arcq_dense_weight_gemm_prefetch",
     "arcq_act_quant_unpack", "arcq_add_layernorm_act_quant_unpack", "arcq_add_layernorm_strided",
+    "arcq_dense_weight_gemm_unpack", "arcq_dense_weight_gemm_unpack_room", "arcq_unpack_beside_gemm", "arcq_dense_weight_gemm_gelu_quant",
 )
 
 _lib = None
@@ -64,6 +65,7 @@ def load() -> ctypes.CDLL:
     lib.arcq_dequant.argtypes = [vp, vp, vp, vp, vp, ci, ci, i64, i64, vp, ci, vp]
     lib.arcq_unpack_weight_f16.argtypes = [vp, vp, vp, vp, vp, ci, ci, i64, i64, vp, vp]
     lib.arcq_dense_weight_gemm_prefetch.argtypes = [vp, vp, vp, i64, i64, i64, vp, ci, vp, vp, vp, vp, vp, ci, ci, i64, i64, vp, vp]
+    lib.arcq_dense_weight_gemm_gelu_quant.argtypes = [vp, vp, vp, i64, i64, i64, vp, vp, ci, ci, vp, vp, ci, vp]
     for name in EXPORTS:
         getattr(lib, name)  # AttributeError here means header and library disagree
     _lib = lib
@@ -125,7 +127,8 @@ class option:
         return False
 
 
-GEMM_ONE_CTA_PACKED, GEMM_ONE_CTA_DENSE, GEMM_PAIR_PACKED, GEMM_PAIR_DENSE, GEMM_PAIR_DENSE_PREFETCH = 1, 2, 3, 4, 5
+E_UNSUPPORTED = -3
+GEMM_ONE_CTA_PACKED, GEMM_ONE_CTA_DENSE, GEMM_PAIR_PACKED, GEMM_PAIR_DENSE, GEMM_PAIR_DENSE_PREFETCH, GEMM_PAIR_DENSE_GELU_QUANT = 1, 2, 3, 4, 5, 6
 
 
 def last_gemm_kernel() -> int:

@@ -20,46 +20,35 @@
 namespace arcq {
 
 // Optional element-wise op applied to the input before it is quantised (fused from the preceding layer).
-// PRE = 1: exact GELU, 0.5*x*(1+erf(x/sqrt 2)) in fp32, then rounded to the input's element type -- the
-// value a separate GELU kernel would have stored -- so the quantizer sees the same numbers as unfused.
+// PRE = 1: exact (erf) GELU in fp32, then rounded to the input's element type -- the value a separate GELU kernel would have
+// stored -- so the quantizer sees the same numbers as unfused.
 template <typename T> __device__ __forceinline__ float round_to(float v);
 template <> __device__ __forceinline__ float round_to<float>(float v) { return v; }
 template <> __device__ __forceinline__ float round_to<__half>(float v) { return __half2float(__float2half_rn(v)); }
 template <> __device__ __forceinline__ float round_to<__nv_bfloat16>(float v) {
   return __bfloat162float(__float2bfloat16_rn(v));
 }
+// GELU of an fp16 value in fp32, in all kernels the same to the bit: x * (0.5 + x * R(x^2)) for |x| < 2, with
+// x * R(x^2) = erf(x / sqrt 2) / 2 and R of degree 7, fitted on Chebyshev nodes; erff beyond.  Over every fp16 input of that
+// range the fp16 result differs from the correctly rounded one for 3 inputs of 32 768 (0.5 x (1 + erff(x / sqrt 2)) in fp32: 3).
+constexpr float kGeluLimit = 2.0f;
+__device__ __forceinline__ float gelu_r(int k) {       // k is a constant wherever this is used
+  const float c[8] = {0.398942292f,    -0.0664903149f,  0.00997320935f, -0.0011866159f,
+                      0.000114711416f, -9.03896398e-06f, 5.35578579e-07f, -1.75760011e-08f};
+  return c[k];
+}
+__device__ __forceinline__ float gelu_large(float x) { return x * 0.5f * (1.0f + erff(x * 0.70710678118654752440f)); }
+__device__ __forceinline__ float gelu(float x) {
+  if (!(fabsf(x) < kGeluLimit)) return gelu_large(x);
+  const float s = __fmul_rn(x, x);
+  float r = gelu_r(7);
+#pragma unroll
+  for (int k = 6; k >= 0; --k) r = fmaf(r, s, gelu_r(k));
+  return __fmul_rn(x, fmaf(x, r, 0.5f));
+}
 template <typename T, int PRE> __device__ __forceinline__ float pre_op(float x) {
-  if (PRE == 1) return round_to<T>(x * 0.5f * (1.0f + erff(x * 0.70710678118654752440f)));
-  return x;
+  return PRE == 1 ? round_to<T>(gelu(x)) : x;
 }
-
-// Exact GELU, 0.5*x*(1+erf(x/sqrt 2)) in fp32, for code that all 32 lanes of a warp run together.
-// erf(z) for |z| < 0.9277 is z*P(z*z) with a degree-7 least-squares fit on Chebyshev nodes (max error 1e-11
-// before rounding); over every fp16 input in that range the GELU rounded to fp16 differs from the exactly
-// rounded one for 3 inputs of 31 360 -- the library erff gives 2.  Larger arguments call erff, but only when
-// some lane of the warp needs it: the branch is warp-uniform, so the common case (pre-activations of a few
-// units at most) never executes the long path.  Each element's result depends on its own value only.
-__device__ __forceinline__ float gelu_warp(float x) {
-  const float z = x * 0.70710678118654752440f;
-  const float s = z * z;
-  float r = -1.0267135621688794e-05f;
-  r = fmaf(r, s, 0.00011447568977018818f);
-  r = fmaf(r, s, -0.0008505592122673988f);
-  r = fmaf(r, s, 0.005222289357334375f);
-  r = fmaf(r, s, -0.026865806430578232f);
-  r = fmaf(r, s, 0.11283788084983826f);
-  r = fmaf(r, s, -0.37612637877464294f);
-  r = fmaf(r, s, 1.128379225730896f);
-  float e = z * r;
-  const bool big = !(fabsf(z) < 0.9277f);
-  if (__any_sync(0xffffffffu, big)) {
-    const float el = erff(z);
-    e = big ? el : e;
-  }
-  return x * 0.5f * (1.0f + e);
-}
-// The same, rounded to the element type T: the value a separate GELU kernel would have stored.
-template <typename T> __device__ __forceinline__ float gelu_rounded_warp(float x) { return round_to<T>(gelu_warp(x)); }
 
 // Sum of the value held by the 8 lanes of an octet, lane 0 first, as a chain of fp32 additions.
 __device__ __forceinline__ float octet_chain_sum(float p, int octet_base) {

@@ -81,7 +81,7 @@ enum Opt {
   O_WS_BN, O_WS_SA, O_WS_WS, O_WS_STATIONARY, O_WS_NBB, O_WS_GRID, O_WS_TMA_STORE, O_WS_ROTATE,
   O_ACT_QUANT_V1, O_ACT_QUANT_V2, O_LN_PLAIN,
   O_PAIR, O_PAIR_MIN_M, O_PAIR_BN, O_PAIR_SA, O_PAIR_KS, O_PAIR_NBB, O_PAIR_LUT, O_PAIR_PAIRS, O_PAIR_STATIONARY,
-  O_PAIR_WS, O_LNQ_SMALL, O_AQ2_MIN_GROUPS, O_PDL, O_POLL_LIMIT, O_SPIN_LIMIT, O_COUNT
+  O_PAIR_WS, O_LNQ_SMALL, O_AQ2_MIN_GROUPS, O_PDL, O_GELU_GEMM, O_GEMM_UNPACK, O_POLL_LIMIT, O_SPIN_LIMIT, O_COUNT
 };
 struct OptDef { const char* name; int dflt; };
 const OptDef kOptDefs[O_COUNT] = {
@@ -91,6 +91,7 @@ const OptDef kOptDefs[O_COUNT] = {
     {"ARCQ_PAIR", 1},         {"ARCQ_PAIR_MIN_M", 1024},  {"ARCQ_PAIR_BN", 0},     {"ARCQ_PAIR_SA", 0},
     {"ARCQ_PAIR_KS", 0},      {"ARCQ_PAIR_NBB", 0},       {"ARCQ_PAIR_LUT", 0},    {"ARCQ_PAIR_PAIRS", 0},
     {"ARCQ_PAIR_STATIONARY", -1}, {"ARCQ_PAIR_WS", 0}, {"ARCQ_LNQ_SMALL", 1}, {"ARCQ_AQ2_MIN_GROUPS", 0}, {"ARCQ_PDL", 1},
+    {"ARCQ_GELU_GEMM", -1}, {"ARCQ_GEMM_UNPACK", 1},
     {"ARCQ_POLL_LIMIT", 1 << 21}, {"ARCQ_SPIN_LIMIT", 1 << 25},
 };
 int g_opt[O_COUNT];
@@ -650,6 +651,66 @@ bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32,
   return true;
 }
 
+// Slab width, stages and grid of the form with GELU and quantizer in its epilogue; false: none fits.
+bool choose_pair_quant_config(long long M, long long N, long long K, PairDenseConfig* c) {
+  if (opt(O_PAIR) == 0) return false;
+  const int G = static_cast<int>(K / 64);
+  const long long tiles_m = (M + arcq::kPairTileM - 1) / arcq::kPairTileM;
+  int max_pairs = max_resident_dense_pairs(kSmemBudget + 1024);
+  if (opt(O_PAIR_PAIRS) > 0 && opt(O_PAIR_PAIRS) < max_pairs) max_pairs = opt(O_PAIR_PAIRS);
+  static const int cand[] = {192, 128, 64};                  // whole groups, at most one per epilogue warp of a lane quarter
+  double best_cost = 0;
+  bool found = false;
+  for (int bn : cand) {
+    if (N % bn != 0 || (opt(O_PAIR_BN) > 0 && bn != opt(O_PAIR_BN))) continue;
+    const long long slabs = N / bn;
+    if (slabs > max_pairs) continue;
+    long long per = max_pairs / slabs;
+    if (per > tiles_m) per = tiles_m;
+    const long long tiles_pp = (tiles_m + per - 1) / per;
+    // The epilogue bounds every tile: one, two or three warps per scheduler share its issue slots (a single tile of
+    // 64 / 128 / 192 columns, K = 384: 8.7 / 9.8 / 11.4 us).
+    const double cost = tiles_pp * (2.5 + 0.9 * (bn / 64));
+    if (found && cost >= best_cost) continue;
+    for (int stationary = 1; stationary >= 0; --stationary) {
+      if (stationary && (G > 32 || tiles_pp < 3)) continue;    // too few tiles to pay for loading the whole slab first
+      PairDenseConfig k = {};
+      k.bn = bn; k.pairs = static_cast<int>(slabs * per); k.stationary = stationary;
+      k.ks = (G % 2 == 0) ? 2 : (G % 3 == 0) ? 3 : 1;
+      bool fits = false;
+      for (int sa = 8 / k.ks; sa >= 2 && !fits; --sa) {
+        const size_t need = arcq::pair_dense_smem_layout(bn, sa, k.ks, G, stationary != 0, true).total;
+        if (need <= kSmemBudget) { k.sa = sa; k.smem = need + 1024; fits = true; }
+      }
+      if (!fits || (stationary && k.sa * k.ks < 4)) continue;
+      *c = k;
+      best_cost = cost;
+      found = true;
+      break;
+    }
+  }
+  return found;
+}
+
+// Small inputs, where most SMs would get no 128-group tile, take the twelve-warp form of LayerNorm + quantizer (48 groups per
+// block, lower latency).  Both forms give the same bits.  The line is where they measured equal: 4 137 groups 3.4 against 5.9 us,
+// 8 274 groups 6.5 against 5.6 us, 18 912 groups 9.8 against 6.0 us.
+bool small_layernorm_quant(long long M, long long K) {
+  return M * (K / 64) < static_cast<long long>(sm_count()) * 48 && opt(O_LNQ_SMALL) != 0;
+}
+
+// fc1 with GELU and quantizer in its epilogue, or GEMM and quantizer kernel?  Whole forwards through a graph (two kernels /
+// one): its 12 epilogue warps hide latency worse than the quantizer kernel's 16, so it pays where the tiles are one round (DeiT-S
+// batch 6 / 8: 714 -> 676, 724 -> 679 us; DeiT-T batch 16: 656 -> 618) but not below five row tiles (DeiT-T batch 2: 449 ->
+// 463), where the products under it are long (DeiT-B batch 4: 874 -> 821 us) or where the matrix between the two no longer stays
+// in L2 (DeiT-S batch 128: 2722 -> 2618 us, DeiT-B: 7341 -> 6902); in between the rounds eat it (DeiT-S batch 64: 1540 -> 1588).
+bool choose_gelu_quant(long long M, long long N, long long K, PairDenseConfig* pc) {
+  const int force = opt(O_GELU_GEMM);
+  if (force == 0 || N % 64 != 0 || !choose_pair_quant_config(M, N, K, pc)) return false;
+  const bool one_round = 1ll * pc->pairs * pc->bn >= (M + arcq::kPairTileM - 1) / arcq::kPairTileM * N;
+  return force > 0 || K >= 768 || M >= 20000 || (M > 1024 && one_round);
+}
+
 }  // namespace
 
 extern "C" {
@@ -710,7 +771,7 @@ int arcq_device_status(void) {
 
 // The unpack jobs of a call as kernel argument.  Blocks of 128 threads or more, each thread taking four 16-byte chunks a
 // round: enough blocks for one round, two per SM at most (they share the SMs with the kernel's own blocks).
-static int make_unpack_jobs(const arcq_unpack_job* jobs, int n, arcq::UnpackJobs* out) {
+static int make_unpack_jobs(const arcq_unpack_job* jobs, int n, arcq::UnpackJobs* out, int max_blocks = 0) {
   *out = arcq::UnpackJobs{};
   if (n == 0) return ARCQ_OK;
   if (jobs == nullptr || n < 0 || n > 2) return fail(ARCQ_E_BAD_ARG, "between 0 and 2 unpack jobs");
@@ -725,7 +786,7 @@ static int make_unpack_jobs(const arcq_unpack_job* jobs, int n, arcq::UnpackJobs
                                         static_cast<long long>(j.rows), static_cast<int>(j.K), j.bits};
     chunks += j.rows * (j.K / 8);
   }
-  const long long want = (chunks + 511) / 512, cap = 2ll * sm_count();
+  const long long want = (chunks + 511) / 512, cap = max_blocks > 0 ? max_blocks : 2ll * sm_count();
   out->blocks = static_cast<int>(want < cap ? want : cap);
   return ARCQ_OK;
 }
@@ -960,7 +1021,8 @@ static int launch_pair_gemm(const PairConfig& cfg, const void* xhat, const void*
 
 static int launch_pair_dense_gemm(const PairDenseConfig& cfg, const void* xhat, const void* w16, const float* bias,
                                   int64_t M, int64_t N, int64_t K, void* y, int y_dtype, void* stream,
-                                  const arcq::UnpackWeightJob* next = nullptr) {
+                                  const arcq::UnpackWeightJob* next = nullptr, const arcq::UnpackJobs& jobs = {},
+                                  const float* q_thresholds = nullptr, const float* q_codebook = nullptr, int q_bits = 0) {
   CUtensorMap tm_a, tm_w, tm_y;
   if (!make_tensor_map_2d(&tm_a, xhat, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, static_cast<uint64_t>(M),
                           static_cast<uint64_t>(K), 64, arcq::kTileM, CU_TENSOR_MAP_SWIZZLE_128B))
@@ -968,12 +1030,16 @@ static int launch_pair_dense_gemm(const PairDenseConfig& cfg, const void* xhat, 
   if (!make_tensor_map_2d(&tm_w, w16, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, static_cast<uint64_t>(N),
                           static_cast<uint64_t>(K), 64, cfg.bn / 2, CU_TENSOR_MAP_SWIZZLE_128B))
     return fail(ARCQ_E_CUDA, "cuTensorMapEncodeTiled failed for the weight matrix");
-  const int out_cw = (y_dtype == ARCQ_DT_F32) ? 16 : 32;
+  // 64 bytes of a row per store; a whole group of 64 values in the quantizer form
+  const int out_cw = q_bits != 0 ? 64 : (y_dtype == ARCQ_DT_F32) ? 16 : 32;
   if (!make_tensor_map_2d(&tm_y, y, (y_dtype == ARCQ_DT_F32) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
                           (y_dtype == ARCQ_DT_F32) ? 4 : 2, static_cast<uint64_t>(M), static_cast<uint64_t>(N),
-                          out_cw, 32, CU_TENSOR_MAP_SWIZZLE_64B))
+                          out_cw, 32, q_bits != 0 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B))
     return fail(ARCQ_E_CUDA, "cuTensorMapEncodeTiled failed for the output matrix");
   arcq::PairDenseParams p;
+  p.pairs = cfg.pairs;
+  p.thresholds = q_thresholds;
+  p.codebook = q_codebook;
   p.bias = bias;
   p.M = static_cast<int>(M); p.N = static_cast<int>(N); p.K = static_cast<int>(K); p.G = static_cast<int>(K / 64);
   p.bn = cfg.bn; p.sa = cfg.sa; p.ks = cfg.ks;
@@ -984,8 +1050,34 @@ static int launch_pair_dense_gemm(const PairDenseConfig& cfg, const void* xhat, 
   if (p.status == nullptr) return fail(ARCQ_E_CUDA, "device status word not reachable");
   p.next = arcq::UnpackWeightJob{};
   if (next != nullptr) p.next = *next;
-  const unsigned grid = static_cast<unsigned>(2 * cfg.pairs);
+  const unsigned grid = static_cast<unsigned>(2 * cfg.pairs + jobs.blocks);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (q_bits != 0) {
+    auto launch = [&](auto kernel, int* done_dev) {
+      int dev = 0;
+      cudaGetDevice(&dev);
+      if (*done_dev != dev) {                   // shared-memory ceiling, once per (thread, device)
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBudget + 1024));
+        if (e != cudaSuccess) return e;
+        *done_dev = dev;
+      }
+      launch_pdl(kernel, grid, arcq::kPairQuantThreads, cfg.smem, st, tm_a, tm_w, tm_y, p, jobs);
+      return cudaGetLastError();
+    };
+    static thread_local int done[6] = {-1, -1, -1, -1, -1, -1};
+    cudaError_t e = cudaSuccess;
+    if (cfg.stationary)
+      e = q_bits == 4 ? launch(arcq::dense_weight_gemm_pair_kernel<true, false, 4>, done)
+          : q_bits == 3 ? launch(arcq::dense_weight_gemm_pair_kernel<true, false, 3>, done + 1)
+                        : launch(arcq::dense_weight_gemm_pair_kernel<true, false, 2>, done + 2);
+    else
+      e = q_bits == 4 ? launch(arcq::dense_weight_gemm_pair_kernel<false, false, 4>, done + 3)
+          : q_bits == 3 ? launch(arcq::dense_weight_gemm_pair_kernel<false, false, 3>, done + 4)
+                        : launch(arcq::dense_weight_gemm_pair_kernel<false, false, 2>, done + 5);
+    g_last_gemm_kernel = ARCQ_GEMM_PAIR_DENSE_GELU_QUANT;
+    if (e != cudaSuccess) return cuda_fail(e, "dense_weight_gemm_gelu_quant launch");
+    return ARCQ_OK;
+  }
   if (next != nullptr) {
     static thread_local int done_dev = -1;      // the prefetch form's shared-memory ceiling, once per (thread, device)
     int dev = 0;
@@ -998,13 +1090,13 @@ static int launch_pair_dense_gemm(const PairDenseConfig& cfg, const void* xhat, 
       done_dev = dev;
     }
     if (cfg.stationary)
-      launch_pdl(arcq::dense_weight_gemm_pair_kernel<true, true>, grid, arcq::kPairDenseThreads, cfg.smem, st, tm_a, tm_w, tm_y, p);
+      launch_pdl(arcq::dense_weight_gemm_pair_kernel<true, true>, grid, arcq::kPairDenseThreads, cfg.smem, st, tm_a, tm_w, tm_y, p, jobs);
     else
-      launch_pdl(arcq::dense_weight_gemm_pair_kernel<false, true>, grid, arcq::kPairDenseThreads, cfg.smem, st, tm_a, tm_w, tm_y, p);
+      launch_pdl(arcq::dense_weight_gemm_pair_kernel<false, true>, grid, arcq::kPairDenseThreads, cfg.smem, st, tm_a, tm_w, tm_y, p, jobs);
   } else if (cfg.stationary) {
-    launch_pdl(arcq::dense_weight_gemm_pair_kernel<true>, grid, arcq::kPairDenseThreads, cfg.smem, st, tm_a, tm_w, tm_y, p);
+    launch_pdl(arcq::dense_weight_gemm_pair_kernel<true>, grid, arcq::kPairDenseThreads, cfg.smem, st, tm_a, tm_w, tm_y, p, jobs);
   } else {
-    launch_pdl(arcq::dense_weight_gemm_pair_kernel<false>, grid, arcq::kPairDenseThreads, cfg.smem, st, tm_a, tm_w, tm_y, p);
+    launch_pdl(arcq::dense_weight_gemm_pair_kernel<false>, grid, arcq::kPairDenseThreads, cfg.smem, st, tm_a, tm_w, tm_y, p, jobs);
   }
   g_last_gemm_kernel = next != nullptr ? ARCQ_GEMM_PAIR_DENSE_PREFETCH : ARCQ_GEMM_PAIR_DENSE;
   const cudaError_t e = cudaGetLastError();
@@ -1040,8 +1132,16 @@ int arcq_packed_weight_gemm(const void* xhat, const uint8_t* packed_w, const flo
                         stream);
 }
 
-int arcq_dense_weight_gemm(const void* xhat, const void* w16, const float* bias, int64_t M, int64_t N, int64_t K,
-                           void* y, int y_dtype, void* stream) {
+// Unpack jobs for the SMs that `pairs` CTA pairs leave idle, in whole pairs of blocks.
+static int make_idle_jobs(const arcq_unpack_job* unpack, int n_unpack, int pairs, arcq::UnpackJobs* jobs) {
+  const int idle = sm_count() - 2 * pairs;
+  const int rc = make_unpack_jobs(unpack, n_unpack, jobs, idle > 2 ? idle : 2);
+  jobs->blocks = (jobs->blocks + 1) / 2 * 2;
+  return rc;
+}
+
+static int dense_weight_gemm_impl(const void* xhat, const void* w16, const float* bias, int64_t M, int64_t N, int64_t K,
+                                  void* y, int y_dtype, const arcq_unpack_job* unpack, int n_unpack, void* stream) {
   if (!xhat || !w16 || !y) return fail(ARCQ_E_BAD_ARG, "null pointer argument");
   if (y_dtype != ARCQ_DT_F16 && y_dtype != ARCQ_DT_F32) return fail(ARCQ_E_BAD_ARG, "y_dtype must be f16 or f32");
   if (M < 0 || N <= 0 || K <= 0) return fail(ARCQ_E_BAD_SHAPE, "bad shape M=%lld N=%lld K=%lld", (long long)M,
@@ -1051,11 +1151,68 @@ int arcq_dense_weight_gemm(const void* xhat, const void* w16, const float* bias,
   if (M > 0x7fffffffLL || N > 0x7fffffffLL || K > (1 << 20)) return fail(ARCQ_E_TOO_LARGE, "shape too large");
   if (!aligned(xhat, 16) || !aligned(w16, 16) || !aligned(y, 16))
     return fail(ARCQ_E_ALIGN, "xhat, w16 and y must be 16-byte aligned");
+  if (M == 0 && n_unpack == 0) return ARCQ_OK;
+  PairDenseConfig pc;
+  if (M > 0 && choose_pair_dense_config(M, N, K, y_dtype == ARCQ_DT_F32, &pc)) {
+    arcq::UnpackJobs jobs;
+    if (const int rc = make_idle_jobs(unpack, n_unpack, pc.pairs, &jobs)) return rc;
+    return launch_pair_dense_gemm(pc, xhat, w16, bias, M, N, K, y, y_dtype, stream, nullptr, jobs);
+  }
+  // no pair configuration (or nothing to multiply): the unpack by its own kernel
+  for (int i = 0; i < n_unpack; ++i) {
+    const arcq_unpack_job& j = unpack[i];
+    if (const int rc = arcq_unpack_weight_f16(j.packed, j.mu, j.sigma, j.codesum, j.codebook, j.bits, 64, j.rows, j.K, j.out, stream)) return rc;
+  }
+  if (M == 0) return ARCQ_OK;
+  return launch_ws_gemm(true, xhat, w16, nullptr, nullptr, nullptr, nullptr, bias, 4, M, N, K, y, y_dtype, stream);
+}
+
+int arcq_dense_weight_gemm(const void* xhat, const void* w16, const float* bias, int64_t M, int64_t N, int64_t K,
+                           void* y, int y_dtype, void* stream) {
+  return dense_weight_gemm_impl(xhat, w16, bias, M, N, K, y, y_dtype, nullptr, 0, stream);
+}
+
+int arcq_dense_weight_gemm_unpack(const void* xhat, const void* w16, const float* bias, int64_t M, int64_t N, int64_t K,
+                                  void* y, int y_dtype, const arcq_unpack_job* unpack, int n_unpack, void* stream) {
+  if (n_unpack < 0 || n_unpack > 2 || (n_unpack > 0 && unpack == nullptr)) return fail(ARCQ_E_BAD_ARG, "between 0 and 2 unpack jobs");
+  return dense_weight_gemm_impl(xhat, w16, bias, M, N, K, y, y_dtype, unpack, n_unpack, stream);
+}
+
+// Unpack jobs beside GEMMs or beside the LayerNorm + quantizer: where that takes its latency form, blocks added to it lengthen
+// it, and where it takes the tile form they do not.  Whole forwards through a graph (LayerNorm / GEMM): DeiT-S batch 1 554 / 506,
+// batch 6 714 / 628, batch 8 724 / 772 us; DeiT-T batch 12 613 / 570, batch 16 656 / 689 us; DeiT-B batch 3 898 / 793, batch 4
+// 867 / 923 us: the line between the two forms runs through each of these.
+int arcq_unpack_beside_gemm(int64_t M, int64_t width) { return small_layernorm_quant(M, width) && opt(O_GEMM_UNPACK) != 0 ? 1 : 0; }
+
+int64_t arcq_dense_weight_gemm_unpack_room(int64_t M, int64_t N, int64_t K, int gelu_quant) {
+  PairDenseConfig pc;
+  if (M <= 0 || N <= 0 || K <= 0 || K % 64 != 0 || N % 16 != 0 || M > 0x7fffffffLL || N > 0x7fffffffLL || K > (1 << 20)) return 0;
+  if (!(gelu_quant ? choose_gelu_quant(M, N, K, &pc) : choose_pair_dense_config(M, N, K, false, &pc))) return 0;
+  // five rounds of four chunks of eight values per thread: about what a GEMM of a few hundred rows takes itself
+  const long long idle = sm_count() - 2 * pc.pairs;
+  return idle > 0 ? idle * arcq::kPairDenseThreads * 160 : 0;
+}
+
+int arcq_dense_weight_gemm_gelu_quant(const void* xhat, const void* w16, const float* bias, int64_t M, int64_t N, int64_t K,
+                                      const float* thresholds, const float* codebook, int bits, int group_size, void* out,
+                                      const arcq_unpack_job* unpack, int n_unpack, void* stream) {
+  if (!xhat || !w16 || !out || !thresholds || !codebook) return fail(ARCQ_E_BAD_ARG, "null pointer argument");
+  if (bits < 2 || bits > 4) return fail(ARCQ_E_BAD_ARG, "bits must be 2, 3 or 4, got %d", bits);
+  if (group_size != 64) return fail(ARCQ_E_UNSUPPORTED, "group_size %d: only 64 is built", group_size);
+  if (M < 0 || N <= 0 || K <= 0) return fail(ARCQ_E_BAD_SHAPE, "bad shape M=%lld N=%lld K=%lld", (long long)M,
+                                              (long long)N, (long long)K);
+  if (K % 64 != 0 || N % 64 != 0) return fail(ARCQ_E_UNSUPPORTED, "K=%lld, N=%lld: this entry point needs multiples of 64", (long long)K, (long long)N);
+  if (M > 0x7fffffffLL || N > 0x7fffffffLL || K > (1 << 20)) return fail(ARCQ_E_TOO_LARGE, "shape too large");
+  if (!aligned(xhat, 16) || !aligned(w16, 16) || !aligned(out, 16))
+    return fail(ARCQ_E_ALIGN, "xhat, w16 and out must be 16-byte aligned");
+  if (M == 0 && n_unpack != 0) return fail(ARCQ_E_BAD_SHAPE, "no rows to unpack weights beside");
   if (M == 0) return ARCQ_OK;
   PairDenseConfig pc;
-  if (choose_pair_dense_config(M, N, K, y_dtype == ARCQ_DT_F32, &pc))
-    return launch_pair_dense_gemm(pc, xhat, w16, bias, M, N, K, y, y_dtype, stream);
-  return launch_ws_gemm(true, xhat, w16, nullptr, nullptr, nullptr, nullptr, bias, 4, M, N, K, y, y_dtype, stream);
+  if (!choose_gelu_quant(M, N, K, &pc))
+    return fail(ARCQ_E_UNSUPPORTED, "M=%lld, N=%lld, K=%lld: left to arcq_dense_weight_gemm and arcq_gelu_act_quant", (long long)M, (long long)N, (long long)K);
+  arcq::UnpackJobs jobs;
+  if (const int rc = make_idle_jobs(unpack, n_unpack, pc.pairs, &jobs)) return rc;
+  return launch_pair_dense_gemm(pc, xhat, w16, bias, M, N, K, out, ARCQ_DT_F16, stream, nullptr, jobs, thresholds, codebook, bits);
 }
 
 int arcq_dense_weight_gemm_prefetch(const void* xhat, const void* w16, const float* bias, int64_t M, int64_t N,
@@ -1159,10 +1316,7 @@ int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const floa
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int G = static_cast<int>(K / 64);
   {
-    // Small inputs, where most SMs would get no 128-group tile: the twelve-warp form (48 groups per block, lower
-    // latency).  Both forms give the same bits.  The line is where they measured equal: 4 137 groups 3.4 against 5.9 us,
-    // 8 274 groups 6.5 against 5.6 us, 18 912 groups 9.8 against 6.0 us.
-    const bool small = M * G < static_cast<long long>(sm_count()) * 48 && opt(O_LNQ_SMALL) != 0;
+    const bool small = small_layernorm_quant(M, K);
     if (small) {
       const __half *xs = static_cast<const __half*>(x), *ys = static_cast<const __half*>(y);
       __half *so2 = static_cast<__half*>(sum_out), *ho2 = static_cast<__half*>(h_out), *xo2 = static_cast<__half*>(xhat);

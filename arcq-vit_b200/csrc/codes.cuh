@@ -170,25 +170,29 @@ struct UnpackJobs {
   UnpackWeightJob job[2];
   int blocks;                // 0: none
 };
-__device__ __forceinline__ void unpack_jobs_block(const UnpackJobs& u) {
-  __shared__ __half s_ucb[2][16];
+// `block` of u.blocks; s_ucb: 32 values of shared memory.
+__device__ __forceinline__ void unpack_jobs_run(const UnpackJobs& u, int block, __half* s_ucb) {
   const int tid = threadIdx.x;
   if (tid < 32) {
     const UnpackWeightJob& j = u.job[tid >> 4];
     const int i = tid & 15;
-    s_ucb[tid >> 4][i] = __float2half_rn(j.packed != nullptr && i < (1 << j.bits) ? __ldg(j.codebook + i) : 0.0f);
+    s_ucb[tid] = __float2half_rn(j.packed != nullptr && i < (1 << j.bits) ? __ldg(j.codebook + i) : 0.0f);
   }
   __syncthreads();
   pdl_wait();                // the matrices written here may still be read by the kernel before this one
-  const long long first = static_cast<long long>(blockIdx.x) * blockDim.x + tid, stride = static_cast<long long>(u.blocks) * blockDim.x;
+  const long long first = static_cast<long long>(block) * blockDim.x + tid, stride = static_cast<long long>(u.blocks) * blockDim.x;
 #pragma unroll 1
   for (int k = 0; k < 2; ++k) {
     const UnpackWeightJob& j = u.job[k];
     if (j.packed == nullptr) break;
-    if (j.bits == 4) unpack_weight_f16_chunks<4>(j, s_ucb[k], first, stride);
-    else if (j.bits == 3) unpack_weight_f16_chunks<3>(j, s_ucb[k], first, stride);
-    else unpack_weight_f16_chunks<2>(j, s_ucb[k], first, stride);
+    if (j.bits == 4) unpack_weight_f16_chunks<4>(j, s_ucb + 16 * k, first, stride);
+    else if (j.bits == 3) unpack_weight_f16_chunks<3>(j, s_ucb + 16 * k, first, stride);
+    else unpack_weight_f16_chunks<2>(j, s_ucb + 16 * k, first, stride);
   }
+}
+__device__ __forceinline__ void unpack_jobs_block(const UnpackJobs& u) {
+  __shared__ __half s_ucb[32];
+  unpack_jobs_run(u, static_cast<int>(blockIdx.x), s_ucb);
 }
 
 template <int BITS>

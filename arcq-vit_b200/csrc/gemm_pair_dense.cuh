@@ -29,6 +29,7 @@
 #include "ptx.cuh"
 #include "gemm_pair.cuh"
 #include "codes.cuh"
+#include "group_quant.cuh"
 
 namespace arcq {
 
@@ -42,10 +43,19 @@ struct PairDenseParams {
   uint32_t poll_limit;  // sleeping waits give up after this many polls
   uint32_t spin_limit;  // the issuing thread's busy waits give up after this many probes
   int* status;
+  int pairs;       // CTA pairs that multiply; pairs beyond them take the unpack jobs
+  const float* thresholds;   // quantizer form only
+  const float* codebook;
   UnpackWeightJob next;  // the weight of the layer that runs after this one, unpacked by two spare warps (or none)
 };
 
 constexpr int kPairDenseThreads = (2 + kPairEpiWarps) * 32;
+// The quantizer form has three epilogue warps per lane quarter, one per 64-column group of a 192-column slab (14 warps: 128
+// registers a thread, which the quantizer needs; 18 would leave 112).
+constexpr int kPairQuantEpiWarps = 12;
+constexpr int kPairQuantThreads = (2 + kPairQuantEpiWarps) * 32;
+constexpr uint32_t kPairQuantStageBytes = kPairQuantEpiWarps * 4096;       // 32 rows of 128 bytes per warp
+constexpr uint32_t kPairQuantTableBytes = (sizeof(GroupQuantTables) + 15) / 16 * 16;
 // Staging blocks (2 KB: 32 rows x 64 bytes) per epilogue warp; a block can be rewritten once the TMA store that
 // reads it has done so.  Four blocks instead of two measured slower on every DeiT-S shape (qkv 13.6 -> 15.5 us,
 // fc2 17.5 -> 22.3 us): the 32 KB they take away from the operand stages cost more than deeper stores gain.  One
@@ -58,28 +68,38 @@ constexpr int kDenseStageBlocks = ARCQ_DENSE_STAGE_BLOCKS;
 constexpr uint32_t kPairDenseEpiStageBytes = kPairEpiWarps * kDenseStageBlocks * 2048;
 
 struct PairDenseSmem {
-  uint32_t stages, slab, stage, misc, total;
+  uint32_t stages, slab, stage, tables, misc, total;
 };
 constexpr int kPairDenseBarriers = 72;
-__host__ __device__ inline PairDenseSmem pair_dense_smem_layout(int bn, int sa, int ks, int G, bool stationary) {
+__host__ __device__ inline PairDenseSmem pair_dense_smem_layout(int bn, int sa, int ks, int G, bool stationary, bool quant = false) {
   PairDenseSmem s;
   const uint32_t wtile = static_cast<uint32_t>(bn / 2) * 128u;
   const uint32_t stage_bytes = static_cast<uint32_t>(ks) * (kStageA + (stationary ? 0u : wtile));
   s.stages = 0;
   s.slab = static_cast<uint32_t>(sa) * stage_bytes;
   s.stage = s.slab + (stationary ? static_cast<uint32_t>(G) * wtile : 0u);
-  s.misc = s.stage + kPairDenseEpiStageBytes;
+  s.tables = s.stage + (quant ? kPairQuantStageBytes : kPairDenseEpiStageBytes);     // on a 1 KB boundary
+  s.misc = s.tables + (quant ? kPairQuantTableBytes : 0u);
   s.total = s.misc + 256 * 4 /*bias*/ + kPairDenseBarriers * 8 + 16 /*tensor-memory address*/ + 32 /*next codebook*/;
   return s;
 }
 
-template <bool STATIONARY, bool PREFETCH = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairDenseThreads, 1)
+// QBITS: width of the codes of the quantizer form (GELU and activation quantizer of the next layer in the epilogue), 0: plain.
+template <bool STATIONARY, bool PREFETCH = false, int QBITS = 0>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantThreads : kPairDenseThreads, 1)
     dense_weight_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
-                                  const __grid_constant__ CUtensorMap tm_y, const PairDenseParams p) {
+                                  const __grid_constant__ CUtensorMap tm_y, const PairDenseParams p,
+                                  const __grid_constant__ UnpackJobs jobs) {
+  constexpr int kEpi = QBITS ? kPairQuantEpiWarps : kPairEpiWarps;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* const smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  const PairDenseSmem L = pair_dense_smem_layout(p.bn, p.sa, p.ks, p.G, STATIONARY);
+  const PairDenseSmem L = pair_dense_smem_layout(p.bn, p.sa, p.ks, p.G, STATIONARY, QBITS != 0);
+  if (static_cast<int>(blockIdx.x) >= 2 * p.pairs) {
+    // both CTAs of such a pair: weights of layers further on, on SMs that this GEMM leaves idle
+    pdl_launch_dependents();
+    unpack_jobs_run(jobs, static_cast<int>(blockIdx.x) - 2 * p.pairs, reinterpret_cast<__half*>(smem_raw));
+    return;
+  }
   uint8_t* const sStages = smem + L.stages;
   uint8_t* const sSlab = smem + L.slab;
   uint8_t* const sStage = smem + L.stage;
@@ -97,7 +117,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairDenseThreads, 1
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t crank = cluster_ctarank();     // 0: leader
   const int bn = p.bn, hb = bn >> 1, G = p.G, ks = p.ks;
-  const int n_pairs = static_cast<int>(gridDim.x) >> 1;
+  const int n_pairs = p.pairs;
   const int pair = static_cast<int>(blockIdx.x) >> 1;
   const int n_slabs = p.N / bn;
   const int slab = pair % n_slabs;
@@ -121,7 +141,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairDenseThreads, 1
   pdl_launch_dependents();
   if (tid == 0) {
     for (int i = 0; i < p.sa; ++i) { mbar_init(&bars[i], 1); mbar_init(&bars[16 + i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars[32 + i], 1); mbar_init(&bars[34 + i], 2 * kPairEpiWarps); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars[32 + i], 1); mbar_init(&bars[34 + i], 2 * kEpi); }
     if (STATIONARY)
       for (int i = 0; i < p.G; ++i) mbar_init(&bars[40 + i], 1);
     mbar_fence_init();
@@ -240,6 +260,76 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairDenseThreads, 1
       __syncwarp();
       if (!ok && lane == 0) atomicExch(p.status, kStatusPairTimeout);
     }
+  } else if constexpr (QBITS != 0) {
+    // ------------------------------------------------------------------ epilogue with GELU and quantizer
+    // A thread owns one row and 64 columns, i.e. one group of the next layer's activation quantizer: tensor memory -> + bias ->
+    // fp16 (what the plain form stores) -> GELU -> quantizer -> reconstruction, in registers but for the exchange of large GELU
+    // arguments, then through this warp's staging rows to a TMA store.  Issue slots of these warps bound the kernel (about 30
+    // instructions a value); the products run underneath.  N = 3072, K = 768: M = 12608 72.9 us against 49.4 + 40.3 us for GEMM
+    // and quantizer kernel, M = 100864 618 against 457 + 407 us.
+    const int ew = warp - 2, lq = warp & 3, grp = ew >> 2;
+    GroupQuantTables* const tables = reinterpret_cast<GroupQuantTables*>(smem + L.tables);
+    for (int i = tid - 64; i < bn; i += kEpi * 32) s_bias[i] = (p.bias != nullptr) ? __ldg(p.bias + n0 + i) : 0.0f;
+    const GroupQuantParams gp = group_quant_tables<1 << QBITS>(tables, p.thresholds, p.codebook, tid - 64, kEpi * 32, [](bool b) {
+      asm volatile("bar.sync 2, %0;" ::"n"(kEpi * 32) : "memory");
+      return b;
+    });
+    const uint32_t acc_empty_leader = mapa_shared(acc_empty, 0);
+    uint8_t* const stg = sStage + ew * 4096;
+    const uint32_t row = smem_u32(stg) + lane * 128, x7 = lane & 7;
+    for (int t = 0; t < my_tiles && ok; ++t) {
+      const uint32_t buf = static_cast<uint32_t>(t) & 1;
+      if (!mbar_wait_sleep_a(acc_full + buf * 8, (static_cast<uint32_t>(t) >> 1) & 1, poll_limit, 32)) { ok = false; break; }
+      tc_fence_after_sync();
+      const int row0 = row_of(t) + lq * 32;
+      const bool live = row0 < p.M && grp * 64 < bn;      // some of these 32 rows are inside the matrix, and the group is one
+      uint32_t w[32];
+      if (live) {
+        const uint32_t t_row = tmem_base + buf * 256 + (static_cast<uint32_t>(lq * 32) << 16) + grp * 64;
+        const float* const b = s_bias + grp * 64;
+#pragma unroll
+        for (int half_id = 0; half_id < 2; ++half_id) {
+          uint32_t a[32];
+          tmem_ld_32x32(t_row + half_id * 32, a);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float4 b4 = *reinterpret_cast<const float4*>(b + half_id * 32 + 4 * i);
+            const __half2 h0 = __floats2half2_rn(__uint_as_float(a[4 * i]) + b4.x, __uint_as_float(a[4 * i + 1]) + b4.y);
+            const __half2 h1 = __floats2half2_rn(__uint_as_float(a[4 * i + 2]) + b4.z, __uint_as_float(a[4 * i + 3]) + b4.w);
+            w[half_id * 16 + 2 * i] = *reinterpret_cast<const uint32_t*>(&h0);
+            w[half_id * 16 + 2 * i + 1] = *reinterpret_cast<const uint32_t*>(&h1);
+          }
+        }
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive_cluster(acc_empty_leader + buf * 8);
+        tma_store_wait_read();                            // the store that last used the staging rows has read them
+      }
+      __syncwarp();
+      if (live) {
+        gelu_words<1>(w, row, x7);
+        f32x2 v[32];
+        uint32_t words[8];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = sixteen_to_pair<__half>(w[i]);
+        const GroupStats st = group_quantize<QBITS, false, 1>(v, tables, gp, words);
+        const GroupRecon g = group_recon(st, gp);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) w[i] = pair_to_sixteen<__half>(group_recon_pair(g, v[i]));
+        row_store<1>(w, row, x7);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(&tm_y, stg, n0 + grp * 64, row0);  // rows beyond M are clipped
+          tma_store_commit();
+        }
+      }
+    }
+    if (lane == 0) tma_store_wait_all();
+    if (!ok && lane == 0) atomicExch(p.status, kStatusPairTimeout);
   } else {
     // ------------------------------------------------------------------ epilogue (own 128 rows of each tile)
     // Eight warps: two per tensor-memory lane quarter, taking alternate column steps of 64 bytes per row.
@@ -255,7 +345,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairDenseThreads, 1
       // first: the scratch matrix being overwritten was last read two GEMMs back and is then free for certain.
       pdl_wait();
       const long long first = static_cast<long long>(blockIdx.x) * (kPairEpiWarps * 32) + (tid - 64);
-      const long long stride = static_cast<long long>(gridDim.x) * (kPairEpiWarps * 32);
+      const long long stride = 2ll * p.pairs * (kPairEpiWarps * 32);
       if (p.next.bits == 4) unpack_weight_f16_chunks<4>(p.next, s_next_cb, first, stride);
       else if (p.next.bits == 3) unpack_weight_f16_chunks<3>(p.next, s_next_cb, first, stride);
       else unpack_weight_f16_chunks<2>(p.next, s_next_cb, first, stride);

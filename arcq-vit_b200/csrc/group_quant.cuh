@@ -3,7 +3,7 @@
 //
 // Two lanes a group (lane h holds the reference's summation lanes l = 4h .. 4h+3, half of every 16-byte chunk) need 64
 // registers instead of 128 and half the straight-line code: 32 warps an SM instead of 16, and fewer instruction-cache
-// misses.  LASTLINE
+// misses; measured slower all the same (GELU [12608, 1536] 28.1 against 24.1 us: 25 instructions a value instead of 17).
 //
 // What bounds it is issue slots: nothing here waits for memory once the row is in shared memory.  So the arithmetic is
 // two values per instruction (add / mul / fma.f32x2; each half rounds like the scalar instruction, so the bits are those of
@@ -310,20 +310,17 @@ __device__ __forceinline__ void row_store(const uint32_t (&w)[32 / LPG], uint32_
 }
 
 // ---------------------------------------------------------------- GELU of a group's fp16 values
-// g = x * (0.5 + x * R(x^2)) for |x| < 1.3125, with x * R(x^2) = erf(x / sqrt 2) / 2: R of degree 5 in x^2, fitted on
-// Chebyshev nodes (2e-8 relative before rounding).  Over every fp16 input of that range the fp16 result differs from the
-// correctly rounded one for 3 inputs of 31 742 (0.5 x (1 + erff(x / sqrt 2)) in fp32: 2).  Larger arguments keep the value of
-// x, are counted in a bit mask, and go through erff one by one in a loop over the lane's part of the row in shared memory:
-// few of them sit in a group, and the loop is one copy of erff in the code instead of 64.  The row is used for that
-// exchange only.  The result is rounded to fp16, the value a separate GELU kernel would store.
+// The arithmetic of gelu (act_quant.cuh), two values per instruction.  Arguments of 2 and more keep the value of x, are
+// marked in a bit mask, and go through erff one by one in a loop over the lane's part of the row in shared memory: few of
+// them sit in a group, and the loop is one copy of erff in the code instead of 64.  Each costs its whole warp an iteration,
+// which is why the polynomial reaches to 2 (up to 1.3125 degree 5 would do, one instruction a value less: [100864, 3072] with
+// values of 0.55 rms takes 407 us instead of 647).  The row is used for that exchange only.  The result is rounded to fp16,
+// the value a separate GELU kernel would store.
 template <int LPG>
 __device__ __forceinline__ void gelu_words(uint32_t (&w)[32 / LPG], uint32_t row, uint32_t x7) {
   constexpr int PJ = 4 / LPG;
-  const f32x2 c5 = pack2(-6.607886916754069e-06f, -6.607886916754069e-06f), c4 = pack2(0.00011030046152882278f, 0.00011030046152882278f);
-  const f32x2 c3 = pack2(-0.0011828974820673466f, -0.0011828974820673466f), c2 = pack2(0.009971804916858673f, 0.009971804916858673f);
-  const f32x2 c1 = pack2(-0.06649012118577957f, -0.06649012118577957f), c0 = pack2(0.3989422619342804f, 0.3989422619342804f);
   const f32x2 half = pack2(0.5f, 0.5f);
-  const __half2 lim = __floats2half2_rn(1.3125f, 1.3125f);
+  const __half2 lim = __floats2half2_rn(kGeluLimit, kGeluLimit);
   uint32_t big[2] = {0u, 0u};
 #pragma unroll
   for (int i = 0; i < 32 / LPG; ++i) {
@@ -331,11 +328,9 @@ __device__ __forceinline__ void gelu_words(uint32_t (&w)[32 / LPG], uint32_t row
     const uint32_t m = __hgeu2_mask(__habs2(xh), lim);                  // 0xffff per half (unordered: NaN counts as large)
     const f32x2 x = sixteen_to_pair<__half>(w[i]);
     const f32x2 s = mul2(x, x);
-    f32x2 r = fma2(c5, s, c4);
-    r = fma2(r, s, c3);
-    r = fma2(r, s, c2);
-    r = fma2(r, s, c1);
-    r = fma2(r, s, c0);
+    f32x2 r = pack2(gelu_r(7), gelu_r(7));
+#pragma unroll
+    for (int k = 6; k >= 0; --k) r = fma2(r, s, pack2(gelu_r(k), gelu_r(k)));
     const uint32_t g = pair_to_sixteen<__half>(mul2(x, fma2(x, r, half)));
     big[i >> 4] |= m & (0x00010001u << (i & 15));
     w[i] = (m & w[i]) | (~m & g);
@@ -352,8 +347,7 @@ __device__ __forceinline__ void gelu_words(uint32_t (&w)[32 / LPG], uint32_t row
         const uint32_t i = 16u * hw + (k & 15);                          // the word, in chunk i / PJ
         const uint32_t a = row + (((i / PJ) ^ x7) << 4) + 4u * (i % PJ) + 2u * (k >> 4);
         const float x = __half2float(__ushort_as_half(static_cast<unsigned short>(lds16(a))));
-        const float g = x * 0.5f * (1.0f + erff(x * 0.70710678118654752440f));
-        sts16(a, __half_as_ushort(__float2half_rn(g)));
+        sts16(a, __half_as_ushort(__float2half_rn(gelu_large(x))));
       }
     }
     row_load<LPG>(w, row, x7);

@@ -398,10 +398,16 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
     gemm(xhat, *proj, branch);
     norm_quant(branch, gb[4 * i + 2], gb[4 * i + 3], b.norm2.eps, *fc1, *fc2);
-    gemm(xhat, *fc1, mid);
-    check(arcq_gelu_act_quant(mid, ARCQ_DT_F16, M, fc2->K, fc2->th, fc2->acb, fc2->bits, 64, nullptr, nullptr, nullptr, nullptr, xhat4,
-                              ARCQ_DT_F16, st),
-          "arcq_gelu_act_quant");
+    const int rc = arcq_dense_weight_gemm_gelu_quant(xhat, fc1->job.out, fc1->bias, M, fc1->N, fc1->K, fc2->th, fc2->acb, fc2->bits, 64,
+                                                     xhat4, nullptr, 0, st);
+    if (rc != ARCQ_E_UNSUPPORTED) {
+      check(rc, "arcq_dense_weight_gemm_gelu_quant");
+    } else {
+      gemm(xhat, *fc1, mid);
+      check(arcq_gelu_act_quant(mid, ARCQ_DT_F16, M, fc2->K, fc2->th, fc2->acb, fc2->bits, 64, nullptr, nullptr, nullptr, nullptr, xhat4,
+                                ARCQ_DT_F16, st),
+            "arcq_gelu_act_quant");
+    }
     gemm(xhat4, *fc2, branch);
     y = branch;
   }

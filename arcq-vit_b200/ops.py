@@ -382,6 +382,36 @@ def dense_weight_gemm(xhat: torch.Tensor, w16: torch.Tensor, bias, out_dtype: to
     return y
 
 
+def dense_weight_gemm_gelu_quant(xhat: torch.Tensor, w16: torch.Tensor, bias, thresholds: torch.Tensor, codebook: torch.Tensor,
+                                 bits: int, group_size: int) -> torch.Tensor:
+    """``dense_weight_gemm`` (fp16) and the GELU + activation quantizer of the layer behind it in one kernel: the fp16
+    reconstruction [M, N], the same bits as the two separate operators (which run where the kernel is not the better choice)."""
+    lib = _cabi.load()
+    xhat = _dev(xhat, "xhat", torch.float16)
+    w16 = _dev(w16, "w16", torch.float16)
+    thresholds, codebook = _dev(thresholds, "thresholds", torch.float32), _dev(codebook, "codebook", torch.float32)
+    M, K = xhat.shape
+    N = w16.shape[0]
+    if w16.dim() != 2 or w16.shape[1] != K:
+        raise RuntimeError(f"weight {tuple(w16.shape)} does not match K={K}")
+    if codebook.numel() != 2 ** bits or thresholds.numel() != 2 ** bits - 1:
+        raise RuntimeError(f"expected {2 ** bits} levels and {2 ** bits - 1} thresholds")
+    b = None
+    if bias is not None and bias.numel() > 0:
+        b = _dev(bias, "bias", torch.float32)
+        if b.numel() != N:
+            raise RuntimeError("bias must have out_features entries")
+    out = torch.empty((M, N), dtype=torch.float16, device=xhat.device)
+    rc = lib.arcq_dense_weight_gemm_gelu_quant(xhat.data_ptr(), w16.data_ptr(), b.data_ptr() if b is not None else None, M, N, K,
+                                               thresholds.data_ptr(), codebook.data_ptr(), bits, group_size, out.data_ptr(),
+                                               None, 0, _stream())
+    if rc == _cabi.E_UNSUPPORTED:
+        return quantize_activation_dequant(dense_weight_gemm(xhat, w16, bias), thresholds, codebook, bits, group_size,
+                                           torch.float16, True)
+    _check(rc, "arcq_dense_weight_gemm_gelu_quant")
+    return out
+
+
 def dequant(packed, center, scale, code_sum, codebook, bits: int, group_size: int,
             out_dtype: torch.dtype = torch.float16, out: torch.Tensor = None) -> torch.Tensor:
     """Packed codes + statistics -> [R, K] matrix; what the reference's ``unpack_weight_triton``

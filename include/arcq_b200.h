@@ -88,7 +88,8 @@ int arcq_debug_get_option(const char* name, int* value_out);
  */
 enum {
   ARCQ_GEMM_ONE_CTA_PACKED = 1, ARCQ_GEMM_ONE_CTA_DENSE = 2, ARCQ_GEMM_PAIR_PACKED = 3, ARCQ_GEMM_PAIR_DENSE = 4,
-  ARCQ_GEMM_PAIR_DENSE_PREFETCH = 5
+  ARCQ_GEMM_PAIR_DENSE_PREFETCH = 5,
+  ARCQ_GEMM_PAIR_DENSE_GELU_QUANT = 6
 };
 int arcq_debug_last_gemm_kernel(void);
 
@@ -328,6 +329,29 @@ int arcq_dequant(const uint8_t* packed, const float* mu, const float* sigma, con
 int arcq_unpack_weight_f16(const uint8_t* packed, const float* mu, const float* sigma, const float* codesum,
                            const float* codebook, int bits, int group_size, int64_t rows, int64_t K,
                            void* out, void* stream);
+
+/*
+ * arcq_dense_weight_gemm with unpack jobs (see arcq_unpack_job) on the SMs that its tiles leave idle: weights of layers that
+ * run later, not the one it multiplies with.  arcq_dense_weight_gemm_unpack_room says how many values a GEMM of that shape
+ * can take along without being prolonged (gelu_quant = 1: of arcq_dense_weight_gemm_gelu_quant; 0 also where that is left to
+ * the two calls), arcq_unpack_beside_gemm (1 / 0) whether a transformer block on M rows of `width` values gains from it over
+ * jobs on the LayerNorm + quantizer launch.
+ */
+int arcq_dense_weight_gemm_unpack(const void* xhat, const void* w16, const float* bias, int64_t M, int64_t N, int64_t K,
+                                  void* y, int y_dtype, const arcq_unpack_job* unpack, int n_unpack, void* stream);
+int64_t arcq_dense_weight_gemm_unpack_room(int64_t M, int64_t N, int64_t K, int gelu_quant);
+int arcq_unpack_beside_gemm(int64_t M, int64_t width);
+
+/*
+ * arcq_dense_weight_gemm (fp16 result) followed by arcq_gelu_act_quant with an fp16 reconstruction, in one kernel: the
+ * input of fc2 from that of fc1 (timm Mlp.forward: fc1, GELU; step 2 of ARCQPackedLinearOnTheFly.forward of fc2,
+ * FQ/fair_qat/arcq_packed_on_the_fly.py:143-145).  Bit for bit what the two calls give; out fp16 [M, N], thresholds and
+ * codebook those of the layer that reads it.  N % 64 == 0.  ARCQ_E_UNSUPPORTED where the two calls are the better choice.
+ * Unpack jobs as in arcq_dense_weight_gemm_unpack.
+ */
+int arcq_dense_weight_gemm_gelu_quant(const void* xhat, const void* w16, const float* bias, int64_t M, int64_t N, int64_t K,
+                                      const float* thresholds, const float* codebook, int bits, int group_size, void* out,
+                                      const arcq_unpack_job* unpack, int n_unpack, void* stream);
 
 /*
  * arcq_dense_weight_gemm that also unpacks the weight of the layer that runs NEXT (arcq_unpack_weight_f16 of
