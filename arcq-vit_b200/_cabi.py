@@ -20,6 +20,7 @@ EXPORTS = (
     "arcq_unpack_codes", "arcq_pack_codes", "arcq_dequant", "arcq_unpack_weight_f16", "arcq_dense_weight_gemm_prefetch",
     "arcq_act_quant_unpack", "arcq_add_layernorm_act_quant_unpack", "arcq_add_layernorm_strided",
     "arcq_dense_weight_gemm_unpack", "arcq_dense_weight_gemm_unpack_room", "arcq_unpack_beside_gemm", "arcq_dense_weight_gemm_gelu_quant",
+    "arcq_dense_weight_gemm_gelu_quant_applies",
 )
 
 _lib = None

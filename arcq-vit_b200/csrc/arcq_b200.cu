@@ -1193,6 +1193,12 @@ int64_t arcq_dense_weight_gemm_unpack_room(int64_t M, int64_t N, int64_t K, int 
   return idle > 0 ? idle * arcq::kPairDenseThreads * 160 : 0;
 }
 
+int arcq_dense_weight_gemm_gelu_quant_applies(int64_t M, int64_t N, int64_t K) {
+  PairDenseConfig pc;
+  if (M <= 0 || N <= 0 || K <= 0 || K % 64 != 0 || M > 0x7fffffffLL || N > 0x7fffffffLL || K > (1 << 20)) return 0;
+  return choose_gelu_quant(M, N, K, &pc) ? 1 : 0;
+}
+
 int arcq_dense_weight_gemm_gelu_quant(const void* xhat, const void* w16, const float* bias, int64_t M, int64_t N, int64_t K,
                                       const float* thresholds, const float* codebook, int bits, int group_size, void* out,
                                       const arcq_unpack_job* unpack, int n_unpack, void* stream) {

@@ -364,15 +364,57 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     lin[4 * i + 2].job.out = w_mlp;
     lin[4 * i + 3].job.out = w_mlp + lin[4 * i + 2].weight_elems();
   }
-  auto norm_quant = [&](const at::Half* y, const float* gamma, const float* beta, double eps, const Linear& first, const Linear& second) {
-    const arcq_unpack_job jobs[2] = {first.job, second.job};
-    check(arcq_add_layernorm_act_quant_unpack(x, y, gamma, beta, static_cast<float>(eps), M, D, first.th, first.acb, first.bits, 64,
-                                              y != nullptr ? x_next : nullptr, nullptr, xhat, jobs, 2, st),
+  // Where the weights of a half block (qkv + proj, fc1 + fc2) are unpacked.  Few rows: by the GEMM that ends the half block
+  // before, on the SMs it leaves idle, while it reads the other scratch matrix; what has no room there by the half block's own
+  // first GEMM (its second weight) or the LayerNorm.  Many rows: the GEMMs fill the machine, and extra blocks of the LayerNorm
+  // + quantizer launch do it.
+  const bool beside_gemm = arcq_unpack_beside_gemm(M, D) != 0;
+  int done = 0;                        // of the next half block's two weights
+  auto jobs_of = [&](const Linear* half, int from, int to, arcq_unpack_job (&jobs)[2]) {
+    for (int k = from; k < to; ++k) jobs[k - from] = half[k].job;
+    return to - from;
+  };
+  // what the GEMM of a layer can take along, asked once per shape
+  struct Room {
+    int64_t N, K, values;
+    int gelu_quant;
+  };
+  std::vector<Room> rooms;
+  auto room_of = [&](const Linear& l, int gelu_quant) {
+    for (const Room& r : rooms)
+      if (r.N == l.N && r.K == l.K && r.gelu_quant == gelu_quant) return r.values;
+    rooms.push_back({l.N, l.K, arcq_dense_weight_gemm_unpack_room(M, l.N, l.K, gelu_quant), gelu_quant});
+    return rooms.back().values;
+  };
+  // how far the weights of `half` from `from` on fit into what the GEMM of `l` can take along
+  auto fits = [&](const Linear* half, int from, const Linear& l, int gelu_quant) {
+    if (!beside_gemm || half == nullptr) return from;
+    int64_t room = room_of(l, gelu_quant);
+    while (from < 2 && half[from].weight_elems() <= room) room -= half[from++].weight_elems();
+    return from;
+  };
+  auto norm_quant = [&](const at::Half* y, const float* gamma, const float* beta, double eps, const Linear* half, int gelu_quant) {
+    // the first weight has to be there before the half block's first GEMM, the second may be that GEMM's job
+    const int first = std::max(done, 1), to = fits(half, first, half[0], gelu_quant) == 2 ? first : 2;
+    arcq_unpack_job jobs[2];
+    const int n = jobs_of(half, done, to, jobs);
+    check(arcq_add_layernorm_act_quant_unpack(x, y, gamma, beta, static_cast<float>(eps), M, D, half[0].th, half[0].acb, half[0].bits, 64,
+                                              y != nullptr ? x_next : nullptr, nullptr, xhat, jobs, n, st),
           "arcq_add_layernorm_act_quant");
     if (y != nullptr) std::swap(x, x_next);
+    done = to;
   };
-  auto gemm = [&](const at::Half* a, const Linear& l, at::Half* y) {
-    check(arcq_dense_weight_gemm(a, l.job.out, l.bias, M, l.N, l.K, y, ARCQ_DT_F16, st), "arcq_dense_weight_gemm");
+  auto gemm = [&](const at::Half* a, const Linear& l, at::Half* y, const arcq_unpack_job* jobs, int n) {
+    check(arcq_dense_weight_gemm_unpack(a, l.job.out, l.bias, M, l.N, l.K, y, ARCQ_DT_F16, jobs, n, st), "arcq_dense_weight_gemm");
+  };
+  // The last GEMM of a half block; next: the linears of the next one, or null.  Both weights in two rounds of the idle SMs'
+  // threads, or the second one left to the next GEMM if that has room.
+  auto last_gemm = [&](const at::Half* a, const Linear& l, at::Half* y, const Linear* next, int next_gelu_quant) {
+    arcq_unpack_job jobs[2];
+    done = fits(next, 0, l, 0);
+    if (done == 2 && next[0].weight_elems() + next[1].weight_elems() > room_of(l, 0) * 2 / 5 && fits(next, 1, next[0], next_gelu_quant) == 2)
+      done = 1;
+    gemm(a, l, y, jobs, jobs_of(next, 0, done, jobs));
   };
 
   {
@@ -383,11 +425,19 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
           "arcq_assemble_tokens");
   }
   const at::Half* y = nullptr;
+  int64_t asked[2] = {0, 0};            // the shape of fc1 that `fused` holds for
+  bool fused = false;
   for (size_t i = 0; i < depth; ++i) {
     const VitBlock& b = p->blocks[i];
     const Linear *qkv = &lin[4 * i], *proj = qkv + 1, *fc1 = qkv + 2, *fc2 = qkv + 3;
-    norm_quant(y, gb[4 * i], gb[4 * i + 1], b.norm1.eps, *qkv, *proj);
-    gemm(xhat, *qkv, mid);
+    if (asked[0] != fc1->N || asked[1] != fc1->K) {
+      fused = arcq_dense_weight_gemm_gelu_quant_applies(M, fc1->N, fc1->K) != 0;
+      asked[0] = fc1->N;
+      asked[1] = fc1->K;
+    }
+    arcq_unpack_job jobs[2];
+    norm_quant(y, gb[4 * i], gb[4 * i + 1], b.norm1.eps, qkv, 0);
+    gemm(xhat, *qkv, mid, jobs, jobs_of(qkv, done, 2, jobs));
     {
       const at::Tensor t = at::from_blob(mid, {B, T, 3, p->heads, D / p->heads}, at::TensorOptions().dtype(at::kHalf).device(dev));
       const at::Tensor r = t.permute({2, 0, 3, 1, 4});
@@ -396,19 +446,20 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                            xhat, ARCQ_DT_F16, st),
             "arcq_act_quant");
     }
-    gemm(xhat, *proj, branch);
-    norm_quant(branch, gb[4 * i + 2], gb[4 * i + 3], b.norm2.eps, *fc1, *fc2);
-    const int rc = arcq_dense_weight_gemm_gelu_quant(xhat, fc1->job.out, fc1->bias, M, fc1->N, fc1->K, fc2->th, fc2->acb, fc2->bits, 64,
-                                                     xhat4, nullptr, 0, st);
-    if (rc != ARCQ_E_UNSUPPORTED) {
-      check(rc, "arcq_dense_weight_gemm_gelu_quant");
+    last_gemm(xhat, *proj, branch, fc1, fused);
+    norm_quant(branch, gb[4 * i + 2], gb[4 * i + 3], b.norm2.eps, fc1, fused);
+    const int n = jobs_of(fc1, done, 2, jobs);
+    if (fused) {
+      check(arcq_dense_weight_gemm_gelu_quant(xhat, fc1->job.out, fc1->bias, M, fc1->N, fc1->K, fc2->th, fc2->acb, fc2->bits, 64, xhat4,
+                                              jobs, n, st),
+            "arcq_dense_weight_gemm_gelu_quant");
     } else {
-      gemm(xhat, *fc1, mid);
+      gemm(xhat, *fc1, mid, jobs, n);
       check(arcq_gelu_act_quant(mid, ARCQ_DT_F16, M, fc2->K, fc2->th, fc2->acb, fc2->bits, 64, nullptr, nullptr, nullptr, nullptr, xhat4,
                                 ARCQ_DT_F16, st),
             "arcq_gelu_act_quant");
     }
-    gemm(xhat4, *fc2, branch);
+    last_gemm(xhat4, *fc2, branch, i + 1 < depth ? qkv + 4 : nullptr, 0);
     y = branch;
   }
   // the head reads the class token of every image only

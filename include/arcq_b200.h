@@ -346,9 +346,10 @@ int arcq_unpack_beside_gemm(int64_t M, int64_t width);
  * arcq_dense_weight_gemm (fp16 result) followed by arcq_gelu_act_quant with an fp16 reconstruction, in one kernel: the
  * input of fc2 from that of fc1 (timm Mlp.forward: fc1, GELU; step 2 of ARCQPackedLinearOnTheFly.forward of fc2,
  * FQ/fair_qat/arcq_packed_on_the_fly.py:143-145).  Bit for bit what the two calls give; out fp16 [M, N], thresholds and
- * codebook those of the layer that reads it.  N % 64 == 0.  ARCQ_E_UNSUPPORTED where the two calls are the better choice.
- * Unpack jobs as in arcq_dense_weight_gemm_unpack.
+ * codebook those of the layer that reads it.  N % 64 == 0.  ARCQ_E_UNSUPPORTED where the two calls are the better choice,
+ * which arcq_dense_weight_gemm_gelu_quant_applies (1 / 0) says beforehand.  Unpack jobs as in arcq_dense_weight_gemm_unpack.
  */
+int arcq_dense_weight_gemm_gelu_quant_applies(int64_t M, int64_t N, int64_t K);
 int arcq_dense_weight_gemm_gelu_quant(const void* xhat, const void* w16, const float* bias, int64_t M, int64_t N, int64_t K,
                                       const float* thresholds, const float* codebook, int bits, int group_size, void* out,
                                       const arcq_unpack_job* unpack, int n_unpack, void* stream);
