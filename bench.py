@@ -310,7 +310,7 @@ def kernel_rooflines(pkg, a, dev, pk):
         mbytes = 4 * M * dim * 2
         merged = {"kernel": "add_layernorm_act_quant_kernel", "ms": t_merged, "separate_kernels_ms": t_apart,
                   "bytes": mbytes, "achieved": mbytes / t_merged / 1e6, "frac": mbytes / t_merged / 1e6 / pk["hbm_gbs"]}
-    out["roofline_act_quant"] = {"kernel": "act_quant_v2_kernel (qkv / proj / fc1 inputs), act_quant_v4_kernel with GELU (fc2 input)", "bound": "hbm", "achieved": aq, "peak": pk["hbm_gbs"],
+    out["roofline_act_quant"] = {"kernel": "act_quant_tile_kernel (qkv / proj / fc1 inputs; with GELU for the fc2 input)", "bound": "hbm", "achieved": aq, "peak": pk["hbm_gbs"],
                                  "unit": "GB/s", "frac": aq / pk["hbm_gbs"], "traffic": None,
                                  "peak_source": pk["source"] + " copy",
                                  "frac_of_same_size_copy": aq_copy_ms / aq_ms,
