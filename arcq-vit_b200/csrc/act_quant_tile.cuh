@@ -1,10 +1,10 @@
-// Activation quantizer for large inputs (group_quant.cuh): each warp works on its own tiles of 32 groups (16 with two lanes a
-// group).  It brings a tile in by TMA (a row per group, 128-byte swizzle, so that lanes read their rows without bank
-// conflicts), quantises it in place and sends the reconstruction out by TMA, with the next tile's load and the previous
+// Activation quantizer for large inputs (group_quant.cuh): each warp works on its own tiles of 32 groups.  It brings
+// a tile in by TMA (a row per group, 128-byte swizzle, so that lanes read their rows without bank conflicts), quantises it in place and sends the reconstruction out by TMA, with the next tile's load and the previous
 // tile's store in flight meanwhile.  No block-wide synchronisation after the table set-up.
 //
 // Bound by issue slots, then by shared-memory reads (about four wavefronts per 32 values); memory is half idle.
-// Reconstruction only: two lanes a group, 32 warps an SM.  With codes: one lane a group, which assembles the words.
+// One lane a group, 16 warps an SM.  [12608, 384] 5.7 us, with GELU [12608, 1536] 25.4 us (before the shared group routine 7.7
+// and 37.6 us).
 #pragma once
 #include <cuda.h>
 #include "ptx.cuh"

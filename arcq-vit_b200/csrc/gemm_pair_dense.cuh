@@ -21,6 +21,10 @@
 // 256 x 192 tile are used for so few flops that the L2 -> shared-memory traffic (about 8 TB/s over all SMs)
 // bounds the kernel, and the slab is 43 % of that traffic.
 //
+// Pairs of CTAs beyond the ones that multiply (PairDenseParams::pairs) unpack weights of later layers on SMs that would idle: a
+// ViT block of a few hundred rows keeps 24 to 100 of them busy (DeiT-S batch 1: 552 us with the unpack on the LayerNorm + quantizer
+// launch, 497 us here).
+//
 // Each output element is the fp32 sum over k in ascending order of 16-wide steps, as in every other GEMM
 // kernel of this library.
 #pragma once
