@@ -29,11 +29,12 @@ template <> __device__ __forceinline__ float round_to<__nv_bfloat16>(float v) {
   return __bfloat162float(__float2bfloat16_rn(v));
 }
 // GELU of an fp16 value in fp32, in all kernels the same to the bit: x * (0.5 + x * R(x^2)) for |x| < 2, with
-// x * R(x^2) = erf(x / sqrt 2) / 2 and R of degree 7, fitted on Chebyshev nodes; erff beyond.  Over every fp16 input of that
-// range the fp16 result differs from the correctly rounded one for 3 inputs of 32 768 (0.5 x (1 + erff(x / sqrt 2)) in fp32: 3).
+// x * R(x^2) = erf(x / sqrt 2) / 2 and R of degree 7, fitted on Chebyshev nodes; erff beyond.  Rounded to fp16 it is, for each
+// of the 65 536 inputs, what 0.5 x (1 + erff(x / sqrt 2)) in fp32 rounds to: the coefficient of degree 3 is three units in the
+// last place off the fit, because with the fit itself x = -1.4853515625 came out one unit off.
 constexpr float kGeluLimit = 2.0f;
 __device__ __forceinline__ float gelu_r(int k) {       // k is a constant wherever this is used
-  const float c[8] = {0.398942292f,    -0.0664903149f,  0.00997320935f, -0.0011866159f,
+  const float c[8] = {0.398942292f,    -0.0664903149f,  0.00997320935f, -0.00118661555f,
                       0.000114711416f, -9.03896398e-06f, 5.35578579e-07f, -1.75760011e-08f};
   return c[k];
 }

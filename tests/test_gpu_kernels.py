@@ -531,6 +531,22 @@ def test_fused_gelu_over_every_fp16_input(pkg, cuda_device, report):
     assert pkg.ops.device_status() == 0
 
 
+@pytest.mark.parametrize("rows", [31, 1240])                       # 992 groups: eight lanes a group; 39 680: tiles
+def test_fused_gelu_stores_the_bits_of_the_separate_gelu(pkg, cuda_device, rows):
+    """Mean and scale of a group move with the last bit of any of its 64 values, so they are compared as bits: every finite
+    fp16 input, in groups of like magnitude, through the fused GELU and through torch's fp16 GELU."""
+    vals = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.float16)
+    vals = vals[torch.isfinite(vals)].reshape(31, 2048)
+    pre = vals.repeat(rows // 31, 1).to(cuda_device)
+    cb = torch.linspace(-2.6, 2.55, 16, device=cuda_device)
+    th = (cb[:-1] + cb[1:]) / 2
+    want = pkg.ops.quantize_activation(torch.nn.functional.gelu(pre), th, cb, 4, 64)
+    got = pkg.ops.quantize_activation(pre, th, cb, 4, 64, True, True)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    assert pkg.ops.device_status() == 0
+
+
 @pytest.mark.parametrize("out_dtype", [torch.float16, torch.float32])
 @pytest.mark.parametrize("M,K,N", [(1, 64, 16), (129, 128, 48), (197, 384, 1152), (300, 1536, 384), (1000, 768, 2304),
                                    (64 * 197, 1536, 384), (64 * 197, 384, 1536)])
