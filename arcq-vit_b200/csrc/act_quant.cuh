@@ -51,6 +51,22 @@ template <typename T, int PRE> __device__ __forceinline__ float pre_op(float x) 
   return PRE == 1 ? round_to<T>(gelu(x)) : x;
 }
 
+// The reconstruction of a level as c + (scale * (level + a) + b), in either of the two forms the GEMMs were built for:
+//   three steps   mean + scale * (level - code_sum / 64), each rounded, as the reference's fp32 tensor operations;
+//   one_fma       fma(scale, level, mean - scale * code_sum / 64), what arcq_packed_gemm rebuilds from packed codes.
+// The other two operations add -0, which changes nothing.
+struct ReconTerms {
+  float a, b, c;
+};
+__device__ __forceinline__ ReconTerms recon_terms(float mean, float scale, float code_sum, bool one_fma) {
+  const float vm = __fmul_rn(code_sum, 0.015625f);           // / 64: exact
+  if (one_fma) return {-0.0f, __fmaf_rn(-scale, vm, mean), -0.0f};
+  return {-vm, -0.0f, mean};
+}
+__device__ __forceinline__ float recon_value(const ReconTerms& t, float scale, float level) {
+  return __fadd_rn(t.c, __fmaf_rn(scale, __fadd_rn(level, t.a), t.b));
+}
+
 // Sum of the value held by the 8 lanes of an octet, lane 0 first, as a chain of fp32 additions.
 __device__ __forceinline__ float octet_chain_sum(float p, int octet_base) {
   float s = __shfl_sync(0xffffffffu, p, octet_base);
@@ -93,7 +109,7 @@ __global__ void __launch_bounds__(256) act_quant_kernel(const T* __restrict__ x,
                                                         uint8_t* __restrict__ packed, float* __restrict__ mu_out,
                                                         float* __restrict__ sigma_out,
                                                         float* __restrict__ codesum_out, XH* __restrict__ xhat,
-                                                        const __grid_constant__ UnpackJobs jobs) {
+                                                        int one_fma, const __grid_constant__ UnpackJobs jobs) {
   pdl_launch_dependents();   // the next kernel of the stream may start its set-up
   if (static_cast<int>(blockIdx.x) < jobs.blocks) {
     unpack_jobs_block(jobs);
@@ -167,13 +183,12 @@ __global__ void __launch_bounds__(256) act_quant_kernel(const T* __restrict__ x,
     const float code_sum = octet_chain_sum(part, octet_base);
 
     if (WRITE_XHAT) {
-      // mean + scale * (cb[c] - code_sum/64), each step rounded as the reference's fp32 tensor ops
-      const float vm = __fdiv_rn(code_sum, 64.0f);
+      const ReconTerms rt = recon_terms(mean, scale, code_sum, one_fma != 0);
       if (valid) {
         XH* og = xhat + gi * 64 + l;
 #pragma unroll
         for (int c = 0; c < 8; ++c)
-          store_from_f32<XH>(og + 8 * c, __fadd_rn(mean, __fmul_rn(scale, __fsub_rn(cv[c], vm))));
+          store_from_f32<XH>(og + 8 * c, recon_value(rt, scale, cv[c]));
       }
     }
 

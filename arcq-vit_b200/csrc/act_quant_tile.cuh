@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(AqtShape<T, WRITE_PACKED>::kThreads, AqtShape<
     act_quant_tile_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_out,
                           long long total_groups, const float* __restrict__ thresholds, const float* __restrict__ codebook,
                           uint8_t* __restrict__ packed, float* __restrict__ mu_out, float* __restrict__ sigma_out,
-                          float* __restrict__ codesum_out, int* status, const __grid_constant__ UnpackJobs jobs) {
+                          float* __restrict__ codesum_out, int one_fma, int* status, const __grid_constant__ UnpackJobs jobs) {
   pdl_launch_dependents();   // the next kernel of the stream may start its set-up
   if (static_cast<int>(blockIdx.x) < jobs.blocks) {
     unpack_jobs_block(jobs);
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(AqtShape<T, WRITE_PACKED>::kThreads, AqtShape<
       }
     }
     if (WRITE_XHAT) {
-      const GroupRecon g = group_recon(st, gp);
+      const GroupRecon g = group_recon(st, gp, one_fma != 0);
       if constexpr (sizeof(XH) == 2) {
         if (sizeof(T) == 4) __syncwarp();                    // the fp16 rows overlap other lanes' fp32 rows
         uint32_t w[32 / LPG];

@@ -140,17 +140,17 @@ int grid_for(long long work_items, int per_block, int blocks_per_sm) {
 template <typename T, int BITS, int PRE = 0>
 cudaError_t launch_act_quant(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed,
                              float* mu, float* sg, float* cs, void* xhat, int xhat_dtype, cudaStream_t st,
-                             const arcq::UnpackJobs& jobs) {
+                             int one_fma, const arcq::UnpackJobs& jobs) {
   const int grid = grid_for((groups + 3) / 4, 8, 8) + jobs.blocks;
   const T* xt = static_cast<const T*>(x);
   if (xhat == nullptr) {
-    launch_pdl(arcq::act_quant_kernel<T, BITS, float, false, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<float*>(nullptr), jobs);
+    launch_pdl(arcq::act_quant_kernel<T, BITS, float, false, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<float*>(nullptr), one_fma, jobs);
   } else if (xhat_dtype == ARCQ_DT_F32) {
-    launch_pdl(arcq::act_quant_kernel<T, BITS, float, true, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<float*>(xhat), jobs);
+    launch_pdl(arcq::act_quant_kernel<T, BITS, float, true, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<float*>(xhat), one_fma, jobs);
   } else if (xhat_dtype == ARCQ_DT_F16) {
-    launch_pdl(arcq::act_quant_kernel<T, BITS, __half, true, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<__half*>(xhat), jobs);
+    launch_pdl(arcq::act_quant_kernel<T, BITS, __half, true, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<__half*>(xhat), one_fma, jobs);
   } else {
-    launch_pdl(arcq::act_quant_kernel<T, BITS, __nv_bfloat16, true, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<__nv_bfloat16*>(xhat), jobs);
+    launch_pdl(arcq::act_quant_kernel<T, BITS, __nv_bfloat16, true, PRE>, grid, 256, 0, st, xt, groups, th, cb, packed, mu, sg, cs, static_cast<__nv_bfloat16*>(xhat), one_fma, jobs);
   }
   return cudaGetLastError();
 }
@@ -213,8 +213,8 @@ bool make_tensor_map_2d(CUtensorMap* tm, const void* base, CUtensorMapDataType d
 // the reconstruction, if asked for, has the input's element type or is the fp16 one of an fp32 input.
 template <typename T, int BITS, int PRE, typename XH, bool WX, bool WP>
 cudaError_t launch_act_quant_tile(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed,
-                                  float* mu, float* sg, float* cs, void* xhat, cudaStream_t st,
-                             const arcq::UnpackJobs& jobs) {
+                                  float* mu, float* sg, float* cs, void* xhat, cudaStream_t st, int one_fma,
+                                  const arcq::UnpackJobs& jobs) {
   auto k = arcq::act_quant_tile_kernel<T, BITS, XH, WX, PRE, WP>;
   using Shape = arcq::AqtShape<T, WP>;
   constexpr int smem = Shape::kSmem;
@@ -249,35 +249,35 @@ cudaError_t launch_act_quant_tile(const void* x, long long groups, const float* 
   const long long blocks = (groups + per_block - 1) / per_block;
   const long long cap = static_cast<long long>(sm_count()) * Shape::kBlocksPerSm;
   launch_pdl(k, static_cast<unsigned>((blocks < cap ? blocks : cap) + jobs.blocks), Shape::kThreads, smem, st, tm_x, tm_out, groups, th, cb,
-             packed, mu, sg, cs, status_ptr(), jobs);
+             packed, mu, sg, cs, one_fma, status_ptr(), jobs);
   return cudaGetLastError();
 }
 
 template <typename T, int BITS, int PRE, typename XH>
 cudaError_t launch_act_quant_tile_outputs(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed,
-                                          float* mu, float* sg, float* cs, void* xhat, cudaStream_t st,
-                             const arcq::UnpackJobs& jobs) {
-  if (xhat == nullptr) return launch_act_quant_tile<T, BITS, PRE, XH, false, true>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, jobs);
-  if (packed == nullptr) return launch_act_quant_tile<T, BITS, PRE, XH, true, false>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, jobs);
-  return launch_act_quant_tile<T, BITS, PRE, XH, true, true>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, jobs);
+                                          float* mu, float* sg, float* cs, void* xhat, cudaStream_t st, int one_fma,
+                                  const arcq::UnpackJobs& jobs) {
+  if (xhat == nullptr) return launch_act_quant_tile<T, BITS, PRE, XH, false, true>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, one_fma, jobs);
+  if (packed == nullptr) return launch_act_quant_tile<T, BITS, PRE, XH, true, false>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, one_fma, jobs);
+  return launch_act_quant_tile<T, BITS, PRE, XH, true, true>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, one_fma, jobs);
 }
 
 template <typename T, int BITS, int PRE>
 cudaError_t dispatch_act_quant_tile(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed, float* mu,
-                                    float* sg, float* cs, void* xhat, bool xhat_f16, cudaStream_t st,
-                             const arcq::UnpackJobs& jobs) {
+                                    float* sg, float* cs, void* xhat, bool xhat_f16, cudaStream_t st, int one_fma,
+                                  const arcq::UnpackJobs& jobs) {
   if constexpr (sizeof(T) == 4) {
     if (xhat != nullptr && xhat_f16)
-      return launch_act_quant_tile_outputs<T, BITS, PRE, __half>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, jobs);
+      return launch_act_quant_tile_outputs<T, BITS, PRE, __half>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, one_fma, jobs);
   }
-  return launch_act_quant_tile_outputs<T, BITS, PRE, T>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, jobs);
+  return launch_act_quant_tile_outputs<T, BITS, PRE, T>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, one_fma, jobs);
 }
 
 template <typename T, int PRE>
 cudaError_t dispatch_act_quant_bits(int bits, const void* x, int x_dtype, long long groups, const float* th,
                                     const float* cb, uint8_t* packed, float* mu, float* sg, float* cs, void* xhat,
-                                    int xhat_dtype, cudaStream_t st,
-                             const arcq::UnpackJobs& jobs) {
+                                    int xhat_dtype, cudaStream_t st, int one_fma,
+                                  const arcq::UnpackJobs& jobs) {
   // The one-thread-per-group kernel needs enough groups to fill the machine (148 SMs x 4 blocks x 128
   // threads); below that the 8-lanes-per-group kernel has 8 times the parallelism and lower latency.
   const long long min_groups = opt(O_AQ2_MIN_GROUPS) > 0 ? opt(O_AQ2_MIN_GROUPS) : static_cast<long long>(sm_count()) * 256;
@@ -287,15 +287,15 @@ cudaError_t dispatch_act_quant_bits(int bits, const void* x, int x_dtype, long l
                     (xhat == nullptr || ((xhat_dtype == x_dtype || (x_dtype == ARCQ_DT_F32 && xhat_f16)) && aligned(xhat, 16)));
   if (tile) {
     switch (bits) {
-      case 4: return dispatch_act_quant_tile<T, 4, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st, jobs);
-      case 3: return dispatch_act_quant_tile<T, 3, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st, jobs);
-      default: return dispatch_act_quant_tile<T, 2, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st, jobs);
+      case 4: return dispatch_act_quant_tile<T, 4, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st, one_fma, jobs);
+      case 3: return dispatch_act_quant_tile<T, 3, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st, one_fma, jobs);
+      default: return dispatch_act_quant_tile<T, 2, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st, one_fma, jobs);
     }
   }
   switch (bits) {
-    case 4: return launch_act_quant<T, 4, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st, jobs);
-    case 3: return launch_act_quant<T, 3, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st, jobs);
-    default: return launch_act_quant<T, 2, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st, jobs);
+    case 4: return launch_act_quant<T, 4, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st, one_fma, jobs);
+    case 3: return launch_act_quant<T, 3, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st, one_fma, jobs);
+    default: return launch_act_quant<T, 2, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_dtype, st, one_fma, jobs);
   }
 }
 
@@ -769,6 +769,10 @@ int arcq_device_status(void) {
   return v;
 }
 
+// Layers whose packed rows are no multiple of 16 bytes (3 bits, an odd number of groups) have always been multiplied by
+// arcq_packed_gemm, which rebuilds both operands in fp32 and rounds once.  The other routes keep its operands.
+static int fp32_rebuild(int64_t K, int bits) { return K * bits / 8 % 16 != 0; }
+
 // The unpack jobs of a call as kernel argument.  Blocks of 128 threads or more, each thread taking four 16-byte chunks a
 // round: enough blocks for one round, two per SM at most (they share the SMs with the kernel's own blocks).
 static int make_unpack_jobs(const arcq_unpack_job* jobs, int n, arcq::UnpackJobs* out, int max_blocks = 0) {
@@ -783,7 +787,7 @@ static int make_unpack_jobs(const arcq_unpack_job* jobs, int n, arcq::UnpackJobs
     if (j.rows <= 0 || j.K <= 0 || j.K % 64 != 0) return fail(ARCQ_E_BAD_SHAPE, "bad shape of a weight: rows=%lld K=%lld", (long long)j.rows, (long long)j.K);
     if (!aligned(j.packed, 4) || !aligned(j.out, 16)) return fail(ARCQ_E_ALIGN, "packed codes must be 4-byte, out 16-byte aligned");
     out->job[i] = arcq::UnpackWeightJob{j.packed, j.mu, j.sigma, j.codesum, j.codebook, static_cast<__half*>(j.out),
-                                        static_cast<long long>(j.rows), static_cast<int>(j.K), j.bits};
+                                        static_cast<long long>(j.rows), static_cast<int>(j.K), j.bits, fp32_rebuild(j.K, j.bits)};
     chunks += j.rows * (j.K / 8);
   }
   const long long want = (chunks + 511) / 512, cap = max_blocks > 0 ? max_blocks : 2ll * sm_count();
@@ -791,9 +795,20 @@ static int make_unpack_jobs(const arcq_unpack_job* jobs, int n, arcq::UnpackJobs
   return ARCQ_OK;
 }
 
+// The jobs alone, where there is no kernel for them to go beside.
+static int run_unpack_jobs(const arcq_unpack_job* unpack, int n, void* stream) {
+  arcq::UnpackJobs jobs;
+  if (const int rc = make_unpack_jobs(unpack, n, &jobs)) return rc;
+  if (n == 0) return ARCQ_OK;
+  launch_pdl(arcq::unpack_jobs_kernel, jobs.blocks, 256, 0, static_cast<cudaStream_t>(stream), jobs);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(e, "unpack launch");
+  return ARCQ_OK;
+}
+
 static int act_quant_impl(int pre, const void* x, int x_dtype, int64_t M, int64_t K, const float* thresholds,
                           const float* codebook, int bits, int group_size, uint8_t* packed_out, float* mu_out,
-                          float* sigma_out, float* codesum_out, void* xhat_out, int xhat_dtype,
+                          float* sigma_out, float* codesum_out, void* xhat_out, int xhat_dtype, int one_fma,
                           const arcq_unpack_job* unpack, int n_unpack, void* stream) {
   if (x == nullptr || thresholds == nullptr || codebook == nullptr) return fail(ARCQ_E_BAD_ARG, "null input pointer");
   if (packed_out == nullptr && xhat_out == nullptr) return fail(ARCQ_E_BAD_ARG, "no output requested");
@@ -818,16 +833,16 @@ static int act_quant_impl(int pre, const void* x, int x_dtype, int64_t M, int64_
   if (pre == 1) {
     if (x_dtype != ARCQ_DT_F16) return fail(ARCQ_E_UNSUPPORTED, "the fused GELU is built for fp16 input only");
     e = dispatch_act_quant_bits<__half, 1>(bits, x, x_dtype, groups, thresholds, codebook, packed_out, mu_out,
-                                           sigma_out, codesum_out, xhat_out, xhat_dtype, st, jobs);
+                                           sigma_out, codesum_out, xhat_out, xhat_dtype, st, one_fma, jobs);
   } else if (x_dtype == ARCQ_DT_F32)
     e = dispatch_act_quant_bits<float, 0>(bits, x, x_dtype, groups, thresholds, codebook, packed_out, mu_out, sigma_out,
-                                          codesum_out, xhat_out, xhat_dtype, st, jobs);
+                                          codesum_out, xhat_out, xhat_dtype, st, one_fma, jobs);
   else if (x_dtype == ARCQ_DT_F16)
     e = dispatch_act_quant_bits<__half, 0>(bits, x, x_dtype, groups, thresholds, codebook, packed_out, mu_out, sigma_out,
-                                           codesum_out, xhat_out, xhat_dtype, st, jobs);
+                                           codesum_out, xhat_out, xhat_dtype, st, one_fma, jobs);
   else
     e = dispatch_act_quant_bits<__nv_bfloat16, 0>(bits, x, x_dtype, groups, thresholds, codebook, packed_out, mu_out,
-                                                  sigma_out, codesum_out, xhat_out, xhat_dtype, st, jobs);
+                                                  sigma_out, codesum_out, xhat_out, xhat_dtype, st, one_fma, jobs);
   if (e != cudaSuccess) return cuda_fail(e, "act_quant launch");
   return ARCQ_OK;
 }
@@ -836,21 +851,21 @@ int arcq_act_quant(const void* x, int x_dtype, int64_t M, int64_t K, const float
                    int bits, int group_size, uint8_t* packed_out, float* mu_out, float* sigma_out, float* codesum_out,
                    void* xhat_out, int xhat_dtype, void* stream) {
   return act_quant_impl(0, x, x_dtype, M, K, thresholds, codebook, bits, group_size, packed_out, mu_out, sigma_out,
-                        codesum_out, xhat_out, xhat_dtype, nullptr, 0, stream);
+                        codesum_out, xhat_out, xhat_dtype, 0, nullptr, 0, stream);
 }
 
 int arcq_gelu_act_quant(const void* x, int x_dtype, int64_t M, int64_t K, const float* thresholds,
                         const float* codebook, int bits, int group_size, uint8_t* packed_out, float* mu_out,
                         float* sigma_out, float* codesum_out, void* xhat_out, int xhat_dtype, void* stream) {
   return act_quant_impl(1, x, x_dtype, M, K, thresholds, codebook, bits, group_size, packed_out, mu_out, sigma_out,
-                        codesum_out, xhat_out, xhat_dtype, nullptr, 0, stream);
+                        codesum_out, xhat_out, xhat_dtype, 0, nullptr, 0, stream);
 }
 
 int arcq_act_quant_unpack(int pre_gelu, const void* x, int x_dtype, int64_t M, int64_t K, const float* thresholds,
                           const float* codebook, int bits, int group_size, void* xhat_out, int xhat_dtype,
                           const arcq_unpack_job* unpack, int n_unpack, void* stream) {
   return act_quant_impl(pre_gelu != 0, x, x_dtype, M, K, thresholds, codebook, bits, group_size, nullptr, nullptr, nullptr, nullptr,
-                        xhat_out, xhat_dtype, unpack, n_unpack, stream);
+                        xhat_out, xhat_dtype, fp32_rebuild(K, bits), unpack, n_unpack, stream);
 }
 
 int arcq_packed_gemm(const uint8_t* packed_x, const float* mu_a, const float* sigma_a, const float* codesum_a,
@@ -1159,10 +1174,7 @@ static int dense_weight_gemm_impl(const void* xhat, const void* w16, const float
     return launch_pair_dense_gemm(pc, xhat, w16, bias, M, N, K, y, y_dtype, stream, nullptr, jobs);
   }
   // no pair configuration (or nothing to multiply): the unpack by its own kernel
-  for (int i = 0; i < n_unpack; ++i) {
-    const arcq_unpack_job& j = unpack[i];
-    if (const int rc = arcq_unpack_weight_f16(j.packed, j.mu, j.sigma, j.codesum, j.codebook, j.bits, 64, j.rows, j.K, j.out, stream)) return rc;
-  }
+  if (const int rc = run_unpack_jobs(unpack, n_unpack, stream)) return rc;
   if (M == 0) return ARCQ_OK;
   return launch_ws_gemm(true, xhat, w16, nullptr, nullptr, nullptr, nullptr, bias, 4, M, N, K, y, y_dtype, stream);
 }
@@ -1245,7 +1257,7 @@ int arcq_dense_weight_gemm_prefetch(const void* xhat, const void* w16, const flo
     return fail(ARCQ_E_ALIGN, "xhat, w16 and y must be 16-byte aligned");
   const arcq::UnpackWeightJob job = {next_packed, next_mu, next_sigma, next_codesum, next_codebook,
                                      static_cast<__half*>(next_out), static_cast<long long>(next_rows),
-                                     static_cast<int>(next_K), next_bits};
+                                     static_cast<int>(next_K), next_bits, 0};
   PairDenseConfig pc;
   if (M > 0 && choose_pair_dense_config(M, N, K, y_dtype == ARCQ_DT_F32, &pc))
     return launch_pair_dense_gemm(pc, xhat, w16, bias, M, N, K, y, y_dtype, stream, &job);
@@ -1293,17 +1305,28 @@ int arcq_add_layernorm_strided(const void* x, const void* y, const float* gamma,
   return ARCQ_OK;
 }
 
+static int layernorm_quant_impl(const void* x, const void* y, const float* gamma, const float* beta, float eps, int64_t M, int64_t K,
+                                const float* thresholds, const float* codebook, int bits, int group_size, void* sum_out, void* h_out,
+                                void* xhat, int one_fma, const arcq_unpack_job* unpack, int n_unpack, void* stream);
+
 int arcq_add_layernorm_act_quant(const void* x, const void* y, const float* gamma, const float* beta, float eps,
                                  int64_t M, int64_t K, const float* thresholds, const float* codebook, int bits,
                                  int group_size, void* sum_out, void* h_out, void* xhat, void* stream) {
-  return arcq_add_layernorm_act_quant_unpack(x, y, gamma, beta, eps, M, K, thresholds, codebook, bits, group_size, sum_out, h_out,
-                                             xhat, nullptr, 0, stream);
+  return layernorm_quant_impl(x, y, gamma, beta, eps, M, K, thresholds, codebook, bits, group_size, sum_out, h_out, xhat, 0, nullptr,
+                              0, stream);
 }
 
 int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const float* gamma, const float* beta, float eps,
                                         int64_t M, int64_t K, const float* thresholds, const float* codebook, int bits,
                                         int group_size, void* sum_out, void* h_out, void* xhat,
                                         const arcq_unpack_job* unpack, int n_unpack, void* stream) {
+  return layernorm_quant_impl(x, y, gamma, beta, eps, M, K, thresholds, codebook, bits, group_size, sum_out, h_out, xhat,
+                              fp32_rebuild(K, bits), unpack, n_unpack, stream);
+}
+
+static int layernorm_quant_impl(const void* x, const void* y, const float* gamma, const float* beta, float eps, int64_t M, int64_t K,
+                                const float* thresholds, const float* codebook, int bits, int group_size, void* sum_out, void* h_out,
+                                void* xhat, int one_fma, const arcq_unpack_job* unpack, int n_unpack, void* stream) {
   if (x == nullptr || gamma == nullptr || beta == nullptr || thresholds == nullptr || codebook == nullptr || xhat == nullptr)
     return fail(ARCQ_E_BAD_ARG, "null pointer argument");
   if (bits < 2 || bits > 4) return fail(ARCQ_E_BAD_ARG, "bits must be 2, 3 or 4, got %d", bits);
@@ -1332,7 +1355,7 @@ int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const floa
       const unsigned grid2 = static_cast<unsigned>((tiles2 < cap2 ? tiles2 : cap2) + jobs.blocks);
 #define ARCQ_LAUNCH_LNQ_ROWS(LN, B, HASY)                                                                            \
   launch_pdl(arcq::add_layernorm_act_quant_rows_kernel<LN, B, HASY>, grid2, arcq::kLnqRowsThreads, 0, st, xs, ys, gamma, beta, eps,     \
-             static_cast<long long>(M), thresholds, codebook, so2, ho2, xo2, jobs)
+             static_cast<long long>(M), thresholds, codebook, so2, ho2, xo2, one_fma, jobs)
 #define ARCQ_LNQ_ROWS_BITS(LN, HASY)                                                                                  \
   do {                                                                                                                \
     if (bits == 4) ARCQ_LAUNCH_LNQ_ROWS(LN, 4, HASY);                                                                  \
@@ -1364,7 +1387,7 @@ int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const floa
     return fail(ARCQ_E_CUDA, "cuTensorMapEncodeTiled failed for the reconstruction");
 #define ARCQ_LAUNCH_LNQ(LN, B, HASY)                                                                                   \
   launch_pdl(arcq::add_layernorm_act_quant_kernel<LN, B, HASY>, grid, arcq::kLnqThreads, smem, st, tm_out, xh, yh, gamma, \
-             beta, eps, static_cast<long long>(M), thresholds, codebook, so, ho, jobs)
+             beta, eps, static_cast<long long>(M), thresholds, codebook, so, ho, one_fma, jobs)
 #define ARCQ_LNQ_BITS(LN, HASY)                                                                                         \
   do {                                                                                                                  \
     if (bits == 4) ARCQ_LAUNCH_LNQ(LN, 4, HASY);                                                                         \

@@ -105,6 +105,10 @@ __global__ void dequant_kernel(const uint8_t* __restrict__ packed, const float* 
 // cb16 = fp16(cb[c]) and one half-precision fused multiply-add: bit for bit the weight the packed-weight
 // GEMM kernels rebuild in shared memory, written out so that a dense GEMM can read it by TMA.
 // One thread per chunk of 8 codes (16 bytes of output); groups of 64.
+// `fp32_form`: fp16(sigma * cb[c] + mu') with everything in fp32 up to the one rounding, which is what arcq_packed_gemm rebuilds:
+// the weight of layers whose packed rows are no multiple of 16 bytes (only 3-bit rows of an odd number of groups, so it is
+// built for 3 bits), which the packed-weight kernels do not take.  (576 x 192, 3 bits: rms relative error of the rebuilt weight
+// 2.1e-4 against 3.6e-4 in the fp16 form.)
 struct UnpackWeightJob {
   const uint8_t* packed;     // null: nothing to do
   const float* mu;
@@ -115,13 +119,14 @@ struct UnpackWeightJob {
   long long rows;
   int K;
   int bits;
+  int fp32_form;
 };
 
-// Chunks first, first + stride, ... of the job; `s_cb` holds the 16 codebook values in fp16.  Four chunks per
-// round, all their loads issued before the first result is used: a caller with few warps (the spare warps of a
+// Chunks first, first + stride, ... of the job; `s_cb` holds the 16 codebook values, of type CB: __half, or float for the
+// fp32 form.  Four chunks per round, all their loads issued before the first result is used: a caller with few warps (the spare warps of a
 // GEMM kernel) has nothing else to hide the load latency with.
-template <int BITS>
-__device__ __forceinline__ void unpack_weight_f16_chunks(const UnpackWeightJob& j, const __half* s_cb, long long first,
+template <int BITS, typename CB>
+__device__ __forceinline__ void unpack_weight_f16_chunks(const UnpackWeightJob& j, const CB* s_cb, long long first,
                                                          long long stride) {
   const int chunks = j.K / 8;
   const int G = j.K / 64;
@@ -149,14 +154,24 @@ __device__ __forceinline__ void unpack_weight_f16_chunks(const UnpackWeightJob& 
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (off[u] < 0) continue;
-      const __half2 f2 = __floats2half2_rn(sg[u], fmaf(-sg[u], cs[u] * (1.0f / 64.0f), mu[u]));
-      const __half2 s2 = __low2half2(f2), m2 = __high2half2(f2);
+      const float m = fmaf(-sg[u], cs[u] * (1.0f / 64.0f), mu[u]);
       uint32_t h[4];
+      if constexpr (sizeof(CB) == 4) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const __half2 v2 = __halves2half2(s_cb[(w[u] >> (8 * q)) & 15u], s_cb[(w[u] >> (8 * q + 4)) & 15u]);
-        const __half2 r2 = __hfma2(s2, v2, m2);
-        h[q] = *reinterpret_cast<const uint32_t*>(&r2);
+        for (int q = 0; q < 4; ++q) {
+          const __half2 r2 = __floats2half2_rn(fmaf(sg[u], s_cb[(w[u] >> (8 * q)) & 15u], m),
+                                               fmaf(sg[u], s_cb[(w[u] >> (8 * q + 4)) & 15u], m));
+          h[q] = *reinterpret_cast<const uint32_t*>(&r2);
+        }
+      } else {
+        const __half2 f2 = __floats2half2_rn(sg[u], m);
+        const __half2 s2 = __low2half2(f2), m2 = __high2half2(f2);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const __half2 v2 = __halves2half2(s_cb[(w[u] >> (8 * q)) & 15u], s_cb[(w[u] >> (8 * q + 4)) & 15u]);
+          const __half2 r2 = __hfma2(s2, v2, m2);
+          h[q] = *reinterpret_cast<const uint32_t*>(&r2);
+        }
       }
       *reinterpret_cast<uint4*>(j.out + off[u]) = make_uint4(h[0], h[1], h[2], h[3]);
     }
@@ -170,13 +185,16 @@ struct UnpackJobs {
   UnpackWeightJob job[2];
   int blocks;                // 0: none
 };
-// `block` of u.blocks; s_ucb: 32 values of shared memory.
-__device__ __forceinline__ void unpack_jobs_run(const UnpackJobs& u, int block, __half* s_ucb) {
+// `block` of u.blocks; s_ucb: 32 words of shared memory, 16 for the levels of each job.
+__device__ __forceinline__ void unpack_jobs_run(const UnpackJobs& u, int block, float* s_ucb) {
   const int tid = threadIdx.x;
   if (tid < 32) {
     const UnpackWeightJob& j = u.job[tid >> 4];
     const int i = tid & 15;
-    s_ucb[tid] = __float2half_rn(j.packed != nullptr && i < (1 << j.bits) ? __ldg(j.codebook + i) : 0.0f);
+    const float level = j.packed != nullptr && i < (1 << j.bits) ? __ldg(j.codebook + i) : 0.0f;
+    float* const cb = s_ucb + (tid & 16);
+    if (j.fp32_form) cb[i] = level;
+    else reinterpret_cast<__half*>(cb)[i] = __float2half_rn(level);
   }
   __syncthreads();
   pdl_wait();                // the matrices written here may still be read by the kernel before this one
@@ -185,14 +203,23 @@ __device__ __forceinline__ void unpack_jobs_run(const UnpackJobs& u, int block, 
   for (int k = 0; k < 2; ++k) {
     const UnpackWeightJob& j = u.job[k];
     if (j.packed == nullptr) break;
-    if (j.bits == 4) unpack_weight_f16_chunks<4>(j, s_ucb + 16 * k, first, stride);
-    else if (j.bits == 3) unpack_weight_f16_chunks<3>(j, s_ucb + 16 * k, first, stride);
-    else unpack_weight_f16_chunks<2>(j, s_ucb + 16 * k, first, stride);
+    const float* const cb = s_ucb + 16 * k;
+    const __half* const cb16 = reinterpret_cast<const __half*>(cb);
+    if (j.bits == 4) unpack_weight_f16_chunks<4>(j, cb16, first, stride);
+    else if (j.bits == 3 && j.fp32_form) unpack_weight_f16_chunks<3>(j, cb, first, stride);
+    else if (j.bits == 3) unpack_weight_f16_chunks<3>(j, cb16, first, stride);
+    else unpack_weight_f16_chunks<2>(j, cb16, first, stride);
   }
 }
 __device__ __forceinline__ void unpack_jobs_block(const UnpackJobs& u) {
-  __shared__ __half s_ucb[32];
+  __shared__ float s_ucb[32];
   unpack_jobs_run(u, static_cast<int>(blockIdx.x), s_ucb);
+}
+
+// The jobs on their own.
+__global__ void __launch_bounds__(256) unpack_jobs_kernel(const __grid_constant__ UnpackJobs jobs) {
+  pdl_launch_dependents();
+  unpack_jobs_block(jobs);
 }
 
 template <int BITS>
@@ -203,7 +230,7 @@ __global__ void unpack_weight_f16_kernel(const uint8_t* __restrict__ packed, con
   __shared__ __half s_cb[16];
   if (threadIdx.x < 16) s_cb[threadIdx.x] = __float2half_rn((threadIdx.x < (1 << BITS)) ? codebook[threadIdx.x] : 0.0f);
   __syncthreads();
-  const UnpackWeightJob j = {packed, mu, sigma, codesum, codebook, out, rows, K, BITS};
+  const UnpackWeightJob j = {packed, mu, sigma, codesum, codebook, out, rows, K, BITS, 0};
   unpack_weight_f16_chunks<BITS>(j, s_cb, blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x,
                                  static_cast<long long>(gridDim.x) * blockDim.x);
 }

@@ -101,7 +101,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
   if (static_cast<int>(blockIdx.x) >= 2 * p.pairs) {
     // both CTAs of such a pair: weights of layers further on, on SMs that this GEMM leaves idle
     pdl_launch_dependents();
-    unpack_jobs_run(jobs, static_cast<int>(blockIdx.x) - 2 * p.pairs, reinterpret_cast<__half*>(smem_raw));
+    unpack_jobs_run(jobs, static_cast<int>(blockIdx.x) - 2 * p.pairs, reinterpret_cast<float*>(smem_raw));
     return;
   }
   uint8_t* const sStages = smem + L.stages;

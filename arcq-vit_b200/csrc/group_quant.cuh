@@ -248,16 +248,17 @@ __device__ __forceinline__ GroupStats group_quantize(f32x2 (&v)[32 / LPG], const
   return st;
 }
 
-// mean + scale * (level - code_sum / 64) in the reference's three rounded steps
+// recon_value (act_quant.cuh) of two levels
 struct GroupRecon {
-  f32x2 mean, scale, nvm, nz;
+  f32x2 scale, a, b, c;
 };
-__device__ __forceinline__ GroupRecon group_recon(const GroupStats& st, const GroupQuantParams& p) {
-  const float vm = __fmul_rn(st.code_sum, 0.015625f);        // exact
-  return {pack2(st.mean, st.mean), pack2(st.scale, st.scale), pack2(-vm, -vm), p.nz};
+__device__ __forceinline__ GroupRecon group_recon(const GroupStats& st, const GroupQuantParams& p, bool one_fma = false) {
+  const ReconTerms t = recon_terms(st.mean, st.scale, st.code_sum, one_fma);
+  // p.nz, not the constant -0 of t.b: the product must not be contracted with the last addition (see mul2_rn)
+  return {pack2(st.scale, st.scale), pack2(t.a, t.a), one_fma ? pack2(t.b, t.b) : p.nz, pack2(t.c, t.c)};
 }
 __device__ __forceinline__ f32x2 group_recon_pair(const GroupRecon& g, f32x2 level) {
-  return add2(g.mean, mul2_rn(g.scale, add2(level, g.nvm), g.nz));
+  return add2(g.c, fma2(g.scale, add2(level, g.a), g.b));
 }
 
 // ---------------------------------------------------------------- 16-bit element types and rows in shared memory
@@ -357,7 +358,7 @@ __device__ __forceinline__ void gelu_words(uint32_t (&w)[32 / LPG], uint32_t row
 // The quantizer on a fp16 row in shared memory, in place: values in, reconstruction out.
 template <typename T, int BITS, bool GELU, int LPG>
 __device__ __forceinline__ void group_quantize_row(uint32_t row, uint32_t x7, const GroupQuantTables* t,
-                                                   const GroupQuantParams& p, GroupStats* stats = nullptr) {
+                                                   const GroupQuantParams& p, bool one_fma = false) {
   uint32_t w[32 / LPG], words[8];
   f32x2 v[32 / LPG];
   row_load<LPG>(w, row, x7);
@@ -365,11 +366,10 @@ __device__ __forceinline__ void group_quantize_row(uint32_t row, uint32_t x7, co
 #pragma unroll
   for (int i = 0; i < 32 / LPG; ++i) v[i] = sixteen_to_pair<T>(w[i]);
   const GroupStats st = group_quantize<BITS, false, LPG>(v, t, p, words);
-  const GroupRecon g = group_recon(st, p);
+  const GroupRecon g = group_recon(st, p, one_fma);
 #pragma unroll
   for (int i = 0; i < 32 / LPG; ++i) w[i] = pair_to_sixteen<T>(group_recon_pair(g, v[i]));
   row_store<LPG>(w, row, x7);
-  if (stats != nullptr) *stats = st;
 }
 
 }  // namespace arcq

@@ -68,6 +68,7 @@ struct Linear {
   const float *th, *acb, *bias;
   arcq_unpack_job job;
   int64_t weight_elems() const { return N * K; }
+  bool rows_of_16_bytes() const { return K * bits / 8 % 16 == 0; }
 };
 
 bool read_linear(PyObject* buffers, Key bias_key, const c10::Device& dev, Linear* l) {
@@ -109,7 +110,7 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Linear l;
   if (!read_linear(args[0], PyObject_IsTrue(args[2]) ? kBias : kBiasTensor, x->device(), &l)) Py_RETURN_NONE;
   const int64_t numel = x->numel();
-  if (x->size(-1) != l.K || numel == 0 || !aligned16(x->const_data_ptr())) Py_RETURN_NONE;
+  if (x->size(-1) != l.K || numel == 0 || !aligned16(x->const_data_ptr()) || (ready && !l.rows_of_16_bytes())) Py_RETURN_NONE;
   const int64_t M = numel / l.K;
   const c10::cuda::CUDAGuard guard(x->device());
   void* const st = c10::cuda::getCurrentCUDAStream().stream();
@@ -425,16 +426,17 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
           "arcq_assemble_tokens");
   }
   const at::Half* y = nullptr;
-  int64_t asked[2] = {0, 0};            // the shape of fc1 that `fused` holds for
-  bool fused = false;
+  int64_t asked[2] = {0, 0};            // the shape of fc1 that `applies` holds for
+  bool applies = false;
   for (size_t i = 0; i < depth; ++i) {
     const VitBlock& b = p->blocks[i];
     const Linear *qkv = &lin[4 * i], *proj = qkv + 1, *fc1 = qkv + 2, *fc2 = qkv + 3;
     if (asked[0] != fc1->N || asked[1] != fc1->K) {
-      fused = arcq_dense_weight_gemm_gelu_quant_applies(M, fc1->N, fc1->K) != 0;
+      applies = arcq_dense_weight_gemm_gelu_quant_applies(M, fc1->N, fc1->K) != 0;
       asked[0] = fc1->N;
       asked[1] = fc1->K;
     }
+    const bool fused = applies && fc2->rows_of_16_bytes();     // the fused form reconstructs in three steps only
     arcq_unpack_job jobs[2];
     norm_quant(y, gb[4 * i], gb[4 * i + 1], b.norm1.eps, qkv, 0);
     gemm(xhat, *qkv, mid, jobs, jobs_of(qkv, done, 2, jobs));
@@ -442,8 +444,8 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
       const at::Tensor t = at::from_blob(mid, {B, T, 3, p->heads, D / p->heads}, at::TensorOptions().dtype(at::kHalf).device(dev));
       const at::Tensor r = t.permute({2, 0, 3, 1, 4});
       const at::Tensor o = at::scaled_dot_product_attention(r[0], r[1], r[2]).transpose(1, 2).reshape({M, D});
-      check(arcq_act_quant(o.const_data_ptr(), ARCQ_DT_F16, M, D, proj->th, proj->acb, proj->bits, 64, nullptr, nullptr, nullptr, nullptr,
-                           xhat, ARCQ_DT_F16, st),
+      check(arcq_act_quant_unpack(0, o.const_data_ptr(), ARCQ_DT_F16, M, D, proj->th, proj->acb, proj->bits, 64, xhat, ARCQ_DT_F16,
+                                  nullptr, 0, st),
             "arcq_act_quant");
     }
     last_gemm(xhat, *proj, branch, fc1, fused);
@@ -455,8 +457,7 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
             "arcq_dense_weight_gemm_gelu_quant");
     } else {
       gemm(xhat, *fc1, mid, jobs, n);
-      check(arcq_gelu_act_quant(mid, ARCQ_DT_F16, M, fc2->K, fc2->th, fc2->acb, fc2->bits, 64, nullptr, nullptr, nullptr, nullptr, xhat4,
-                                ARCQ_DT_F16, st),
+      check(arcq_act_quant_unpack(1, mid, ARCQ_DT_F16, M, fc2->K, fc2->th, fc2->acb, fc2->bits, 64, xhat4, ARCQ_DT_F16, nullptr, 0, st),
             "arcq_gelu_act_quant");
     }
     last_gemm(xhat4, *fc2, branch, i + 1 < depth ? qkv + 4 : nullptr, 0);

@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(kLnqThreads, 4)
                                    const __half* __restrict__ y, const float* __restrict__ gamma,
                                    const float* __restrict__ beta, float eps, long long M,
                                    const float* __restrict__ thresholds, const float* __restrict__ codebook,
-                                   __half* __restrict__ sum_out, __half* __restrict__ h_out,
+                                   __half* __restrict__ sum_out, __half* __restrict__ h_out, int one_fma,
                                    const __grid_constant__ UnpackJobs jobs) {
   pdl_launch_dependents();   // the next kernel of the stream may start its set-up
   if (static_cast<int>(blockIdx.x) < jobs.blocks) {
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(kLnqThreads, 4)
 
     // ---- phase 2: the activation quantizer on h, one thread per group, in place; a warp sends its 32 rows out by TMA
     // (rows of the last tile beyond the matrix hold stale values; the store clips them)
-    if (tid < ngroups) group_quantize_row<__half, BITS, false, 1>(smem_u32(s_rows) + tid * 128, lane & 7, tables, gp);
+    if (tid < ngroups) group_quantize_row<__half, BITS, false, 1>(smem_u32(s_rows) + tid * 128, lane & 7, tables, gp, one_fma != 0);
     fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) {
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kLnqRowsThreads) add_layernorm_act_quant_rows_
                                                                           const float* __restrict__ codebook,
                                                                           __half* __restrict__ sum_out,
                                                                           __half* __restrict__ h_out,
-                                                                          __half* __restrict__ xhat,
+                                                                          __half* __restrict__ xhat, int one_fma,
                                                                           const __grid_constant__ UnpackJobs jobs) {
   pdl_launch_dependents();
   if (static_cast<int>(blockIdx.x) < jobs.blocks) {
@@ -216,11 +216,11 @@ __global__ void __launch_bounds__(kLnqRowsThreads) add_layernorm_act_quant_rows_
       a2 = __fadd_rn(cv[2], cv[6]); a3 = __fadd_rn(cv[3], cv[7]);
       part = __fadd_rn(__fadd_rn(__fadd_rn(a0, a1), a2), a3);
       const float code_sum = octet_chain_sum(part, octet_base);
-      const float vm = __fdiv_rn(code_sum, 64.0f);
+      const ReconTerms rt = recon_terms(mean, scale, code_sum, one_fma != 0);
       if (valid) {
         __half* og = xhat + row * K + g * 64 + l8;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) og[8 * c] = __float2half_rn(__fadd_rn(mean, __fmul_rn(scale, __fsub_rn(cv[c], vm))));
+        for (int c = 0; c < 8; ++c) og[8 * c] = __float2half_rn(recon_value(rt, scale, cv[c]));
       }
     }
     __syncthreads();   // the tile's rows in shared memory are free for the next tile

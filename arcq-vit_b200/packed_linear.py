@@ -272,8 +272,9 @@ class ARCQPackedLinearOnTheFly(_KeepsFp32Metadata):
     #   "auto":   unpacked by blocks of the quantizer's own launch into a scratch matrix of the call (one native call a
     #             layer).  Inputs that call does not take (other dtypes or devices, non-contiguous) go on as "staged" when
     #             the model has a stager and the GEMM has at least WeightStager.min_rows rows, else as "packed".
-    # All forms produce the same bits: the unpack kernel writes exactly the fp16 values the packed-weight
-    # kernels rebuild on chip.
+    # All forms produce the same bits: what is unpacked is exactly the fp16 values the packed-weight kernels rebuild on
+    # chip.  Layers whose packed rows are no multiple of 16 bytes (3 bits, an odd number of groups) take the native call, or
+    # else ``ops.arcq_linear_forward`` on the packed codes of both sides, whatever the form; those two give the same bits.
     weight_form = os.environ.get("ARCQ_WEIGHT_FORM", "auto")
     _scratch: dict = {}
 
@@ -306,7 +307,8 @@ class ARCQPackedLinearOnTheFly(_KeepsFp32Metadata):
         """True if ``forward(x_hat, pre_quantized=True)`` is available: the layer runs the two-kernel route whose
         GEMM reads the reconstructed activation, so a caller may produce that activation itself
         (``ops.add_layernorm_quant`` with this layer's ``activation_thresholds`` / ``activation_codebook``)."""
-        return self.group_size == 64 and self.in_features <= 1024 and self.out_features % 16 == 0
+        return (self.group_size == 64 and self.in_features <= 1024
+                and ops.packed_weight_gemm_supported(self.in_features, self.out_features, self.bits, self.group_size))
 
     def forward(self, x: torch.Tensor, pre_gelu: bool = False, pre_quantized: bool = False) -> torch.Tensor:
         """``pre_gelu=True``: x is the pre-activation of the GELU in front of this layer; the result
@@ -324,13 +326,10 @@ class ARCQPackedLinearOnTheFly(_KeepsFp32Metadata):
             raise ValueError(f"expected last dim {self.in_features}, got {shape[-1]}")
         x2 = x.reshape(-1, self.in_features).to(device=self.packed_weight_codes.device, dtype=torch.float16).contiguous()
         bias = self.bias_tensor if self.bias_tensor.numel() else None
-        if self.group_size == 64 and self.out_features % 16 == 0:
+        if ops.packed_weight_gemm_supported(self.in_features, self.out_features, self.bits, self.group_size):
             # the reference's own data flow: fp16 activation quantised and reconstructed (its step 2),
             # then weight unpack + contraction + bias (its steps 3-5) in one persistent kernel
             route = self._weight_route(x2.shape[0])
-            if route == "packed" and not ops.packed_weight_gemm_supported(self.in_features, self.out_features, self.bits,
-                                                                          self.group_size):
-                route = "dense"         # e.g. 3-bit rows of 72 bytes: the packed-weight kernels want multiples of 16
             if route == "staged":
                 w16, ready, prefetch = self._stager.stage(self)     # also arranges the next layer's unpack
             x_hat = x2 if pre_quantized else ops.quantize_activation_dequant(
@@ -350,7 +349,7 @@ class ARCQPackedLinearOnTheFly(_KeepsFp32Metadata):
                                            self.weight_code_sum, self.weight_codebook, bias, self.bits,
                                            self.group_size, torch.float16)
         else:
-            # output widths the persistent kernels do not take: packed codes on both sides
+            # shapes the persistent kernels do not take (e.g. 3-bit rows of 72 bytes): packed codes on both sides
             packed_x, mu, sg, cs = ops.quantize_activation(x2, self.activation_thresholds, self.activation_codebook,
                                                            self.bits, self.group_size, True, pre_gelu)
             y = ops.arcq_linear_forward(packed_x, mu, sg, cs, self.packed_weight_codes, self.weight_center,

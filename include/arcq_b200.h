@@ -138,8 +138,10 @@ int arcq_gelu_act_quant(const void* x, int x_dtype, int64_t M, int64_t K,
                         void* xhat_out, int xhat_dtype, void* stream);
 
 /*
- * A packed weight to be unpacked by blocks of the activation path's kernels (what arcq_unpack_weight_f16 writes):
- * packed [rows, K*bits/8], statistics fp32 [rows, K/64], out fp16 [rows, K], 16-byte aligned; group size 64.
+ * A packed weight to be unpacked by blocks of the activation path's kernels: packed [rows, K*bits/8], statistics fp32
+ * [rows, K/64], out fp16 [rows, K], 16-byte aligned; group size 64.  Written is the fp16 matrix that the GEMM on packed codes
+ * multiplies with: arcq_packed_weight_gemm's (what arcq_unpack_weight_f16 writes) where packed rows are a multiple of 16 bytes,
+ * else arcq_packed_gemm's, fp16(fma(sigma, level, mu - sigma * codesum / 64)) in fp32 with one rounding.
  * The linear that consumes the quantizer's output needs its weight next: unpacked beside the quantizer it costs no
  * launch of its own.  Up to two jobs a call; `out` must not be read by any kernel still running before the call.
  */
@@ -157,7 +159,8 @@ typedef struct arcq_unpack_job {
 /*
  * arcq_act_quant (pre_gelu = 0) or arcq_gelu_act_quant (1) with reconstruction output only, plus unpack jobs: steps 2
  * and 3 of ARCQPackedLinearOnTheFly.forward (FQ/fair_qat/arcq_packed_on_the_fly.py:143-158: dequant_activation_triton,
- * unpack_weight_triton) in one launch.
+ * unpack_weight_triton) in one launch.  K and bits are the layer's: where its packed rows are no multiple of 16 bytes, xhat is
+ * the operand that arcq_packed_gemm rebuilds (one fma per value) instead of the three rounded steps.
  */
 int arcq_act_quant_unpack(int pre_gelu, const void* x, int x_dtype, int64_t M, int64_t K, const float* thresholds,
                           const float* codebook, int bits, int group_size, void* xhat_out, int xhat_dtype,
@@ -259,7 +262,7 @@ int arcq_add_layernorm_act_quant(const void* x, const void* y, const float* gamm
                                  int64_t M, int64_t K, const float* thresholds, const float* codebook, int bits,
                                  int group_size, void* sum_out, void* h_out, void* xhat, void* stream);
 
-/* The same with unpack jobs (see arcq_unpack_job) taken along by the launch. */
+/* The same with unpack jobs (see arcq_unpack_job) taken along by the launch; xhat as in arcq_act_quant_unpack. */
 int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const float* gamma, const float* beta, float eps,
                                         int64_t M, int64_t K, const float* thresholds, const float* codebook, int bits,
                                         int group_size, void* sum_out, void* h_out, void* xhat,

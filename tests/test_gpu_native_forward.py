@@ -1,4 +1,4 @@
-"""What only the one-call ViT forward uses, against the separate operators and the Python forward it merges: same bits."""
+"""What only the native host path uses, against the separate operators and the Python code it stands for: same bits."""
 import pytest
 import torch
 
@@ -51,4 +51,35 @@ def test_native_forward_equals_the_python_forward(pkg, cuda_device, name, bits, 
         monkeypatch.setattr(pkg.vit.VisionTransformer, "_forward_native", lambda self, x: None)
         for b, y in got.items():
             assert torch.equal(y, model(images[:b])), f"batch {b}"
+    assert pkg.ops.device_status() == 0
+
+
+def _packed_layer(pkg, bits, K, N, dev, on_the_fly, bias=True):
+    gen = torch.Generator().manual_seed(K + N + bits)
+    linear = torch.nn.Linear(K, N, bias=bias)
+    with torch.no_grad():
+        linear.weight.copy_(torch.randn(N, K, generator=gen) * 0.03)
+        if bias:
+            linear.bias.copy_(torch.randn(N, generator=gen) * 0.1)
+    cb, th = _codebook(gen, bits, dev)
+    return pkg.pack_linear(linear.to(dev), bits, cb, th, group_size=64, on_the_fly=on_the_fly), gen
+
+
+# packed rows of 24, 72, 120 and 192 bytes (the last a multiple of 16); rows of x on both sides of the quantizers' size rule
+@pytest.mark.parametrize("K,N", [(64, 64), (192, 576), (320, 48), (512, 192)])
+@pytest.mark.parametrize("M", [1, 197, 12700])
+def test_three_bit_rows_of_any_length_equal_the_packed_operators(pkg, cuda_device, K, N, M):
+    """The packed linears against quantize_activation + arcq_linear_forward on their buffers, which rebuilds rows that are no
+    multiple of 16 bytes in fp32 with one rounding: same bits."""
+    for on_the_fly, dtype in ((True, torch.float16), (False, torch.float32), (False, torch.bfloat16)):
+        layer, gen = _packed_layer(pkg, 3, K, N, cuda_device, on_the_fly)
+        x = torch.randn(M, K, generator=gen).to(dtype).to(cuda_device)
+        b = layer._buffers
+        codes = pkg.ops.quantize_activation(x, layer.activation_thresholds, layer.activation_codebook, 3, 64)
+        want = pkg.ops.arcq_linear_forward(*codes, b["packed_weight_codes"], b["weight_center"], b["weight_scale"], b["weight_code_sum"],
+                                           b["activation_codebook"], b["weight_codebook"], b.get("bias", b.get("bias_tensor")), 3, 64, K, N,
+                                           torch.float16 if on_the_fly else torch.float32)
+        assert torch.equal(layer(x), want)
+        wide = torch.empty(M, K + 8, dtype=dtype, device=cuda_device)[:, :K].copy_(x)      # not contiguous: the Python route
+        assert torch.equal(layer(wide), want)
     assert pkg.ops.device_status() == 0
