@@ -56,6 +56,8 @@ def load() -> ctypes.CDLL:
     lib.arcq_dense_weight_gemm.argtypes = [vp, vp, vp, i64, i64, i64, vp, ci, vp]
     lib.arcq_packed_linear_static_scratch.argtypes = lib.arcq_packed_weight_gemm.argtypes
     lib.arcq_add_layernorm.argtypes = [vp, vp, vp, vp, ctypes.c_float, i64, i64, vp, vp, vp]
+    lib.arcq_add_layernorm_strided.argtypes = [vp, vp, vp, vp, ci, ctypes.c_float, i64, i64, i64, vp, vp, vp]
+    lib.arcq_add_layernorm_act_quant_unpack.argtypes = [vp, vp, vp, vp, ci, ctypes.c_float, i64, i64, vp, vp, ci, ci, vp, vp, vp, ci, vp, ci, vp]
     lib.arcq_add_layernorm_act_quant.argtypes = [vp, vp, vp, vp, ctypes.c_float, i64, i64, vp, vp, ci, ci, vp, vp, vp, vp]
     lib.arcq_attention.argtypes = [vp, i64, i64, i64, ci, vp, vp]
     lib.arcq_attention_act_quant.argtypes = [vp, i64, i64, i64, ci, vp, vp, ci, ci, vp, vp]

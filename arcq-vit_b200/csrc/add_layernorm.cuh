@@ -9,11 +9,34 @@
 
 namespace arcq {
 
+// gamma and beta in the type the module holds them in, so that nobody has to keep converted copies: the ARCQ_DT_* numbers.
+struct NormParams {
+  const void* gamma;
+  const void* beta;
+  int dtype;          // 0 fp32, 1 fp16, 2 bf16
+};
+// values 8 * chunk .. 8 * chunk + 7 as fp32
+__device__ __forceinline__ void load_norm_chunk(const void* p, int dtype, int chunk, float (&v)[8]) {
+  if (dtype == 0) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p) + 2 * chunk), b = __ldg(reinterpret_cast<const float4*>(p) + 2 * chunk + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {
+    const uint4 u = __ldg(reinterpret_cast<const uint4*>(p) + chunk);
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+      v[2 * j] = dtype == 1 ? f.x : __uint_as_float(w[j] << 16);
+      v[2 * j + 1] = dtype == 1 ? f.y : __uint_as_float(w[j] & 0xFFFF0000u);
+    }
+  }
+}
+
 constexpr int kLnMaxChunks = 8;  // 16-byte chunks per lane: rows up to 32 * 8 * 8 = 2048 values
 
 __global__ void __launch_bounds__(256) add_layernorm_kernel(const __half* __restrict__ x, const __half* __restrict__ y,
-                                                            const float* __restrict__ gamma,
-                                                            const float* __restrict__ beta, float eps, long long M, int K,
+                                                            const NormParams np, float eps, long long M, int K,
                                                             long long ld, __half* __restrict__ sum_out,
                                                             __half* __restrict__ h_out) {
   pdl_launch_dependents();   // the next kernel of the stream may start its set-up
@@ -80,12 +103,9 @@ __global__ void __launch_bounds__(256) add_layernorm_kernel(const __half* __rest
     for (int i = 0; i < kLnMaxChunks; ++i) {
       const int c = lane + 32 * i;
       if (c < chunks) {
-        const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma) + 2 * c);
-        const float4 g1 = __ldg(reinterpret_cast<const float4*>(gamma) + 2 * c + 1);
-        const float4 b0 = __ldg(reinterpret_cast<const float4*>(beta) + 2 * c);
-        const float4 b1 = __ldg(reinterpret_cast<const float4*>(beta) + 2 * c + 1);
-        const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-        const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+        float gg[8], bb[8];
+        load_norm_chunk(np.gamma, np.dtype, c, gg);
+        load_norm_chunk(np.beta, np.dtype, c, bb);
         uint4 o;
         __half2* oh = reinterpret_cast<__half2*>(&o);
 #pragma unroll
@@ -192,19 +212,11 @@ __device__ __forceinline__ void layernorm_row(const __half* __restrict__ x, cons
 
 // gamma and beta of the lane's three chunks
 template <int LANES>
-__device__ __forceinline__ void layernorm_lane_params(const float* __restrict__ gamma, const float* __restrict__ beta,
-                                                      int l, float (&gg)[3][8], float (&bb)[3][8]) {
+__device__ __forceinline__ void layernorm_lane_params(const NormParams& np, int l, float (&gg)[3][8], float (&bb)[3][8]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const int c = l + LANES * i;
-    const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma) + 2 * c);
-    const float4 g1 = __ldg(reinterpret_cast<const float4*>(gamma) + 2 * c + 1);
-    const float4 b0 = __ldg(reinterpret_cast<const float4*>(beta) + 2 * c);
-    const float4 b1 = __ldg(reinterpret_cast<const float4*>(beta) + 2 * c + 1);
-    gg[i][0] = g0.x; gg[i][1] = g0.y; gg[i][2] = g0.z; gg[i][3] = g0.w;
-    gg[i][4] = g1.x; gg[i][5] = g1.y; gg[i][6] = g1.z; gg[i][7] = g1.w;
-    bb[i][0] = b0.x; bb[i][1] = b0.y; bb[i][2] = b0.z; bb[i][3] = b0.w;
-    bb[i][4] = b1.x; bb[i][5] = b1.y; bb[i][6] = b1.z; bb[i][7] = b1.w;
+    load_norm_chunk(np.gamma, np.dtype, l + LANES * i, gg[i]);
+    load_norm_chunk(np.beta, np.dtype, l + LANES * i, bb[i]);
   }
 }
 
@@ -213,8 +225,7 @@ __device__ __forceinline__ void layernorm_lane_params(const float* __restrict__ 
 template <int LANES>
 __global__ void __launch_bounds__(256) add_layernorm_rows_kernel(const __half* __restrict__ x,
                                                                  const __half* __restrict__ y,
-                                                                 const float* __restrict__ gamma,
-                                                                 const float* __restrict__ beta, float eps,
+                                                                 const NormParams np, float eps,
                                                                  long long M, long long ld,
                                                                  __half* __restrict__ sum_out,
                                                                  __half* __restrict__ h_out) {
@@ -223,7 +234,7 @@ __global__ void __launch_bounds__(256) add_layernorm_rows_kernel(const __half* _
   constexpr int K = LANES * 24, kRowsPerWarp = 32 / LANES;
   const int lane = threadIdx.x & 31, l = lane % LANES, sub = lane / LANES;
   float gg[3][8], bb[3][8];
-  layernorm_lane_params<LANES>(gamma, beta, l, gg, bb);
+  layernorm_lane_params<LANES>(np, l, gg, bb);
   pdl_wait();                // gamma and beta are the layer's constants; x and y may be the previous kernel's output
   const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
   const long long first = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kRowsPerWarp;

@@ -769,8 +769,8 @@ int arcq_device_status(void) {
   return v;
 }
 
-// Layers whose packed rows are no multiple of 16 bytes (3 bits, an odd number of groups) have always been multiplied by
-// arcq_packed_gemm, which rebuilds both operands in fp32 and rounds once.  The other routes keep its operands.
+// Weights whose packed rows are no multiple of 16 bytes (3 bits, an odd number of groups) have always been multiplied by
+// arcq_packed_gemm, which rebuilds them in fp32 and rounds once.  The unpacked ones are the same.
 static int fp32_rebuild(int64_t K, int bits) { return K * bits / 8 % 16 != 0; }
 
 // The unpack jobs of a call as kernel argument.  Blocks of 128 threads or more, each thread taking four 16-byte chunks a
@@ -862,10 +862,10 @@ int arcq_gelu_act_quant(const void* x, int x_dtype, int64_t M, int64_t K, const 
 }
 
 int arcq_act_quant_unpack(int pre_gelu, const void* x, int x_dtype, int64_t M, int64_t K, const float* thresholds,
-                          const float* codebook, int bits, int group_size, void* xhat_out, int xhat_dtype,
+                          const float* codebook, int bits, int group_size, void* xhat_out, int xhat_dtype, int one_fma,
                           const arcq_unpack_job* unpack, int n_unpack, void* stream) {
   return act_quant_impl(pre_gelu != 0, x, x_dtype, M, K, thresholds, codebook, bits, group_size, nullptr, nullptr, nullptr, nullptr,
-                        xhat_out, xhat_dtype, fp32_rebuild(K, bits), unpack, n_unpack, stream);
+                        xhat_out, xhat_dtype, one_fma != 0, unpack, n_unpack, stream);
 }
 
 int arcq_packed_gemm(const uint8_t* packed_x, const float* mu_a, const float* sigma_a, const float* codesum_a,
@@ -1272,13 +1272,14 @@ int arcq_dense_weight_gemm_prefetch(const void* xhat, const void* w16, const flo
 
 int arcq_add_layernorm(const void* x, const void* y, const float* gamma, const float* beta, float eps, int64_t M,
                        int64_t K, void* sum_out, void* h_out, void* stream) {
-  return arcq_add_layernorm_strided(x, y, gamma, beta, eps, M, K, K, sum_out, h_out, stream);
+  return arcq_add_layernorm_strided(x, y, gamma, beta, ARCQ_DT_F32, eps, M, K, K, sum_out, h_out, stream);
 }
 
-int arcq_add_layernorm_strided(const void* x, const void* y, const float* gamma, const float* beta, float eps, int64_t M,
-                               int64_t K, int64_t ld, void* sum_out, void* h_out, void* stream) {
+int arcq_add_layernorm_strided(const void* x, const void* y, const void* gamma, const void* beta, int param_dtype, float eps,
+                               int64_t M, int64_t K, int64_t ld, void* sum_out, void* h_out, void* stream) {
   if (x == nullptr || gamma == nullptr || beta == nullptr || h_out == nullptr)
     return fail(ARCQ_E_BAD_ARG, "null pointer argument");
+  if (param_dtype < ARCQ_DT_F32 || param_dtype > ARCQ_DT_BF16) return fail(ARCQ_E_BAD_ARG, "bad param_dtype %d", param_dtype);
   if (M < 0 || K <= 0) return fail(ARCQ_E_BAD_SHAPE, "bad shape M=%lld K=%lld", (long long)M, (long long)K);
   if (K % 8 != 0) return fail(ARCQ_E_BAD_SHAPE, "K=%lld must be a multiple of 8", (long long)K);
   if (ld < K || ld % 8 != 0) return fail(ARCQ_E_BAD_SHAPE, "row stride %lld must be a multiple of 8, at least K", (long long)ld);
@@ -1290,59 +1291,51 @@ int arcq_add_layernorm_strided(const void* x, const void* y, const float* gamma,
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const __half *xh = static_cast<const __half*>(x), *yh = static_cast<const __half*>(y);
   __half *so = static_cast<__half*>(sum_out), *ho = static_cast<__half*>(h_out);
+  const arcq::NormParams np = {gamma, beta, param_dtype};
   const bool plain = opt(O_LN_PLAIN) != 0;
   if (K == 384 && !plain) {          // 16 lanes per row, 2 rows per warp
-    launch_pdl(arcq::add_layernorm_rows_kernel<16>, grid_for(M, 16, 6), 256, 0, st, xh, yh, gamma, beta, eps, M, ld, so, ho);
+    launch_pdl(arcq::add_layernorm_rows_kernel<16>, grid_for(M, 16, 6), 256, 0, st, xh, yh, np, eps, M, ld, so, ho);
   } else if (K == 192 && !plain) {
-    launch_pdl(arcq::add_layernorm_rows_kernel<8>, grid_for(M, 32, 6), 256, 0, st, xh, yh, gamma, beta, eps, M, ld, so, ho);
+    launch_pdl(arcq::add_layernorm_rows_kernel<8>, grid_for(M, 32, 6), 256, 0, st, xh, yh, np, eps, M, ld, so, ho);
   } else if (K == 768 && !plain) {
-    launch_pdl(arcq::add_layernorm_rows_kernel<32>, grid_for(M, 8, 6), 256, 0, st, xh, yh, gamma, beta, eps, M, ld, so, ho);
+    launch_pdl(arcq::add_layernorm_rows_kernel<32>, grid_for(M, 8, 6), 256, 0, st, xh, yh, np, eps, M, ld, so, ho);
   } else {
-    launch_pdl(arcq::add_layernorm_kernel, grid_for(M, 8, 8), 256, 0, st, xh, yh, gamma, beta, eps, M, static_cast<int>(K), ld, so, ho);
+    launch_pdl(arcq::add_layernorm_kernel, grid_for(M, 8, 8), 256, 0, st, xh, yh, np, eps, M, static_cast<int>(K), ld, so, ho);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "add_layernorm launch");
   return ARCQ_OK;
 }
 
-static int layernorm_quant_impl(const void* x, const void* y, const float* gamma, const float* beta, float eps, int64_t M, int64_t K,
-                                const float* thresholds, const float* codebook, int bits, int group_size, void* sum_out, void* h_out,
-                                void* xhat, int one_fma, const arcq_unpack_job* unpack, int n_unpack, void* stream);
-
 int arcq_add_layernorm_act_quant(const void* x, const void* y, const float* gamma, const float* beta, float eps,
                                  int64_t M, int64_t K, const float* thresholds, const float* codebook, int bits,
                                  int group_size, void* sum_out, void* h_out, void* xhat, void* stream) {
-  return layernorm_quant_impl(x, y, gamma, beta, eps, M, K, thresholds, codebook, bits, group_size, sum_out, h_out, xhat, 0, nullptr,
-                              0, stream);
+  return arcq_add_layernorm_act_quant_unpack(x, y, gamma, beta, ARCQ_DT_F32, eps, M, K, thresholds, codebook, bits, group_size,
+                                             sum_out, h_out, xhat, 0, nullptr, 0, stream);
 }
 
-int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const float* gamma, const float* beta, float eps,
-                                        int64_t M, int64_t K, const float* thresholds, const float* codebook, int bits,
-                                        int group_size, void* sum_out, void* h_out, void* xhat,
+int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const void* gamma, const void* beta, int param_dtype,
+                                        float eps, int64_t M, int64_t K, const float* thresholds, const float* codebook,
+                                        int bits, int group_size, void* sum_out, void* h_out, void* xhat, int one_fma,
                                         const arcq_unpack_job* unpack, int n_unpack, void* stream) {
-  return layernorm_quant_impl(x, y, gamma, beta, eps, M, K, thresholds, codebook, bits, group_size, sum_out, h_out, xhat,
-                              fp32_rebuild(K, bits), unpack, n_unpack, stream);
-}
-
-static int layernorm_quant_impl(const void* x, const void* y, const float* gamma, const float* beta, float eps, int64_t M, int64_t K,
-                                const float* thresholds, const float* codebook, int bits, int group_size, void* sum_out, void* h_out,
-                                void* xhat, int one_fma, const arcq_unpack_job* unpack, int n_unpack, void* stream) {
   if (x == nullptr || gamma == nullptr || beta == nullptr || thresholds == nullptr || codebook == nullptr || xhat == nullptr)
     return fail(ARCQ_E_BAD_ARG, "null pointer argument");
   if (bits < 2 || bits > 4) return fail(ARCQ_E_BAD_ARG, "bits must be 2, 3 or 4, got %d", bits);
   if (group_size != 64) return fail(ARCQ_E_UNSUPPORTED, "group_size %d: only 64 is built", group_size);
+  if (param_dtype < ARCQ_DT_F32 || param_dtype > ARCQ_DT_BF16) return fail(ARCQ_E_BAD_ARG, "bad param_dtype %d", param_dtype);
   if (M < 0 || K <= 0) return fail(ARCQ_E_BAD_SHAPE, "bad shape M=%lld K=%lld", (long long)M, (long long)K);
   if (K % 64 != 0) return fail(ARCQ_E_BAD_SHAPE, "K=%lld is not a multiple of the group size 64", (long long)K);
   if (K != 192 && K != 384 && K != 768)
     return fail(ARCQ_E_UNSUPPORTED, "K=%lld: the merged kernel is built for rows of 192, 384 and 768 values", (long long)K);
   if (y == nullptr && sum_out != nullptr) return fail(ARCQ_E_BAD_ARG, "sum_out without y");
   if (!aligned(x, 16) || !aligned(xhat, 16) || (y != nullptr && !aligned(y, 16)) ||
-      (sum_out != nullptr && !aligned(sum_out, 16)) || (h_out != nullptr && !aligned(h_out, 16)))
-    return fail(ARCQ_E_ALIGN, "all matrices must be 16-byte aligned");
+      (sum_out != nullptr && !aligned(sum_out, 16)) || (h_out != nullptr && !aligned(h_out, 16)) || !aligned(gamma, 16) || !aligned(beta, 16))
+    return fail(ARCQ_E_ALIGN, "all matrices and the parameters must be 16-byte aligned");
   if (M == 0) return ARCQ_OK;
   arcq::UnpackJobs jobs;
   if (const int rc = make_unpack_jobs(unpack, n_unpack, &jobs)) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const arcq::NormParams np = {gamma, beta, param_dtype};
   const int G = static_cast<int>(K / 64);
   {
     const bool small = small_layernorm_quant(M, K);
@@ -1354,7 +1347,7 @@ static int layernorm_quant_impl(const void* x, const void* y, const float* gamma
       const long long cap2 = static_cast<long long>(sm_count()) * 8;
       const unsigned grid2 = static_cast<unsigned>((tiles2 < cap2 ? tiles2 : cap2) + jobs.blocks);
 #define ARCQ_LAUNCH_LNQ_ROWS(LN, B, HASY)                                                                            \
-  launch_pdl(arcq::add_layernorm_act_quant_rows_kernel<LN, B, HASY>, grid2, arcq::kLnqRowsThreads, 0, st, xs, ys, gamma, beta, eps,     \
+  launch_pdl(arcq::add_layernorm_act_quant_rows_kernel<LN, B, HASY>, grid2, arcq::kLnqRowsThreads, 0, st, xs, ys, np, eps,     \
              static_cast<long long>(M), thresholds, codebook, so2, ho2, xo2, one_fma, jobs)
 #define ARCQ_LNQ_ROWS_BITS(LN, HASY)                                                                                  \
   do {                                                                                                                \
@@ -1386,8 +1379,8 @@ static int layernorm_quant_impl(const void* x, const void* y, const float* gamma
                           CU_TENSOR_MAP_SWIZZLE_128B))
     return fail(ARCQ_E_CUDA, "cuTensorMapEncodeTiled failed for the reconstruction");
 #define ARCQ_LAUNCH_LNQ(LN, B, HASY)                                                                                   \
-  launch_pdl(arcq::add_layernorm_act_quant_kernel<LN, B, HASY>, grid, arcq::kLnqThreads, smem, st, tm_out, xh, yh, gamma, \
-             beta, eps, static_cast<long long>(M), thresholds, codebook, so, ho, one_fma, jobs)
+  launch_pdl(arcq::add_layernorm_act_quant_kernel<LN, B, HASY>, grid, arcq::kLnqThreads, smem, st, tm_out, xh, yh, np, \
+             eps, static_cast<long long>(M), thresholds, codebook, so, ho, one_fma, jobs)
 #define ARCQ_LNQ_BITS(LN, HASY)                                                                                         \
   do {                                                                                                                  \
     if (bits == 4) ARCQ_LAUNCH_LNQ(LN, 4, HASY);                                                                         \

@@ -68,7 +68,8 @@ struct Linear {
   const float *th, *acb, *bias;
   arcq_unpack_job job;
   int64_t weight_elems() const { return N * K; }
-  bool rows_of_16_bytes() const { return K * bits / 8 % 16 == 0; }
+  // 3-bit rows of an odd number of groups: the operands are those of arcq_packed_gemm, activations rebuilt with one fma
+  bool one_fma() const { return K * bits / 8 % 16 != 0; }
 };
 
 bool read_linear(PyObject* buffers, Key bias_key, const c10::Device& dev, Linear* l) {
@@ -110,7 +111,7 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Linear l;
   if (!read_linear(args[0], PyObject_IsTrue(args[2]) ? kBias : kBiasTensor, x->device(), &l)) Py_RETURN_NONE;
   const int64_t numel = x->numel();
-  if (x->size(-1) != l.K || numel == 0 || !aligned16(x->const_data_ptr()) || (ready && !l.rows_of_16_bytes())) Py_RETURN_NONE;
+  if (x->size(-1) != l.K || numel == 0 || !aligned16(x->const_data_ptr()) || (ready && l.one_fma())) Py_RETURN_NONE;
   const int64_t M = numel / l.K;
   const c10::cuda::CUDAGuard guard(x->device());
   void* const st = c10::cuda::getCurrentCUDAStream().stream();
@@ -124,7 +125,8 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
           "arcq_unpack_weight_f16");
   } else {
     void* const xh = w16 + l.weight_elems();
-    check(arcq_act_quant_unpack(pre_gelu, xhat, xt, M, l.K, l.th, l.acb, l.bits, 64, xh, ARCQ_DT_F16, &l.job, 1, st), "arcq_act_quant");
+    check(arcq_act_quant_unpack(pre_gelu, xhat, xt, M, l.K, l.th, l.acb, l.bits, 64, xh, ARCQ_DT_F16, l.one_fma(), &l.job, 1, st),
+          "arcq_act_quant");
     xhat = xh;
   }
   c10::SmallVector<int64_t, 5> sizes(x->sizes().begin(), x->sizes().end());
@@ -202,9 +204,6 @@ PyObject* dequant(PyObject*, PyObject* const* args, Py_ssize_t n) {
 struct Norm {
   PyObject* params;             // _parameters of the LayerNorm
   double eps;
-  at::Tensor gamma, beta;       // fp32 copies when the parameters are not fp32, remade when those change
-  const void* seen[2] = {nullptr, nullptr};
-  uint32_t version[2] = {0, 0};
 };
 struct VitBlock {
   Norm norm1, norm2;
@@ -223,25 +222,23 @@ struct VitPlan {
   }
 };
 
-uint32_t version_of(const at::Tensor& t) { return t.is_inference() ? 0u : static_cast<uint32_t>(t._version()); }
-
-bool read_norm(Norm* n, const c10::Device& dev, int64_t dim, const float** gamma, const float** beta) {
-  const at::Tensor* t[2] = {tensor_of(PyDict_GetItem(n->params, g_key[kWeight])), tensor_of(PyDict_GetItem(n->params, g_key[kBias]))};
+// The kernels' view of one LayerNorm, parameters as the module holds them.
+struct NormView {
+  const void *gamma, *beta;
+  int dtype;
+};
+bool read_norm(const Norm& n, const c10::Device& dev, int64_t dim, NormView* v) {
+  const void* p[2];
   for (int i = 0; i < 2; ++i) {
-    if (t[i] == nullptr || t[i]->device() != dev || t[i]->numel() != dim || dtype_code(t[i]->scalar_type()) < 0) return false;
-    at::Tensor& copy = i ? n->beta : n->gamma;
-    if (t[i]->scalar_type() == at::kFloat && t[i]->is_contiguous() && aligned16(t[i]->const_data_ptr())) {
-      *(i ? beta : gamma) = t[i]->const_data_ptr<float>();
-      continue;
-    }
-    const void* p = t[i]->const_data_ptr();
-    if (!copy.defined() || n->seen[i] != p || n->version[i] != version_of(*t[i]) || t[i]->is_inference() || copy.device() != dev) {
-      copy = t[i]->detach().to(at::kFloat).contiguous();
-      n->seen[i] = p;
-      n->version[i] = version_of(*t[i]);
-    }
-    *(i ? beta : gamma) = copy.const_data_ptr<float>();
+    const at::Tensor* t = tensor_of(PyDict_GetItem(n.params, g_key[i ? kBias : kWeight]));
+    if (t == nullptr || t->device() != dev || t->numel() != dim || !t->is_contiguous() || !aligned16(t->const_data_ptr())) return false;
+    const int d = dtype_code(t->scalar_type());
+    if (d < 0 || (i == 1 && d != v->dtype)) return false;
+    v->dtype = d;
+    p[i] = t->const_data_ptr();
   }
+  v->gamma = p[0];
+  v->beta = p[1];
   return true;
 }
 
@@ -325,7 +322,7 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     Py_RETURN_NONE;
   const size_t depth = p->blocks.size();
   std::vector<Linear> lin(4 * depth);
-  std::vector<const float*> gb(4 * depth + 2);
+  std::vector<NormView> norms(2 * depth + 1);
   int64_t scratch_elems[2] = {0, 0};                       // qkv + proj, fc1 + fc2
   for (size_t i = 0; i < depth; ++i) {
     VitBlock& b = p->blocks[i];
@@ -339,10 +336,9 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
     scratch_elems[0] = std::max(scratch_elems[0], lin[4 * i].weight_elems() + lin[4 * i + 1].weight_elems());
     scratch_elems[1] = std::max(scratch_elems[1], lin[4 * i + 2].weight_elems() + lin[4 * i + 3].weight_elems());
-    if (!read_norm(&b.norm1, dev, D, &gb[4 * i], &gb[4 * i + 1]) || !read_norm(&b.norm2, dev, D, &gb[4 * i + 2], &gb[4 * i + 3]))
-      Py_RETURN_NONE;
+    if (!read_norm(b.norm1, dev, D, &norms[2 * i]) || !read_norm(b.norm2, dev, D, &norms[2 * i + 1])) Py_RETURN_NONE;
   }
-  if (!read_norm(&p->norm, dev, D, &gb[4 * depth], &gb[4 * depth + 1])) Py_RETURN_NONE;
+  if (!read_norm(p->norm, dev, D, &norms[2 * depth])) Py_RETURN_NONE;
   int64_t hidden = 0;
   for (size_t i = 0; i < depth; ++i) hidden = std::max(hidden, lin[4 * i + 2].N);
 
@@ -394,13 +390,14 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     while (from < 2 && half[from].weight_elems() <= room) room -= half[from++].weight_elems();
     return from;
   };
-  auto norm_quant = [&](const at::Half* y, const float* gamma, const float* beta, double eps, const Linear* half, int gelu_quant) {
+  auto norm_quant = [&](const at::Half* y, const NormView& nv, double eps, const Linear* half, int gelu_quant) {
     // the first weight has to be there before the half block's first GEMM, the second may be that GEMM's job
     const int first = std::max(done, 1), to = fits(half, first, half[0], gelu_quant) == 2 ? first : 2;
     arcq_unpack_job jobs[2];
     const int n = jobs_of(half, done, to, jobs);
-    check(arcq_add_layernorm_act_quant_unpack(x, y, gamma, beta, static_cast<float>(eps), M, D, half[0].th, half[0].acb, half[0].bits, 64,
-                                              y != nullptr ? x_next : nullptr, nullptr, xhat, jobs, n, st),
+    check(arcq_add_layernorm_act_quant_unpack(x, y, nv.gamma, nv.beta, nv.dtype, static_cast<float>(eps), M, D, half[0].th, half[0].acb,
+                                              half[0].bits, 64, y != nullptr ? x_next : nullptr, nullptr, xhat, half[0].one_fma(), jobs,
+                                              n, st),
           "arcq_add_layernorm_act_quant");
     if (y != nullptr) std::swap(x, x_next);
     done = to;
@@ -436,20 +433,20 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
       asked[0] = fc1->N;
       asked[1] = fc1->K;
     }
-    const bool fused = applies && fc2->rows_of_16_bytes();     // the fused form reconstructs in three steps only
+    const bool fused = applies && !fc2->one_fma();     // the fused form reconstructs in three steps only
     arcq_unpack_job jobs[2];
-    norm_quant(y, gb[4 * i], gb[4 * i + 1], b.norm1.eps, qkv, 0);
+    norm_quant(y, norms[2 * i], b.norm1.eps, qkv, 0);
     gemm(xhat, *qkv, mid, jobs, jobs_of(qkv, done, 2, jobs));
     {
       const at::Tensor t = at::from_blob(mid, {B, T, 3, p->heads, D / p->heads}, at::TensorOptions().dtype(at::kHalf).device(dev));
       const at::Tensor r = t.permute({2, 0, 3, 1, 4});
       const at::Tensor o = at::scaled_dot_product_attention(r[0], r[1], r[2]).transpose(1, 2).reshape({M, D});
       check(arcq_act_quant_unpack(0, o.const_data_ptr(), ARCQ_DT_F16, M, D, proj->th, proj->acb, proj->bits, 64, xhat, ARCQ_DT_F16,
-                                  nullptr, 0, st),
+                                  proj->one_fma(), nullptr, 0, st),
             "arcq_act_quant");
     }
     last_gemm(xhat, *proj, branch, fc1, fused);
-    norm_quant(branch, gb[4 * i + 2], gb[4 * i + 3], b.norm2.eps, fc1, fused);
+    norm_quant(branch, norms[2 * i + 1], b.norm2.eps, fc1, fused);
     const int n = jobs_of(fc1, done, 2, jobs);
     if (fused) {
       check(arcq_dense_weight_gemm_gelu_quant(xhat, fc1->job.out, fc1->bias, M, fc1->N, fc1->K, fc2->th, fc2->acb, fc2->bits, 64, xhat4,
@@ -457,7 +454,8 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
             "arcq_dense_weight_gemm_gelu_quant");
     } else {
       gemm(xhat, *fc1, mid, jobs, n);
-      check(arcq_act_quant_unpack(1, mid, ARCQ_DT_F16, M, fc2->K, fc2->th, fc2->acb, fc2->bits, 64, xhat4, ARCQ_DT_F16, nullptr, 0, st),
+      check(arcq_act_quant_unpack(1, mid, ARCQ_DT_F16, M, fc2->K, fc2->th, fc2->acb, fc2->bits, 64, xhat4, ARCQ_DT_F16, fc2->one_fma(),
+                                  nullptr, 0, st),
             "arcq_gelu_act_quant");
     }
     last_gemm(xhat4, *fc2, branch, i + 1 < depth ? qkv + 4 : nullptr, 0);
@@ -465,7 +463,8 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
   // the head reads the class token of every image only
   const at::Tensor h = empty_cuda({B, D}, at::kHalf, dev);
-  check(arcq_add_layernorm_strided(x, y, gb[4 * depth], gb[4 * depth + 1], static_cast<float>(p->norm.eps), B, D, T * D, nullptr,
+  const NormView& nv = norms[2 * depth];
+  check(arcq_add_layernorm_strided(x, y, nv.gamma, nv.beta, nv.dtype, static_cast<float>(p->norm.eps), B, D, T * D, nullptr,
                                    h.mutable_data_ptr(), st),
         "arcq_add_layernorm");
   return THPVariable_Wrap(at::linear(h, *hw, *hb));

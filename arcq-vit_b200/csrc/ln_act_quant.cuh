@@ -36,8 +36,7 @@ __host__ __device__ constexpr size_t lnq_smem_bytes() {
 template <int LANES, int BITS, bool HAS_Y>
 __global__ void __launch_bounds__(kLnqThreads, 4)
     add_layernorm_act_quant_kernel(const __grid_constant__ CUtensorMap tm_out, const __half* __restrict__ x,
-                                   const __half* __restrict__ y, const float* __restrict__ gamma,
-                                   const float* __restrict__ beta, float eps, long long M,
+                                   const __half* __restrict__ y, const NormParams np, float eps, long long M,
                                    const float* __restrict__ thresholds, const float* __restrict__ codebook,
                                    __half* __restrict__ sum_out, __half* __restrict__ h_out, int one_fma,
                                    const __grid_constant__ UnpackJobs jobs) {
@@ -71,7 +70,7 @@ __global__ void __launch_bounds__(kLnqThreads, 4)
     // ---- phase 1: LayerNorm of every row the tile touches, LANES lanes per row
     {
       float gg[3][8], bb[3][8];
-      layernorm_lane_params<LANES>(gamma, beta, l, gg, bb);
+      layernorm_lane_params<LANES>(np, l, gg, bb);
       // (issuing the loads of all passes before the first pass computes was tried: 72 more live registers, spills,
       // 13.5 us instead of 11.3 us; one pass ahead, with gamma and beta re-read per pass to make room: 11.4 us, no gain)
 #pragma unroll 1
@@ -128,8 +127,7 @@ constexpr int kLnqRowsThreads = 384;
 template <int LANES, int BITS, bool HAS_Y>
 __global__ void __launch_bounds__(kLnqRowsThreads) add_layernorm_act_quant_rows_kernel(const __half* __restrict__ x,
                                                                           const __half* __restrict__ y,
-                                                                          const float* __restrict__ gamma,
-                                                                          const float* __restrict__ beta, float eps,
+                                                                          const NormParams np, float eps,
                                                                           long long M,
                                                                           const float* __restrict__ thresholds,
                                                                           const float* __restrict__ codebook,
@@ -155,7 +153,7 @@ __global__ void __launch_bounds__(kLnqRowsThreads) add_layernorm_act_quant_rows_
     s_cb[tid] = (tid < L) ? codebook[tid] : 0.0f;
   }
   float gg[3][8] = {}, bb[3][8] = {};
-  if (warp < 4) layernorm_lane_params<LANES>(gamma, beta, l, gg, bb);
+  if (warp < 4) layernorm_lane_params<LANES>(np, l, gg, bb);
   __syncthreads();
   pdl_wait();                // everything above is the layer's constants; x and y may be the previous kernel's output
 

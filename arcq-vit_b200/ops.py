@@ -202,26 +202,24 @@ def add_layernorm(x: torch.Tensor, y, norm: torch.nn.LayerNorm):
     K = shape[-1]
     x2 = _dev(x.reshape(-1, K), "x", torch.float16)
     y2 = None if y is None else _dev(y.reshape(-1, K), "y", torch.float16)
-    g32, b32 = _norm_params_f32(norm, x2.device)
+    gamma, beta = _norm_params(norm, x2.device)
     h = torch.empty_like(x2)
     s_out = torch.empty_like(x2) if y2 is not None else None
     if x2.shape[0] > 0:
-        rc = lib.arcq_add_layernorm(x2.data_ptr(), y2.data_ptr() if y2 is not None else None, g32.data_ptr(),
-                                    b32.data_ptr(), float(norm.eps), x2.shape[0], K,
-                                    s_out.data_ptr() if s_out is not None else None, h.data_ptr(), _stream())
+        rc = lib.arcq_add_layernorm_strided(x2.data_ptr(), y2.data_ptr() if y2 is not None else None, gamma.data_ptr(),
+                                            beta.data_ptr(), _DT[gamma.dtype], float(norm.eps), x2.shape[0], K, K,
+                                            s_out.data_ptr() if s_out is not None else None, h.data_ptr(), _stream())
         _check(rc, "arcq_add_layernorm")
     return (x if s_out is None else s_out.reshape(shape)), h.reshape(shape)
 
 
-def _norm_params_f32(norm: torch.nn.LayerNorm, device):
-    """fp32 copies of the affine parameters, remade whenever the parameters were replaced, written to or moved."""
-    key = (norm.weight.data_ptr(), norm.weight._version, norm.bias.data_ptr(), norm.bias._version, device)
-    cached = getattr(norm, "_arcq_f32", None)
-    if cached is None or cached[0] != key:
-        cached = (key, norm.weight.detach().to(device=device, dtype=torch.float32).contiguous(),
-                  norm.bias.detach().to(device=device, dtype=torch.float32).contiguous())
-        norm._arcq_f32 = cached
-    return cached[1], cached[2]
+def _norm_params(norm: torch.nn.LayerNorm, device):
+    """gamma and beta as the kernels read them: the parameters themselves, or fp32 copies for this call where the two differ in
+    type, are elsewhere, or are not laid out for 16-byte reads."""
+    w, b = norm.weight.detach(), norm.bias.detach()
+    if w.dtype == b.dtype and w.dtype in _DT and all(t.device == device and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (w, b)):
+        return w, b
+    return tuple(t.to(device=device, dtype=torch.float32).contiguous() for t in (w, b))
 
 
 def add_layernorm_quant(x: torch.Tensor, y, norm: torch.nn.LayerNorm, thresholds: torch.Tensor, codebook: torch.Tensor,
@@ -241,16 +239,16 @@ def add_layernorm_quant(x: torch.Tensor, y, norm: torch.nn.LayerNorm, thresholds
         s, h = add_layernorm(x, y, norm)
         xh = quantize_activation_dequant(h.reshape(-1, K), thresholds, codebook, bits, group_size, torch.float16)
         return (s, xh.reshape(shape), h) if want_h else (s, xh.reshape(shape))
-    g32, b32 = _norm_params_f32(norm, x2.device)
+    gamma, beta = _norm_params(norm, x2.device)
     xhat = torch.empty_like(x2)
     s_out = torch.empty_like(x2) if y2 is not None else None
     h = torch.empty_like(x2) if want_h else None
     if x2.shape[0] > 0:
-        rc = lib.arcq_add_layernorm_act_quant(x2.data_ptr(), y2.data_ptr() if y2 is not None else None, g32.data_ptr(),
-                                              b32.data_ptr(), float(norm.eps), x2.shape[0], K, thresholds.data_ptr(),
-                                              codebook.data_ptr(), bits, group_size,
-                                              s_out.data_ptr() if s_out is not None else None,
-                                              h.data_ptr() if h is not None else None, xhat.data_ptr(), _stream())
+        rc = lib.arcq_add_layernorm_act_quant_unpack(
+            x2.data_ptr(), y2.data_ptr() if y2 is not None else None, gamma.data_ptr(), beta.data_ptr(), _DT[gamma.dtype],
+            float(norm.eps), x2.shape[0], K, thresholds.data_ptr(), codebook.data_ptr(), bits, group_size,
+            s_out.data_ptr() if s_out is not None else None, h.data_ptr() if h is not None else None, xhat.data_ptr(),
+            0, None, 0, _stream())
         _check(rc, "arcq_add_layernorm_act_quant")
     out = ((x if s_out is None else s_out.reshape(shape)), xhat.reshape(shape))
     return out + (h.reshape(shape),) if want_h else out

@@ -159,11 +159,11 @@ typedef struct arcq_unpack_job {
 /*
  * arcq_act_quant (pre_gelu = 0) or arcq_gelu_act_quant (1) with reconstruction output only, plus unpack jobs: steps 2
  * and 3 of ARCQPackedLinearOnTheFly.forward (FQ/fair_qat/arcq_packed_on_the_fly.py:143-158: dequant_activation_triton,
- * unpack_weight_triton) in one launch.  K and bits are the layer's: where its packed rows are no multiple of 16 bytes, xhat is
- * the operand that arcq_packed_gemm rebuilds (one fma per value) instead of the three rounded steps.
+ * unpack_weight_triton) in one launch.  one_fma = 1: xhat is the operand that arcq_packed_gemm rebuilds from the codes,
+ * fma(scale, level, center - scale * code_sum / 64), instead of the three rounded steps.
  */
 int arcq_act_quant_unpack(int pre_gelu, const void* x, int x_dtype, int64_t M, int64_t K, const float* thresholds,
-                          const float* codebook, int bits, int group_size, void* xhat_out, int xhat_dtype,
+                          const float* codebook, int bits, int group_size, void* xhat_out, int xhat_dtype, int one_fma,
                           const arcq_unpack_job* unpack, int n_unpack, void* stream);
 
 /*
@@ -244,10 +244,11 @@ int arcq_packed_linear_static_scratch(const void* xhat, const uint8_t* packed_w,
 int arcq_add_layernorm(const void* x, const void* y, const float* gamma, const float* beta, float eps,
                        int64_t M, int64_t K, void* sum_out, void* h_out, void* stream);
 
-/* The same with input rows `ld` values apart (ld >= K, a multiple of 8); sum_out and h_out stay contiguous.  The final
- * norm of a ViT runs on the class token of every image: ld = tokens * K. */
-int arcq_add_layernorm_strided(const void* x, const void* y, const float* gamma, const float* beta, float eps, int64_t M,
-                               int64_t K, int64_t ld, void* sum_out, void* h_out, void* stream);
+/* The same with input rows `ld` values apart (ld >= K, a multiple of 8; sum_out and h_out stay contiguous) and gamma and beta of
+ * any element type (ARCQ_DT_*), read as they are: a half-precision model's parameters need no fp32 copy.  The final norm of a ViT
+ * runs on the class token of every image: ld = tokens * K. */
+int arcq_add_layernorm_strided(const void* x, const void* y, const void* gamma, const void* beta, int param_dtype, float eps,
+                               int64_t M, int64_t K, int64_t ld, void* sum_out, void* h_out, void* stream);
 
 /*
  * arcq_add_layernorm followed by the activation quantizer of the packed linear that consumes the LayerNorm
@@ -262,10 +263,11 @@ int arcq_add_layernorm_act_quant(const void* x, const void* y, const float* gamm
                                  int64_t M, int64_t K, const float* thresholds, const float* codebook, int bits,
                                  int group_size, void* sum_out, void* h_out, void* xhat, void* stream);
 
-/* The same with unpack jobs (see arcq_unpack_job) taken along by the launch; xhat as in arcq_act_quant_unpack. */
-int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const float* gamma, const float* beta, float eps,
-                                        int64_t M, int64_t K, const float* thresholds, const float* codebook, int bits,
-                                        int group_size, void* sum_out, void* h_out, void* xhat,
+/* The same with parameters of any element type, unpack jobs (see arcq_unpack_job) taken along by the launch, and one_fma as in
+ * arcq_act_quant_unpack. */
+int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const void* gamma, const void* beta, int param_dtype,
+                                        float eps, int64_t M, int64_t K, const float* thresholds, const float* codebook,
+                                        int bits, int group_size, void* sum_out, void* h_out, void* xhat, int one_fma,
                                         const arcq_unpack_job* unpack, int n_unpack, void* stream);
 
 /*

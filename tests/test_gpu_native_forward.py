@@ -83,3 +83,73 @@ def test_three_bit_rows_of_any_length_equal_the_packed_operators(pkg, cuda_devic
         wide = torch.empty(M, K + 8, dtype=dtype, device=cuda_device)[:, :K].copy_(x)      # not contiguous: the Python route
         assert torch.equal(layer(wide), want)
     assert pkg.ops.device_status() == 0
+
+
+def _small_model(pkg, name, bits, dev, blocks=2):
+    model = pkg.create_vit(name, seed=1)
+    model.blocks = torch.nn.ModuleList(list(model.blocks)[:blocks])
+    model = model.half().to(dev)
+    images = torch.randn(8, 3, 224, 224, generator=torch.Generator().manual_seed(5)).half().to(dev)
+    with torch.no_grad():
+        for n, p in model.named_parameters():                  # LayerNorms that do something
+            if "norm" in n:
+                p.add_(torch.randn(p.shape, generator=torch.Generator().manual_seed(len(n))).to(p) * 0.2)
+        return pkg.quantise_model(model, images[:4], bits), images
+
+
+@torch.no_grad()
+def test_a_captured_forward_outlives_what_later_calls_do(pkg, cuda_device):
+    """A graph of the native forward, then calls that the native forward does not take, allocations and changed parameters of
+    another model: the replay still gives the bits of the capture."""
+    model, images = _small_model(pkg, "deit_small", 4, cuda_device)
+    want = model(images).clone()
+    runner = pkg.GraphedModel(model, images)
+    model(images.contiguous(memory_format=torch.channels_last))
+    model(images[::2])
+    model(images.float()[:, :, ::1].half())
+    filler = [torch.full((n,), float("nan"), device=cuda_device) for n in (96, 192, 384, 768) for _ in range(64)]
+    assert torch.equal(runner(images), want)
+    del filler
+
+
+@torch.no_grad()
+def test_layernorm_parameters_are_read_on_every_call(pkg, cuda_device):
+    """Written through .data (no version count), replaced, or in another type: the next forward sees them, on the native and on the
+    Python route."""
+    model, images = _small_model(pkg, "deit_small", 4, cuda_device)
+    strided = images[::2].contiguous(memory_format=torch.channels_last)
+    seen = []
+    for change in (lambda n: None, lambda n: n.weight.data.mul_(1.5), lambda n: n.bias.data.add_(0.25),
+                   lambda n: setattr(n, "weight", torch.nn.Parameter(n.weight * 0.5))):
+        for norm in (model.blocks[1].norm1, model.norm):
+            change(norm)
+        seen.append(model(images[::2].contiguous()))
+        assert torch.equal(seen[-1], model(strided))
+    for i in range(1, len(seen)):
+        assert not torch.equal(seen[i], seen[i - 1])
+    for norm in (model.blocks[1].norm1, model.norm):
+        norm.float()                                           # the same values
+    assert torch.equal(model(images[::2].contiguous()), seen[-1])
+    assert pkg.ops.device_status() == 0
+
+
+# rows of the lane-layout kernels and of the general one; one row, a ragged tile and many tiles
+@pytest.mark.parametrize("K", [192, 384, 768, 1000])
+@pytest.mark.parametrize("M", [1, 2500])
+@torch.no_grad()
+def test_layernorm_kernels_read_parameters_of_any_type(pkg, cuda_device, K, M):
+    gen = torch.Generator().manual_seed(K + M)
+    x, y = (torch.randn(M, K, generator=gen).half().to(cuda_device) for _ in range(2))
+    cb, th = _codebook(gen, 4, cuda_device)
+    for dtype in (torch.float16, torch.bfloat16):
+        norm = torch.nn.LayerNorm(K, eps=1e-6)
+        norm.weight.copy_(torch.randn(K, generator=gen)), norm.bias.copy_(torch.randn(K, generator=gen))
+        norm = norm.to(dtype).to(cuda_device)
+        wide = torch.nn.LayerNorm(K, eps=1e-6).to(cuda_device)
+        wide.weight.copy_(norm.weight), wide.bias.copy_(norm.bias)
+        for a, b in zip(pkg.ops.add_layernorm(x, y, norm), pkg.ops.add_layernorm(x, y, wide)):
+            assert torch.equal(a, b)
+        if K != 1000:
+            for a, b in zip(pkg.ops.add_layernorm_quant(x, y, norm, th, cb, 4), pkg.ops.add_layernorm_quant(x, y, wide, th, cb, 4)):
+                assert torch.equal(a, b)
+    assert pkg.ops.device_status() == 0
