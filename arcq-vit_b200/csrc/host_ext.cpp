@@ -10,6 +10,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -201,6 +202,13 @@ PyObject* dequant(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 // ---------------------------------------------------------------- the forward of a packed ViT
 // What a plan holds are references to the dictionaries of the model's modules; nothing of their content.
+// The data of a framework operator's fp16 result, which the kernels read as a dense matrix.
+const void* half_matrix(const at::Tensor& t, int64_t elems, const c10::Device& dev) {
+  TORCH_CHECK(t.scalar_type() == at::kHalf && t.device() == dev && t.is_contiguous() && t.numel() == elems,
+              "a framework operator of the ViT forward returned ", t.scalar_type(), " ", t.sizes(), " on ", t.device());
+  return t.const_data_ptr();
+}
+
 struct Norm {
   PyObject* params;             // _parameters of the LayerNorm
   double eps;
@@ -296,6 +304,8 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (img == nullptr || !img->is_cuda() || img->scalar_type() != at::kHalf || img->dim() != 4 || !img->is_contiguous() ||
       img->numel() == 0 || !aligned16(img->const_data_ptr()))
     Py_RETURN_NONE;
+  // autocast to another type changes what the framework's linear and attention below take and give
+  if (at::autocast::is_autocast_enabled(at::kCUDA) && at::autocast::get_autocast_dtype(at::kCUDA) != at::kHalf) Py_RETURN_NONE;
   for (size_t i = 0; i < p->watch.size(); i += 3) {
     PyObject* const got = PyDict_GetItem(p->watch[i], p->watch[i + 1]);
     if (got != p->watch[i + 2] && !(got == nullptr && p->watch[i + 2] == Py_None)) Py_RETURN_NONE;   // None: no such module
@@ -419,7 +429,7 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const at::Tensor rows = empty_cuda({B * (T - 1), C * P * P}, at::kHalf, dev);
     check(arcq_patchify(img->const_data_ptr(), B, C, H, W, static_cast<int>(P), rows.mutable_data_ptr(), st), "arcq_patchify");
     const at::Tensor patches = at::linear(rows, pw->view({D, C * P * P}), *pb);
-    check(arcq_assemble_tokens(patches.const_data_ptr(), cls->const_data_ptr(), pos->const_data_ptr(), B, T - 1, D, x, st),
+    check(arcq_assemble_tokens(half_matrix(patches, B * (T - 1) * D, dev), cls->const_data_ptr(), pos->const_data_ptr(), B, T - 1, D, x, st),
           "arcq_assemble_tokens");
   }
   const at::Half* y = nullptr;
@@ -440,9 +450,9 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     {
       const at::Tensor t = at::from_blob(mid, {B, T, 3, p->heads, D / p->heads}, at::TensorOptions().dtype(at::kHalf).device(dev));
       const at::Tensor r = t.permute({2, 0, 3, 1, 4});
-      const at::Tensor o = at::scaled_dot_product_attention(r[0], r[1], r[2]).transpose(1, 2).reshape({M, D});
-      check(arcq_act_quant_unpack(0, o.const_data_ptr(), ARCQ_DT_F16, M, D, proj->th, proj->acb, proj->bits, 64, xhat, ARCQ_DT_F16,
-                                  proj->one_fma(), nullptr, 0, st),
+      const at::Tensor o = at::scaled_dot_product_attention(r[0], r[1], r[2]).transpose(1, 2).reshape({M, D}).contiguous();
+      check(arcq_act_quant_unpack(0, half_matrix(o, M * D, dev), ARCQ_DT_F16, M, D, proj->th, proj->acb, proj->bits, 64, xhat,
+                                  ARCQ_DT_F16, proj->one_fma(), nullptr, 0, st),
             "arcq_act_quant");
     }
     last_gemm(xhat, *proj, branch, fc1, fused);

@@ -153,3 +153,17 @@ def test_layernorm_kernels_read_parameters_of_any_type(pkg, cuda_device, K, M):
             for a, b in zip(pkg.ops.add_layernorm_quant(x, y, norm, th, cb, 4), pkg.ops.add_layernorm_quant(x, y, wide, th, cb, 4)):
                 assert torch.equal(a, b)
     assert pkg.ops.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@torch.no_grad()
+def test_autocast_gives_what_the_python_forward_gives(pkg, cuda_device, dtype, monkeypatch):
+    model, images = _small_model(pkg, "deit_small", 4, cuda_device)
+    plain = model(images)
+    with torch.autocast("cuda", dtype):
+        got = model(images)
+        monkeypatch.setattr(pkg.vit.VisionTransformer, "_forward_native", lambda self, x: None)
+        want = model(images)
+    assert got.dtype == want.dtype and torch.equal(got, want)
+    assert dtype != torch.float16 or torch.equal(got, plain)
+    assert pkg.ops.device_status() == 0
