@@ -201,7 +201,6 @@ PyObject* dequant(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // ---------------------------------------------------------------- the forward of a packed ViT
-// What a plan holds are references to the dictionaries of the model's modules; nothing of their content.
 // The data of a framework operator's fp16 result, which the kernels read as a dense matrix.
 const void* half_matrix(const at::Tensor& t, int64_t elems, const c10::Device& dev) {
   TORCH_CHECK(t.scalar_type() == at::kHalf && t.device() == dev && t.is_contiguous() && t.numel() == elems,
@@ -209,6 +208,9 @@ const void* half_matrix(const at::Tensor& t, int64_t elems, const c10::Device& d
   return t.const_data_ptr();
 }
 
+// What a plan holds are references to the dictionaries of the model's modules and, in `watch`, every plain value and module that
+// it was made from; no tensors.  A call compares all of `watch` first, so that a plan is never used for another model than the
+// one it describes.
 struct Norm {
   PyObject* params;             // _parameters of the LayerNorm
   double eps;
@@ -222,7 +224,7 @@ struct VitPlan {
   PyObject *own, *patch_params, *head_params;      // _parameters of the model, of patch_embed.proj and of head
   std::vector<VitBlock> blocks;
   Norm norm;
-  std::vector<PyObject*> watch;       // (dict, key, expected value) triples: the modules the plan was made for
+  std::vector<PyObject*> watch;       // (dict, key, expected value) triples; None: absent or None
   std::vector<PyObject*> empty;       // hook dictionaries that have to be empty
   std::vector<PyObject*> refs;
   ~VitPlan() {
@@ -295,21 +297,21 @@ PyObject* vit_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return PyCapsule_New(p, "arcq_vit_plan", free_plan);
 }
 
-// vit_forward(plan, images) -> logits; None: the model or the input is not one the plan covers
+// vit_forward(plan, images) -> logits; None: not a call the plan covers; False: the model has changed, the plan is void
 PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 2) Py_RETURN_NONE;
   auto* p = static_cast<VitPlan*>(PyCapsule_GetPointer(args[0], "arcq_vit_plan"));
   if (p == nullptr) return nullptr;
+  for (size_t i = 0; i < p->watch.size(); i += 3) {
+    PyObject* const got = PyDict_GetItem(p->watch[i], p->watch[i + 1]);
+    if (got != p->watch[i + 2] && !(got == nullptr && p->watch[i + 2] == Py_None)) Py_RETURN_FALSE;
+  }
   const at::Tensor* img = tensor_of(args[1]);
   if (img == nullptr || !img->is_cuda() || img->scalar_type() != at::kHalf || img->dim() != 4 || !img->is_contiguous() ||
       img->numel() == 0 || !aligned16(img->const_data_ptr()))
     Py_RETURN_NONE;
   // autocast to another type changes what the framework's linear and attention below take and give
   if (at::autocast::is_autocast_enabled(at::kCUDA) && at::autocast::get_autocast_dtype(at::kCUDA) != at::kHalf) Py_RETURN_NONE;
-  for (size_t i = 0; i < p->watch.size(); i += 3) {
-    PyObject* const got = PyDict_GetItem(p->watch[i], p->watch[i + 1]);
-    if (got != p->watch[i + 2] && !(got == nullptr && p->watch[i + 2] == Py_None)) Py_RETURN_NONE;   // None: no such module
-  }
   for (PyObject* d : p->empty)
     if (PyDict_Size(d) != 0) Py_RETURN_NONE;
   const c10::Device dev = img->device();

@@ -145,22 +145,25 @@ class VisionTransformer(nn.Module):
 
     def _forward_native(self, x: torch.Tensor):
         """The whole forward as one native call that launches every kernel (``csrc/host_ext.cpp``), or None where it does
-        not apply: anything but an unmodified packed model (hooks, replaced modules, tuning switches) on fp16 CUDA images
-        without gradients.  Same kernels in the same order as the code below."""
+        not apply: anything but an unmodified packed model (hooks, replaced modules or forwards, tuning switches) on fp16 CUDA
+        images without gradients.  Same kernels in the same order as the code below."""
         if (not x.is_cuda or torch.is_grad_enabled() or len(self.blocks) == 0 or self.fuse_norm_quant != "auto"
                 or type(self) is not VisionTransformer or ARCQPackedLinearOnTheFly.weight_form != "auto"
-                or WeightStager.mode != "stream" or Attention.implementation != "auto" or _has_global_hooks()):
+                or WeightStager.mode != "stream" or Attention.implementation != "auto" or _has_global_hooks()
+                or "_forward_fused_glue" in self.__dict__ or any(getattr(c, n) is not f for c, n, f in _STANDS_FOR)):
             return None
         plan = _PLANS.get(self)
-        y = None if plan is None else _cabi.host().vit_forward(plan, x)
-        if y is None and isinstance(getattr(getattr(self.blocks[0], "attn", None), "qkv", None), ARCQPackedLinearOnTheFly):
-            # no plan yet, or the modules it was made for have changed
-            plan = _make_plan(self)
-            if plan is None:
-                _PLANS.pop(self, None)
+        if plan is None:
+            plan = _PLANS[self] = _make_plan(self)
+        if callable(plan):                             # why there is none
+            if plan():
                 return None
-            _PLANS[self] = plan
+            y = False
+        else:
             y = _cabi.host().vit_forward(plan, x)
+        if y is False:                                 # made for another state of the model
+            plan = _PLANS[self] = _make_plan(self)
+            y = None if callable(plan) else _cabi.host().vit_forward(plan, x)
         return y
 
     def _forward_fused_glue(self, x: torch.Tensor) -> torch.Tensor:
@@ -203,45 +206,63 @@ def _has_global_hooks() -> bool:
     return bool(m._global_forward_hooks or m._global_forward_pre_hooks)
 
 
+# the Python code that a native forward stands for: replaced on its class or module, it is called as before
+_STANDS_FOR = tuple((c, n, getattr(c, n)) for c, n in (
+    (PatchEmbed, "forward"), (Attention, "forward"), (Mlp, "forward"), (ARCQPackedLinearOnTheFly, "forward"), (nn.Linear, "forward"),
+    (VisionTransformer, "_forward_fused_glue"), (F, "linear"), (F, "scaled_dot_product_attention")))
+
+
+class _NotNative(Exception):
+    """Carries a function that says whether the reason still holds."""
+
+
 def _make_plan(model: VisionTransformer):
-    """References to the module dictionaries a native forward reads (parameters, buffers), the modules it was made for
-    (checked on every call) and the hook dictionaries that have to be empty; None for a model it cannot run."""
+    """What a native forward of the model reads: references to the module dictionaries (parameters, buffers), every value and
+    module it was made from (compared on every call), and the hook dictionaries that have to be empty.  For a model that it cannot
+    run, a function that is true as long as that is so."""
     watch, empty, blocks = [], [], []
 
-    def child(parent: nn.Module, name: str, kind: type):
-        m = parent._modules.get(name)
-        if type(m) is not kind:
-            raise LookupError(name)
-        watch.extend((parent._modules, name, m))
+    def expect(owner: dict, name: str, ok: Callable):
+        value = owner.get(name)
+        if not ok(value):
+            raise _NotNative(lambda: not ok(owner.get(name)))
+        watch.extend((owner, name, value))
+        return value
+
+    def child(parent: nn.Module, name: str, kind: type, *switches: str):
+        m = expect(parent._modules, name, lambda v: type(v) is kind)
+        for attr in ("forward", "_compiled_call_impl", *switches):     # nothing set on the instance
+            expect(m.__dict__, attr, lambda v: v is None)
         empty.extend((m._forward_hooks, m._forward_pre_hooks))
         return m
 
     def linear(parent: nn.Module, name: str):
-        m = child(parent, name, ARCQPackedLinearOnTheFly)
-        if m.group_size != 64 or m.__dict__.get("weight_form", "auto") != "auto" or not m.supports_pre_gelu:
-            raise LookupError(name)
+        m = child(parent, name, ARCQPackedLinearOnTheFly, "weight_form", "supports_pre_gelu")
+        expect(m.__dict__, "group_size", lambda v: v == 64)
         return m._buffers
+
+    def norm(parent: nn.Module, name: str):
+        m = child(parent, name, nn.LayerNorm)
+        return m._parameters, float(expect(m.__dict__, "eps", lambda v: isinstance(v, (int, float))))
 
     try:
         patch = child(child(model, "patch_embed", PatchEmbed), "proj", nn.Conv2d)
-        dim, heads = model.embed_dim, model.num_heads
-        if dim not in (192, 384, 768) or dim != 64 * heads or patch.kernel_size[0] != patch.kernel_size[1] or patch.kernel_size[0] % 8:
-            return None
+        size = expect(patch.__dict__, "kernel_size", lambda v: isinstance(v, tuple) and len(v) == 2 and v[0] == v[1] and v[0] % 8 == 0)
+        dim = expect(model.__dict__, "embed_dim", lambda v: v in (192, 384, 768))
+        heads = dim // 64
         stack = child(model, "blocks", nn.ModuleList)
         for i in range(len(stack)):
             blk = child(stack, str(i), Block)
-            attn, mlp = child(blk, "attn", Attention), child(blk, "mlp", Mlp)
-            n1, n2 = child(blk, "norm1", nn.LayerNorm), child(blk, "norm2", nn.LayerNorm)
-            if attn.num_heads != heads or "implementation" in attn.__dict__:
-                return None
-            blocks.append((n1._parameters, float(n1.eps), n2._parameters, float(n2.eps), linear(attn, "qkv"), linear(attn, "proj"),
+            attn, mlp = child(blk, "attn", Attention, "implementation"), child(blk, "mlp", Mlp)
+            expect(attn.__dict__, "num_heads", lambda v: v == heads)
+            blocks.append((*norm(blk, "norm1"), *norm(blk, "norm2"), linear(attn, "qkv"), linear(attn, "proj"),
                            linear(mlp, "fc1"), linear(mlp, "fc2")))
-        norm, head = child(model, "norm", nn.LayerNorm), child(model, "head", nn.Linear)
-    except LookupError:
-        return None
-    watch.extend((stack._modules, str(len(stack)), None))          # no block was appended
-    return _cabi.host().vit_plan(dim, heads, int(patch.kernel_size[0]), model._parameters, patch._parameters, head._parameters,
-                                 norm._parameters, float(norm.eps), blocks, watch, empty)
+        expect(stack._modules, str(len(stack)), lambda v: v is None)       # no block was appended
+        last, head = norm(model, "norm"), child(model, "head", nn.Linear)
+    except _NotNative as e:
+        return e.args[0]
+    return _cabi.host().vit_plan(dim, heads, int(size[0]), model._parameters, patch._parameters, head._parameters, *last, blocks,
+                                 watch, empty)
 
 
 def create_vit(name: str, seed: int = 0, num_classes: int = 1000) -> VisionTransformer:

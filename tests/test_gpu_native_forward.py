@@ -167,3 +167,36 @@ def test_autocast_gives_what_the_python_forward_gives(pkg, cuda_device, dtype, m
     assert got.dtype == want.dtype and torch.equal(got, want)
     assert dtype != torch.float16 or torch.equal(got, plain)
     assert pkg.ops.device_status() == 0
+
+
+def _counting(calls):
+    def forward(self, x, **kw):
+        calls.append(type(self).__name__)
+        return type(self).forward(self, x, **kw)
+    return forward
+
+
+@torch.no_grad()
+def test_changes_after_the_first_forward_are_seen(pkg, cuda_device, monkeypatch):
+    """eps, and a forward set on an instance or on a class, against the Python forward; inputs that are not taken keep the plan."""
+    model, images = _small_model(pkg, "deit_small", 4, cuda_device)
+    before = model(images)
+    model.blocks[0].norm1.eps, model.norm.eps = 0.5, 0.25
+    got = model(images)
+    assert not torch.equal(got, before)
+    plan = pkg.vit._PLANS[model]
+    assert torch.equal(model(images.contiguous(memory_format=torch.channels_last)), got)        # the Python forward
+    handle = model.blocks[0].mlp.register_forward_hook(lambda *a: None)
+    assert torch.equal(model(images), got)
+    handle.remove()
+    assert pkg.vit._PLANS[model] is plan
+    calls = []
+    for module in (model.patch_embed, model.blocks[1].attn, model.blocks[0].mlp, model.blocks[1].mlp.fc2, model.head):
+        module.forward = _counting(calls).__get__(module)
+        assert torch.equal(model(images), got) and calls.pop() == type(module).__name__ and not calls
+        del module.forward
+        assert torch.equal(model(images), got) and not calls
+    attention = pkg.vit.Attention.forward
+    monkeypatch.setattr(pkg.vit.Attention, "forward", lambda self, x, **kw: calls.append(1) or attention(self, x, **kw))
+    assert torch.equal(model(images), got) and len(calls) == 2
+    assert pkg.ops.device_status() == 0
