@@ -89,8 +89,9 @@ bool read_linear(PyObject* buffers, Key bias_key, const c10::Device& dev, Linear
       f[1]->numel() != f[0]->numel() || f[2]->numel() != f[0]->numel() || f[4]->numel() != levels || f[5]->numel() != levels - 1)
     return false;
   const at::Tensor* b = tensor_of(PyDict_GetItem(buffers, g_key[bias_key]));
+  if (b == nullptr) return false;                          // no bias is an empty tensor; not among the buffers: a parameter, say
   l->bias = nullptr;
-  if (b != nullptr && b->numel() > 0) {
+  if (b->numel() > 0) {
     if (b->scalar_type() != at::kFloat || b->device() != dev || !b->is_contiguous() || b->numel() != l->N) return false;
     l->bias = b->const_data_ptr<float>();
   }

@@ -200,3 +200,24 @@ def test_changes_after_the_first_forward_are_seen(pkg, cuda_device, monkeypatch)
     monkeypatch.setattr(pkg.vit.Attention, "forward", lambda self, x, **kw: calls.append(1) or attention(self, x, **kw))
     assert torch.equal(model(images), got) and len(calls) == 2
     assert pkg.ops.device_status() == 0
+
+
+@torch.no_grad()
+def test_a_bias_that_is_a_parameter(pkg, cuda_device):
+    """An assigned Parameter is not among the module's buffers, where the native call looks."""
+    for on_the_fly, name in ((True, "bias_tensor"), (False, "bias")):
+        layer, gen = _packed_layer(pkg, 4, 192, 64, cuda_device, on_the_fly)
+        x = torch.randn(50, 192, generator=gen).to(torch.float16 if on_the_fly else torch.float32).to(cuda_device)
+        bias = getattr(layer, name)
+        want = layer(x)
+        delattr(layer, name)
+        setattr(layer, name, torch.nn.Parameter(bias.clone()))
+        assert name not in layer._buffers and torch.equal(layer(x), want)
+    model, images = _small_model(pkg, "deit_tiny", 4, cuda_device)
+    want = model(images)
+    fc1 = model.blocks[0].mlp.fc1
+    bias = fc1.bias_tensor
+    del fc1.bias_tensor
+    fc1.bias_tensor = torch.nn.Parameter(bias.clone())
+    assert torch.equal(model(images), want)
+    assert pkg.ops.device_status() == 0
