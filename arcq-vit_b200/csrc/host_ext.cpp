@@ -49,6 +49,18 @@ at::Tensor empty_cuda(at::IntArrayRef sizes, at::ScalarType t, c10::Device dev) 
 
 const at::Tensor* tensor_of(PyObject* o) { return o != nullptr && THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
 
+// Arguments of another Python type than these are left to the Python code, which takes or refuses them as ever.
+long int_of(PyObject* o) {               // -1: not an int, or out of range
+  int overflow = 0;
+  const long v = PyLong_Check(o) ? PyLong_AsLongAndOverflow(o, &overflow) : -1;
+  return overflow != 0 ? -1 : v;
+}
+bool all_bools(PyObject* const* args, std::initializer_list<int> which) {
+  for (int i : which)
+    if (!PyBool_Check(args[i])) return false;
+  return true;
+}
+
 PyObject* g_oom_error = nullptr;    // torch.OutOfMemoryError
 PyObject* g_key[16];
 enum Key { kPacked, kCenter, kScale, kCodeSum, kWCodebook, kACodebook, kAThresholds, kBiasTensor, kBias, kWeight, kKeys };
@@ -106,12 +118,12 @@ bool read_linear(PyObject* buffers, Key bias_key, const c10::Device& dev, Linear
 // linear(buffers, x, bias key 0 "bias_tensor" / 1 "bias", fp32 output, pre_gelu, pre_quantized) -> y or None
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const at::Tensor* x = n == 6 ? tensor_of(args[1]) : nullptr;
-  if (x == nullptr || !x->is_cuda() || x->dim() < 1 || !x->is_contiguous()) Py_RETURN_NONE;
-  const bool float_chain = PyObject_IsTrue(args[3]), pre_gelu = PyObject_IsTrue(args[4]), ready = PyObject_IsTrue(args[5]);
+  if (x == nullptr || !x->is_cuda() || x->dim() < 1 || !x->is_contiguous() || !all_bools(args, {2, 3, 4, 5})) Py_RETURN_NONE;
+  const bool float_chain = args[3] == Py_True, pre_gelu = args[4] == Py_True, ready = args[5] == Py_True;
   const int xt = dtype_code(x->scalar_type());
   if (xt < 0 || (!float_chain && xt != ARCQ_DT_F16) || ((pre_gelu || ready) && xt != ARCQ_DT_F16)) Py_RETURN_NONE;
   Linear l;
-  if (!read_linear(args[0], PyObject_IsTrue(args[2]) ? kBias : kBiasTensor, x->device(), &l)) Py_RETURN_NONE;
+  if (!read_linear(args[0], args[2] == Py_True ? kBias : kBiasTensor, x->device(), &l)) Py_RETURN_NONE;
   const int64_t numel = x->numel();
   if (x->size(-1) != l.K || numel == 0 || !aligned16(x->const_data_ptr()) || (ready && l.one_fma())) Py_RETURN_NONE;
   const int64_t M = numel / l.K;
@@ -145,14 +157,15 @@ PyObject* quantize_activation(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 6) Py_RETURN_NONE;
   const at::Tensor *x = tensor_of(args[0]), *th = tensor_of(args[1]), *cb = tensor_of(args[2]);
   if (x == nullptr || th == nullptr || cb == nullptr || !x->is_cuda() || x->dim() != 2 || !x->is_contiguous()) Py_RETURN_NONE;
-  const long bits = PyLong_AsLong(args[3]);
+  const long bits = int_of(args[3]);
   const int xt = dtype_code(x->scalar_type());
   for (const at::Tensor* t : {th, cb})
     if (t->scalar_type() != at::kFloat || t->device() != x->device() || !t->is_contiguous()) Py_RETURN_NONE;
   const int64_t M = x->size(0), K = x->size(1);
   if (xt < 0 || bits < 2 || bits > 4 || cb->numel() != (1 << bits) || th->numel() != (1 << bits) - 1 || M == 0 || K == 0 || K % 64 != 0)
     Py_RETURN_NONE;
-  const bool want_cs = PyObject_IsTrue(args[4]), pre_gelu = PyObject_IsTrue(args[5]);
+  if (!all_bools(args, {4, 5})) Py_RETURN_NONE;
+  const bool want_cs = args[4] == Py_True, pre_gelu = args[5] == Py_True;
   const c10::cuda::CUDAGuard guard(x->device());
   at::Tensor packed = empty_cuda({M, K * bits / 8}, at::kByte, x->device());
   at::Tensor mu = empty_cuda({M, K / 64}, at::kFloat, x->device()), sg = empty_cuda({M, K / 64}, at::kFloat, x->device());
@@ -185,13 +198,14 @@ PyObject* dequant(PyObject*, PyObject* const* args, Py_ssize_t n) {
         t[i]->device() != t[0]->device())
       Py_RETURN_NONE;
   }
-  const long bits = PyLong_AsLong(args[5]);
+  const long bits = int_of(args[5]);
   if (bits < 2 || bits > 4 || t[0]->dim() != 2 || t[1]->dim() != 2) Py_RETURN_NONE;
   const int64_t R = t[1]->size(0), K = t[1]->size(1) * 64;
   if (R == 0 || K == 0 || t[0]->size(0) != R || t[0]->size(1) != K * bits / 8 || t[2]->numel() != t[1]->numel() ||
       t[3]->numel() != t[1]->numel() || t[4]->numel() != (1 << bits))
     Py_RETURN_NONE;
-  const bool f32 = PyObject_IsTrue(args[6]);
+  if (!all_bools(args, {6})) Py_RETURN_NONE;
+  const bool f32 = args[6] == Py_True;
   const c10::cuda::CUDAGuard guard(t[0]->device());
   at::Tensor out = empty_cuda({R, K}, f32 ? at::kFloat : at::kHalf, t[0]->device());
   check(arcq_dequant(t[0]->const_data_ptr<uint8_t>(), t[1]->const_data_ptr<float>(), t[2]->const_data_ptr<float>(),

@@ -1,4 +1,6 @@
 """What only the native host path uses, against the separate operators and the Python code it stands for: same bits."""
+import ctypes
+
 import pytest
 import torch
 
@@ -221,3 +223,17 @@ def test_a_bias_that_is_a_parameter(pkg, cuda_device):
     fc1.bias_tensor = torch.nn.Parameter(bias.clone())
     assert torch.equal(model(images), want)
     assert pkg.ops.device_status() == 0
+
+
+def test_arguments_of_other_types_are_the_python_codes(pkg, cuda_device):
+    cb, th = _codebook(torch.Generator().manual_seed(1), 4, cuda_device)
+    x = torch.randn(8, 128, device=cuda_device)
+    want = pkg.ops.quantize_activation(x, th, cb, 4, 64)
+    for bits in (4.0, "4"):
+        with pytest.raises((TypeError, ctypes.ArgumentError)):
+            pkg.ops.quantize_activation(x, th, cb, bits, 64)
+        with pytest.raises((TypeError, ctypes.ArgumentError)):
+            pkg.ops.dequant(*want, cb, bits, 64)
+    for a, b in zip(pkg.ops.quantize_activation(x, th, cb, 4, 64, 1, 0), want):
+        assert torch.equal(a, b)
+    assert pkg.ops.quantize_activation(x, th, cb, 4, 64, False)[3] is None
