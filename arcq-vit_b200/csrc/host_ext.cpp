@@ -10,9 +10,11 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -47,7 +49,12 @@ at::Tensor empty_cuda(at::IntArrayRef sizes, at::ScalarType t, c10::Device dev) 
   return at::detail::empty_cuda(sizes, t, dev, std::nullopt);
 }
 
-const at::Tensor* tensor_of(PyObject* o) { return o != nullptr && THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+// A plain torch.Tensor or Parameter; subclasses, functorch wrappers and the like have behaviour of their own.
+const at::Tensor* tensor_of(PyObject* o) {
+  if (o == nullptr || !THPVariable_CheckExact(o)) return nullptr;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  return at::isTensorSubclassLike(t) ? nullptr : &t;
+}
 
 // Arguments of another Python type than these are left to the Python code, which takes or refuses them as ever.
 long int_of(PyObject* o) {               // -1: not an int, or out of range
@@ -499,6 +506,7 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
 PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+  if (F != &vit_plan && c10::impl::TorchDispatchModeTLS::any_modes_set()) Py_RETURN_NONE;      // the mode wants to see the operators
   try {
     return F(self, args, n);
   } catch (const Fail&) {

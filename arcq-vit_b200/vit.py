@@ -19,6 +19,8 @@ from typing import Callable, Dict, List, Tuple
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 from . import _cabi
 from . import codebook as cbk
@@ -149,7 +151,7 @@ class VisionTransformer(nn.Module):
         images without gradients.  Same kernels in the same order as the code below."""
         if (not x.is_cuda or torch.is_grad_enabled() or len(self.blocks) == 0 or self.fuse_norm_quant != "auto"
                 or type(self) is not VisionTransformer or ARCQPackedLinearOnTheFly.weight_form != "auto"
-                or WeightStager.mode != "stream" or Attention.implementation != "auto" or _has_global_hooks()
+                or WeightStager.mode != "stream" or Attention.implementation != "auto" or _has_global_hooks() or _under_a_mode()
                 or "_forward_fused_glue" in self.__dict__ or any(getattr(c, n) is not f for c, n, f in _STANDS_FOR)):
             return None
         plan = _PLANS.get(self)
@@ -199,6 +201,12 @@ class VisionTransformer(nn.Module):
 
 
 _PLANS: "weakref.WeakKeyDictionary[VisionTransformer, object]" = weakref.WeakKeyDictionary()
+
+
+def _under_a_mode() -> bool:
+    """A function or dispatch mode that wants to see the operators of a forward (a default device is no such mode)."""
+    return (torch._C._len_torch_function_stack() > 0
+            and any(type(m) is not DeviceContext for m in _get_current_function_mode_stack())) or torch._C._len_torch_dispatch_stack() > 0
 
 
 def _has_global_hooks() -> bool:

@@ -237,3 +237,37 @@ def test_arguments_of_other_types_are_the_python_codes(pkg, cuda_device):
     for a, b in zip(pkg.ops.quantize_activation(x, th, cb, 4, 64, 1, 0), want):
         assert torch.equal(a, b)
     assert pkg.ops.quantize_activation(x, th, cb, 4, 64, False)[3] is None
+
+
+@torch.no_grad()
+def test_modes_and_subclasses_see_what_the_python_forward_shows_them(pkg, cuda_device):
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Seen(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            names.append(getattr(func, "__name__", ""))
+            return func(*args, **(kwargs or {}))
+
+    class Dispatched(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            names.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    class Image(torch.Tensor):
+        pass
+
+    model, images = _small_model(pkg, "deit_small", 4, cuda_device)
+    want = model(images)
+    names = []
+    with Seen():
+        assert torch.equal(model(images), want)
+    assert names.count("scaled_dot_product_attention") == 2 and names.count("linear") == 2
+    names = []
+    with Dispatched():
+        assert torch.equal(model(images), want)
+    assert any("attention" in n for n in names)
+    assert model._forward_native(images.as_subclass(Image)) is None
+    assert torch.equal(model(images.as_subclass(Image)).as_subclass(torch.Tensor), want)
+    with torch.device(cuda_device):                            # a default device is no reason to leave the native forward
+        assert torch.equal(model._forward_native(images), want)
