@@ -21,7 +21,7 @@ HOST_PATH = PKG_DIR / "_arcq_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-    "--shared", "-Xcompiler", "-fPIC", "--split-compile=0",
+    "--shared", "-Xcompiler", "-fPIC",
 ]
 
 
