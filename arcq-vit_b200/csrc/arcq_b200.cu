@@ -769,10 +769,6 @@ int arcq_device_status(void) {
   return v;
 }
 
-// Weights whose packed rows are no multiple of 16 bytes (3 bits, an odd number of groups) have always been multiplied by
-// arcq_packed_gemm, which rebuilds them in fp32 and rounds once.  The unpacked ones are the same.
-static int fp32_rebuild(int64_t K, int bits) { return K * bits / 8 % 16 != 0; }
-
 // The unpack jobs of a call as kernel argument.  Blocks of 128 threads or more, each thread taking four 16-byte chunks a
 // round: enough blocks for one round, two per SM at most (they share the SMs with the kernel's own blocks).
 static int make_unpack_jobs(const arcq_unpack_job* jobs, int n, arcq::UnpackJobs* out, int max_blocks = 0) {
@@ -787,7 +783,7 @@ static int make_unpack_jobs(const arcq_unpack_job* jobs, int n, arcq::UnpackJobs
     if (j.rows <= 0 || j.K <= 0 || j.K % 64 != 0) return fail(ARCQ_E_BAD_SHAPE, "bad shape of a weight: rows=%lld K=%lld", (long long)j.rows, (long long)j.K);
     if (!aligned(j.packed, 4) || !aligned(j.out, 16)) return fail(ARCQ_E_ALIGN, "packed codes must be 4-byte, out 16-byte aligned");
     out->job[i] = arcq::UnpackWeightJob{j.packed, j.mu, j.sigma, j.codesum, j.codebook, static_cast<__half*>(j.out),
-                                        static_cast<long long>(j.rows), static_cast<int>(j.K), j.bits, fp32_rebuild(j.K, j.bits)};
+                                        static_cast<long long>(j.rows), static_cast<int>(j.K), j.bits};
     chunks += j.rows * (j.K / 8);
   }
   const long long want = (chunks + 511) / 512, cap = max_blocks > 0 ? max_blocks : 2ll * sm_count();
@@ -1257,7 +1253,7 @@ int arcq_dense_weight_gemm_prefetch(const void* xhat, const void* w16, const flo
     return fail(ARCQ_E_ALIGN, "xhat, w16 and y must be 16-byte aligned");
   const arcq::UnpackWeightJob job = {next_packed, next_mu, next_sigma, next_codesum, next_codebook,
                                      static_cast<__half*>(next_out), static_cast<long long>(next_rows),
-                                     static_cast<int>(next_K), next_bits, 0};
+                                     static_cast<int>(next_K), next_bits};
   PairDenseConfig pc;
   if (M > 0 && choose_pair_dense_config(M, N, K, y_dtype == ARCQ_DT_F32, &pc))
     return launch_pair_dense_gemm(pc, xhat, w16, bias, M, N, K, y, y_dtype, stream, &job);

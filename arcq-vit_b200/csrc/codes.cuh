@@ -105,7 +105,7 @@ __global__ void dequant_kernel(const uint8_t* __restrict__ packed, const float* 
 // cb16 = fp16(cb[c]) and one half-precision fused multiply-add: bit for bit the weight the packed-weight
 // GEMM kernels rebuild in shared memory, written out so that a dense GEMM can read it by TMA.
 // One thread per chunk of 8 codes (16 bytes of output); groups of 64.
-// `fp32_form`: fp16(sigma * cb[c] + mu') with everything in fp32 up to the one rounding, which is what arcq_packed_gemm rebuilds:
+// fp32_form(): fp16(sigma * cb[c] + mu') with everything in fp32 up to the one rounding, which is what arcq_packed_gemm rebuilds:
 // the weight of layers whose packed rows are no multiple of 16 bytes (only 3-bit rows of an odd number of groups, so it is
 // built for 3 bits), which the packed-weight kernels do not take.  (576 x 192, 3 bits: rms relative error of the rebuilt weight
 // 2.1e-4 against 3.6e-4 in the fp16 form.)
@@ -119,7 +119,8 @@ struct UnpackWeightJob {
   long long rows;
   int K;
   int bits;
-  int fp32_form;
+  // see above; not a member, so that the launches that carry jobs keep their size
+  __device__ __forceinline__ bool fp32_form() const { return bits == 3 && (K & 64) != 0; }
 };
 
 // Chunks first, first + stride, ... of the job; `s_cb` holds the 16 codebook values, of type CB: __half, or float for the
@@ -193,7 +194,7 @@ __device__ __forceinline__ void unpack_jobs_run(const UnpackJobs& u, int block, 
     const int i = tid & 15;
     const float level = j.packed != nullptr && i < (1 << j.bits) ? __ldg(j.codebook + i) : 0.0f;
     float* const cb = s_ucb + (tid & 16);
-    if (j.fp32_form) cb[i] = level;
+    if (j.fp32_form()) cb[i] = level;
     else reinterpret_cast<__half*>(cb)[i] = __float2half_rn(level);
   }
   __syncthreads();
@@ -206,7 +207,7 @@ __device__ __forceinline__ void unpack_jobs_run(const UnpackJobs& u, int block, 
     const float* const cb = s_ucb + 16 * k;
     const __half* const cb16 = reinterpret_cast<const __half*>(cb);
     if (j.bits == 4) unpack_weight_f16_chunks<4>(j, cb16, first, stride);
-    else if (j.bits == 3 && j.fp32_form) unpack_weight_f16_chunks<3>(j, cb, first, stride);
+    else if (j.fp32_form()) unpack_weight_f16_chunks<3>(j, cb, first, stride);
     else if (j.bits == 3) unpack_weight_f16_chunks<3>(j, cb16, first, stride);
     else unpack_weight_f16_chunks<2>(j, cb16, first, stride);
   }
@@ -230,7 +231,7 @@ __global__ void unpack_weight_f16_kernel(const uint8_t* __restrict__ packed, con
   __shared__ __half s_cb[16];
   if (threadIdx.x < 16) s_cb[threadIdx.x] = __float2half_rn((threadIdx.x < (1 << BITS)) ? codebook[threadIdx.x] : 0.0f);
   __syncthreads();
-  const UnpackWeightJob j = {packed, mu, sigma, codesum, codebook, out, rows, K, BITS, 0};
+  const UnpackWeightJob j = {packed, mu, sigma, codesum, codebook, out, rows, K, BITS};
   unpack_weight_f16_chunks<BITS>(j, s_cb, blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x,
                                  static_cast<long long>(gridDim.x) * blockDim.x);
 }
