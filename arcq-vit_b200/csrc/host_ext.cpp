@@ -10,7 +10,6 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
-#include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -18,6 +17,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <stdexcept>
 #include <string>
 #include <vector>
 
@@ -25,14 +25,38 @@
 
 namespace {
 
-struct Fail {};   // a Python error is set
-
 void check(int rc, const char* what) {
-  if (rc != ARCQ_OK) {
-    PyErr_Format(PyExc_RuntimeError, "%s failed (%d): %s", what, rc, arcq_last_error_string());
-    throw Fail{};
-  }
+  if (rc != ARCQ_OK)
+    throw std::runtime_error(std::string(what) + " failed (" + std::to_string(rc) + "): " + arcq_last_error_string());
 }
+
+// Other Python threads run while a call allocates and launches: with a full launch queue that waits for the GPU.  What the call
+// reads out of Python objects is read, and held, before.
+struct WithoutGil {
+  PyThreadState* const state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+template <typename F> auto without_gil(F work) {
+  const WithoutGil released;
+  return work();
+}
+// The Python tensors that a call reads, kept from being replaced under it (references counted with the lock held: cheaper than
+// copies of the tensors, 0.5 us a layer).
+class Held {
+ public:
+  Held() = default;
+  Held(const Held&) = delete;
+  ~Held() {
+    for (PyObject* o : objects_) Py_DECREF(o);
+  }
+  void add(PyObject* o) {
+    Py_INCREF(o);
+    objects_.push_back(o);
+  }
+
+ private:
+  c10::SmallVector<PyObject*, 16> objects_;
+};
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
@@ -53,7 +77,10 @@ at::Tensor empty_cuda(at::IntArrayRef sizes, at::ScalarType t, c10::Device dev) 
 const at::Tensor* tensor_of(PyObject* o) {
   if (o == nullptr || !THPVariable_CheckExact(o)) return nullptr;
   const at::Tensor& t = THPVariable_Unpack(o);
-  return at::isTensorSubclassLike(t) ? nullptr : &t;
+  using K = c10::DispatchKey;
+  constexpr c10::DispatchKeySet wrappers({K::Python, K::Functionalize, K::FuncTorchBatched, K::FuncTorchGradWrapper, K::BatchedNestedTensor,
+                                          K::NestedTensor});
+  return t.key_set().has_any(wrappers) ? nullptr : &t;
 }
 
 // Arguments of another Python type than these are left to the Python code, which takes or refuses them as ever.
@@ -75,9 +102,11 @@ const char* const kKeyNames[kKeys] = {"packed_weight_codes", "weight_center", "w
                                       "activation_codebook", "activation_thresholds", "bias_tensor", "bias", "weight"};
 
 // A contiguous CUDA tensor of the given type out of a module's dictionary, or null.
-const at::Tensor* device_tensor(PyObject* dict, Key key, at::ScalarType t, const c10::Device& dev) {
-  const at::Tensor* v = tensor_of(PyDict_GetItem(dict, g_key[key]));
+const at::Tensor* device_tensor(PyObject* dict, PyObject* key, at::ScalarType t, const c10::Device& dev, Held* held) {
+  PyObject* const o = PyDict_GetItemWithError(dict, key);
+  const at::Tensor* v = tensor_of(o);
   if (v == nullptr || v->scalar_type() != t || v->device() != dev || !v->is_contiguous()) return nullptr;
+  held->add(o);
   return v;
 }
 
@@ -92,13 +121,13 @@ struct Linear {
   bool one_fma() const { return K * bits / 8 % 16 != 0; }
 };
 
-bool read_linear(PyObject* buffers, Key bias_key, const c10::Device& dev, Linear* l) {
+bool read_linear(PyObject* buffers, Key bias_key, const c10::Device& dev, Linear* l, Held* held) {
   if (!PyDict_Check(buffers)) return false;
-  const at::Tensor* codes = device_tensor(buffers, kPacked, at::kByte, dev);
+  const at::Tensor* codes = device_tensor(buffers, g_key[kPacked], at::kByte, dev, held);
   const at::Tensor* f[6];
   const Key keys[6] = {kCenter, kScale, kCodeSum, kWCodebook, kACodebook, kAThresholds};
   for (int i = 0; i < 6; ++i)
-    if ((f[i] = device_tensor(buffers, keys[i], at::kFloat, dev)) == nullptr) return false;
+    if ((f[i] = device_tensor(buffers, g_key[keys[i]], at::kFloat, dev, held)) == nullptr) return false;
   if (codes == nullptr || codes->dim() != 2 || f[0]->dim() != 2) return false;
   const int64_t levels = f[3]->numel();
   l->bits = levels == 16 ? 4 : levels == 8 ? 3 : levels == 4 ? 2 : 0;
@@ -107,7 +136,8 @@ bool read_linear(PyObject* buffers, Key bias_key, const c10::Device& dev, Linear
   if (l->bits == 0 || l->N % 16 != 0 || l->N == 0 || l->K == 0 || codes->size(0) != l->N || codes->size(1) != l->K * l->bits / 8 ||
       f[1]->numel() != f[0]->numel() || f[2]->numel() != f[0]->numel() || f[4]->numel() != levels || f[5]->numel() != levels - 1)
     return false;
-  const at::Tensor* b = tensor_of(PyDict_GetItem(buffers, g_key[bias_key]));
+  PyObject* const bias = PyDict_GetItemWithError(buffers, g_key[bias_key]);
+  const at::Tensor* b = tensor_of(bias);
   if (b == nullptr) return false;                          // no bias is an empty tensor; not among the buffers: a parameter, say
   l->bias = nullptr;
   if (b->numel() > 0) {
@@ -118,6 +148,7 @@ bool read_linear(PyObject* buffers, Key bias_key, const c10::Device& dev, Linear
   l->th = f[5]->const_data_ptr<float>();
   l->job = arcq_unpack_job{codes->const_data_ptr<uint8_t>(), f[0]->const_data_ptr<float>(), f[1]->const_data_ptr<float>(),
                            f[2]->const_data_ptr<float>(), f[3]->const_data_ptr<float>(), nullptr, l->N, l->K, l->bits};
+  held->add(bias);
   return (reinterpret_cast<uintptr_t>(l->job.packed) & 3u) == 0;
 }
 
@@ -130,31 +161,35 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const int xt = dtype_code(x->scalar_type());
   if (xt < 0 || (!float_chain && xt != ARCQ_DT_F16) || ((pre_gelu || ready) && xt != ARCQ_DT_F16)) Py_RETURN_NONE;
   Linear l;
-  if (!read_linear(args[0], args[2] == Py_True ? kBias : kBiasTensor, x->device(), &l)) Py_RETURN_NONE;
+  Held held;
+  if (!read_linear(args[0], args[2] == Py_True ? kBias : kBiasTensor, x->device(), &l, &held)) Py_RETURN_NONE;
   const int64_t numel = x->numel();
   if (x->size(-1) != l.K || numel == 0 || !aligned16(x->const_data_ptr()) || (ready && l.one_fma())) Py_RETURN_NONE;
   const int64_t M = numel / l.K;
-  const c10::cuda::CUDAGuard guard(x->device());
-  void* const st = c10::cuda::getCurrentCUDAStream().stream();
-  // the reconstructed activation and the unpacked weight, given back to the caching allocator on return
-  const at::Tensor scratch = empty_cuda({(ready ? 0 : numel) + l.weight_elems() + 8}, at::kHalf, x->device());
-  at::Half* const w16 = scratch.mutable_data_ptr<at::Half>();
-  const void* xhat = x->const_data_ptr();
-  l.job.out = w16;
-  if (ready) {
-    check(arcq_unpack_weight_f16(l.job.packed, l.job.mu, l.job.sigma, l.job.codesum, l.job.codebook, l.bits, 64, l.N, l.K, w16, st),
-          "arcq_unpack_weight_f16");
-  } else {
-    void* const xh = w16 + l.weight_elems();
-    check(arcq_act_quant_unpack(pre_gelu, xhat, xt, M, l.K, l.th, l.acb, l.bits, 64, xh, ARCQ_DT_F16, l.one_fma(), &l.job, 1, st),
-          "arcq_act_quant");
-    xhat = xh;
-  }
-  c10::SmallVector<int64_t, 5> sizes(x->sizes().begin(), x->sizes().end());
-  sizes.back() = l.N;
-  at::Tensor y = empty_cuda(sizes, float_chain ? at::kFloat : at::kHalf, x->device());
-  check(arcq_dense_weight_gemm(xhat, w16, l.bias, M, l.N, l.K, y.mutable_data_ptr(), float_chain ? ARCQ_DT_F32 : ARCQ_DT_F16, st),
-        "arcq_dense_weight_gemm");
+  at::Tensor y = without_gil([&] {
+    const c10::cuda::CUDAGuard guard(x->device());
+    void* const st = c10::cuda::getCurrentCUDAStream().stream();
+    // the reconstructed activation and the unpacked weight, given back to the caching allocator on return
+    const at::Tensor scratch = empty_cuda({(ready ? 0 : numel) + l.weight_elems() + 8}, at::kHalf, x->device());
+    at::Half* const w16 = scratch.mutable_data_ptr<at::Half>();
+    const void* xhat = x->const_data_ptr();
+    l.job.out = w16;
+    if (ready) {
+      check(arcq_unpack_weight_f16(l.job.packed, l.job.mu, l.job.sigma, l.job.codesum, l.job.codebook, l.bits, 64, l.N, l.K, w16, st),
+            "arcq_unpack_weight_f16");
+    } else {
+      void* const xh = w16 + l.weight_elems();
+      check(arcq_act_quant_unpack(pre_gelu, xhat, xt, M, l.K, l.th, l.acb, l.bits, 64, xh, ARCQ_DT_F16, l.one_fma(), &l.job, 1, st),
+            "arcq_act_quant");
+      xhat = xh;
+    }
+    c10::SmallVector<int64_t, 5> sizes(x->sizes().begin(), x->sizes().end());
+    sizes.back() = l.N;
+    at::Tensor y = empty_cuda(sizes, float_chain ? at::kFloat : at::kHalf, x->device());
+    check(arcq_dense_weight_gemm(xhat, w16, l.bias, M, l.N, l.K, y.mutable_data_ptr(), float_chain ? ARCQ_DT_F32 : ARCQ_DT_F16, st),
+          "arcq_dense_weight_gemm");
+    return y;
+  });
   return THPVariable_Wrap(std::move(y));
 }
 
@@ -173,15 +208,19 @@ PyObject* quantize_activation(PyObject*, PyObject* const* args, Py_ssize_t n) {
     Py_RETURN_NONE;
   if (!all_bools(args, {4, 5})) Py_RETURN_NONE;
   const bool want_cs = args[4] == Py_True, pre_gelu = args[5] == Py_True;
-  const c10::cuda::CUDAGuard guard(x->device());
-  at::Tensor packed = empty_cuda({M, K * bits / 8}, at::kByte, x->device());
-  at::Tensor mu = empty_cuda({M, K / 64}, at::kFloat, x->device()), sg = empty_cuda({M, K / 64}, at::kFloat, x->device());
-  at::Tensor cs = want_cs ? empty_cuda({M, K / 64}, at::kFloat, x->device()) : at::Tensor();
-  check((pre_gelu ? arcq_gelu_act_quant : arcq_act_quant)(
-            x->const_data_ptr(), xt, M, K, th->const_data_ptr<float>(), cb->const_data_ptr<float>(), static_cast<int>(bits), 64,
-            packed.mutable_data_ptr<uint8_t>(), mu.mutable_data_ptr<float>(), sg.mutable_data_ptr<float>(),
-            want_cs ? cs.mutable_data_ptr<float>() : nullptr, nullptr, 0, c10::cuda::getCurrentCUDAStream().stream()),
-        "arcq_act_quant");
+  at::Tensor packed, mu, sg, cs;
+  without_gil([&] {
+    const c10::cuda::CUDAGuard guard(x->device());
+    packed = empty_cuda({M, K * bits / 8}, at::kByte, x->device());
+    mu = empty_cuda({M, K / 64}, at::kFloat, x->device());
+    sg = empty_cuda({M, K / 64}, at::kFloat, x->device());
+    if (want_cs) cs = empty_cuda({M, K / 64}, at::kFloat, x->device());
+    check((pre_gelu ? arcq_gelu_act_quant : arcq_act_quant)(
+              x->const_data_ptr(), xt, M, K, th->const_data_ptr<float>(), cb->const_data_ptr<float>(), static_cast<int>(bits), 64,
+              packed.mutable_data_ptr<uint8_t>(), mu.mutable_data_ptr<float>(), sg.mutable_data_ptr<float>(),
+              want_cs ? cs.mutable_data_ptr<float>() : nullptr, nullptr, 0, c10::cuda::getCurrentCUDAStream().stream()),
+          "arcq_act_quant");
+  });
   PyObject* out = PyTuple_New(4);
   PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(std::move(packed)));
   PyTuple_SET_ITEM(out, 1, THPVariable_Wrap(std::move(mu)));
@@ -213,12 +252,15 @@ PyObject* dequant(PyObject*, PyObject* const* args, Py_ssize_t n) {
     Py_RETURN_NONE;
   if (!all_bools(args, {6})) Py_RETURN_NONE;
   const bool f32 = args[6] == Py_True;
-  const c10::cuda::CUDAGuard guard(t[0]->device());
-  at::Tensor out = empty_cuda({R, K}, f32 ? at::kFloat : at::kHalf, t[0]->device());
-  check(arcq_dequant(t[0]->const_data_ptr<uint8_t>(), t[1]->const_data_ptr<float>(), t[2]->const_data_ptr<float>(),
-                     t[3]->const_data_ptr<float>(), t[4]->const_data_ptr<float>(), static_cast<int>(bits), 64, R, K,
-                     out.mutable_data_ptr(), f32 ? ARCQ_DT_F32 : ARCQ_DT_F16, c10::cuda::getCurrentCUDAStream().stream()),
-        "arcq_dequant");
+  at::Tensor out = without_gil([&] {
+    const c10::cuda::CUDAGuard guard(t[0]->device());
+    at::Tensor out = empty_cuda({R, K}, f32 ? at::kFloat : at::kHalf, t[0]->device());
+    check(arcq_dequant(t[0]->const_data_ptr<uint8_t>(), t[1]->const_data_ptr<float>(), t[2]->const_data_ptr<float>(),
+                       t[3]->const_data_ptr<float>(), t[4]->const_data_ptr<float>(), static_cast<int>(bits), 64, R, K,
+                       out.mutable_data_ptr(), f32 ? ARCQ_DT_F32 : ARCQ_DT_F16, c10::cuda::getCurrentCUDAStream().stream()),
+          "arcq_dequant");
+    return out;
+  });
   return THPVariable_Wrap(std::move(out));
 }
 
@@ -259,14 +301,16 @@ struct NormView {
   const void *gamma, *beta;
   int dtype;
 };
-bool read_norm(const Norm& n, const c10::Device& dev, int64_t dim, NormView* v) {
+bool read_norm(const Norm& n, const c10::Device& dev, int64_t dim, NormView* v, Held* held) {
   const void* p[2];
   for (int i = 0; i < 2; ++i) {
-    const at::Tensor* t = tensor_of(PyDict_GetItem(n.params, g_key[i ? kBias : kWeight]));
+    PyObject* const o = PyDict_GetItemWithError(n.params, g_key[i ? kBias : kWeight]);
+    const at::Tensor* t = tensor_of(o);
     if (t == nullptr || t->device() != dev || t->numel() != dim || !t->is_contiguous() || !aligned16(t->const_data_ptr())) return false;
     const int d = dtype_code(t->scalar_type());
     if (d < 0 || (i == 1 && d != v->dtype)) return false;
     v->dtype = d;
+    held->add(o);
     p[i] = t->const_data_ptr();
   }
   v->gamma = p[0];
@@ -325,7 +369,7 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
   auto* p = static_cast<VitPlan*>(PyCapsule_GetPointer(args[0], "arcq_vit_plan"));
   if (p == nullptr) return nullptr;
   for (size_t i = 0; i < p->watch.size(); i += 3) {
-    PyObject* const got = PyDict_GetItem(p->watch[i], p->watch[i + 1]);
+    PyObject* const got = PyDict_GetItemWithError(p->watch[i], p->watch[i + 1]);
     if (got != p->watch[i + 2] && !(got == nullptr && p->watch[i + 2] == Py_None)) Py_RETURN_FALSE;
   }
   const at::Tensor* img = tensor_of(args[1]);
@@ -343,14 +387,14 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
   static PyObject* const k_cls = PyUnicode_InternFromString("cls_token");
   static PyObject* const k_pos = PyUnicode_InternFromString("pos_embed");
-  const at::Tensor *cls = tensor_of(PyDict_GetItem(p->own, k_cls)), *pos = tensor_of(PyDict_GetItem(p->own, k_pos));
-  const at::Tensor* pw = device_tensor(p->patch_params, kWeight, at::kHalf, dev);
-  const at::Tensor* pb = device_tensor(p->patch_params, kBias, at::kHalf, dev);
-  const at::Tensor* hw = device_tensor(p->head_params, kWeight, at::kHalf, dev);
-  const at::Tensor* hb = device_tensor(p->head_params, kBias, at::kHalf, dev);
+  Held held;
+  const at::Tensor *cls = device_tensor(p->own, k_cls, at::kHalf, dev, &held), *pos = device_tensor(p->own, k_pos, at::kHalf, dev, &held);
+  const at::Tensor* pw = device_tensor(p->patch_params, g_key[kWeight], at::kHalf, dev, &held);
+  const at::Tensor* pb = device_tensor(p->patch_params, g_key[kBias], at::kHalf, dev, &held);
+  const at::Tensor* hw = device_tensor(p->head_params, g_key[kWeight], at::kHalf, dev, &held);
+  const at::Tensor* hb = device_tensor(p->head_params, g_key[kBias], at::kHalf, dev, &held);
   for (const at::Tensor* t : {cls, pos})
-    if (t == nullptr || t->scalar_type() != at::kHalf || t->device() != dev || !t->is_contiguous() || !aligned16(t->const_data_ptr()))
-      Py_RETURN_NONE;
+    if (t == nullptr || !aligned16(t->const_data_ptr())) Py_RETURN_NONE;
   if (pw == nullptr || pb == nullptr || hw == nullptr || hb == nullptr || cls->numel() != D || pos->numel() != T * D ||
       pw->numel() != D * C * P * P)
     Py_RETURN_NONE;
@@ -364,144 +408,148 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const int64_t shape[4][2] = {{3 * D, D}, {D, D}, {4 * D, D}, {D, 4 * D}};
     for (int k = 0; k < 4; ++k) {
       Linear& l = lin[4 * i + k];
-      if (!read_linear(d[k], kBiasTensor, dev, &l)) Py_RETURN_NONE;
+      if (!read_linear(d[k], kBiasTensor, dev, &l, &held)) Py_RETURN_NONE;
       // any hidden width, the rest as the block's structure fixes it
       if (k < 2 ? (l.N != shape[k][0] || l.K != shape[k][1]) : k == 2 ? l.K != D : (l.N != D || l.K != lin[4 * i + 2].N)) Py_RETURN_NONE;
     }
     scratch_elems[0] = std::max(scratch_elems[0], lin[4 * i].weight_elems() + lin[4 * i + 1].weight_elems());
     scratch_elems[1] = std::max(scratch_elems[1], lin[4 * i + 2].weight_elems() + lin[4 * i + 3].weight_elems());
-    if (!read_norm(b.norm1, dev, D, &norms[2 * i]) || !read_norm(b.norm2, dev, D, &norms[2 * i + 1])) Py_RETURN_NONE;
+    if (!read_norm(b.norm1, dev, D, &norms[2 * i], &held) || !read_norm(b.norm2, dev, D, &norms[2 * i + 1], &held)) Py_RETURN_NONE;
   }
-  if (!read_norm(p->norm, dev, D, &norms[2 * depth])) Py_RETURN_NONE;
+  if (!read_norm(p->norm, dev, D, &norms[2 * depth], &held)) Py_RETURN_NONE;
   int64_t hidden = 0;
   for (size_t i = 0; i < depth; ++i) hidden = std::max(hidden, lin[4 * i + 2].N);
 
-  const c10::cuda::CUDAGuard guard(dev);
-  void* const st = c10::cuda::getCurrentCUDAStream().stream();
-  // one workspace: residual stream (two, written in turn), reconstruction, branch output, qkv / fc1 output, fc2 input, weights
-  const int64_t wide = std::max<int64_t>(3 * D, hidden);
-  const at::Tensor ws = empty_cuda({M * (4 * D + wide + hidden) + scratch_elems[0] + scratch_elems[1] + 64}, at::kHalf, dev);
-  at::Half* at_ptr = ws.mutable_data_ptr<at::Half>();
-  auto take = [&](int64_t elems) {
-    at::Half* r = at_ptr;
-    at_ptr += (elems + 7) / 8 * 8;
-    return r;
-  };
-  at::Half *x = take(M * D), *x_next = take(M * D), *xhat = take(M * D), *branch = take(M * D), *mid = take(M * wide), *xhat4 = take(M * hidden);
-  at::Half *w_attn = take(scratch_elems[0]), *w_mlp = take(scratch_elems[1]);
-  for (size_t i = 0; i < depth; ++i) {
-    lin[4 * i].job.out = w_attn;
-    lin[4 * i + 1].job.out = w_attn + lin[4 * i].weight_elems();
-    lin[4 * i + 2].job.out = w_mlp;
-    lin[4 * i + 3].job.out = w_mlp + lin[4 * i + 2].weight_elems();
-  }
-  // Where the weights of a half block (qkv + proj, fc1 + fc2) are unpacked.  Few rows: by the GEMM that ends the half block
-  // before, on the SMs it leaves idle, while it reads the other scratch matrix; what has no room there by the half block's own
-  // first GEMM (its second weight) or the LayerNorm.  Many rows: the GEMMs fill the machine, and extra blocks of the LayerNorm
-  // + quantizer launch do it.
-  const bool beside_gemm = arcq_unpack_beside_gemm(M, D) != 0;
-  int done = 0;                        // of the next half block's two weights
-  auto jobs_of = [&](const Linear* half, int from, int to, arcq_unpack_job (&jobs)[2]) {
-    for (int k = from; k < to; ++k) jobs[k - from] = half[k].job;
-    return to - from;
-  };
-  // what the GEMM of a layer can take along, asked once per shape
-  struct Room {
-    int64_t N, K, values;
-    int gelu_quant;
-  };
-  std::vector<Room> rooms;
-  auto room_of = [&](const Linear& l, int gelu_quant) {
-    for (const Room& r : rooms)
-      if (r.N == l.N && r.K == l.K && r.gelu_quant == gelu_quant) return r.values;
-    rooms.push_back({l.N, l.K, arcq_dense_weight_gemm_unpack_room(M, l.N, l.K, gelu_quant), gelu_quant});
-    return rooms.back().values;
-  };
-  // how far the weights of `half` from `from` on fit into what the GEMM of `l` can take along
-  auto fits = [&](const Linear* half, int from, const Linear& l, int gelu_quant) {
-    if (!beside_gemm || half == nullptr) return from;
-    int64_t room = room_of(l, gelu_quant);
-    while (from < 2 && half[from].weight_elems() <= room) room -= half[from++].weight_elems();
-    return from;
-  };
-  auto norm_quant = [&](const at::Half* y, const NormView& nv, double eps, const Linear* half, int gelu_quant) {
-    // the first weight has to be there before the half block's first GEMM, the second may be that GEMM's job
-    const int first = std::max(done, 1), to = fits(half, first, half[0], gelu_quant) == 2 ? first : 2;
-    arcq_unpack_job jobs[2];
-    const int n = jobs_of(half, done, to, jobs);
-    check(arcq_add_layernorm_act_quant_unpack(x, y, nv.gamma, nv.beta, nv.dtype, static_cast<float>(eps), M, D, half[0].th, half[0].acb,
-                                              half[0].bits, 64, y != nullptr ? x_next : nullptr, nullptr, xhat, half[0].one_fma(), jobs,
-                                              n, st),
-          "arcq_add_layernorm_act_quant");
-    if (y != nullptr) std::swap(x, x_next);
-    done = to;
-  };
-  auto gemm = [&](const at::Half* a, const Linear& l, at::Half* y, const arcq_unpack_job* jobs, int n) {
-    check(arcq_dense_weight_gemm_unpack(a, l.job.out, l.bias, M, l.N, l.K, y, ARCQ_DT_F16, jobs, n, st), "arcq_dense_weight_gemm");
-  };
-  // The last GEMM of a half block; next: the linears of the next one, or null.  Both weights in two rounds of the idle SMs'
-  // threads, or the second one left to the next GEMM if that has room.
-  auto last_gemm = [&](const at::Half* a, const Linear& l, at::Half* y, const Linear* next, int next_gelu_quant) {
-    arcq_unpack_job jobs[2];
-    done = fits(next, 0, l, 0);
-    if (done == 2 && next[0].weight_elems() + next[1].weight_elems() > room_of(l, 0) * 2 / 5 && fits(next, 1, next[0], next_gelu_quant) == 2)
-      done = 1;
-    gemm(a, l, y, jobs, jobs_of(next, 0, done, jobs));
-  };
+  at::Tensor logits = without_gil([&] {
+    const c10::cuda::CUDAGuard guard(dev);
+    void* const st = c10::cuda::getCurrentCUDAStream().stream();
+    // one workspace: residual stream (two, written in turn), reconstruction, branch output, qkv / fc1 output, fc2 input, weights
+    const int64_t wide = std::max<int64_t>(3 * D, hidden);
+    const at::Tensor ws = empty_cuda({M * (4 * D + wide + hidden) + scratch_elems[0] + scratch_elems[1] + 64}, at::kHalf, dev);
+    at::Half* at_ptr = ws.mutable_data_ptr<at::Half>();
+    auto take = [&](int64_t elems) {
+      at::Half* r = at_ptr;
+      at_ptr += (elems + 7) / 8 * 8;
+      return r;
+    };
+    at::Half *x = take(M * D), *x_next = take(M * D), *xhat = take(M * D), *branch = take(M * D), *mid = take(M * wide), *xhat4 = take(M * hidden);
+    at::Half *w_attn = take(scratch_elems[0]), *w_mlp = take(scratch_elems[1]);
+    for (size_t i = 0; i < depth; ++i) {
+      lin[4 * i].job.out = w_attn;
+      lin[4 * i + 1].job.out = w_attn + lin[4 * i].weight_elems();
+      lin[4 * i + 2].job.out = w_mlp;
+      lin[4 * i + 3].job.out = w_mlp + lin[4 * i + 2].weight_elems();
+    }
+    // Where the weights of a half block (qkv + proj, fc1 + fc2) are unpacked.  Few rows: by the GEMM that ends the half block
+    // before, on the SMs it leaves idle, while it reads the other scratch matrix; what has no room there by the half block's own
+    // first GEMM (its second weight) or the LayerNorm.  Many rows: the GEMMs fill the machine, and extra blocks of the LayerNorm
+    // + quantizer launch do it.
+    const bool beside_gemm = arcq_unpack_beside_gemm(M, D) != 0;
+    int done = 0;                        // of the next half block's two weights
+    auto jobs_of = [&](const Linear* half, int from, int to, arcq_unpack_job (&jobs)[2]) {
+      for (int k = from; k < to; ++k) jobs[k - from] = half[k].job;
+      return to - from;
+    };
+    // what the GEMM of a layer can take along, asked once per shape
+    struct Room {
+      int64_t N, K, values;
+      int gelu_quant;
+    };
+    std::vector<Room> rooms;
+    auto room_of = [&](const Linear& l, int gelu_quant) {
+      for (const Room& r : rooms)
+        if (r.N == l.N && r.K == l.K && r.gelu_quant == gelu_quant) return r.values;
+      rooms.push_back({l.N, l.K, arcq_dense_weight_gemm_unpack_room(M, l.N, l.K, gelu_quant), gelu_quant});
+      return rooms.back().values;
+    };
+    // how far the weights of `half` from `from` on fit into what the GEMM of `l` can take along
+    auto fits = [&](const Linear* half, int from, const Linear& l, int gelu_quant) {
+      if (!beside_gemm || half == nullptr) return from;
+      int64_t room = room_of(l, gelu_quant);
+      while (from < 2 && half[from].weight_elems() <= room) room -= half[from++].weight_elems();
+      return from;
+    };
+    auto norm_quant = [&](const at::Half* y, const NormView& nv, double eps, const Linear* half, int gelu_quant) {
+      // the first weight has to be there before the half block's first GEMM, the second may be that GEMM's job
+      const int first = std::max(done, 1), to = fits(half, first, half[0], gelu_quant) == 2 ? first : 2;
+      arcq_unpack_job jobs[2];
+      const int n = jobs_of(half, done, to, jobs);
+      check(arcq_add_layernorm_act_quant_unpack(x, y, nv.gamma, nv.beta, nv.dtype, static_cast<float>(eps), M, D, half[0].th, half[0].acb,
+                                                half[0].bits, 64, y != nullptr ? x_next : nullptr, nullptr, xhat, half[0].one_fma(), jobs,
+                                                n, st),
+            "arcq_add_layernorm_act_quant");
+      if (y != nullptr) std::swap(x, x_next);
+      done = to;
+    };
+    auto gemm = [&](const at::Half* a, const Linear& l, at::Half* y, const arcq_unpack_job* jobs, int n) {
+      check(arcq_dense_weight_gemm_unpack(a, l.job.out, l.bias, M, l.N, l.K, y, ARCQ_DT_F16, jobs, n, st), "arcq_dense_weight_gemm");
+    };
+    // The last GEMM of a half block; next: the linears of the next one, or null.  Both weights in two rounds of the idle SMs'
+    // threads, or the second one left to the next GEMM if that has room.
+    auto last_gemm = [&](const at::Half* a, const Linear& l, at::Half* y, const Linear* next, int next_gelu_quant) {
+      arcq_unpack_job jobs[2];
+      done = fits(next, 0, l, 0);
+      if (done == 2 && next[0].weight_elems() + next[1].weight_elems() > room_of(l, 0) * 2 / 5 && fits(next, 1, next[0], next_gelu_quant) == 2)
+        done = 1;
+      gemm(a, l, y, jobs, jobs_of(next, 0, done, jobs));
+    };
 
-  {
-    const at::Tensor rows = empty_cuda({B * (T - 1), C * P * P}, at::kHalf, dev);
-    check(arcq_patchify(img->const_data_ptr(), B, C, H, W, static_cast<int>(P), rows.mutable_data_ptr(), st), "arcq_patchify");
-    const at::Tensor patches = at::linear(rows, pw->view({D, C * P * P}), *pb);
-    check(arcq_assemble_tokens(half_matrix(patches, B * (T - 1) * D, dev), cls->const_data_ptr(), pos->const_data_ptr(), B, T - 1, D, x, st),
-          "arcq_assemble_tokens");
-  }
-  const at::Half* y = nullptr;
-  int64_t asked[2] = {0, 0};            // the shape of fc1 that `applies` holds for
-  bool applies = false;
-  for (size_t i = 0; i < depth; ++i) {
-    const VitBlock& b = p->blocks[i];
-    const Linear *qkv = &lin[4 * i], *proj = qkv + 1, *fc1 = qkv + 2, *fc2 = qkv + 3;
-    if (asked[0] != fc1->N || asked[1] != fc1->K) {
-      applies = arcq_dense_weight_gemm_gelu_quant_applies(M, fc1->N, fc1->K) != 0;
-      asked[0] = fc1->N;
-      asked[1] = fc1->K;
-    }
-    const bool fused = applies && !fc2->one_fma();     // the fused form reconstructs in three steps only
-    arcq_unpack_job jobs[2];
-    norm_quant(y, norms[2 * i], b.norm1.eps, qkv, 0);
-    gemm(xhat, *qkv, mid, jobs, jobs_of(qkv, done, 2, jobs));
     {
-      const at::Tensor t = at::from_blob(mid, {B, T, 3, p->heads, D / p->heads}, at::TensorOptions().dtype(at::kHalf).device(dev));
-      const at::Tensor r = t.permute({2, 0, 3, 1, 4});
-      const at::Tensor o = at::scaled_dot_product_attention(r[0], r[1], r[2]).transpose(1, 2).reshape({M, D}).contiguous();
-      check(arcq_act_quant_unpack(0, half_matrix(o, M * D, dev), ARCQ_DT_F16, M, D, proj->th, proj->acb, proj->bits, 64, xhat,
-                                  ARCQ_DT_F16, proj->one_fma(), nullptr, 0, st),
-            "arcq_act_quant");
+      const at::Tensor rows = empty_cuda({B * (T - 1), C * P * P}, at::kHalf, dev);
+      check(arcq_patchify(img->const_data_ptr(), B, C, H, W, static_cast<int>(P), rows.mutable_data_ptr(), st), "arcq_patchify");
+      const at::Tensor patches = at::linear(rows, pw->view({D, C * P * P}), *pb);
+      check(arcq_assemble_tokens(half_matrix(patches, B * (T - 1) * D, dev), cls->const_data_ptr(), pos->const_data_ptr(), B, T - 1, D, x,
+                                 st),
+            "arcq_assemble_tokens");
     }
-    last_gemm(xhat, *proj, branch, fc1, fused);
-    norm_quant(branch, norms[2 * i + 1], b.norm2.eps, fc1, fused);
-    const int n = jobs_of(fc1, done, 2, jobs);
-    if (fused) {
-      check(arcq_dense_weight_gemm_gelu_quant(xhat, fc1->job.out, fc1->bias, M, fc1->N, fc1->K, fc2->th, fc2->acb, fc2->bits, 64, xhat4,
-                                              jobs, n, st),
-            "arcq_dense_weight_gemm_gelu_quant");
-    } else {
-      gemm(xhat, *fc1, mid, jobs, n);
-      check(arcq_act_quant_unpack(1, mid, ARCQ_DT_F16, M, fc2->K, fc2->th, fc2->acb, fc2->bits, 64, xhat4, ARCQ_DT_F16, fc2->one_fma(),
-                                  nullptr, 0, st),
-            "arcq_gelu_act_quant");
+    const at::Half* y = nullptr;
+    int64_t asked[2] = {0, 0};            // the shape of fc1 that `applies` holds for
+    bool applies = false;
+    for (size_t i = 0; i < depth; ++i) {
+      const VitBlock& b = p->blocks[i];
+      const Linear *qkv = &lin[4 * i], *proj = qkv + 1, *fc1 = qkv + 2, *fc2 = qkv + 3;
+      if (asked[0] != fc1->N || asked[1] != fc1->K) {
+        applies = arcq_dense_weight_gemm_gelu_quant_applies(M, fc1->N, fc1->K) != 0;
+        asked[0] = fc1->N;
+        asked[1] = fc1->K;
+      }
+      const bool fused = applies && !fc2->one_fma();     // the fused form reconstructs in three steps only
+      arcq_unpack_job jobs[2];
+      norm_quant(y, norms[2 * i], b.norm1.eps, qkv, 0);
+      gemm(xhat, *qkv, mid, jobs, jobs_of(qkv, done, 2, jobs));
+      {
+        const at::Tensor t = at::from_blob(mid, {B, T, 3, p->heads, D / p->heads}, at::TensorOptions().dtype(at::kHalf).device(dev));
+        const at::Tensor r = t.permute({2, 0, 3, 1, 4});
+        const at::Tensor o = at::scaled_dot_product_attention(r[0], r[1], r[2]).transpose(1, 2).reshape({M, D}).contiguous();
+        check(arcq_act_quant_unpack(0, half_matrix(o, M * D, dev), ARCQ_DT_F16, M, D, proj->th, proj->acb, proj->bits, 64, xhat,
+                                    ARCQ_DT_F16, proj->one_fma(), nullptr, 0, st),
+              "arcq_act_quant");
+      }
+      last_gemm(xhat, *proj, branch, fc1, fused);
+      norm_quant(branch, norms[2 * i + 1], b.norm2.eps, fc1, fused);
+      const int n = jobs_of(fc1, done, 2, jobs);
+      if (fused) {
+        check(arcq_dense_weight_gemm_gelu_quant(xhat, fc1->job.out, fc1->bias, M, fc1->N, fc1->K, fc2->th, fc2->acb, fc2->bits, 64, xhat4,
+                                                jobs, n, st),
+              "arcq_dense_weight_gemm_gelu_quant");
+      } else {
+        gemm(xhat, *fc1, mid, jobs, n);
+        check(arcq_act_quant_unpack(1, mid, ARCQ_DT_F16, M, fc2->K, fc2->th, fc2->acb, fc2->bits, 64, xhat4, ARCQ_DT_F16, fc2->one_fma(),
+                                    nullptr, 0, st),
+              "arcq_gelu_act_quant");
+      }
+      last_gemm(xhat4, *fc2, branch, i + 1 < depth ? qkv + 4 : nullptr, 0);
+      y = branch;
     }
-    last_gemm(xhat4, *fc2, branch, i + 1 < depth ? qkv + 4 : nullptr, 0);
-    y = branch;
-  }
-  // the head reads the class token of every image only
-  const at::Tensor h = empty_cuda({B, D}, at::kHalf, dev);
-  const NormView& nv = norms[2 * depth];
-  check(arcq_add_layernorm_strided(x, y, nv.gamma, nv.beta, nv.dtype, static_cast<float>(p->norm.eps), B, D, T * D, nullptr,
-                                   h.mutable_data_ptr(), st),
-        "arcq_add_layernorm");
-  return THPVariable_Wrap(at::linear(h, *hw, *hb));
+    // the head reads the class token of every image only
+    const at::Tensor h = empty_cuda({B, D}, at::kHalf, dev);
+    const NormView& nv = norms[2 * depth];
+    check(arcq_add_layernorm_strided(x, y, nv.gamma, nv.beta, nv.dtype, static_cast<float>(p->norm.eps), B, D, T * D, nullptr,
+                                     h.mutable_data_ptr(), st),
+          "arcq_add_layernorm");
+    return at::linear(h, *hw, *hb);
+  });
+  return THPVariable_Wrap(std::move(logits));
 }
 
 template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
@@ -509,8 +557,6 @@ PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {
   if (F != &vit_plan && c10::impl::TorchDispatchModeTLS::any_modes_set()) Py_RETURN_NONE;      // the mode wants to see the operators
   try {
     return F(self, args, n);
-  } catch (const Fail&) {
-    return nullptr;
   } catch (const c10::OutOfMemoryError& e) {
     PyErr_SetString(g_oom_error, e.what_without_backtrace());
     return nullptr;

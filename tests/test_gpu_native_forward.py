@@ -271,3 +271,42 @@ def test_modes_and_subclasses_see_what_the_python_forward_shows_them(pkg, cuda_d
     assert torch.equal(model(images.as_subclass(Image)).as_subclass(torch.Tensor), want)
     with torch.device(cuda_device):                            # a default device is no reason to leave the native forward
         assert torch.equal(model._forward_native(images), want)
+
+
+@torch.no_grad()
+def test_other_threads_run_while_a_native_call_waits_for_the_gpu(pkg, cuda_device):
+    """Calls pile up behind a busy GPU until the launch queue is full and the last one has to wait; another Python thread goes on
+    meanwhile."""
+    import threading
+    import time
+    model, images = _small_model(pkg, "deit_tiny", 4, cuda_device)
+    layer = model.blocks[0].mlp.fc1
+    rows = torch.randn(8, 192, device=cuda_device).half()
+    for call in (lambda: model(images), lambda: layer(rows)):
+        for _ in range(3):
+            call()
+        torch.cuda.synchronize()
+        gaps, stop = [], threading.Event()
+
+        def tick():
+            last = time.perf_counter()
+            while not stop.is_set():
+                time.sleep(0.001)
+                now = time.perf_counter()
+                gaps.append(now - last)
+                last = now
+
+        thread = threading.Thread(target=tick)
+        thread.start()
+        torch.cuda._sleep(1_500_000_000)                     # cycles: 0.8 s
+        start = time.perf_counter()
+        for _ in range(1500):
+            call()
+            if time.perf_counter() - start > 0.5:
+                break
+        waited = time.perf_counter() - start
+        stop.set()
+        thread.join()
+        torch.cuda.synchronize()
+        assert waited > 0.5 and max(gaps) < 0.25, (waited, max(gaps))
+    assert pkg.ops.device_status() == 0
