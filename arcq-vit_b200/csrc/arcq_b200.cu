@@ -820,7 +820,7 @@ static int act_quant_impl(int pre, const void* x, int x_dtype, int64_t M, int64_
     return fail(ARCQ_E_BAD_SHAPE, "K=%lld is not a multiple of group_size=%d", (long long)K, group_size);
   if (group_size != 64) return fail(ARCQ_E_UNSUPPORTED, "group_size %d: only 64 is built", group_size);
   if (packed_out != nullptr && !aligned(packed_out, 4)) return fail(ARCQ_E_ALIGN, "packed_out must be 4-byte aligned");
-  if (M == 0) return ARCQ_OK;
+  if (M == 0) return run_unpack_jobs(unpack, n_unpack, stream);
   arcq::UnpackJobs jobs;
   if (const int rc = make_unpack_jobs(unpack, n_unpack, &jobs)) return rc;
   const long long groups = static_cast<long long>(M) * (K / 64);
@@ -1327,7 +1327,7 @@ int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const void
   if (!aligned(x, 16) || !aligned(xhat, 16) || (y != nullptr && !aligned(y, 16)) ||
       (sum_out != nullptr && !aligned(sum_out, 16)) || (h_out != nullptr && !aligned(h_out, 16)) || !aligned(gamma, 16) || !aligned(beta, 16))
     return fail(ARCQ_E_ALIGN, "all matrices and the parameters must be 16-byte aligned");
-  if (M == 0) return ARCQ_OK;
+  if (M == 0) return run_unpack_jobs(unpack, n_unpack, stream);
   arcq::UnpackJobs jobs;
   if (const int rc = make_unpack_jobs(unpack, n_unpack, &jobs)) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);

@@ -143,7 +143,8 @@ int arcq_gelu_act_quant(const void* x, int x_dtype, int64_t M, int64_t K,
  * multiplies with: arcq_packed_weight_gemm's (what arcq_unpack_weight_f16 writes) where packed rows are a multiple of 16 bytes,
  * else arcq_packed_gemm's, fp16(fma(sigma, level, mu - sigma * codesum / 64)) in fp32 with one rounding.
  * The linear that consumes the quantizer's output needs its weight next: unpacked beside the quantizer it costs no
- * launch of its own.  Up to two jobs a call; `out` must not be read by any kernel still running before the call.
+ * launch of its own.  Up to two jobs a call, done also where M is 0; `out` must not be read by any kernel still
+ * running before the call.
  */
 typedef struct arcq_unpack_job {
   const uint8_t* packed;

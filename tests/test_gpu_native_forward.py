@@ -310,3 +310,34 @@ def test_other_threads_run_while_a_native_call_waits_for_the_gpu(pkg, cuda_devic
         torch.cuda.synchronize()
         assert waited > 0.5 and max(gaps) < 0.25, (waited, max(gaps))
     assert pkg.ops.device_status() == 0
+
+
+class _UnpackJob(ctypes.Structure):
+    _fields_ = ([(n, ctypes.c_void_p) for n in ("packed", "mu", "sigma", "codesum", "codebook", "out")]
+                + [("rows", ctypes.c_int64), ("K", ctypes.c_int64), ("bits", ctypes.c_int)])
+
+
+@pytest.mark.parametrize("bits", [4, 3, 2])
+@pytest.mark.parametrize("M", [0, 5])
+def test_unpack_jobs_of_every_entry_point_run_whatever_the_rows(pkg, cuda_device, bits, M):
+    lib, gen = pkg._cabi.load(), torch.Generator().manual_seed(bits)
+    K, N, st = 384, 64, torch.cuda.current_stream().cuda_stream
+    cb, th = _codebook(gen, bits, cuda_device)
+    packed, mu, sg, cs = pkg.ops.quantize_activation(torch.randn(N, K, generator=gen).to(cuda_device), th, cb, bits, 64)
+    want = pkg.ops.unpack_weight_f16(packed, mu, sg, cs, cb, bits, 64)
+    x, h = torch.randn(M + 1, K, generator=gen).half().to(cuda_device), torch.empty(M + 1, K, dtype=torch.float16, device=cuda_device)
+    one = torch.ones(K, device=cuda_device)
+
+    def run(call):
+        out = torch.zeros(N, K, dtype=torch.float16, device=cuda_device)
+        job = _UnpackJob(*(t.data_ptr() for t in (packed, mu, sg, cs, cb, out)), N, K, bits)
+        assert call(ctypes.addressof(job)) == 0
+        assert torch.equal(out, want)
+
+    p = [ctypes.c_void_p(t.data_ptr()) for t in (x, h, th, cb, one)]
+    i64, vp = ctypes.c_int64, ctypes.c_void_p
+    run(lambda j: lib.arcq_act_quant_unpack(0, p[0], 1, i64(M), i64(K), p[2], p[3], bits, 64, p[1], 1, 0, vp(j), 1, vp(st)))
+    run(lambda j: lib.arcq_add_layernorm_act_quant_unpack(x.data_ptr(), None, one.data_ptr(), one.data_ptr(), 0, 1e-6, M, K, th.data_ptr(),
+                                                          cb.data_ptr(), bits, 64, None, None, h.data_ptr(), 0, j, 1, st))
+    run(lambda j: lib.arcq_dense_weight_gemm_unpack(p[0], vp(want.data_ptr()), None, i64(M), i64(N), i64(K), p[1], 1, vp(j), 1, vp(st)))
+    assert pkg.ops.device_status() == 0
