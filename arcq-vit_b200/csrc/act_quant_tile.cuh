@@ -27,7 +27,7 @@ template <typename T, bool WRITE_PACKED> struct AqtShape {
   static constexpr int kBlocksPerSm = sizeof(T) == 4 ? 3 : 4;
 };
 
-// XH: element type of the reconstruction: T, or fp16 for an fp32 input.  PRE = 1: GELU first (fp16 input).
+// XH: element type of the reconstruction: T or fp16.  PRE = 1: GELU first (fp16 input).
 template <typename T, int BITS, typename XH, bool WRITE_XHAT, int PRE, bool WRITE_PACKED>
 __global__ void __launch_bounds__(AqtShape<T, WRITE_PACKED>::kThreads, AqtShape<T, WRITE_PACKED>::kBlocksPerSm)
     act_quant_tile_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_out,

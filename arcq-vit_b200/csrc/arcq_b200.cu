@@ -210,7 +210,7 @@ bool make_tensor_map_2d(CUtensorMap* tm, const void* base, CUtensorMapDataType d
 }
 
 // Tile form of the quantizer (a thread per group, tiles by TMA): taken when the buffers are aligned for 16-byte accesses and
-// the reconstruction, if asked for, has the input's element type or is the fp16 one of an fp32 input.
+// the reconstruction, if asked for, is fp16 or has the input's element type.
 template <typename T, int BITS, int PRE, typename XH, bool WX, bool WP>
 cudaError_t launch_act_quant_tile(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed,
                                   float* mu, float* sg, float* cs, void* xhat, cudaStream_t st, int one_fma,
@@ -266,7 +266,7 @@ template <typename T, int BITS, int PRE>
 cudaError_t dispatch_act_quant_tile(const void* x, long long groups, const float* th, const float* cb, uint8_t* packed, float* mu,
                                     float* sg, float* cs, void* xhat, bool xhat_f16, cudaStream_t st, int one_fma,
                                   const arcq::UnpackJobs& jobs) {
-  if constexpr (sizeof(T) == 4) {
+  if constexpr (!std::is_same<T, __half>::value) {
     if (xhat != nullptr && xhat_f16)
       return launch_act_quant_tile_outputs<T, BITS, PRE, __half>(x, groups, th, cb, packed, mu, sg, cs, xhat, st, one_fma, jobs);
   }
@@ -284,7 +284,7 @@ cudaError_t dispatch_act_quant_bits(int bits, const void* x, int x_dtype, long l
   const bool xhat_f16 = xhat != nullptr && xhat_dtype == ARCQ_DT_F16;
   const bool tile = groups >= min_groups && groups < (1ll << 30) && opt(O_ACT_QUANT_V1) == 0 && aligned(x, 16) &&
                     (packed == nullptr || aligned(packed, 16)) &&
-                    (xhat == nullptr || ((xhat_dtype == x_dtype || (x_dtype == ARCQ_DT_F32 && xhat_f16)) && aligned(xhat, 16)));
+                    (xhat == nullptr || ((xhat_dtype == x_dtype || xhat_f16) && aligned(xhat, 16)));
   if (tile) {
     switch (bits) {
       case 4: return dispatch_act_quant_tile<T, 4, PRE>(x, groups, th, cb, packed, mu, sg, cs, xhat, xhat_f16, st, one_fma, jobs);

@@ -420,6 +420,20 @@ def test_staged_quantizer_kernel_matches_oracle_and_the_parallel_kernel(pkg, ora
     assert pkg.ops.device_status() == 0
 
 
+@pytest.mark.parametrize("bits", [4, 3, 2])
+@pytest.mark.parametrize("M", [1579, 2049])                   # 37 896 groups, in a ragged last tile, and 49 176
+def test_half_reconstruction_of_a_bf16_input_by_tiles(pkg, cuda_device, bits, M):
+    gen = torch.Generator().manual_seed(bits)
+    x = (torch.randn(M, 1536, generator=gen) * 3).to(torch.bfloat16).to(cuda_device)
+    cb = torch.sort(torch.randn(2 ** bits, generator=gen) * 1.3)[0].to(cuda_device)
+    th = (cb[:-1] + cb[1:]) / 2
+    got = pkg.ops.quantize_activation_dequant(x, th, cb, bits, 64, torch.float16)
+    with pkg._cabi.option("ARCQ_ACT_QUANT_V1", 1):           # the small-input kernel
+        assert torch.equal(got, pkg.ops.quantize_activation_dequant(x, th, cb, bits, 64, torch.float16))
+    assert torch.equal(got, pkg.ops.quantize_activation_dequant(x.float(), th, cb, bits, 64, torch.float16))
+    assert pkg.ops.device_status() == 0
+
+
 def test_staged_quantizer_with_close_thresholds_falls_back_to_the_search(pkg, oracle, cuda_device):
     # two thresholds closer than a grid cell: the first-guess table is not valid, the search must be used
     cb = np.array([-2.5, -2.0, -1.5, -1.0, -0.6, -0.3, -0.1, 0.0, 0.004, 0.008, 0.3, 0.7, 1.1, 1.6, 2.1, 2.6], np.float32)
