@@ -540,29 +540,33 @@ struct PairDenseConfig {
   size_t smem;
 };
 
-int max_resident_dense_pairs(size_t smem) {
-  static thread_local int cached_dev = -1, cached = 0;
+// CTA pairs of a form of the kernel that are resident at once with all of the shared memory, kept per host thread and device.
+// The limit is raised before the question, whichever entry point asks first; a question that fails is not remembered.
+struct ResidentPairs {
+  int dev = -1, n = 0;
+};
+template <typename Kernel> int max_resident_dense_pairs(Kernel kernel, int threads, ResidentPairs* known) {
+  const size_t smem = kSmemBudget + 1024;
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev == cached_dev && cached > 0) return cached;
+  if (dev == known->dev) return known->n;
   int n = 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(sm_count() / 2 * 2));
-  cfg.blockDim = dim3(arcq::kPairDenseThreads);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, arcq::dense_weight_gemm_pair_kernel<true>, &cfg);
-  if (e != cudaSuccess || n <= 0) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
     cudaGetLastError();
-    n = sm_count() / 2;
+    return sm_count() / 2;
   }
   if (n > sm_count() / 2) n = sm_count() / 2;
-  cached = n;
-  cached_dev = dev;
+  *known = {dev, n};
   return n;
 }
 
@@ -592,7 +596,8 @@ bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32,
       done_dev = dev;
     }
   }
-  int max_pairs = max_resident_dense_pairs(full_smem);
+  static thread_local ResidentPairs known;
+  int max_pairs = max_resident_dense_pairs(arcq::dense_weight_gemm_pair_kernel<true>, arcq::kPairDenseThreads, &known);
   if (opt(O_PAIR_PAIRS) > 0 && opt(O_PAIR_PAIRS) < max_pairs) max_pairs = opt(O_PAIR_PAIRS);
   static const int cand[] = {256, 192, 160, 128, 96, 64, 32};
   double best_cost = 0;
@@ -656,7 +661,8 @@ bool choose_pair_quant_config(long long M, long long N, long long K, PairDenseCo
   if (opt(O_PAIR) == 0) return false;
   const int G = static_cast<int>(K / 64);
   const long long tiles_m = (M + arcq::kPairTileM - 1) / arcq::kPairTileM;
-  int max_pairs = max_resident_dense_pairs(kSmemBudget + 1024);
+  static thread_local ResidentPairs known;
+  int max_pairs = max_resident_dense_pairs(arcq::dense_weight_gemm_pair_kernel<true, false, 4>, arcq::kPairQuantThreads, &known);
   if (opt(O_PAIR_PAIRS) > 0 && opt(O_PAIR_PAIRS) < max_pairs) max_pairs = opt(O_PAIR_PAIRS);
   static const int cand[] = {192, 128, 64};                  // whole groups, at most one per epilogue warp of a lane quarter
   double best_cost = 0;

@@ -1,8 +1,12 @@
 """What only the native host path uses, against the separate operators and the Python code it stands for: same bits."""
 import ctypes
+import subprocess
+import sys
 
 import pytest
 import torch
+
+from conftest import ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -341,3 +345,14 @@ def test_unpack_jobs_of_every_entry_point_run_whatever_the_rows(pkg, cuda_device
                                                           cb.data_ptr(), bits, 64, None, None, h.data_ptr(), 0, j, 1, st))
     run(lambda j: lib.arcq_dense_weight_gemm_unpack(p[0], vp(want.data_ptr()), None, i64(M), i64(N), i64(K), p[1], 1, vp(j), 1, vp(st)))
     assert pkg.ops.device_status() == 0
+
+
+def test_gemm_layout_does_not_depend_on_the_first_question(pkg, cuda_device):
+    """In a fresh process, whichever of the two forms of the pair GEMM is asked about first: the same room beside both."""
+    code = ("import sys, ctypes; sys.path.insert(0, '.'); import __graft_entry__ as e, torch; torch.zeros(1, device='cuda')\n"
+            "l = e.import_package()._cabi.load(); f = l.arcq_dense_weight_gemm_unpack_room; f.restype = ctypes.c_int64\n"
+            "i = ctypes.c_int64\n"
+            "print([f(i(m), i(n), i(k), q) for q in (%s) for m, n, k in ((12608, 1152, 384), (3000, 768, 3072), (12608, 3072, 768))])")
+    rooms = [eval(subprocess.run([sys.executable, "-c", code % order], cwd=ROOT, capture_output=True, text=True, check=True).stdout)
+             for order in ("0, 1", "1, 0")]
+    assert rooms[0] == rooms[1][3:] + rooms[1][:3]
