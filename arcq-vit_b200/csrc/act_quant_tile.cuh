@@ -159,6 +159,7 @@ __global__ void __launch_bounds__(AqtShape<T, WRITE_PACKED>::kThreads, AqtShape<
         tma_store_commit();
       }
     } else {
+      if (PRE == 1) fence_proxy_async_smem();                 // the GELU may have written to it
       __syncwarp();                                           // every lane has read its row before the buffer is refilled
     }
     if (next_buf == 0) ph ^= 1;
