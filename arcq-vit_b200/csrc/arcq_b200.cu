@@ -79,7 +79,7 @@ int sm_count() {
 // library is first used, or arcq_debug_set_option() at any time, overrides it.  Normal use sets none of them.
 enum Opt {
   O_WS_BN, O_WS_SA, O_WS_WS, O_WS_STATIONARY, O_WS_NBB, O_WS_GRID, O_WS_TMA_STORE, O_WS_ROTATE,
-  O_ACT_QUANT_V1, O_ACT_QUANT_V2, O_LN_PLAIN,
+  O_ACT_QUANT_V1, O_LN_PLAIN,
   O_PAIR, O_PAIR_MIN_M, O_PAIR_BN, O_PAIR_SA, O_PAIR_KS, O_PAIR_NBB, O_PAIR_LUT, O_PAIR_PAIRS, O_PAIR_STATIONARY,
   O_PAIR_WS, O_LNQ_SMALL, O_AQ2_MIN_GROUPS, O_PDL, O_GELU_GEMM, O_GEMM_UNPACK, O_POLL_LIMIT, O_SPIN_LIMIT, O_COUNT
 };
@@ -87,7 +87,7 @@ struct OptDef { const char* name; int dflt; };
 const OptDef kOptDefs[O_COUNT] = {
     {"ARCQ_WS_BN", 0},        {"ARCQ_WS_SA", 0},          {"ARCQ_WS_WS", 0},       {"ARCQ_WS_STATIONARY", -1},
     {"ARCQ_WS_NBB", 0},       {"ARCQ_WS_GRID", 0},        {"ARCQ_WS_TMA_STORE", 1}, {"ARCQ_WS_ROTATE", 1},
-    {"ARCQ_ACT_QUANT_V1", 0}, {"ARCQ_ACT_QUANT_V2", 0},   {"ARCQ_LN_PLAIN", 0},
+    {"ARCQ_ACT_QUANT_V1", 0}, {"ARCQ_LN_PLAIN", 0},
     {"ARCQ_PAIR", 1},         {"ARCQ_PAIR_MIN_M", 1024},  {"ARCQ_PAIR_BN", 0},     {"ARCQ_PAIR_SA", 0},
     {"ARCQ_PAIR_KS", 0},      {"ARCQ_PAIR_NBB", 0},       {"ARCQ_PAIR_LUT", 0},    {"ARCQ_PAIR_PAIRS", 0},
     {"ARCQ_PAIR_STATIONARY", -1}, {"ARCQ_PAIR_WS", 0}, {"ARCQ_LNQ_SMALL", 1}, {"ARCQ_AQ2_MIN_GROUPS", 0}, {"ARCQ_PDL", 1},
@@ -278,7 +278,7 @@ cudaError_t dispatch_act_quant_bits(int bits, const void* x, int x_dtype, long l
                                     const float* cb, uint8_t* packed, float* mu, float* sg, float* cs, void* xhat,
                                     int xhat_dtype, cudaStream_t st, int one_fma,
                                   const arcq::UnpackJobs& jobs) {
-  // The one-thread-per-group kernel needs enough groups to fill the machine (148 SMs x 4 blocks x 128
+  // The one-thread-per-group kernel needs enough groups to half fill the machine (256 per SM of 4 blocks x 128
   // threads); below that the 8-lanes-per-group kernel has 8 times the parallelism and lower latency.
   const long long min_groups = opt(O_AQ2_MIN_GROUPS) > 0 ? opt(O_AQ2_MIN_GROUPS) : static_cast<long long>(sm_count()) * 256;
   const bool xhat_f16 = xhat != nullptr && xhat_dtype == ARCQ_DT_F16;
