@@ -68,6 +68,7 @@ def load() -> ctypes.CDLL:
     lib.arcq_dequant.argtypes = [vp, vp, vp, vp, vp, ci, ci, i64, i64, vp, ci, vp]
     lib.arcq_unpack_weight_f16.argtypes = [vp, vp, vp, vp, vp, ci, ci, i64, i64, vp, vp]
     lib.arcq_dense_weight_gemm_prefetch.argtypes = [vp, vp, vp, i64, i64, i64, vp, ci, vp, vp, vp, vp, vp, ci, ci, i64, i64, vp, vp]
+    lib.arcq_dense_weight_gemm_gelu_quant_applies.argtypes = [i64, i64, i64]
     lib.arcq_dense_weight_gemm_gelu_quant.argtypes = [vp, vp, vp, i64, i64, i64, vp, vp, ci, ci, vp, vp, ci, vp]
     for name in EXPORTS:
         getattr(lib, name)  # AttributeError here means header and library disagree
