@@ -16,7 +16,7 @@ DT_F32, DT_F16, DT_BF16 = 0, 1, 2
 
 # every symbol include/arcq_b200.h declares
 EXPORTS = (
-    "arcq_version", "arcq_last_error_string", "arcq_device_status", "arcq_debug_trace", "arcq_debug_set_option", "arcq_debug_get_option", "arcq_debug_last_gemm_kernel", "arcq_debug_wait_timeout", "arcq_act_quant", "arcq_gelu_act_quant", "arcq_packed_gemm", "arcq_packed_weight_gemm", "arcq_dense_weight_gemm", "arcq_packed_linear_static_scratch", "arcq_add_layernorm", "arcq_add_layernorm_act_quant", "arcq_attention", "arcq_attention_act_quant", "arcq_patchify", "arcq_assemble_tokens",
+    "arcq_version", "arcq_last_error_string", "arcq_device_status", "arcq_debug_trace", "arcq_debug_set_option", "arcq_debug_get_option", "arcq_debug_last_gemm_kernel", "arcq_debug_wait_timeout", "arcq_act_quant", "arcq_gelu_act_quant", "arcq_packed_gemm", "arcq_packed_weight_gemm", "arcq_dense_weight_gemm", "arcq_packed_linear_static_scratch", "arcq_add_layernorm", "arcq_add_layernorm_act_quant", "arcq_attention", "arcq_attention_act_quant", "arcq_attention_act_quant_form", "arcq_patchify", "arcq_assemble_tokens",
     "arcq_unpack_codes", "arcq_pack_codes", "arcq_dequant", "arcq_unpack_weight_f16", "arcq_dense_weight_gemm_prefetch",
     "arcq_act_quant_unpack", "arcq_add_layernorm_act_quant_unpack", "arcq_add_layernorm_strided",
     "arcq_dense_weight_gemm_unpack", "arcq_dense_weight_gemm_unpack_room", "arcq_unpack_beside_gemm", "arcq_dense_weight_gemm_gelu_quant",
@@ -61,6 +61,7 @@ def load() -> ctypes.CDLL:
     lib.arcq_add_layernorm_act_quant.argtypes = [vp, vp, vp, vp, ctypes.c_float, i64, i64, vp, vp, ci, ci, vp, vp, vp, vp]
     lib.arcq_attention.argtypes = [vp, i64, i64, i64, ci, vp, vp]
     lib.arcq_attention_act_quant.argtypes = [vp, i64, i64, i64, ci, vp, vp, ci, ci, vp, vp]
+    lib.arcq_attention_act_quant_form.argtypes = [vp, i64, i64, i64, ci, vp, vp, ci, ci, vp, ci, vp]
     lib.arcq_patchify.argtypes = [vp, i64, i64, i64, i64, ci, vp, vp]
     lib.arcq_assemble_tokens.argtypes = [vp, vp, vp, i64, i64, i64, vp, vp]
     lib.arcq_unpack_codes.argtypes = [vp, i64, i64, ci, vp, vp]

@@ -168,26 +168,26 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-// 2-D row-major tensor [rows, cols] of `elem_bytes`-byte elements, box [box_cols x box_rows].  A descriptor
-// depends only on these values (not on what the memory holds), so the last few are kept per host thread:
-// a model's layers present the same (pointer, shape) again on every forward.
+// Row-major tensor [rows, cols] of `elem_bytes`-byte elements, or `planes` of them one after the other (0: a matrix), box
+// [box_cols x box_rows].  A descriptor depends only on these values (not on what the memory holds), so the last few are kept
+// per host thread: a model's layers present the same (pointer, shape) again on every forward.
 struct TensorMapKey {
   const void* base;
-  uint64_t rows, cols;
+  uint64_t planes, rows, cols;
   uint32_t box_cols, box_rows;
   int dt, swz;
   bool operator==(const TensorMapKey& o) const {
-    return base == o.base && rows == o.rows && cols == o.cols && box_cols == o.box_cols && box_rows == o.box_rows &&
-           dt == o.dt && swz == o.swz;
+    return base == o.base && planes == o.planes && rows == o.rows && cols == o.cols && box_cols == o.box_cols &&
+           box_rows == o.box_rows && dt == o.dt && swz == o.swz;
   }
 };
-bool make_tensor_map_2d(CUtensorMap* tm, const void* base, CUtensorMapDataType dt, int elem_bytes, uint64_t rows,
-                        uint64_t cols, uint32_t box_cols, uint32_t box_rows, CUtensorMapSwizzle swz) {
+bool make_tensor_map(CUtensorMap* tm, const void* base, CUtensorMapDataType dt, int elem_bytes, uint64_t planes, uint64_t rows,
+                     uint64_t cols, uint32_t box_cols, uint32_t box_rows, CUtensorMapSwizzle swz) {
   constexpr int kSlots = 256;
   struct Slot { TensorMapKey key; CUtensorMap map; bool used; };
   static thread_local Slot cache[kSlots] = {};
-  const TensorMapKey key{base, rows, cols, box_cols, box_rows, static_cast<int>(dt), static_cast<int>(swz)};
-  uint64_t h = reinterpret_cast<uintptr_t>(base) >> 4;
+  const TensorMapKey key{base, planes, rows, cols, box_cols, box_rows, static_cast<int>(dt), static_cast<int>(swz)};
+  uint64_t h = (reinterpret_cast<uintptr_t>(base) >> 4) ^ (planes << 50);
   h = (h ^ (rows * 0x9E3779B97F4A7C15ull) ^ (cols << 7) ^ (static_cast<uint64_t>(box_rows) << 29) ^ (static_cast<uint64_t>(box_cols) << 41)) * 0xD6E8FEB86659FD93ull;
   Slot& slot = cache[(h >> 40) % kSlots];
   if (slot.used && slot.key == key) {
@@ -196,17 +196,22 @@ bool make_tensor_map_2d(CUtensorMap* tm, const void* base, CUtensorMapDataType d
   }
   PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
   if (enc == nullptr) return false;
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {cols * static_cast<uint64_t>(elem_bytes)};
-  cuuint32_t box[2] = {box_cols, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  if (enc(tm, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
+  const cuuint64_t row_bytes = cols * static_cast<uint64_t>(elem_bytes);
+  cuuint64_t dims[3] = {cols, rows, planes};
+  cuuint64_t strides[2] = {row_bytes, rows * row_bytes};
+  cuuint32_t box[3] = {box_cols, box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  if (enc(tm, dt, planes > 0 ? 3 : 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return false;
   slot.key = key;
   slot.map = *tm;
   slot.used = true;
   return true;
+}
+bool make_tensor_map_2d(CUtensorMap* tm, const void* base, CUtensorMapDataType dt, int elem_bytes, uint64_t rows,
+                        uint64_t cols, uint32_t box_cols, uint32_t box_rows, CUtensorMapSwizzle swz) {
+  return make_tensor_map(tm, base, dt, elem_bytes, 0, rows, cols, box_cols, box_rows, swz);
 }
 
 // Tile form of the quantizer (a thread per group, tiles by TMA): taken when the buffers are aligned for 16-byte accesses and
@@ -1405,23 +1410,34 @@ int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const void
 }
 
 static int launch_attention(const void* qkv, int64_t B, int64_t T, int64_t H, int head_dim, const float* thresholds,
-                            const float* codebook, int bits, void* out, void* stream) {
+                            const float* codebook, int bits, int one_fma, void* out, void* stream) {
   if (qkv == nullptr || out == nullptr) return fail(ARCQ_E_BAD_ARG, "null pointer argument");
   if (head_dim != 64) return fail(ARCQ_E_UNSUPPORTED, "head_dim %d: only 64 is built", head_dim);
   if (B < 0 || T <= 0 || H <= 0) return fail(ARCQ_E_BAD_SHAPE, "bad shape B=%lld T=%lld H=%lld", (long long)B, (long long)T, (long long)H);
   if (T > arcq::kAttnMaxT) return fail(ARCQ_E_TOO_LARGE, "sequences longer than %d tokens are not built", arcq::kAttnMaxT);
-  if (B * H > 0x7fffffffLL) return fail(ARCQ_E_TOO_LARGE, "too many (image, head) pairs");
+  // (a matrix of 2^30 heads would be 400 GB)
+  if (B > 0x3fffffffLL || H > 0x7fffffLL || B * H > 0x3fffffffLL) return fail(ARCQ_E_TOO_LARGE, "too many (image, head) pairs");
   if (!aligned(qkv, 16) || !aligned(out, 16)) return fail(ARCQ_E_ALIGN, "qkv and out must be 16-byte aligned");
   if (B == 0) return ARCQ_OK;
   arcq::AttnParams p;
-  p.qkv = static_cast<const __half*>(qkv);
-  p.out = static_cast<__half*>(out);
-  p.B = static_cast<int>(B); p.T = static_cast<int>(T); p.H = static_cast<int>(H);
-  p.tp = static_cast<int>((T + 15) / 16 * 16);
+  p.T = static_cast<int>(T); p.H = static_cast<int>(H);
+  p.tk = static_cast<int>((T + 15) / 16 * 16);
+  p.qtiles = static_cast<int>((T + arcq::kAttnQueries - 1) / arcq::kAttnQueries);
+  p.items = static_cast<int>(B * H * p.qtiles);
   p.thresholds = thresholds;
   p.codebook = codebook;
-  const size_t smem = arcq::attn_smem_bytes(p.tp);
-  const unsigned grid = static_cast<unsigned>(B * H);
+  p.one_fma = one_fma;
+  p.status = status_ptr();
+  CUtensorMap tm_q, tm_kv, tm_out;
+  auto map = [&](CUtensorMap* tm, const void* base, int64_t cols, int box_rows) {
+    return make_tensor_map(tm, base, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, static_cast<uint64_t>(B), static_cast<uint64_t>(T),
+                           static_cast<uint64_t>(cols), 64, static_cast<uint32_t>(box_rows), CU_TENSOR_MAP_SWIZZLE_128B);
+  };
+  if (!map(&tm_q, qkv, 3 * H * 64, arcq::kAttnQueries) || !map(&tm_kv, qkv, 3 * H * 64, p.tk) || !map(&tm_out, out, H * 64, 32))
+    return fail(ARCQ_E_CUDA, "cuTensorMapEncodeTiled failed");
+  const size_t smem = arcq::attn_smem_layout(p.tk).total;
+  const int cap = 2 * sm_count();
+  const unsigned grid = static_cast<unsigned>(p.items < cap ? p.items : cap);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 #define ARCQ_LAUNCH_ATTN(Q, BT)                                                                                      \
   do {                                                                                                                \
@@ -1429,11 +1445,12 @@ static int launch_attention(const void* qkv, int64_t B, int64_t T, int64_t H, in
     int dev = 0;                                                                                                      \
     cudaGetDevice(&dev);                                                                                              \
     if (done_dev != dev) {                                                                                            \
-      cudaFuncSetAttribute(arcq::attention_kernel<Q, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize,                \
-                           static_cast<int>(arcq::attn_smem_bytes(arcq::kAttnMaxT)));                                 \
+      const cudaError_t se = cudaFuncSetAttribute(arcq::attention_kernel<Q, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                                  static_cast<int>(arcq::attn_smem_layout(arcq::kAttnMaxT).total));   \
+      if (se != cudaSuccess) return cuda_fail(se, "attention shared memory");                                         \
       done_dev = dev;                                                                                                 \
     }                                                                                                                 \
-    launch_pdl(arcq::attention_kernel<Q, BT>, grid, arcq::kAttnThreads, smem, st, p);                                 \
+    launch_pdl(arcq::attention_kernel<Q, BT>, grid, arcq::kAttnThreads, smem, st, tm_q, tm_kv, tm_out, p);            \
   } while (0)
   if (thresholds == nullptr) ARCQ_LAUNCH_ATTN(false, 4);
   else if (bits == 4) ARCQ_LAUNCH_ATTN(true, 4);
@@ -1446,15 +1463,20 @@ static int launch_attention(const void* qkv, int64_t B, int64_t T, int64_t H, in
 }
 
 int arcq_attention(const void* qkv, int64_t B, int64_t T, int64_t H, int head_dim, void* out, void* stream) {
-  return launch_attention(qkv, B, T, H, head_dim, nullptr, nullptr, 4, out, stream);
+  return launch_attention(qkv, B, T, H, head_dim, nullptr, nullptr, 4, 0, out, stream);
+}
+
+int arcq_attention_act_quant_form(const void* qkv, int64_t B, int64_t T, int64_t H, int head_dim, const float* thresholds,
+                                  const float* codebook, int bits, int group_size, void* xhat, int one_fma, void* stream) {
+  if (thresholds == nullptr || codebook == nullptr) return fail(ARCQ_E_BAD_ARG, "null pointer argument");
+  if (bits < 2 || bits > 4) return fail(ARCQ_E_BAD_ARG, "bits must be 2, 3 or 4, got %d", bits);
+  if (group_size != 64) return fail(ARCQ_E_UNSUPPORTED, "group_size %d: only 64 is built", group_size);
+  return launch_attention(qkv, B, T, H, head_dim, thresholds, codebook, bits, one_fma, xhat, stream);
 }
 
 int arcq_attention_act_quant(const void* qkv, int64_t B, int64_t T, int64_t H, int head_dim, const float* thresholds,
                              const float* codebook, int bits, int group_size, void* xhat, void* stream) {
-  if (thresholds == nullptr || codebook == nullptr) return fail(ARCQ_E_BAD_ARG, "null pointer argument");
-  if (bits < 2 || bits > 4) return fail(ARCQ_E_BAD_ARG, "bits must be 2, 3 or 4, got %d", bits);
-  if (group_size != 64) return fail(ARCQ_E_UNSUPPORTED, "group_size %d: only 64 is built", group_size);
-  return launch_attention(qkv, B, T, H, head_dim, thresholds, codebook, bits, xhat, stream);
+  return arcq_attention_act_quant_form(qkv, B, T, H, head_dim, thresholds, codebook, bits, group_size, xhat, 0, stream);
 }
 
 int arcq_patchify(const void* images, int64_t B, int64_t C, int64_t H, int64_t W, int patch, void* rows, void* stream) {

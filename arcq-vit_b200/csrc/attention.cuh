@@ -1,331 +1,406 @@
-// Multi-head self-attention for short sequences (ViT: 197 tokens, head width 64), optionally fused with the
-// activation quantizer of the projection that consumes its output.
+// Multi-head self-attention for short sequences (ViT: 197 tokens, head width 64) on the fifth-generation tensor cores,
+// optionally with the activation quantizer of the projection that consumes its output.
 //   qkv  [B*T, 3*H*64] fp16: the output of the packed qkv linear (q | k | v, each H heads of 64)
 //   out  [B*T, H*64] fp16:   softmax(q k^T / 8) v, heads side by side (the layout timm's Attention feeds to proj)
 //   or   xhat [B*T, H*64] fp16: the ARCQ reconstruction of that matrix in groups of 64.  A head's 64 outputs of a
-//        token are exactly one quantizer group, so the quantizer needs nothing beyond the registers that hold them.
+//        token are exactly one quantizer group, and one thread holds them.
 //
-// One CTA per (image, head), seven warps.  K and V of the head (T x 64 each) are staged once in shared memory
-// (16-byte cp.async, XOR-swizzled rows so that ldmatrix is conflict-free); each warp owns 16-row blocks of queries
-// and walks the keys in blocks of 64 with an online softmax: S = Q K^T on mma.sync.m16n8k16 (fp32 accumulate), row
-// maxima and sums in fp32, P rounded to fp16 and fed straight from the accumulator registers into the second
-// product O += P V -- the sequence never leaves registers.  The whole problem is 2 x 197 x 197 x 64 flops per head:
-// too small for a 128-row tensor-memory tile to pay (two thirds of a second tile would be padding), and the kernel is
-// bound by its latency chain, not by the tensor pipe.
+// A work item is 128 queries of one (image, head); a block walks consecutive items, so that the second tile of a head finds
+// its keys and values in shared memory.  The whole score row of a query (T <= 256 keys) fits tensor memory, so there is no
+// online softmax and no rescaling: per item
+//   S = Q K^T       128 x tk fp32 in tensor memory (tk: T rounded up to 16; the TMA fills the rows beyond T with zeros)
+//   P = exp2(...)   a thread owns a query row: maximum, exponentials, sum; P as fp16 over the columns of S already read
+//   O = P V         P from tensor memory, V from shared memory as it lies (keys outside, no transposition)
+//   out             O / sum rounded to fp16, the quantizer of group_quant.cuh, 32 rows per warp to a TMA store
+// Warps: 0-3 softmax and 4-7 output and quantizer (one tensor-memory lane quarter each), 8 TMA loads, 9 products.  Two blocks an
+// SM, 256 tensor-memory columns each.  The next item's scores are computed, and its softmax runs, while this one's rows are
+// quantised; the product with the upper half of the keys runs while the lower half's exponentials are computed.
 //
-// Quantizer epilogue: same arithmetic as the quantizer kernels (group_quant.cuh), on the fp16-rounded outputs, so
-// the result is bit-identical to quantising the matrix the plain form of this kernel writes.  A row's 64 values
-// sit in four lanes (lane%4 = q holds columns 8n+2q, 8n+2q+1, n = 0..7): the reference's lane sums
-//   v[l] = ((x[l]+x[32+l]) + (x[8+l]+x[40+l])) + (x[16+l]+x[48+l])) + (x[24+l]+x[56+l])   for l = 2q, 2q+1
-// are thread-local, and the closing chain ((((((v0+v1)+v2)+v3)+v4)+v5)+v6)+v7 is evaluated by every lane on the
-// eight values gathered with shuffles.
+// Tensor memory is allocated after the previous kernel has ended and before the next one may start: a GEMM that holds all of
+// it while it waits for this kernel's result can then never be in the way.
 #pragma once
+#include <cuda.h>
 #include <cuda_fp16.h>
 #include "ptx.cuh"
+#include "gemm_pair.cuh"
 #include "act_quant.cuh"
+#include "group_quant.cuh"
 
 namespace arcq {
 
-constexpr int kAttnWarps = 7;
-constexpr int kAttnThreads = kAttnWarps * 32;
+constexpr int kStatusAttentionTimeout = 0x501;
+constexpr int kAttnRowWarps = 4;                  // softmax warps, and as many output warps
+constexpr int kAttnThreads = 3 * 128;             // the third warp group: TMA and products
+// Registers a thread, moved between the warp groups once they are running; the sum is that of the launch (80 each)
+constexpr int kAttnLaunchRegs = 80, kAttnSoftmaxRegs = 88, kAttnOutputRegs = 120, kAttnIssueRegs = 32;
+static_assert(kAttnSoftmaxRegs + kAttnOutputRegs + kAttnIssueRegs <= 3 * kAttnLaunchRegs, "registers beyond the launch's never come");
 constexpr int kAttnMaxT = 256;
+constexpr int kAttnQueries = 128;                 // per work item
+// Tensor memory of an item: S in columns 0 .. tk-1.  P takes the first half of the columns of the part of S that it was made
+// from: keys below attn_split(tk) at column 0, the others from column attn_split(tk) on.  O at 192, where S and P have ended
+// once the upper part has been read.
+constexpr uint32_t kAttnTmemCols = 256, kAttnOutCol = 192;
+__host__ __device__ constexpr int attn_split(int tk) { return (tk / 2 + 15) / 16 * 16; }
 
 struct AttnParams {
-  const __half* qkv;
-  __half* out;
-  int B, T, H;
-  int tp;                      // T rounded up to 16: rows of K / V held in shared memory
+  int T, H;
+  int tk;                      // T rounded up to 16: keys of the products
+  int qtiles;                  // work items of a head
+  int items;                   // of all heads of all images
   const float* thresholds;     // quantizer form only
   const float* codebook;
+  int one_fma;
+  int* status;
 };
 
-__host__ __device__ constexpr size_t attn_smem_bytes(int tp) {
-  return static_cast<size_t>(2) * tp * 128 + kAttnWarps * 2048 + 3 * 16 * 4;
-}
-
-__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-// D (16x8, fp32) += A (16x16, fp16, row) . B (16x8, fp16, col)
-__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t pack_half2(float a, float b) {
-  const __half2 h = __floats2half2_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-// The reference's closing chain over the eight lane sums of a row; lane q of the row's four lanes holds
-// (v_even, v_odd) = (v[2q], v[2q+1]).  Every lane returns the same value.
-__device__ __forceinline__ float row_chain_sum(float v_even, float v_odd, int lane) {
-  const int base = lane & ~3;
-  float s = 0.0f;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float e = __shfl_sync(0xffffffffu, v_even, base + j);
-    const float o = __shfl_sync(0xffffffffu, v_odd, base + j);
-    s = (j == 0) ? __fadd_rn(e, o) : __fadd_rn(__fadd_rn(s, e), o);
-  }
+struct AttnSmem {
+  uint32_t q, k, v, stage, tables, sums, bars, total;
+};
+__host__ __device__ inline AttnSmem attn_smem_layout(int tk) {
+  AttnSmem s;
+  s.q = 0;
+  s.k = s.q + kAttnQueries * 128;
+  s.v = s.k + static_cast<uint32_t>(tk) * 128;              // tk * 128 is a multiple of 2 KB
+  s.stage = s.v + static_cast<uint32_t>(tk) * 128;
+  s.tables = s.stage + kAttnRowWarps * 4096;
+  s.sums = s.tables + (static_cast<uint32_t>(sizeof(GroupQuantTables)) + 15) / 16 * 16;
+  s.bars = s.sums + kAttnQueries * 4;
+  s.total = s.bars + 16 * 8 + 16 + 1024 /* alignment */;
   return s;
 }
-// lane sums v[2q], v[2q+1] of one row from its 16 thread-local values x[2n], x[2n+1] = columns 8n+2q, 8n+2q+1
-__device__ __forceinline__ void lane_sums(const float (&x)[16], float& v_even, float& v_odd) {
-  // l = 2q:   a0 = x[l] + x[32+l] -> n = 0, 4;  a1 -> n = 1, 5;  a2 -> n = 2, 6;  a3 -> n = 3, 7
-  v_even = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(x[0], x[8]), __fadd_rn(x[2], x[10])), __fadd_rn(x[4], x[12])), __fadd_rn(x[6], x[14]));
-  v_odd = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(x[1], x[9]), __fadd_rn(x[3], x[11])), __fadd_rn(x[5], x[13])), __fadd_rn(x[7], x[15]));
+
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, uint64_t* bar, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+__device__ __forceinline__ void tma_store_3d(const void* tmap, const void* smem_src, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(tmap)),
+               "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
+// D[tmem] (+)= A[tmem, fp16 pairs] * B[smem]; issued by one thread
+__device__ __forceinline__ void umma_f16_tmem_a(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ float exp2_approx(float x) {
+  float d;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(d) : "f"(x));
+  return d;
 }
 
 template <bool QUANT, int BITS>
-__global__ void __launch_bounds__(kAttnThreads, 2) attention_kernel(const AttnParams p) {
-  pdl_launch_dependents();
-  constexpr int L = 1 << BITS;
-  extern __shared__ __align__(128) uint8_t attn_smem[];
-  const int tp = p.tp, T = p.T, C = p.H * 64;
-  uint8_t* const sK = attn_smem;
-  uint8_t* const sV = sK + tp * 128;
-  uint8_t* const sStage = sV + tp * 128;
-  float* const s_th = reinterpret_cast<float*>(sStage + kAttnWarps * 2048);   // [16] thresholds, +inf padded
-  float* const s_h = s_th + 16;                                               // [16] half-gaps to the next float
-  float* const s_cb = s_h + 16;                                               // [16] codebook
+__global__ void __launch_bounds__(kAttnThreads, 2)
+    attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
+                     const __grid_constant__ CUtensorMap tm_out, const AttnParams p) {
+  extern __shared__ uint8_t attn_smem_raw[];
+  uint8_t* const smem = attn_smem_raw + ((1024u - (smem_u32(attn_smem_raw) & 1023u)) & 1023u);
+  const AttnSmem L = attn_smem_layout(p.tk);
+  uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + L.bars);
+  uint64_t *const q_full = bars, *const q_free = bars + 1, *const k_full = bars + 2, *const k_free = bars + 3,
+           *const v_full = bars + 4, *const v_free = bars + 5, *const s_full = bars + 6, *const o_full = bars + 7,
+           *const p_upper = bars + 8, *const p_lower = bars + 9, *const o_read = bars + 10;
+  uint32_t* const s_tmem = reinterpret_cast<uint32_t*>(bars + 16);
+  float* const s_sums = reinterpret_cast<float*>(smem + L.sums);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int b = blockIdx.x / p.H, h = blockIdx.x - b * p.H;
-  const __half* const base = p.qkv + static_cast<long long>(b) * T * (3 * C) + h * 64;
+  const int T = p.T, C = p.H * 64;
+  const int grid = static_cast<int>(gridDim.x), block = static_cast<int>(blockIdx.x);
+  const int first = static_cast<int>(1ll * p.items * block / grid), last = static_cast<int>(1ll * p.items * (block + 1) / grid);
+  // head of an item (image, first column), first query
+  auto place = [&](int it, int* b, int* x) {
+    const int head = it / p.qtiles;
+    *b = head / p.H;
+    *x = (head - *b * p.H) * 64;
+    return (it - head * p.qtiles) * kAttnQueries;
+  };
 
-  int my_exact = 1;
-  if (QUANT) {
-    if (tid < 16) {
-      float th = __int_as_float(0x7f800000), hg = 0.0f;
-      if (tid < L - 1) {
-        th = p.thresholds[tid];
-        if (th == 0.0f) {
-          hg = 0x1p-100f;
-        } else {
-          const int bi = __float_as_int(th);
-          const float up = __int_as_float(th > 0.0f ? bi + 1 : bi - 1);
-          hg = __fmul_rn(__fsub_rn(up, th), 0.5f);
-        }
-        my_exact = (th == 0.0f || fabsf(th) > 1.0e-15f) ? 1 : 0;
-      }
-      s_th[tid] = th;
-      s_h[tid] = hg;
-      s_cb[tid] = tid < L ? p.codebook[tid] : 0.0f;
-    }
+  if (tid == 0) {
+    for (int i = 0; i < 8; ++i) mbar_init(bars + i, 1);
+    for (int i = 8; i < 11; ++i) mbar_init(bars + i, kAttnRowWarps);
+    mbar_fence_init();
   }
-
-  pdl_wait();                // qkv is the previous kernel's output
-  // ---- K and V of this head into shared memory: row r at r*128, 16-byte chunk c at ((c ^ (r & 7)) * 16)
-  {
-    const uint32_t k0 = smem_u32(sK), v0 = smem_u32(sV);
-    for (int i = tid; i < tp * 8; i += kAttnThreads) {
-      const int r = i >> 3, c = i & 7;
-      const uint32_t off = r * 128 + ((c ^ (r & 7)) << 4);
-      if (r < T) {
-        const __half* src = base + static_cast<long long>(r) * (3 * C) + c * 8;
-        cp_async16(k0 + off, src + C);
-        cp_async16(v0 + off, src + 2 * C);
-      } else {
-        *reinterpret_cast<uint4*>(sK + off) = make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(sV + off) = make_uint4(0, 0, 0, 0);
-      }
-    }
-    cp_async_commit();
-  }
-  const bool exact_r = QUANT ? (__syncthreads_and(my_exact) != 0) : true;
-  cp_async_wait<0>();
   __syncthreads();
+  bool ok = true;
 
-  const int q4 = lane & 3, r8 = lane >> 2;
-  const float c_exp = 0.125f * 1.4426950408889634f;      // 1/sqrt(64) * log2(e)
-  const uint32_t sK0 = smem_u32(sK), sV0 = smem_u32(sV);
-  const int n_row_blocks = tp >> 4;
-  const int key_blocks = (tp + 63) >> 6;
-
-  for (int rb = warp; rb < n_row_blocks; rb += kAttnWarps) {
-    // ---- Q fragments of this warp's 16 rows (rows beyond T shadow the last row; they are not stored)
-    uint32_t qa[4][4];
-    {
-      const int row_lo = min(rb * 16 + r8, T - 1), row_hi = min(rb * 16 + r8 + 8, T - 1);
-      const uint32_t* q_lo = reinterpret_cast<const uint32_t*>(base + static_cast<long long>(row_lo) * (3 * C));
-      const uint32_t* q_hi = reinterpret_cast<const uint32_t*>(base + static_cast<long long>(row_hi) * (3 * C));
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        qa[ks][0] = __ldg(q_lo + ks * 8 + q4);
-        qa[ks][1] = __ldg(q_hi + ks * 8 + q4);
-        qa[ks][2] = __ldg(q_lo + ks * 8 + 4 + q4);
-        qa[ks][3] = __ldg(q_hi + ks * 8 + 4 + q4);
+  if (warp >= 8) {
+    fewer_registers<kAttnIssueRegs>();
+    if (warp == 8) {
+      // ---------------------------------------------------------------- TMA loads
+      if (lane == 0) {
+        tma_prefetch_desc(&tm_q);
+        tma_prefetch_desc(&tm_kv);
+        tma_prefetch_desc(&tm_out);
       }
+      pdl_wait();
+      uint32_t heads = 0;
+      auto loads = [&](int it) {
+        const uint32_t i = static_cast<uint32_t>(it - first);
+        int b, x;
+        const int q0 = place(it, &b, &x);
+        if (i > 0 && !mbar_wait(q_free, (i - 1) & 1)) return false;
+        mbar_arrive_expect_tx(q_full, kAttnQueries * 128);
+        tma_load_3d(smem + L.q, &tm_q, q_full, x, q0, b);
+        if (i == 0 || q0 == 0) {
+          if (heads > 0 && !mbar_wait(k_free, (heads - 1) & 1)) return false;
+          mbar_arrive_expect_tx(k_full, static_cast<uint32_t>(p.tk) * 128);
+          tma_load_3d(smem + L.k, &tm_kv, k_full, C + x, 0, b);
+          if (heads > 0 && !mbar_wait(v_free, (heads - 1) & 1)) return false;
+          mbar_arrive_expect_tx(v_full, static_cast<uint32_t>(p.tk) * 128);
+          tma_load_3d(smem + L.v, &tm_kv, v_full, 2 * C + x, 0, b);
+          ++heads;
+        }
+        return true;
+      };
+      if (lane == 0) ok = loads(first);
+      __syncwarp();
+      __syncthreads();                    // tensor memory allocated
+      pdl_launch_dependents();
+      if (lane == 0) {
+        for (int it = first + 1; it < last && ok; ++it) ok = loads(it);
+        if (!ok) {
+          // give copies that are still in flight time to land before this block's shared memory goes away
+          for (int i = 0; i < 64; ++i) __nanosleep(1000);
+          atomicExch(p.status, kStatusAttentionTimeout);
+        }
+      }
+      __syncwarp();
+    } else {
+      // ---------------------------------------------------------------- products (warp 9); warps 10 and 11 only keep step
+      if (warp == 9) {
+        pdl_wait();
+        tmem_alloc(s_tmem, kAttnTmemCols);
+        tmem_relinquish();
+        tc_fence_before_sync();
+      }
+      __syncthreads();
+      pdl_launch_dependents();
+      tc_fence_after_sync();
+      if (warp == 9 && lane == 0) {
+        const uint32_t tmem = *s_tmem;
+        const uint32_t idesc_s = umma_idesc_f16(kAttnQueries, p.tk);
+        const uint32_t idesc_o = umma_idesc_f16(kAttnQueries, 64) | (1u << 16);      // B with its rows (keys) along K
+        const uint64_t dq = umma_desc_sw128(smem_u32(smem + L.q)), dk = umma_desc_sw128(smem_u32(smem + L.k)),
+                       dv = umma_desc_sw128(smem_u32(smem + L.v));
+        const int split = attn_split(p.tk);
+        uint32_t heads = 0;
+        for (int it = first; it < last; ++it) {
+          const uint32_t i = static_cast<uint32_t>(it - first);
+          const int q_tile = it % p.qtiles;
+          const bool new_head = i == 0 || q_tile == 0, end_head = it + 1 == last || q_tile + 1 == p.qtiles;
+          heads += new_head ? 1 : 0;
+          ok = (!new_head || mbar_wait(k_full, (heads - 1) & 1)) && mbar_wait(q_full, i & 1) && (i == 0 || mbar_wait(o_read, (i - 1) & 1));
+          if (!ok) break;
+          tc_fence_after_sync();
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_f16(tmem, dq + 2 * k, dk + 2 * k, idesc_s, k > 0);
+          umma_commit(s_full);
+          umma_commit(q_free);
+          if (end_head) umma_commit(k_free);
+          ok = (!new_head || mbar_wait(v_full, (heads - 1) & 1)) && mbar_wait(p_upper, i & 1);
+          if (!ok) break;
+          tc_fence_after_sync();
+          uint32_t acc = 0;
+          for (int k = split; k < p.tk; k += 16, acc = 1)
+            umma_f16_tmem_a(tmem + kAttnOutCol, tmem + split + (k - split) / 2, dv + 8 * k, idesc_o, acc);
+          ok = mbar_wait(p_lower, i & 1);
+          if (!ok) break;
+          tc_fence_after_sync();
+          for (int k = 0; k < split; k += 16, acc = 1) umma_f16_tmem_a(tmem + kAttnOutCol, tmem + k / 2, dv + 8 * k, idesc_o, acc);
+          umma_commit(o_full);
+          if (end_head) umma_commit(v_free);
+        }
+        if (!ok) atomicExch(p.status, kStatusAttentionTimeout);
+      }
+      __syncwarp();
     }
-    float o[8][4];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f; }
-    float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.0f, l_hi = 0.0f;
-
-    for (int kb = 0; kb < key_blocks; ++kb) {
-      const int key0 = kb * 64;
-      const int nb16 = min(4, (tp - key0) >> 4);          // 16-key steps in this block
-      float s[8][4];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) { s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.0f; }
-      // S = Q K^T: B fragments by ldmatrix from K rows (keys), 16 keys x 16 d per instruction
-      // (d step outermost: the eight products of a step go to eight different accumulators)
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-          if (jj < nb16) {
-            const int mi = lane >> 3, rr = lane & 7;
-            const int key = key0 + jj * 16 + (mi >> 1) * 8 + rr;
-            const int chunk = ks * 2 + (mi & 1);
-            uint32_t kf[4];
-            ldmatrix_x4(sK0 + key * 128 + ((chunk ^ (key & 7)) << 4), kf);
-            mma_16816(s[2 * jj], qa[ks], kf[0], kf[1]);
-            mma_16816(s[2 * jj + 1], qa[ks], kf[2], kf[3]);
+  } else if (warp < kAttnRowWarps) {
+    // ------------------------------------------------------------------ softmax: a thread per query row
+    more_registers<kAttnSoftmaxRegs>();
+    __syncthreads();
+    pdl_launch_dependents();
+    tc_fence_after_sync();
+    const uint32_t slot = *s_tmem + (static_cast<uint32_t>(warp * 32) << 16);
+    constexpr float kScale = 0.125f * 1.44269504088896340736f;             // 1 / sqrt(64) and base 2
+    const int split = attn_split(p.tk), tk = p.tk;
+    const float ninf = __int_as_float(0xff800000);
+    for (int it = first; it < last; ++it) {
+      const uint32_t ph = static_cast<uint32_t>(it - first) & 1;
+      const bool live = (it % p.qtiles) * kAttnQueries + warp * 32 < T;    // some of the warp's rows are queries
+      if (!mbar_wait(s_full, ph)) { ok = false; break; }
+      tc_fence_after_sync();
+      // S from column `from` to `to` in pieces of 32 (the last one 16 where that is all), one piece ahead
+      uint32_t a[2][32];
+      auto load = [&](uint32_t (&s)[32], int c, int to) {
+        if (c + 16 < to) tmem_ld_32x32(slot + c, s);
+        else tmem_ld_32x16(slot + c, *reinterpret_cast<uint32_t(*)[16]>(&s[0]));
+      };
+      auto pieces = [&](int from, int to, auto work) {
+        if (from >= to) return;
+        load(a[0], from, to);
+        for (int c = from; c < to; c += 64) {
+          tmem_ld_wait();
+          if (c + 32 < to) load(a[1], c + 32, to);
+          work(a[0], c);
+          if (c + 32 < to) {
+            tmem_ld_wait();
+            if (c + 64 < to) load(a[0], c + 64, to);
+            work(a[1], c + 32);
           }
         }
-      }
-      // mask keys beyond T (only the last block can have them), row maxima
-      float mx_lo = -INFINITY, mx_hi = -INFINITY;
+      };
+      float m0 = ninf, m1 = ninf, m2 = ninf, m3 = ninf;
+      auto maxima = [&](uint32_t (&s)[32], int c) {
+        if (c + 32 > T) {                                                  // keys beyond T, and what a piece of 16 did not load
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int col = key0 + j * 8 + 2 * q4;
-        if (j >= 2 * nb16 || col >= T) { s[j][0] = -INFINITY; s[j][2] = -INFINITY; }
-        if (j >= 2 * nb16 || col + 1 >= T) { s[j][1] = -INFINITY; s[j][3] = -INFINITY; }
-        mx_lo = fmaxf(mx_lo, fmaxf(s[j][0], s[j][1]));
-        mx_hi = fmaxf(mx_hi, fmaxf(s[j][2], s[j][3]));
-      }
-      mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1));
-      mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
-      mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
-      mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
-      const float mn_lo = fmaxf(m_lo, mx_lo), mn_hi = fmaxf(m_hi, mx_hi);     // finite: key 0 is never masked
-      const float al_lo = exp2f((m_lo - mn_lo) * c_exp), al_hi = exp2f((m_hi - mn_hi) * c_exp);
-      m_lo = mn_lo;
-      m_hi = mn_hi;
-      l_lo *= al_lo;
-      l_hi *= al_hi;
+          for (int j = 0; j < 32; ++j)
+            if (c + j >= T) s[j] = 0xff800000u;
+        }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { o[j][0] *= al_lo; o[j][1] *= al_lo; o[j][2] *= al_hi; o[j][3] *= al_hi; }
-      const float ms_lo = m_lo * c_exp, ms_hi = m_hi * c_exp;
+        for (int j = 0; j < 32; j += 8) {
+          m0 = max3(m0, __uint_as_float(s[j]), __uint_as_float(s[j + 1]));
+          m1 = max3(m1, __uint_as_float(s[j + 2]), __uint_as_float(s[j + 3]));
+          m2 = max3(m2, __uint_as_float(s[j + 4]), __uint_as_float(s[j + 5]));
+          m3 = max3(m3, __uint_as_float(s[j + 6]), __uint_as_float(s[j + 7]));
+        }
+      };
+      float nm = 0.0f;
+      f32x2 sum0 = pack2(0.0f, 0.0f), sum1 = sum0;
+      auto exponentials = [&](uint32_t (&s)[32], int c, int to, uint32_t p_col) {
+        const f32x2 k2 = pack2(kScale, kScale), nm2 = pack2(nm, nm);
+        if (c + 32 > T) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        s[j][0] = exp2f(fmaf(s[j][0], c_exp, -ms_lo));
-        s[j][1] = exp2f(fmaf(s[j][1], c_exp, -ms_lo));
-        s[j][2] = exp2f(fmaf(s[j][2], c_exp, -ms_hi));
-        s[j][3] = exp2f(fmaf(s[j][3], c_exp, -ms_hi));
-        l_lo += s[j][0] + s[j][1];
-        l_hi += s[j][2] + s[j][3];
-      }
-      // O += P V: P from the accumulator registers, V fragments by transposing ldmatrix (16 keys x 16 d)
+          for (int j = 0; j < 32; ++j)
+            if (c + j >= T) s[j] = 0xff800000u;
+        }
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        if (jj < nb16) {
-          uint32_t pa[4];
-          pa[0] = pack_half2(s[2 * jj][0], s[2 * jj][1]);
-          pa[1] = pack_half2(s[2 * jj][2], s[2 * jj][3]);
-          pa[2] = pack_half2(s[2 * jj + 1][0], s[2 * jj + 1][1]);
-          pa[3] = pack_half2(s[2 * jj + 1][2], s[2 * jj + 1][3]);
+        for (int h = 0; h < 2; ++h) {
+          if (h == 1 && c + 16 >= to) break;
+          uint32_t w[8];
 #pragma unroll
-          for (int nn = 0; nn < 4; ++nn) {
-            const int mi = lane >> 3, rr = lane & 7;
-            const int key = key0 + jj * 16 + (mi & 1) * 8 + rr;
-            const int chunk = nn * 2 + (mi >> 1);
-            uint32_t vf[4];
-            ldmatrix_x4_trans(sV0 + key * 128 + ((chunk ^ (key & 7)) << 4), vf);
-            mma_16816(o[2 * nn], pa, vf[0], vf[1]);
-            mma_16816(o[2 * nn + 1], pa, vf[2], vf[3]);
+          for (int j = 0; j < 8; ++j) {
+            float e0, e1;
+            unpack2(fma2(pack2(__uint_as_float(s[16 * h + 2 * j]), __uint_as_float(s[16 * h + 2 * j + 1])), k2, nm2), e0, e1);
+            const f32x2 e = pack2(exp2_approx(e0), exp2_approx(e1));
+            if (j & 1) sum1 = add2(sum1, e); else sum0 = add2(sum0, e);
+            w[j] = pair_to_sixteen<__half>(e);
           }
+          tmem_st_32x8(p_col + 8 * h, w);                  // over columns of S that have been read
+        }
+      };
+      auto hand_over = [&](uint64_t* bar) {
+        if (live) tmem_st_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar);
+      };
+      if (live) {
+        pieces(0, tk, maxima);
+        nm = -kScale * fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+        pieces(split, tk, [&](uint32_t (&s)[32], int c) { exponentials(s, c, tk, slot + split + (c - split) / 2); });
+      }
+      hand_over(p_upper);
+      if (live) {
+        pieces(0, split, [&](uint32_t (&s)[32], int c) { exponentials(s, c, split, slot + c / 2); });
+        float x0, x1;
+        unpack2(add2(sum0, sum1), x0, x1);
+        s_sums[warp * 32 + lane] = x0 + x1;
+      }
+      hand_over(p_lower);
+    }
+    if (!ok && lane == 0) atomicExch(p.status, kStatusAttentionTimeout);
+  } else {
+    // ------------------------------------------------------------------ output: a thread per query row
+    more_registers<kAttnOutputRegs>();
+    const int quarter = warp - kAttnRowWarps;
+    GroupQuantTables* const tables = reinterpret_cast<GroupQuantTables*>(smem + L.tables);
+    GroupQuantParams gp = {};
+    // reads only the layer's constants: done while the previous kernel still runs
+    if (QUANT)
+      gp = group_quant_tables<1 << BITS>(tables, p.thresholds, p.codebook, tid - 128, kAttnRowWarps * 32, [](bool b) {
+        asm volatile("bar.sync 1, %0;" ::"n"(kAttnRowWarps * 32) : "memory");
+        return b;
+      });
+    __syncthreads();
+    pdl_launch_dependents();
+    tc_fence_after_sync();
+    const uint32_t t_out = *s_tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kAttnOutCol;
+    uint8_t* const stage = smem + L.stage + quarter * 4096;
+    const uint32_t row = smem_u32(stage) + lane * 128, x7 = lane & 7;
+    for (int it = first; it < last; ++it) {
+      const uint32_t ph = static_cast<uint32_t>(it - first) & 1;
+      int b, x;
+      const int t0 = place(it, &b, &x) + quarter * 32;
+      const bool live = t0 < T;
+      // p_lower: the sums are there
+      if (!mbar_wait(p_lower, ph) || !mbar_wait(o_full, ph)) { ok = false; break; }
+      tc_fence_after_sync();
+      uint32_t w[32];
+      if (live) {
+        const float inv = __fdividef(1.0f, s_sums[quarter * 32 + lane]);
+        const f32x2 inv2 = pack2(inv, inv);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t o[32];
+          tmem_ld_32x32(t_out + 32 * h, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            w[16 * h + j] = pair_to_sixteen<__half>(mul2(pack2(__uint_as_float(o[2 * j]), __uint_as_float(o[2 * j + 1])), inv2));
+        }
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(o_read);
+        tma_store_wait_read();                             // the store that last used the staging rows has read them
+      }
+      __syncwarp();
+      if (live) {
+        if (QUANT) {
+          f32x2 v[32];
+          uint32_t words[8];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = sixteen_to_pair<__half>(w[j]);
+          const GroupStats st = group_quantize<BITS, false, 1>(v, tables, gp, words);
+          const GroupRecon g = group_recon(st, gp, p.one_fma != 0);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) w[j] = pair_to_sixteen<__half>(group_recon_pair(g, v[j]));
+        }
+        row_store<1>(w, row, x7);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_3d(&tm_out, stage, x, t0, b);          // tokens beyond T are clipped
+          tma_store_commit();
         }
       }
     }
-    // ---- normalise
-    l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
-    l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
-    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
-    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
-    const float inv_lo = 1.0f / l_lo, inv_hi = 1.0f / l_hi;
-    // the fp16 outputs: x_lo[2n], x_lo[2n+1] = columns 8n+2q, 8n+2q+1 of row r8; x_hi the same of row r8 + 8
-    uint32_t w_lo[8], w_hi[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      w_lo[j] = pack_half2(o[j][0] * inv_lo, o[j][1] * inv_lo);
-      w_hi[j] = pack_half2(o[j][2] * inv_hi, o[j][3] * inv_hi);
-    }
-    if (QUANT) {
-#pragma unroll
-      for (int half_id = 0; half_id < 2; ++half_id) {
-        uint32_t (&w)[8] = half_id ? w_hi : w_lo;
-        float x[16];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
-          x[2 * j] = f.x;
-          x[2 * j + 1] = f.y;
-        }
-        float ve, vo;
-        lane_sums(x, ve, vo);
-        const float mean = __fdiv_rn(row_chain_sum(ve, vo, lane), 64.0f);
-        float sq[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          x[i] = __fsub_rn(x[i], mean);
-          sq[i] = __fmul_rn(x[i], x[i]);
-        }
-        lane_sums(sq, ve, vo);
-        const float var = __fdiv_rn(row_chain_sum(ve, vo, lane), 64.0f);
-        const float scale = __fsqrt_rn(__fadd_rn(var, 1.0e-6f));
-        // codes: number of thresholds below r / scale, by the exact division-free test (or the IEEE quotient
-        // for thresholds too close to zero), then the codebook value
-        int code[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) code[i] = 0;
-        if (!exact_r) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) x[i] = __fdiv_rn(x[i], scale);       // compared against the thresholds themselves
-        }
-#pragma unroll
-        for (int t = 0; t < L - 1; ++t) {
-          const float th = s_th[t];
-          const float hs = __fmul_rd(__fmul_rn(s_h[t], scale), th == 0.0f ? 0x1p-50f : 1.0f);
-          const float lim = exact_r ? __fmaf_rd(th, scale, hs) : th;
-#pragma unroll
-          for (int i = 0; i < 16; ++i) code[i] += (x[i] > lim) ? 1 : 0;
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = s_cb[code[i]];
-        lane_sums(x, ve, vo);
-        const float code_sum = row_chain_sum(ve, vo, lane);
-        const float vm = __fmul_rn(code_sum, 1.0f / 64.0f);
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          w[j] = pack_half2(__fadd_rn(mean, __fmul_rn(scale, __fsub_rn(x[2 * j], vm))),
-                            __fadd_rn(mean, __fmul_rn(scale, __fsub_rn(x[2 * j + 1], vm))));
-      }
-    }
-    // ---- through this warp's staging block (16 rows x 128 bytes, XOR-swizzled) to 16-byte row stores
-    uint8_t* const stg = sStage + warp * 2048;
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      *reinterpret_cast<uint32_t*>(stg + r8 * 128 + ((j ^ (r8 & 7)) << 4) + q4 * 4) = w_lo[j];
-      *reinterpret_cast<uint32_t*>(stg + (r8 + 8) * 128 + ((j ^ (r8 & 7)) << 4) + q4 * 4) = w_hi[j];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int idx = lane + 32 * i, r = idx >> 3, c = idx & 7;
-      const int row = rb * 16 + r;
-      if (row < T) {
-        const uint4 v = *reinterpret_cast<const uint4*>(stg + r * 128 + ((c ^ (r & 7)) << 4));
-        *reinterpret_cast<uint4*>(p.out + (static_cast<long long>(b) * T + row) * C + h * 64 + c * 8) = v;
-      }
-    }
+    if (lane == 0) tma_store_wait_all();
+    if (!ok && lane == 0) atomicExch(p.status, kStatusAttentionTimeout);
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 9) {
+    tc_fence_after_sync();
+    tmem_dealloc(*s_tmem, kAttnTmemCols);
   }
 }
 

@@ -285,6 +285,10 @@ int arcq_attention(const void* qkv, int64_t B, int64_t T, int64_t H, int head_di
 int arcq_attention_act_quant(const void* qkv, int64_t B, int64_t T, int64_t H, int head_dim,
                              const float* thresholds, const float* codebook, int bits, int group_size,
                              void* xhat, void* stream);
+/* The same, reconstructing with one fma where one_fma is not 0, as in arcq_act_quant_unpack. */
+int arcq_attention_act_quant_form(const void* qkv, int64_t B, int64_t T, int64_t H, int head_dim,
+                                  const float* thresholds, const float* codebook, int bits, int group_size,
+                                  void* xhat, int one_fma, void* stream);
 
 /*
  * The data movement around a ViT's patch-embedding GEMM (timm PatchEmbed.forward and VisionTransformer._pos_embed),

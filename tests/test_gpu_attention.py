@@ -84,3 +84,42 @@ def test_model_with_the_attention_kernel(pkg, cuda_device):
         assert float((y1.float() - y0.float()).pow(2).mean().sqrt()) < 0.5 * rms
     finally:
         attn_cls.implementation = saved
+
+
+@pytest.mark.parametrize("B,T,H", [(3, 17, 2), (2, 33, 1), (2, 128, 3), (2, 129, 3), (1, 144, 2), (1, 224, 1), (1, 225, 1), (2, 240, 2),
+                                   (3, 255, 1), (130, 100, 3), (70, 197, 6)])
+def test_attention_kernel_tile_edges(pkg, cuda_device, B, T, H):
+    """Token counts around the edges of the products (multiples of 16), of the score pieces (32), of the query tiles (128) and of
+    the tensor-memory layout, and more heads than blocks.  An output is a convex combination of fp16 values up to 8: rounding P and
+    the output to fp16 gives at most 2^-11 of the largest value each, 2^-10 * 8 in all."""
+    gen = torch.Generator().manual_seed(T)
+    qkv = (torch.randn(B * T, 3 * H * 64, generator=gen) * 1.5).clamp(-8, 8).half().to(cuda_device)
+    out = pkg.ops.attention(qkv, B, T, H)
+    ref = _fp64(qkv, B, T, H)
+    assert float((out.double() - ref).abs().max()) <= 8 * 2.0 ** -10
+    # no further from 64 bits than the library's kernel, over the whole matrix
+    err = [float((y.double() - ref).norm() / ref.norm()) for y in (out, _library(qkv, B, T, H))]
+    assert err[0] <= 1.05 * err[1], err
+    cb = torch.linspace(-2.5, 2.5, 8, device=cuda_device)
+    th = (cb[:-1] + cb[1:]) / 2
+    assert torch.equal(pkg.ops.attention(qkv, B, T, H, th, cb, 3), pkg.ops.quantize_activation_dequant(out, th, cb, 3, 64, torch.float16))
+    assert pkg.ops.device_status() == 0
+
+
+def test_attention_kernel_extreme_scores(pkg, cuda_device):
+    """Large scores of one sign (nothing but the maximum may decide which exponentials survive), equal scores, and values that are
+    not finite: like softmax in the library."""
+    B, T, H = 2, 197, 1
+    gen = torch.Generator().manual_seed(5)
+    qkv = torch.randn(B * T, 192, generator=gen)
+    qkv[:T, :64], qkv[:T, 64:128] = 30.0, -30.0 - torch.rand(T, 1, generator=gen)      # scores around -7200
+    qkv[T:, :64] = 0.0                                                                # equal scores
+    x = qkv.half().to(cuda_device)
+    out, ref = pkg.ops.attention(x, B, T, H), _fp64(x, B, T, H)
+    assert float((out.double() - ref).abs().max()) <= 8 * 2.0 ** -10
+    x[3, 0] = float("nan")                                                            # one query: its row only
+    x[T + 5, 70] = float("inf")                                                       # one key of the second image
+    got, want = pkg.ops.attention(x, B, T, H), _library(x, B, T, H)
+    assert torch.equal(got.isnan().any(1), want.isnan().any(1))
+    assert torch.equal(got[4:T], out[4:T])
+    assert pkg.ops.device_status() == 0
