@@ -2,9 +2,10 @@
 // a tile in by TMA (a row per group, 128-byte swizzle, so that lanes read their rows without bank conflicts), quantises it in place and sends the reconstruction out by TMA, with the next tile's load and the previous
 // tile's store in flight meanwhile.  No block-wide synchronisation after the table set-up.
 //
-// Bound by issue slots, then by shared-memory reads (about four wavefronts per 32 values); memory is half idle.
-// One lane a group, 16 warps an SM.  [12608, 384] 5.7 us, with GELU [12608, 1536] 25.4 us (before the shared group routine 7.7
-// and 37.6 us).
+// Bound by issue slots (half of them used: fixed latencies and instruction fetches of the straight-line group routine), then by
+// shared-memory reads (about three wavefronts per 32 values).  One lane a group, 16 warps an SM.  [12608, 384] 5.2 us, [50432,
+// 768] 29.3 us (5.3 TB/s), with GELU [12608, 1536] 24.1 us; 6.3, 31.2 and 24.5 us when a level took three table reads and a value
+// at a threshold sent its seven neighbours through the exact path too.
 #pragma once
 #include <cuda.h>
 #include "ptx.cuh"

@@ -7,20 +7,22 @@
 //
 // What bounds it is issue slots: nothing here waits for memory once the row is in shared memory.  So the arithmetic is
 // two values per instruction (add / mul / fma.f32x2; each half rounds like the scalar instruction, so the bits are those of
-// scalar code), and a code costs three table values and one compare:
+// scalar code), and a level costs two table reads and one compare:
 //
 //   * Bounded argument.  sum r^2 = 64 var, so |r| / s <= 8 for every element of a group: a grid over [-16, 16) needs no
 //     clamp.  One fma, rounded down, turns r into 1.5 * 2^21 + cell with two fraction bits below the cell, i.e. the low
 //     bits of the result are 4 * cell: the byte offset into the tables.
 //   * cell -> (threshold, level below it, level above it).  Consecutive cells lie in consecutive banks and the values of a
 //     group span some twenty cells, so the reads are conflict-free without copies of the tables.
-//   * level = r > th * s ? above : below, the sign of d = fma(-th, s, r).
+//   * level = r > th * s ? above : below: the sign of d = fma(-th, s, r) picks the table that is read.  (Both levels read and one
+//     selected: a third read, and [50432, 768] 31.2 instead of 29.3 us together with the next item.)
 //
 // Exactness.  The code is the number of thresholds with RN(r / s) > th.  With h half the gap from th to the next fp32
 // number, RN(r / s) > th <=> r > (th + h) * s, while the sign of d (rounding to nearest keeps signs) tells r > th * s.
-// The two differ only if 0 < r - th * s <= h * s, so a chunk of eight values with some |d| <= s * max h goes through the
-// IEEE quotient and a search over all thresholds: about one value in a million.  A codebook with two thresholds
-// closer than 1.1 cells takes that path for every value.
+// The two differ only if 0 < r - th * s <= h * s, so a value with |d| <= s * max h goes through the IEEE quotient and a search
+// over all thresholds: about one in a million (15 thresholds, +-1.5e-7 each, at a density of 0.3), i.e. a few of nearly every
+// launch's warps, which the launch then waits for.  A codebook with two thresholds closer than 1.1 cells takes that path for every
+// value.
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
@@ -67,6 +69,12 @@ __device__ __forceinline__ float min3_abs(float m, float a, float b) {
   float d;
   asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(m), "f"(fabsf(a)), "f"(fabsf(b)));
   return d;
+}
+
+// a + OFFSET where d > 0
+template <uint32_t OFFSET> __device__ __forceinline__ uint32_t offset_if_positive(uint32_t a, float d) {
+  asm("{\n\t.reg .pred p;\n\tsetp.gt.f32 p, %1, 0f00000000;\n\t@p add.u32 %0, %0, %2;\n\t}" : "+r"(a) : "f"(d), "n"(OFFSET));
+  return a;
 }
 
 // ---------------------------------------------------------------- per-layer tables in shared memory
@@ -200,11 +208,12 @@ __device__ __forceinline__ GroupStats group_quantize(f32x2 (&v)[32 / LPG], const
   constexpr uint32_t kLo = kGqCells * 4, kHi = 2 * kGqCells * 4, kCode = 3 * kGqCells * 4, kCb = 4 * kGqCells * 4 + 64;
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
-    float m = 1.0e38f, out[CH];
+    float m = 1.0e38f, out[CH], d[CH];
     uint32_t w = 0;
 #pragma unroll
     for (int j = 0; j < PJ; ++j) {
-      float u0, u1, d0, d1;
+      float u0, u1;
+      float &d0 = d[2 * j], &d1 = d[2 * j + 1];
       unpack2(fma2_down(v[c * PJ + j], a2, magic), u0, u1);
       const uint32_t o0 = (__float_as_uint(u0) & 0x3FCu) | tab, o1 = (__float_as_uint(u1) & 0x3FCu) | tab;
       unpack2(fma2(pack2(lds_const_f32(o0), lds_const_f32(o1)), s2, v[c * PJ + j]), d0, d1);
@@ -218,28 +227,33 @@ __device__ __forceinline__ GroupStats group_quantize(f32x2 (&v)[32 / LPG], const
         w |= (c0 | (c1 << 4)) << (8 * j);                    // four times the codes; shifted down once per word below
         if (j == PJ - 1) words[c] = (w >> 2) | ((c1 >> 4) << 30);
       } else {
-        const float l0 = lds_const_f32(o0 + kLo), h0 = lds_const_f32(o0 + kHi);
-        const float l1 = lds_const_f32(o1 + kLo), h1 = lds_const_f32(o1 + kHi);
-        out[2 * j] = d0 > 0.0f ? h0 : l0;
-        out[2 * j + 1] = d1 > 0.0f ? h1 : l1;
+        out[2 * j] = lds_const_f32(offset_if_positive<kHi - kLo>(o0, d0) + kLo);
+        out[2 * j + 1] = lds_const_f32(offset_if_positive<kHi - kLo>(o1, d1) + kLo);
       }
     }
     if (__builtin_expect(m <= tie, 0)) {
-      // rare: some value of the chunk is too close to a threshold for the sign of d alone (through local memory, so that the
-      // common path keeps its registers where they are)
-      float r[CH];
+      // rare: a value of the chunk is too close to a threshold for the sign of d alone.  One of a kernel's warps gets here in
+      // most launches, and the others wait for it at the end, so it looks at the values in question only (through local memory,
+      // so that the common path keeps its registers where they are): all eight values took 1.1 us.
+      float r[CH], level[CH];
+      uint32_t hits = 0;
 #pragma unroll
       for (int j = 0; j < PJ; ++j) unpack2(v[c * PJ + j], r[2 * j], r[2 * j + 1]);
-      uint32_t we = 0;
-#pragma unroll 1
+#pragma unroll
       for (int j = 0; j < CH; ++j) {
+        level[j] = out[j];
+        hits |= fabsf(d[j]) <= tie ? 1u << j : 0u;
+      }
+#pragma unroll 1
+      while (hits != 0) {
+        const int j = __ffs(hits) - 1;
+        hits &= hits - 1;
         const int code = group_quant_exact_code<L>(t, r[j], s);
-        r[j] = t->cb[code];
-        we |= static_cast<uint32_t>(code) << (4 * j);
+        level[j] = t->cb[code];
+        if (CODES) words[c] = (words[c] & ~(15u << (4 * j))) | (static_cast<uint32_t>(code) << (4 * j));
       }
 #pragma unroll
-      for (int j = 0; j < CH; ++j) out[j] = r[j];
-      if (CODES) words[c] = we;
+      for (int j = 0; j < CH; ++j) out[j] = level[j];
     }
 #pragma unroll
     for (int j = 0; j < PJ; ++j) v[c * PJ + j] = pack2(out[2 * j], out[2 * j + 1]);

@@ -440,6 +440,38 @@ def test_staged_quantizer_with_close_thresholds_falls_back_to_the_search(pkg, or
     assert np.array_equal(c.cpu().numpy(), cs)
 
 
+@pytest.mark.parametrize("bits", [4, 3, 2])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32, torch.bfloat16])
+def test_values_on_thresholds_among_others(pkg, oracle, cuda_device, bits, dtype):
+    """Thresholds that are quotients of the data, all in one chunk of eight of the same group, which is repeated: several values of
+    a chunk need the exact comparison, their neighbours do not, and other groups hold none."""
+    rng = np.random.default_rng(bits)
+    X = torch.from_numpy(rng.standard_normal((1600, 1536), dtype=np.float32)).to(dtype)      # 38 400 groups
+    n = 2 ** bits - 1
+    want = np.linspace(-2.4, 2.4, n)
+    X[0, :64] = torch.from_numpy(rng.standard_normal(64, dtype=np.float32) * 0.7).to(dtype)
+    X[0, 24:24 + min(n, 8)] = torch.from_numpy(want[:: max(1, n // 8)][: min(n, 8)].astype(np.float32)).to(dtype)
+    X[::7, 64:128] = X[0, :64]
+    X = X.float()
+    cb0 = np.linspace(-2, 2, n + 1).astype(np.float32)
+    _, mu, sg, _ = oracle.quantize(X[:1, :64].numpy(), ((cb0[:-1] + cb0[1:]) / 2).astype(np.float32), cb0, 64)
+    q = (X[0, :64].numpy() - mu[0, 0]) / sg[0, 0]                                            # fp32, as the quantizer divides
+    th = want.astype(np.float32)
+    for i in range(24, 24 + min(n, 8)):
+        th[np.abs(th - q[i]).argmin()] = q[i]
+    th = np.sort(th)
+    cb = np.concatenate([th[:1] - 0.3, (th[:-1] + th[1:]) / 2, th[-1:] + 0.3]).astype(np.float32)
+    assert np.diff(th).min() > 0.15 and np.isin(q, th).sum() >= min(n, 4)
+    codes, mu, sg, cs = oracle.quantize(X.numpy(), th, cb, 64)
+    x = X.to(dtype).to(cuda_device)
+    p, m, s, c = pkg.ops.quantize_activation(x, _t(th, cuda_device), _t(cb, cuda_device), bits, 64)
+    assert np.array_equal(p.cpu().numpy(), oracle.pack(codes, bits))
+    assert np.array_equal(m.cpu().numpy(), mu) and np.array_equal(s.cpu().numpy(), sg) and np.array_equal(c.cpu().numpy(), cs)
+    xh = pkg.ops.quantize_activation_dequant(x, _t(th, cuda_device), _t(cb, cuda_device), bits, 64, torch.float16)
+    assert torch.equal(xh.cpu(), torch.from_numpy(oracle.dequant(codes, mu, sg, cb, 64)).to(torch.float16))
+    assert pkg.ops.device_status() == 0
+
+
 def _dequant_with_stats(pkg, x, th, cb, bits, pre_gelu=False):
     """arcq_act_quant through the C ABI with no packed output: reconstruction plus the three statistics."""
     lib = pkg._cabi.load()
