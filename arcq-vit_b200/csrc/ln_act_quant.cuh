@@ -94,6 +94,16 @@ __global__ void __launch_bounds__(kLnqThreads, 4)
         }
       }
     }
+    if (tid == 0) {
+      // the rows of this block's next tile: from HBM to L2 while this one is quantised (the loads of a tile start after a barrier,
+      // with nothing else of the block to do: [50432, 768] 73.3 -> 68.2 us, [201728, 768] 277 -> 257 us)
+      const long long next = (tile + gridDim.x - jobs.blocks) * kLnqThreads, end = min(next + kLnqThreads, total_groups);
+      if (next < end) {
+        const uint32_t bytes = static_cast<uint32_t>((end - next) * 128);
+        bulk_prefetch_l2(x + next * 64, bytes);
+        if (HAS_Y) bulk_prefetch_l2(y + next * 64, bytes);
+      }
+    }
     __syncthreads();
 
     // ---- phase 2: the activation quantizer on h, one thread per group, in place; a warp sends its 32 rows out by TMA
