@@ -54,10 +54,14 @@ struct PairDenseParams {
 };
 
 constexpr int kPairDenseThreads = (2 + kPairEpiWarps) * 32;
-// The quantizer form has three epilogue warps per lane quarter, one per 64-column group of a 192-column slab (14 warps: 128
-// registers a thread, which the quantizer needs; 18 would leave 112).
-constexpr int kPairQuantEpiWarps = 12;
-constexpr int kPairQuantThreads = (2 + kPairQuantEpiWarps) * 32;
+// The quantizer form has three epilogue warps per lane quarter, one per 64-column group of a 192-column slab.  The issuing warps
+// are a warp group of their own (two of its warps idle), whose registers the epilogue warps take over: 152 instead of the
+// launch's 128 ([12608, 3072] x 768 76.3 -> 75.1 us, [50432, 3072] x 768 357 -> 350 us).
+constexpr int kPairQuantEpiWarps = 12, kPairQuantIssueWarps = 4;
+constexpr int kPairQuantThreads = (kPairQuantIssueWarps + kPairQuantEpiWarps) * 32;
+constexpr int kPairQuantEpiRegs = 152, kPairQuantIssueRegs = 56;
+static_assert(kPairQuantEpiRegs * kPairQuantEpiWarps + kPairQuantIssueRegs * kPairQuantIssueWarps <= 128 * (kPairQuantThreads / 32),
+              "registers beyond the launch's never come");
 constexpr uint32_t kPairQuantStageBytes = kPairQuantEpiWarps * 4096;       // 32 rows of 128 bytes per warp
 constexpr uint32_t kPairQuantTableBytes = (sizeof(GroupQuantTables) + 15) / 16 * 16;
 // Staging blocks (2 KB: 32 rows x 64 bytes) per epilogue warp; a block can be rewritten once the TMA store that
@@ -94,7 +98,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
     dense_weight_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                                   const __grid_constant__ CUtensorMap tm_y, const PairDenseParams p,
                                   const __grid_constant__ UnpackJobs jobs) {
-  constexpr int kEpi = QBITS ? kPairQuantEpiWarps : kPairEpiWarps;
+  constexpr int kEpi = QBITS ? kPairQuantEpiWarps : kPairEpiWarps, kIssue = QBITS ? kPairQuantIssueWarps : 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* const smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const PairDenseSmem L = pair_dense_smem_layout(p.bn, p.sa, p.ks, p.G, STATIONARY, QBITS != 0);
@@ -165,6 +169,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA: this CTA's half of every stage
+    if constexpr (QBITS != 0) fewer_registers<kPairQuantIssueRegs>();
     const uint32_t sa = p.sa;
     const uint32_t full_leader = mapa_shared(full, 0);
     const uint32_t st0 = smem_u32(sStages);
@@ -212,6 +217,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issue (leader CTA only)
+    if constexpr (QBITS != 0) fewer_registers<kPairQuantIssueRegs>();
     if (crank == 0 && my_tiles > 0) {
       const uint32_t idesc = umma_idesc_f16(kPairTileM, bn);
       const uint32_t sa = p.sa;
@@ -264,17 +270,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
       __syncwarp();
       if (!ok && lane == 0) atomicExch(p.status, kStatusPairTimeout);
     }
+  } else if (QBITS != 0 && warp < kIssue) {
+    // the quantizer form's idle warps (no register instruction in the plain form, not even where nothing gets to it: 2 to 8 % slower)
+    if constexpr (QBITS != 0) fewer_registers<kPairQuantIssueRegs>();
   } else if constexpr (QBITS != 0) {
+    more_registers<kPairQuantEpiRegs>();
     // ------------------------------------------------------------------ epilogue with GELU and quantizer
     // A thread owns one row and 64 columns, i.e. one group of the next layer's activation quantizer: tensor memory -> + bias ->
     // fp16 (what the plain form stores) -> GELU -> quantizer -> reconstruction, in registers but for the exchange of large GELU
     // arguments, then through this warp's staging rows to a TMA store.  Issue slots of these warps bound the kernel (about 30
     // instructions a value); the products run underneath.  N = 3072, K = 768: M = 12608 72.9 us against 49.4 + 40.3 us for GEMM
     // and quantizer kernel, M = 100864 618 against 457 + 407 us.
-    const int ew = warp - 2, lq = warp & 3, grp = ew >> 2;
+    const int ew = warp - kIssue, lq = warp & 3, grp = ew >> 2;
     GroupQuantTables* const tables = reinterpret_cast<GroupQuantTables*>(smem + L.tables);
-    for (int i = tid - 64; i < bn; i += kEpi * 32) s_bias[i] = (p.bias != nullptr) ? __ldg(p.bias + n0 + i) : 0.0f;
-    const GroupQuantParams gp = group_quant_tables<1 << QBITS>(tables, p.thresholds, p.codebook, tid - 64, kEpi * 32, [](bool b) {
+    for (int i = tid - kIssue * 32; i < bn; i += kEpi * 32) s_bias[i] = (p.bias != nullptr) ? __ldg(p.bias + n0 + i) : 0.0f;
+    const GroupQuantParams gp = group_quant_tables<1 << QBITS>(tables, p.thresholds, p.codebook, tid - kIssue * 32, kEpi * 32, [](bool b) {
       asm volatile("bar.sync 2, %0;" ::"n"(kEpi * 32) : "memory");
       return b;
     });
