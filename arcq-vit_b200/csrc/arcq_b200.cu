@@ -648,7 +648,10 @@ bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32,
       // W16 rows too unless the slab is stationary
       const double fill_mb = (static_cast<double>(slabs) * M * K * 2.0 +
                               (stationary ? static_cast<double>(k.pairs) : static_cast<double>(slabs * tiles_m)) * bn * K * 2.0) / 1.0e6;
-      const double t_fill = fill_mb / 8.0;
+      // ... and 12 TB/s where the tiles stream long rows (8 throughout took 256-column slabs for [7289, 3072] x 768: 34.5 us against
+      // 29.6, [12608, 768] x 768: 17.5 against 16.0, [12608, 3072] x 768: 58.6 against 55.0; 12 throughout took 96-column slabs for
+      // [12608, 384] x 384: 9.5 us against 8.5)
+      const double t_fill = fill_mb / (K >= 768 ? 12.0 : 8.0);
       // 0.45 us per tile that neither the stores nor the issue account for (measured: at equal store volume, 192-wide
       // slabs beat 128-wide ones on N = 1152 by 1 us over 5 against 7 tiles per pair)
       const double path = tiles_pp * ((t_write > t_issue ? t_write : t_issue) + 0.45) * (stationary ? 0.95 : 1.0);
