@@ -277,6 +277,21 @@ def attention(qkv: torch.Tensor, batch: int, tokens: int, heads: int, thresholds
     return out
 
 
+# The same as an operator of the framework, for callers inside a model: function and dispatch modes see it by the name of what it
+# stands for, tensor subclasses are unwrapped as for any other operator.  No gradient.
+if not hasattr(torch.ops.arcq, "scaled_dot_product_attention"):
+    torch.library.define("arcq::scaled_dot_product_attention",
+                         "(Tensor qkv, int batch, int tokens, int heads, Tensor? thresholds, Tensor? codebook, int bits) -> Tensor")
+
+    @torch.library.impl("arcq::scaled_dot_product_attention", "cuda")
+    def _attention_op(qkv, batch, tokens, heads, thresholds, codebook, bits):
+        return attention(qkv, batch, tokens, heads, thresholds, codebook, bits)
+
+    @torch.library.register_fake("arcq::scaled_dot_product_attention")
+    def _attention_shape(qkv, batch, tokens, heads, thresholds, codebook, bits):
+        return qkv.new_empty((batch * tokens, heads * 64))
+
+
 def patchify(images: torch.Tensor, patch: int) -> torch.Tensor:
     """fp16 images [B, C, H, W] -> [B, (H/patch)*(W/patch), C*patch*patch]: row (gy, gx), column (c, py, px), i.e.
     ``images.reshape(B, C, gh, p, gw, p).permute(0, 2, 4, 1, 3, 5).reshape(B, gh*gw, C*p*p)`` in one kernel."""

@@ -35,10 +35,13 @@ DEIT_CONFIGS: Dict[str, Tuple[int, int, int]] = {
 }
 
 
+_LIBRARY_ATTENTION = F.scaled_dot_product_attention
+
+
 class Attention(nn.Module):
     # "kernel": this package's attention kernel (heads of 64, at most 256 tokens, fp16 on a GPU), which also runs
     # proj's activation quantizer when proj can take a reconstructed input; "sdpa": the library attention; "auto": the
-    # library attention, inside the model's one-call forward where that applies.
+    # kernel between packed linears (alone or inside the model's one-call forward), the library attention elsewhere.
     implementation = os.environ.get("ARCQ_ATTENTION", "auto")
 
     def __init__(self, dim: int, heads: int):
@@ -50,18 +53,28 @@ class Attention(nn.Module):
     def forward(self, x: torch.Tensor, pre_quantized: bool = False) -> torch.Tensor:
         B, T, C = x.shape
         qkv = self.qkv(x, pre_quantized=True) if pre_quantized else self.qkv(x)
-        if (self.implementation == "kernel" and qkv.is_cuda and qkv.dtype == torch.float16 and C == 64 * self.num_heads
-                and T <= 256):
-            from . import ops
-            proj = self.proj
-            if isinstance(proj, ARCQPackedLinearOnTheFly) and proj.takes_reconstructed_input():
-                xh = ops.attention(qkv, B, T, self.num_heads, proj.activation_thresholds, proj.activation_codebook,
-                                   proj.bits, proj.group_size)
+        proj = self.proj
+        if (qkv.is_cuda and qkv.dtype == torch.float16 and C == 64 * self.num_heads and T <= 256
+                and (self.implementation == "kernel" or self.implementation == "auto" and _replaces_library_attention(qkv, proj))):
+            from . import ops  # noqa: F401  registers the operator
+            attention = torch.ops.arcq.scaled_dot_product_attention
+            if isinstance(proj, ARCQPackedLinearOnTheFly) and proj.takes_reconstructed_input() and proj.group_size == 64:
+                xh = attention(qkv, B, T, self.num_heads, proj.activation_thresholds, proj.activation_codebook, proj.bits)
                 return proj(xh.reshape(B, T, C), pre_quantized=True)
-            return proj(ops.attention(qkv, B, T, self.num_heads).reshape(B, T, C))
+            return proj(attention(qkv, B, T, self.num_heads, None, None, 4).reshape(B, T, C))
         qkv = qkv.reshape(B, T, 3, self.num_heads, C // self.num_heads).permute(2, 0, 3, 1, 4)
         o = F.scaled_dot_product_attention(qkv[0], qkv[1], qkv[2])
         return self.proj(o.transpose(1, 2).reshape(B, T, C))
+
+
+def _replaces_library_attention(qkv: torch.Tensor, proj: nn.Module) -> bool:
+    """Whether the attention kernel stands for ``F.scaled_dot_product_attention``: between packed linears, where no gradient is
+    asked for, with the library function and the choice of its back ends as they come."""
+    b = torch.backends.cuda
+    return (type(proj) is ARCQPackedLinearOnTheFly and not (torch.is_grad_enabled() and qkv.requires_grad)
+            and F.scaled_dot_product_attention is _LIBRARY_ATTENTION
+            and b.flash_sdp_enabled() and b.mem_efficient_sdp_enabled() and b.math_sdp_enabled() and b.cudnn_sdp_enabled()
+            and not (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != torch.float16))
 
 
 class Mlp(nn.Module):

@@ -123,3 +123,22 @@ def test_attention_kernel_extreme_scores(pkg, cuda_device):
     assert torch.equal(got.isnan().any(1), want.isnan().any(1))
     assert torch.equal(got[4:T], out[4:T])
     assert pkg.ops.device_status() == 0
+
+
+def test_chosen_back_ends_are_kept(pkg, cuda_device):
+    """A program that chooses among the library's attention back ends gets the one it chose, alone or in the model's one call."""
+    gen = torch.Generator().manual_seed(14)
+    model = pkg.create_vit("deit_tiny", seed=3).half().to(cuda_device)
+    x = torch.randn(2, 3, 224, 224, generator=gen).half().to(cuda_device)
+    attn_cls = type(model.blocks[0].attn)
+    saved = attn_cls.implementation
+    try:
+        with torch.no_grad():
+            model = pkg.quantise_model(model, x, 4)
+            with torch.nn.attention.sdpa_kernel(torch.nn.attention.SDPBackend.MATH):
+                chosen = model(x).clone()
+                attn_cls.implementation = "sdpa"
+                want = model(x).clone()
+        assert torch.equal(chosen, want)
+    finally:
+        attn_cls.implementation = saved
