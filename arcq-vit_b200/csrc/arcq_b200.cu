@@ -717,12 +717,13 @@ bool small_layernorm_quant(long long M, long long K) {
 // one): its 12 epilogue warps hide latency worse than the quantizer kernel's 16, so it pays where the tiles are one round (DeiT-S
 // batch 6 / 8: 714 -> 676, 724 -> 679 us; DeiT-T batch 16: 656 -> 618) but not below five row tiles (DeiT-T batch 2: 449 ->
 // 463), where the products under it are long (DeiT-B batch 4: 874 -> 821 us) or where the matrix between the two no longer stays
-// in L2 (DeiT-S batch 128: 2722 -> 2618 us, DeiT-B: 7341 -> 6902); in between the rounds eat it (DeiT-S batch 64: 1540 -> 1588).
+// in L2 (DeiT-S batch 128: 2678 -> 2575 us, DeiT-B: 7341 -> 6902), and from some 6000 rows on (DeiT-T batch 37: 817 -> 789, 64: 952
+// -> 945, DeiT-S batch 32: 1029 -> 1016, 64: 1558 -> 1548); in between the rounds eat it (DeiT-S batch 16: 785 -> 804).
 bool choose_gelu_quant(long long M, long long N, long long K, PairDenseConfig* pc) {
   const int force = opt(O_GELU_GEMM);
   if (force == 0 || N % 64 != 0 || !choose_pair_quant_config(M, N, K, pc)) return false;
   const bool one_round = 1ll * pc->pairs * pc->bn >= (M + arcq::kPairTileM - 1) / arcq::kPairTileM * N;
-  return force > 0 || K >= 768 || M >= 20000 || (M > 1024 && one_round);
+  return force > 0 || K >= 768 || M >= 6000 || (M > 1024 && one_round);
 }
 
 }  // namespace
