@@ -266,14 +266,15 @@ def attention(qkv: torch.Tensor, batch: int, tokens: int, heads: int, thresholds
     if q2.shape[0] != batch * tokens:
         raise RuntimeError(f"qkv has {q2.shape[0]} rows, expected {batch} x {tokens}")
     out = torch.empty((batch * tokens, C), dtype=torch.float16, device=q2.device)
-    if thresholds is None:
-        rc = lib.arcq_attention(q2.data_ptr(), batch, tokens, heads, 64, out.data_ptr(), _stream())
-        _check(rc, "arcq_attention")
-    else:
+    if thresholds is not None:
         thresholds, codebook = _dev(thresholds, "thresholds", torch.float32), _dev(codebook, "codebook", torch.float32)
-        rc = lib.arcq_attention_act_quant(q2.data_ptr(), batch, tokens, heads, 64, thresholds.data_ptr(),
-                                          codebook.data_ptr(), bits, group_size, out.data_ptr(), _stream())
-        _check(rc, "arcq_attention_act_quant")
+    # stands in for an operator of the framework, which launches where its tensors are whatever the current device is
+    with torch.cuda.device(q2.device):
+        if thresholds is None:
+            _check(lib.arcq_attention(q2.data_ptr(), batch, tokens, heads, 64, out.data_ptr(), _stream()), "arcq_attention")
+        else:
+            _check(lib.arcq_attention_act_quant(q2.data_ptr(), batch, tokens, heads, 64, thresholds.data_ptr(), codebook.data_ptr(), bits,
+                                                group_size, out.data_ptr(), _stream()), "arcq_attention_act_quant")
     return out
 
 

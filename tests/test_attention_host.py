@@ -1,0 +1,32 @@
+"""What surrounds the attention kernel on the host, with a stand-in for the library: no GPU."""
+import contextlib
+import types
+
+import pytest
+import torch
+
+
+@pytest.mark.parametrize("quantise", [False, True])
+def test_attention_launches_on_the_device_of_its_tensors(pkg, monkeypatch, quantise):
+    """The stand-in records the device that is current when the kernel is launched and the one whose stream it is given."""
+    current, launches = ["the current device"], []
+
+    @contextlib.contextmanager
+    def device(d):
+        current.append(d)
+        yield
+        current.pop()
+
+    def launch(*args):
+        launches.append((current[-1], args[-1]))
+        return 0
+
+    ops = pkg.ops
+    monkeypatch.setattr(ops, "_dev", lambda t, *_: t.contiguous())
+    monkeypatch.setattr(ops, "_stream", lambda: ("stream of", current[-1]))
+    monkeypatch.setattr(ops._cabi, "load", lambda: types.SimpleNamespace(arcq_attention=launch, arcq_attention_act_quant=launch))
+    monkeypatch.setattr(torch.cuda, "device", device)
+    qkv = torch.zeros(2 * 5, 3 * 64, dtype=torch.float16)
+    out = ops.attention(qkv, 2, 5, 1, *((torch.zeros(15), torch.zeros(16)) if quantise else ()))
+    assert launches == [(qkv.device, ("stream of", qkv.device))] and current == ["the current device"]
+    assert out.shape == (10, 64)
