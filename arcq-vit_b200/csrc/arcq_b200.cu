@@ -1415,7 +1415,8 @@ int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const void
 
 static int launch_attention(const void* qkv, int64_t B, int64_t T, int64_t H, int head_dim, const float* thresholds,
                             const float* codebook, int bits, int one_fma, void* out, void* stream) {
-  if (qkv == nullptr || out == nullptr) return fail(ARCQ_E_BAD_ARG, "null pointer argument");
+  // (tensors of an empty batch have null pointers)
+  if (B != 0 && (qkv == nullptr || out == nullptr)) return fail(ARCQ_E_BAD_ARG, "null pointer argument");
   if (head_dim != 64) return fail(ARCQ_E_UNSUPPORTED, "head_dim %d: only 64 is built", head_dim);
   if (B < 0 || T <= 0 || H <= 0) return fail(ARCQ_E_BAD_SHAPE, "bad shape B=%lld T=%lld H=%lld", (long long)B, (long long)T, (long long)H);
   if (T > arcq::kAttnMaxT) return fail(ARCQ_E_TOO_LARGE, "sequences longer than %d tokens are not built", arcq::kAttnMaxT);

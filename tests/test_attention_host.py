@@ -30,3 +30,14 @@ def test_attention_launches_on_the_device_of_its_tensors(pkg, monkeypatch, quant
     out = ops.attention(qkv, 2, 5, 1, *((torch.zeros(15), torch.zeros(16)) if quantise else ()))
     assert launches == [(qkv.device, ("stream of", qkv.device))] and current == ["the current device"]
     assert out.shape == (10, 64)
+
+
+def test_an_empty_batch_is_nothing_to_do(pkg):
+    """Tensors of an empty batch have null pointers; null pointers of any other batch, and bad shapes of an empty one, are refused."""
+    lib, some = pkg._cabi.load(), 16
+    assert lib.arcq_attention(None, 0, 197, 3, 64, None, None) == 0
+    assert lib.arcq_attention_act_quant(None, 0, 197, 3, 64, some, some, 4, 64, None, None) == 0
+    for args in ((None, 1, 197, 3, 64, None, None), (some, 1, 197, 3, 64, None, None), (None, 0, 0, 3, 64, None, None),
+                 (None, 0, 257, 3, 64, None, None), (None, 0, 197, 3, 32, None, None)):
+        assert lib.arcq_attention(*args) < 0
+    assert lib.arcq_attention_act_quant(None, 0, 197, 3, 64, None, some, 4, 64, None, None) < 0

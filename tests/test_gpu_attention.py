@@ -142,3 +142,29 @@ def test_chosen_back_ends_are_kept(pkg, cuda_device):
         assert torch.equal(chosen, want)
     finally:
         attn_cls.implementation = saved
+
+
+def _block(pkg, dev, name="deit_tiny", bits=4):
+    """A packed block in a model of one, and input of its attention."""
+    model = pkg.create_vit(name, seed=3)
+    model.blocks = torch.nn.ModuleList(list(model.blocks)[:1])
+    model = model.half().to(dev)
+    gen = torch.Generator().manual_seed(14)
+    images = torch.randn(2, 3, 224, 224, generator=gen).half().to(dev)
+    with torch.no_grad():
+        model = pkg.quantise_model(model, images, bits)
+    return model, images, torch.randn(2, 197, model.embed_dim, generator=gen).half().to(dev)
+
+
+@pytest.mark.parametrize("name,bits", [("deit_small", 4), ("deit_tiny", 3)])      # proj takes a reconstruction, and does not
+@torch.no_grad()
+def test_attention_of_nothing(pkg, cuda_device, name, bits):
+    """No images, and no tokens."""
+    model, _, x = _block(pkg, cuda_device, name, bits)
+    attn = model.blocks[0].attn
+    for empty in (x[:0], x[:, :0]):
+        assert attn(empty).shape == empty.shape
+    C = 64 * model.num_heads
+    for quantizer in ((), (attn.proj.activation_thresholds, attn.proj.activation_codebook, bits)):
+        assert pkg.ops.attention(x.new_empty(0, 3 * C), 0, 197, model.num_heads, *quantizer).shape == (0, C)
+    assert pkg.ops.device_status() == 0
