@@ -71,7 +71,7 @@ def _replaces_library_attention(qkv: torch.Tensor, proj: nn.Module) -> bool:
     """Whether the attention kernel stands for ``F.scaled_dot_product_attention``: between packed linears, where no gradient is
     asked for, with the library function and the choice of its back ends as they come."""
     b = torch.backends.cuda
-    return (type(proj) is ARCQPackedLinearOnTheFly and qkv.numel() > 0 and not (torch.is_grad_enabled() and qkv.requires_grad)
+    return (type(proj) is ARCQPackedLinearOnTheFly and qkv.shape[1] > 0 and not (torch.is_grad_enabled() and qkv.requires_grad)
             and F.scaled_dot_product_attention is _LIBRARY_ATTENTION
             and b.flash_sdp_enabled() and b.mem_efficient_sdp_enabled() and b.math_sdp_enabled() and b.cudnn_sdp_enabled()
             and not (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != torch.float16))
