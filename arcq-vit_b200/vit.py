@@ -36,6 +36,7 @@ DEIT_CONFIGS: Dict[str, Tuple[int, int, int]] = {
 
 
 _LIBRARY_ATTENTION = F.scaled_dot_product_attention
+_PACKED_FORWARD = ARCQPackedLinearOnTheFly.forward
 
 
 class Attention(nn.Module):
@@ -58,7 +59,7 @@ class Attention(nn.Module):
                 and (self.implementation == "kernel" or self.implementation == "auto" and _replaces_library_attention(qkv, proj))):
             from . import ops  # noqa: F401  registers the operator
             attention = torch.ops.arcq.scaled_dot_product_attention
-            if isinstance(proj, ARCQPackedLinearOnTheFly) and proj.takes_reconstructed_input() and proj.group_size == 64:
+            if isinstance(proj, ARCQPackedLinearOnTheFly) and proj.takes_reconstructed_input() and _called_as_built(proj):
                 xh = attention(qkv, B, T, self.num_heads, proj.activation_thresholds, proj.activation_codebook, proj.bits)
                 return proj(xh.reshape(B, T, C), pre_quantized=True)
             return proj(attention(qkv, B, T, self.num_heads, None, None, 4).reshape(B, T, C))
@@ -75,6 +76,13 @@ def _replaces_library_attention(qkv: torch.Tensor, proj: nn.Module) -> bool:
             and F.scaled_dot_product_attention is _LIBRARY_ATTENTION
             and b.flash_sdp_enabled() and b.mem_efficient_sdp_enabled() and b.math_sdp_enabled() and b.cudnn_sdp_enabled()
             and not (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != torch.float16))
+
+
+def _called_as_built(proj: ARCQPackedLinearOnTheFly) -> bool:
+    """Nothing sees what proj is given but its own forward: hooks and a forward of somebody else's get the attention output and no
+    argument beside it, whose quantisation inside proj gives the same bits."""
+    return not (proj._forward_hooks or proj._forward_pre_hooks or _has_global_hooks() or "forward" in proj.__dict__
+                or proj._compiled_call_impl is not None) and type(proj).forward is _PACKED_FORWARD
 
 
 class Mlp(nn.Module):

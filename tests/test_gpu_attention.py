@@ -168,3 +168,43 @@ def test_attention_of_nothing(pkg, cuda_device, name, bits):
     for quantizer in ((), (attn.proj.activation_thresholds, attn.proj.activation_codebook, bits)):
         assert pkg.ops.attention(x.new_empty(0, 3 * C), 0, 197, model.num_heads, *quantizer).shape == (0, C)
     assert pkg.ops.device_status() == 0
+
+
+def _pre_hook(proj, seen, monkeypatch):
+    proj.register_forward_pre_hook(lambda m, args, kwargs: seen.append((args, kwargs)), with_kwargs=True)
+
+
+def _hook(proj, seen, monkeypatch):
+    proj.register_forward_hook(lambda m, args, kwargs, y: seen.append((args, kwargs)), with_kwargs=True)
+
+
+def _global_pre_hook(proj, seen, monkeypatch):
+    module = torch.nn.modules.module
+    monkeypatch.setattr(module, "_global_forward_pre_hooks", {0: lambda m, args: seen.append((args, {})) if m is proj else None})
+
+
+def _own_forward(proj, seen, monkeypatch):
+    proj.forward = lambda x: seen.append(((x,), {})) or type(proj).forward(proj, x)
+
+
+def _class_forward(proj, seen, monkeypatch):
+    forward = type(proj).forward
+    monkeypatch.setattr(type(proj), "forward", lambda self, x: (seen.append(((x,), {})) if self is proj else None) or forward(self, x))
+
+
+@pytest.mark.parametrize("watch", [_pre_hook, _hook, _global_pre_hook, _own_forward, _class_forward])
+@torch.no_grad()
+def test_what_watches_proj_sees_the_attention_output(pkg, cuda_device, watch, monkeypatch):
+    """Hooks on proj, and a forward of its own that takes x only, get what the attention gives and nothing else; same bits."""
+    model, images, x = _block(pkg, cuda_device)
+    attn = model.blocks[0].attn
+    want, seen = attn(x), []
+    qkv = attn.qkv(x)
+    watch(attn.proj, seen, monkeypatch)
+    assert torch.equal(attn(x), want)
+    (given,), kwargs = seen.pop()
+    assert not kwargs and not seen
+    C = 64 * model.num_heads
+    assert torch.equal(given.reshape(-1, C), pkg.ops.attention(qkv.reshape(-1, 3 * C), 2, 197, model.num_heads))
+    error = (given.reshape(-1, C).double() - _fp64(qkv.reshape(-1, 3 * C), 2, 197, model.num_heads)).abs().max()
+    assert float(error) <= 2.0 ** -10 * float(qkv.abs().max())         # P and the output rounded to fp16
