@@ -268,7 +268,7 @@ def attention(qkv: torch.Tensor, batch: int, tokens: int, heads: int, thresholds
     out = torch.empty((batch * tokens, C), dtype=torch.float16, device=q2.device)
     if thresholds is not None:
         thresholds, codebook = _dev(thresholds, "thresholds", torch.float32), _dev(codebook, "codebook", torch.float32)
-    # stands in for an operator of the framework, which launches where its tensors are whatever the current device is
+    # like an operator of the framework, which launches where its tensors are whatever the current device is
     with torch.cuda.device(q2.device):
         if thresholds is None:
             _check(lib.arcq_attention(q2.data_ptr(), batch, tokens, heads, 64, out.data_ptr(), _stream()), "arcq_attention")
@@ -276,21 +276,6 @@ def attention(qkv: torch.Tensor, batch: int, tokens: int, heads: int, thresholds
             _check(lib.arcq_attention_act_quant(q2.data_ptr(), batch, tokens, heads, 64, thresholds.data_ptr(), codebook.data_ptr(), bits,
                                                 group_size, out.data_ptr(), _stream()), "arcq_attention_act_quant")
     return out
-
-
-# The same as an operator of the framework, for callers inside a model: function and dispatch modes see it by the name of what it
-# stands for, tensor subclasses are unwrapped as for any other operator.  No gradient.
-if not hasattr(torch.ops.arcq, "scaled_dot_product_attention"):
-    torch.library.define("arcq::scaled_dot_product_attention",
-                         "(Tensor qkv, int batch, int tokens, int heads, Tensor? thresholds, Tensor? codebook, int bits) -> Tensor")
-
-    @torch.library.impl("arcq::scaled_dot_product_attention", "cuda")
-    def _attention_op(qkv, batch, tokens, heads, thresholds, codebook, bits):
-        return attention(qkv, batch, tokens, heads, thresholds, codebook, bits)
-
-    @torch.library.register_fake("arcq::scaled_dot_product_attention")
-    def _attention_shape(qkv, batch, tokens, heads, thresholds, codebook, bits):
-        return qkv.new_empty((batch * tokens, heads * 64))
 
 
 def patchify(images: torch.Tensor, patch: int) -> torch.Tensor:

@@ -21,6 +21,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 from torch.overrides import _get_current_function_mode_stack
 from torch.utils._device import DeviceContext
+from torch.utils._mode_utils import no_dispatch
 
 from . import _cabi
 from . import codebook as cbk
@@ -54,25 +55,61 @@ class Attention(nn.Module):
     def forward(self, x: torch.Tensor, pre_quantized: bool = False) -> torch.Tensor:
         B, T, C = x.shape
         qkv = self.qkv(x, pre_quantized=True) if pre_quantized else self.qkv(x)
-        proj = self.proj
-        if (qkv.is_cuda and qkv.dtype == torch.float16 and C == 64 * self.num_heads and T <= 256
-                and (self.implementation == "kernel" or self.implementation == "auto" and _replaces_library_attention(qkv, proj))):
-            from . import ops  # noqa: F401  registers the operator
-            attention = torch.ops.arcq.scaled_dot_product_attention
+        proj, heads = self.proj, self.num_heads
+        own = (qkv.is_cuda and qkv.dtype == torch.float16 and C == 64 * heads and T <= 256
+               and (self.implementation == "kernel" or self.implementation == "auto" and _replaces_library_attention(qkv, proj)))
+        shown = own and self.implementation == "auto" and _under_a_mode()
+        if own and not shown:
+            from . import ops
             if isinstance(proj, ARCQPackedLinearOnTheFly) and proj.takes_reconstructed_input() and _called_as_built(proj):
-                xh = attention(qkv, B, T, self.num_heads, proj.activation_thresholds, proj.activation_codebook, proj.bits)
+                xh = ops.attention(qkv, B, T, heads, proj.activation_thresholds, proj.activation_codebook, proj.bits, proj.group_size)
                 return proj(xh.reshape(B, T, C), pre_quantized=True)
-            return proj(attention(qkv, B, T, self.num_heads, None, None, 4).reshape(B, T, C))
-        qkv = qkv.reshape(B, T, 3, self.num_heads, C // self.num_heads).permute(2, 0, 3, 1, 4)
-        o = F.scaled_dot_product_attention(qkv[0], qkv[1], qkv[2])
-        return self.proj(o.transpose(1, 2).reshape(B, T, C))
+            return proj(ops.attention(qkv, B, T, heads).reshape(B, T, C))
+        r = qkv.reshape(B, T, 3, heads, C // heads).permute(2, 0, 3, 1, 4)
+        q, k, v = r[0], r[1], r[2]
+        if shown:
+            q, k, v = _ShownOperand.three(qkv, q, k, v)
+        return proj(F.scaled_dot_product_attention(q, k, v).transpose(1, 2).reshape(B, T, C))
+
+
+class _ShownOperand(torch.Tensor):
+    """q, k or v under a function or dispatch mode: the mode sees the library's function, or its operator, called with these three.
+    What it lets through gives the kernel's result, the bits that the forward has without the mode; what it does itself with the
+    tensors is done on plain ones."""
+
+    __torch_function__ = torch._C._disabled_torch_function_impl
+
+    @classmethod
+    def three(cls, qkv: torch.Tensor, *qkv_views: torch.Tensor):
+        with torch._C.DisableTorchFunction(), no_dispatch():
+            made = [torch.Tensor._make_subclass(cls, t) for t in qkv_views]
+        for i, t in enumerate(made):
+            t.role = (qkv, i)
+        return made
+
+    @classmethod
+    def __torch_dispatch__(cls, func, types, args=(), kwargs=None):
+        kwargs = kwargs or {}
+        with no_dispatch():
+            y = func(*args, **kwargs)
+            roles = [getattr(t, "role", (None, -1)) for t in args[:3]] if "scaled_dot_product" in func.name() else []
+            qkv = roles[0][0] if roles else None
+            # this layer's three in their places, with no mask, not causal and no scale given
+            if (len(roles) == 3 and all(r[0] is qkv is not None and r[1] == i for i, r in enumerate(roles))
+                    and all(a is None or isinstance(a, (bool, int, float)) and not a for a in (*args[3:], *kwargs.values()))):
+                from . import ops
+                B, H, T, W = args[0].shape
+                out = y if isinstance(y, torch.Tensor) else y[0]
+                out.copy_(ops.attention(qkv, B, T, H).reshape(B, T, H, W).transpose(1, 2))
+        return y
 
 
 def _replaces_library_attention(qkv: torch.Tensor, proj: nn.Module) -> bool:
     """Whether the attention kernel stands for ``F.scaled_dot_product_attention``: between packed linears, where no gradient is
     asked for, with the library function and the choice of its back ends as they come."""
     b = torch.backends.cuda
-    return (type(proj) is ARCQPackedLinearOnTheFly and qkv.shape[1] > 0 and not (torch.is_grad_enabled() and qkv.requires_grad)
+    return (type(qkv) is torch.Tensor and type(proj) is ARCQPackedLinearOnTheFly and qkv.shape[1] > 0
+            and not (torch.is_grad_enabled() and qkv.requires_grad)
             and F.scaled_dot_product_attention is _LIBRARY_ATTENTION
             and b.flash_sdp_enabled() and b.mem_efficient_sdp_enabled() and b.math_sdp_enabled() and b.cudnn_sdp_enabled()
             and not (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != torch.float16))

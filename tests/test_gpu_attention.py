@@ -208,3 +208,56 @@ def test_what_watches_proj_sees_the_attention_output(pkg, cuda_device, watch, mo
     assert torch.equal(given.reshape(-1, C), pkg.ops.attention(qkv.reshape(-1, 3 * C), 2, 197, model.num_heads))
     error = (given.reshape(-1, C).double() - _fp64(qkv.reshape(-1, 3 * C), 2, 197, model.num_heads)).abs().max()
     assert float(error) <= 2.0 ** -10 * float(qkv.abs().max())         # P and the output rounded to fp16
+
+
+class _OnAttention(torch.overrides.TorchFunctionMode):
+    """A function mode that knows the library's attention by identity and puts something in its place."""
+
+    def __init__(self, instead):
+        super().__init__()
+        self.calls, self.instead = 0, instead
+
+    def __torch_function__(self, func, types, args=(), kwargs=None):
+        if func is F.scaled_dot_product_attention:
+            self.calls += 1
+            return self.instead(*args, **(kwargs or {}))
+        return func(*args, **(kwargs or {}))
+
+
+@pytest.mark.parametrize("whole", [False, True])                   # the attention module, the model
+@torch.no_grad()
+def test_a_function_mode_sees_and_replaces_the_attention(pkg, cuda_device, whole, monkeypatch):
+    model, images, x = _block(pkg, cuda_device)
+    call = (lambda: model(images)) if whole else (lambda: model.blocks[0].attn(x))
+    want = call()
+    sdpa = F.scaled_dot_product_attention
+    with _OnAttention(sdpa) as seen:
+        assert torch.equal(call(), want) and seen.calls == 1
+    cls = type(model.blocks[0].attn)
+    for instead in (lambda q, k, v: torch.zeros_like(q), lambda q, k, v: sdpa(q, k, v, is_causal=True), lambda q, k, v: sdpa(q, k, q),
+                    lambda q, k, v: sdpa(q, k, v, scale=0.5), lambda q, k, v: torch.softmax(q @ k.transpose(-1, -2) / 8, -1) @ v):
+        results = []
+        for implementation in ("auto", "sdpa"):
+            monkeypatch.setattr(cls, "implementation", implementation)
+            with _OnAttention(instead) as seen:
+                results.append(call())
+            assert seen.calls == 1
+        assert torch.equal(*results) and not torch.equal(results[0], want)
+    assert pkg.ops.device_status() == 0
+
+
+@torch.no_grad()
+def test_a_dispatch_mode_sees_the_attention_operator(pkg, cuda_device):
+    """By the framework's own name: its counter of operations knows it.  Same bits, also in inference mode."""
+    from torch.utils.flop_counter import FlopCounterMode
+    model, _, x = _block(pkg, cuda_device)
+    attn = model.blocks[0].attn
+    want = attn(x)
+    with FlopCounterMode(display=False) as counter:
+        assert torch.equal(attn(x), want)
+    assert counter.get_total_flops() == 4 * 2 * model.num_heads * 197 * 197 * 64
+    with torch.inference_mode(), FlopCounterMode(display=False):
+        assert torch.equal(attn(x), want)
+    with torch.autocast("cuda", torch.float16), FlopCounterMode(display=False):
+        assert torch.equal(attn(x), want)
+    assert pkg.ops.device_status() == 0
