@@ -18,6 +18,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <array>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -265,6 +266,22 @@ PyObject* dequant(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return THPVariable_Wrap(std::move(out));
 }
 
+// ---------------------------------------------------------------- the library's attention
+// Whether nothing was chosen about it: all back ends allowed, in the order that the framework starts with or in the one that its first
+// call puts there on a GPU whose cuDNN it prefers.
+bool back_ends_as_they_come() {
+  using B = at::SDPBackend;
+  using Order = std::array<B, at::num_sdp_backends>;
+  constexpr Order first = {B::flash_attention, B::efficient_attention, B::math, B::cudnn_attention, B::overrideable};
+  constexpr Order later = {B::cudnn_attention, B::flash_attention, B::efficient_attention, B::math, B::overrideable};
+  at::Context& ctx = at::globalContext();
+  const Order order = ctx.sDPPriorityOrder();
+  return ctx.userEnabledFlashSDP() && ctx.userEnabledMemEfficientSDP() && ctx.userEnabledMathSDP() && ctx.userEnabledCuDNNSDP() &&
+         (order == first || order == later);
+}
+// attention_back_ends_as_they_come() -> bool
+PyObject* attention_back_ends_as_they_come(PyObject*, PyObject* const*, Py_ssize_t) { return PyBool_FromLong(back_ends_as_they_come()); }
+
 // ---------------------------------------------------------------- the forward of a packed ViT
 // The data of a framework operator's fp16 result, which the kernels read as a dense matrix.
 const void* half_matrix(const at::Tensor& t, int64_t elems, const c10::Device& dev) {
@@ -421,9 +438,7 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
   // The attention kernel, which also quantises for proj, instead of the library's attention and a quantizer launch: a whole forward
   // of DeiT-S batch 64 1611 -> 1559 us, batch 8 786 -> 749, batch 1 equal, DeiT-T batch 37 867 -> 823, DeiT-B batch 1024 58.9 -> 57.7
   // ms.  The library's where a sequence is too long for the kernel, and where its back ends were chosen among.
-  const at::Context& ctx = at::globalContext();
-  const bool own_attention = T <= 256 && D == 64 * p->heads && ctx.userEnabledFlashSDP() && ctx.userEnabledMemEfficientSDP() &&
-                             ctx.userEnabledMathSDP() && ctx.userEnabledCuDNNSDP();
+  const bool own_attention = T <= 256 && D == 64 * p->heads && back_ends_as_they_come();
   int64_t hidden = 0;
   for (size_t i = 0; i < depth; ++i) hidden = std::max(hidden, lin[4 * i + 2].N);
 
@@ -564,7 +579,7 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
 PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {
-  if (F != &vit_plan && c10::impl::TorchDispatchModeTLS::any_modes_set()) Py_RETURN_NONE;      // the mode wants to see the operators
+  if (F != &vit_plan && F != &attention_back_ends_as_they_come && c10::impl::TorchDispatchModeTLS::any_modes_set()) Py_RETURN_NONE;      // the mode wants to see the operators
   try {
     return F(self, args, n);
   } catch (const c10::OutOfMemoryError& e) {
@@ -577,7 +592,7 @@ PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {
 }
 #define ARCQ_METHOD(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&guarded<f>)), METH_FASTCALL, nullptr}
 PyMethodDef g_methods[] = {ARCQ_METHOD(linear), ARCQ_METHOD(quantize_activation), ARCQ_METHOD(dequant), ARCQ_METHOD(vit_plan),
-                           ARCQ_METHOD(vit_forward), {nullptr, nullptr, 0, nullptr}};
+                           ARCQ_METHOD(vit_forward), ARCQ_METHOD(attention_back_ends_as_they_come), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_arcq_host", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

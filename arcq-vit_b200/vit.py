@@ -36,7 +36,7 @@ DEIT_CONFIGS: Dict[str, Tuple[int, int, int]] = {
 }
 
 
-_LIBRARY_ATTENTION = F.scaled_dot_product_attention
+_LIBRARY_ATTENTION = torch._C._nn.scaled_dot_product_attention      # what F has unless somebody put another function there
 _PACKED_FORWARD = ARCQPackedLinearOnTheFly.forward
 
 
@@ -107,11 +107,9 @@ class _ShownOperand(torch.Tensor):
 def _replaces_library_attention(qkv: torch.Tensor, proj: nn.Module) -> bool:
     """Whether the attention kernel stands for ``F.scaled_dot_product_attention``: between packed linears, where no gradient is
     asked for, with the library function and the choice of its back ends as they come."""
-    b = torch.backends.cuda
     return (type(qkv) is torch.Tensor and type(proj) is ARCQPackedLinearOnTheFly and qkv.shape[1] > 0
             and not (torch.is_grad_enabled() and qkv.requires_grad)
-            and F.scaled_dot_product_attention is _LIBRARY_ATTENTION
-            and b.flash_sdp_enabled() and b.mem_efficient_sdp_enabled() and b.math_sdp_enabled() and b.cudnn_sdp_enabled()
+            and F.scaled_dot_product_attention is _LIBRARY_ATTENTION and _cabi.host().attention_back_ends_as_they_come()
             and not (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != torch.float16))
 
 
@@ -275,7 +273,7 @@ def _has_global_hooks() -> bool:
 # the Python code that a native forward stands for: replaced on its class or module, it is called as before
 _STANDS_FOR = tuple((c, n, getattr(c, n)) for c, n in (
     (PatchEmbed, "forward"), (Attention, "forward"), (Mlp, "forward"), (ARCQPackedLinearOnTheFly, "forward"), (nn.Linear, "forward"),
-    (VisionTransformer, "_forward_fused_glue"), (F, "linear"), (F, "scaled_dot_product_attention")))
+    (VisionTransformer, "_forward_fused_glue"), (F, "linear"))) + ((F, "scaled_dot_product_attention", _LIBRARY_ATTENTION),)
 
 
 class _NotNative(Exception):

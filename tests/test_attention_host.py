@@ -1,9 +1,14 @@
 """What surrounds the attention kernel on the host, with a stand-in for the library: no GPU."""
 import contextlib
+import subprocess
+import sys
 import types
 
 import pytest
 import torch
+from torch.nn.attention import SDPBackend, sdpa_kernel
+
+from conftest import ROOT
 
 
 @pytest.mark.parametrize("quantise", [False, True])
@@ -41,3 +46,37 @@ def test_an_empty_batch_is_nothing_to_do(pkg):
                  (None, 0, 257, 3, 64, None, None), (None, 0, 197, 3, 32, None, None)):
         assert lib.arcq_attention(*args) < 0
     assert lib.arcq_attention_act_quant(None, 0, 197, 3, 64, None, some, 4, 64, None, None) < 0
+
+
+def test_a_choice_among_the_librarys_back_ends_is_noticed(pkg):
+    """A back end left out, or all of them in an order of the program's own."""
+    untouched = pkg._cabi.host().attention_back_ends_as_they_come
+    every = [SDPBackend.FLASH_ATTENTION, SDPBackend.EFFICIENT_ATTENTION, SDPBackend.MATH, SDPBackend.CUDNN_ATTENTION]
+    assert untouched()
+    for i in range(4):
+        with sdpa_kernel(every[:i] + every[i + 1:]):
+            assert not untouched()
+    with sdpa_kernel(every[::-1], set_priority=True):
+        assert not untouched()
+    with sdpa_kernel(every):
+        assert untouched()
+    with sdpa_kernel(every[3:] + every[:3], set_priority=True):     # the framework's own once cuDNN is preferred
+        assert untouched()
+    assert untouched()
+
+
+def test_an_attention_put_in_the_librarys_place_before_the_import_is_noticed():
+    """By the attention module and by the native forward, whose reasons not to run are looked at in this order."""
+    code = """
+import sys; sys.path.insert(0, '.')
+import torch, torch.nn.functional as F
+library = F.scaled_dot_product_attention
+F.scaled_dot_product_attention = lambda *a, **k: library(*a, **k)
+import __graft_entry__ as entry
+vit = entry.import_package().vit
+def differs(): return [n for c, n, f in vit._STANDS_FOR if getattr(c, n) is not f], F.scaled_dot_product_attention is vit._LIBRARY_ATTENTION
+assert differs() == (['scaled_dot_product_attention'], False), differs()
+F.scaled_dot_product_attention = library
+assert differs() == ([], True), differs()
+"""
+    subprocess.run([sys.executable, "-c", code], cwd=ROOT, check=True)

@@ -261,3 +261,23 @@ def test_a_dispatch_mode_sees_the_attention_operator(pkg, cuda_device):
     with torch.autocast("cuda", torch.float16), FlopCounterMode(display=False):
         assert torch.equal(attn(x), want)
     assert pkg.ops.device_status() == 0
+
+
+@pytest.mark.parametrize("native", [True, False])
+@torch.no_grad()
+def test_a_set_order_of_the_back_ends_is_kept(pkg, cuda_device, native, monkeypatch):
+    """All four back ends, the slowest first: the library's attention runs, in the model's one call and in the attention module."""
+    from torch.nn.attention import SDPBackend, sdpa_kernel
+    model, images, _ = _block(pkg, cuda_device)
+    if not native:
+        monkeypatch.setattr(pkg.vit.VisionTransformer, "_forward_native", lambda self, x: None)
+    own = model(images)
+    monkeypatch.setattr(type(model.blocks[0].attn), "implementation", "kernel")
+    assert torch.equal(model(images), own)                      # the library has run by now, in the calibration
+    monkeypatch.setattr(type(model.blocks[0].attn), "implementation", "auto")
+    order = [SDPBackend.MATH, SDPBackend.EFFICIENT_ATTENTION, SDPBackend.FLASH_ATTENTION, SDPBackend.CUDNN_ATTENTION]
+    with sdpa_kernel(order, set_priority=True):
+        chosen = model(images)
+        monkeypatch.setattr(type(model.blocks[0].attn), "implementation", "sdpa")
+        assert torch.equal(chosen, model(images)) and not torch.equal(chosen, own)
+    assert pkg.ops.device_status() == 0
