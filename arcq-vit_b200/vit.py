@@ -56,8 +56,8 @@ class Attention(nn.Module):
         B, T, C = x.shape
         qkv = self.qkv(x, pre_quantized=True) if pre_quantized else self.qkv(x)
         proj, heads = self.proj, self.num_heads
-        own = (qkv.is_cuda and qkv.dtype == torch.float16 and C == 64 * heads and T <= 256
-               and (self.implementation == "kernel" or self.implementation == "auto" and _replaces_library_attention(qkv, proj)))
+        own = _replaces_library_attention(qkv, proj, T, C, heads) if self.implementation == "auto" else (
+            self.implementation == "kernel" and _kernel_takes(qkv, T, C, heads))
         shown = own and self.implementation == "auto" and _under_a_mode()
         if own and not shown:
             from . import ops
@@ -104,11 +104,16 @@ class _ShownOperand(torch.Tensor):
         return y
 
 
-def _replaces_library_attention(qkv: torch.Tensor, proj: nn.Module) -> bool:
+def _kernel_takes(qkv: torch.Tensor, tokens: int, dim: int, heads: int) -> bool:
+    return qkv.is_cuda and qkv.dtype == torch.float16 and dim == 64 * heads and tokens <= 256
+
+
+def _replaces_library_attention(qkv: torch.Tensor, proj: nn.Module, tokens: int, dim: int, heads: int) -> bool:
     """Whether the attention kernel stands for ``F.scaled_dot_product_attention``: between packed linears, where no gradient is
-    asked for, with the library function and the choice of its back ends as they come."""
-    return (type(qkv) is torch.Tensor and type(proj) is ARCQPackedLinearOnTheFly and qkv.shape[1] > 0
-            and not (torch.is_grad_enabled() and qkv.requires_grad)
+    asked for, with the library function and the choice of its back ends as they come.  Not where a graph of operators is being
+    made, nor for tensors of other classes (an fx proxy among them, asked nothing but its type)."""
+    return (type(qkv) is torch.Tensor and not torch.compiler.is_compiling() and type(proj) is ARCQPackedLinearOnTheFly
+            and _kernel_takes(qkv, tokens, dim, heads) and tokens > 0 and not (torch.is_grad_enabled() and qkv.requires_grad)
             and F.scaled_dot_product_attention is _LIBRARY_ATTENTION and _cabi.host().attention_back_ends_as_they_come()
             and not (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != torch.float16))
 

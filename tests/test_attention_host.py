@@ -80,3 +80,12 @@ F.scaled_dot_product_attention = library
 assert differs() == ([], True), differs()
 """
     subprocess.run([sys.executable, "-c", code], cwd=ROOT, check=True)
+
+
+def test_a_block_can_be_traced_symbolically(pkg):
+    """A tracer's proxies are asked nothing that has no answer yet."""
+    block = pkg.vit.Block(128, 2)
+    x = torch.randn(2, 5, 128, generator=torch.Generator().manual_seed(1))
+    graph = torch.fx.symbolic_trace(block)
+    assert any(n.target is torch.nn.functional.scaled_dot_product_attention for n in graph.graph.nodes)
+    assert torch.equal(graph(x), block(x))

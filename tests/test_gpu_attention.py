@@ -281,3 +281,13 @@ def test_a_set_order_of_the_back_ends_is_kept(pkg, cuda_device, native, monkeypa
         monkeypatch.setattr(type(model.blocks[0].attn), "implementation", "sdpa")
         assert torch.equal(chosen, model(images)) and not torch.equal(chosen, own)
     assert pkg.ops.device_status() == 0
+
+
+@torch.no_grad()
+def test_a_graph_of_operators_has_the_librarys_attention(pkg, cuda_device, monkeypatch):
+    model, _, x = _block(pkg, cuda_device)
+    attn = model.blocks[0].attn
+    got = torch.compile(attn, backend="eager")(x)
+    monkeypatch.setattr(type(attn), "implementation", "sdpa")
+    assert torch.equal(got, attn(x))
+    assert pkg.ops.device_status() == 0
