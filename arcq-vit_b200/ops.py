@@ -265,6 +265,8 @@ def attention(qkv: torch.Tensor, batch: int, tokens: int, heads: int, thresholds
     q2 = _dev(qkv.reshape(-1, 3 * C), "qkv", torch.float16)
     if q2.shape[0] != batch * tokens:
         raise RuntimeError(f"qkv has {q2.shape[0]} rows, expected {batch} x {tokens}")
+    if q2.data_ptr() % 16 != 0:                 # what a hook on the qkv linear gives back, say
+        q2 = q2.clone()
     out = torch.empty((batch * tokens, C), dtype=torch.float16, device=q2.device)
     if thresholds is not None:
         thresholds, codebook = _dev(thresholds, "thresholds", torch.float32), _dev(codebook, "codebook", torch.float32)

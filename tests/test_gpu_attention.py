@@ -284,6 +284,26 @@ def test_a_set_order_of_the_back_ends_is_kept(pkg, cuda_device, native, monkeypa
 
 
 @torch.no_grad()
+def test_qkv_that_the_kernel_cannot_read_in_place(pkg, cuda_device):
+    """A hook that gives back qkv two bytes off, and one with a gap between its rows: read from a copy, same bits."""
+    model, _, x = _block(pkg, cuda_device)
+    attn = model.blocks[0].attn
+    want = attn(x)
+
+    def off(m, args, y):
+        return torch.empty(y.numel() + 1, dtype=y.dtype, device=y.device)[1:].reshape(y.shape).copy_(y)
+
+    def gap(m, args, y):
+        return torch.empty(*y.shape[:-1], y.shape[-1] + 3, dtype=y.dtype, device=y.device)[..., :-3].copy_(y)
+
+    for hook in (off, gap):
+        handle = attn.qkv.register_forward_hook(hook)
+        assert torch.equal(attn(x), want)
+        handle.remove()
+    assert pkg.ops.device_status() == 0
+
+
+@torch.no_grad()
 def test_a_graph_of_operators_has_the_librarys_attention(pkg, cuda_device, monkeypatch):
     model, _, x = _block(pkg, cuda_device)
     attn = model.blocks[0].attn
