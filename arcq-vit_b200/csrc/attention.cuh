@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
       tc_fence_after_sync();
       uint32_t w[32];
       if (live) {
-        const float inv = __fdividef(1.0f, s_sums[quarter * 32 + lane]);
+        const float inv = __frcp_rn(s_sums[quarter * 32 + lane]);
         const f32x2 inv2 = pack2(inv, inv);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {

@@ -311,3 +311,19 @@ def test_a_graph_of_operators_has_the_librarys_attention(pkg, cuda_device, monke
     monkeypatch.setattr(type(attn), "implementation", "sdpa")
     assert torch.equal(got, attn(x))
     assert pkg.ops.device_status() == 0
+
+
+def test_probabilities_are_divided_by_a_correctly_rounded_sum(pkg, cuda_device):
+    """Equal scores: every probability before the division is one and the sum is T.  The values are halfway between two fp16 numbers
+    times T, in two summands that fp16 holds, so which way an output is rounded depends on the last bit of 1 / T in fp32."""
+    gen = torch.Generator().manual_seed(3)
+    for T in range(2, 257):
+        half = (2048 + 2 * torch.randint(0, 1024, (64,), generator=gen) + 1).float() / 2048       # twelve bits, in [1, 2)
+        qkv = torch.zeros(T, 192)
+        qkv[0, 128:] = (half * T).half().float()
+        qkv[1, 128:] = half * T - qkv[0, 128:]
+        assert torch.equal(qkv.half().float(), qkv)
+        want = ((half * T) * torch.tensor(T, dtype=torch.float32).reciprocal()).half()
+        got = pkg.ops.attention(qkv.half().to(cuda_device), 1, T, 1).cpu()
+        assert torch.equal(got, want.expand(T, 64)), T
+    assert pkg.ops.device_status() == 0
