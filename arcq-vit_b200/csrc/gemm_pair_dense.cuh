@@ -167,112 +167,118 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
   const uint32_t tmem_base = *s_tmem;
   bool ok = true;
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA: this CTA's half of every stage
+  if (warp < kIssue) {
+    // One instruction that the whole warp group executes, before its warps part: two issue, two (of the quantizer form) have nothing
+    // to do.  (None in the plain form, not even where nothing gets to it: 2 to 8 % slower.)  The loops over the sub-tiles of a stage
+    // stay loops: unrolled they spill in 56 registers (12608 rows, K = 768, N = 3072 99.0 us against 95.6) and cost the plain form 1 to
+    // 3 % too (3001 rows, K = 384, N = 1536 8.1 against 7.8 us).
     if constexpr (QBITS != 0) fewer_registers<kPairQuantIssueRegs>();
-    const uint32_t sa = p.sa;
-    const uint32_t full_leader = mapa_shared(full, 0);
-    const uint32_t st0 = smem_u32(sStages);
-    uint32_t slot = 0, ph = 1;     // "empty" barriers: the first pass is free
-    uint32_t good = 1;
-    // Both operands are other kernels' outputs (the activation quantizer's and the weight unpack's).
-    pdl_wait();
-    if (STATIONARY && my_tiles > 0) {
-      // the whole slab, once; its sub-tiles land while the first A stages do
-      if (elect_one()) {
-        const uint32_t slab_leader = mapa_shared(slab_full, 0);
-        const uint32_t sl0 = smem_u32(sSlab);
-        for (int g = 0; g < G; ++g) {
-          if (crank == 0) mbar_expect_tx(slab_full + g * 8, 2u * wtile_bytes);
-          tma_load_2d_pair(sl0 + g * wtile_bytes, &tm_w, slab_leader + g * 8, g * 64, nh0);
-        }
-      }
-      __syncwarp();
-    }
-    for (int t = 0; t < my_tiles; ++t) {
-      const int row0 = row_of(t);
-      for (int g0 = 0; g0 < G; g0 += ks) {
-        good &= mbar_park_flag(empty + slot * 8, ph, good ? poll_limit : 0u);
+    if (warp == 0) {
+      // ------------------------------------------------------------------ TMA: this CTA's half of every stage
+      const uint32_t sa = p.sa;
+      const uint32_t full_leader = mapa_shared(full, 0);
+      const uint32_t st0 = smem_u32(sStages);
+      uint32_t slot = 0, ph = 1;     // "empty" barriers: the first pass is free
+      uint32_t good = 1;
+      // Both operands are other kernels' outputs (the activation quantizer's and the weight unpack's).
+      pdl_wait();
+      if (STATIONARY && my_tiles > 0) {
+        // the whole slab, once; its sub-tiles land while the first A stages do
         if (elect_one()) {
-          if (good) {
-            if (crank == 0) mbar_expect_tx(full + slot * 8, 2u * stage_bytes);
-            const uint32_t dst = st0 + slot * stage_bytes;
-            for (int q = 0; q < ks; ++q)
-              tma_load_2d_pair(dst + q * kStageA, &tm_a, full_leader + slot * 8, (g0 + q) * 64, row0);
-            if (!STATIONARY)
-              for (int q = 0; q < ks; ++q)
-                tma_load_2d_pair(dst + ks * kStageA + q * wtile_bytes, &tm_w, full_leader + slot * 8, (g0 + q) * 64, nh0);
+          const uint32_t slab_leader = mapa_shared(slab_full, 0);
+          const uint32_t sl0 = smem_u32(sSlab);
+          for (int g = 0; g < G; ++g) {
+            if (crank == 0) mbar_expect_tx(slab_full + g * 8, 2u * wtile_bytes);
+            tma_load_2d_pair(sl0 + g * wtile_bytes, &tm_w, slab_leader + g * 8, g * 64, nh0);
           }
         }
         __syncwarp();
-        if (++slot == sa) { slot = 0; ph ^= 1; }
       }
-      if (__any_sync(0xffffffffu, good == 0)) break;
-    }
-    ok = __all_sync(0xffffffffu, good != 0);
-    if (!ok) {
-      // give copies that are still in flight time to land before this CTA's shared memory goes away
-      for (int i = 0; i < 64; ++i) __nanosleep(1000);
-      if (lane == 0) atomicExch(p.status, kStatusPairTimeout);
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issue (leader CTA only)
-    if constexpr (QBITS != 0) fewer_registers<kPairQuantIssueRegs>();
-    if (crank == 0 && my_tiles > 0) {
-      const uint32_t idesc = umma_idesc_f16(kPairTileM, bn);
-      const uint32_t sa = p.sa;
-      const uint32_t lo0 = ((smem_u32(sStages) & 0x3FFFFu) >> 4) | (1u << 16);
-      const uint32_t s_step = stage_bytes >> 4, w_off = (static_cast<uint32_t>(ks) * kStageA) >> 4, w_step = wtile_bytes >> 4;
-      const uint32_t slab_lo0 = ((smem_u32(sSlab) & 0x3FFFFu) >> 4) | (1u << 16);
-      const uint32_t empty_r = mapa_shared(empty, 1), acc_full_r = mapa_shared(acc_full, 1);
-      uint32_t slot = 0, ph = 0, lo = lo0;
-      uint32_t acc_ph0 = 1, acc_ph1 = 1;   // acc_empty phases: the first use of each buffer is free
-      uint32_t buf = 0;
-      uint32_t good = 1;
       for (int t = 0; t < my_tiles; ++t) {
-        good &= mbar_park_flag(acc_empty + buf * 8, buf ? acc_ph1 : acc_ph0, good ? poll_limit : 0u);
-        acc_ph0 ^= buf ? 0u : 1u;
-        acc_ph1 ^= buf ? 1u : 0u;
-        tc_fence_after_sync();
-        const uint32_t d = tmem_base + buf * 256;
-        uint32_t acc = 0;
+        const int row0 = row_of(t);
         for (int g0 = 0; g0 < G; g0 += ks) {
-          if (STATIONARY && t == 0) {   // the slab lands while the first tile runs
-            for (int q = 0; q < ks; ++q) good &= mbar_spin_flag(slab_full + (g0 + q) * 8, 0u, good ? spin_limit : 0u);
-          }
-          good &= mbar_spin_flag(full + slot * 8, ph, good ? spin_limit : 0u);
-          tc_fence_after_sync();
+          good &= mbar_park_flag(empty + slot * 8, ph, good ? poll_limit : 0u);
           if (elect_one()) {
             if (good) {
-              uint32_t al = lo, wl = STATIONARY ? slab_lo0 + static_cast<uint32_t>(g0) * w_step : lo + w_off;
-              for (int q = 0; q < ks; ++q) {
-                umma_pair_f16_x4(d, al, wl, idesc, (q == 0) ? acc : 1u);
-                al += kStageA >> 4;
-                wl += w_step;
-              }
-              umma_pair_commit(empty + slot * 8);
-              umma_pair_commit(empty_r + slot * 8);
-              if (g0 + ks >= G) {
-                umma_pair_commit(acc_full + buf * 8);
-                umma_pair_commit(acc_full_r + buf * 8);
-              }
+              if (crank == 0) mbar_expect_tx(full + slot * 8, 2u * stage_bytes);
+              const uint32_t dst = st0 + slot * stage_bytes;
+#pragma unroll 1
+              for (int q = 0; q < ks; ++q)
+                tma_load_2d_pair(dst + q * kStageA, &tm_a, full_leader + slot * 8, (g0 + q) * 64, row0);
+              if (!STATIONARY)
+#pragma unroll 1
+                for (int q = 0; q < ks; ++q)
+                  tma_load_2d_pair(dst + ks * kStageA + q * wtile_bytes, &tm_w, full_leader + slot * 8, (g0 + q) * 64, nh0);
             }
           }
           __syncwarp();
-          acc = 1u;
-          lo += s_step;
-          if (++slot == sa) { slot = 0; ph ^= 1; lo = lo0; }
+          if (++slot == sa) { slot = 0; ph ^= 1; }
         }
-        buf ^= 1;
         if (__any_sync(0xffffffffu, good == 0)) break;
       }
       ok = __all_sync(0xffffffffu, good != 0);
-      __syncwarp();
-      if (!ok && lane == 0) atomicExch(p.status, kStatusPairTimeout);
+      if (!ok) {
+        // give copies that are still in flight time to land before this CTA's shared memory goes away
+        for (int i = 0; i < 64; ++i) __nanosleep(1000);
+        if (lane == 0) atomicExch(p.status, kStatusPairTimeout);
+      }
+    } else if (warp == 1) {
+      // ------------------------------------------------------------------ MMA issue (leader CTA only)
+      if (crank == 0 && my_tiles > 0) {
+        const uint32_t idesc = umma_idesc_f16(kPairTileM, bn);
+        const uint32_t sa = p.sa;
+        const uint32_t lo0 = ((smem_u32(sStages) & 0x3FFFFu) >> 4) | (1u << 16);
+        const uint32_t s_step = stage_bytes >> 4, w_off = (static_cast<uint32_t>(ks) * kStageA) >> 4, w_step = wtile_bytes >> 4;
+        const uint32_t slab_lo0 = ((smem_u32(sSlab) & 0x3FFFFu) >> 4) | (1u << 16);
+        const uint32_t empty_r = mapa_shared(empty, 1), acc_full_r = mapa_shared(acc_full, 1);
+        uint32_t slot = 0, ph = 0, lo = lo0;
+        uint32_t acc_ph0 = 1, acc_ph1 = 1;   // acc_empty phases: the first use of each buffer is free
+        uint32_t buf = 0;
+        uint32_t good = 1;
+        for (int t = 0; t < my_tiles; ++t) {
+          good &= mbar_park_flag(acc_empty + buf * 8, buf ? acc_ph1 : acc_ph0, good ? poll_limit : 0u);
+          acc_ph0 ^= buf ? 0u : 1u;
+          acc_ph1 ^= buf ? 1u : 0u;
+          tc_fence_after_sync();
+          const uint32_t d = tmem_base + buf * 256;
+          uint32_t acc = 0;
+          for (int g0 = 0; g0 < G; g0 += ks) {
+            if (STATIONARY && t == 0) {   // the slab lands while the first tile runs
+#pragma unroll 1
+              for (int q = 0; q < ks; ++q) good &= mbar_spin_flag(slab_full + (g0 + q) * 8, 0u, good ? spin_limit : 0u);
+            }
+            good &= mbar_spin_flag(full + slot * 8, ph, good ? spin_limit : 0u);
+            tc_fence_after_sync();
+            if (elect_one()) {
+              if (good) {
+                uint32_t al = lo, wl = STATIONARY ? slab_lo0 + static_cast<uint32_t>(g0) * w_step : lo + w_off;
+#pragma unroll 1
+                for (int q = 0; q < ks; ++q) {
+                  umma_pair_f16_x4(d, al, wl, idesc, (q == 0) ? acc : 1u);
+                  al += kStageA >> 4;
+                  wl += w_step;
+                }
+                umma_pair_commit(empty + slot * 8);
+                umma_pair_commit(empty_r + slot * 8);
+                if (g0 + ks >= G) {
+                  umma_pair_commit(acc_full + buf * 8);
+                  umma_pair_commit(acc_full_r + buf * 8);
+                }
+              }
+            }
+            __syncwarp();
+            acc = 1u;
+            lo += s_step;
+            if (++slot == sa) { slot = 0; ph ^= 1; lo = lo0; }
+          }
+          buf ^= 1;
+          if (__any_sync(0xffffffffu, good == 0)) break;
+        }
+        ok = __all_sync(0xffffffffu, good != 0);
+        __syncwarp();
+        if (!ok && lane == 0) atomicExch(p.status, kStatusPairTimeout);
+      }
     }
-  } else if (QBITS != 0 && warp < kIssue) {
-    // the quantizer form's idle warps (no register instruction in the plain form, not even where nothing gets to it: 2 to 8 % slower)
-    if constexpr (QBITS != 0) fewer_registers<kPairQuantIssueRegs>();
   } else if constexpr (QBITS != 0) {
     more_registers<kPairQuantEpiRegs>();
     // ------------------------------------------------------------------ epilogue with GELU and quantizer
