@@ -81,7 +81,8 @@ enum Opt {
   O_WS_BN, O_WS_SA, O_WS_WS, O_WS_STATIONARY, O_WS_NBB, O_WS_GRID, O_WS_TMA_STORE, O_WS_ROTATE,
   O_ACT_QUANT_V1, O_LN_PLAIN,
   O_PAIR, O_PAIR_MIN_M, O_PAIR_BN, O_PAIR_SA, O_PAIR_KS, O_PAIR_NBB, O_PAIR_LUT, O_PAIR_PAIRS, O_PAIR_STATIONARY,
-  O_PAIR_WS, O_LNQ_SMALL, O_AQ2_MIN_GROUPS, O_PDL, O_GELU_GEMM, O_GEMM_UNPACK, O_POLL_LIMIT, O_SPIN_LIMIT, O_COUNT
+  O_PAIR_WS, O_LNQ_SMALL, O_AQ2_MIN_GROUPS, O_PDL, O_GELU_GEMM, O_GEMM_UNPACK, O_POLL_LIMIT, O_SPIN_LIMIT, O_LAUNCH_REGS,
+  O_COUNT
 };
 struct OptDef { const char* name; int dflt; };
 const OptDef kOptDefs[O_COUNT] = {
@@ -92,7 +93,7 @@ const OptDef kOptDefs[O_COUNT] = {
     {"ARCQ_PAIR_KS", 0},      {"ARCQ_PAIR_NBB", 0},       {"ARCQ_PAIR_LUT", 0},    {"ARCQ_PAIR_PAIRS", 0},
     {"ARCQ_PAIR_STATIONARY", -1}, {"ARCQ_PAIR_WS", 0}, {"ARCQ_LNQ_SMALL", 1}, {"ARCQ_AQ2_MIN_GROUPS", 0}, {"ARCQ_PDL", 1},
     {"ARCQ_GELU_GEMM", -1}, {"ARCQ_GEMM_UNPACK", 1},
-    {"ARCQ_POLL_LIMIT", 1 << 21}, {"ARCQ_SPIN_LIMIT", 1 << 25},
+    {"ARCQ_POLL_LIMIT", 1 << 21}, {"ARCQ_SPIN_LIMIT", 1 << 25}, {"ARCQ_LAUNCH_REGS", 0},
 };
 int g_opt[O_COUNT];
 void load_options() {
@@ -126,6 +127,19 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
   lc.attrs = attr;
   lc.numAttrs = opt(O_PDL) != 0 ? 1 : 0;
   return cudaLaunchKernelEx(&lc, kernel, static_cast<KArgs>(args)...);
+}
+
+// Set-up of a kernel whose warp groups hand registers over: its shared-memory limit, and whether a launch brings the registers a
+// thread that the hand-over counts on.  An increase beyond them waits for good, and a changed flag or compiler is enough for that, so
+// such a build is refused here.  ARCQ_LAUNCH_REGS stands for what the compiled kernel says, in tests.
+template <typename Kernel> int prepare_register_kernel(Kernel kernel, size_t smem, int regs, const char* what) {
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  cudaFuncAttributes a = {};
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+  if (e != cudaSuccess) return cuda_fail(e, what);
+  const int got = opt(O_LAUNCH_REGS) > 0 ? opt(O_LAUNCH_REGS) : a.numRegs;
+  if (got < regs) return fail(ARCQ_E_CUDA, "%s: compiled for %d registers a thread, its warp groups share out %d", what, got, regs);
+  return ARCQ_OK;
 }
 
 bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
@@ -1082,27 +1096,27 @@ static int launch_pair_dense_gemm(const PairDenseConfig& cfg, const void* xhat, 
     auto launch = [&](auto kernel, int* done_dev) {
       int dev = 0;
       cudaGetDevice(&dev);
-      if (*done_dev != dev) {                   // shared-memory ceiling, once per (thread, device)
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBudget + 1024));
-        if (e != cudaSuccess) return e;
+      if (*done_dev != dev) {                   // once per (thread, device)
+        const int rc = prepare_register_kernel(kernel, kSmemBudget + 1024, arcq::kPairQuantLaunchRegs, "dense_weight_gemm_gelu_quant");
+        if (rc != ARCQ_OK) return rc;
         *done_dev = dev;
       }
       launch_pdl(kernel, grid, arcq::kPairQuantThreads, cfg.smem, st, tm_a, tm_w, tm_y, p, jobs);
-      return cudaGetLastError();
+      const cudaError_t e = cudaGetLastError();
+      return e != cudaSuccess ? cuda_fail(e, "dense_weight_gemm_gelu_quant launch") : ARCQ_OK;
     };
     static thread_local int done[6] = {-1, -1, -1, -1, -1, -1};
-    cudaError_t e = cudaSuccess;
+    int rc;
     if (cfg.stationary)
-      e = q_bits == 4 ? launch(arcq::dense_weight_gemm_pair_kernel<true, false, 4>, done)
+      rc = q_bits == 4 ? launch(arcq::dense_weight_gemm_pair_kernel<true, false, 4>, done)
           : q_bits == 3 ? launch(arcq::dense_weight_gemm_pair_kernel<true, false, 3>, done + 1)
                         : launch(arcq::dense_weight_gemm_pair_kernel<true, false, 2>, done + 2);
     else
-      e = q_bits == 4 ? launch(arcq::dense_weight_gemm_pair_kernel<false, false, 4>, done + 3)
+      rc = q_bits == 4 ? launch(arcq::dense_weight_gemm_pair_kernel<false, false, 4>, done + 3)
           : q_bits == 3 ? launch(arcq::dense_weight_gemm_pair_kernel<false, false, 3>, done + 4)
                         : launch(arcq::dense_weight_gemm_pair_kernel<false, false, 2>, done + 5);
     g_last_gemm_kernel = ARCQ_GEMM_PAIR_DENSE_GELU_QUANT;
-    if (e != cudaSuccess) return cuda_fail(e, "dense_weight_gemm_gelu_quant launch");
-    return ARCQ_OK;
+    return rc;
   }
   if (next != nullptr) {
     static thread_local int done_dev = -1;      // the prefetch form's shared-memory ceiling, once per (thread, device)
@@ -1450,9 +1464,9 @@ static int launch_attention(const void* qkv, int64_t B, int64_t T, int64_t H, in
     int dev = 0;                                                                                                      \
     cudaGetDevice(&dev);                                                                                              \
     if (done_dev != dev) {                                                                                            \
-      const cudaError_t se = cudaFuncSetAttribute(arcq::attention_kernel<Q, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                                  static_cast<int>(arcq::attn_smem_layout(arcq::kAttnMaxT).total));   \
-      if (se != cudaSuccess) return cuda_fail(se, "attention shared memory");                                         \
+      const int rc = prepare_register_kernel(arcq::attention_kernel<Q, BT>, arcq::attn_smem_layout(arcq::kAttnMaxT).total, \
+                                             arcq::kAttnLaunchRegs, "attention");                                    \
+      if (rc != ARCQ_OK) return rc;                                                                                   \
       done_dev = dev;                                                                                                 \
     }                                                                                                                 \
     launch_pdl(arcq::attention_kernel<Q, BT>, grid, arcq::kAttnThreads, smem, st, tm_q, tm_kv, tm_out, p);            \

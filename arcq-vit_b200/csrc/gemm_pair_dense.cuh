@@ -59,8 +59,9 @@ constexpr int kPairDenseThreads = (2 + kPairEpiWarps) * 32;
 // launch's 128 ([12608, 3072] x 768 76.3 -> 75.1 us, [50432, 3072] x 768 357 -> 350 us).
 constexpr int kPairQuantEpiWarps = 12, kPairQuantIssueWarps = 4;
 constexpr int kPairQuantThreads = (kPairQuantIssueWarps + kPairQuantEpiWarps) * 32;
-constexpr int kPairQuantEpiRegs = 152, kPairQuantIssueRegs = 56;
-static_assert(kPairQuantEpiRegs * kPairQuantEpiWarps + kPairQuantIssueRegs * kPairQuantIssueWarps <= 128 * (kPairQuantThreads / 32),
+constexpr int kPairQuantLaunchRegs = 128, kPairQuantEpiRegs = 152, kPairQuantIssueRegs = 56;
+static_assert(kPairQuantEpiRegs * kPairQuantEpiWarps + kPairQuantIssueRegs * kPairQuantIssueWarps <=
+                  kPairQuantLaunchRegs * (kPairQuantThreads / 32),
               "registers beyond the launch's never come");
 constexpr uint32_t kPairQuantStageBytes = kPairQuantEpiWarps * 4096;       // 32 rows of 128 bytes per warp
 constexpr uint32_t kPairQuantTableBytes = (sizeof(GroupQuantTables) + 15) / 16 * 16;

@@ -656,3 +656,38 @@ def test_sixteen_bit_tiles_with_search_and_zero_threshold(pkg, oracle, cuda_devi
             p = pkg.ops.quantize_activation(x.to(cuda_device), _t(th, cuda_device), _t(cb, cuda_device), bits, 64)[0]
             assert np.array_equal(p.cpu().numpy(), oracle.pack(codes, bits))
     assert pkg.ops.device_status() == 0
+
+
+@pytest.mark.parametrize("kernel", ["attention", "gelu quant"])
+def test_kernels_that_hand_registers_over_check_what_a_launch_brings(pkg, cuda_device, kernel):
+    """With eight registers a thread fewer than the hand-over counts on, an increase would wait for good: an error, nothing launched.
+    Looked at once per thread and device, hence the threads."""
+    import threading
+    cb = torch.linspace(-2.0, 2.0, 16, device=cuda_device)
+    th = (cb[:-1] + cb[1:]) / 2
+    if kernel == "attention":
+        qkv, regs = torch.zeros(17, 192, dtype=torch.float16, device=cuda_device), 80
+        call = lambda: pkg.ops.attention(qkv, 1, 17, 1, th, cb, 4)                                                    # noqa: E731
+    else:
+        x, regs = torch.zeros(64, 64, dtype=torch.float16, device=cuda_device), 128
+        call = lambda: pkg.ops.dense_weight_gemm_gelu_quant(x, x, None, th, cb, 4, 64)                                # noqa: E731
+    results = []
+
+    def run():
+        try:
+            results.append(call())
+        except RuntimeError as e:
+            results.append(str(e))
+
+    def in_a_thread(launch_regs):
+        with pkg._cabi.option("ARCQ_LAUNCH_REGS", launch_regs), pkg._cabi.option("ARCQ_GELU_GEMM", 1):
+            t = threading.Thread(target=run)
+            t.start()
+            t.join()
+        return results.pop()
+
+    refused = in_a_thread(regs - 8)
+    assert isinstance(refused, str) and f"compiled for {regs - 8} registers" in refused
+    for launch_regs in (regs, 0):                                   # what it needs, what the kernel really has
+        assert torch.is_tensor(in_a_thread(launch_regs))
+    assert pkg.ops.device_status() == 0
