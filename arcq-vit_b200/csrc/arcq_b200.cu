@@ -1446,7 +1446,9 @@ static int launch_attention(const void* qkv, int64_t B, int64_t T, int64_t H, in
   p.thresholds = thresholds;
   p.codebook = codebook;
   p.one_fma = one_fma;
+  p.poll_limit = static_cast<uint32_t>(opt(O_POLL_LIMIT));
   p.status = status_ptr();
+  if (p.status == nullptr) return fail(ARCQ_E_CUDA, "device status word not reachable");
   CUtensorMap tm_q, tm_kv, tm_out;
   auto map = [&](CUtensorMap* tm, const void* base, int64_t cols, int box_rows) {
     return make_tensor_map(tm, base, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, static_cast<uint64_t>(B), static_cast<uint64_t>(T),

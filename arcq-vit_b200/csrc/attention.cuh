@@ -50,6 +50,7 @@ struct AttnParams {
   const float* thresholds;     // quantizer form only
   const float* codebook;
   int one_fma;
+  uint32_t poll_limit;         // waits of one warp for another give up after this many polls
   int* status;
 };
 
@@ -125,7 +126,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
   uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + L.bars);
   uint64_t *const q_full = bars, *const q_free = bars + 1, *const k_full = bars + 2, *const k_free = bars + 3,
            *const v_full = bars + 4, *const v_free = bars + 5, *const s_full = bars + 6, *const o_full = bars + 7,
-           *const p_upper = bars + 8, *const p_lower = bars + 9, *const o_read = bars + 10;
+           *const p_upper = bars + 8, *const p_lower = bars + 9, *const o_read = bars + 10, *const stopped = bars + 11;
   uint32_t* const s_tmem = reinterpret_cast<uint32_t*>(bars + 16);
   float* const s_sums = reinterpret_cast<float*>(smem + L.sums);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -143,9 +144,11 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
   if (tid == 0) {
     for (int i = 0; i < 8; ++i) mbar_init(bars + i, 1);
     for (int i = 8; i < 11; ++i) mbar_init(bars + i, kAttnRowWarps);
+    mbar_init(stopped, 1);
     mbar_fence_init();
   }
   __syncthreads();
+  const uint32_t polls = p.poll_limit;
   bool ok = true;
 
   if (warp >= 8) {
@@ -158,19 +161,21 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
         tma_prefetch_desc(&tm_out);
       }
       pdl_wait();
-      uint32_t heads = 0;
+      uint32_t heads = 0, q_loads = 0, k_loads = 0;
       auto loads = [&](int it) {
         const uint32_t i = static_cast<uint32_t>(it - first);
         int b, x;
         const int q0 = place(it, &b, &x);
-        if (i > 0 && !mbar_wait(q_free, (i - 1) & 1)) return false;
+        if (i > 0 && !mbar_wait(q_free, (i - 1) & 1, polls)) return false;
         mbar_arrive_expect_tx(q_full, kAttnQueries * 128);
         tma_load_3d(smem + L.q, &tm_q, q_full, x, q0, b);
+        ++q_loads;
         if (i == 0 || q0 == 0) {
-          if (heads > 0 && !mbar_wait(k_free, (heads - 1) & 1)) return false;
+          if (heads > 0 && !mbar_wait(k_free, (heads - 1) & 1, polls)) return false;
           mbar_arrive_expect_tx(k_full, static_cast<uint32_t>(p.tk) * 128);
           tma_load_3d(smem + L.k, &tm_kv, k_full, C + x, 0, b);
-          if (heads > 0 && !mbar_wait(v_free, (heads - 1) & 1)) return false;
+          ++k_loads;
+          if (heads > 0 && !mbar_wait(v_free, (heads - 1) & 1, polls)) return false;
           mbar_arrive_expect_tx(v_full, static_cast<uint32_t>(p.tk) * 128);
           tma_load_3d(smem + L.v, &tm_kv, v_full, 2 * C + x, 0, b);
           ++heads;
@@ -183,11 +188,9 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
       pdl_launch_dependents();
       if (lane == 0) {
         for (int it = first + 1; it < last && ok; ++it) ok = loads(it);
-        if (!ok) {
-          // give copies that are still in flight time to land before this block's shared memory goes away
-          for (int i = 0; i < 64; ++i) __nanosleep(1000);
-          atomicExch(p.status, kStatusAttentionTimeout);
-        }
+        // No copy may land after the block has left, whichever warp has given up: the last one of each kind.
+        ok &= mbar_wait(q_full, (q_loads - 1) & 1) && mbar_wait(k_full, (k_loads - 1) & 1) && mbar_wait(v_full, (heads - 1) & 1);
+        if (!ok) atomicExch(p.status, kStatusAttentionTimeout);
       }
       __syncwarp();
     } else {
@@ -214,7 +217,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
           const int q_tile = it % p.qtiles;
           const bool new_head = i == 0 || q_tile == 0, end_head = it + 1 == last || q_tile + 1 == p.qtiles;
           heads += new_head ? 1 : 0;
-          ok = (!new_head || mbar_wait(k_full, (heads - 1) & 1)) && mbar_wait(q_full, i & 1) && (i == 0 || mbar_wait(o_read, (i - 1) & 1));
+          ok = (!new_head || mbar_wait(k_full, (heads - 1) & 1, polls)) && mbar_wait(q_full, i & 1, polls) &&
+               (i == 0 || mbar_wait(o_read, (i - 1) & 1, polls));
           if (!ok) break;
           tc_fence_after_sync();
 #pragma unroll
@@ -222,20 +226,25 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
           umma_commit(s_full);
           umma_commit(q_free);
           if (end_head) umma_commit(k_free);
-          ok = (!new_head || mbar_wait(v_full, (heads - 1) & 1)) && mbar_wait(p_upper, i & 1);
+          ok = (!new_head || mbar_wait(v_full, (heads - 1) & 1, polls)) && mbar_wait(p_upper, i & 1, polls);
           if (!ok) break;
           tc_fence_after_sync();
           uint32_t acc = 0;
           for (int k = split; k < p.tk; k += 16, acc = 1)
             umma_f16_tmem_a(tmem + kAttnOutCol, tmem + split + (k - split) / 2, dv + 8 * k, idesc_o, acc);
-          ok = mbar_wait(p_lower, i & 1);
+          ok = mbar_wait(p_lower, i & 1, polls);
           if (!ok) break;
           tc_fence_after_sync();
           for (int k = 0; k < split; k += 16, acc = 1) umma_f16_tmem_a(tmem + kAttnOutCol, tmem + k / 2, dv + 8 * k, idesc_o, acc);
           umma_commit(o_full);
           if (end_head) umma_commit(v_free);
         }
-        if (!ok) atomicExch(p.status, kStatusAttentionTimeout);
+        if (!ok) {
+          // products that were issued end before their tensor memory is given back
+          umma_commit(stopped);
+          mbar_wait(stopped, 0);
+          atomicExch(p.status, kStatusAttentionTimeout);
+        }
       }
       __syncwarp();
     }
@@ -252,7 +261,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
     for (int it = first; it < last; ++it) {
       const uint32_t ph = static_cast<uint32_t>(it - first) & 1;
       const bool live = (it % p.qtiles) * kAttnQueries + warp * 32 < T;    // some of the warp's rows are queries
-      if (!mbar_wait(s_full, ph)) { ok = false; break; }
+      if (!mbar_wait(s_full, ph, polls)) { ok = false; break; }
       tc_fence_after_sync();
       // Loops with one body each, not unrolled over the row: the softmax and output warps of two blocks share an instruction
       // cache, and unrolled passes stalled on it more than on anything else (DeiT-S batch 64, with the quantizer: 27.0 -> 24.1 us).
@@ -359,7 +368,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
       const int t0 = place(it, &b, &x) + quarter * 32;
       const bool live = t0 < T;
       // p_lower: the sums are there
-      if (!mbar_wait(p_lower, ph) || !mbar_wait(o_full, ph)) { ok = false; break; }
+      if (!mbar_wait(p_lower, ph, polls) || !mbar_wait(o_full, ph, polls)) { ok = false; break; }
       tc_fence_after_sync();
       uint32_t w[32];
       if (live) {

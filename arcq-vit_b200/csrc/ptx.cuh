@@ -99,8 +99,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // Bounded wait.  try_wait itself blocks for a hardware-defined slice, so the poll count below is a
 // budget of a few seconds at most, far beyond any healthy wait in these kernels.
 constexpr uint32_t kMaxPolls = 4u << 20;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  for (uint32_t i = 0; i < kMaxPolls; ++i) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t polls = kMaxPolls) {
+  for (uint32_t i = 0; i < polls; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
   }
   return false;

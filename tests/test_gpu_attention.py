@@ -327,3 +327,20 @@ def test_probabilities_are_divided_by_a_correctly_rounded_sum(pkg, cuda_device):
         got = pkg.ops.attention(qkv.half().to(cuda_device), 1, T, 1).cpu()
         assert torch.equal(got, want.expand(T, 64)), T
     assert pkg.ops.device_status() == 0
+
+
+@pytest.mark.parametrize("B,T", [(1, 17), (1, 197), (200, 197)])       # one item, two of a head, several blocks an SM and heads a block
+def test_waits_of_the_attention_kernel_that_run_out(pkg, cuda_device, B, T):
+    """With no polls every warp gives up at its first wait: the kernel ends and leaves its code in the status word, and the next launch
+    is none the worse."""
+    H = 3
+    qkv = torch.randn(B * T, 3 * H * 64, generator=torch.Generator().manual_seed(T)).half().to(cuda_device)
+    want = pkg.ops.attention(qkv, B, T, H)
+    cb = torch.linspace(-2.5, 2.5, 16, device=cuda_device)
+    for quantizer in ((), ((cb[:-1] + cb[1:]) / 2, cb, 4)):
+        with pkg._cabi.option("ARCQ_POLL_LIMIT", 0):
+            pkg.ops.attention(qkv, B, T, H, *quantizer)
+        assert pkg.ops.device_status() == 0x501
+        assert pkg.ops.device_status() == 0
+    assert torch.equal(pkg.ops.attention(qkv, B, T, H), want)
+    assert pkg.ops.device_status() == 0
