@@ -590,8 +590,8 @@ template <typename Kernel> int max_resident_dense_pairs(Kernel kernel, int threa
 }
 
 // Slab width, stages and grid for the dense-weight pair kernel; false leaves the shape to the one-CTA kernel.
-// Cost model in microseconds, same constants as the packed-weight pair kernel's: a tile is bound by its output
-// stores (about 22 GB/s per SM) or by the issuing thread, and every slab streams the whole activation from L2.
+// Cost model in microseconds: a tile is bound by its output stores (about 22 GB/s per SM) or by the issuing thread, and every slab
+// streams the whole activation from L2.
 bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32, PairDenseConfig* c) {
   // No row threshold (ARCQ_PAIR_MIN_M gates the packed-weight pair kernel only): with nothing to rebuild, the pair
   // form measured faster than the one-CTA form from one row tile on (DeiT-S batch 1: 0.55 against 0.68 ms).
@@ -658,18 +658,16 @@ bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32,
       if (stationary && opt(O_PAIR_STATIONARY) < 0 && (k.sa * k.ks < 4 || tiles_pp < 3))
         continue;   // too little room left for A, or too few tiles to pay for loading the whole slab first
       const double t_issue = (G / k.ks) * (k.ks * 4 * (bn > 128 ? 0.056 * bn / 192.0 : 0.04) + 0.1);
-      // shared-memory fill through L2, about 8 TB/s over the machine: every tile streams its A rows, and its
-      // W16 rows too unless the slab is stationary
+      // what goes through L2 into shared memory: every tile streams its A rows, and its W16 rows too unless the slab is stationary
       const double fill_mb = (static_cast<double>(slabs) * M * K * 2.0 +
                               (stationary ? static_cast<double>(k.pairs) : static_cast<double>(slabs * tiles_m)) * bn * K * 2.0) / 1.0e6;
-      // ... and 12 TB/s where the tiles stream long rows (8 throughout took 256-column slabs for [7289, 3072] x 768: 34.5 us against
-      // 29.6, [12608, 768] x 768: 17.5 against 16.0, [12608, 3072] x 768: 58.6 against 55.0; 12 throughout took 96-column slabs for
-      // [12608, 384] x 384: 9.5 us against 8.5)
-      const double t_fill = fill_mb / (K >= 768 ? 12.0 : 8.0);
-      // 0.45 us per tile that neither the stores nor the issue account for (measured: at equal store volume, 192-wide
-      // slabs beat 128-wide ones on N = 1152 by 1 us over 5 against 7 tiles per pair)
-      const double path = tiles_pp * ((t_write > t_issue ? t_write : t_issue) + 0.45) * (stationary ? 0.95 : 1.0);
-      const double cost = 1.5 + (path > t_fill ? path : t_fill);
+      // A tile's stores or its issue, whichever is longer, 0.8 us a tile that neither accounts for, and a twentieth of a microsecond
+      // for every megabyte of fill: it is hidden in part only, behind wide slabs as behind narrow ones.  Fitted to every slab width on
+      // 462 shapes (eleven layers of the three widths, 394 to 25216 rows, both output types): the slab chosen is 1.7 % slower than the
+      // fastest on average, 25 % at worst.  The larger of the tiles' time and of the fill at 8 TB/s had 3.2 and 29 %, with 12 TB/s
+      // from K = 768 on 2.7 and 25 %, and that took narrow slabs for wide fp32 outputs: N = 3072, K = 768, 25216 rows 151 us against
+      // 122, N = 2304 114 against 94; now no shape is more than 2.4 % behind the better of the two.
+      const double cost = tiles_pp * ((t_write > t_issue ? t_write : t_issue) + 0.8) + fill_mb / 20.0;
       if (!found || cost < best_cost) { best = k; best_cost = cost; found = true; }
     }
   }
