@@ -557,6 +557,7 @@ bool choose_pair_config(long long M, long long N, long long K, int bits, bool y_
 struct PairDenseConfig {
   int bn, sa, ks, pairs, stationary;
   size_t smem;
+  double cost;     // of the model that chose it
 };
 
 // CTA pairs of a form of the kernel that are resident at once with all of the shared memory, kept per host thread and device.
@@ -619,7 +620,6 @@ bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32,
   int max_pairs = max_resident_dense_pairs(arcq::dense_weight_gemm_pair_kernel<true>, arcq::kPairDenseThreads, &known);
   if (opt(O_PAIR_PAIRS) > 0 && opt(O_PAIR_PAIRS) < max_pairs) max_pairs = opt(O_PAIR_PAIRS);
   static const int cand[] = {256, 192, 160, 128, 96, 64, 32};
-  double best_cost = 0;
   bool found = false;
   PairDenseConfig best = {};
   // One or two row tiles (batch 1-2 of a ViT): the launch is a latency chain, not a throughput problem.  The
@@ -668,7 +668,8 @@ bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32,
       // from K = 768 on 2.7 and 25 %, and that took narrow slabs for wide fp32 outputs: N = 3072, K = 768, 25216 rows 151 us against
       // 122, N = 2304 114 against 94; now no shape is more than 2.4 % behind the better of the two.
       const double cost = tiles_pp * ((t_write > t_issue ? t_write : t_issue) + 0.8) + fill_mb / 20.0;
-      if (!found || cost < best_cost) { best = k; best_cost = cost; found = true; }
+      k.cost = cost;
+      if (!found || cost < best.cost) { best = k; found = true; }
     }
   }
   if (!found) return false;
@@ -685,7 +686,6 @@ bool choose_pair_quant_config(long long M, long long N, long long K, PairDenseCo
   int max_pairs = max_resident_dense_pairs(arcq::dense_weight_gemm_pair_kernel<true, false, 4>, arcq::kPairQuantThreads, &known);
   if (opt(O_PAIR_PAIRS) > 0 && opt(O_PAIR_PAIRS) < max_pairs) max_pairs = opt(O_PAIR_PAIRS);
   static const int cand[] = {192, 128, 64};                  // whole groups, at most one per epilogue warp of a lane quarter
-  double best_cost = 0;
   bool found = false;
   for (int bn : cand) {
     if (N % bn != 0 || (opt(O_PAIR_BN) > 0 && bn != opt(O_PAIR_BN))) continue;
@@ -697,7 +697,7 @@ bool choose_pair_quant_config(long long M, long long N, long long K, PairDenseCo
     // The epilogue bounds every tile: one, two or three warps per scheduler share its issue slots (a single tile of
     // 64 / 128 / 192 columns, K = 384: 8.7 / 9.8 / 11.4 us).
     const double cost = tiles_pp * (2.5 + 0.9 * (bn / 64));
-    if (found && cost >= best_cost) continue;
+    if (found && cost >= c->cost) continue;
     for (int stationary = 1; stationary >= 0; --stationary) {
       if (stationary && (G > 32 || tiles_pp < 3)) continue;    // too few tiles to pay for loading the whole slab first
       PairDenseConfig k = {};
@@ -709,8 +709,8 @@ bool choose_pair_quant_config(long long M, long long N, long long K, PairDenseCo
         if (need <= kSmemBudget) { k.sa = sa; k.smem = need + 1024; fits = true; }
       }
       if (!fits || (stationary && k.sa * k.ks < 4)) continue;
+      k.cost = cost;
       *c = k;
-      best_cost = cost;
       found = true;
       break;
     }
@@ -725,17 +725,25 @@ bool small_layernorm_quant(long long M, long long K) {
   return M * (K / 64) < static_cast<long long>(sm_count()) * 48 && opt(O_LNQ_SMALL) != 0;
 }
 
-// fc1 with GELU and quantizer in its epilogue, or GEMM and quantizer kernel?  Whole forwards through a graph (two kernels /
-// one): its 12 epilogue warps hide latency worse than the quantizer kernel's 16, so it pays where the tiles are one round (DeiT-S
-// batch 6 / 8: 714 -> 676, 724 -> 679 us; DeiT-T batch 16: 656 -> 618) but not below five row tiles (DeiT-T batch 2: 449 ->
-// 463), where the products under it are long (DeiT-B batch 4: 874 -> 821 us) or where the matrix between the two no longer stays
-// in L2 (DeiT-S batch 128: 2678 -> 2575 us, DeiT-B: 7341 -> 6902), and from some 6000 rows on (DeiT-T batch 37: 817 -> 789, 64: 952
-// -> 945, DeiT-S batch 32: 1029 -> 1016, 64: 1558 -> 1548); in between the rounds eat it (DeiT-S batch 16: 785 -> 804).
+// fc1 with GELU and quantizer in its epilogue, or GEMM and quantizer kernel?  Whole forwards through a graph, microseconds, two
+// kernels / one.  The epilogue's 12 warps hide latency worse than the quantizer kernel's 16, so it is rounds that decide: of the
+// fused form's tiles on the pairs against the quantizer's blocks (512 groups an SM).  The line below is fitted to 35 batch sizes of
+// DeiT-T and DeiT-S (DeiT-T batch 32: 717 / 729, 34, where the quantizer starts a second round: 778 / 736; DeiT-S batch 16: 757 /
+// 772, 18: 832 / 785, 48: 1234 / 1259): at one of them it is 15 us, 1 %, off the better form, 40 us over all; "from 6000 rows on"
+// was 186 us off, one round of tiles only 381, both 48 at worst.  Always where the products under the epilogue are long (DeiT-B batch
+// 4: 874 / 821) or the matrix between the two no longer stays in L2 (DeiT-S batch 128: 2678 / 2575, DeiT-B: 7341 / 6902).  Where the
+// quantizer takes its form for small inputs: one round of tiles (DeiT-S batch 6 / 8: 584 / 564, 712 / 660; DeiT-T batch 12: 552 / 527)
+// but not below five row tiles (DeiT-T batch 2: 449 / 463).
 bool choose_gelu_quant(long long M, long long N, long long K, PairDenseConfig* pc) {
   const int force = opt(O_GELU_GEMM);
   if (force == 0 || N % 64 != 0 || !choose_pair_quant_config(M, N, K, pc)) return false;
-  const bool one_round = 1ll * pc->pairs * pc->bn >= (M + arcq::kPairTileM - 1) / arcq::kPairTileM * N;
-  return force > 0 || K >= 768 || M >= 6000 || (M > 1024 && one_round);
+  if (force > 0 || K >= 768 || M >= 20000) return true;
+  const long long groups = M * (N / 64), sms = sm_count();
+  PairDenseConfig plain;
+  if (groups < sms * 256 || !choose_pair_dense_config(M, N, K, false, &plain))
+    return M > 1024 && 1ll * pc->pairs * pc->bn >= (M + arcq::kPairTileM - 1) / arcq::kPairTileM * N;
+  const double rounds = static_cast<double>((groups + sms * 512 - 1) / (sms * 512));
+  return 1.3 * pc->cost < 4.6 * rounds + plain.cost + 1.0;
 }
 
 }  // namespace
