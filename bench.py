@@ -323,7 +323,7 @@ def launches_per_forward(pkg, a, n_lin: int, batch: int) -> int:
     dim, _, depth = pkg.DEIT_CONFIGS[a.model]
     if (pkg.ARCQPackedLinearOnTheFly.weight_form == "auto" and pkg.VisionTransformer.fuse_norm_quant == "auto"
             and pkg.WeightStager.mode == "stream" and pkg.vit.Attention.implementation == "auto"):
-        # the native forward: per block LayerNorm + quantizer, qkv, quantizer, proj, LayerNorm + quantizer, fc1, GELU + quantizer
+        # the native forward: per block LayerNorm + quantizer, qkv, attention + quantizer, proj, LayerNorm + quantizer, fc1, GELU + quantizer
         # (or all of that in fc1), fc2; patch gathering, token assembly and the final norm once.  No launch for the unpacking.
         fused = pkg._cabi.load().arcq_dense_weight_gemm_gelu_quant_applies(batch * TOKENS, 4 * dim, dim)
         return depth * (8 - fused) + 3

@@ -1,6 +1,6 @@
-"""The attention kernel between the qkv and proj linears (an opt-in replacement for the library attention) and its
-form that also runs proj's activation quantizer: against an fp64 evaluation and the library kernel, and -- for the
-quantizer form -- bit for bit against the quantizer kernel applied to the plain form's output."""
+"""The attention kernel between the qkv and proj linears and its form that also runs proj's activation quantizer: against an fp64
+evaluation and the library kernel, and -- for the quantizer form -- bit for bit against the quantizer kernel applied to the plain
+form's output.  Then where the modules take it, what they show of it, and where they take the library's attention."""
 import numpy as np
 import pytest
 import torch
@@ -125,23 +125,27 @@ def test_attention_kernel_extreme_scores(pkg, cuda_device):
     assert pkg.ops.device_status() == 0
 
 
-def test_chosen_back_ends_are_kept(pkg, cuda_device):
-    """A program that chooses among the library's attention back ends gets the one it chose, alone or in the model's one call."""
+def test_chosen_back_ends_are_kept(pkg, cuda_device, monkeypatch):
+    """A program that chooses among the library's attention back ends gets the one it chose: in the model's one call, in the Python
+    forward and from the attention module alone."""
     gen = torch.Generator().manual_seed(14)
     model = pkg.create_vit("deit_tiny", seed=3).half().to(cuda_device)
     x = torch.randn(2, 3, 224, 224, generator=gen).half().to(cuda_device)
-    attn_cls = type(model.blocks[0].attn)
-    saved = attn_cls.implementation
-    try:
-        with torch.no_grad():
-            model = pkg.quantise_model(model, x, 4)
+    tokens = torch.randn(2, 197, 192, generator=gen).half().to(cuda_device)
+    attn = model.blocks[0].attn
+    forward_native = pkg.vit.VisionTransformer._forward_native
+    calls = (lambda: model(x), lambda: model(x), lambda: attn(tokens))
+    with torch.no_grad():
+        model = pkg.quantise_model(model, x, 4)
+        for call, native in zip(calls, (True, False, False)):
+            monkeypatch.setattr(pkg.vit.VisionTransformer, "_forward_native", forward_native if native else lambda self, x: None)
+            own = call().clone()
             with torch.nn.attention.sdpa_kernel(torch.nn.attention.SDPBackend.MATH):
-                chosen = model(x).clone()
-                attn_cls.implementation = "sdpa"
-                want = model(x).clone()
-        assert torch.equal(chosen, want)
-    finally:
-        attn_cls.implementation = saved
+                chosen = call().clone()
+                monkeypatch.setattr(type(attn), "implementation", "sdpa")
+                want = call().clone()
+                monkeypatch.setattr(type(attn), "implementation", "auto")
+            assert torch.equal(chosen, want) and not torch.equal(chosen, own)
 
 
 def _block(pkg, dev, name="deit_tiny", bits=4):
@@ -343,4 +347,48 @@ def test_waits_of_the_attention_kernel_that_run_out(pkg, cuda_device, B, T):
         assert pkg.ops.device_status() == 0x501
         assert pkg.ops.device_status() == 0
     assert torch.equal(pkg.ops.attention(qkv, B, T, H), want)
+    assert pkg.ops.device_status() == 0
+
+
+@torch.no_grad()
+def test_auto_is_the_kernel_between_packed_linears(pkg, cuda_device, monkeypatch):
+    model, images, x = _block(pkg, cuda_device, "deit_small")
+    attn = model.blocks[0].attn
+    got = [attn(x), model(images), model._forward_native(images)]
+    monkeypatch.setattr(type(attn), "implementation", "kernel")
+    assert model._forward_native(images) is None
+    for y, want in zip(got, (attn(x), model(images), model(images))):
+        assert torch.equal(y, want)
+    monkeypatch.setattr(type(attn), "implementation", "sdpa")
+    assert not torch.equal(got[0], attn(x))
+
+
+def _replaced(attn, monkeypatch):
+    library = F.scaled_dot_product_attention
+    monkeypatch.setattr(F, "scaled_dot_product_attention", lambda *a, **k: library(*a, **k))
+
+
+def _asks_for_gradients(attn, monkeypatch):
+    attn.qkv = torch.nn.Linear(192, 576).half().to(attn.qkv.packed_weight_codes.device)
+
+
+def _autocast(attn, monkeypatch):
+    """Entered around the call."""
+
+
+@pytest.mark.parametrize("why", [_replaced, _asks_for_gradients, _autocast])
+def test_where_the_library_attention_stays(pkg, cuda_device, why, monkeypatch):
+    """A function in its place, a qkv that wants a gradient, autocast to another type: bit for bit the library's route."""
+    model, _, x = _block(pkg, cuda_device)
+    attn = model.blocks[0].attn
+    why(attn, monkeypatch)
+    results = []
+    for implementation in ("auto", "sdpa"):
+        monkeypatch.setattr(type(attn), "implementation", implementation)
+        with torch.autocast("cuda", torch.bfloat16, enabled=why is _autocast), torch.set_grad_enabled(why is _asks_for_gradients):
+            results.append(attn(x).detach())
+    assert torch.equal(*results)
+    monkeypatch.undo()
+    with torch.no_grad():
+        assert not torch.equal(attn(x), results[0])              # without the reason: the kernel
     assert pkg.ops.device_status() == 0

@@ -691,3 +691,12 @@ def test_kernels_that_hand_registers_over_check_what_a_launch_brings(pkg, cuda_d
     for launch_regs in (regs, 0):                                   # what it needs, what the kernel really has
         assert torch.is_tensor(in_a_thread(launch_regs))
     assert pkg.ops.device_status() == 0
+
+
+# rows on both sides of where the quantizer kernel or the fused tiles start another round, and of the fixed parts of the rule
+@pytest.mark.parametrize("K,rows", [(192, {985: False, 2364: True, 6304: False, 6698: True, 9456: False, 25216: True}),
+                                    (384, {788: False, 1576: True, 3152: False, 3546: True, 7092: True, 9456: False, 25216: True}),
+                                    (768, {197: True, 3152: True, 12608: True})])
+def test_fc1_runs_fused_where_the_rounds_favour_it(pkg, cuda_device, K, rows):
+    applies = pkg._cabi.load().arcq_dense_weight_gemm_gelu_quant_applies
+    assert {M: bool(applies(M, 4 * K, K)) for M in rows} == rows
