@@ -19,6 +19,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <array>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -267,17 +268,27 @@ PyObject* dequant(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // ---------------------------------------------------------------- the library's attention
-// Whether nothing was chosen about it: all back ends allowed, in the order that the framework starts with or in the one that its first
-// call puts there on a GPU whose cuDNN it prefers.
+// Whether nothing was chosen about it: all back ends allowed, in the order that the framework settles on.  It does so when it is first
+// asked for a back end, whatever the order was until then; after that, the order that it starts with is a choice like any other.  So
+// where that order stands it is asked, once, about tensors without elements.
 bool back_ends_as_they_come() {
   using B = at::SDPBackend;
   using Order = std::array<B, at::num_sdp_backends>;
-  constexpr Order first = {B::flash_attention, B::efficient_attention, B::math, B::cudnn_attention, B::overrideable};
-  constexpr Order later = {B::cudnn_attention, B::flash_attention, B::efficient_attention, B::math, B::overrideable};
+  constexpr Order initial = {B::flash_attention, B::efficient_attention, B::math, B::cudnn_attention, B::overrideable};
+  constexpr Order settled = {B::cudnn_attention, B::flash_attention, B::efficient_attention, B::math, B::overrideable};
   at::Context& ctx = at::globalContext();
-  const Order order = ctx.sDPPriorityOrder();
-  return ctx.userEnabledFlashSDP() && ctx.userEnabledMemEfficientSDP() && ctx.userEnabledMathSDP() && ctx.userEnabledCuDNNSDP() &&
-         (order == first || order == later);
+  if (!ctx.userEnabledFlashSDP() || !ctx.userEnabledMemEfficientSDP() || !ctx.userEnabledMathSDP() || !ctx.userEnabledCuDNNSDP())
+    return false;
+  if (ctx.sDPPriorityOrder() == initial) {
+    if (c10::cuda::device_count() == 0) return true;
+    static std::once_flag asked;
+    std::call_once(asked, [] {
+      const c10::impl::ExcludeDispatchKeyGuard unseen(c10::python_ks);       // no operator of the program's
+      const at::Tensor none = at::empty({1, 1, 0, 64}, at::TensorOptions().dtype(at::kHalf).device(at::kCUDA));
+      at::_fused_sdp_choice(none, none, none);
+    });
+  }
+  return ctx.sDPPriorityOrder() == settled;
 }
 // attention_back_ends_as_they_come() -> bool
 PyObject* attention_back_ends_as_they_come(PyObject*, PyObject* const*, Py_ssize_t) { return PyBool_FromLong(back_ends_as_they_come()); }

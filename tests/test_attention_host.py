@@ -60,7 +60,7 @@ def test_a_choice_among_the_librarys_back_ends_is_noticed(pkg):
         assert not untouched()
     with sdpa_kernel(every):
         assert untouched()
-    with sdpa_kernel(every[3:] + every[:3], set_priority=True):     # the framework's own once cuDNN is preferred
+    with sdpa_kernel(every[3:] + every[:3], set_priority=True):     # what the framework settles on
         assert untouched()
     assert untouched()
 

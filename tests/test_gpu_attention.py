@@ -1,10 +1,15 @@
 """The attention kernel between the qkv and proj linears and its form that also runs proj's activation quantizer: against an fp64
 evaluation and the library kernel, and -- for the quantizer form -- bit for bit against the quantizer kernel applied to the plain
 form's output.  Then where the modules take it, what they show of it, and where they take the library's attention."""
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
 import torch.nn.functional as F
+
+from conftest import ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -267,10 +272,16 @@ def test_a_dispatch_mode_sees_the_attention_operator(pkg, cuda_device):
     assert pkg.ops.device_status() == 0
 
 
+_BACK_ENDS = ("MATH", "EFFICIENT_ATTENTION", "FLASH_ATTENTION", "CUDNN_ATTENTION")
+
+
+# the slowest first; the order that the framework starts with and leaves when it is first asked for a back end
+@pytest.mark.parametrize("order", [(0, 1, 2, 3), (2, 1, 0, 3)])
 @pytest.mark.parametrize("native", [True, False])
 @torch.no_grad()
-def test_a_set_order_of_the_back_ends_is_kept(pkg, cuda_device, native, monkeypatch):
-    """All four back ends, the slowest first: the library's attention runs, in the model's one call and in the attention module."""
+def test_a_set_order_of_the_back_ends_is_kept(pkg, cuda_device, native, order, monkeypatch):
+    """All four back ends in an order of the program's: the library's attention runs, in the model's one call and in the attention
+    module."""
     from torch.nn.attention import SDPBackend, sdpa_kernel
     model, images, _ = _block(pkg, cuda_device)
     if not native:
@@ -279,12 +290,28 @@ def test_a_set_order_of_the_back_ends_is_kept(pkg, cuda_device, native, monkeypa
     monkeypatch.setattr(type(model.blocks[0].attn), "implementation", "kernel")
     assert torch.equal(model(images), own)                      # the library has run by now, in the calibration
     monkeypatch.setattr(type(model.blocks[0].attn), "implementation", "auto")
-    order = [SDPBackend.MATH, SDPBackend.EFFICIENT_ATTENTION, SDPBackend.FLASH_ATTENTION, SDPBackend.CUDNN_ATTENTION]
-    with sdpa_kernel(order, set_priority=True):
+    with sdpa_kernel([getattr(SDPBackend, _BACK_ENDS[i]) for i in order], set_priority=True):
         chosen = model(images)
         monkeypatch.setattr(type(model.blocks[0].attn), "implementation", "sdpa")
         assert torch.equal(chosen, model(images)) and not torch.equal(chosen, own)
     assert pkg.ops.device_status() == 0
+
+
+def test_the_order_of_a_fresh_process_is_no_choice(cuda_device):
+    """Before the library's attention has run, and after."""
+    code = """
+import sys; sys.path.insert(0, '.')
+import torch, __graft_entry__ as entry
+from torch.nn.attention import SDPBackend as B, sdpa_kernel
+untouched = entry.import_package()._cabi.host().attention_back_ends_as_they_come
+assert untouched()
+with sdpa_kernel([B.FLASH_ATTENTION, B.EFFICIENT_ATTENTION, B.MATH, B.CUDNN_ATTENTION], set_priority=True):
+    assert not untouched()
+q = torch.randn(1, 1, 8, 64, device='cuda').half()
+torch.nn.functional.scaled_dot_product_attention(q, q, q)
+assert untouched()
+"""
+    subprocess.run([sys.executable, "-c", code], cwd=ROOT, check=True)
 
 
 @torch.no_grad()
