@@ -265,6 +265,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
       tc_fence_after_sync();
       // Loops with one body each, not unrolled over the row: the softmax and output warps of two blocks share an instruction
       // cache, and unrolled passes stalled on it more than on anything else (DeiT-S batch 64, with the quantizer: 27.0 -> 24.1 us).
+      // The wait loops are part of that: with a constant limit instead of poll_limit 24.3 us against 21.4, 256 images of 12 heads 146
+      // against 113.
       float nm = 0.0f;
       if (live) {
         float m0 = ninf, m1 = ninf, m2 = ninf, m3 = ninf;

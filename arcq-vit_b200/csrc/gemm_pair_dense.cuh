@@ -56,7 +56,7 @@ struct PairDenseParams {
 constexpr int kPairDenseThreads = (2 + kPairEpiWarps) * 32;
 // The quantizer form has three epilogue warps per lane quarter, one per 64-column group of a 192-column slab.  The issuing warps
 // are a warp group of their own (two of its warps idle), whose registers the epilogue warps take over: 152 instead of the
-// launch's 128 ([12608, 3072] x 768 76.3 -> 75.1 us, [50432, 3072] x 768 357 -> 350 us).
+// launch's 128 (K = 768, N = 3072: 12608 rows 76.3 -> 75.1 us, 50432 rows 357 -> 350 us).  Neither role spills.
 constexpr int kPairQuantEpiWarps = 12, kPairQuantIssueWarps = 4;
 constexpr int kPairQuantThreads = (kPairQuantIssueWarps + kPairQuantEpiWarps) * 32;
 constexpr int kPairQuantLaunchRegs = 128, kPairQuantEpiRegs = 152, kPairQuantIssueRegs = 56;
@@ -286,8 +286,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
     // A thread owns one row and 64 columns, i.e. one group of the next layer's activation quantizer: tensor memory -> + bias ->
     // fp16 (what the plain form stores) -> GELU -> quantizer -> reconstruction, in registers but for the exchange of large GELU
     // arguments, then through this warp's staging rows to a TMA store.  Issue slots of these warps bound the kernel (about 30
-    // instructions a value); the products run underneath.  N = 3072, K = 768: M = 12608 72.9 us against 49.4 + 40.3 us for GEMM
-    // and quantizer kernel, M = 100864 618 against 457 + 407 us.
+    // instructions a value); the products run underneath.  K = 768, N = 3072, back to back with inputs in turn: 12608 rows 90.7 us
+    // against 101.4 for GEMM and quantizer kernel, 100864 rows 787 against 984.
     const int ew = warp - kIssue, lq = warp & 3, grp = ew >> 2;
     GroupQuantTables* const tables = reinterpret_cast<GroupQuantTables*>(smem + L.tables);
     for (int i = tid - kIssue * 32; i < bn; i += kEpi * 32) s_bias[i] = (p.bias != nullptr) ? __ldg(p.bias + n0 + i) : 0.0f;

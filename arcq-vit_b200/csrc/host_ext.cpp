@@ -447,8 +447,8 @@ PyObject* vit_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
   if (!read_norm(p->norm, dev, D, &norms[2 * depth], &held)) Py_RETURN_NONE;
   // The attention kernel, which also quantises for proj, instead of the library's attention and a quantizer launch: a whole forward
-  // of DeiT-S batch 64 1611 -> 1559 us, batch 8 786 -> 749, batch 1 equal, DeiT-T batch 37 867 -> 823, DeiT-B batch 1024 58.9 -> 57.7
-  // ms.  The library's where a sequence is too long for the kernel, and where its back ends were chosen among.
+  // of DeiT-S batch 64 1552 -> 1466 us, batch 8 679 -> 634, batch 1 488 -> 467, DeiT-T batch 37 785 -> 724, DeiT-B batch 256 14.14 ->
+  // 13.89 ms.  The library's where a sequence is too long for the kernel, and where its back ends were chosen among.
   const bool own_attention = T <= 256 && D == 64 * p->heads && back_ends_as_they_come();
   int64_t hidden = 0;
   for (size_t i = 0; i < depth; ++i) hidden = std::max(hidden, lin[4 * i + 2].N);

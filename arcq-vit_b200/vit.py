@@ -7,8 +7,8 @@ the linears.  This file is an independent skeleton with the same architecture fa
 multi-head self-attention and a GELU MLP, final LayerNorm, linear head -- and the parameter
 names the reference's tools rely on (``blocks.<i>.attn.qkv``, ``blocks.<i>.attn.proj``,
 ``blocks.<i>.mlp.fc1``, ``blocks.<i>.mlp.fc2``, ``head``).  Only the four linears of each block
-are quantised; patch embedding, LayerNorm, softmax attention, GELU and the head stay in
-floating point (ordinary PyTorch ops).
+are quantised; patch embedding, LayerNorm, softmax attention, GELU and the head stay in floating point: PyTorch ops, or on a
+GPU kernels of this package that give or quantise the same tensors.
 """
 from __future__ import annotations
 
