@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(AqtShape<T, WRITE_PACKED>::kThreads, AqtShape<
     if (WRITE_XHAT) tma_prefetch_desc(&tm_out);
   }
   // reads only the layer's constants, which no kernel of this library writes: done while the previous kernel still runs
-  const GroupQuantParams gp = group_quant_tables<L>(tables, thresholds, codebook, tid, S::kThreads,
+  const GroupQuantParams gp = group_quant_tables<L, WRITE_PACKED>(tables, thresholds, codebook, tid, S::kThreads,
                                                     [](bool b) { return __syncthreads_and(b) != 0; });
   const long long tiles = (total_groups + kGroups - 1) / kGroups;
   const long long stride = static_cast<long long>(gridDim.x - jobs.blocks) * S::kWarps;

@@ -6,6 +6,7 @@
 #pragma once
 #include <cuda_fp16.h>
 #include "ptx.cuh"
+#include "f32x2.cuh"
 
 namespace arcq {
 
@@ -138,86 +139,94 @@ __device__ __forceinline__ void layernorm_row_load(const __half* __restrict__ x,
   }
 }
 
-// The arithmetic of one row on chunks already loaded (`has_y`: b holds the residual branch).
+// gamma and beta of the lane's three chunks
+struct LaneNorm {
+  f32x2 g[3][4], b[3][4];
+};
+template <int LANES> __device__ __forceinline__ void layernorm_lane_params(const NormParams& np, int l, LaneNorm* n) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    float g[8], b[8];
+    load_norm_chunk(np.gamma, np.dtype, l + LANES * i, g);
+    load_norm_chunk(np.beta, np.dtype, l + LANES * i, b);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      n->g[i][j] = pack2(g[2 * j], g[2 * j + 1]);
+      n->b[i][j] = pack2(b[2 * j], b[2 * j + 1]);
+    }
+  }
+}
+
+// The sum of a chunk's eight values (SQUARES: of their squares).  A row's sum is taken chunk by chunk, then over the lane's chunks,
+// then over the lanes, so that a kernel that holds the row in another layout can add in the same order.
+template <bool SQUARES> __device__ __forceinline__ float layernorm_chunk_sum(const f32x2 (&v)[4]) {
+  float lo, hi;
+  if (SQUARES) unpack2(fma2(v[3], v[3], fma2(v[2], v[2], fma2(v[1], v[1], mul2(v[0], v[0])))), lo, hi);
+  else unpack2(add2(add2(v[0], v[1]), add2(v[2], v[3])), lo, hi);
+  return lo + hi;
+}
+__device__ __forceinline__ float layernorm_rstd(float squares, float k_inv, float eps) { return rsqrtf(squares * k_inv + eps); }
+
+// The arithmetic of one row on chunks already loaded (`has_y`: b holds the residual branch).  Two values per instruction; the sum of
+// two fp16 values rounded once is what the fp32 sum rounds to (their bits span less than fp32 holds wherever that could tie).
+// About 10 instructions a value, loads and stores included; with scalar arithmetic on converted values it was 20.
 template <int LANES>
 __device__ __forceinline__ void layernorm_row_compute(const uint4 (&a)[3], const uint4 (&b)[3], bool has_y,
-                                                      long long row, bool valid, int l, const float (&gg)[3][8],
-                                                      const float (&bb)[3][8], float eps,
+                                                      long long row, bool valid, int l, const LaneNorm& n, float eps,
                                                       __half* __restrict__ sum_out, uint4 (&h)[3]) {
   constexpr int K = LANES * 24;
-  const bool yr = has_y;
-  float v[3][8];
+  constexpr float kInv = 1.0f / static_cast<float>(K);
+  f32x2 v[3][4];
   float sum = 0.0f;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const __half2* ah = reinterpret_cast<const __half2*>(&a[i]);
-    if (yr) {
-      const __half2* bh = reinterpret_cast<const __half2*>(&b[i]);
-      uint4 so;
-      __half2* sh = reinterpret_cast<__half2*>(&so);
+    uint32_t s[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+    if (has_y) {
+      const uint32_t t[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float2 fa = __half22float2(ah[j]), fb = __half22float2(bh[j]);
-        sh[j] = __floats2half2_rn(fa.x + fb.x, fa.y + fb.y);   // the fp16 sum a separate add would store
-        const float2 fs = __half22float2(sh[j]);
-        v[i][2 * j] = fs.x;
-        v[i][2 * j + 1] = fs.y;
+        const __half2 r = __hadd2(*reinterpret_cast<const __half2*>(&s[j]), *reinterpret_cast<const __half2*>(&t[j]));
+        s[j] = *reinterpret_cast<const uint32_t*>(&r);
       }
-      if (valid && sum_out != nullptr) reinterpret_cast<uint4*>(sum_out + row * K)[l + LANES * i] = so;
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 fa = __half22float2(ah[j]);
-        v[i][2 * j] = fa.x;
-        v[i][2 * j + 1] = fa.y;
-      }
+      if (valid && sum_out != nullptr) reinterpret_cast<uint4*>(sum_out + row * K)[l + LANES * i] = make_uint4(s[0], s[1], s[2], s[3]);
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) sum += v[i][j];
+    for (int j = 0; j < 4; ++j) v[i][j] = sixteen_to_pair<__half>(s[j]);
+    const float c = layernorm_chunk_sum<false>(v[i]);
+    sum = i == 0 ? c : sum + c;
   }
 #pragma unroll
   for (int o = LANES / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  const float mean = sum * (1.0f / static_cast<float>(K));
+  const float nm = -(sum * kInv);
+  const f32x2 nm2 = pack2(nm, nm);
   float sq = 0.0f;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float d = v[i][j] - mean;
-      sq += d * d;
-    }
+    for (int j = 0; j < 4; ++j) v[i][j] = add2(v[i][j], nm2);
+    const float c = layernorm_chunk_sum<true>(v[i]);
+    sq = i == 0 ? c : sq + c;
   }
 #pragma unroll
   for (int o = LANES / 2; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-  const float rstd = rsqrtf(sq * (1.0f / static_cast<float>(K)) + eps);
+  const float rstd = layernorm_rstd(sq, kInv, eps);
+  const f32x2 rstd2 = pack2(rstd, rstd);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    __half2* oh = reinterpret_cast<__half2*>(&h[i]);
+    uint32_t w[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      oh[j] = __floats2half2_rn((v[i][2 * j] - mean) * rstd * gg[i][2 * j] + bb[i][2 * j],
-                                (v[i][2 * j + 1] - mean) * rstd * gg[i][2 * j + 1] + bb[i][2 * j + 1]);
+    for (int j = 0; j < 4; ++j) w[j] = pair_to_sixteen<__half>(fma2(mul2(v[i][j], rstd2), n.g[i][j], n.b[i][j]));
+    h[i] = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
 template <int LANES>
 __device__ __forceinline__ void layernorm_row(const __half* __restrict__ x, const __half* __restrict__ y, long long rs,
-                                              long long row, bool valid, int l, const float (&gg)[3][8],
-                                              const float (&bb)[3][8], float eps, __half* __restrict__ sum_out,
-                                              uint4 (&h)[3]) {
+                                              long long row, bool valid, int l, const LaneNorm& n, float eps,
+                                              __half* __restrict__ sum_out, uint4 (&h)[3]) {
   uint4 a[3], b[3];
   layernorm_row_load<LANES>(x, y, rs, l, a, b);
-  layernorm_row_compute<LANES>(a, b, y != nullptr, row, valid, l, gg, bb, eps, sum_out, h);
-}
-
-// gamma and beta of the lane's three chunks
-template <int LANES>
-__device__ __forceinline__ void layernorm_lane_params(const NormParams& np, int l, float (&gg)[3][8], float (&bb)[3][8]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    load_norm_chunk(np.gamma, np.dtype, l + LANES * i, gg[i]);
-    load_norm_chunk(np.beta, np.dtype, l + LANES * i, bb[i]);
-  }
+  layernorm_row_compute<LANES>(a, b, y != nullptr, row, valid, l, n, eps, sum_out, h);
 }
 
 // Residual add + LayerNorm for rows of LANES * 24 values: LANES lanes per row, so every lane carries the same load
@@ -233,8 +242,8 @@ __global__ void __launch_bounds__(256) add_layernorm_rows_kernel(const __half* _
 
   constexpr int K = LANES * 24, kRowsPerWarp = 32 / LANES;
   const int lane = threadIdx.x & 31, l = lane % LANES, sub = lane / LANES;
-  float gg[3][8], bb[3][8];
-  layernorm_lane_params<LANES>(np, l, gg, bb);
+  LaneNorm n;
+  layernorm_lane_params<LANES>(np, l, &n);
   pdl_wait();                // gamma and beta are the layer's constants; x and y may be the previous kernel's output
   const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
   const long long first = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kRowsPerWarp;
@@ -244,7 +253,7 @@ __global__ void __launch_bounds__(256) add_layernorm_rows_kernel(const __half* _
     const long long rs = valid ? row : M - 1;          // idle sub-warps shadow the last row, store nothing
     uint4 h[3];
     const long long skip = rs * (ld - K);              // input rows are ld values apart
-    layernorm_row<LANES>(x + skip, y != nullptr ? y + skip : nullptr, rs, row, valid, l, gg, bb, eps, sum_out, h);
+    layernorm_row<LANES>(x + skip, y != nullptr ? y + skip : nullptr, rs, row, valid, l, n, eps, sum_out, h);
     if (valid) {
 #pragma unroll
       for (int i = 0; i < 3; ++i) reinterpret_cast<uint4*>(h_out + row * K)[l + LANES * i] = h[i];

@@ -1401,7 +1401,6 @@ int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const void
   const long long tiles = (M * G + arcq::kLnqThreads - 1) / arcq::kLnqThreads;
   const long long cap = static_cast<long long>(sm_count()) * 4;
   const unsigned grid = static_cast<unsigned>((tiles < cap ? tiles : cap) + jobs.blocks);
-  const size_t smem = arcq::lnq_smem_bytes();
   const __half *xh = static_cast<const __half*>(x), *yh = static_cast<const __half*>(y);
   __half *so = static_cast<__half*>(sum_out), *ho = static_cast<__half*>(h_out);
   if (M * G >= (1ll << 30)) return fail(ARCQ_E_TOO_LARGE, "too many groups");
@@ -1409,9 +1408,23 @@ int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const void
   if (!make_tensor_map_2d(&tm_out, xhat, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, static_cast<uint64_t>(M * G), 64, 64, 32,
                           CU_TENSOR_MAP_SWIZZLE_128B))
     return fail(ARCQ_E_CUDA, "cuTensorMapEncodeTiled failed for the reconstruction");
+  int* const status = status_ptr();
+  if (status == nullptr) return fail(ARCQ_E_CUDA, "device status word not reachable");
 #define ARCQ_LAUNCH_LNQ(LN, B, HASY)                                                                                   \
-  launch_pdl(arcq::add_layernorm_act_quant_kernel<LN, B, HASY>, grid, arcq::kLnqThreads, smem, st, tm_out, xh, yh, np, \
-             eps, static_cast<long long>(M), thresholds, codebook, so, ho, one_fma, jobs)
+  do {                                                                                                                 \
+    auto k = arcq::add_layernorm_act_quant_kernel<LN, B, HASY>;                                                        \
+    constexpr int smem = arcq::lnq_smem_layout(LN, HASY).total;                                                        \
+    static thread_local int done_dev = -1;      /* shared-memory ceiling raised once per (host thread, device) */      \
+    int dev = 0;                                                                                                       \
+    cudaGetDevice(&dev);                                                                                               \
+    if (done_dev != dev) {                                                                                             \
+      const cudaError_t e1 = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);               \
+      if (e1 != cudaSuccess) return cuda_fail(e1, "add_layernorm_act_quant");                                          \
+      done_dev = dev;                                                                                                  \
+    }                                                                                                                  \
+    launch_pdl(k, grid, arcq::kLnqThreads, smem, st, tm_out, xh, yh, np, eps, static_cast<long long>(M), thresholds,   \
+               codebook, so, ho, one_fma, status, jobs);                                                               \
+  } while (0)
 #define ARCQ_LNQ_BITS(LN, HASY)                                                                                         \
   do {                                                                                                                  \
     if (bits == 4) ARCQ_LAUNCH_LNQ(LN, 4, HASY);                                                                         \

@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
     GroupQuantParams gp = {};
     // reads only the layer's constants: done while the previous kernel still runs
     if (QUANT)
-      gp = group_quant_tables<1 << BITS>(tables, p.thresholds, p.codebook, tid - 128, kAttnRowWarps * 32, [](bool b) {
+      gp = group_quant_tables<1 << BITS, false>(tables, p.thresholds, p.codebook, tid - 128, kAttnRowWarps * 32, [](bool b) {
         asm volatile("bar.sync 1, %0;" ::"n"(kAttnRowWarps * 32) : "memory");
         return b;
       });

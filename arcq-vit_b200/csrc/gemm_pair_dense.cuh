@@ -291,7 +291,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
     const int ew = warp - kIssue, lq = warp & 3, grp = ew >> 2;
     GroupQuantTables* const tables = reinterpret_cast<GroupQuantTables*>(smem + L.tables);
     for (int i = tid - kIssue * 32; i < bn; i += kEpi * 32) s_bias[i] = (p.bias != nullptr) ? __ldg(p.bias + n0 + i) : 0.0f;
-    const GroupQuantParams gp = group_quant_tables<1 << QBITS>(tables, p.thresholds, p.codebook, tid - kIssue * 32, kEpi * 32, [](bool b) {
+    const GroupQuantParams gp = group_quant_tables<1 << QBITS, false>(tables, p.thresholds, p.codebook, tid - kIssue * 32, kEpi * 32, [](bool b) {
       asm volatile("bar.sync 2, %0;" ::"n"(kEpi * 32) : "memory");
       return b;
     });

@@ -27,49 +27,10 @@
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 #include "ptx.cuh"
+#include "f32x2.cuh"
 #include "act_quant.cuh"
 
 namespace arcq {
-
-// ---------------------------------------------------------------- two fp32 values per instruction
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-  f32x2 d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
-  return d;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-// A packed mul whose result feeds a packed add is contracted into one fma by the assembler, .rn on both notwithstanding (one
-// rounding instead of two: a scale came out one unit in the last place off).  Where that matters, mul2_rn adds a -0 that
-// the compiler cannot see (GroupQuantParams::nz), which leaves every product as it is.
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ f32x2 mul2_rn(f32x2 a, f32x2 b, f32x2 nz) { return fma2(a, b, nz); }
-__device__ __forceinline__ f32x2 fma2_down(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ float min3_abs(float m, float a, float b) {
-  float d;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(m), "f"(fabsf(a)), "f"(fabsf(b)));
-  return d;
-}
 
 // a + OFFSET where d > 0
 template <uint32_t OFFSET> __device__ __forceinline__ uint32_t offset_if_positive(uint32_t a, float d) {
@@ -79,14 +40,16 @@ template <uint32_t OFFSET> __device__ __forceinline__ uint32_t offset_if_positiv
 
 // ---------------------------------------------------------------- per-layer tables in shared memory
 constexpr int kGqCells = 256;
-struct GroupQuantTables {            // 4 KB + 132 bytes; placed on a 1 KB boundary, so that cell offset and base merge in one OR
+struct GroupQuantTables {            // 3 KB + 144 bytes, 1 KB more with codes; placed on a 1 KB boundary, so that cell offset and base merge in one OR
   float cell_nth[kGqCells];          // minus the threshold that a value of the cell can be above or below
   float cell_lo[kGqCells];           // the level below that threshold ...
   float cell_hi[kGqCells];           // ... and above
-  uint32_t cell_code4[kGqCells];     // 4 * (code below the threshold), for kernels that also write codes
   float th[16], cb[16];              // +inf padded thresholds, levels
   float nz;                          // -0
+  float pad[3];
+  uint32_t cell_code4[kGqCells];     // 4 * (code below the threshold); only kernels that also write codes have it
 };
+constexpr uint32_t kGroupQuantTableBytes = 3 * kGqCells * 4 + 144;        // without it
 struct GroupQuantParams {            // the same in every thread of the block
   float cells_per_unit;              // 4 or 8
   float tie;                         // times s: the |d| up to which a chunk takes the exact path (inf: always)
@@ -95,7 +58,7 @@ struct GroupQuantParams {            // the same in every thread of the block
 
 // Fills the tables; `sync_and(bool)` is a barrier over exactly the `nthreads` calling threads (numbered `tid`) that
 // returns the conjunction of its arguments.  Ends with a barrier: the tables are complete on return.
-template <int L, typename SyncAnd>
+template <int L, bool CODES, typename SyncAnd>
 __device__ __forceinline__ GroupQuantParams group_quant_tables(GroupQuantTables* t, const float* __restrict__ thresholds,
                                                                const float* __restrict__ codebook, int tid, int nthreads,
                                                                SyncAnd sync_and) {
@@ -130,7 +93,7 @@ __device__ __forceinline__ GroupQuantParams group_quant_tables(GroupQuantTables*
     t->cell_nth[k] = -t->th[c];                               // c == L - 1: -inf, nothing is above it
     t->cell_lo[k] = t->cb[c];
     t->cell_hi[k] = t->cb[c + 1 < L ? c + 1 : L - 1];
-    t->cell_code4[k] = 4u * static_cast<uint32_t>(c);
+    if (CODES) t->cell_code4[k] = 4u * static_cast<uint32_t>(c);
   }
   p.nz = pack2(t->nz, t->nz);
   sync_and(true);
@@ -205,7 +168,7 @@ __device__ __forceinline__ GroupStats group_quantize(f32x2 (&v)[32 / LPG], const
   const f32x2 a2 = pack2(a, a), s2 = pack2(s, s), magic = pack2(3145728.0f + 128.0f, 3145728.0f + 128.0f);
   const float tie = __fmul_rn(p.tie, s);
   const uint32_t tab = smem_u32(t);
-  constexpr uint32_t kLo = kGqCells * 4, kHi = 2 * kGqCells * 4, kCode = 3 * kGqCells * 4, kCb = 4 * kGqCells * 4 + 64;
+  constexpr uint32_t kLo = kGqCells * 4, kHi = 2 * kGqCells * 4, kCode = kGroupQuantTableBytes, kCb = 3 * kGqCells * 4 + 64;
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
     float m = 1.0e38f, out[CH], d[CH];
@@ -275,29 +238,7 @@ __device__ __forceinline__ f32x2 group_recon_pair(const GroupRecon& g, f32x2 lev
   return add2(g.c, fma2(g.scale, add2(level, g.a), g.b));
 }
 
-// ---------------------------------------------------------------- 16-bit element types and rows in shared memory
-template <typename T> __device__ __forceinline__ f32x2 sixteen_to_pair(uint32_t w);
-template <> __device__ __forceinline__ f32x2 sixteen_to_pair<__half>(uint32_t w) {
-  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
-  return pack2(f.x, f.y);
-}
-template <> __device__ __forceinline__ f32x2 sixteen_to_pair<__nv_bfloat16>(uint32_t w) {
-  return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
-}
-template <typename T> __device__ __forceinline__ uint32_t pair_to_sixteen(f32x2 v);
-template <> __device__ __forceinline__ uint32_t pair_to_sixteen<__half>(f32x2 v) {
-  float a, b;
-  unpack2(v, a, b);
-  const __half2 h = __floats2half2_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
-template <> __device__ __forceinline__ uint32_t pair_to_sixteen<__nv_bfloat16>(f32x2 v) {
-  float a, b;
-  unpack2(v, a, b);
-  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
-
+// ---------------------------------------------------------------- rows in shared memory
 // The lane's part of a group's 128-byte row, 16-byte chunk c at ((c ^ x7) << 4): w[c * PJ + j] = the 32-bit word of pair j.
 // With two lanes `row` already includes 8 * h.
 template <int LPG>

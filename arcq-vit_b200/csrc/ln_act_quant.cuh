@@ -5,6 +5,10 @@
 //   xhat = fp16(reconstruction of the ARCQ quantization of h in groups of 64)
 // The separate kernels write h and read it back; here it goes through shared memory.
 //
+// Bound by HBM for large inputs: [201728, 768] 211 us, 1.24 GB at 5.9 TB/s of the 6.5 a copy reaches ([50432, 768] 57.5 us, [12608, 384]
+// 10.7 us).  253, 67.3 and 11.2 us with rows read by ordinary loads, whose latency every pass of phase 1 waited for, and with scalar
+// arithmetic (36 instructions a value instead of 26).
+//
 // Two phases per tile, each in the thread layout that suits it, and each with the arithmetic of the kernel it
 // replaces, so that the results are bit-identical to arcq_add_layernorm followed by arcq_act_quant:
 //   1. LayerNorm with the lane layout of add_layernorm_rows_kernel (LANES lanes per row, 16-byte accesses, the same
@@ -27,98 +31,126 @@
 namespace arcq {
 
 constexpr int kLnqThreads = 128;
+constexpr int kStatusLnqTimeout = 0x411;
 
-__host__ __device__ constexpr size_t lnq_smem_bytes() {
-  return 1024 /* alignment */ + kLnqThreads * 128 /* h, then reconstruction: one group per row, 128-byte swizzle */ +
-         sizeof(GroupQuantTables);
+// Rows that a tile of 128 groups can touch, and the block's shared memory: h and then the reconstruction, one group per row with the
+// 128-byte swizzle; the tables; the tile's rows of x and y.  57.5 KB at most with what the system takes of each block: four an SM.
+__host__ __device__ constexpr int lnq_max_rows(int lanes) { return kLnqThreads / (lanes * 24 / 64) + 2; }
+struct LnqSmem {
+  uint32_t tables, bar, x, y, total;
+};
+__host__ __device__ constexpr LnqSmem lnq_smem_layout(int lanes, bool has_y) {
+  LnqSmem s = {};
+  const uint32_t rows = static_cast<uint32_t>(lnq_max_rows(lanes) * lanes * 48);
+  s.tables = kLnqThreads * 128;
+  s.bar = s.tables + kGroupQuantTableBytes;
+  s.x = s.bar + 16;
+  s.y = s.x + rows;
+  s.total = s.y + (has_y ? rows : 0);
+  return s;
 }
+static_assert(lnq_smem_layout(8, true).total <= 57344 && lnq_smem_layout(16, true).total <= 57344 && lnq_smem_layout(32, true).total <= 57344,
+              "four blocks an SM");
 
 template <int LANES, int BITS, bool HAS_Y>
 __global__ void __launch_bounds__(kLnqThreads, 4)
     add_layernorm_act_quant_kernel(const __grid_constant__ CUtensorMap tm_out, const __half* __restrict__ x,
                                    const __half* __restrict__ y, const NormParams np, float eps, long long M,
                                    const float* __restrict__ thresholds, const float* __restrict__ codebook,
-                                   __half* __restrict__ sum_out, __half* __restrict__ h_out, int one_fma,
+                                   __half* __restrict__ sum_out, __half* __restrict__ h_out, int one_fma, int* status,
                                    const __grid_constant__ UnpackJobs jobs) {
   pdl_launch_dependents();   // the next kernel of the stream may start its set-up
+  extern __shared__ __align__(1024) uint8_t lnq_smem[];
   if (static_cast<int>(blockIdx.x) < jobs.blocks) {
-    unpack_jobs_block(jobs);
+    unpack_jobs_run(jobs, static_cast<int>(blockIdx.x), reinterpret_cast<float*>(lnq_smem));
     return;
   }
 
   constexpr int L = 1 << BITS;
   constexpr int K = LANES * 24, G = K / 64, kRowsPerWarp = 32 / LANES, kRowsPerPass = 4 * kRowsPerWarp;
-  constexpr int kMaxRows = kLnqThreads / G + 2;                       // rows a tile of 128 groups can touch
-  constexpr int kPasses = (kMaxRows + kRowsPerPass - 1) / kRowsPerPass;
-  extern __shared__ uint8_t lnq_smem_raw[];
-  uint8_t* const s_rows = lnq_smem_raw + ((1024u - (smem_u32(lnq_smem_raw) & 1023u)) & 1023u);
-  GroupQuantTables* const tables = reinterpret_cast<GroupQuantTables*>(s_rows + kLnqThreads * 128);
+  constexpr int kPasses = (lnq_max_rows(LANES) + kRowsPerPass - 1) / kRowsPerPass;
+  constexpr LnqSmem S = lnq_smem_layout(LANES, HAS_Y);
+  GroupQuantTables* const tables = reinterpret_cast<GroupQuantTables*>(lnq_smem + S.tables);
+  uint64_t* const bar = reinterpret_cast<uint64_t*>(lnq_smem + S.bar);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, l = lane % LANES, sub = lane / LANES;
-  if (tid == 0) tma_prefetch_desc(&tm_out);
+  if (tid == 0) {
+    mbar_init(bar, 1);
+    mbar_fence_init();
+    tma_prefetch_desc(&tm_out);
+  }
   // reads only this layer's constants, so it runs before the wait below
-  const GroupQuantParams gp = group_quant_tables<L>(tables, thresholds, codebook, tid, kLnqThreads,
-                                                    [](bool b) { return __syncthreads_and(b) != 0; });
-
-  pdl_wait();                // x and y may be the previous kernels' outputs
+  const GroupQuantParams gp = group_quant_tables<L, false>(tables, thresholds, codebook, tid, kLnqThreads,
+                                                           [](bool b) { return __syncthreads_and(b) != 0; });
 
   const long long total_groups = M * G;
   const long long tiles = (total_groups + kLnqThreads - 1) / kLnqThreads;
-  for (long long tile = blockIdx.x - jobs.blocks; tile < tiles; tile += gridDim.x - jobs.blocks) {
+  const long long stride = gridDim.x - jobs.blocks;
+  // The rows of a tile, contiguous in x and in y, come by one bulk copy each: all of them are on their way at once, and the next
+  // tile's while this one is quantised.  (A copy and a barrier for each pass, so that the first pass starts early: no better where a
+  // block has one tile, [201728, 768] 222 us instead of 211.)
+  auto load = [&](long long tile) {
+    const long long gi0 = tile * kLnqThreads, r0 = gi0 / G, r1 = min(gi0 + kLnqThreads - 1, total_groups - 1) / G;
+    const uint32_t bytes = static_cast<uint32_t>((r1 - r0 + 1) * (K * 2));
+    mbar_arrive_expect_tx(bar, HAS_Y ? 2 * bytes : bytes);
+    bulk_load_1d(lnq_smem + S.x, x + r0 * K, bytes, bar);
+    if (HAS_Y) bulk_load_1d(lnq_smem + S.y, y + r0 * K, bytes, bar);
+  };
+  pdl_wait();                // x and y may be the previous kernels' outputs
+  long long tile = static_cast<long long>(blockIdx.x) - jobs.blocks;
+  if (tid == 0 && tile < tiles) load(tile);
+  uint32_t ph = 0;
+  bool ok = true;
+  for (; tile < tiles; tile += stride, ph ^= 1) {
     const long long gi0 = tile * kLnqThreads;
     const int ngroups = static_cast<int>(min(static_cast<long long>(kLnqThreads), total_groups - gi0));
     const long long r_first = gi0 / G;
     // ---- phase 1: LayerNorm of every row the tile touches, LANES lanes per row
-    {
-      float gg[3][8], bb[3][8];
-      layernorm_lane_params<LANES>(np, l, gg, bb);
-      // (issuing the loads of all passes before the first pass computes was tried: 72 more live registers, spills,
-      // 13.5 us instead of 11.3 us; one pass ahead, with gamma and beta re-read per pass to make room: 11.4 us, no gain)
+    LaneNorm norm;                          // read for each tile: the quantizer needs the registers
+    layernorm_lane_params<LANES>(np, l, &norm);
+    ok = ok && mbar_wait(bar, ph);          // (given up once: the block goes on without waiting, and says so below)
 #pragma unroll 1
-      for (int pass = 0; pass < kPasses; ++pass) {
-        const long long row = r_first + pass * kRowsPerPass + warp * kRowsPerWarp + sub;
-        const long long lg0 = row * G - gi0;                       // tile-local index of the row's first group
-        const bool in_tile = row < M && lg0 < ngroups;             // the row has groups in this tile
-        const bool owned = in_tile && lg0 >= 0;                    // ... and its first group is one of them
-        const long long rs = row < M ? row : M - 1;                // idle sub-warps shadow the last row
-        uint4 h[3];
-        layernorm_row<LANES>(x, HAS_Y ? y : nullptr, rs, row, owned, l, gg, bb, eps, sum_out, h);
-        if (in_tile) {
+    for (int pass = 0; pass < kPasses; ++pass) {
+      const int lr = pass * kRowsPerPass + warp * kRowsPerWarp + sub;
+      const long long row = r_first + lr;
+      const long long lg0 = row * G - gi0;                       // tile-local index of the row's first group
+      const bool in_tile = row < M && lg0 < ngroups;             // the row has groups in this tile
+      const bool owned = in_tile && lg0 >= 0;                    // ... and its first group is one of them
+      const int off = (in_tile ? lr : 0) * (K * 2) + l * 16;     // idle sub-warps shadow the first row
+      uint4 a[3], b[3], h[3];
 #pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            const int ch = l + LANES * i;                          // 16-byte chunk of the row: group ch / 8, part ch % 8
-            const int lg = static_cast<int>(lg0) + (ch >> 3);
-            if (lg >= 0 && lg < ngroups)
-              *reinterpret_cast<uint4*>(s_rows + lg * 128 + (((ch ^ lg) & 7) << 4)) = h[i];
-            if (owned && h_out != nullptr) reinterpret_cast<uint4*>(h_out + row * K)[ch] = h[i];
-          }
+      for (int i = 0; i < 3; ++i) {
+        a[i] = *reinterpret_cast<const uint4*>(lnq_smem + S.x + off + LANES * 16 * i);
+        if (HAS_Y) b[i] = *reinterpret_cast<const uint4*>(lnq_smem + S.y + off + LANES * 16 * i);
+      }
+      layernorm_row_compute<LANES>(a, b, HAS_Y, row, owned, l, norm, eps, sum_out, h);
+      if (in_tile) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const int ch = l + LANES * i;                          // 16-byte chunk of the row: group ch / 8, part ch % 8
+          const int lg = static_cast<int>(lg0) + (ch >> 3);
+          if (lg >= 0 && lg < ngroups)
+            *reinterpret_cast<uint4*>(lnq_smem + lg * 128 + (((ch ^ lg) & 7) << 4)) = h[i];
+          if (owned && h_out != nullptr) reinterpret_cast<uint4*>(h_out + row * K)[ch] = h[i];
         }
       }
     }
-    if (tid == 0) {
-      // the rows of this block's next tile: from HBM to L2 while this one is quantised (the loads of a tile start after a barrier,
-      // with nothing else of the block to do: [50432, 768] 73.3 -> 68.2 us, [201728, 768] 277 -> 257 us)
-      const long long next = (tile + gridDim.x - jobs.blocks) * kLnqThreads, end = min(next + kLnqThreads, total_groups);
-      if (next < end) {
-        const uint32_t bytes = static_cast<uint32_t>((end - next) * 128);
-        bulk_prefetch_l2(x + next * 64, bytes);
-        if (HAS_Y) bulk_prefetch_l2(y + next * 64, bytes);
-      }
-    }
     __syncthreads();
+    if (tid == 0 && tile + stride < tiles) load(tile + stride);
 
     // ---- phase 2: the activation quantizer on h, one thread per group, in place; a warp sends its 32 rows out by TMA
     // (rows of the last tile beyond the matrix hold stale values; the store clips them)
-    if (tid < ngroups) group_quantize_row<__half, BITS, false, 1>(smem_u32(s_rows) + tid * 128, lane & 7, tables, gp, one_fma != 0);
+    if (tid < ngroups) group_quantize_row<__half, BITS, false, 1>(smem_u32(lnq_smem) + tid * 128, lane & 7, tables, gp, one_fma != 0);
     fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) {
-      tma_store_2d(&tm_out, s_rows + warp * 4096, 0, static_cast<int>(gi0) + warp * 32);
+      tma_store_2d(&tm_out, lnq_smem + warp * 4096, 0, static_cast<int>(gi0) + warp * 32);
       tma_store_commit();
       tma_store_wait_read();
     }
     __syncthreads();   // the rows are free for the next tile
   }
   if (lane == 0) tma_store_wait_all();
+  if (!ok && tid == 0) atomicExch(status, kStatusLnqTimeout);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -135,7 +167,7 @@ __global__ void __launch_bounds__(kLnqThreads, 4)
 constexpr int kLnqRowsThreads = 384;
 
 template <int LANES, int BITS, bool HAS_Y>
-__global__ void __launch_bounds__(kLnqRowsThreads) add_layernorm_act_quant_rows_kernel(const __half* __restrict__ x,
+__global__ void __launch_bounds__(kLnqRowsThreads, 1) add_layernorm_act_quant_rows_kernel(const __half* __restrict__ x,
                                                                           const __half* __restrict__ y,
                                                                           const NormParams np, float eps,
                                                                           long long M,
@@ -162,8 +194,8 @@ __global__ void __launch_bounds__(kLnqRowsThreads) add_layernorm_act_quant_rows_
     s_th[tid] = (tid < L - 1) ? thresholds[tid] : __int_as_float(0x7f800000);
     s_cb[tid] = (tid < L) ? codebook[tid] : 0.0f;
   }
-  float gg[3][8] = {}, bb[3][8] = {};
-  if (warp < 4) layernorm_lane_params<LANES>(np, l, gg, bb);
+  LaneNorm norm = {};
+  if (warp < 4) layernorm_lane_params<LANES>(np, l, &norm);
   __syncthreads();
   pdl_wait();                // everything above is the layer's constants; x and y may be the previous kernel's output
 
@@ -176,7 +208,7 @@ __global__ void __launch_bounds__(kLnqRowsThreads) add_layernorm_act_quant_rows_
       const bool valid = row < M;
       const long long rs = valid ? row : M - 1;
       uint4 h[3];
-      layernorm_row<LANES>(x, HAS_Y ? y : nullptr, rs, row, valid, l, gg, bb, eps, sum_out, h);
+      layernorm_row<LANES>(x, HAS_Y ? y : nullptr, rs, row, valid, l, norm, eps, sum_out, h);
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
         reinterpret_cast<uint4*>(s_hid + local * K)[l + LANES * i] = h[i];
