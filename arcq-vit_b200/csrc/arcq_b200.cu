@@ -590,6 +590,13 @@ template <typename Kernel> int max_resident_dense_pairs(Kernel kernel, int threa
   return n;
 }
 
+// Pairs of a launch: as many for each slab that stays, else up to one for each (row tile, slab).
+long long dense_pairs(long long slabs, long long tiles_m, long long max_pairs, bool stationary) {
+  if (!stationary) return slabs * tiles_m < max_pairs ? slabs * tiles_m : max_pairs;
+  const long long per = max_pairs / slabs;
+  return slabs * (per < tiles_m ? per : tiles_m);
+}
+
 // Slab width, stages and grid for the dense-weight pair kernel; false leaves the shape to the one-CTA kernel.
 // Cost model in microseconds: a tile is bound by its output stores (about 22 GB/s per SM) or by the issuing thread, and every slab
 // streams the whole activation from L2.
@@ -637,14 +644,15 @@ bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32,
     if (slabs > max_pairs) continue;
     long long per = max_pairs / slabs;
     if (per > tiles_m) per = tiles_m;
-    const long long tiles_pp = (tiles_m + per - 1) / per;
     const int esize = y_f32 ? 4 : 2;
     const double t_write = 128.0 * bn * esize / 22.0e3;
     for (int stationary = 1; stationary >= 0; --stationary) {
       if (opt(O_PAIR_STATIONARY) >= 0 && stationary != opt(O_PAIR_STATIONARY)) continue;
       if (stationary && G > 32) continue;
       PairDenseConfig k = {};
-      k.bn = bn; k.pairs = static_cast<int>(slabs * per); k.stationary = stationary;
+      k.bn = bn; k.stationary = stationary;
+      k.pairs = static_cast<int>(dense_pairs(slabs, tiles_m, max_pairs, stationary));
+      const long long tiles_pp = stationary ? (tiles_m + per - 1) / per : (slabs * tiles_m + k.pairs - 1) / k.pairs;
       k.ks = (G % 2 == 0) ? 2 : (G % 3 == 0) ? 3 : 1;
       if (opt(O_PAIR_KS) > 0 && G % opt(O_PAIR_KS) == 0) k.ks = opt(O_PAIR_KS);
       bool fits = false;
@@ -693,15 +701,14 @@ bool choose_pair_quant_config(long long M, long long N, long long K, PairDenseCo
     if (slabs > max_pairs) continue;
     long long per = max_pairs / slabs;
     if (per > tiles_m) per = tiles_m;
-    const long long tiles_pp = (tiles_m + per - 1) / per;
     // The epilogue bounds every tile: one, two or three warps per scheduler share its issue slots (a single tile of
     // 64 / 128 / 192 columns, K = 384: 8.7 / 9.8 / 11.4 us).
-    const double cost = tiles_pp * (2.5 + 0.9 * (bn / 64));
-    if (found && cost >= c->cost) continue;
     for (int stationary = 1; stationary >= 0; --stationary) {
-      if (stationary && (G > 32 || tiles_pp < 3)) continue;    // too few tiles to pay for loading the whole slab first
       PairDenseConfig k = {};
-      k.bn = bn; k.pairs = static_cast<int>(slabs * per); k.stationary = stationary;
+      k.bn = bn; k.stationary = stationary;
+      k.pairs = static_cast<int>(dense_pairs(slabs, tiles_m, max_pairs, stationary));
+      const long long tiles_pp = stationary ? (tiles_m + per - 1) / per : (slabs * tiles_m + k.pairs - 1) / k.pairs;
+      if (stationary && (G > 32 || tiles_pp < 3)) continue;    // too few tiles to pay for loading the whole slab first
       k.ks = (G % 2 == 0) ? 2 : (G % 3 == 0) ? 3 : 1;
       bool fits = false;
       for (int sa = 8 / k.ks; sa >= 2 && !fits; --sa) {
@@ -709,10 +716,10 @@ bool choose_pair_quant_config(long long M, long long N, long long K, PairDenseCo
         if (need <= kSmemBudget) { k.sa = sa; k.smem = need + 1024; fits = true; }
       }
       if (!fits || (stationary && k.sa * k.ks < 4)) continue;
-      k.cost = cost;
-      *c = k;
+      k.cost = tiles_pp * (2.5 + 0.9 * (bn / 64));
+      if (!found || k.cost < c->cost) *c = k;
       found = true;
-      break;
+      break;                                                   // a slab that can stay does
     }
   }
   return found;

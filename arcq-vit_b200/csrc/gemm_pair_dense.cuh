@@ -64,7 +64,7 @@ static_assert(kPairQuantEpiRegs * kPairQuantEpiWarps + kPairQuantIssueRegs * kPa
                   kPairQuantLaunchRegs * (kPairQuantThreads / 32),
               "registers beyond the launch's never come");
 constexpr uint32_t kPairQuantStageBytes = kPairQuantEpiWarps * 4096;       // 32 rows of 128 bytes per warp
-constexpr uint32_t kPairQuantTableBytes = (sizeof(GroupQuantTables) + 15) / 16 * 16;
+constexpr uint32_t kPairQuantTableBytes = kGroupQuantTableBytes;
 // Staging blocks (2 KB: 32 rows x 64 bytes) per epilogue warp; a block can be rewritten once the TMA store that
 // reads it has done so.  Four blocks instead of two measured slower on every DeiT-S shape (qkv 13.6 -> 15.5 us,
 // fc2 17.5 -> 22.3 us): the 32 KB they take away from the operand stages cost more than deeper stores gain.  One
@@ -77,7 +77,7 @@ constexpr int kDenseStageBlocks = ARCQ_DENSE_STAGE_BLOCKS;
 constexpr uint32_t kPairDenseEpiStageBytes = kPairEpiWarps * kDenseStageBlocks * 2048;
 
 struct PairDenseSmem {
-  uint32_t stages, slab, stage, tables, misc, total;
+  uint32_t stages, slab, stage, tables, misc, bars, total;
 };
 constexpr int kPairDenseBarriers = 72;
 __host__ __device__ inline PairDenseSmem pair_dense_smem_layout(int bn, int sa, int ks, int G, bool stationary, bool quant = false) {
@@ -89,7 +89,8 @@ __host__ __device__ inline PairDenseSmem pair_dense_smem_layout(int bn, int sa, 
   s.stage = s.slab + (stationary ? static_cast<uint32_t>(G) * wtile : 0u);
   s.tables = s.stage + (quant ? kPairQuantStageBytes : kPairDenseEpiStageBytes);     // on a 1 KB boundary
   s.misc = s.tables + (quant ? kPairQuantTableBytes : 0u);
-  s.total = s.misc + 256 * 4 /*bias*/ + kPairDenseBarriers * 8 + 16 /*tensor-memory address*/ + 32 /*next codebook*/;
+  s.bars = s.misc + (quant ? kPairQuantEpiWarps * 64 : 256) * 4 /*bias*/;
+  s.total = s.bars + kPairDenseBarriers * 8 + 16 /*tensor-memory address*/ + 32 /*next codebook*/;
   return s;
 }
 
@@ -113,7 +114,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
   uint8_t* const sSlab = smem + L.slab;
   uint8_t* const sStage = smem + L.stage;
   float* const s_bias = reinterpret_cast<float*>(smem + L.misc);
-  uint64_t* const bars = reinterpret_cast<uint64_t*>(s_bias + 256);
+  uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + L.bars);
   // barriers: full [sa] <= 16 at 0 (leader: both CTAs' bytes of the stage landed);  empty [sa] at 16 (both: the
   // MMAs that read the stage are done);  acc_full [2] at 32 (both);  acc_empty [2] at 34 (leader);
   // slab_full [G] <= 32 at 40 (leader, stationary slab only: sub-tile g of both CTAs landed)
@@ -129,19 +130,36 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
   const int n_pairs = p.pairs;
   const int pair = static_cast<int>(blockIdx.x) >> 1;
   const int n_slabs = p.N / bn;
-  const int slab = pair % n_slabs;
+  const int tiles_m = (p.M + kPairTileM - 1) / kPairTileM;
+  const int slab = pair % n_slabs;     // stationary: the pair's slab
   const int rank = pair / n_slabs;
   const int pairs_in_slab = (n_pairs - slab + n_slabs - 1) / n_slabs;
-  const int tiles_m = (p.M + kPairTileM - 1) / kPairTileM;
-  const int my_tiles = (rank < tiles_m) ? (tiles_m - rank + pairs_in_slab - 1) / pairs_in_slab : 0;
-  const int n0 = slab * bn;            // first column of the slab
-  const int nh0 = n0 + crank * hb;     // first W16 row this CTA loads
+  const int my_tiles = STATIONARY ? ((rank < tiles_m) ? (tiles_m - rank + pairs_in_slab - 1) / pairs_in_slab : 0)
+                                  : (tiles_m * n_slabs - pair + n_pairs - 1) / n_pairs;
   // pairs of different slabs that share a rank walk the same row tiles; stagger their starting points
-  const int rot = (my_tiles > 0) ? (slab * my_tiles) / n_slabs : 0;
-  auto row_of = [&](int t) {
-    int q = t + rot;
-    if (q >= my_tiles) q -= my_tiles;
-    return (rank + q * pairs_in_slab) * kPairTileM + static_cast<int>(crank) * kTileM;
+  const int rot = (STATIONARY && my_tiles > 0) ? (slab * my_tiles) / n_slabs : 0;
+  // The tiles of this pair one after the other: first row of this CTA, first column.  Without a slab that stays, the pairs take the
+  // (row tile, slab) combinations in turn, all slabs of a row tile one after the other: every pair has work (slabs x pairs per slab
+  // left up to ten of 74 idle), and the slabs read a row tile of A at about the same time (100 864 rows of K = 768, N = 3072: 630 us
+  // before, 505 now; plain form, 50 432 rows 219 -> 180; A is larger than L2 there).  No division on the way to a load: the first
+  // tile is known from above, the others follow by steps.
+  const int step_m = STATIONARY ? 0 : n_pairs / n_slabs, step_s = n_pairs - step_m * n_slabs;
+  struct Walk {
+    int q, m, s;       // stationary: q-th of the pair's row tiles; else row tile and slab
+  };
+  auto first_tile = [&]() { return Walk{rot, rank, slab}; };
+  auto row_of = [&](const Walk& w) {
+    return (STATIONARY ? rank + w.q * pairs_in_slab : w.m) * kPairTileM + static_cast<int>(crank) * kTileM;
+  };
+  auto col_of = [&](const Walk& w) { return (STATIONARY ? slab : w.s) * bn; };
+  auto advance = [&](Walk& w) {
+    if constexpr (STATIONARY) {
+      w.q = w.q + 1 == my_tiles ? 0 : w.q + 1;
+    } else {
+      w.m += step_m;
+      w.s += step_s;
+      if (w.s >= n_slabs) { w.s -= n_slabs; ++w.m; }
+    }
   };
   const uint32_t poll_limit = p.poll_limit, spin_limit = p.spin_limit;
   const uint32_t wtile_bytes = static_cast<uint32_t>(hb) * 128u;
@@ -190,13 +208,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
           const uint32_t sl0 = smem_u32(sSlab);
           for (int g = 0; g < G; ++g) {
             if (crank == 0) mbar_expect_tx(slab_full + g * 8, 2u * wtile_bytes);
-            tma_load_2d_pair(sl0 + g * wtile_bytes, &tm_w, slab_leader + g * 8, g * 64, nh0);
+            tma_load_2d_pair(sl0 + g * wtile_bytes, &tm_w, slab_leader + g * 8, g * 64, slab * bn + static_cast<int>(crank) * hb);
           }
         }
         __syncwarp();
       }
-      for (int t = 0; t < my_tiles; ++t) {
-        const int row0 = row_of(t);
+      Walk w = first_tile();
+      for (int t = 0; t < my_tiles; ++t, advance(w)) {
+        const int row0 = row_of(w), nh0 = col_of(w) + static_cast<int>(crank) * hb;     // nh0: first W16 row this CTA loads
         for (int g0 = 0; g0 < G; g0 += ks) {
           good &= mbar_park_flag(empty + slot * 8, ph, good ? poll_limit : 0u);
           if (elect_one()) {
@@ -290,7 +309,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
     // against 101.4 for GEMM and quantizer kernel, 100864 rows 787 against 984.
     const int ew = warp - kIssue, lq = warp & 3, grp = ew >> 2;
     GroupQuantTables* const tables = reinterpret_cast<GroupQuantTables*>(smem + L.tables);
-    for (int i = tid - kIssue * 32; i < bn; i += kEpi * 32) s_bias[i] = (p.bias != nullptr) ? __ldg(p.bias + n0 + i) : 0.0f;
     const GroupQuantParams gp = group_quant_tables<1 << QBITS, false>(tables, p.thresholds, p.codebook, tid - kIssue * 32, kEpi * 32, [](bool b) {
       asm volatile("bar.sync 2, %0;" ::"n"(kEpi * 32) : "memory");
       return b;
@@ -298,16 +316,33 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
     const uint32_t acc_empty_leader = mapa_shared(acc_empty, 0);
     uint8_t* const stg = sStage + ew * 4096;
     const uint32_t row = smem_u32(stg) + lane * 128, x7 = lane & 7;
+    // the bias of this warp's 64 columns: the next tile's is read while this one is worked on
+    float* const b = s_bias + ew * 64;
+    float b0 = 0.0f, b1 = 0.0f;
+    auto read_bias = [&](const Walk& w) {
+      if (grp * 64 < bn && p.bias != nullptr) {
+        b0 = __ldg(p.bias + col_of(w) + grp * 64 + lane);
+        b1 = __ldg(p.bias + col_of(w) + grp * 64 + 32 + lane);
+      }
+    };
+    Walk next = first_tile();
+    if (my_tiles > 0) read_bias(next);
     for (int t = 0; t < my_tiles && ok; ++t) {
+      const int row0 = row_of(next) + lq * 32, n0 = col_of(next);
+      advance(next);
       const uint32_t buf = static_cast<uint32_t>(t) & 1;
+      if (!STATIONARY || t == 0) {
+        b[lane] = b0;                                        // every lane has read the last tile's: it has gone through __syncwarp since
+        b[32 + lane] = b1;
+        __syncwarp();
+        if (!STATIONARY && t + 1 < my_tiles) read_bias(next);
+      }
       if (!mbar_wait_sleep_a(acc_full + buf * 8, (static_cast<uint32_t>(t) >> 1) & 1, poll_limit, 32)) { ok = false; break; }
       tc_fence_after_sync();
-      const int row0 = row_of(t) + lq * 32;
       const bool live = row0 < p.M && grp * 64 < bn;      // some of these 32 rows are inside the matrix, and the group is one
       uint32_t w[32];
       if (live) {
         const uint32_t t_row = tmem_base + buf * 256 + (static_cast<uint32_t>(lq * 32) << 16) + grp * 64;
-        const float* const b = s_bias + grp * 64;
 #pragma unroll
         for (int half_id = 0; half_id < 2; ++half_id) {
           uint32_t a[32];
@@ -357,11 +392,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
     // A step goes registers -> + bias -> fp16/fp32 -> one of this warp's two 2 KB staging blocks (64-byte
     // swizzle, conflict-free 16-byte stores) -> one TMA store.
     const int ew = warp - 2;
-    for (int i = tid - 64; i < bn; i += kPairEpiWarps * 32) s_bias[i] = (p.bias != nullptr) ? __ldg(p.bias + n0 + i) : 0.0f;
     if (PREFETCH && tid - 64 < 16)
       s_next_cb[tid - 64] = __float2half_rn(tid - 64 < (1 << p.next.bits) ? __ldg(p.next.codebook + (tid - 64)) : 0.0f);
-    asm volatile("bar.sync 2, %0;" ::"n"(kPairEpiWarps * 32) : "memory");   // bias table (and codebook) complete
     if (PREFETCH) {
+      asm volatile("bar.sync 2, %0;" ::"n"(kPairEpiWarps * 32) : "memory");   // codebook complete
       // The next layer's weight, while these warps have no accumulator to drain yet.  Wait for the previous kernel
       // first: the scratch matrix being overwritten was last read two GEMMs back and is then free for certain.
       pdl_wait();
@@ -377,8 +411,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
     uint8_t* const stg = sStage + ew * (kDenseStageBlocks * 2048);
     const int cw = p.y_f32 ? 16 : 32;
     const bool f32 = p.y_f32 != 0;
+    // The bias of the columns that these four warps take, step after step.  Each of their threads carries one value of the next
+    // tile's; the table changes hands between two barriers of the four.
+    float* const sb = s_bias + half_id * 128;
+    const int bi = (ew & 3) * 32 + lane;
+    const int bcol = bi / cw * 2 * cw + half_id * cw + bi % cw;
+    const bool has_bias = p.bias != nullptr && bcol < bn;
+    float next_b = 0.0f;
+    Walk next = first_tile();
+    if (my_tiles > 0 && has_bias) next_b = __ldg(p.bias + col_of(next) + bcol);
+    auto four_warps = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(3 + half_id) : "memory"); };
     uint32_t blk = 0;      // staging block of the next store; the blocks are used in turn
-    auto emit = [&](const uint32_t (&acc)[32], int c0, int row0) {
+    auto emit = [&](const uint32_t (&acc)[32], int c0, int row0, int n0) {
+      const float* const bc = sb + ((c0 - half_id * cw) >> 1);
       if (lane == 0) tma_store_wait_read_n<kDenseStageBlocks - 1>();   // the store that last used this block has read it
       __syncwarp();
       uint8_t* const rowp = stg + blk * 2048 + lane * 64;
@@ -387,14 +432,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
       for (int ch = 0; ch < 4; ++ch) {
         uint4 v;
         if (f32) {
-          const float4 b4 = *reinterpret_cast<const float4*>(s_bias + c0 + 4 * ch);
+          const float4 b4 = *reinterpret_cast<const float4*>(bc + 4 * ch);
           v.x = __float_as_uint(__uint_as_float(acc[4 * ch]) + b4.x);
           v.y = __float_as_uint(__uint_as_float(acc[4 * ch + 1]) + b4.y);
           v.z = __float_as_uint(__uint_as_float(acc[4 * ch + 2]) + b4.z);
           v.w = __float_as_uint(__uint_as_float(acc[4 * ch + 3]) + b4.w);
         } else {
-          const float4 b0 = *reinterpret_cast<const float4*>(s_bias + c0 + 8 * ch);
-          const float4 b1 = *reinterpret_cast<const float4*>(s_bias + c0 + 8 * ch + 4);
+          const float4 b0 = *reinterpret_cast<const float4*>(bc + 8 * ch);
+          const float4 b1 = *reinterpret_cast<const float4*>(bc + 8 * ch + 4);
           __half2 h0 = __floats2half2_rn(__uint_as_float(acc[8 * ch]) + b0.x, __uint_as_float(acc[8 * ch + 1]) + b0.y);
           __half2 h1 = __floats2half2_rn(__uint_as_float(acc[8 * ch + 2]) + b0.z, __uint_as_float(acc[8 * ch + 3]) + b0.w);
           __half2 h2 = __floats2half2_rn(__uint_as_float(acc[8 * ch + 4]) + b1.x, __uint_as_float(acc[8 * ch + 5]) + b1.y);
@@ -419,11 +464,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
       else tmem_ld_32x32(taddr, acc);
     };
     const int step = 2 * cw;
-    for (int t = 0; t < my_tiles && ok; ++t) {
+    for (int t = 0; t < my_tiles; ++t) {
       const uint32_t buf = static_cast<uint32_t>(t) & 1;
-      if (!mbar_wait_sleep_a(acc_full + buf * 8, (static_cast<uint32_t>(t) >> 1) & 1, poll_limit, 32)) { ok = false; break; }
+      const int row0 = row_of(next) + lq * 32, n0 = col_of(next);
+      advance(next);
+      if (!STATIONARY || t == 0) {
+        if (t > 0) four_warps();
+        sb[bi] = next_b;
+        four_warps();
+        if (!STATIONARY && t + 1 < my_tiles && has_bias) next_b = __ldg(p.bias + col_of(next) + bcol);
+      }
+      // (a warp whose wait ran out goes on to the barriers above, without waiting again)
+      ok = ok && mbar_wait_sleep_a(acc_full + buf * 8, (static_cast<uint32_t>(t) >> 1) & 1, poll_limit, 32);
+      if (!ok) continue;
       tc_fence_after_sync();
-      const int row0 = row_of(t) + lq * 32;
       const uint32_t t_row = tmem_base + buf * 256 + (static_cast<uint32_t>(lq * 32) << 16);
       const bool live = row0 < p.M;     // some of these 32 rows are inside the matrix
       // The tensor-memory reads run one step ahead of the conversion, and the accumulator is handed back as
@@ -443,13 +497,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
           tmem_ld_wait();
           bool more = c0 + step < bn;
           if (more) load(rb, t_row + c0 + step); else release();
-          emit(ra, c0, row0);
+          emit(ra, c0, row0, n0);
           if (!more) break;
           c0 += step;
           tmem_ld_wait();
           more = c0 + step < bn;
           if (more) load(ra, t_row + c0 + step); else release();
-          emit(rb, c0, row0);
+          emit(rb, c0, row0, n0);
           if (!more) break;
           c0 += step;
         }
