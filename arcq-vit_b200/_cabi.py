@@ -20,7 +20,7 @@ EXPORTS = (
     "arcq_unpack_codes", "arcq_pack_codes", "arcq_dequant", "arcq_unpack_weight_f16", "arcq_dense_weight_gemm_prefetch",
     "arcq_act_quant_unpack", "arcq_add_layernorm_act_quant_unpack", "arcq_add_layernorm_strided",
     "arcq_dense_weight_gemm_unpack", "arcq_dense_weight_gemm_unpack_room", "arcq_unpack_beside_gemm", "arcq_dense_weight_gemm_gelu_quant",
-    "arcq_dense_weight_gemm_gelu_quant_applies",
+    "arcq_dense_weight_gemm_gelu_quant_applies", "arcq_packed_linear_small", "arcq_packed_linear_small_applies",
 )
 
 _lib = None
@@ -70,6 +70,8 @@ def load() -> ctypes.CDLL:
     lib.arcq_unpack_weight_f16.argtypes = [vp, vp, vp, vp, vp, ci, ci, i64, i64, vp, vp]
     lib.arcq_dense_weight_gemm_prefetch.argtypes = [vp, vp, vp, i64, i64, i64, vp, ci, vp, vp, vp, vp, vp, ci, ci, i64, i64, vp, vp]
     lib.arcq_dense_weight_gemm_gelu_quant_applies.argtypes = [i64, i64, i64]
+    lib.arcq_packed_linear_small_applies.argtypes = [i64, i64, i64]
+    lib.arcq_packed_linear_small.argtypes = [ci, vp, ci, i64, vp, vp, ci, vp, vp, vp, ci, vp]
     lib.arcq_dense_weight_gemm_gelu_quant.argtypes = [vp, vp, vp, i64, i64, i64, vp, vp, ci, ci, vp, vp, ci, vp]
     for name in EXPORTS:
         getattr(lib, name)  # AttributeError here means header and library disagree
@@ -134,6 +136,7 @@ class option:
 
 E_UNSUPPORTED = -3
 GEMM_ONE_CTA_PACKED, GEMM_ONE_CTA_DENSE, GEMM_PAIR_PACKED, GEMM_PAIR_DENSE, GEMM_PAIR_DENSE_PREFETCH, GEMM_PAIR_DENSE_GELU_QUANT = 1, 2, 3, 4, 5, 6
+GEMM_SMALL_LINEAR = 7
 
 
 def last_gemm_kernel() -> int:

@@ -75,6 +75,44 @@ __device__ __forceinline__ float octet_chain_sum(float p, int octet_base) {
   return s;
 }
 
+// The quantizer of one group by an octet.  In: v[c] = element 8c + l in lane l.  Out: the levels of those elements' codes, the codes
+// one per nibble, and the group's statistics.
+struct OctetStats {
+  float mean, scale, code_sum;
+};
+template <int BITS>
+__device__ __forceinline__ OctetStats octet_quantize(const float (&v)[8], const float* s_th, const float* s_cb, int octet_base,
+                                                     float (&level)[8], uint32_t& codes) {
+  auto sum = [&](const float (&e)[8]) {
+    const float a0 = __fadd_rn(e[0], e[4]), a1 = __fadd_rn(e[1], e[5]), a2 = __fadd_rn(e[2], e[6]), a3 = __fadd_rn(e[3], e[7]);
+    return octet_chain_sum(__fadd_rn(__fadd_rn(__fadd_rn(a0, a1), a2), a3), octet_base);
+  };
+  OctetStats st;
+  st.mean = __fdiv_rn(sum(v), 64.0f);
+  float r[8], q[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    r[c] = __fsub_rn(v[c], st.mean);
+    q[c] = __fmul_rn(r[c], r[c]);
+  }
+  st.scale = __fsqrt_rn(__fadd_rn(__fdiv_rn(sum(q), 64.0f), 1.0e-6f));      // sqrt(mean(r^2) + 1e-6)
+  // codes: number of thresholds strictly below t (binary search in the sorted table)
+  codes = 0;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const float t = __fdiv_rn(r[c], st.scale);
+    int code = 0;
+    if (BITS >= 4) code = (t > s_th[7]) ? 8 : 0;
+    if (BITS >= 3) code += (t > s_th[code + 3]) ? 4 : 0;
+    code += (t > s_th[code + 1]) ? 2 : 0;
+    code += (t > s_th[code]) ? 1 : 0;
+    codes |= static_cast<uint32_t>(code) << (4 * c);
+    level[c] = s_cb[code];
+  }
+  st.code_sum = sum(level);
+  return st;
+}
+
 // In: lane l of an octet holds, in nibble c, the code of element 8c + l.
 // Out: lane l holds, in nibble j, the code of element 8l + j (an 8x8 nibble transpose over lanes).
 __device__ __forceinline__ uint32_t octet_transpose_nibbles(uint32_t w, int l) {
@@ -144,43 +182,10 @@ __global__ void __launch_bounds__(256) act_quant_kernel(const T* __restrict__ x,
 #pragma unroll
     for (int c = 0; c < 8; ++c) v[c] = pre_op<T, PRE>(load_f32<T>(xg + 8 * c));
 
-    // mean
-    float a0 = __fadd_rn(v[0], v[4]), a1 = __fadd_rn(v[1], v[5]);
-    float a2 = __fadd_rn(v[2], v[6]), a3 = __fadd_rn(v[3], v[7]);
-    float part = __fadd_rn(__fadd_rn(__fadd_rn(a0, a1), a2), a3);
-    const float mean = __fdiv_rn(octet_chain_sum(part, octet_base), 64.0f);
-
-    // scale = sqrt(mean(r^2) + 1e-6)
-    float r[8], q[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      r[c] = __fsub_rn(v[c], mean);
-      q[c] = __fmul_rn(r[c], r[c]);
-    }
-    a0 = __fadd_rn(q[0], q[4]); a1 = __fadd_rn(q[1], q[5]);
-    a2 = __fadd_rn(q[2], q[6]); a3 = __fadd_rn(q[3], q[7]);
-    part = __fadd_rn(__fadd_rn(__fadd_rn(a0, a1), a2), a3);
-    const float var = __fdiv_rn(octet_chain_sum(part, octet_base), 64.0f);
-    const float scale = __fsqrt_rn(__fadd_rn(var, 1.0e-6f));
-
-    // codes: number of thresholds strictly below t (binary search in the sorted table)
-    uint32_t w = 0;
+    uint32_t w;
     float cv[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const float t = __fdiv_rn(r[c], scale);
-      int code = 0;
-      if (BITS >= 4) code = (t > s_th[7]) ? 8 : 0;
-      if (BITS >= 3) code += (t > s_th[code + 3]) ? 4 : 0;
-      code += (t > s_th[code + 1]) ? 2 : 0;
-      code += (t > s_th[code]) ? 1 : 0;
-      w |= static_cast<uint32_t>(code) << (4 * c);
-      cv[c] = s_cb[code];
-    }
-    a0 = __fadd_rn(cv[0], cv[4]); a1 = __fadd_rn(cv[1], cv[5]);
-    a2 = __fadd_rn(cv[2], cv[6]); a3 = __fadd_rn(cv[3], cv[7]);
-    part = __fadd_rn(__fadd_rn(__fadd_rn(a0, a1), a2), a3);
-    const float code_sum = octet_chain_sum(part, octet_base);
+    const OctetStats st = octet_quantize<BITS>(v, s_th, s_cb, octet_base, cv, w);
+    const float mean = st.mean, scale = st.scale, code_sum = st.code_sum;
 
     if (WRITE_XHAT) {
       const ReconTerms rt = recon_terms(mean, scale, code_sum, one_fma != 0);

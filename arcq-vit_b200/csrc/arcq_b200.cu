@@ -24,6 +24,7 @@
 #include "add_layernorm.cuh"
 #include "ln_act_quant.cuh"
 #include "attention.cuh"
+#include "small_linear.cuh"
 #include "patch_embed.cuh"
 #include <cudaTypedefs.h>
 
@@ -82,6 +83,7 @@ enum Opt {
   O_ACT_QUANT_V1, O_LN_PLAIN,
   O_PAIR, O_PAIR_MIN_M, O_PAIR_BN, O_PAIR_SA, O_PAIR_KS, O_PAIR_NBB, O_PAIR_LUT, O_PAIR_PAIRS, O_PAIR_STATIONARY,
   O_PAIR_WS, O_LNQ_SMALL, O_AQ2_MIN_GROUPS, O_PDL, O_GELU_GEMM, O_GEMM_UNPACK, O_POLL_LIMIT, O_SPIN_LIMIT, O_LAUNCH_REGS,
+  O_SMALL_LINEAR, O_SMALL_R, O_SMALL_BN,
   O_COUNT
 };
 struct OptDef { const char* name; int dflt; };
@@ -94,6 +96,7 @@ const OptDef kOptDefs[O_COUNT] = {
     {"ARCQ_PAIR_STATIONARY", -1}, {"ARCQ_PAIR_WS", 0}, {"ARCQ_LNQ_SMALL", 1}, {"ARCQ_AQ2_MIN_GROUPS", 0}, {"ARCQ_PDL", 1},
     {"ARCQ_GELU_GEMM", -1}, {"ARCQ_GEMM_UNPACK", 1},
     {"ARCQ_POLL_LIMIT", 1 << 21}, {"ARCQ_SPIN_LIMIT", 1 << 25}, {"ARCQ_LAUNCH_REGS", 0},
+    {"ARCQ_SMALL_LINEAR", -1}, {"ARCQ_SMALL_R", 0}, {"ARCQ_SMALL_BN", 0},
 };
 int g_opt[O_COUNT];
 void load_options() {
@@ -753,6 +756,47 @@ bool choose_gelu_quant(long long M, long long N, long long K, PairDenseConfig* p
   return 1.3 * pc->cost < 4.6 * rounds + plain.cost + 1.0;
 }
 
+// ---- packed linear in one launch: configuration ----
+struct SmallLinearConfig {
+  int R, bn;
+  unsigned blocks;
+  size_t smem;
+};
+// Rows and columns of a block, and whether the one launch is taken: microseconds of GPU time, fitted (4 % rms) to every (R, bn) of twelve
+// layers of the three widths with 1 to 788 rows, in graphs.  A block's time is passes of 96 groups, rounds of unpacking, and the products'
+// chain over k; the pair chosen is 0.7 % slower than the fastest on average, 9 % at worst.  The two launches take what the last line
+// says (10 % rms).  A second launch and its scratch cost the host 3.5 us of a module call's 10.2, so up to 0.8 us more of GPU time is
+// taken for the one: K = 192, N = 192 up to 560 rows (560: 6.6 against 6.1 us of GPU time, calls 10.2 -> 7 us), N = 768 up to 128 (6.7 / 6.0),
+// 384 x 384 up to 64 (7.0 / 6.3), 768 x 768 up to 48 (9.0 / 7.5), 768 x 2304 up to 32, 768 x 3072 up to 24 (10.9 / 10.2).
+bool choose_small_linear(long long M, long long N, long long K, SmallLinearConfig* c) {
+  const int force = opt(O_SMALL_LINEAR);
+  if (force == 0 || M <= 0 || M > 4096 || K % 64 != 0 || N % 16 != 0 || K > (1 << 16) || N > (1 << 20)) return false;
+  const int G = static_cast<int>(K / 64), n = static_cast<int>(N), sms = sm_count();
+  const double two_launches = 5.3 + 0.002 * static_cast<double>(K) + 1.6e-6 * static_cast<double>(N * K);
+  double limit = force > 0 ? 1.0e9 : two_launches + 0.8;       // what the next candidate has to be below
+  bool found = false;
+  for (int R : {8, 16, 32, 64, 128}) {
+    if (opt(O_SMALL_R) > 0 && R != opt(O_SMALL_R)) continue;
+    if (R > 8 && R / 2 >= M) break;
+    constexpr int kPass = arcq::kSmallLinearThreads / 8, kRound = arcq::kSmallLinearThreads * 4;
+    const int row_blocks = (static_cast<int>(M) + R - 1) / R, groups = static_cast<int>(M < R ? M : R) * G;
+    const double rows_cost = 0.82 + 2.19 * ((groups + kPass - 1) / kPass) + 1.33 * (groups < kPass ? static_cast<double>(groups) / kPass : 1.0) + 0.078 * G;
+    if (rows_cost + 1.98 > limit) break;                       // more rows a block only cost more
+    for (int bn : {16, 32, 48, 64, 96, 128, 192, 256}) {
+      if (row_blocks * (n / bn) > sms || n % bn != 0 || (opt(O_SMALL_BN) > 0 && bn != opt(O_SMALL_BN))) continue;
+      const int chunks = bn * G * 8;
+      const double cost = rows_cost + 1.98 * ((chunks + kRound - 1) / kRound) + 1.2 * (chunks < kRound ? static_cast<double>(chunks) / kRound : 1.0);
+      if (cost > limit) break;
+      const size_t smem = arcq::small_linear_smem_layout(R, bn, G).total;
+      if (smem > kSmemBudget) break;
+      *c = {R, bn, static_cast<unsigned>(row_blocks * (n / bn)), smem};
+      limit = cost;
+      found = true;
+    }
+  }
+  return found;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1269,6 +1313,65 @@ int arcq_dense_weight_gemm_gelu_quant(const void* xhat, const void* w16, const f
   arcq::UnpackJobs jobs;
   if (const int rc = make_idle_jobs(unpack, n_unpack, pc.pairs, &jobs)) return rc;
   return launch_pair_dense_gemm(pc, xhat, w16, bias, M, N, K, out, ARCQ_DT_F16, stream, nullptr, jobs, thresholds, codebook, bits);
+}
+
+int arcq_packed_linear_small_applies(int64_t M, int64_t N, int64_t K) {
+  SmallLinearConfig c;
+  return choose_small_linear(M, N, K, &c) ? 1 : 0;
+}
+
+int arcq_packed_linear_small(int pre_gelu, const void* x, int x_dtype, int64_t M, const float* thresholds, const float* codebook,
+                             int one_fma, const arcq_unpack_job* weight, const float* bias, void* y, int y_dtype, void* stream) {
+  if (!x || !thresholds || !codebook || !weight || !weight->packed || !weight->mu || !weight->sigma || !weight->codesum || !weight->codebook || !y)
+    return fail(ARCQ_E_BAD_ARG, "null pointer argument");
+  const int bits = weight->bits;
+  const int64_t N = weight->rows, K = weight->K;
+  if (bits < 2 || bits > 4) return fail(ARCQ_E_BAD_ARG, "bits must be 2, 3 or 4, got %d", bits);
+  if (x_dtype < ARCQ_DT_F32 || x_dtype > ARCQ_DT_BF16) return fail(ARCQ_E_BAD_ARG, "bad x_dtype %d", x_dtype);
+  if (pre_gelu && x_dtype != ARCQ_DT_F16) return fail(ARCQ_E_UNSUPPORTED, "the fused GELU is built for fp16 input only");
+  if (y_dtype != ARCQ_DT_F16 && y_dtype != ARCQ_DT_F32) return fail(ARCQ_E_BAD_ARG, "y_dtype must be f16 or f32");
+  if (M < 0 || N <= 0 || K <= 0) return fail(ARCQ_E_BAD_SHAPE, "bad shape M=%lld N=%lld K=%lld", (long long)M, (long long)N, (long long)K);
+  if (K % 64 != 0 || N % 16 != 0) return fail(ARCQ_E_UNSUPPORTED, "K=%lld, N=%lld: this entry point needs multiples of 64 and 16", (long long)K, (long long)N);
+  if (!aligned(weight->packed, 4) || !aligned(y, 16)) return fail(ARCQ_E_ALIGN, "packed codes must be 4-byte, y 16-byte aligned");
+  if (M == 0) return ARCQ_OK;
+  SmallLinearConfig c;
+  if (!choose_small_linear(M, N, K, &c))
+    return fail(ARCQ_E_UNSUPPORTED, "M=%lld, N=%lld, K=%lld: left to arcq_act_quant_unpack and arcq_dense_weight_gemm", (long long)M, (long long)N, (long long)K);
+  arcq::SmallLinearParams p;
+  p.M = static_cast<int>(M); p.N = static_cast<int>(N); p.K = static_cast<int>(K); p.G = static_cast<int>(K / 64);
+  p.R = c.R; p.bn = c.bn;
+  p.thresholds = thresholds; p.codebook = codebook; p.one_fma = one_fma != 0;
+  p.weight = arcq::UnpackWeightJob{weight->packed, weight->mu, weight->sigma, weight->codesum, weight->codebook, nullptr, N, p.K, bits};
+  p.bias = bias; p.y = y; p.y_f32 = y_dtype == ARCQ_DT_F32;
+  p.tmem_cols = 32;
+  while (p.tmem_cols < static_cast<uint32_t>(c.bn)) p.tmem_cols *= 2;
+  p.poll_limit = static_cast<uint32_t>(opt(O_POLL_LIMIT));
+  p.status = status_ptr();
+  if (p.status == nullptr) return fail(ARCQ_E_CUDA, "device status word not reachable");
+  auto launch = [&](auto kernel, auto type, int* done_dev) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (*done_dev != dev) {                   // once per (thread, device)
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBudget));
+      if (e != cudaSuccess) return cuda_fail(e, "packed_linear_small");
+      *done_dev = dev;
+    }
+    launch_pdl(kernel, c.blocks, arcq::kSmallLinearThreads, c.smem, static_cast<cudaStream_t>(stream), static_cast<const decltype(type)*>(x), p);
+    const cudaError_t e = cudaGetLastError();
+    return e != cudaSuccess ? cuda_fail(e, "packed_linear_small launch") : ARCQ_OK;
+  };
+  static thread_local int done[12] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
+  auto by_bits = [&](auto type, auto pre, int* d) {
+    using T = decltype(type);
+    constexpr int PRE = decltype(pre)::value;
+    return bits == 4 ? launch(arcq::small_linear_kernel<T, 4, PRE>, type, d)
+           : bits == 3 ? launch(arcq::small_linear_kernel<T, 3, PRE>, type, d + 1) : launch(arcq::small_linear_kernel<T, 2, PRE>, type, d + 2);
+  };
+  g_last_gemm_kernel = ARCQ_GEMM_SMALL_LINEAR;
+  if (pre_gelu) return by_bits(__half(), std::integral_constant<int, 1>(), done);
+  if (x_dtype == ARCQ_DT_F16) return by_bits(__half(), std::integral_constant<int, 0>(), done + 3);
+  if (x_dtype == ARCQ_DT_F32) return by_bits(float(), std::integral_constant<int, 0>(), done + 6);
+  return by_bits(__nv_bfloat16(), std::integral_constant<int, 0>(), done + 9);
 }
 
 int arcq_dense_weight_gemm_prefetch(const void* xhat, const void* w16, const float* bias, int64_t M, int64_t N,

@@ -126,9 +126,9 @@ struct UnpackWeightJob {
 // Chunks first, first + stride, ... of the job; `s_cb` holds the 16 codebook values, of type CB: __half, or float for the
 // fp32 form.  Four chunks per round, all their loads issued before the first result is used: a caller with few warps (the spare warps of a
 // GEMM kernel) has nothing else to hide the load latency with.
-template <int BITS, typename CB>
-__device__ __forceinline__ void unpack_weight_f16_chunks(const UnpackWeightJob& j, const CB* s_cb, long long first,
-                                                         long long stride) {
+// `store(row, chunk, value)` takes a result.
+template <int BITS, typename CB, typename Store>
+__device__ __forceinline__ void unpack_weight_chunks(const UnpackWeightJob& j, const CB* s_cb, long long first, long long stride, Store store) {
   const int chunks = j.K / 8;
   const int G = j.K / 64;
   const long long pc = static_cast<long long>(j.K) * BITS / 8;
@@ -137,7 +137,8 @@ __device__ __forceinline__ void unpack_weight_f16_chunks(const UnpackWeightJob& 
   for (long long i0 = first; i0 < total; i0 += U * stride) {
     uint32_t w[U];
     float sg[U], cs[U], mu[U];
-    long long off[U];
+    long long row[U];
+    int chunk[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long long i = i0 + u * stride;
@@ -150,11 +151,12 @@ __device__ __forceinline__ void unpack_weight_f16_chunks(const UnpackWeightJob& 
       sg[u] = __ldg(j.sigma + sgi);
       cs[u] = __ldg(j.codesum + sgi);
       mu[u] = __ldg(j.mu + sgi);
-      off[u] = in ? r * j.K + ch * 8 : -1;
+      row[u] = in ? r : -1;
+      chunk[u] = ch;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (off[u] < 0) continue;
+      if (row[u] < 0) continue;
       const float m = fmaf(-sg[u], cs[u] * (1.0f / 64.0f), mu[u]);
       uint32_t h[4];
       if constexpr (sizeof(CB) == 4) {
@@ -174,9 +176,14 @@ __device__ __forceinline__ void unpack_weight_f16_chunks(const UnpackWeightJob& 
           h[q] = *reinterpret_cast<const uint32_t*>(&r2);
         }
       }
-      *reinterpret_cast<uint4*>(j.out + off[u]) = make_uint4(h[0], h[1], h[2], h[3]);
+      store(row[u], chunk[u], make_uint4(h[0], h[1], h[2], h[3]));
     }
   }
+}
+
+template <int BITS, typename CB>
+__device__ __forceinline__ void unpack_weight_f16_chunks(const UnpackWeightJob& j, const CB* s_cb, long long first, long long stride) {
+  unpack_weight_chunks<BITS>(j, s_cb, first, stride, [&](long long r, int ch, uint4 v) { *reinterpret_cast<uint4*>(j.out + r * j.K + ch * 8) = v; });
 }
 
 // Weights that a kernel of the activation path unpacks on the side: its first `blocks` blocks take the jobs (chunks split over

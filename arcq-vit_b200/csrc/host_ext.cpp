@@ -172,6 +172,16 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   at::Tensor y = without_gil([&] {
     const c10::cuda::CUDAGuard guard(x->device());
     void* const st = c10::cuda::getCurrentCUDAStream().stream();
+    c10::SmallVector<int64_t, 5> sizes(x->sizes().begin(), x->sizes().end());
+    sizes.back() = l.N;
+    const auto out = [&] { return empty_cuda(sizes, float_chain ? at::kFloat : at::kHalf, x->device()); };
+    const int yt = float_chain ? ARCQ_DT_F32 : ARCQ_DT_F16;
+    if (!ready && arcq_packed_linear_small_applies(M, l.N, l.K)) {       // few rows: one launch, no scratch
+      at::Tensor y = out();
+      check(arcq_packed_linear_small(pre_gelu, x->const_data_ptr(), xt, M, l.th, l.acb, l.one_fma(), &l.job, l.bias, y.mutable_data_ptr(), yt, st),
+            "arcq_packed_linear_small");
+      return y;
+    }
     // the reconstructed activation and the unpacked weight, given back to the caching allocator on return
     const at::Tensor scratch = empty_cuda({(ready ? 0 : numel) + l.weight_elems() + 8}, at::kHalf, x->device());
     at::Half* const w16 = scratch.mutable_data_ptr<at::Half>();
@@ -186,11 +196,8 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
             "arcq_act_quant");
       xhat = xh;
     }
-    c10::SmallVector<int64_t, 5> sizes(x->sizes().begin(), x->sizes().end());
-    sizes.back() = l.N;
-    at::Tensor y = empty_cuda(sizes, float_chain ? at::kFloat : at::kHalf, x->device());
-    check(arcq_dense_weight_gemm(xhat, w16, l.bias, M, l.N, l.K, y.mutable_data_ptr(), float_chain ? ARCQ_DT_F32 : ARCQ_DT_F16, st),
-          "arcq_dense_weight_gemm");
+    at::Tensor y = out();
+    check(arcq_dense_weight_gemm(xhat, w16, l.bias, M, l.N, l.K, y.mutable_data_ptr(), yt, st), "arcq_dense_weight_gemm");
     return y;
   });
   return THPVariable_Wrap(std::move(y));

@@ -226,41 +226,14 @@ __global__ void __launch_bounds__(kLnqRowsThreads, 1) add_layernorm_act_quant_ro
       float v[8];
 #pragma unroll
       for (int c = 0; c < 8; ++c) v[c] = __half2float(hg[8 * c]);
-      float a0 = __fadd_rn(v[0], v[4]), a1 = __fadd_rn(v[1], v[5]);
-      float a2 = __fadd_rn(v[2], v[6]), a3 = __fadd_rn(v[3], v[7]);
-      float part = __fadd_rn(__fadd_rn(__fadd_rn(a0, a1), a2), a3);
-      const float mean = __fdiv_rn(octet_chain_sum(part, octet_base), 64.0f);
-      float r[8], q[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        r[c] = __fsub_rn(v[c], mean);
-        q[c] = __fmul_rn(r[c], r[c]);
-      }
-      a0 = __fadd_rn(q[0], q[4]); a1 = __fadd_rn(q[1], q[5]);
-      a2 = __fadd_rn(q[2], q[6]); a3 = __fadd_rn(q[3], q[7]);
-      part = __fadd_rn(__fadd_rn(__fadd_rn(a0, a1), a2), a3);
-      const float var = __fdiv_rn(octet_chain_sum(part, octet_base), 64.0f);
-      const float scale = __fsqrt_rn(__fadd_rn(var, 1.0e-6f));
       float cv[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float t = __fdiv_rn(r[c], scale);
-        int code = 0;
-        if (BITS >= 4) code = (t > s_th[7]) ? 8 : 0;
-        if (BITS >= 3) code += (t > s_th[code + 3]) ? 4 : 0;
-        code += (t > s_th[code + 1]) ? 2 : 0;
-        code += (t > s_th[code]) ? 1 : 0;
-        cv[c] = s_cb[code];
-      }
-      a0 = __fadd_rn(cv[0], cv[4]); a1 = __fadd_rn(cv[1], cv[5]);
-      a2 = __fadd_rn(cv[2], cv[6]); a3 = __fadd_rn(cv[3], cv[7]);
-      part = __fadd_rn(__fadd_rn(__fadd_rn(a0, a1), a2), a3);
-      const float code_sum = octet_chain_sum(part, octet_base);
-      const ReconTerms rt = recon_terms(mean, scale, code_sum, one_fma != 0);
+      uint32_t codes;
+      const OctetStats st = octet_quantize<BITS>(v, s_th, s_cb, octet_base, cv, codes);
+      const ReconTerms rt = recon_terms(st.mean, st.scale, st.code_sum, one_fma != 0);
       if (valid) {
         __half* og = xhat + row * K + g * 64 + l8;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) og[8 * c] = __float2half_rn(recon_value(rt, scale, cv[c]));
+        for (int c = 0; c < 8; ++c) og[8 * c] = __float2half_rn(recon_value(rt, st.scale, cv[c]));
       }
     }
     __syncthreads();   // the tile's rows in shared memory are free for the next tile

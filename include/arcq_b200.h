@@ -75,7 +75,7 @@ int arcq_debug_trace(void* device_buffer);
  * ARCQ_WS_GRID, ARCQ_WS_TMA_STORE, ARCQ_WS_ROTATE, ARCQ_ACT_QUANT_V1, ARCQ_LN_PLAIN,
  * ARCQ_PAIR, ARCQ_PAIR_MIN_M, ARCQ_PAIR_BN, ARCQ_PAIR_SA, ARCQ_PAIR_KS, ARCQ_PAIR_NBB, ARCQ_PAIR_LUT,
  * ARCQ_PAIR_PAIRS, ARCQ_PAIR_STATIONARY, ARCQ_PAIR_WS, ARCQ_PDL, ARCQ_GELU_GEMM,
- * ARCQ_GEMM_UNPACK, ARCQ_LNQ_SMALL, ARCQ_AQ2_MIN_GROUPS, ARCQ_POLL_LIMIT, ARCQ_SPIN_LIMIT, ARCQ_LAUNCH_REGS (the
+ * ARCQ_GEMM_UNPACK, ARCQ_LNQ_SMALL, ARCQ_AQ2_MIN_GROUPS, ARCQ_POLL_LIMIT, ARCQ_SPIN_LIMIT, ARCQ_SMALL_LINEAR, ARCQ_SMALL_R, ARCQ_SMALL_BN, ARCQ_LAUNCH_REGS (the
  * registers a thread that kernels are taken to be compiled for, where that is checked).  Normal use sets none.
  * Unknown names return ARCQ_E_BAD_ARG.  No reference counterpart.
  */
@@ -90,7 +90,7 @@ int arcq_debug_get_option(const char* name, int* value_out);
 enum {
   ARCQ_GEMM_ONE_CTA_PACKED = 1, ARCQ_GEMM_ONE_CTA_DENSE = 2, ARCQ_GEMM_PAIR_PACKED = 3, ARCQ_GEMM_PAIR_DENSE = 4,
   ARCQ_GEMM_PAIR_DENSE_PREFETCH = 5,
-  ARCQ_GEMM_PAIR_DENSE_GELU_QUANT = 6
+  ARCQ_GEMM_PAIR_DENSE_GELU_QUANT = 6, ARCQ_GEMM_SMALL_LINEAR = 7
 };
 int arcq_debug_last_gemm_kernel(void);
 
@@ -233,6 +233,18 @@ int arcq_packed_linear_static_scratch(const void* xhat, const uint8_t* packed_w,
                                       const float* sigma_w, const float* codesum_w, const float* w_codebook,
                                       const float* bias, int bits, int group_size, int64_t M, int64_t N,
                                       int64_t K, void* y, int y_dtype, void* stream);
+
+/*
+ * A packed linear on few rows in one launch (ARCQPackedLinearOnTheFly.forward and ARCQPackedLinear.forward of the reference,
+ * arcq_packed_on_the_fly.py:137-161, arcq_packed_linear.py:161-222): arcq_act_quant_unpack followed by arcq_dense_weight_gemm without
+ * the scratch matrices between them, the same bits.  `weight` describes the packed weight [rows = N, K]; its `out` is not used.
+ * x fp32, fp16 or bf16 [M,K] (pre_gelu: fp16), y fp16 or fp32 [M,N], 16-byte aligned; K % 64 == 0, N % 16 == 0, groups of 64.
+ * Where one round of blocks that each make their own operands is not the faster way, ARCQ_E_UNSUPPORTED, which
+ * arcq_packed_linear_small_applies (1 / 0) says beforehand.
+ */
+int arcq_packed_linear_small_applies(int64_t M, int64_t N, int64_t K);
+int arcq_packed_linear_small(int pre_gelu, const void* x, int x_dtype, int64_t M, const float* thresholds, const float* codebook,
+                             int one_fma, const arcq_unpack_job* weight, const float* bias, void* y, int y_dtype, void* stream);
 
 /*
  * Residual add + LayerNorm over fp16 rows, the glue between the packed linears of a transformer block:

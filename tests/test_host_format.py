@@ -186,3 +186,11 @@ def test_c_abi_rejects_bad_arguments_before_any_launch(pkg):
     # empty inputs are a successful no-op
     assert lib.arcq_act_quant(p, 0, 0, 64, p, p, 4, 64, p, p, p, p, None, 0, None) == 0
     assert lib.arcq_unpack_codes(p, 0, 8, 4, p, None) == 0
+
+
+# both sides of the line, and what neither its shared memory nor one round of blocks takes
+@pytest.mark.parametrize("K,N,rows", [(192, 192, {1: True, 197: True, 560: True, 2000: False}), (768, 3072, {1: True, 24: True, 197: False}),
+                                      (1536, 384, {1: True, 16: False}), (192, 200, {1: False}), (100, 192, {1: False})])
+def test_packed_linear_in_one_launch_by_rows(pkg, K, N, rows):
+    applies = pkg._cabi.load().arcq_packed_linear_small_applies
+    assert {M: bool(applies(M, N, K)) for M in rows} == rows
