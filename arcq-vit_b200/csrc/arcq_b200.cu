@@ -1586,7 +1586,7 @@ static int launch_attention(const void* qkv, int64_t B, int64_t T, int64_t H, in
   if (!map(&tm_q, qkv, 3 * H * 64, arcq::kAttnQueries) || !map(&tm_kv, qkv, 3 * H * 64, p.tk) || !map(&tm_out, out, H * 64, 32))
     return fail(ARCQ_E_CUDA, "cuTensorMapEncodeTiled failed");
   const size_t smem = arcq::attn_smem_layout(p.tk).total;
-  const int cap = 2 * sm_count();
+  const int cap = sm_count();
   const unsigned grid = static_cast<unsigned>(p.items < cap ? p.items : cap);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 #define ARCQ_LAUNCH_ATTN(Q, BT)                                                                                      \

@@ -5,16 +5,23 @@
 //   or   xhat [B*T, H*64] fp16: the ARCQ reconstruction of that matrix in groups of 64.  A head's 64 outputs of a
 //        token are exactly one quantizer group, and one thread holds them.
 //
-// A work item is 128 queries of one (image, head); a block walks consecutive items, so that the second tile of a head finds
+// A work item is 128 queries of one (image, head); a block (one an SM) walks consecutive items, so that the second tile of a head finds
 // its keys and values in shared memory.  The whole score row of a query (T <= 256 keys) fits tensor memory, so there is no
 // online softmax and no rescaling: per item
 //   S = Q K^T       128 x tk fp32 in tensor memory (tk: T rounded up to 16; the TMA fills the rows beyond T with zeros)
-//   P = exp2(...)   a thread owns a query row: maximum, exponentials, sum; P as fp16 over the columns of S already read
+//   P = exp2(...)   two threads share a query row, one the lower keys, one the upper: maximum (exchanged through shared memory),
+//                   exponentials, sums; P as fp16 over the columns of S already read
 //   O = P V         P from tensor memory, V from shared memory as it lies (keys outside, no transposition)
 //   out             O / sum rounded to fp16, the quantizer of group_quant.cuh, 32 rows per warp to a TMA store
-// Warps: 0-3 softmax and 4-7 output and quantizer (one tensor-memory lane quarter each), 8 TMA loads, 9 products.  Two blocks an
-// SM, 256 tensor-memory columns each.  The next item's scores are computed, and its softmax runs, while this one's rows are
-// quantised; the product with the upper half of the keys runs while the lower half's exponentials are computed.
+// Warps (a tensor-memory lane quarter each): 0-3 upper keys, 4-7 lower keys, 8-11 and 12-15 output and quantizer of the even and of the
+// odd items, 16 TMA loads, 17 products.
+//
+// Tensor memory holds two items, 256 columns each: while the softmax warps work on one, the other's product runs, its output is read
+// and the scores of the item after the next are computed, so that the softmax warps go from item to item without a wait: 3700 cycles
+// an item (maximum 600, exponentials 2100 alone and 2700 beside the output warps).  What is left is the exponentials' pipe, 8 cycles a
+// warp or 1664 an item, issue slots, about 2400 an item, and instruction fetches.  With quantizer, 197 tokens: 64 images of 6 heads
+// 20.0 -> 18.1 us, 32 images 14.3 -> 11.4, 256 images of 12 heads 112 -> 101, one image 7.7 -> 7.2, against two blocks an SM with one item
+// each and a thread per row, whose softmax warps waited for P V, for the read of O and for the next Q K^T.
 //
 // Tensor memory is allocated after the previous kernel has ended and before the next one may start: a GEMM that holds all of
 // it while it waits for this kernel's result can then never be in the way.
@@ -29,18 +36,18 @@
 namespace arcq {
 
 constexpr int kStatusAttentionTimeout = 0x501;
-constexpr int kAttnRowWarps = 4;                  // softmax warps, and as many output warps
-constexpr int kAttnThreads = 3 * 128;             // the third warp group: TMA and products
-// Registers a thread, moved between the warp groups once they are running; the sum is that of the launch (80 each)
-constexpr int kAttnLaunchRegs = 80, kAttnSoftmaxRegs = 72, kAttnOutputRegs = 120, kAttnIssueRegs = 48;
-static_assert(kAttnSoftmaxRegs + kAttnOutputRegs + kAttnIssueRegs <= 3 * kAttnLaunchRegs, "registers beyond the launch's never come");
+constexpr int kAttnRowWarps = 4;                  // of a group: a warp a tensor-memory lane quarter
+constexpr int kAttnThreads = 5 * 128;             // two softmax groups, two output groups; the last: TMA and products
+// Registers a thread, moved between the warp groups once they are running; the sum is that of a launch with 80 each
+constexpr int kAttnLaunchRegs = 80, kAttnSoftmaxRegs = 80, kAttnOutputRegs = 96, kAttnIssueRegs = 48;
+static_assert(2 * kAttnSoftmaxRegs + 2 * kAttnOutputRegs + kAttnIssueRegs <= 5 * kAttnLaunchRegs, "registers beyond the launch's never come");
 constexpr int kAttnMaxT = 256;
 constexpr int kAttnQueries = 128;                 // per work item
 // Tensor memory of an item: S in columns 0 .. tk-1.  P takes the first half of the columns of the part of S that it was made
 // from: keys below attn_split(tk) at column 0, the others from column attn_split(tk) on.  O at 192, where S and P have ended
 // once the upper part has been read.
-constexpr uint32_t kAttnTmemCols = 256, kAttnOutCol = 192;
-__host__ __device__ constexpr int attn_split(int tk) { return tk < 32 ? tk : (tk / 2 + 31) / 32 * 32; }
+constexpr uint32_t kAttnTmemCols = 512, kAttnItemCols = 256, kAttnOutCol = 192;
+__host__ __device__ constexpr int attn_split(int tk) { return tk < 32 ? tk : tk < 64 ? (tk / 2 + 15) / 16 * 16 : tk / 64 * 32; }
 
 struct AttnParams {
   int T, H;
@@ -55,18 +62,19 @@ struct AttnParams {
 };
 
 struct AttnSmem {
-  uint32_t q, k, v, stage, tables, sums, bars, total;
+  uint32_t q, k, v, stage, tables, max, sums, bars, total;
 };
 __host__ __device__ inline AttnSmem attn_smem_layout(int tk) {
-  AttnSmem s;
+  AttnSmem s;                                               // q, k, v, max and sums twice: even and odd items (k, v: heads)
   s.q = 0;
-  s.k = s.q + kAttnQueries * 128;
-  s.v = s.k + static_cast<uint32_t>(tk) * 128;              // tk * 128 is a multiple of 2 KB
-  s.stage = s.v + static_cast<uint32_t>(tk) * 128;
-  s.tables = s.stage + kAttnRowWarps * 4096;
-  s.sums = s.tables + (static_cast<uint32_t>(sizeof(GroupQuantTables)) + 15) / 16 * 16;
-  s.bars = s.sums + kAttnQueries * 4;
-  s.total = s.bars + 16 * 8 + 16 + 1024 /* alignment */;
+  s.k = s.q + 2 * kAttnQueries * 128;
+  s.v = s.k + 2 * static_cast<uint32_t>(tk) * 128;          // tk * 128 is a multiple of 2 KB
+  s.stage = s.v + 2 * static_cast<uint32_t>(tk) * 128;
+  s.tables = s.stage + 2 * kAttnRowWarps * 4096;
+  s.max = s.tables + kGroupQuantTableBytes;
+  s.sums = s.max + 4 * kAttnQueries * 4;
+  s.bars = s.sums + 4 * kAttnQueries * 4;
+  s.total = s.bars + 24 * 8 + 16 + 1024 /* alignment */;
   return s;
 }
 
@@ -82,13 +90,31 @@ __device__ __forceinline__ void tma_store_3d(const void* tmap, const void* smem_
                "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
                : "memory");
 }
-// D[tmem] (+)= A[tmem, fp16 pairs] * B[smem]; issued by one thread
-__device__ __forceinline__ void umma_f16_tmem_a(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[tmem, fp16 pairs] * B[smem]; issued by one thread.  Operands in shared memory by the low words of their descriptors
+// (gemm_pair.cuh).
+__device__ __forceinline__ void umma_f16_tmem_a_lo(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+      "mov.b64 db, {%2, %5};\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kDescHi)
+      : "memory");
+}
+// D[tmem] = A . B^T over the four 16-wide K steps of one 64-wide sub-tile
+__device__ __forceinline__ void umma_f16_x4(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .b32 al, bl;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %4};\n\t"
+      "mov.b64 db, {%2, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, 0;\n\t"
+      "add.u32 al, %1, 2;\n\tadd.u32 bl, %2, 2;\n\tmov.b64 da, {al, %4};\n\tmov.b64 db, {bl, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, 1;\n\t"
+      "add.u32 al, %1, 4;\n\tadd.u32 bl, %2, 4;\n\tmov.b64 da, {al, %4};\n\tmov.b64 db, {bl, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, 1;\n\t"
+      "add.u32 al, %1, 6;\n\tadd.u32 bl, %2, 6;\n\tmov.b64 da, {al, %4};\n\tmov.b64 db, {bl, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, 1;\n\t}" ::"r"(d_tmem),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kDescHi)
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
@@ -117,22 +143,25 @@ __device__ __forceinline__ float exp2_approx(float x) {
 }
 
 template <bool QUANT, int BITS>
-__global__ void __launch_bounds__(kAttnThreads, 2)
+__global__ void __launch_bounds__(kAttnThreads, 1)
     attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
                      const __grid_constant__ CUtensorMap tm_out, const AttnParams p) {
   extern __shared__ uint8_t attn_smem_raw[];
   uint8_t* const smem = attn_smem_raw + ((1024u - (smem_u32(attn_smem_raw) & 1023u)) & 1023u);
   const AttnSmem L = attn_smem_layout(p.tk);
   uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + L.bars);
-  uint64_t *const q_full = bars, *const q_free = bars + 1, *const k_full = bars + 2, *const k_free = bars + 3,
-           *const v_full = bars + 4, *const v_free = bars + 5, *const s_full = bars + 6, *const o_full = bars + 7,
-           *const p_upper = bars + 8, *const p_lower = bars + 9, *const o_read = bars + 10, *const stopped = bars + 11;
-  uint32_t* const s_tmem = reinterpret_cast<uint32_t*>(bars + 16);
+  // [2] each, by the parity of the item (k, v: of the head)
+  uint64_t *const q_full = bars, *const q_free = bars + 2, *const k_full = bars + 4, *const k_free = bars + 6, *const v_full = bars + 8,
+           *const v_free = bars + 10, *const s_full = bars + 12, *const o_full = bars + 14, *const p_upper = bars + 16,
+           *const p_lower = bars + 18, *const o_read = bars + 20, *const stopped = bars + 22;
+  uint32_t* const s_tmem = reinterpret_cast<uint32_t*>(bars + 24);
+  float* const s_max = reinterpret_cast<float*>(smem + L.max);               // [parity][upper, lower][row]
   float* const s_sums = reinterpret_cast<float*>(smem + L.sums);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int T = p.T, C = p.H * 64;
   const int grid = static_cast<int>(gridDim.x), block = static_cast<int>(blockIdx.x);
   const int first = static_cast<int>(1ll * p.items * block / grid), last = static_cast<int>(1ll * p.items * (block + 1) / grid);
+  const int n = last - first;
   // head of an item (image, first column), first query
   auto place = [&](int it, int* b, int* x) {
     const int head = it / p.qtiles;
@@ -142,8 +171,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
   };
 
   if (tid == 0) {
-    for (int i = 0; i < 8; ++i) mbar_init(bars + i, 1);
-    for (int i = 8; i < 11; ++i) mbar_init(bars + i, kAttnRowWarps);
+    for (int i = 0; i < 16; ++i) mbar_init(bars + i, 1);
+    for (int i = 16; i < 22; ++i) mbar_init(bars + i, kAttnRowWarps);
     mbar_init(stopped, 1);
     mbar_fence_init();
   }
@@ -151,9 +180,9 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
   const uint32_t polls = p.poll_limit;
   bool ok = true;
 
-  if (warp >= 8) {
+  if (warp >= 16) {
     fewer_registers<kAttnIssueRegs>();
-    if (warp == 8) {
+    if (warp == 16) {
       // ---------------------------------------------------------------- TMA loads
       if (lane == 0) {
         tma_prefetch_desc(&tm_q);
@@ -161,41 +190,49 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
         tma_prefetch_desc(&tm_out);
       }
       pdl_wait();
-      uint32_t heads = 0, q_loads = 0, k_loads = 0;
-      auto loads = [&](int it) {
-        const uint32_t i = static_cast<uint32_t>(it - first);
+      int heads = 0, q_loads = 0, k_loads = 0;
+      auto loads = [&](int i) {
         int b, x;
-        const int q0 = place(it, &b, &x);
-        if (i > 0 && !mbar_wait(q_free, (i - 1) & 1, polls)) return false;
-        mbar_arrive_expect_tx(q_full, kAttnQueries * 128);
-        tma_load_3d(smem + L.q, &tm_q, q_full, x, q0, b);
+        const int q0 = place(first + i, &b, &x), qb = i & 1;
+        if (i > 1 && !mbar_wait(q_free + qb, ((i >> 1) - 1) & 1, polls)) return false;
+        mbar_arrive_expect_tx(q_full + qb, kAttnQueries * 128);
+        tma_load_3d(smem + L.q + qb * kAttnQueries * 128, &tm_q, q_full + qb, x, q0, b);
         ++q_loads;
         if (i == 0 || q0 == 0) {
-          if (heads > 0 && !mbar_wait(k_free, (heads - 1) & 1, polls)) return false;
-          mbar_arrive_expect_tx(k_full, static_cast<uint32_t>(p.tk) * 128);
-          tma_load_3d(smem + L.k, &tm_kv, k_full, C + x, 0, b);
+          const int hb = heads & 1, use = heads >> 1;
+          const uint32_t bytes = static_cast<uint32_t>(p.tk) * 128;
+          if (use > 0 && !mbar_wait(k_free + hb, (use - 1) & 1, polls)) return false;
+          mbar_arrive_expect_tx(k_full + hb, bytes);
+          tma_load_3d(smem + L.k + hb * bytes, &tm_kv, k_full + hb, C + x, 0, b);
           ++k_loads;
-          if (heads > 0 && !mbar_wait(v_free, (heads - 1) & 1, polls)) return false;
-          mbar_arrive_expect_tx(v_full, static_cast<uint32_t>(p.tk) * 128);
-          tma_load_3d(smem + L.v, &tm_kv, v_full, 2 * C + x, 0, b);
+          if (use > 0 && !mbar_wait(v_free + hb, (use - 1) & 1, polls)) return false;
+          mbar_arrive_expect_tx(v_full + hb, bytes);
+          tma_load_3d(smem + L.v + hb * bytes, &tm_kv, v_full + hb, 2 * C + x, 0, b);
           ++heads;
         }
         return true;
       };
-      if (lane == 0) ok = loads(first);
+      if (lane == 0) ok = loads(0);
       __syncwarp();
       __syncthreads();                    // tensor memory allocated
       pdl_launch_dependents();
       if (lane == 0) {
-        for (int it = first + 1; it < last && ok; ++it) ok = loads(it);
-        // No copy may land after the block has left, whichever warp has given up: the last one of each kind.
-        ok &= mbar_wait(q_full, (q_loads - 1) & 1) && mbar_wait(k_full, (k_loads - 1) & 1) && mbar_wait(v_full, (heads - 1) & 1);
+        for (int i = 1; i < n && ok; ++i) ok = loads(i);
+        // No copy may land after the block has left, whichever warp has given up: the last two of each kind.
+        auto landed = [&](uint64_t* bar, int loads) {
+          bool in = true;
+          for (int k = max(loads - 2, 0); k < loads; ++k) in &= mbar_wait(bar + (k & 1), (k >> 1) & 1);
+          return in;
+        };
+        ok = landed(q_full, q_loads) && ok;
+        ok = landed(k_full, k_loads) && ok;
+        ok = landed(v_full, heads) && ok;
         if (!ok) atomicExch(p.status, kStatusAttentionTimeout);
       }
       __syncwarp();
     } else {
-      // ---------------------------------------------------------------- products (warp 9); warps 10 and 11 only keep step
-      if (warp == 9) {
+      // ---------------------------------------------------------------- products (warp 17); warps 18 and 19 only keep step
+      if (warp == 17) {
         pdl_wait();
         tmem_alloc(s_tmem, kAttnTmemCols);
         tmem_relinquish();
@@ -204,89 +241,130 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
       __syncthreads();
       pdl_launch_dependents();
       tc_fence_after_sync();
-      if (warp == 9 && lane == 0) {
+      if (warp == 17) {
+        // The whole warp walks the loop, one elected lane issues, and there is one copy of each product: this warp's instructions are
+        // fetched anew for every item, behind the quantizer's.
         const uint32_t tmem = *s_tmem;
         const uint32_t idesc_s = umma_idesc_f16(kAttnQueries, p.tk);
         const uint32_t idesc_o = umma_idesc_f16(kAttnQueries, 64) | (1u << 16);      // B with its rows (keys) along K
-        const uint64_t dq = umma_desc_sw128(smem_u32(smem + L.q)), dk = umma_desc_sw128(smem_u32(smem + L.k)),
-                       dv = umma_desc_sw128(smem_u32(smem + L.v));
-        const int split = attn_split(p.tk);
-        uint32_t heads = 0;
-        for (int it = first; it < last; ++it) {
-          const uint32_t i = static_cast<uint32_t>(it - first);
-          const int q_tile = it % p.qtiles;
-          const bool new_head = i == 0 || q_tile == 0, end_head = it + 1 == last || q_tile + 1 == p.qtiles;
-          heads += new_head ? 1 : 0;
-          ok = (!new_head || mbar_wait(k_full, (heads - 1) & 1, polls)) && mbar_wait(q_full, i & 1, polls) &&
-               (i == 0 || mbar_wait(o_read, (i - 1) & 1, polls));
-          if (!ok) break;
-          tc_fence_after_sync();
-#pragma unroll
-          for (int k = 0; k < 4; ++k) umma_f16(tmem, dq + 2 * k, dk + 2 * k, idesc_s, k > 0);
-          umma_commit(s_full);
-          umma_commit(q_free);
-          if (end_head) umma_commit(k_free);
-          ok = (!new_head || mbar_wait(v_full, (heads - 1) & 1, polls)) && mbar_wait(p_upper, i & 1, polls);
-          if (!ok) break;
-          tc_fence_after_sync();
-          uint32_t acc = 0;
-          for (int k = split; k < p.tk; k += 16, acc = 1)
-            umma_f16_tmem_a(tmem + kAttnOutCol, tmem + split + (k - split) / 2, dv + 8 * k, idesc_o, acc);
-          ok = mbar_wait(p_lower, i & 1, polls);
-          if (!ok) break;
-          tc_fence_after_sync();
-          for (int k = 0; k < split; k += 16, acc = 1) umma_f16_tmem_a(tmem + kAttnOutCol, tmem + k / 2, dv + 8 * k, idesc_o, acc);
-          umma_commit(o_full);
-          if (end_head) umma_commit(v_free);
+        auto desc_lo = [&](uint32_t off) { return ((smem_u32(smem + off) & 0x3FFFFu) >> 4) | (1u << 16); };
+        const uint32_t q0 = desc_lo(L.q), k0 = desc_lo(L.k), v0 = desc_lo(L.v), kv_step = static_cast<uint32_t>(p.tk) * 128u >> 4;
+        const int split = attn_split(p.tk), tk = p.tk;
+        int s_head = -1, o_head = -1, s_tile = first % p.qtiles, o_tile = s_tile;    // heads and tiles of the scores and of the products with V
+#pragma unroll 1
+        for (int j = 0; j < n + 2 && ok; ++j) {
+          const uint32_t b = j & 1, item = tmem + b * kAttnItemCols, ph = (j >> 1) & 1;
+          if (j >= 2) {
+            // ---- P V of item j - 2
+            const bool new_head = j == 2 || o_tile == 0;
+            o_head += new_head ? 1 : 0;
+            if (++o_tile == p.qtiles) o_tile = 0;
+            const uint32_t hb = o_head & 1;
+            ok = (!new_head || mbar_wait(v_full + hb, (o_head >> 1) & 1, polls)) && mbar_wait(p_upper + b, ph ^ 1, polls);
+            tc_fence_after_sync();
+            uint32_t acc = 0;
+            if (ok && elect_one()) {
+#pragma unroll 1
+              for (int k = split; k < tk; k += 16, acc = 1)
+                umma_f16_tmem_a_lo(item + kAttnOutCol, item + split + ((k - split) >> 1), v0 + hb * kv_step + 8 * k, idesc_o, acc);
+            }
+            __syncwarp();
+            acc = split < tk ? 1 : 0;
+            ok = ok && mbar_wait(p_lower + b, ph ^ 1, polls);
+            tc_fence_after_sync();
+            if (ok && elect_one()) {
+#pragma unroll 1
+              for (int k = 0; k < split; k += 16, acc = 1)
+                umma_f16_tmem_a_lo(item + kAttnOutCol, item + (k >> 1), v0 + hb * kv_step + 8 * k, idesc_o, acc);
+              umma_commit(o_full + b);
+              if (j == n + 1 || o_tile == 0) umma_commit(v_free + hb);
+            }
+            __syncwarp();
+          }
+          if (j < n && ok) {
+            // ---- the scores of item j, over an item whose output has been read
+            const bool new_head = j == 0 || s_tile == 0;
+            s_head += new_head ? 1 : 0;
+            if (++s_tile == p.qtiles) s_tile = 0;
+            const uint32_t hb = s_head & 1;
+            ok = (!new_head || mbar_wait(k_full + hb, (s_head >> 1) & 1, polls)) && mbar_wait(q_full + b, ph, polls) &&
+                 (j < 2 || mbar_wait(o_read + b, ph ^ 1, polls));
+            tc_fence_after_sync();
+            if (ok && elect_one()) {
+              umma_f16_x4(item, q0 + b * (kAttnQueries * 128 >> 4), k0 + hb * kv_step, idesc_s);
+              umma_commit(s_full + b);
+              umma_commit(q_free + b);
+              if (j + 1 == n || s_tile == 0) umma_commit(k_free + hb);
+            }
+            __syncwarp();
+          }
         }
         if (!ok) {
           // products that were issued end before their tensor memory is given back
-          umma_commit(stopped);
+          if (elect_one()) umma_commit(stopped);
+          __syncwarp();
           mbar_wait(stopped, 0);
-          atomicExch(p.status, kStatusAttentionTimeout);
+          if (lane == 0) atomicExch(p.status, kStatusAttentionTimeout);
         }
       }
       __syncwarp();
     }
-  } else if (warp < kAttnRowWarps) {
-    // ------------------------------------------------------------------ softmax: a thread per query row
+  } else if (warp < 8) {
+    // ------------------------------------------------------------------ softmax: a query row for two threads
     fewer_registers<kAttnSoftmaxRegs>();
     __syncthreads();
     pdl_launch_dependents();
     tc_fence_after_sync();
-    const uint32_t slot = *s_tmem + (static_cast<uint32_t>(warp * 32) << 16);
+    const int lower = warp >> 2, quarter = warp & 3;
+    const uint32_t slot0 = *s_tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     constexpr float kScale = 0.125f * 1.44269504088896340736f;             // 1 / sqrt(64) and base 2
-    const int split = attn_split(p.tk), tk = p.tk;
+    const int split = attn_split(p.tk);
+    const int from = lower ? 0 : split, to = lower ? split : p.tk, full = min(to, T);      // keys of this thread; those that there are
     const float ninf = __int_as_float(0xff800000);
-    for (int it = first; it < last; ++it) {
-      const uint32_t ph = static_cast<uint32_t>(it - first) & 1;
-      const bool live = (it % p.qtiles) * kAttnQueries + warp * 32 < T;    // some of the warp's rows are queries
-      if (!mbar_wait(s_full, ph, polls)) { ok = false; break; }
+    const int row = quarter * 32 + lane;
+    int q_tile = first % p.qtiles;
+    // (a warp whose wait ran out goes on to the barriers, without waiting again)
+    for (int i = 0; i < n; ++i) {
+      const int b = i & 1;
+      const bool rows = q_tile * kAttnQueries + quarter * 32 < T;          // some of the warp's rows are queries
+      if (++q_tile == p.qtiles) q_tile = 0;
+      ok = ok && mbar_wait(s_full + b, (i >> 1) & 1, polls);
+      const bool live = rows && ok;
       tc_fence_after_sync();
-      // Loops with one body each, not unrolled over the row: the softmax and output warps of two blocks share an instruction
-      // cache, and unrolled passes stalled on it more than on anything else (DeiT-S batch 64, with the quantizer: 27.0 -> 24.1 us).
-      // The wait loops are part of that: with a constant limit instead of poll_limit 24.3 us against 21.4, 256 images of 12 heads 146
-      // against 113.
-      float nm = 0.0f;
+      const uint32_t slot = slot0 + b * kAttnItemCols;
+      // Loops with one body each, not unrolled over the row: the warps of an SM share an instruction cache, and unrolled passes stalled
+      // on it more than on anything else.
+      float* const mx = s_max + b * 2 * kAttnQueries + row;
       if (live) {
         float m0 = ninf, m1 = ninf, m2 = ninf, m3 = ninf;
-        uint32_t s[2][32];
-        int c = 0;
-#pragma unroll 1
-        for (; c + 64 <= T; c += 64) {
-          tmem_ld_32x32(slot + c, s[0]);
-          tmem_ld_32x32(slot + c + 32, s[1]);
-          tmem_ld_wait();
+        int c = from;
+        auto thirty_two = [&](const uint32_t (&s)[32]) {
 #pragma unroll
-          for (int j = 0; j < 64; j += 8) {
-            m0 = max3(m0, __uint_as_float(s[j >> 5][j & 31]), __uint_as_float(s[j >> 5][(j & 31) + 1]));
-            m1 = max3(m1, __uint_as_float(s[j >> 5][(j & 31) + 2]), __uint_as_float(s[j >> 5][(j & 31) + 3]));
-            m2 = max3(m2, __uint_as_float(s[j >> 5][(j & 31) + 4]), __uint_as_float(s[j >> 5][(j & 31) + 5]));
-            m3 = max3(m3, __uint_as_float(s[j >> 5][(j & 31) + 6]), __uint_as_float(s[j >> 5][(j & 31) + 7]));
+          for (int j = 0; j < 32; j += 8) {
+            m0 = max3(m0, __uint_as_float(s[j]), __uint_as_float(s[j + 1]));
+            m1 = max3(m1, __uint_as_float(s[j + 2]), __uint_as_float(s[j + 3]));
+            m2 = max3(m2, __uint_as_float(s[j + 4]), __uint_as_float(s[j + 5]));
+            m3 = max3(m3, __uint_as_float(s[j + 6]), __uint_as_float(s[j + 7]));
           }
+        };
+#pragma unroll 1
+        for (; c + 64 <= full; c += 64) {
+          uint32_t s0[32], s1[32];
+          tmem_ld_32x32(slot + c, s0);
+          tmem_ld_32x32(slot + c + 32, s1);
+          tmem_ld_wait();
+          thirty_two(s0);
+          thirty_two(s1);
+        }
+        if (c + 32 <= full) {
+          uint32_t s[32];
+          tmem_ld_32x32(slot + c, s);
+          tmem_ld_wait();
+          thirty_two(s);
+          c += 32;
         }
 #pragma unroll 1
-        for (; c < T; c += 16) {
+        for (; c < full; c += 16) {
           uint32_t t[16];
           tmem_ld_32x16(slot + c, t);
           tmem_ld_wait();
@@ -294,87 +372,84 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
           for (int j = 0; j < 16; j += 2)
             m0 = max3(m0, c + j < T ? __uint_as_float(t[j]) : ninf, c + j + 1 < T ? __uint_as_float(t[j + 1]) : ninf);
         }
-        nm = -kScale * fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+        mx[lower * kAttnQueries] = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
       }
-      const f32x2 k2 = pack2(kScale, kScale), nm2 = pack2(nm, nm);
-      f32x2 sum0 = pack2(0.0f, 0.0f), sum1 = sum0;
-      // sixteen scores to fp16 probabilities
-      auto exponentials = [&](const uint32_t* s, uint32_t* w) {
+      // the two warps of a lane quarter: each other's maximum is there (and the values of two items ago have been read)
+      asm volatile("bar.sync %0, 64;" ::"r"(4 + quarter) : "memory");
+      if (live) {
+        const float nm = -kScale * fmaxf(mx[0], mx[kAttnQueries]);
+        const f32x2 k2 = pack2(kScale, kScale), nm2 = pack2(nm, nm);
+        f32x2 sum0 = pack2(0.0f, 0.0f), sum1 = sum0;
+        // sixteen scores to fp16 probabilities
+        auto exponentials = [&](const uint32_t* s, uint32_t* w) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          float e0, e1;
-          unpack2(fma2(pack2(__uint_as_float(s[2 * j]), __uint_as_float(s[2 * j + 1])), k2, nm2), e0, e1);
-          const f32x2 e = pack2(exp2_approx(e0), exp2_approx(e1));
-          if (j & 1) sum1 = add2(sum1, e); else sum0 = add2(sum0, e);
-          w[j] = pair_to_sixteen<__half>(e);
-        }
-      };
-#pragma unroll 1
-      for (int part = 1; part >= 0; --part) {                              // upper keys first
-        if (live) {
-          int c = part ? split : 0, p_col = c;
-          const int to = part ? tk : split;
-#pragma unroll 1
-          for (; c + 32 <= min(to, T); c += 32, p_col += 16) {
-            uint32_t s[32], w[16];
-            tmem_ld_32x32(slot + c, s);
-            tmem_ld_wait();
-            exponentials(s, w);
-            exponentials(s + 16, w + 8);
-            tmem_st_32x16(slot + p_col, w);                                // over columns of S that have been read
+          for (int j = 0; j < 8; ++j) {
+            float e0, e1;
+            unpack2(fma2(pack2(__uint_as_float(s[2 * j]), __uint_as_float(s[2 * j + 1])), k2, nm2), e0, e1);
+            const f32x2 e = pack2(exp2_approx(e0), exp2_approx(e1));
+            if (j & 1) sum1 = add2(sum1, e); else sum0 = add2(sum0, e);
+            w[j] = pair_to_sixteen<__half>(e);
           }
+        };
+        int c = from, p_col = from;
 #pragma unroll 1
-          for (; c < to; c += 16, p_col += 8) {
-            uint32_t s[16], w[8];
-            tmem_ld_32x16(slot + c, s);
-            tmem_ld_wait();
+        for (; c + 32 <= full; c += 32, p_col += 16) {
+          uint32_t s[32], w[16];
+          tmem_ld_32x32(slot + c, s);
+          tmem_ld_wait();
+          exponentials(s, w);
+          exponentials(s + 16, w + 8);
+          tmem_st_32x16(slot + p_col, w);                                  // over columns of S that have been read
+        }
+#pragma unroll 1
+        for (; c < to; c += 16, p_col += 8) {
+          uint32_t s[16], w[8];
+          tmem_ld_32x16(slot + c, s);
+          tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 16; ++j) s[j] = c + j < T ? s[j] : 0xff800000u;        // keys beyond T: minus infinity
-            exponentials(s, w);
-            tmem_st_32x8(slot + p_col, w);
-          }
-          if (part == 0) {
-            float x0, x1;
-            unpack2(add2(sum0, sum1), x0, x1);
-            s_sums[warp * 32 + lane] = x0 + x1;
-          }
-          tmem_st_wait();
+          for (int j = 0; j < 16; ++j) s[j] = c + j < T ? s[j] : 0xff800000u;        // keys beyond T: minus infinity
+          exponentials(s, w);
+          tmem_st_32x8(slot + p_col, w);
         }
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(part ? p_upper : p_lower);
+        float x0, x1;
+        unpack2(add2(sum0, sum1), x0, x1);
+        s_sums[(b * 2 + lower) * kAttnQueries + row] = x0 + x1;
+        tmem_st_wait();
       }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive((lower ? p_lower : p_upper) + b);
     }
     if (!ok && lane == 0) atomicExch(p.status, kStatusAttentionTimeout);
   } else {
     // ------------------------------------------------------------------ output: a thread per query row
     more_registers<kAttnOutputRegs>();
-    const int quarter = warp - kAttnRowWarps;
+    const int quarter = warp & 3, parity = (warp - 8) >> 2;
     GroupQuantTables* const tables = reinterpret_cast<GroupQuantTables*>(smem + L.tables);
     GroupQuantParams gp = {};
     // reads only the layer's constants: done while the previous kernel still runs
     if (QUANT)
-      gp = group_quant_tables<1 << BITS, false>(tables, p.thresholds, p.codebook, tid - 128, kAttnRowWarps * 32, [](bool b) {
-        asm volatile("bar.sync 1, %0;" ::"n"(kAttnRowWarps * 32) : "memory");
+      gp = group_quant_tables<1 << BITS, false>(tables, p.thresholds, p.codebook, tid - 256, 2 * kAttnRowWarps * 32, [](bool b) {
+        asm volatile("bar.sync 1, %0;" ::"n"(2 * kAttnRowWarps * 32) : "memory");
         return b;
       });
     __syncthreads();
     pdl_launch_dependents();
     tc_fence_after_sync();
-    const uint32_t t_out = *s_tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kAttnOutCol;
-    uint8_t* const stage = smem + L.stage + quarter * 4096;
+    const uint32_t t_out = *s_tmem + (static_cast<uint32_t>(quarter * 32) << 16) + parity * kAttnItemCols + kAttnOutCol;
+    const float* const sums = s_sums + parity * 2 * kAttnQueries + quarter * 32 + lane;
+    uint8_t* const stage = smem + L.stage + (warp - 8) * 4096;
     const uint32_t row = smem_u32(stage) + lane * 128, x7 = lane & 7;
-    for (int it = first; it < last; ++it) {
-      const uint32_t ph = static_cast<uint32_t>(it - first) & 1;
+    for (int i = parity; i < n; i += 2) {
+      const uint32_t ph = (i >> 1) & 1;
       int b, x;
-      const int t0 = place(it, &b, &x) + quarter * 32;
+      const int t0 = place(first + i, &b, &x) + quarter * 32;
       const bool live = t0 < T;
-      // p_lower: the sums are there
-      if (!mbar_wait(p_lower, ph, polls) || !mbar_wait(o_full, ph, polls)) { ok = false; break; }
+      if (!mbar_wait(o_full + parity, ph, polls) || !mbar_wait(p_upper + parity, ph, polls) || !mbar_wait(p_lower + parity, ph, polls)) { ok = false; break; }
       tc_fence_after_sync();
       uint32_t w[32];
       if (live) {
-        const float inv = __frcp_rn(s_sums[quarter * 32 + lane]);
+        const float inv = __frcp_rn(sums[0] + sums[kAttnQueries]);
         const f32x2 inv2 = pack2(inv, inv);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -389,7 +464,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(o_read);
+        mbar_arrive(o_read + parity);
+
         tma_store_wait_read();                             // the store that last used the staging rows has read them
       }
       __syncwarp();
@@ -418,7 +494,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 9) {
+  if (warp == 17) {
     tc_fence_after_sync();
     tmem_dealloc(*s_tmem, kAttnTmemCols);
   }

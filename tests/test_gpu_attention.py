@@ -419,3 +419,19 @@ def test_where_the_library_attention_stays(pkg, cuda_device, why, monkeypatch):
     with torch.no_grad():
         assert not torch.equal(attn(x), results[0])              # without the reason: the kernel
     assert pkg.ops.device_status() == 0
+
+
+# one to six items a block (both halves of tensor memory in turn), heads of one and of two query tiles, splits of the keys for the two
+# threads of a row: all of them lower, uneven, even, the longest
+@pytest.mark.parametrize("B,T,H", [(1, 5, 1), (150, 17, 1), (40, 33, 5), (75, 64, 6), (30, 100, 12), (150, 129, 1), (40, 197, 12), (60, 240, 6), (37, 256, 12)])
+def test_items_of_a_block_one_after_the_other(pkg, cuda_device, B, T, H):
+    gen = torch.Generator(device=cuda_device).manual_seed(B + T + H)
+    qkv = torch.randn(B * T, 3 * H * 64, generator=gen, device=cuda_device).half()
+    out = pkg.ops.attention(qkv, B, T, H)
+    q, k, v = qkv.double().view(B, T, 3, H, 64).permute(2, 0, 3, 1, 4)
+    want = (torch.softmax(q @ k.transpose(-1, -2) / 8, -1) @ v).transpose(1, 2).reshape(B * T, H * 64)
+    # probabilities rounded to fp16 (2^-11 of each, times |v| < 6), the output's own rounding, fp32 sums of T terms
+    assert float((out.double() - want).abs().max()) <= 6 * 2.0 ** -11 + 2.0 ** -11 * float(want.abs().max()) + T * 6 * 2.0 ** -22
+    part = pkg.ops.attention(qkv[-T:].contiguous(), 1, T, H)              # the last image on its own: other blocks, other halves
+    assert torch.equal(part, out[-T:])
+    assert pkg.ops.device_status() == 0
