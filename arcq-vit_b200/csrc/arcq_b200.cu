@@ -83,7 +83,7 @@ enum Opt {
   O_ACT_QUANT_V1, O_LN_PLAIN,
   O_PAIR, O_PAIR_MIN_M, O_PAIR_BN, O_PAIR_SA, O_PAIR_KS, O_PAIR_NBB, O_PAIR_LUT, O_PAIR_PAIRS, O_PAIR_STATIONARY,
   O_PAIR_WS, O_LNQ_SMALL, O_AQ2_MIN_GROUPS, O_PDL, O_GELU_GEMM, O_GEMM_UNPACK, O_POLL_LIMIT, O_SPIN_LIMIT, O_LAUNCH_REGS,
-  O_SMALL_LINEAR, O_SMALL_R, O_SMALL_BN,
+  O_SMALL_LINEAR, O_SMALL_R, O_SMALL_BN, O_PAIR_SPLIT,
   O_COUNT
 };
 struct OptDef { const char* name; int dflt; };
@@ -96,7 +96,7 @@ const OptDef kOptDefs[O_COUNT] = {
     {"ARCQ_PAIR_STATIONARY", -1}, {"ARCQ_PAIR_WS", 0}, {"ARCQ_LNQ_SMALL", 1}, {"ARCQ_AQ2_MIN_GROUPS", 0}, {"ARCQ_PDL", 1},
     {"ARCQ_GELU_GEMM", -1}, {"ARCQ_GEMM_UNPACK", 1},
     {"ARCQ_POLL_LIMIT", 1 << 21}, {"ARCQ_SPIN_LIMIT", 1 << 25}, {"ARCQ_LAUNCH_REGS", 0},
-    {"ARCQ_SMALL_LINEAR", -1}, {"ARCQ_SMALL_R", 0}, {"ARCQ_SMALL_BN", 0},
+    {"ARCQ_SMALL_LINEAR", -1}, {"ARCQ_SMALL_R", 0}, {"ARCQ_SMALL_BN", 0}, {"ARCQ_PAIR_SPLIT", 1},
 };
 int g_opt[O_COUNT];
 void load_options() {
@@ -558,7 +558,7 @@ bool choose_pair_config(long long M, long long N, long long K, int bits, bool y_
 
 // ---- dense-weight CTA-pair kernel: configuration ----
 struct PairDenseConfig {
-  int bn, sa, ks, pairs, stationary;
+  int bn, sa, ks, pairs, stationary, split_last;
   size_t smem;
   double cost;     // of the model that chose it
 };
@@ -678,7 +678,14 @@ bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32,
       // fastest on average, 25 % at worst.  The larger of the tiles' time and of the fill at 8 TB/s had 3.2 and 29 %, with 12 TB/s
       // from K = 768 on 2.7 and 25 %, and that took narrow slabs for wide fp32 outputs: N = 3072, K = 768, 25216 rows 151 us against
       // 122, N = 2304 114 against 94; now no shape is more than 2.4 % behind the better of the two.
-      const double cost = tiles_pp * ((t_write > t_issue ? t_write : t_issue) + 0.8) + fill_mb / 20.0;
+      const double tile = t_write > t_issue ? t_write : t_issue;
+      double cost = tiles_pp * (tile + 0.8) + fill_mb / 20.0;
+      // Tiles that would fill half of another round at most come as halves (a half has to be a width of the instruction's), from K =
+      // 1024 on: 12 608 rows of K = 1536, N = 384 are 100 tiles on 74 pairs, 19.5 us whole and 18.0 with the last 26 halved.  A shorter tile
+      // is its stores and its latency: K = 384, N = 384 7.5 / 7.8 us, K = 768, N = 768 25.1 / 25.4, N = 2304 38.7 / 37.9.
+      const long long left = slabs * tiles_m % k.pairs;
+      k.split_last = !stationary && opt(O_PAIR_SPLIT) != 0 && G >= 16 && slabs * tiles_m > k.pairs && left > 0 && 2 * left <= k.pairs && bn % 64 == 0;
+      if (k.split_last) cost -= tile / 2;
       k.cost = cost;
       if (!found || cost < best.cost) { best = k; found = true; }
     }
@@ -1139,7 +1146,7 @@ static int launch_pair_dense_gemm(const PairDenseConfig& cfg, const void* xhat, 
   p.codebook = q_codebook;
   p.bias = bias;
   p.M = static_cast<int>(M); p.N = static_cast<int>(N); p.K = static_cast<int>(K); p.G = static_cast<int>(K / 64);
-  p.bn = cfg.bn; p.sa = cfg.sa; p.ks = cfg.ks;
+  p.bn = cfg.bn; p.sa = cfg.sa; p.ks = cfg.ks; p.split_last = cfg.split_last;
   p.y_f32 = (y_dtype == ARCQ_DT_F32) ? 1 : 0;
   p.poll_limit = static_cast<uint32_t>(opt(O_POLL_LIMIT));
   p.spin_limit = static_cast<uint32_t>(opt(O_SPIN_LIMIT));

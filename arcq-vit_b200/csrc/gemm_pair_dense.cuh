@@ -48,6 +48,7 @@ struct PairDenseParams {
   uint32_t spin_limit;  // the issuing thread's busy waits give up after this many probes
   int* status;
   int pairs;       // CTA pairs that multiply; pairs beyond them take the unpack jobs
+  int split_last;  // the tiles that do not fill a round come as two halves of a slab each (streamed form without a quantizer)
   const float* thresholds;   // quantizer form only
   const float* codebook;
   UnpackWeightJob next;  // the weight of the layer that runs after this one, unpacked by two spare warps (or none)
@@ -134,7 +135,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
   const int slab = pair % n_slabs;     // stationary: the pair's slab
   const int rank = pair / n_slabs;
   const int pairs_in_slab = (n_pairs - slab + n_slabs - 1) / n_slabs;
+  // Rounds in which every pair has a whole tile; what is left over is at most half a round where it comes in halves (split_last).
+  const bool split = !STATIONARY && QBITS == 0 && p.split_last != 0;
+  const int full_rounds = split ? tiles_m * n_slabs / n_pairs : 0;
   const int my_tiles = STATIONARY ? ((rank < tiles_m) ? (tiles_m - rank + pairs_in_slab - 1) / pairs_in_slab : 0)
+                       : split    ? full_rounds + (pair < 2 * (tiles_m * n_slabs - full_rounds * n_pairs) ? 1 : 0)
                                   : (tiles_m * n_slabs - pair + n_pairs - 1) / n_pairs;
   // pairs of different slabs that share a rank walk the same row tiles; stagger their starting points
   const int rot = (STATIONARY && my_tiles > 0) ? (slab * my_tiles) / n_slabs : 0;
@@ -145,13 +150,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
   // tile is known from above, the others follow by steps.
   const int step_m = STATIONARY ? 0 : n_pairs / n_slabs, step_s = n_pairs - step_m * n_slabs;
   struct Walk {
-    int q, m, s;       // stationary: q-th of the pair's row tiles; else row tile and slab
+    int q, m, s;       // stationary: q-th of the pair's row tiles; else how many tiles came before, row tile and slab
+    int c, width;      // the tile's columns of the slab
   };
-  auto first_tile = [&]() { return Walk{rot, rank, slab}; };
+  auto first_tile = [&]() { return Walk{STATIONARY ? rot : 0, rank, slab, 0, bn}; };
   auto row_of = [&](const Walk& w) {
     return (STATIONARY ? rank + w.q * pairs_in_slab : w.m) * kPairTileM + static_cast<int>(crank) * kTileM;
   };
-  auto col_of = [&](const Walk& w) { return (STATIONARY ? slab : w.s) * bn; };
+  auto col_of = [&](const Walk& w) { return STATIONARY ? slab * bn : w.s * bn + w.c; };
   auto advance = [&](Walk& w) {
     if constexpr (STATIONARY) {
       w.q = w.q + 1 == my_tiles ? 0 : w.q + 1;
@@ -159,6 +165,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
       w.m += step_m;
       w.s += step_s;
       if (w.s >= n_slabs) { w.s -= n_slabs; ++w.m; }
+      if (QBITS == 0 && split && ++w.q == full_rounds) {
+        const int left = full_rounds * n_pairs + (pair >> 1);
+        w.m = left / n_slabs;
+        w.s = left - w.m * n_slabs;
+        w.width = hb;
+        w.c = (pair & 1) * hb;
+      }
     }
   };
   const uint32_t poll_limit = p.poll_limit, spin_limit = p.spin_limit;
@@ -215,7 +228,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
       }
       Walk w = first_tile();
       for (int t = 0; t < my_tiles; ++t, advance(w)) {
-        const int row0 = row_of(w), nh0 = col_of(w) + static_cast<int>(crank) * hb;     // nh0: first W16 row this CTA loads
+        const int row0 = row_of(w), nh0 = col_of(w) + static_cast<int>(crank) * (w.width >> 1);     // nh0: first W16 row this CTA loads
         for (int g0 = 0; g0 < G; g0 += ks) {
           good &= mbar_park_flag(empty + slot * 8, ph, good ? poll_limit : 0u);
           if (elect_one()) {
@@ -245,7 +258,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
     } else if (warp == 1) {
       // ------------------------------------------------------------------ MMA issue (leader CTA only)
       if (crank == 0 && my_tiles > 0) {
-        const uint32_t idesc = umma_idesc_f16(kPairTileM, bn);
+        const uint32_t idesc_full = umma_idesc_f16(kPairTileM, bn), idesc_half = umma_idesc_f16(kPairTileM, hb);
         const uint32_t sa = p.sa;
         const uint32_t lo0 = ((smem_u32(sStages) & 0x3FFFFu) >> 4) | (1u << 16);
         const uint32_t s_step = stage_bytes >> 4, w_off = (static_cast<uint32_t>(ks) * kStageA) >> 4, w_step = wtile_bytes >> 4;
@@ -261,6 +274,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
           acc_ph1 ^= buf ? 1u : 0u;
           tc_fence_after_sync();
           const uint32_t d = tmem_base + buf * 256;
+          const uint32_t idesc = split && t == full_rounds ? idesc_half : idesc_full;
           uint32_t acc = 0;
           for (int g0 = 0; g0 < G; g0 += ks) {
             if (STATIONARY && t == 0) {   // the slab lands while the first tile runs
@@ -416,10 +430,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
     float* const sb = s_bias + half_id * 128;
     const int bi = (ew & 3) * 32 + lane;
     const int bcol = bi / cw * 2 * cw + half_id * cw + bi % cw;
-    const bool has_bias = p.bias != nullptr && bcol < bn;
     float next_b = 0.0f;
     Walk next = first_tile();
-    if (my_tiles > 0 && has_bias) next_b = __ldg(p.bias + col_of(next) + bcol);
+    auto read_bias = [&]() {
+      if (p.bias != nullptr && bcol < next.width) next_b = __ldg(p.bias + col_of(next) + bcol);
+    };
+    if (my_tiles > 0) read_bias();
     auto four_warps = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(3 + half_id) : "memory"); };
     uint32_t blk = 0;      // staging block of the next store; the blocks are used in turn
     auto emit = [&](const uint32_t (&acc)[32], int c0, int row0, int n0) {
@@ -466,13 +482,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
     const int step = 2 * cw;
     for (int t = 0; t < my_tiles; ++t) {
       const uint32_t buf = static_cast<uint32_t>(t) & 1;
-      const int row0 = row_of(next) + lq * 32, n0 = col_of(next);
+      const int row0 = row_of(next) + lq * 32, n0 = col_of(next), width = next.width;
       advance(next);
       if (!STATIONARY || t == 0) {
         if (t > 0) four_warps();
         sb[bi] = next_b;
         four_warps();
-        if (!STATIONARY && t + 1 < my_tiles && has_bias) next_b = __ldg(p.bias + col_of(next) + bcol);
+        if (!STATIONARY && t + 1 < my_tiles) read_bias();
       }
       // (a warp whose wait ran out goes on to the barriers above, without waiting again)
       ok = ok && mbar_wait_sleep_a(acc_full + buf * 8, (static_cast<uint32_t>(t) >> 1) & 1, poll_limit, 32);
@@ -491,17 +507,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
         if (lane == 0) mbar_arrive_cluster(acc_empty_leader + buf * 8);
         released = true;
       };
-      if (live && c0 < bn) {
+      if (live && c0 < width) {
         load(ra, t_row + c0);
         while (true) {
           tmem_ld_wait();
-          bool more = c0 + step < bn;
+          bool more = c0 + step < width;
           if (more) load(rb, t_row + c0 + step); else release();
           emit(ra, c0, row0, n0);
           if (!more) break;
           c0 += step;
           tmem_ld_wait();
-          more = c0 + step < bn;
+          more = c0 + step < width;
           if (more) load(ra, t_row + c0 + step); else release();
           emit(rb, c0, row0, n0);
           if (!more) break;

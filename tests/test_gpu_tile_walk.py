@@ -6,9 +6,11 @@ pytestmark = pytest.mark.gpu
 
 
 # K = 768 streams both operands: fewer tiles than pairs, one more than a round, several rounds; slabs of every width, ragged rows,
-# widths that leave a slab to one half of the epilogue warps (32, 96, 160)
+# widths that leave a slab to one half of the epilogue warps (32, 96, 160); from K = 1024 on the last round in halves: one tile of it,
+# several, half a round
 @pytest.mark.parametrize("M,N,K", [(1, 32, 768), (300, 96, 768), (300, 160, 768), (1000, 2304, 768), (6305, 768, 768), (6305, 3072, 768),
-                                   (19001, 768, 768), (700, 384, 1536), (12608, 384, 1536)])
+                                   (19001, 768, 768), (700, 384, 1536),
+                                   (12608, 384, 1536), (6305, 768, 1024), (19001, 768, 1024), (9473, 512, 1088)])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
 @pytest.mark.parametrize("bias", ["none", "aligned", "offset"])
 def test_every_tile_gets_its_columns_and_its_bias(pkg, cuda_device, M, N, K, dtype, bias):
@@ -22,7 +24,9 @@ def test_every_tile_gets_its_columns_and_its_bias(pkg, cuda_device, M, N, K, dty
     # fp32 sums of K products of unit variance, then one rounding to the output type
     tol = 2.0 ** -24 * K + want.abs() * (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -23)
     assert bool(((y.double() - want).abs() <= tol + 2.0 ** -25).all())
-    # a row does not depend on the tile it falls in
+    # a row does not depend on the tile it falls in, a whole one or a half
+    with pkg._cabi.option("ARCQ_PAIR_SPLIT", 0):
+        assert torch.equal(pkg.ops.dense_weight_gemm(x, w, b, dtype), y)
     part = pkg.ops.dense_weight_gemm(x[M // 2:].contiguous(), w, b, dtype)
     assert torch.equal(part, y[M // 2:])
     assert pkg.ops.device_status() == 0
