@@ -632,13 +632,16 @@ bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32,
   static const int cand[] = {256, 192, 160, 128, 96, 64, 32};
   bool found = false;
   PairDenseConfig best = {};
-  // One or two row tiles (batch 1-2 of a ViT): the launch is a latency chain, not a throughput problem.  The
-  // narrowest slab that still gives every (tile, slab) its own pair spreads the epilogue over the most SMs
-  // (DeiT-S batch 1: 0.528 ms with 32-column slabs against 0.555 ms with the throughput model's choice).
+  // Up to four row tiles (batch 1-5 of a ViT): the launch is a latency chain, not a throughput problem, and the narrowest slab that gives
+  // every (tile, slab) its own pair is the shortest chain, as long as that is no more than 40 pairs: every pair beyond them costs the launch
+  // more than a narrower slab saves (K = 384, N = 1536: 197 rows 64 columns 4.4 us, 32 4.9; 394 rows 96 columns 4.6, 64 5.1; K = 768, N = 2304,
+  // 197 rows 64 columns 5.6, 32 6.7).  Over twelve layers of the three widths with 197 to 1576 rows the slab chosen is 1.3 % slower than the
+  // fastest; with up to two row tiles and all pairs it was 4.2 %, 24 % at worst.
+  constexpr int kLatencyTiles = 4, kLatencyPairs = 40;
   int narrow_bn = 0;
-  if (tiles_m <= 2 && opt(O_PAIR_BN) == 0)
+  if (tiles_m <= kLatencyTiles && opt(O_PAIR_BN) == 0)
     for (int bn : cand)
-      if (N % bn == 0 && (N / bn) * tiles_m <= max_pairs) narrow_bn = bn;      // candidates descend: keeps the narrowest
+      if (N % bn == 0 && (N / bn) * tiles_m <= (max_pairs < kLatencyPairs ? max_pairs : kLatencyPairs)) narrow_bn = bn;      // candidates descend: keeps the narrowest
   for (int bn : cand) {
     if (N % bn != 0) continue;
     if (opt(O_PAIR_BN) > 0 && bn != opt(O_PAIR_BN)) continue;
