@@ -781,7 +781,11 @@ struct SmallLinearConfig {
 bool choose_small_linear(long long M, long long N, long long K, SmallLinearConfig* c) {
   const int force = opt(O_SMALL_LINEAR);
   if (force == 0 || M <= 0 || M > 4096 || K % 64 != 0 || N % 16 != 0 || K > (1 << 16) || N > (1 << 20)) return false;
-  const int G = static_cast<int>(K / 64), n = static_cast<int>(N), sms = sm_count();
+  const int G = static_cast<int>(K / 64), n = static_cast<int>(N);
+  // More than one round of blocks can take with four times 96 groups and 384 columns of a group a block: calls on many rows end here, before
+  // the search (of some 2400 shapes this refuses seven that the costs below would take, all of K >= 1536 and N >= 2304).
+  if (force < 0 && M * N * G * G > 4ll * 148 * 96 * 384) return false;
+  const int sms = sm_count();
   const double two_launches = 5.3 + 0.002 * static_cast<double>(K) + 1.6e-6 * static_cast<double>(N * K);
   double limit = force > 0 ? 1.0e9 : two_launches + 0.8;       // what the next candidate has to be below
   bool found = false;
