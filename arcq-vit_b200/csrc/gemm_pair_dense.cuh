@@ -318,9 +318,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
     // ------------------------------------------------------------------ epilogue with GELU and quantizer
     // A thread owns one row and 64 columns, i.e. one group of the next layer's activation quantizer: tensor memory -> + bias ->
     // fp16 (what the plain form stores) -> GELU -> quantizer -> reconstruction, in registers but for the exchange of large GELU
-    // arguments, then through this warp's staging rows to a TMA store.  Issue slots of these warps bound the kernel (about 30
-    // instructions a value); the products run underneath.  K = 768, N = 3072, back to back with inputs in turn: 12608 rows 90.7 us
-    // against 101.4 for GEMM and quantizer kernel, 100864 rows 787 against 984.
+    // arguments, then through this warp's staging rows to a TMA store.  Issue slots and the FMA pipe (54 % busy)
+    // of these warps bound the kernel, about 28 instructions a value; the products run underneath.  K = 768, N = 3072, back to back with
+    // inputs in turn: 12608 rows 66 us, 100864 rows 500 (GEMM and quantizer kernel 360 + 329); K = 384, N = 1536, 12608 rows 32.
     const int ew = warp - kIssue, lq = warp & 3, grp = ew >> 2;
     GroupQuantTables* const tables = reinterpret_cast<GroupQuantTables*>(smem + L.tables);
     const GroupQuantParams gp = group_quant_tables<1 << QBITS, false>(tables, p.thresholds, p.codebook, tid - kIssue * 32, kEpi * 32, [](bool b) {
