@@ -110,9 +110,9 @@ __global__ void __launch_bounds__(256) dequant64_kernel(const uint8_t* __restric
                                                         const float* __restrict__ codebook, long long total, OUT* __restrict__ out) {
   pdl_launch_dependents();
   __shared__ float s_cb[16];
+  pdl_wait();                // codes, statistics and levels are a call's arguments: any of them may be the previous kernel's output
   if (threadIdx.x < 16) s_cb[threadIdx.x] = (threadIdx.x < (1 << BITS)) ? __ldg(codebook + threadIdx.x) : 0.0f;
   __syncthreads();
-  pdl_wait();                // codes and statistics may be the previous kernel's output
   const long long stride = static_cast<long long>(gridDim.x) * 256;
   for (long long i0 = blockIdx.x * 256ll + threadIdx.x; i0 < total; i0 += 2 * stride) {
     uint32_t w[2];
