@@ -1547,7 +1547,7 @@ int arcq_add_layernorm_act_quant_unpack(const void* x, const void* y, const void
       done_dev = dev;                                                                                                  \
     }                                                                                                                  \
     launch_pdl(k, grid, arcq::kLnqThreads, smem, st, tm_out, xh, yh, np, eps, static_cast<long long>(M), thresholds,   \
-               codebook, so, ho, one_fma, status, jobs);                                                               \
+               codebook, so, ho, one_fma, static_cast<uint32_t>(opt(O_POLL_LIMIT)), status, jobs);                     \
   } while (0)
 #define ARCQ_LNQ_BITS(LN, HASY)                                                                                         \
   do {                                                                                                                  \

@@ -57,8 +57,8 @@ __global__ void __launch_bounds__(kLnqThreads, 4)
     add_layernorm_act_quant_kernel(const __grid_constant__ CUtensorMap tm_out, const __half* __restrict__ x,
                                    const __half* __restrict__ y, const NormParams np, float eps, long long M,
                                    const float* __restrict__ thresholds, const float* __restrict__ codebook,
-                                   __half* __restrict__ sum_out, __half* __restrict__ h_out, int one_fma, int* status,
-                                   const __grid_constant__ UnpackJobs jobs) {
+                                   __half* __restrict__ sum_out, __half* __restrict__ h_out, int one_fma, uint32_t poll_limit,
+                                   int* status, const __grid_constant__ UnpackJobs jobs) {
   pdl_launch_dependents();   // the next kernel of the stream may start its set-up
   extern __shared__ __align__(1024) uint8_t lnq_smem[];
   if (static_cast<int>(blockIdx.x) < jobs.blocks) {
@@ -107,9 +107,9 @@ __global__ void __launch_bounds__(kLnqThreads, 4)
     // ---- phase 1: LayerNorm of every row the tile touches, LANES lanes per row
     LaneNorm norm;                          // read for each tile: the quantizer needs the registers
     layernorm_lane_params<LANES>(np, l, &norm);
-    ok = ok && mbar_wait(bar, ph);          // (given up once: the block goes on without waiting, and says so below)
+    ok = mbar_wait_warp(bar, ph, poll_limit);
 #pragma unroll 1
-    for (int pass = 0; pass < kPasses; ++pass) {
+    for (int pass = 0; pass < kPasses && ok; ++pass) {
       const int lr = pass * kRowsPerPass + warp * kRowsPerWarp + sub;
       const long long row = r_first + lr;
       const long long lg0 = row * G - gi0;                       // tile-local index of the row's first group
@@ -134,7 +134,8 @@ __global__ void __launch_bounds__(kLnqThreads, 4)
         }
       }
     }
-    __syncthreads();
+    ok = __syncthreads_and(ok) != 0;
+    if (!ok) break;                         // some warp's wait ran out: nothing of this tile is quantised, no copy over rows that may still come
     if (tid == 0 && tile + stride < tiles) load(tile + stride);
 
     // ---- phase 2: the activation quantizer on h, one thread per group, in place; a warp sends its 32 rows out by TMA
@@ -150,7 +151,10 @@ __global__ void __launch_bounds__(kLnqThreads, 4)
     __syncthreads();   // the rows are free for the next tile
   }
   if (lane == 0) tma_store_wait_all();
-  if (!ok && tid == 0) atomicExch(status, kStatusLnqTimeout);
+  if (!ok && tid == 0) {
+    mbar_wait(bar, ph);                     // the copy that is still on its way lands before the block leaves
+    atomicExch(status, kStatusLnqTimeout);
+  }
 }
 
 // ---------------------------------------------------------------------------------------------------------

@@ -96,6 +96,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   }
   return false;
 }
+// The same for a whole warp, with one answer for all its lanes: every lane counts its own polls, so lanes could give up on either side of
+// the phase's end, and what follows a wait is often an instruction that all lanes have to reach together.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint32_t polls = kMaxPolls) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, polls)) != 0;
+}
 // Non-blocking test of a phase (never suspends the thread): for the one thread whose reaction time is on
 // the critical path.
 __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {

@@ -44,3 +44,34 @@ def test_residual_sum_is_rounded_once(pkg, cuda_device):
     s, _ = pkg.ops.add_layernorm(x, y, norm)
     want = (x.float() + y.float()).half()
     assert torch.equal(torch.nan_to_num(s.float(), nan=1e9), torch.nan_to_num(want.float(), nan=1e9))
+
+
+@pytest.mark.parametrize("K,M", [(192, 43), (384, 12651), (768, 13001)])      # one tile, and several tiles a block
+@pytest.mark.parametrize("with_y", [True, False])
+def test_a_wait_for_the_rows_that_runs_out(pkg, cuda_device, K, M, with_y):
+    """No poll: the kernel ends, says so in the status word and has stored nothing, and the next launch is none the worse."""
+    gen = torch.Generator(device=cuda_device).manual_seed(K + M)
+    x = torch.randn(M, K, generator=gen, device=cuda_device).half()
+    y = torch.randn(M, K, generator=gen, device=cuda_device).half()
+    gamma, beta = torch.ones(K, device=cuda_device).half(), torch.zeros(K, device=cuda_device).half()
+    cb = torch.linspace(-2.2, 2.2, 16, device=cuda_device)
+    th = (cb[:-1] + cb[1:]) / 2
+    lib = pkg._cabi.load()
+
+    def run():
+        outs = [torch.full((M, K), 77.0, device=cuda_device).half() for _ in range(3)]
+        torch.cuda.synchronize()
+        rc = lib.arcq_add_layernorm_act_quant_unpack(
+            x.data_ptr(), y.data_ptr() if with_y else None, gamma.data_ptr(), beta.data_ptr(), pkg._cabi.DT_F16, 1e-6, M, K, th.data_ptr(),
+            cb.data_ptr(), 4, 64, outs[0].data_ptr() if with_y else None, outs[1].data_ptr(), outs[2].data_ptr(), 0, None, 0, None)
+        assert rc == 0
+        return outs
+    with pkg._cabi.option("ARCQ_LNQ_SMALL", 0):
+        want = run()
+        with pkg._cabi.option("ARCQ_POLL_LIMIT", 0):
+            got = run()
+        assert pkg.ops.device_status() == 0x411
+        assert pkg.ops.device_status() == 0
+        assert all(bool((o == 77.0).all()) for o in got)
+        assert all(torch.equal(a, b) for a, b in zip(run(), want))
+    assert pkg.ops.device_status() == 0
