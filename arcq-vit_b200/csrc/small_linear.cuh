@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kSmallLinearThreads, 1) small_linear_kernel(co
     umma_commit(bar);
   }
   __syncwarp();
-  const bool ok = mbar_wait(bar, 0, p.poll_limit);
+  const bool ok = mbar_wait_warp(bar, 0, p.poll_limit);     // a warp whose wait ran out stores none of its rows, and says so
   tc_fence_after_sync();
   // ---- a thread per row, the warps of a tensor-memory lane quarter sixteen columns each
   const int quarter = warp & 3, r = quarter * 32 + lane;
@@ -175,10 +175,8 @@ __global__ void __launch_bounds__(kSmallLinearThreads, 1) small_linear_kernel(co
       }
     }
   }
-  if (!ok && tid == 0) {
-    mbar_wait(bar, 0);       // the products end before their memory is given back
-    atomicExch(p.status, kStatusSmallLinearTimeout);
-  }
+  if (!ok && lane == 0) atomicExch(p.status, kStatusSmallLinearTimeout);
+  if (!ok && tid == 0) mbar_wait(bar, 0);                   // the products end before their memory is given back
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) {

@@ -1,4 +1,6 @@
 """The packed linear in one launch against the two launches it stands for: the same bits, whatever rows and columns a block takes."""
+import ctypes
+
 import pytest
 import torch
 
@@ -18,6 +20,22 @@ def _layer(pkg, dev, K, N, bits, on_the_fly, bias=True, pre_gelu=False, seed=0):
     if pre_gelu:
         layer.pre_gelu = True
     return layer, gen
+
+
+class _Job(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p) for n in ("packed", "mu", "sigma", "codesum", "codebook", "out")] + [
+        ("rows", ctypes.c_int64), ("K", ctypes.c_int64), ("bits", ctypes.c_int)]
+
+
+def _call(pkg, layer, x, y):
+    """The C entry point, into an output of the caller's."""
+    ptr = lambda t: t.data_ptr()
+    job = _Job(ptr(layer.packed_weight_codes), ptr(layer.weight_center), ptr(layer.weight_scale), ptr(layer.weight_code_sum),
+               ptr(layer.weight_codebook), None, y.shape[1], x.shape[1], 4)
+    rc = pkg._cabi.load().arcq_packed_linear_small(0, ptr(x), pkg._cabi.DT_F16, x.shape[0], ptr(layer.activation_thresholds),
+                                                   ptr(layer.activation_codebook), 0, ctypes.byref(job), ptr(layer.bias_tensor), ptr(y),
+                                                   pkg._cabi.DT_F16, None)
+    assert rc == 0, pkg._cabi.last_error()
 
 
 def _both(pkg, layer, x):
@@ -77,6 +95,25 @@ def test_a_wait_that_runs_out(pkg, cuda_device):
         torch.cuda.synchronize()
         assert pkg.ops.device_status() == 0x601
     assert torch.equal(*_both(pkg, layer, x))
+
+
+@pytest.mark.parametrize("polls", [0, 1, 2, 3, 5, 8])
+@pytest.mark.parametrize("M,K,N", [(20, 192, 192), (33, 768, 768), (128, 192, 768)])
+def test_no_row_is_missing_without_a_word(pkg, cuda_device, polls, M, K, N):
+    """Waits that may run out in some warps of a block and not in others: what is not in the output is in the status word."""
+    layer, gen = _layer(pkg, cuda_device, K, N, 4, True)
+    x = torch.randn(M, K, generator=gen, device=cuda_device).half()
+    want, _ = _both(pkg, layer, x)
+    y = torch.empty(M, N, device=cuda_device).half()
+    for _ in range(20):
+        y.fill_(777.0)
+        torch.cuda.synchronize()
+        with pkg._cabi.option("ARCQ_SMALL_LINEAR", 1), pkg._cabi.option("ARCQ_POLL_LIMIT", polls):
+            _call(pkg, layer, x, y)
+        status = pkg.ops.device_status()
+        assert status in (0, 0x601)
+        assert bool(((y == want) | (y == 777.0)).all()) and (status != 0 or torch.equal(y, want))
+    assert torch.equal(layer(x), want) and pkg.ops.device_status() == 0
 
 
 def test_new_inputs_streams_and_capture(pkg, cuda_device):
