@@ -377,6 +377,25 @@ def test_waits_of_the_attention_kernel_that_run_out(pkg, cuda_device, B, T):
     assert pkg.ops.device_status() == 0
 
 
+@pytest.mark.parametrize("polls", [1, 2, 4, 8])
+@pytest.mark.parametrize("B,T", [(1, 17), (1, 197), (200, 197)])
+def test_waits_of_some_warps_that_run_out(pkg, cuda_device, polls, B, T):
+    """A few polls: some warps' waits run out and others' do not.  The kernel ends, a result that is not the whole one has left its code,
+    and the next launch is none the worse."""
+    H = 3
+    qkv = torch.randn(B * T, 3 * H * 64, generator=torch.Generator().manual_seed(T)).half().to(cuda_device)
+    cb = torch.linspace(-2.5, 2.5, 16, device=cuda_device)
+    for quantizer in ((), ((cb[:-1] + cb[1:]) / 2, cb, 4)):
+        want = pkg.ops.attention(qkv, B, T, H, *quantizer)
+        for _ in range(5):
+            with pkg._cabi.option("ARCQ_POLL_LIMIT", polls):
+                got = pkg.ops.attention(qkv, B, T, H, *quantizer)
+            status = pkg.ops.device_status()
+            assert status in (0, 0x501) and (status != 0 or torch.equal(got, want))
+        assert torch.equal(pkg.ops.attention(qkv, B, T, H, *quantizer), want)
+    assert pkg.ops.device_status() == 0
+
+
 @torch.no_grad()
 def test_auto_is_the_kernel_between_packed_linears(pkg, cuda_device, monkeypatch):
     model, images, x = _block(pkg, cuda_device, "deit_small")
