@@ -116,6 +116,10 @@ __device__ __forceinline__ bool mbar_wait_sleep_a(uint32_t bar, uint32_t parity,
   }
   return false;
 }
+// One answer for the whole warp, as mbar_wait_warp.
+__device__ __forceinline__ bool mbar_wait_sleep_warp(uint32_t bar, uint32_t parity, uint32_t limit, uint32_t ns) {
+  return __all_sync(0xffffffffu, mbar_wait_sleep_a(bar, parity, limit, ns)) != 0;
+}
 __device__ __forceinline__ bool mbar_wait_spin_a(uint32_t bar, uint32_t parity, uint32_t limit) {
   for (uint32_t i = 0; i < limit; ++i) {
     if (mbar_test_wait_a(bar, parity)) return true;
@@ -759,7 +763,7 @@ packed_weight_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const _
       const int step = 2 * cw;
       for (int t = 0; t < my_tiles && ok; ++t) {
         const uint32_t buf = static_cast<uint32_t>(t) & 1;
-        if (!mbar_wait_sleep_a(acc_full + buf * 8, (static_cast<uint32_t>(t) >> 1) & 1, poll_limit, 32)) { ok = false; break; }
+        if (!mbar_wait_sleep_warp(acc_full + buf * 8, (static_cast<uint32_t>(t) >> 1) & 1, poll_limit, 32)) { ok = false; break; }
         tc_fence_after_sync();
         const int row0 = row_of(t) + lq * 32;
         const uint32_t t_row = tmem_base + buf * 256 + (static_cast<uint32_t>(lq * 32) << 16);

@@ -351,7 +351,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
         __syncwarp();
         if (!STATIONARY && t + 1 < my_tiles) read_bias(next);
       }
-      if (!mbar_wait_sleep_a(acc_full + buf * 8, (static_cast<uint32_t>(t) >> 1) & 1, poll_limit, 32)) { ok = false; break; }
+      if (!mbar_wait_sleep_warp(acc_full + buf * 8, (static_cast<uint32_t>(t) >> 1) & 1, poll_limit, 32)) { ok = false; break; }
       tc_fence_after_sync();
       const bool live = row0 < p.M && grp * 64 < bn;      // some of these 32 rows are inside the matrix, and the group is one
       uint32_t w[32];
@@ -491,7 +491,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
         if (!STATIONARY && t + 1 < my_tiles) read_bias();
       }
       // (a warp whose wait ran out goes on to the barriers above, without waiting again)
-      ok = ok && mbar_wait_sleep_a(acc_full + buf * 8, (static_cast<uint32_t>(t) >> 1) & 1, poll_limit, 32);
+      ok = ok && mbar_wait_sleep_warp(acc_full + buf * 8, (static_cast<uint32_t>(t) >> 1) & 1, poll_limit, 32);
       if (!ok) continue;
       tc_fence_after_sync();
       const uint32_t t_row = tmem_base + buf * 256 + (static_cast<uint32_t>(lq * 32) << 16);
