@@ -83,7 +83,7 @@ enum Opt {
   O_ACT_QUANT_V1, O_LN_PLAIN,
   O_PAIR, O_PAIR_MIN_M, O_PAIR_BN, O_PAIR_SA, O_PAIR_KS, O_PAIR_NBB, O_PAIR_LUT, O_PAIR_PAIRS, O_PAIR_STATIONARY,
   O_PAIR_WS, O_LNQ_SMALL, O_AQ2_MIN_GROUPS, O_PDL, O_GELU_GEMM, O_GEMM_UNPACK, O_POLL_LIMIT, O_SPIN_LIMIT, O_LAUNCH_REGS,
-  O_SMALL_LINEAR, O_SMALL_R, O_SMALL_BN, O_PAIR_SPLIT,
+  O_SMALL_LINEAR, O_SMALL_R, O_SMALL_BN, O_PAIR_SPLIT, O_PAIR_STAGGER,
   O_COUNT
 };
 struct OptDef { const char* name; int dflt; };
@@ -96,7 +96,7 @@ const OptDef kOptDefs[O_COUNT] = {
     {"ARCQ_PAIR_STATIONARY", -1}, {"ARCQ_PAIR_WS", 0}, {"ARCQ_LNQ_SMALL", 1}, {"ARCQ_AQ2_MIN_GROUPS", 0}, {"ARCQ_PDL", 1},
     {"ARCQ_GELU_GEMM", -1}, {"ARCQ_GEMM_UNPACK", 1},
     {"ARCQ_POLL_LIMIT", 1 << 21}, {"ARCQ_SPIN_LIMIT", 1 << 25}, {"ARCQ_LAUNCH_REGS", 0},
-    {"ARCQ_SMALL_LINEAR", -1}, {"ARCQ_SMALL_R", 0}, {"ARCQ_SMALL_BN", 0}, {"ARCQ_PAIR_SPLIT", 1},
+    {"ARCQ_SMALL_LINEAR", -1}, {"ARCQ_SMALL_R", 0}, {"ARCQ_SMALL_BN", 0}, {"ARCQ_PAIR_SPLIT", 1}, {"ARCQ_PAIR_STAGGER", -1},
 };
 int g_opt[O_COUNT];
 void load_options() {
@@ -558,7 +558,7 @@ bool choose_pair_config(long long M, long long N, long long K, int bits, bool y_
 
 // ---- dense-weight CTA-pair kernel: configuration ----
 struct PairDenseConfig {
-  int bn, sa, ks, pairs, stationary, split_last;
+  int bn, sa, ks, pairs, stationary, split_last, stagger;
   size_t smem;
   double cost;     // of the model that chose it
 };
@@ -689,6 +689,14 @@ bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32,
       const long long left = slabs * tiles_m % k.pairs;
       k.split_last = !stationary && opt(O_PAIR_SPLIT) != 0 && G >= 16 && slabs * tiles_m > k.pairs && left > 0 && 2 * left <= k.pairs && bn % 64 == 0;
       if (k.split_last) cost -= tile / 2;
+      // fp32 outputs at least twice as wide as the rows of A: pairs that keep their slabs and start at different row tiles, where that
+      // takes no more rounds, the last one is 0.3 full at least (a shorter one is over sooner with the tiles dealt out) and A, read for each
+      // slab anew, is well inside L2.  K = 768, N = 2304, 5517 rows 25.9 -> 24.6 us, 9850 rows 42.7 -> 40.5; N = 3072, 7289 rows 42.0 -> 39.9; 15 760
+      // rows, a last round of 4 pairs, 79.8 against 83.4 dealt out; N = 768 the same either way, fp16 outputs 1 to 2 % slower.
+      if (!stationary && !k.split_last && slabs * tiles_m > k.pairs && opt(O_PAIR_STAGGER) != 0) {
+        const bool rule = y_f32 && N >= 2 * K && (tiles_m + per - 1) / per == tiles_pp && (left == 0 || 10 * left >= 3 * k.pairs) && M * K <= (24ll << 20);
+        if (rule || opt(O_PAIR_STAGGER) > 0) { k.pairs = static_cast<int>(slabs * per); k.stagger = 1; }
+      }
       k.cost = cost;
       if (!found || cost < best.cost) { best = k; found = true; }
     }
@@ -1153,7 +1161,7 @@ static int launch_pair_dense_gemm(const PairDenseConfig& cfg, const void* xhat, 
   p.codebook = q_codebook;
   p.bias = bias;
   p.M = static_cast<int>(M); p.N = static_cast<int>(N); p.K = static_cast<int>(K); p.G = static_cast<int>(K / 64);
-  p.bn = cfg.bn; p.sa = cfg.sa; p.ks = cfg.ks; p.split_last = cfg.split_last;
+  p.bn = cfg.bn; p.sa = cfg.sa; p.ks = cfg.ks; p.split_last = cfg.split_last; p.stagger = cfg.stagger;
   p.y_f32 = (y_dtype == ARCQ_DT_F32) ? 1 : 0;
   p.poll_limit = static_cast<uint32_t>(opt(O_POLL_LIMIT));
   p.spin_limit = static_cast<uint32_t>(opt(O_SPIN_LIMIT));

@@ -48,6 +48,7 @@ struct PairDenseParams {
   uint32_t spin_limit;  // the issuing thread's busy waits give up after this many probes
   int* status;
   int pairs;       // CTA pairs that multiply; pairs beyond them take the unpack jobs
+  int stagger;     // pairs are a multiple of the slabs, so that each keeps its slab: those of a rank start at different row tiles (streamed form)
   int split_last;  // the tiles that do not fill a round come as two halves of a slab each (streamed form without a quantizer)
   const float* thresholds;   // quantizer form only
   const float* codebook;
@@ -142,18 +143,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
                        : split    ? full_rounds + (pair < 2 * (tiles_m * n_slabs - full_rounds * n_pairs) ? 1 : 0)
                                   : (tiles_m * n_slabs - pair + n_pairs - 1) / n_pairs;
   // pairs of different slabs that share a rank walk the same row tiles; stagger their starting points
-  const int rot = (STATIONARY && my_tiles > 0) ? (slab * my_tiles) / n_slabs : 0;
+  const bool keeps = STATIONARY || (QBITS == 0 && p.stagger != 0);
+  const int rot = keeps && my_tiles > 0 ? (slab * my_tiles) / n_slabs : 0;
   // The tiles of this pair one after the other: first row of this CTA, first column.  Without a slab that stays, the pairs take the
   // (row tile, slab) combinations in turn, all slabs of a row tile one after the other: every pair has work (slabs x pairs per slab
   // left up to ten of 74 idle), and the slabs read a row tile of A at about the same time (100 864 rows of K = 768, N = 3072: 630 us
-  // before, 505 now; plain form, 50 432 rows 219 -> 180; A is larger than L2 there).  No division on the way to a load: the first
+  // before, 505 now; plain form, 50 432 rows 219 -> 180; A is larger than L2 there).  Wide fp32 outputs of a smaller A are 3 to 5 % faster the
+  // other way, where the pairs keep their slabs and start at different row tiles (stagger).  No division on the way to a load: the first
   // tile is known from above, the others follow by steps.
   const int step_m = STATIONARY ? 0 : n_pairs / n_slabs, step_s = n_pairs - step_m * n_slabs;
   struct Walk {
     int q, m, s;       // stationary: q-th of the pair's row tiles; else how many tiles came before, row tile and slab
     int c, width;      // the tile's columns of the slab
   };
-  auto first_tile = [&]() { return Walk{STATIONARY ? rot : 0, rank, slab, 0, bn}; };
+  auto first_tile = [&]() { return Walk{rot, rank + rot * step_m, slab, 0, bn}; };
   auto row_of = [&](const Walk& w) {
     return (STATIONARY ? rank + w.q * pairs_in_slab : w.m) * kPairTileM + static_cast<int>(crank) * kTileM;
   };
@@ -165,7 +168,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
       w.m += step_m;
       w.s += step_s;
       if (w.s >= n_slabs) { w.s -= n_slabs; ++w.m; }
-      if (QBITS == 0 && split && ++w.q == full_rounds) {
+      ++w.q;
+      if (QBITS == 0 && keeps && w.q == my_tiles) { w.q = 0; w.m = rank; }
+      if (QBITS == 0 && split && w.q == full_rounds) {
         const int left = full_rounds * n_pairs + (pair >> 1);
         w.m = left / n_slabs;
         w.s = left - w.m * n_slabs;
@@ -484,11 +489,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
       const uint32_t buf = static_cast<uint32_t>(t) & 1;
       const int row0 = row_of(next) + lq * 32, n0 = col_of(next), width = next.width;
       advance(next);
-      if (!STATIONARY || t == 0) {
+      if (!keeps || t == 0) {
         if (t > 0) four_warps();
         sb[bi] = next_b;
         four_warps();
-        if (!STATIONARY && t + 1 < my_tiles) read_bias();
+        if (!keeps && t + 1 < my_tiles) read_bias();
       }
       // (a warp whose wait ran out goes on to the barriers above, without waiting again)
       ok = ok && mbar_wait_sleep_warp(acc_full + buf * 8, (static_cast<uint32_t>(t) >> 1) & 1, poll_limit, 32);

@@ -27,6 +27,10 @@ def test_every_tile_gets_its_columns_and_its_bias(pkg, cuda_device, M, N, K, dty
     # a row does not depend on the tile it falls in, a whole one or a half
     with pkg._cabi.option("ARCQ_PAIR_SPLIT", 0):
         assert torch.equal(pkg.ops.dense_weight_gemm(x, w, b, dtype), y)
+        with pkg._cabi.option("ARCQ_PAIR_STAGGER", 1):          # pairs that keep their slabs
+            assert torch.equal(pkg.ops.dense_weight_gemm(x, w, b, dtype), y)
+    with pkg._cabi.option("ARCQ_PAIR_STAGGER", 0):
+        assert torch.equal(pkg.ops.dense_weight_gemm(x, w, b, dtype), y)
     part = pkg.ops.dense_weight_gemm(x[M // 2:].contiguous(), w, b, dtype)
     assert torch.equal(part, y[M // 2:])
     assert pkg.ops.device_status() == 0
