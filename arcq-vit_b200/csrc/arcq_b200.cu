@@ -601,7 +601,7 @@ long long dense_pairs(long long slabs, long long tiles_m, long long max_pairs, b
 }
 
 // Slab width, stages and grid for the dense-weight pair kernel; false leaves the shape to the one-CTA kernel.
-// Cost model in microseconds: a tile is bound by its output stores (about 22 GB/s per SM) or by the issuing thread, and every slab
+// Cost model in microseconds: a tile is bound by its output stores (about 24 GB/s per SM) or by the issuing thread, and every slab
 // streams the whole activation from L2.
 bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32, PairDenseConfig* c) {
   // No row threshold (ARCQ_PAIR_MIN_M gates the packed-weight pair kernel only): with nothing to rebuild, the pair
@@ -635,13 +635,16 @@ bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32,
   // Up to four row tiles (batch 1-5 of a ViT): the launch is a latency chain, not a throughput problem, and the narrowest slab that gives
   // every (tile, slab) its own pair is the shortest chain, as long as that is no more than 40 pairs: every pair beyond them costs the launch
   // more than a narrower slab saves (K = 384, N = 1536: 197 rows 64 columns 4.4 us, 32 4.9; 394 rows 96 columns 4.6, 64 5.1; K = 768, N = 2304,
-  // 197 rows 64 columns 5.6, 32 6.7).  Over twelve layers of the three widths with 197 to 1576 rows the slab chosen is 1.3 % slower than the
-  // fastest; with up to two row tiles and all pairs it was 4.2 %, 24 % at worst.
-  constexpr int kLatencyTiles = 4, kLatencyPairs = 40;
+  // 197 rows 64 columns 5.6, 32 6.7).  Where 40 pairs leave only slabs of more than 128 columns the model below has it: a tile is then
+  // longer than a few pairs more cost (K = 768, N = 2304, 788 rows: 256 columns on 36 pairs 7.7 us, 128 on 72 6.6; N = 3072, 394 rows 192 columns 6.7,
+  // 128 6.1).  Over the same layers with 197 to 788 rows the slab chosen is 0.03 % slower than the fastest, 2.7 % at worst; without the
+  // limit on its width 1.4 and 22 %, with up to two row tiles and all pairs 4.6 and 26 %.
+  constexpr int kLatencyTiles = 4, kLatencyPairs = 40, kLatencyColumns = 128;
   int narrow_bn = 0;
   if (tiles_m <= kLatencyTiles && opt(O_PAIR_BN) == 0)
     for (int bn : cand)
-      if (N % bn == 0 && (N / bn) * tiles_m <= (max_pairs < kLatencyPairs ? max_pairs : kLatencyPairs)) narrow_bn = bn;      // candidates descend: keeps the narrowest
+      if (bn <= kLatencyColumns && N % bn == 0 && (N / bn) * tiles_m <= (max_pairs < kLatencyPairs ? max_pairs : kLatencyPairs))
+        narrow_bn = bn;                                        // candidates descend: keeps the narrowest
   for (int bn : cand) {
     if (N % bn != 0) continue;
     if (opt(O_PAIR_BN) > 0 && bn != opt(O_PAIR_BN)) continue;
@@ -651,7 +654,7 @@ bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32,
     long long per = max_pairs / slabs;
     if (per > tiles_m) per = tiles_m;
     const int esize = y_f32 ? 4 : 2;
-    const double t_write = 128.0 * bn * esize / 22.0e3;
+    const double t_write = 128.0 * bn * esize / 24.4e3;
     for (int stationary = 1; stationary >= 0; --stationary) {
       if (opt(O_PAIR_STATIONARY) >= 0 && stationary != opt(O_PAIR_STATIONARY)) continue;
       if (stationary && G > 32) continue;
@@ -675,26 +678,30 @@ bool choose_pair_dense_config(long long M, long long N, long long K, bool y_f32,
       // what goes through L2 into shared memory: every tile streams its A rows, and its W16 rows too unless the slab is stationary
       const double fill_mb = (static_cast<double>(slabs) * M * K * 2.0 +
                               (stationary ? static_cast<double>(k.pairs) : static_cast<double>(slabs * tiles_m)) * bn * K * 2.0) / 1.0e6;
-      // A tile's stores or its issue, whichever is longer, 0.8 us a tile that neither accounts for, and a twentieth of a microsecond
-      // for every megabyte of fill: it is hidden in part only, behind wide slabs as behind narrow ones.  Fitted to every slab width on
-      // 462 shapes (eleven layers of the three widths, 394 to 25216 rows, both output types): the slab chosen is 1.7 % slower than the
-      // fastest on average, 25 % at worst.  The larger of the tiles' time and of the fill at 8 TB/s had 3.2 and 29 %, with 12 TB/s
-      // from K = 768 on 2.7 and 25 %, and that took narrow slabs for wide fp32 outputs: N = 3072, K = 768, 25216 rows 151 us against
-      // 122, N = 2304 114 against 94; now no shape is more than 2.4 % behind the better of the two.
+      // A tile's stores or its issue, whichever is longer, 0.6 us a tile that neither accounts for, and a twentieth of a microsecond
+      // for every megabyte of fill: it is hidden in part only, behind wide slabs as behind narrow ones.  Fitted to every slab width, with
+      // and without a slab that stays and half tiles, on 600 shapes (twelve layers of the three widths, 197 to 50 432 rows, both output
+      // types): the slab chosen is 1.1 % slower than the fastest on average, 24 % at worst (3001 rows of 192 x 192 to fp32, 32 columns 4.7 us, 64
+      // 3.8), eight shapes by more than 10 %.  The constants fitted to the former order of the tiles (22 GB/s, 0.8 us, a half tile as half
+      // a tile) had 1.6 %, and took 16 % more time than that order for K = 1536, N = 384, 9850 rows (17.1 us, 14.9 with this slab) and 7 %
+      // for K = 384, N = 1536, 18 912 rows (23.5, 22.0).
       const double tile = t_write > t_issue ? t_write : t_issue;
-      double cost = tiles_pp * (tile + 0.8) + fill_mb / 20.0;
+      double cost = tiles_pp * (tile + 0.6) + fill_mb / 20.0;
       // Tiles that would fill half of another round at most come as halves (a half has to be a width of the instruction's), from K =
-      // 1024 on: 12 608 rows of K = 1536, N = 384 are 100 tiles on 74 pairs, 19.5 us whole and 18.0 with the last 26 halved.  A shorter tile
-      // is its stores and its latency: K = 384, N = 384 7.5 / 7.8 us, K = 768, N = 768 25.1 / 25.4, N = 2304 38.7 / 37.9.
+      // 1024 on: 12 608 rows of K = 1536, N = 384 are 100 tiles on 74 pairs, 19.8 us whole and 18.4 with the last 26 halved; a slab of 256
+      // columns is 10 % faster so on average, of 192 6, of 128 2.  In the choice of a width a half counts as nine tenths of a tile: its
+      // stores are half, its latency is not.  From K = 768 down it does not pay: K = 384, N = 384 7.5 / 7.8 us, K = 768, N = 768 25.1 / 25.4, N = 2304 38.7 / 37.9.
       const long long left = slabs * tiles_m % k.pairs;
       k.split_last = !stationary && opt(O_PAIR_SPLIT) != 0 && G >= 16 && slabs * tiles_m > k.pairs && left > 0 && 2 * left <= k.pairs && bn % 64 == 0;
-      if (k.split_last) cost -= tile / 2;
+      if (k.split_last) cost -= tile / 10;
       // fp32 outputs at least twice as wide as the rows of A: pairs that keep their slabs and start at different row tiles, where that
-      // takes no more rounds, the last one is 0.3 full at least (a shorter one is over sooner with the tiles dealt out) and A, read for each
-      // slab anew, is well inside L2.  K = 768, N = 2304, 5517 rows 25.9 -> 24.6 us, 9850 rows 42.7 -> 40.5; N = 3072, 7289 rows 42.0 -> 39.9; 15 760
-      // rows, a last round of 4 pairs, 79.8 against 83.4 dealt out; N = 768 the same either way, fp16 outputs 1 to 2 % slower.
+      // takes no more rounds and A, read for each slab anew, is well inside L2; beyond 16 MB of A only if the last round is 0.3 full at least (a
+      // shorter one is over sooner with the tiles dealt out).  K = 768, N = 2304, 5517 rows 25.9 -> 24.6 us, 8471 rows, a last round of 10 pairs,
+      // 39.4 -> 37.9, 9850 rows 42.7 -> 40.5; N = 3072, 7289 rows 42.0 -> 39.9; 15 760 rows, a last round of 4 pairs, 79.8 against 83.4 dealt out;
+      // N = 768 the same either way, fp16 outputs 1 to 2 % slower.
       if (!stationary && !k.split_last && slabs * tiles_m > k.pairs && opt(O_PAIR_STAGGER) != 0) {
-        const bool rule = y_f32 && N >= 2 * K && (tiles_m + per - 1) / per == tiles_pp && (left == 0 || 10 * left >= 3 * k.pairs) && M * K <= (24ll << 20);
+        const bool rule = y_f32 && N >= 2 * K && (tiles_m + per - 1) / per == tiles_pp && (left == 0 || 10 * left >= 3 * k.pairs || M * K <= (8ll << 20)) &&
+                          M * K <= (24ll << 20);
         if (rule || opt(O_PAIR_STAGGER) > 0) { k.pairs = static_cast<int>(slabs * per); k.stagger = 1; }
       }
       k.cost = cost;
@@ -755,13 +762,14 @@ bool small_layernorm_quant(long long M, long long K) {
 
 // fc1 with GELU and quantizer in its epilogue, or GEMM and quantizer kernel?  Whole forwards through a graph, microseconds, two
 // kernels / one.  The epilogue's 12 warps hide latency worse than the quantizer kernel's 16, so it is rounds that decide: of the
-// fused form's tiles on the pairs against the quantizer's blocks (512 groups an SM).  The line below is fitted to 35 batch sizes of
-// DeiT-T and DeiT-S (DeiT-T batch 32: 717 / 729, 34, where the quantizer starts a second round: 778 / 736; DeiT-S batch 16: 757 /
-// 772, 18: 832 / 785, 48: 1234 / 1259): at one of them it is 15 us, 1 %, off the better form, 40 us over all; "from 6000 rows on"
-// was 186 us off, one round of tiles only 381, both 48 at worst.  Always where the products under the epilogue are long (DeiT-B batch
-// 4: 874 / 821) or the matrix between the two no longer stays in L2 (DeiT-S batch 128: 2678 / 2575, DeiT-B: 7341 / 6902).  Where the
-// quantizer takes its form for small inputs: one round of tiles (DeiT-S batch 6 / 8: 584 / 564, 712 / 660; DeiT-T batch 12: 552 / 527)
-// but not below five row tiles (DeiT-T batch 2: 449 / 463).
+// fused form's tiles on the pairs against the quantizer's blocks (512 groups an SM).  The line below is fitted to 62 batch sizes of
+// DeiT-T, DeiT-S and DeiT-B (DeiT-T batch 32: 679 / 685, 37, where the quantizer has started a second round: 760 / 713; DeiT-S batch 16: 729 /
+// 737, 18: 799 / 749, 64: 1413 / 1379): the worst it does there is two kernels for DeiT-T batch 48, 789 / 781.  The line fitted when every
+// slab had the same number of pairs chose two kernels at thirteen of them, up to 5 % slower (DeiT-T batch 80: 1009 / 956).  Always where
+// the products under the epilogue are long (DeiT-B batch 8: 880 / 871) or the matrix between the two no longer stays in L2 (DeiT-S
+// batch 128: 2483 / 2377, DeiT-B: 6860 / 6188).  Where the quantizer takes its form for small inputs: one round of tiles (DeiT-S
+// batch 6 / 8: 564 / 533, 661 / 608; DeiT-T batch 12: 525 / 496, but 8: 473 / 483), but not below five row tiles (DeiT-T batch 2: 449 / 463,
+// although DeiT-S batch 4: 510 / 503).
 bool choose_gelu_quant(long long M, long long N, long long K, PairDenseConfig* pc) {
   const int force = opt(O_GELU_GEMM);
   if (force == 0 || N % 64 != 0 || !choose_pair_quant_config(M, N, K, pc)) return false;
@@ -771,7 +779,7 @@ bool choose_gelu_quant(long long M, long long N, long long K, PairDenseConfig* p
   if (groups < sms * 256 || !choose_pair_dense_config(M, N, K, false, &plain))
     return M > 1024 && 1ll * pc->pairs * pc->bn >= (M + arcq::kPairTileM - 1) / arcq::kPairTileM * N;
   const double rounds = static_cast<double>((groups + sms * 512 - 1) / (sms * 512));
-  return 1.3 * pc->cost < 4.6 * rounds + plain.cost + 1.0;
+  return 1.2 * pc->cost < 5.7 * rounds + plain.cost - 0.3;
 }
 
 // ---- packed linear in one launch: configuration ----

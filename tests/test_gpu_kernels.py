@@ -700,3 +700,10 @@ def test_kernels_that_hand_registers_over_check_what_a_launch_brings(pkg, cuda_d
 def test_fc1_runs_fused_where_the_rounds_favour_it(pkg, cuda_device, K, rows):
     applies = pkg._cabi.load().arcq_dense_weight_gemm_gelu_quant_applies
     assert {M: bool(applies(M, 4 * K, K)) for M in rows} == rows
+
+
+# where the fused form's tiles, dealt out over all pairs, win although they need a round more than the quantizer
+@pytest.mark.parametrize("K,rows", [(192, {6304: False, 11032: True, 15760: True}), (384, {3152: False, 4728: True, 12608: True, 18912: True})])
+def test_fc1_runs_fused_where_dealt_out_tiles_favour_it(pkg, cuda_device, K, rows):
+    applies = pkg._cabi.load().arcq_dense_weight_gemm_gelu_quant_applies
+    assert {M: bool(applies(M, 4 * K, K)) for M in rows} == rows
