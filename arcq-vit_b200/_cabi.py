@@ -21,6 +21,7 @@ EXPORTS = (
     "arcq_act_quant_unpack", "arcq_add_layernorm_act_quant_unpack", "arcq_add_layernorm_strided",
     "arcq_dense_weight_gemm_unpack", "arcq_dense_weight_gemm_unpack_room", "arcq_unpack_beside_gemm", "arcq_dense_weight_gemm_gelu_quant",
     "arcq_dense_weight_gemm_gelu_quant_applies", "arcq_packed_linear_small", "arcq_packed_linear_small_applies",
+    "arcq_packed_linear_small_applies_captured",
 )
 
 _lib = None
@@ -71,6 +72,7 @@ def load() -> ctypes.CDLL:
     lib.arcq_dense_weight_gemm_prefetch.argtypes = [vp, vp, vp, i64, i64, i64, vp, ci, vp, vp, vp, vp, vp, ci, ci, i64, i64, vp, vp]
     lib.arcq_dense_weight_gemm_gelu_quant_applies.argtypes = [i64, i64, i64]
     lib.arcq_packed_linear_small_applies.argtypes = [i64, i64, i64]
+    lib.arcq_packed_linear_small_applies_captured.argtypes = [i64, i64, i64]
     lib.arcq_packed_linear_small.argtypes = [ci, vp, ci, i64, vp, vp, ci, vp, vp, vp, ci, vp]
     lib.arcq_dense_weight_gemm_gelu_quant.argtypes = [vp, vp, vp, i64, i64, i64, vp, vp, ci, ci, vp, vp, ci, vp]
     for name in EXPORTS:

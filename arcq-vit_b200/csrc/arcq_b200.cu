@@ -1,6 +1,7 @@
 // C ABI of the B200 back end: argument checks, launch configuration, error reporting.
 // The kernels live in the .cuh files included below; this is the only translation unit.
 #include <cuda_runtime.h>
+#include <cmath>
 #include <mutex>
 #include <type_traits>
 #include <cuda_fp16.h>
@@ -787,44 +788,69 @@ struct SmallLinearConfig {
   int R, bn;
   unsigned blocks;
   size_t smem;
+  bool captured;     // the faster way in GPU time too
 };
-// Rows and columns of a block, and whether the one launch is taken: microseconds of GPU time, fitted (4 % rms) to every (R, bn) of twelve
-// layers of the three widths with 1 to 788 rows, in graphs.  A block's time is passes of 96 groups, rounds of unpacking, and the products'
-// chain over k; the pair chosen is 0.7 % slower than the fastest on average, 9 % at worst.  The two launches take what the last line
-// says (10 % rms).  A second launch and its scratch cost the host 3.5 us of a module call's 10.2, so up to 0.8 us more of GPU time is
-// taken for the one: K = 192, N = 192 up to 560 rows (560: 6.6 against 6.1 us of GPU time, calls 10.2 -> 7 us), N = 768 up to 128 (6.7 / 6.0),
-// 384 x 384 up to 64 (7.0 / 6.3), 768 x 768 up to 48 (9.0 / 7.5), 768 x 2304 up to 32, 768 x 3072 up to 24 (10.9 / 10.2).
-bool choose_small_linear(long long M, long long N, long long K, SmallLinearConfig* c) {
+// Rows and columns of a block, and whether the one launch is taken: microseconds of GPU time, fitted to every (R, bn) and to the two
+// launches on 312 combinations of 20 layers and 1 to 1000 rows, in graphs.  A block's time is passes of 96 groups, rounds of unpacking
+// and the products' chain over k; the pair chosen is 1 % slower than the fastest on average, 12 % at worst.  For the comparison the blocks
+// count too (3 % rms, the two launches 6 %).
+//
+// In a captured graph a call costs what the GPU needs, so there the one launch has to be below 0.96 of the two: 88 of the 312, 9 % faster on
+// average, 2.5 % slower at worst (64 x 256, 1000 rows).  Elsewhere the host needs 8.8 to 10.2 us for a call of two launches and 5.3 for the one.
+// While the two are no longer than that on the GPU, 0.8 us more of it by these costs are taken: K = 192, N = 192, 197 rows 6.0 us against 5.6 in a
+// graph, 6.0 against 8.8 a call; 192 x 768, 197 rows 7.0 / 5.6 (the worst of the 312), 7.1 / 8.7 a call; 384 x 1536, 48 rows 7.6 / 7.0 and 7.6 / 8.7; only
+// 768 x 3072 with 16 to 24 rows is slower both ways, 10.5 / 9.3 and 10.5 / 10.2.
+bool search_small_linear(long long M, long long N, long long K, SmallLinearConfig* c) {
   const int force = opt(O_SMALL_LINEAR);
-  if (force == 0 || M <= 0 || M > 4096 || K % 64 != 0 || N % 16 != 0 || K > (1 << 16) || N > (1 << 20)) return false;
-  const int G = static_cast<int>(K / 64), n = static_cast<int>(N);
-  // More than one round of blocks can take with four times 96 groups and 384 columns of a group a block: calls on many rows end here, before
-  // the search (of some 2400 shapes this refuses seven that the costs below would take, all of K >= 1536 and N >= 2304).
-  if (force < 0 && M * N * G * G > 4ll * 148 * 96 * 384) return false;
-  const int sms = sm_count();
-  const double two_launches = 5.3 + 0.002 * static_cast<double>(K) + 1.6e-6 * static_cast<double>(N * K);
-  double limit = force > 0 ? 1.0e9 : two_launches + 0.8;       // what the next candidate has to be below
-  bool found = false;
+  const int G = static_cast<int>(K / 64), n = static_cast<int>(N), sms = sm_count();
+  constexpr int kPass = arcq::kSmallLinearThreads / 8, kRound = arcq::kSmallLinearThreads * 4;
+  // More than one round of blocks can take with four times 96 groups and 384 columns of a group a block: calls on many rows end here.
+  if (force < 0 && M * N * G * G > 4ll * sms * kPass * 384) return false;
+  const auto part = [](int of, int whole) { return of < whole ? static_cast<double>(of) / whole : 1.0; };
+  const auto more = [](int of, int whole) { return (of + whole - 1) / whole - 1; };
+  double best = 1.0e9;
   for (int R : {8, 16, 32, 64, 128}) {
     if (opt(O_SMALL_R) > 0 && R != opt(O_SMALL_R)) continue;
     if (R > 8 && R / 2 >= M) break;
-    constexpr int kPass = arcq::kSmallLinearThreads / 8, kRound = arcq::kSmallLinearThreads * 4;
     const int row_blocks = (static_cast<int>(M) + R - 1) / R, groups = static_cast<int>(M < R ? M : R) * G;
-    const double rows_cost = 0.82 + 2.19 * ((groups + kPass - 1) / kPass) + 1.33 * (groups < kPass ? static_cast<double>(groups) / kPass : 1.0) + 0.078 * G;
-    if (rows_cost + 1.98 > limit) break;                       // more rows a block only cost more
+    const double rows_cost = 4.40 + 2.10 * more(groups, kPass) + 1.23 * part(groups, kPass) + 0.072 * G;
+    if (rows_cost > best) break;                               // more rows a block only cost more
     for (int bn : {16, 32, 48, 64, 96, 128, 192, 256}) {
       if (row_blocks * (n / bn) > sms || n % bn != 0 || (opt(O_SMALL_BN) > 0 && bn != opt(O_SMALL_BN))) continue;
       const int chunks = bn * G * 8;
-      const double cost = rows_cost + 1.98 * ((chunks + kRound - 1) / kRound) + 1.2 * (chunks < kRound ? static_cast<double>(chunks) / kRound : 1.0);
-      if (cost > limit) break;
+      const double cost = rows_cost + 1.77 * more(chunks, kRound) + 1.77 * part(chunks, kRound);
+      if (cost > best) break;
       const size_t smem = arcq::small_linear_smem_layout(R, bn, G).total;
       if (smem > kSmemBudget) break;
-      *c = {R, bn, static_cast<unsigned>(row_blocks * (n / bn)), smem};
-      limit = cost;
-      found = true;
+      *c = {R, bn, static_cast<unsigned>(row_blocks * (n / bn)), smem, false};
+      best = cost;
     }
   }
-  return found;
+  if (best == 1.0e9) return false;
+  const int groups = static_cast<int>(M < c->R ? M : c->R) * G, chunks = c->bn * G * 8;
+  const double one = 4.0 + 2.04 * more(groups, kPass) + 1.2 * part(groups, kPass) + 0.115 * G + 1.78 * more(chunks, kRound) +
+                     1.39 * part(chunks, kRound) + 0.63 * c->blocks / sms;
+  const double two = 4.38 + 0.0021 * static_cast<double>(K) + 1.365e-6 * static_cast<double>(N * K) + 0.112 * std::log2(static_cast<double>(M));
+  c->captured = force > 0 || one <= 0.96 * two;
+  return c->captured || one <= (two < 10.0 ? two + 0.8 : two);
+}
+// The last answer is kept, for the call that follows the question.
+bool choose_small_linear(long long M, long long N, long long K, SmallLinearConfig* c) {
+  if (opt(O_SMALL_LINEAR) == 0 || M <= 0 || M > 4096 || K % 64 != 0 || N % 16 != 0 || K > (1 << 16) || N > (1 << 20)) return false;
+  struct Answer {
+    long long M, N, K;
+    int force, R, bn, sms;
+    bool found;
+    SmallLinearConfig c;
+  };
+  static thread_local Answer last = {};
+  const int force = opt(O_SMALL_LINEAR), R = opt(O_SMALL_R), bn = opt(O_SMALL_BN), sms = sm_count();
+  if (last.M != M || last.N != N || last.K != K || last.force != force || last.R != R || last.bn != bn || last.sms != sms) {
+    last = {M, N, K, force, R, bn, sms, false, {}};
+    last.found = search_small_linear(M, N, K, &last.c);
+  }
+  *c = last.c;
+  return last.found;
 }
 
 }  // namespace
@@ -1348,6 +1374,11 @@ int arcq_dense_weight_gemm_gelu_quant(const void* xhat, const void* w16, const f
 int arcq_packed_linear_small_applies(int64_t M, int64_t N, int64_t K) {
   SmallLinearConfig c;
   return choose_small_linear(M, N, K, &c) ? 1 : 0;
+}
+
+int arcq_packed_linear_small_applies_captured(int64_t M, int64_t N, int64_t K) {
+  SmallLinearConfig c;
+  return choose_small_linear(M, N, K, &c) && c.captured ? 1 : 0;
 }
 
 int arcq_packed_linear_small(int pre_gelu, const void* x, int x_dtype, int64_t M, const float* thresholds, const float* codebook,

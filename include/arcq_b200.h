@@ -240,9 +240,11 @@ int arcq_packed_linear_static_scratch(const void* xhat, const uint8_t* packed_w,
  * the scratch matrices between them, the same bits.  `weight` describes the packed weight [rows = N, K]; its `out` is not used.
  * x fp32, fp16 or bf16 [M,K] (pre_gelu: fp16), y fp16 or fp32 [M,N], 16-byte aligned; K % 64 == 0, N % 16 == 0, groups of 64.
  * Where one round of blocks that each make their own operands is not the faster way, ARCQ_E_UNSUPPORTED, which
- * arcq_packed_linear_small_applies (1 / 0) says beforehand.
+ * arcq_packed_linear_small_applies (1 / 0) says beforehand.  That is judged for calls whose host time counts;
+ * arcq_packed_linear_small_applies_captured is 1 where the GPU's time alone is shorter too: the question for a stream under capture.
  */
 int arcq_packed_linear_small_applies(int64_t M, int64_t N, int64_t K);
+int arcq_packed_linear_small_applies_captured(int64_t M, int64_t N, int64_t K);
 int arcq_packed_linear_small(int pre_gelu, const void* x, int x_dtype, int64_t M, const float* thresholds, const float* codebook,
                              int one_fma, const arcq_unpack_job* weight, const float* bias, void* y, int y_dtype, void* stream);
 

@@ -136,3 +136,20 @@ def test_new_inputs_streams_and_capture(pkg, cuda_device):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, want[2]) and torch.equal(z, layer(want[2]))
+
+
+def test_a_captured_call_takes_what_the_gpu_does_faster(pkg, cuda_device):
+    """192 x 192: eight rows in one launch either way, 197 only where the host's time counts; the same bits."""
+    layer, gen = _layer(pkg, cuda_device, 192, 192, 4, True)
+    for M, captured in ((8, True), (197, False)):
+        x = torch.randn(M, 192, generator=gen, device=cuda_device).half()
+        want = layer(x)
+        assert pkg._cabi.last_gemm_kernel() == pkg._cabi.GEMM_SMALL_LINEAR
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            y = layer(x)
+            assert (pkg._cabi.last_gemm_kernel() == pkg._cabi.GEMM_SMALL_LINEAR) == captured
+        y.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, want)

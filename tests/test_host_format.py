@@ -194,3 +194,13 @@ def test_c_abi_rejects_bad_arguments_before_any_launch(pkg):
 def test_packed_linear_in_one_launch_by_rows(pkg, K, N, rows):
     applies = pkg._cabi.load().arcq_packed_linear_small_applies
     assert {M: bool(applies(M, N, K)) for M in rows} == rows
+
+
+# what the host's time is worth is not worth it in a captured graph; never there what is not taken outside
+@pytest.mark.parametrize("K,N,rows", [(192, 192, {8: True, 32: True, 197: False, 560: False}), (768, 192, {8: False, 96: False}),
+                                      (768, 3072, {1: True, 24: False}), (384, 384, {1: False, 64: False}), (384, 1536, {1: True, 48: False})])
+def test_packed_linear_in_one_launch_under_capture(pkg, K, N, rows):
+    lib = pkg._cabi.load()
+    assert {M: bool(lib.arcq_packed_linear_small_applies_captured(M, N, K)) for M in rows} == rows
+    for M in range(1, 1200):
+        assert lib.arcq_packed_linear_small_applies(M, N, K) >= lib.arcq_packed_linear_small_applies_captured(M, N, K)
