@@ -35,6 +35,19 @@ def _dev(t: torch.Tensor, name: str, dtype=None) -> torch.Tensor:
     return t.contiguous()
 
 
+def _const(t: torch.Tensor, name: str, dtype=None) -> torch.Tensor:
+    """``_dev`` for what belongs to a layer: the kernels read it while the kernel before theirs may still run."""
+    c = _dev(t, name, dtype)
+    return c if c.data_ptr() == t.data_ptr() else _settled(c)
+
+
+def _settled(*copies: torch.Tensor):
+    """Copies made for a call that a kernel reads early: with another kernel launched behind them, they are written before that kernel
+    starts and not only before it ends."""
+    torch.zeros(1, device=copies[0].device)
+    return copies if len(copies) > 1 else copies[0]
+
+
 def packed_cols(length: int, bits: int) -> int:
     return (length * bits + 7) // 8
 
@@ -61,8 +74,8 @@ def quantize_activation(x: torch.Tensor, thresholds: torch.Tensor, codebook: tor
     if x.dtype not in _DT:
         raise RuntimeError(f"x must be float32, float16 or bfloat16, got {x.dtype}")
     x = _dev(x, "x")
-    th = _dev(thresholds, "thresholds", torch.float32)
-    cb = _dev(codebook, "codebook", torch.float32)
+    th = _const(thresholds, "thresholds", torch.float32)
+    cb = _const(codebook, "codebook", torch.float32)
     if cb.numel() != 2 ** bits or th.numel() != 2 ** bits - 1:
         raise RuntimeError(f"codebook/thresholds must have {2 ** bits}/{2 ** bits - 1} entries")
     M, K = x.shape
@@ -92,8 +105,8 @@ def quantize_activation_dequant(x: torch.Tensor, thresholds: torch.Tensor, codeb
     if x.dim() != 2 or x.dtype not in _DT or out_dtype not in _DT:
         raise RuntimeError("x must be a 2-D float tensor and out_dtype a float dtype")
     x = _dev(x, "x")
-    th = _dev(thresholds, "thresholds", torch.float32)
-    cb = _dev(codebook, "codebook", torch.float32)
+    th = _const(thresholds, "thresholds", torch.float32)
+    cb = _const(codebook, "codebook", torch.float32)
     M, K = x.shape
     out = torch.empty((M, K), dtype=out_dtype, device=x.device)
     if M == 0:
@@ -121,8 +134,8 @@ def arcq_linear_forward(packed_x, x_center, x_scale, x_code_sum, packed_w, w_cen
     """
     lib = _cabi.load()
     packed_x = _dev(packed_x, "packed_x", torch.uint8)
-    packed_w = _dev(packed_w, "packed_w", torch.uint8)
-    f = [_dev(t, n, torch.float32) for t, n in (
+    packed_w = _const(packed_w, "packed_w", torch.uint8)
+    f = [_const(t, n, torch.float32) for t, n in (
         (x_center, "x_center"), (x_scale, "x_scale"), (x_code_sum, "x_code_sum"), (w_center, "w_center"),
         (w_scale, "w_scale"), (w_code_sum, "w_code_sum"), (act_codebook, "act_codebook"), (w_codebook, "w_codebook"))]
     if out_dtype not in (torch.float32, torch.float16):
@@ -134,7 +147,7 @@ def arcq_linear_forward(packed_x, x_center, x_scale, x_code_sum, packed_w, w_cen
                            f"K={in_features} N={out_features} bits={bits}")
     b = None
     if bias is not None and bias.numel() > 0:
-        b = _dev(bias, "bias", torch.float32)
+        b = _const(bias, "bias", torch.float32)
         if b.numel() != out_features:
             raise RuntimeError("bias must have out_features entries")
     if (LINEAR_FORWARD_ROUTE != "single" and M > 0
@@ -170,8 +183,8 @@ def packed_weight_gemm(xhat: torch.Tensor, packed_w, w_center, w_scale, w_code_s
     """
     lib = _cabi.load()
     xhat = _dev(xhat, "xhat", torch.float16)
-    packed_w = _dev(packed_w, "packed_w", torch.uint8)
-    f = [_dev(t, n, torch.float32) for t, n in ((w_center, "w_center"), (w_scale, "w_scale"),
+    packed_w = _const(packed_w, "packed_w", torch.uint8)
+    f = [_const(t, n, torch.float32) for t, n in ((w_center, "w_center"), (w_scale, "w_scale"),
                                                 (w_code_sum, "w_code_sum"), (w_codebook, "w_codebook"))]
     if out_dtype not in (torch.float32, torch.float16):
         raise RuntimeError("out_dtype must be float32 or float16")
@@ -181,7 +194,7 @@ def packed_weight_gemm(xhat: torch.Tensor, packed_w, w_center, w_scale, w_code_s
         raise RuntimeError(f"packed weight {tuple(packed_w.shape)} / stats {tuple(f[0].shape)} do not match K={K}")
     b = None
     if bias is not None and bias.numel() > 0:
-        b = _dev(bias, "bias", torch.float32)
+        b = _const(bias, "bias", torch.float32)
         if b.numel() != N:
             raise RuntimeError("bias must have out_features entries")
     y = torch.empty((M, N), dtype=out_dtype, device=xhat.device)
@@ -219,7 +232,7 @@ def _norm_params(norm: torch.nn.LayerNorm, device):
     w, b = norm.weight.detach(), norm.bias.detach()
     if w.dtype == b.dtype and w.dtype in _DT and all(t.device == device and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (w, b)):
         return w, b
-    return tuple(t.to(device=device, dtype=torch.float32).contiguous() for t in (w, b))
+    return _settled(*(t.to(device=device, dtype=torch.float32).contiguous() for t in (w, b)))
 
 
 def add_layernorm_quant(x: torch.Tensor, y, norm: torch.nn.LayerNorm, thresholds: torch.Tensor, codebook: torch.Tensor,
@@ -233,7 +246,7 @@ def add_layernorm_quant(x: torch.Tensor, y, norm: torch.nn.LayerNorm, thresholds
     K = shape[-1]
     x2 = _dev(x.reshape(-1, K), "x", torch.float16)
     y2 = None if y is None else _dev(y.reshape(-1, K), "y", torch.float16)
-    thresholds, codebook = _dev(thresholds, "thresholds", torch.float32), _dev(codebook, "codebook", torch.float32)
+    thresholds, codebook = _const(thresholds, "thresholds", torch.float32), _const(codebook, "codebook", torch.float32)
     if K not in (192, 384, 768):
         # widths the merged kernel is not built for: the two kernels it stands for (same results)
         s, h = add_layernorm(x, y, norm)
@@ -269,7 +282,7 @@ def attention(qkv: torch.Tensor, batch: int, tokens: int, heads: int, thresholds
         q2 = q2.clone()
     out = torch.empty((batch * tokens, C), dtype=torch.float16, device=q2.device)
     if thresholds is not None:
-        thresholds, codebook = _dev(thresholds, "thresholds", torch.float32), _dev(codebook, "codebook", torch.float32)
+        thresholds, codebook = _const(thresholds, "thresholds", torch.float32), _const(codebook, "codebook", torch.float32)
     # like an operator of the framework, which launches where its tensors are whatever the current device is
     with torch.cuda.device(q2.device):
         if thresholds is None:
@@ -355,7 +368,7 @@ def dense_weight_gemm(xhat: torch.Tensor, w16: torch.Tensor, bias, out_dtype: to
         raise RuntimeError(f"weight {tuple(w16.shape)} does not match K={K}")
     b = None
     if bias is not None and bias.numel() > 0:
-        b = _dev(bias, "bias", torch.float32)
+        b = _const(bias, "bias", torch.float32)
         if b.numel() != N:
             raise RuntimeError("bias must have out_features entries")
     y = torch.empty((M, N), dtype=out_dtype, device=xhat.device)
@@ -390,7 +403,7 @@ def dense_weight_gemm_gelu_quant(xhat: torch.Tensor, w16: torch.Tensor, bias, th
     lib = _cabi.load()
     xhat = _dev(xhat, "xhat", torch.float16)
     w16 = _dev(w16, "w16", torch.float16)
-    thresholds, codebook = _dev(thresholds, "thresholds", torch.float32), _dev(codebook, "codebook", torch.float32)
+    thresholds, codebook = _const(thresholds, "thresholds", torch.float32), _const(codebook, "codebook", torch.float32)
     M, K = xhat.shape
     N = w16.shape[0]
     if w16.dim() != 2 or w16.shape[1] != K:
@@ -399,7 +412,7 @@ def dense_weight_gemm_gelu_quant(xhat: torch.Tensor, w16: torch.Tensor, bias, th
         raise RuntimeError(f"expected {2 ** bits} levels and {2 ** bits - 1} thresholds")
     b = None
     if bias is not None and bias.numel() > 0:
-        b = _dev(bias, "bias", torch.float32)
+        b = _const(bias, "bias", torch.float32)
         if b.numel() != N:
             raise RuntimeError("bias must have out_features entries")
     out = torch.empty((M, N), dtype=torch.float16, device=xhat.device)

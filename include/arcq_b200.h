@@ -17,6 +17,11 @@
  *                  a little-endian bit stream (FQ/fair_qat/arcq_packed_py.py:8-78)
  *   per-group stats fp32 [rows, len/group_size]   mean, scale, sum of code values
  *   codebook       fp32 [2^bits] ascending;  thresholds fp32 [2^bits-1] = midpoints
+ *
+ * Order on the stream: a call runs behind everything enqueued before it, with one exception.  What belongs to a layer (thresholds,
+ * codebooks, bias, LayerNorm parameters, packed weights and their statistics) may be read while the kernel enqueued just before is
+ * still running, so an earlier one has to have written it.  arcq_dequant, arcq_unpack_weight_f16, arcq_pack_codes and arcq_unpack_codes
+ * read nothing early.
  */
 #ifndef ARCQ_B200_H_
 #define ARCQ_B200_H_
