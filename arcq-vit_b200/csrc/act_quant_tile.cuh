@@ -3,9 +3,10 @@
 // tile's store in flight meanwhile.  No block-wide synchronisation after the table set-up.
 //
 // Bound by issue slots (half of them used: fixed latencies and instruction fetches of the straight-line group routine), then by
-// shared-memory reads (about three wavefronts per 32 values).  One lane a group, 16 warps an SM.  [12608, 384] 5.2 us, [50432,
-// 768] 29.3 us (5.3 TB/s), with GELU [12608, 1536] 24.1 us; 6.3, 31.2 and 24.5 us when a level took three table reads and a value
-// at a threshold sent its seven neighbours through the exact path too.
+// shared-memory reads (about three wavefronts per 32 values).  One lane a group, 16 warps an SM.  [12608, 384] 4.9 us, [50432,
+// 768] 28.7 us (5.4 TB/s), with GELU [12608, 1536] 25.1 us; 6.3, 31.2 and 24.5 us when a level took three table reads and a value
+// at a threshold sent its seven neighbours through the exact path too.  Groups whose values are all equal, those beyond the matrix in the
+// last tile among them, take that path for every value if a threshold is 0 (group_quant.cuh): [3001, 3072] with such a codebook 24.6 us.
 #pragma once
 #include <cuda.h>
 #include "ptx.cuh"

@@ -20,7 +20,7 @@
 // and the scores of the item after the next are computed, so that the softmax warps go from item to item without a wait: 3700 cycles
 // an item (maximum 600, exponentials 2100 alone and 2700 beside the output warps).  What is left is the exponentials' pipe, 8 cycles a
 // warp or 1664 an item, issue slots, about 2400 an item, and instruction fetches.  With quantizer, 197 tokens: 64 images of 6 heads
-// 20.0 -> 18.1 us, 32 images 14.3 -> 11.4, 256 images of 12 heads 112 -> 101, one image 7.7 -> 7.2, against two blocks an SM with one item
+// 20.0 -> 18.1 us, 32 images 14.3 -> 11.5, 256 images of 12 heads 112 -> 102, one image 7.7 -> 7.3, against two blocks an SM with one item
 // each and a thread per row, whose softmax warps waited for P V, for the read of O and for the next Q K^T.
 //
 // Tensor memory is allocated after the previous kernel has ended and before the next one may start: a GEMM that holds all of

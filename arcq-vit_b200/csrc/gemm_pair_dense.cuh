@@ -147,8 +147,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
   const int rot = keeps && my_tiles > 0 ? (slab * my_tiles) / n_slabs : 0;
   // The tiles of this pair one after the other: first row of this CTA, first column.  Without a slab that stays, the pairs take the
   // (row tile, slab) combinations in turn, all slabs of a row tile one after the other: every pair has work (slabs x pairs per slab
-  // left up to ten of 74 idle), and the slabs read a row tile of A at about the same time (100 864 rows of K = 768, N = 3072: 630 us
-  // before, 505 now; plain form, 50 432 rows 219 -> 180; A is larger than L2 there).  Wide fp32 outputs of a smaller A are 3 to 5 % faster the
+  // left up to ten of 74 idle), and the slabs read a row tile of A at about the same time (100 864 rows of K = 768, N = 3072: 634 us
+  // before, 499 now; plain form, 50 432 rows 224 -> 186; A is larger than L2 there; medians with pauses between, back to back under the
+  // power cap 642 and 602).  Wide fp32 outputs of a smaller A are 3 to 5 % faster the
   // other way, where the pairs keep their slabs and start at different row tiles (stagger).  No division on the way to a load: the first
   // tile is known from above, the others follow by steps.
   const int step_m = STATIONARY ? 0 : n_pairs / n_slabs, step_s = n_pairs - step_m * n_slabs;
@@ -324,8 +325,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QBITS ? kPairQuantTh
     // A thread owns one row and 64 columns, i.e. one group of the next layer's activation quantizer: tensor memory -> + bias ->
     // fp16 (what the plain form stores) -> GELU -> quantizer -> reconstruction, in registers but for the exchange of large GELU
     // arguments, then through this warp's staging rows to a TMA store.  Issue slots and the FMA pipe (54 % busy)
-    // of these warps bound the kernel, about 28 instructions a value; the products run underneath.  K = 768, N = 3072, back to back with
-    // inputs in turn: 12608 rows 66 us, 100864 rows 500 (GEMM and quantizer kernel 360 + 329); K = 384, N = 1536, 12608 rows 32.
+    // of these warps bound the kernel, about 28 instructions a value; the products run underneath.  K = 768, N = 3072, inputs in
+    // turn: 12608 rows 66 us, 100864 rows 499, 560 to 600 back to back under the power cap (GEMM and quantizer kernel 360 + 329); K = 384, N = 1536,
+    // 12608 rows 32.
     const int ew = warp - kIssue, lq = warp & 3, grp = ew >> 2;
     GroupQuantTables* const tables = reinterpret_cast<GroupQuantTables*>(smem + L.tables);
     const GroupQuantParams gp = group_quant_tables<1 << QBITS, false>(tables, p.thresholds, p.codebook, tid - kIssue * 32, kEpi * 32, [](bool b) {

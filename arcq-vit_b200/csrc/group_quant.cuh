@@ -22,7 +22,8 @@
 // The two differ only if 0 < r - th * s <= h * s, so a value with |d| <= s * max h goes through the IEEE quotient and a search
 // over all thresholds: about one in a million (15 thresholds, +-1.5e-7 each, at a density of 0.3), i.e. a few of nearly every
 // launch's warps, which the launch then waits for.  A codebook with two thresholds closer than 1.1 cells takes that path for every
-// value.
+// value, and a threshold of exactly 0 (symmetric codebooks, every 2-bit one that is fitted) sends every value of a group of equal values
+// there: one such warp costs a launch 16 us ([3001, 3072] 24.6 us, 8.3 with the thresholds moved by 0.01).
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>

@@ -6,7 +6,7 @@
 // The separate kernels write h and read it back; here it goes through shared memory.
 //
 // Bound by HBM for large inputs: [201728, 768] 211 us, 1.24 GB at 5.9 TB/s of the 6.5 a copy reaches ([50432, 768] 57.5 us, [12608, 384]
-// 10.7 us).  253, 67.3 and 11.2 us with rows read by ordinary loads, whose latency every pass of phase 1 waited for, and with scalar
+// 10.5 us).  253, 67.3 and 11.2 us with rows read by ordinary loads, whose latency every pass of phase 1 waited for, and with scalar
 // arithmetic (36 instructions a value instead of 26).
 //
 // Two phases per tile, each in the thread layout that suits it, and each with the arithmetic of the kernel it
