@@ -483,13 +483,15 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     }
     if (lane == 0) tma_store_wait_all();
   }
-  if (!ok) atomicExch(p.status, kStatusAttentionTimeout);
   tc_fence_before_sync();
   const bool gave_up = __syncthreads_or(!ok) != 0;
   if (warp == 17) {
     tc_fence_after_sync();
     if (gave_up) {                                // nobody may have waited for the last products: they end before their memory is given back
-      if (elect_one()) umma_commit(stopped);
+      if (elect_one()) {
+        umma_commit(stopped);
+        atomicExch(p.status, kStatusAttentionTimeout);
+      }
       __syncwarp();
       mbar_wait(stopped, 0);
       __syncwarp();
